@@ -189,6 +189,143 @@ __global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* __rest
   }
 }
 
+// The same logits, bit for bit, at prefill width (tokens > kMaxTok). Bound: the fp32 pipe (tokens x rows x 2560
+// multiply-adds). router_kernel above re-reads x for every row and keeps four tokens in flight: 0.96 us per token,
+// 963 us at 1003 tokens; this kernel takes 105 us there (fp32 pipe 43 % busy, 3.7 waves of blocks) and 27 us for up
+// to 256 tokens.
+// A block owns 32 rows x 32 tokens; its sixteen warps split K the way router_kernel's lanes do: the partial sum of
+// lane l (elements 256 c + 8 l + i, added over c, then i) belongs to warp l mod 16, which adds those of lanes l and
+// l + 16; the sixteen results meet in shared memory in the butterfly's order. A thread accumulates 8 rows x 4 tokens
+// in packed pairs of rows (fma.rn.f32x2: two multiply-adds per instruction, each rounded as fmaf is). 256-wide K
+// chunks lie row-major in three cp.async buffers, rows 16 bytes apart modulo the banks: one 16-byte load brings a
+// row's eight elements of a lane class, and the widening to fp32 (a shift or a mask) shares the issue slots that the
+// packed multiply-adds leave. (A K-major copy in fp32, widened while staging, took 142 us: its global loads touched
+// 32 rows per instruction.)
+constexpr int kRtRows = 32, kRtTok = 32, kRtChunk = 256, kRtBufs = 3;
+template <bool XBF16>
+constexpr int router_tile_pitch() { return kRtChunk * (XBF16 ? 2 : 4) + 16; }  // bytes between token rows
+constexpr int kRtWPitch = kRtChunk * 2 + 16;                                  // and between weight rows
+template <bool XBF16>
+constexpr int router_tile_buf() { return kRtRows * kRtWPitch + kRtTok * router_tile_pitch<XBF16>(); }
+template <bool XBF16>
+constexpr int router_tile_smem() { return kRtBufs * router_tile_buf<XBF16>(); }
+static_assert(16 * kRtRows * kRtTok * 4 <= router_tile_smem<true>(), "the warps' partial tiles reuse the buffers");
+
+__device__ __forceinline__ void fma_f32x2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+__device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
+}
+
+template <bool XBF16>
+__global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16* __restrict__ w, int rows,
+                                                             const void* __restrict__ xv, int tokens,
+                                                             float* __restrict__ logits, int stride) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int kXPitch = router_tile_pitch<XBF16>(), kBuf = router_tile_buf<XBF16>(), kChunks = H / kRtChunk;
+  pdl_launch_dependents();
+  pdl_wait_prior();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row_base = blockIdx.x * kRtRows, tok_base = blockIdx.y * kRtTok;
+  // a warp copies two weight rows and two token rows of a chunk; rows and tokens beyond the end repeat the last one
+  // (they are computed and not stored)
+  auto fetch = [&](int c) {
+    uint8_t* buf = smem + (c % kRtBufs) * kBuf;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int r = warp + 16 * p;
+      cp_async_16(buf + r * kRtWPitch + 16 * lane, w + size_t(min(row_base + r, rows - 1)) * H + kRtChunk * c + 8 * lane);
+      uint8_t* xd = buf + kRtRows * kRtWPitch + r * kXPitch + 16 * lane;
+      const size_t at = size_t(min(tok_base + r, tokens - 1)) * H + kRtChunk * c;
+      if constexpr (XBF16) {
+        cp_async_16(xd, static_cast<const __nv_bfloat16*>(xv) + at + 8 * lane);
+      } else {
+        cp_async_16(xd, static_cast<const float*>(xv) + at + 4 * lane);
+        cp_async_16(xd + 512, static_cast<const float*>(xv) + at + 128 + 4 * lane);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // thread = rows rg + 4 j (j = 0..7, pairs of neighbouring j) x tokens tg + 8 t (t = 0..3)
+  const int rg = lane >> 3, tg = lane & 7;
+  uint64_t acc[2][4][4];  // [lane class warp, warp + 16][row pair][token]
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) acc[c][r][t] = 0;
+  fetch(0);
+  fetch(1);
+  for (int c = 0; c < kChunks; ++c) {
+    if (c + 1 < kChunks) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // chunk c is in place, and nobody reads the buffer that the next fetch fills
+    if (c + 2 < kChunks) fetch(c + 2);
+    const uint8_t* buf = smem + (c % kRtBufs) * kBuf;
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) {
+      const int cls = ch >> 1, e = 4 * (ch & 1);
+      const int piece = warp + 16 * cls;  // elements 8 piece + e .. + 3 of the chunk
+      uint64_t xx[4][4];                  // token values, both halves alike: made once, used by four row pairs
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const uint8_t* xp = buf + kRtRows * kRtWPitch + (tg + 8 * t) * kXPitch + (8 * piece + e) * (XBF16 ? 2 : 4);
+        uint32_t v[4];
+        if constexpr (XBF16) {
+          const uint2 a = *reinterpret_cast<const uint2*>(xp);
+          v[0] = a.x << 16; v[1] = a.x & 0xFFFF0000u; v[2] = a.y << 16; v[3] = a.y & 0xFFFF0000u;
+        } else {
+          const uint4 a = *reinterpret_cast<const uint4*>(xp);
+          v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) xx[t][i] = pack_f32x2(v[i], v[i]);
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint2 a = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r) * kRtWPitch + 16 * piece + 2 * e);
+        const uint2 b = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r + 4) * kRtWPitch + 16 * piece + 2 * e);
+        const uint64_t wp[4] = {pack_f32x2(a.x << 16, b.x << 16), pack_f32x2(a.x & 0xFFFF0000u, b.x & 0xFFFF0000u),
+                                pack_f32x2(a.y << 16, b.y << 16), pack_f32x2(a.y & 0xFFFF0000u, b.y & 0xFFFF0000u)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) fma_f32x2(acc[cls][r][t], wp[i], xx[t][i]);
+      }
+    }
+  }
+  __syncthreads();
+  float* part = reinterpret_cast<float*>(smem);  // [warp][token][row]
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float2 a = *reinterpret_cast<const float2*>(&acc[0][r][t]), b = *reinterpret_cast<const float2*>(&acc[1][r][t]);
+      float* q = part + (warp * kRtTok + tg + 8 * t) * kRtRows + rg + 8 * r;
+      q[0] = a.x + b.x;
+      q[4] = a.y + b.y;
+    }
+  __syncthreads();
+  for (int o = tid; o < kRtRows * kRtTok; o += 512) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = part[i * kRtRows * kRtTok + o];
+#pragma unroll
+    for (int n = 8; n >= 1; n >>= 1)
+#pragma unroll
+      for (int i = 0; i < n; ++i) v[i] += v[i + n];
+    const int t = tok_base + o / kRtRows, r = row_base + (o & (kRtRows - 1));
+    if (t < tokens && r < rows) logits[size_t(t) * stride + r] = v[0];
+  }
+}
+
 // The part of the work list a producer needs, in shared memory: the producer is a single thread, and a
 // chain of dependent global loads per tile (visiting order -> item -> its pairs -> their tokens and
 // weights, about two microseconds) would pace the whole kernel. Either copied from the device work list
@@ -1322,6 +1459,27 @@ int32_t fb_router_logits(const void* w_bf16, int32_t rows, const void* x, int32_
                          float* logits, int32_t logits_stride, void* stream) {
   if (!w_bf16 || !x || !logits || rows <= 0 || tokens <= 0 || logits_stride < rows)
     return invalid("router_logits: bad arguments");
+  if (tokens > kMaxTok) {
+    static PerDeviceOnce once;
+    const cudaError_t attr = per_device_once(once, [] {
+      cudaError_t a = opt_in_smem(router_tile_kernel<true>, router_tile_smem<true>());
+      return a == cudaSuccess ? opt_in_smem(router_tile_kernel<false>, router_tile_smem<false>()) : a;
+    });
+    if (attr != cudaSuccess) {
+      set_error("router_logits: shared-memory opt-in: %s", cudaGetErrorString(attr));
+      return int32_t(attr);
+    }
+    const dim3 tiles((rows + kRtRows - 1) / kRtRows, (tokens + kRtTok - 1) / kRtTok);
+    const auto* wb = static_cast<const __nv_bfloat16*>(w_bf16);
+    const cudaError_t e =
+        x_dtype == FB_DT_BF16
+            ? launch_pdl(router_tile_kernel<true>, tiles, dim3(512), size_t(router_tile_smem<true>()), as_stream(stream),
+                         wb, rows, x, tokens, logits, logits_stride)
+            : launch_pdl(router_tile_kernel<false>, tiles, dim3(512), size_t(router_tile_smem<false>()),
+                         as_stream(stream), wb, rows, x, tokens, logits, logits_stride);
+    if (e != cudaSuccess) return check_launch("router_logits");
+    return 0;
+  }
   const dim3 grid((rows + 3) / 4), block(128);
   cudaError_t e = x_dtype == FB_DT_BF16
                       ? launch_pdl(router_kernel<true>, grid, block, 0, as_stream(stream),

@@ -244,6 +244,23 @@ def forced_logits(tokens, experts_per_token):
     return l
 
 
+@pytest.mark.parametrize("rows,tokens,bf16", [(513, 17, True), (513, 33, False), (40, 65, True), (1, 100, False)])
+def test_wide_router_gives_the_bits_of_the_narrow_one(rows, tokens, bf16):
+    """Above 16 tokens fb_router_logits runs in tiles of 32 rows x 32 tokens that add the products in the same
+    order: the same bits as slices of at most 16 tokens, and nothing written outside [tokens][rows]."""
+    torch = _torch()
+    from fngine_b200 import moe
+    w = torch.from_numpy(synth.router_weights(5, rows=rows).view(np.int16)).cuda().view(torch.bfloat16)
+    x = torch.from_numpy(synth.activations(6, tokens)).cuda()
+    x = x.to(torch.bfloat16) if bf16 else x
+    wide = torch.full((tokens + 1, rows + 3), -7.0, device="cuda")
+    narrow = wide.clone()
+    moe.router_logits(w, x, wide, rows + 3)
+    for t in range(0, tokens, 16):
+        moe.router_logits(w, x[t:t + 16], narrow[t:], rows + 3)
+    assert torch.equal(wide, narrow)
+
+
 @pytest.mark.parametrize("fg,fd,inter", [(IQ3_S, IQ3_S, 512), (IQ4_NL, IQ4_NL, 512), (IQ3_S, IQ4_NL, 640),
                                          (IQ4_NL, IQ4_NL, 640)])
 def test_single_expert_rows(fg, fd, inter):
