@@ -182,20 +182,6 @@ struct RingN {
   volatile int* end_seq;
 };
 
-// try_wait with a suspend-time hint: the thread may sleep inside the instruction until the phase
-// completes or about a microsecond has passed, instead of spinning through issue slots the working
-// warps need.
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
-      : "memory");
-  return ok != 0;
-}
 // Bounded: 2^21 tries of at most about a microsecond each.
 __device__ __forceinline__ bool mbar_wait_hint(uint64_t* bar, uint32_t parity) {
   for (uint32_t i = 0; i < (1u << 21); ++i)

@@ -1,0 +1,645 @@
+// The grouped GEMM kernel of the prefill path, included by moe_prefill.cu inside namespace fb's anonymous namespace.
+// One persistent kernel, one CTA per SM, for both projections:
+//   gate/up  unit = 64 intermediate rows of one expert x up to 256 of its tokens; the 128 tensor-memory lanes hold
+//            gate and up rows in turn (lane 2i = gate row i, lane 2i + 1 = up row i), so that SwiGLU pairs a lane with
+//            its neighbour;
+//   down     unit = 128 output rows x up to 128 tokens (two accumulators: the epilogue, which is half of the work here,
+//            overlaps the next unit; with 256 tokens per unit the projection took 667 instead of 411 us at 8192 tokens).
+//
+// What bounds it is the decoding of the weights: every weight passes the integer pipe once per (expert, 256-token
+// unit) however few tokens the unit has. So the decoded bf16 values go from registers straight into TENSOR MEMORY,
+// where tcgen05.mma takes its A operand from: no shared-memory store of the tile, no read of it by the tensor core,
+// no proxy fence, and 256 columns of ring space (K = 512) that cost no shared memory. (The version before this one
+// stored swizzled tiles into a three-stage shared-memory ring: 8 weights per clock and SM.)
+//
+// The B operand comes by TMA from rows in pair order: h for the down projection; for gate/up the token rows are first
+// copied into that order (gather_rows_kernel). (Gathered by cp.async inside this kernel, a unit of 256 tokens cost
+// 2048 load/store cycles per 256 K beside the decoding's thousand; by TMA gather, 52 cycles per four rows.)
+//
+// Roles: warp 0 issues the MMAs, warp 1 the TMA copies, two warps copy raw weight bytes with cp.async; 16 decoding
+// warps, lane = weight row (tensor-memory lane quarter = warp % 4); eight epilogue warps.
+// Tensor memory: columns 0..255 accumulators (two of 128 tokens or one of 256), 256..511 two A stages of 256 K.
+// All hand-offs are mbarriers with bounded waits.
+#pragma once
+
+constexpr int kGgBStages = 3, kGgAStages = 2, kGgMaxRawSlots = 6;
+constexpr int kGgRawWarps = 2, kGgDecodeWarps = 16, kGgEpiWarps = 8;
+constexpr int kGgFirstDecode = 2 + kGgRawWarps, kGgFirstEpi = kGgFirstDecode + kGgDecodeWarps;
+constexpr int kGgThreads = (kGgFirstEpi + kGgEpiWarps) * 32;
+constexpr int kGgABase = 256;  // first tensor-memory column of the A slots
+constexpr int kGgBox = 32;     // token (h) rows per TMA box
+
+struct GgBars {
+  uint64_t b_full[kGgBStages], b_empty[kGgBStages];
+  uint64_t a_full[kGgAStages], a_empty[kGgAStages];
+  uint64_t raw_full[kGgMaxRawSlots], raw_empty[kGgMaxRawSlots];
+  uint64_t acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  int abort;
+};
+
+// Raw bytes of a round (256 weights) of one row in shared memory. IQ3_S: the 28 words that cover the 110-byte block,
+// 29 words apart (an odd number: 32 lanes reading the same word of 32 rows meet 32 banks). IQ4_NL: 144 bytes,
+// back to back (16-byte reads of eight neighbouring rows cover all banks).
+static __constant__ int8_t c_iq4nl_levels[16] = {FB_IQ4NL_LEVELS};
+
+template <int FMT>
+struct GgRaw;
+template <>
+struct GgRaw<FB_FMT_IQ3_S> {
+  static constexpr int kPiece = 110, kPitch = 116, kSlots = 6;
+};
+template <>
+struct GgRaw<FB_FMT_IQ4_NL> {
+  static constexpr int kPiece = 144, kPitch = 144, kSlots = 5;
+};
+// IQ3_S selectors, 16 bits per index and lane: entry i of lane l at byte 64 i + 2 l. Two lanes share a bank, so a
+// warp's look-up takes two passes at most where one shared copy takes three to four.
+// IQ4_NL level pairs, entry b of lane l at byte 128 b + 4 l.
+template <int FMT>
+constexpr int kGgTableBytes = FMT == FB_FMT_IQ3_S ? 512 * 64 : 256 * 128;
+template <int FMT>
+constexpr int gg_smem() {
+  return 1024 + kGgBStages * kTileB + GgRaw<FMT>::kSlots * kTileM * GgRaw<FMT>::kPitch + kGgTableBytes<FMT> +
+         int(sizeof(GgBars)) + 64;
+}
+static_assert(gg_smem<FB_FMT_IQ3_S>() <= 232448 && gg_smem<FB_FMT_IQ4_NL>() <= 232448, "shared memory per block");
+
+__device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// ------------------------------------------------------------------------------ tensor memory
+// D[tmem] (+)= A[tmem] * B[smem], bf16 operands, 16 K.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiK128)
+      : "memory");
+}
+// True in one lane of a converged warp. Code behind it is known to run in one thread, so the operands of
+// tcgen05.mma go to uniform registers directly: 8 cycles per instruction of 16 columns on an idle SM against 52 behind
+// a `lane == 0` branch (and 130 to 150 in the running kernel).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// ------------------------------------------------------------------------------ decoding
+// IQ3_S, one sub-block (32 weights). A weight is db * g * sign with g one of the 8 odd magnitudes 1..15, so the 8
+// possible bf16 values of the sub-block are computed once (db * (2k+1) is exact in fp32, then rounded like the
+// reference rounds) and kept as two byte planes in four registers; the codebook table holds, per 9-bit index, the
+// four 3-bit magnitude numbers as PRMT selector nibbles, so one PRMT per plane picks four weights, one XOR flips
+// their signs (bit 7 of the high bytes; rounding is sign-symmetric) and two PRMTs interleave the planes into bf16
+// pairs. B = the sub-block's eight ninth index bits, lane_pat = 2 * lane in both halves of the word.
+__device__ __forceinline__ void gg_decode_iq3s(float db, uint32_t qs_lo, uint32_t qs_hi, uint32_t B, uint32_t sg,
+                                               uint32_t sel_base, uint32_t lane_pat, uint32_t (&out)[16]) {
+  const float db2 = db + db;
+  float pv[8];
+  pv[0] = db;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) pv[k] = fmaf(float(2 * k), db, db);  // exact: (2k+1) * db has at most 20 significant bits
+  (void)db2;
+  const uint32_t t01 = pack_bf16(pv[0], pv[1]), t23 = pack_bf16(pv[2], pv[3]);
+  const uint32_t t45 = pack_bf16(pv[4], pv[5]), t67 = pack_bf16(pv[6], pv[7]);
+  const uint32_t lo_a = prmt(t01, t23, 0x6420u), hi_a = prmt(t01, t23, 0x7531u);
+  const uint32_t lo_b = prmt(t45, t67, 0x6420u), hi_b = prmt(t45, t67, 0x7531u);
+  // Table byte offsets (64 * index + 2 * lane) of two look-ups per word: qs byte in bits 6..13 (22..29), the ninth
+  // index bit, taken from B by a multiply that lands it on bit 14 (30).
+  constexpr uint32_t kM = 0x3FC03FC0u, kM2 = 0x40004000u;
+  uint32_t a[4];
+  a[0] = (((qs_lo << 6) & kM) | lane_pat) | ((B * 0x10004000u) & kM2);  // look-ups 0, 2
+  a[1] = (((qs_lo >> 2) & kM) | lane_pat) | ((B * 0x08002000u) & kM2);  // look-ups 1, 3
+  a[2] = (((qs_hi << 6) & kM) | lane_pat) | ((B * 0x01000400u) & kM2);  // look-ups 4, 6
+  a[3] = (((qs_hi >> 2) & kM) | lane_pat) | ((B * 0x00800200u) & kM2);  // look-ups 5, 7
+  const uint32_t s_even = sg & 0x0F0F0F0Fu, s_odd = (sg >> 4) & 0x0F0F0F0Fu;
+#pragma unroll
+  for (int l = 0; l < 8; ++l) {
+    const uint32_t aw = a[2 * (l >> 2) + (l & 1)];
+    const uint32_t off = (l & 2) ? (aw >> 16) : (aw & 0xFFFFu);
+    const uint32_t sel = lds_u16<0>(sel_base + off);
+    const uint32_t nib = prmt((l & 1) ? s_odd : s_even, 0u, 0x4440u | uint32_t(l >> 1));
+    const uint32_t sx = nib * 0x10204080u;  // sign bit j -> bit 7 of byte j
+    const uint32_t lo4 = prmt(lo_a, lo_b, sel);
+    const uint32_t hi4 = prmt(hi_a, hi_b, sel) ^ (sx & 0x80808080u);
+    out[2 * l] = prmt(lo4, hi4, 0x5140u);
+    out[2 * l + 1] = prmt(lo4, hi4, 0x7362u);
+  }
+}
+
+// IQ4_NL, one block (32 weights) from its scale and 16 code bytes. A byte holds the codes of elements i and i + 16; a
+// table in shared memory (one copy per lane: a look-up takes one pass) gives both levels as a bf16 pair (exact:
+// |level| <= 127), which widen to fp32 by a shift and a mask; d * level is exact in fp32 (19 significant bits) and
+// rounded once to bf16. Two operations of the half-rate integer pipe per weight; looking the levels up by byte-permutes
+// and converting them through the mantissa took 3.5.
+__device__ __forceinline__ void gg_decode_iq4nl(float d, const uint32_t (&q)[4], uint32_t pair_base, uint32_t lane_pat,
+                                                uint32_t (&out)[16]) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    // byte offsets 128 * code byte + 4 * lane of two look-ups per word
+    const uint32_t a02 = ((q[m] * 128u) & 0x7F807F80u) | lane_pat, a13 = ((q[m] >> 1) & 0x7F807F80u) | lane_pat;
+    float lo[4], hi[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const uint32_t a = (b & 1) ? a13 : a02;
+      const uint32_t v = lds_u32<0>(pair_base + ((b & 2) ? a >> 16 : a & 0xFFFFu));
+      lo[b] = __fmul_rn(d, __uint_as_float(v * 65536u));
+      hi[b] = __fmul_rn(d, __uint_as_float(v & 0xFFFF0000u));
+    }
+    out[2 * m] = pack_bf16(lo[0], lo[1]);
+    out[2 * m + 1] = pack_bf16(lo[2], lo[3]);
+    out[8 + 2 * m] = pack_bf16(hi[0], hi[1]);
+    out[8 + 2 * m + 1] = pack_bf16(hi[2], hi[3]);
+  }
+}
+
+// The raw words of one warp step (64 weights of the lane's row), in registers, and their decoding half by half.
+struct GgDecodeConst {
+  uint32_t table, lane_pat;  // window address of the format's table, this lane's address bits in it
+};
+template <int FMT>
+struct GgStep;
+template <>
+struct GgStep<FB_FMT_IQ3_S> {
+  uint32_t qs[4], sg[2], qh, sc;
+  float d;
+  // `row` = the row's words of the round, `shift` = 2 if the block starts in the middle of the first word, pos = K step.
+  // The 27 words behind the scale then lie on word boundaries (shift 2) or two bytes off (shift 0).
+  __device__ __forceinline__ void load(uint32_t row, int shift, int pos) {
+    const uint32_t blk = row + shift, p = row + 2 * shift, sh = shift ? 0u : 16u;
+    const uint32_t pq = p + 16 * pos, ps = p + 8 * pos;
+    d = __half2float(__ushort_as_half(static_cast<unsigned short>(lds_u16<0>(blk))));
+    qh = lds_u16<66>(blk + 2 * pos);
+    sc = lds_u8(blk + 106 + pos);
+    const uint32_t w0 = lds_u32<0>(pq), w1 = lds_u32<4>(pq), w2 = lds_u32<8>(pq), w3 = lds_u32<12>(pq), w4 = lds_u32<16>(pq);
+    const uint32_t g0 = lds_u32<72>(ps), g1 = lds_u32<76>(ps), g2 = lds_u32<80>(ps);
+    qs[0] = __funnelshift_r(w0, w1, sh);
+    qs[1] = __funnelshift_r(w1, w2, sh);
+    qs[2] = __funnelshift_r(w2, w3, sh);
+    qs[3] = __funnelshift_r(w3, w4, sh);
+    sg[0] = __funnelshift_r(g0, g1, sh);
+    sg[1] = __funnelshift_r(g1, g2, sh);
+  }
+  template <int HALF>
+  __device__ __forceinline__ void decode(const GgDecodeConst& c, uint32_t (&out)[16]) const {
+    // multiplier 2 s + 1 as a float through the mantissa of 2^23
+    const float m = __uint_as_float(0x4B000001u | ((HALF ? sc >> 4 : sc & 15u) << 1)) - 8388608.0f;
+    gg_decode_iq3s(__fmul_rn(d, m), qs[2 * HALF], qs[2 * HALF + 1], HALF ? qh >> 8 : qh & 0xFFu, sg[HALF], c.table,
+                   c.lane_pat, out);
+  }
+};
+template <>
+struct GgStep<FB_FMT_IQ4_NL> {
+  uint32_t w[9];  // two 18-byte blocks
+  __device__ __forceinline__ void load(uint32_t row, int, int pos) {
+    const uint32_t b = row + 36 * pos;
+    w[0] = lds_u32<0>(b); w[1] = lds_u32<4>(b); w[2] = lds_u32<8>(b); w[3] = lds_u32<12>(b); w[4] = lds_u32<16>(b);
+    w[5] = lds_u32<20>(b); w[6] = lds_u32<24>(b); w[7] = lds_u32<28>(b); w[8] = lds_u32<32>(b);
+  }
+  template <int HALF>
+  __device__ __forceinline__ void decode(const GgDecodeConst& c, uint32_t (&out)[16]) const {
+    if constexpr (HALF == 0) {
+      const uint32_t q[4] = {__funnelshift_r(w[0], w[1], 16), __funnelshift_r(w[1], w[2], 16),
+                             __funnelshift_r(w[2], w[3], 16), __funnelshift_r(w[3], w[4], 16)};
+      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[0] & 0xFFFFu))), q, c.table, c.lane_pat, out);
+    } else {
+      const uint32_t q[4] = {w[5], w[6], w[7], w[8]};
+      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[4] >> 16))), q, c.table, c.lane_pat, out);
+    }
+  }
+};
+
+// ------------------------------------------------------------------------------ raw bytes into shared memory
+// One loader warp copies the pieces of 32 rows (`bytes` of each) into its part of a raw slot. row_at(r) = address of
+// the piece of row r (IQ3_S: of the word that holds its first byte). Copy size: the largest the alignment allows; pieces two bytes off word alignment (an expert
+// table may hold any even address) go through registers. Returns true if the copies are asynchronous.
+template <int B, class RowF>
+__device__ __forceinline__ void gg_copy_pieces(uint32_t dst, int pitch, int bytes, int lane, RowF row_at) {
+  const int per_row = bytes / B;
+  for (int id = lane; id < 32 * per_row; id += 32) {
+    const int r = id / per_row, c = id - r * per_row;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + r * pitch + c * B), "l"(row_at(r) + c * B), "n"(B)
+                 : "memory");
+  }
+}
+template <int FMT, class RowF>
+__device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t align, int lane, const uint8_t* base,
+                                            const int (&piece)[9], uint32_t short_mask, RowF row_at) {
+  if constexpr (FMT == FB_FMT_IQ3_S) {
+    // 28 words from the word that holds the block's first byte (never one that starts behind the matrix)
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      if (lane < 28)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + r * GgRaw<FMT>::kPitch + 4 * lane),
+                     "l"(row_at(r) + 4 * lane)
+                     : "memory");
+    }
+    return true;
+  } else {
+    constexpr int P = GgRaw<FMT>::kPitch;
+    if ((align & 15u) == 0 && bytes == P) {
+      // 16-byte pieces, nine per row: piece id -> shared-memory byte 16 id. `piece[i]` = where this lane's i-th piece
+      // lies from the first row's, the same for every round: recomputing it made the two loader warps, which get an
+      // issue slot every eight cycles or so, the pace of the kernel (2400 cycles per round).
+#pragma unroll
+      for (int i = 0; i < 9; ++i)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * lane + 512 * i), "l"(base + piece[i]) : "memory");
+    } else if ((align & 15u) == 8) {
+      // rows of 360 bytes: 8-byte pieces, eighteen per row, sixteen rows per nine instructions; a short last round
+      // keeps the first nine of each row
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const uint8_t* b = hf ? row_at(16) : base;
+#pragma unroll
+        for (int i = 0; i < 9; ++i)
+          if (bytes == P || ((short_mask >> i) & 1u))
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8 * lane + 256 * i + 16 * P * hf),
+                         "l"(b + piece[i]) : "memory");
+      }
+    } else if ((align & 7u) == 0) {
+      gg_copy_pieces<8>(dst, P, bytes, lane, row_at);
+    } else if ((align & 3u) == 0) {
+      gg_copy_pieces<4>(dst, P, bytes, lane, row_at);
+    } else {
+      const int per_row = bytes / 4;
+      for (int id = lane; id < 32 * per_row; id += 32) {
+        const int r = id / per_row, c = id - r * per_row;
+        const unsigned short* p = reinterpret_cast<const unsigned short*>(row_at(r) + 4 * c);
+        sts_u32<0>(dst + r * P + 4 * c, uint32_t(p[0]) | (uint32_t(p[1]) << 16));
+      }
+      return false;
+    }
+    return true;
+  }
+}
+
+// A stage of the token ring holds this many 64-wide K steps: 256 / n rounded down to 1, 2 or 4. A unit of few tokens
+// then takes one hand-off per 256 K instead of four: a wait costs the MMA thread a few hundred cycles, as much as a
+// whole K step of such a unit.
+__device__ __forceinline__ int gg_b_steps(int n) { return n <= 64 ? 4 : n <= 128 ? 2 : 1; }
+
+struct GgArgs {
+  fb_moe_expert_layout L;
+  const uint8_t* const* expert_blob;  // [512] blob addresses, or nullptr: slots + e * blob_stride
+  const int4* tiles;                  // token tiles {expert, 0, first pair, tokens}
+  const int32_t* n_units;             // 128-row units: tiles x (rows / 128)
+  const int32_t* pair_token;
+  __nv_bfloat16* h;                   // gate/up: output rows, one per pair
+  const float* pair_weight;           // down
+  float* yp;                          // down: output rows, one per pair
+  unsigned long long* y_fixed;        // down: fixed-point sums instead, one row per token
+  uint32_t* status;
+};
+
+template <int FMT, bool DOWN>
+__global__ void __launch_bounds__(kGgThreads, 1)
+grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
+  using R = GgRaw<FMT>;
+  constexpr bool kIq3s = FMT == FB_FMT_IQ3_S;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ringb = smem;
+  uint8_t* rawb = smem + kGgBStages * kTileB;
+  uint8_t* table = rawb + R::kSlots * kTileM * R::kPitch;
+  GgBars* bars = reinterpret_cast<GgBars*>(table + kGgTableBytes<FMT>);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int I = A.L.inter;
+  const int k_steps = (DOWN ? I : H) / kBK, rounds = (k_steps + 3) / 4;
+  // gate/up: 128 intermediate rows are two units here, of 64 gate and 64 up rows each
+  const int n_units = DOWN ? *A.n_units : 2 * *A.n_units;
+  // (IQ3_S down comes at intermediate 512 only: its row length is a constant of the copies' addresses)
+  const int row_bytes = kIq3s ? (DOWN ? 512 : H) / 256 * 110 : (DOWN ? I : H) / 32 * 18;
+  const Abort ab{&bars->abort, A.status};
+
+  if constexpr (kIq3s) {
+    for (int i = tid; i < 512 * 4; i += kGgThreads) {  // 16 bytes = eight lanes' copies of an entry
+      const uint32_t p = c_iq3s_grid_packed[i >> 2];
+      const uint32_t e = (p & 7u) | (((p >> 3) & 7u) << 4) | (((p >> 6) & 7u) << 8) | (((p >> 9) & 7u) << 12);
+      const uint32_t w = e * 0x00010001u;
+      reinterpret_cast<uint4*>(table)[i] = make_uint4(w, w, w, w);
+    }
+  } else {
+    for (int i = tid; i < 256 * 8; i += kGgThreads) {  // 16 bytes = four lanes' copies of an entry
+      const uint32_t w = pack_bf16(float(c_iq4nl_levels[(i >> 3) & 15]), float(c_iq4nl_levels[i >> 7]));
+      reinterpret_cast<uint4*>(table)[i] = make_uint4(w, w, w, w);
+    }
+  }
+  if (tid == 0) {
+    for (int i = 0; i < kGgBStages; ++i) {
+      mbar_init(&bars->b_full[i], 1);
+      mbar_init(&bars->b_empty[i], 1);
+    }
+    for (int i = 0; i < kGgAStages; ++i) {
+      mbar_init(&bars->a_full[i], 8);  // two warps per lane quarter
+      mbar_init(&bars->a_empty[i], 1);
+    }
+    for (int i = 0; i < R::kSlots; ++i) {
+      mbar_init(&bars->raw_full[i], 32 * kGgRawWarps);
+      mbar_init(&bars->raw_empty[i], 8);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->acc_full[i], 1);
+      mbar_init(&bars->acc_empty[i], kGgEpiWarps);
+    }
+    bars->abort = 0;
+    mbar_fence_init();
+  }
+  if (warp == 0) tmem_alloc(&bars->tmem_base, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  auto unit_at = [&](int u) -> int4 {  // {expert, first weight row, first pair, tokens}
+    const int per_tile = DOWN ? H / kTileM : I / 64, tile = DOWN ? u / (H / kTileM) : I == 512 ? u / 8 : u / 10;
+    int4 un = A.tiles[tile];
+    un.y = (u - tile * per_tile) * (DOWN ? kTileM : 64);
+    return un;
+  };
+  // every role reads its unit one ahead of its use
+  auto unit_or_none = [&](int u) -> int4 { return u < n_units ? unit_at(u) : make_int4(0, 0, 0, 0); };
+  auto blob_of = [&](int e) -> const uint8_t* {
+    return A.expert_blob ? A.expert_blob[e] : A.L.slots + int64_t(e) * A.L.blob_stride;
+  };
+
+  if (warp == 0) {
+    // ---------------- MMA issuer. A unit of at most 128 tokens takes one of two 128-column accumulators, so its
+    // epilogue overlaps the next unit's K loop; a wider unit takes both.
+    if (elect_one()) {
+      const uint32_t ring_lo = umma_desc_lo_k128(smem_u32(ringb));
+      uint32_t ra = 0, sbc = 0, use0 = 0, use1 = 0, nb = 0;
+      int tokens = unit_or_none(blockIdx.x).w;
+      for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+        const int n = (tokens + 15) & ~15;
+        tokens = unit_or_none(u + gridDim.x).w;
+        const bool wide = n > 128;
+        const uint32_t idesc = idesc_bf16(n);
+        bool ok = true;
+        if (wide || nb == 0) ok = ab.wait(&bars->acc_empty[0], (use0 & 1) ^ 1);
+        if (ok && (wide || nb == 1)) ok = ab.wait(&bars->acc_empty[1], (use1 & 1) ^ 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t dcol = tmem_base + (wide ? 0u : nb * 128u);
+        const int S = gg_b_steps(n);
+        const uint32_t b_step = (kTileB >> 4) / S;  // descriptor distance of a stage's K steps
+        for (int rd = 0; rd < rounds; ++rd, ++ra) {
+          const uint32_t sa = ra % kGgAStages;
+          if (!(ok = ab.wait(&bars->a_full[sa], (ra / kGgAStages) & 1))) break;
+          const int steps = min(4, k_steps - 4 * rd);
+          uint32_t la = tmem_base + kGgABase + sa * 128;
+          for (int k0 = 0; k0 < steps; k0 += S, ++sbc) {
+            const uint32_t sb = sbc % kGgBStages;
+            if (!(ok = ab.wait(&bars->b_full[sb], (sbc / kGgBStages) & 1))) break;
+            tc_fence_after();
+            uint32_t lb = ring_lo + sb * (kTileB >> 4);
+            for (int k = k0; k < min(k0 + S, steps); ++k, la += 32, lb += b_step) {
+              umma_bf16_ts(dcol, la, lb, idesc, (rd | k) ? 1u : 0u);
+#pragma unroll
+              for (int k4 = 1; k4 < 4; ++k4) umma_bf16_ts(dcol, la + 8 * k4, lb + 2 * k4, idesc, 1u);
+            }
+            umma_commit(&bars->b_empty[sb]);
+          }
+          if (!ok) break;
+          umma_commit(&bars->a_empty[sa]);
+        }
+        if (!ok) break;
+        if (wide || nb == 0) { umma_commit(&bars->acc_full[0]); ++use0; }
+        if (wide || nb == 1) { umma_commit(&bars->acc_full[1]); ++use1; }
+        if (!wide) nb ^= 1u;
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- token (h) rows of the unit's pairs: boxes of 32 rows by TMA (one thread)
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      int4 un = unit_or_none(blockIdx.x), un_next;
+      for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, un = un_next) {
+        un_next = unit_or_none(u + gridDim.x);
+        const int boxes = (un.w + kGgBox - 1) / kGgBox;
+        const int S = gg_b_steps((un.w + 15) & ~15);
+        for (int k0 = 0; k0 < k_steps; k0 += S, ++it) {
+          const uint32_t s = it % kGgBStages;
+          if (!(ok = ab.wait(&bars->b_empty[s], ((it / kGgBStages) & 1) ^ 1))) break;
+          const int k1 = min(k0 + S, k_steps);
+          mbar_expect_tx(&bars->b_full[s], uint32_t((k1 - k0) * boxes) * (kGgBox * 128));
+          for (int k = k0; k < k1; ++k)
+            for (int b = 0; b < boxes; ++b)
+              tma_load_2d(ringb + s * kTileB + (k - k0) * (kTileB / S) + b * (kGgBox * 128), &map_b, k * kBK,
+                          un.z + b * kGgBox, &bars->b_full[s]);
+        }
+      }
+    }
+  } else if (warp < kGgFirstDecode) {
+    // ---------------- raw weight bytes, up to three rounds ahead of the decoding; a warp copies 64 of the 128 rows
+    constexpr int kRows = kTileM / kGgRawWarps;
+    const int row0 = kRows * (warp - 2);
+    int piece[9] = {};  // IQ4_NL, see gg_load_raw
+    uint32_t short_mask = 0;
+    if constexpr (!kIq3s) {
+      const int per_row = row_bytes % 16 == 0 ? 9 : 18, bytes = 144 / per_row;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const int id = lane + 32 * i, r = id / per_row, c = id - per_row * r;
+        piece[i] = bytes * c + (DOWN ? r * row_bytes : (r >> 1) * row_bytes + ((r & 1) ? int(A.L.up_offset - A.L.gate_offset) : 0));
+        short_mask |= (c < 9 ? 1u : 0u) << i;
+      }
+    }
+    uint32_t rcount = 0;
+    int4 un = unit_or_none(blockIdx.x), un_next;
+    bool ok = true;
+    for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, un = un_next) {
+      un_next = unit_or_none(u + gridDim.x);
+      const uint8_t* blob = blob_of(un.x);
+      const uint8_t* rg = DOWN ? blob + A.L.down_offset + size_t(un.y + row0) * row_bytes  // first gate (down) row
+                               : blob + A.L.gate_offset + size_t(un.y + row0 / 2) * row_bytes;
+      const uint8_t* rup = DOWN ? rg : blob + A.L.up_offset + size_t(un.y + row0 / 2) * row_bytes;  // first up row
+      for (int rd = 0; rd < rounds; ++rd, ++rcount) {
+        const uint32_t s = rcount % R::kSlots;
+        if (!(ok = ab.wait_warp(&bars->raw_empty[s], ((rcount / R::kSlots) & 1) ^ 1))) break;
+        const int off = rd * R::kPiece;
+        const int bytes = min(R::kPitch, row_bytes - off);
+        const uint8_t *pg = rg + off, *pu = rup + off;
+        uint32_t align = uint32_t(reinterpret_cast<uintptr_t>(pg) | reinterpret_cast<uintptr_t>(pu)) | uint32_t(row_bytes);
+        if constexpr (kIq3s) {
+          pg -= reinterpret_cast<uintptr_t>(pg) & 3;
+          pu -= reinterpret_cast<uintptr_t>(pu) & 3;
+        }
+        bool async = true;
+        for (int hf = 0; hf < kRows / 32; ++hf) {
+          const uint32_t dst = smem_u32(rawb) + (s * kTileM + row0 + 32 * hf) * R::kPitch;
+          if constexpr (DOWN) {
+            const uint8_t* p = pg + size_t(32 * hf) * row_bytes;
+            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece, short_mask, [&](int r) { return p + r * row_bytes; });
+          } else {
+            const uint8_t *p = pg + 16 * hf * row_bytes, *p2 = pu + 16 * hf * row_bytes;
+            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece, short_mask,
+                                     [&](int r) { return ((r & 1) ? p2 : p) + (r >> 1) * row_bytes; });
+          }
+        }
+        if (async) cp_async_arrive_noinc(&bars->raw_full[s]);
+        else mbar_arrive(&bars->raw_full[s]);
+      }
+    }
+    cp_async_wait_all();
+  } else if (warp < kGgFirstEpi) {
+    // ---------------- decoding warps: lane = row 32 q + lane. Two groups of eight warps take alternate rounds of 256 K
+    // and own one A stage each: while one group waits (raw bytes, its stage, its tensor-memory stores) the other one
+    // decodes. In a group, a quarter's two warps take 128 K each. (Sixteen warps on every round ran in phase and waited
+    // in phase; four groups on 128 K each double the hand-offs of the MMA thread, which then paces the kernel.)
+    const int q = warp & 3, j = (warp - kGgFirstDecode) >> 2, grp = j >> 1;
+    const uint32_t raw_row = smem_u32(rawb) + (32 * q + lane) * R::kPitch;
+    const uint32_t ta = tmem_base + (uint32_t(32 * q) << 16) + kGgABase + grp * 128;
+    const GgDecodeConst dc{smem_u32(table), uint32_t(lane) * (kIq3s ? 0x00020002u : 0x00040004u)};
+    // bytes from the covering word to the first block of the lane's row (IQ3_S: 0 or 2; rows are multiples of 4 apart)
+    auto row_shift = [&](const int4& w) -> int {
+      if constexpr (!kIq3s) return 0;
+      const int64_t off = DOWN ? A.L.down_offset : (lane & 1) ? A.L.up_offset : A.L.gate_offset;
+      return int(reinterpret_cast<uintptr_t>(blob_of(w.x) + off)) & 3;
+    };
+    uint32_t r0 = 0;  // rounds before this unit
+    int4 un_next = unit_or_none(blockIdx.x);
+    for (int u = blockIdx.x; u < n_units; u += gridDim.x, r0 += rounds) {
+      const int shift0 = row_shift(un_next);
+      un_next = unit_or_none(u + gridDim.x);
+      bool ok = true;
+      for (int rd = (grp ^ int(r0)) & 1; rd < rounds; rd += 2) {
+        const uint32_t rc = r0 + rd, rs = rc % R::kSlots, pa = ((rc / kGgAStages) & 1) ^ 1;
+        const int m = (j ^ int(rc >> 1)) & 1;  // this warp's half of the round (a short round's only half changes hands)
+        const uint32_t row = raw_row + rs * (kTileM * R::kPitch), tcol = ta + m * 64;
+        const int shift = (shift0 + rd * R::kPiece) & 3;
+        if (!(ok = ab.wait_warp(&bars->raw_full[rs], (rc / R::kSlots) & 1))) break;
+        const bool mine = 4 * rd + 2 * m < k_steps;
+        GgStep<FMT> raw;
+        uint32_t out[16];
+        if (mine) {
+          raw.load(row, shift, 2 * m);
+          raw.template decode<0>(dc, out);
+        }
+        if (!(ok = ab.wait_warp(&bars->a_empty[grp], pa))) break;
+        tc_fence_after();
+        if (mine) {
+          tmem_st16(tcol, out);
+          raw.template decode<1>(dc, out);
+          tmem_st16(tcol + 16, out);
+          raw.load(row, shift, 2 * m + 1);
+          raw.template decode<0>(dc, out);
+          tmem_st16(tcol + 32, out);
+          raw.template decode<1>(dc, out);
+          tmem_st16(tcol + 48, out);
+          tmem_st_wait();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&bars->a_full[grp]);
+          mbar_arrive(&bars->raw_empty[rs]);
+        }
+      }
+      if (!ok) break;
+    }
+  } else {
+    // ---------------- epilogue: lane quarter = warp % 4, two warps per quarter take alternate chunks of 16 tokens
+    const int q = warp & 3, chunk0 = 16 * ((warp - kGgFirstEpi) >> 2);
+    uint32_t use0 = 0, use1 = 0, nb = 0;
+    int4 un = unit_or_none(blockIdx.x), un_next;
+    for (int u = blockIdx.x; u < n_units; u += gridDim.x, un = un_next) {
+      un_next = unit_or_none(u + gridDim.x);
+      const bool wide = ((un.w + 15) & ~15) > 128;
+      bool ok = true;
+      if (wide || nb == 0) ok = ab.wait_warp(&bars->acc_full[0], use0 & 1);
+      if (ok && (wide || nb == 1)) ok = ab.wait_warp(&bars->acc_full[1], use1 & 1);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t dcol = tmem_base + (uint32_t(32 * q) << 16) + (wide ? 0u : nb * 128u);
+      for (int c0 = chunk0; c0 < un.w; c0 += 4 * kGgEpiWarps) {
+        uint32_t r[16];
+        tmem_ld16(dcol + uint32_t(c0), r);
+        tmem_ld_wait();
+        if constexpr (!DOWN) {
+          // even lanes hold gate rows, odd lanes the matching up rows: an even lane finishes tokens 0..7 of the chunk,
+          // its neighbour tokens 8..15
+          const bool odd = (lane & 1) != 0;
+          const int j = un.y + 16 * q + (lane >> 1);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? r[i] : r[8 + i], 1);
+            const float gv = __uint_as_float(odd ? got : r[i]), uv = __uint_as_float(odd ? r[8 + i] : got);
+            const int t = c0 + i + (odd ? 8 : 0);
+            // silu(g) * u; fast exp and divide: their error (a few fp32 ulp) is far below the bf16 step of h
+            const float hv = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
+            if (t < un.w) A.h[size_t(un.z + t) * I + j] = __float2bfloat16_rn(hv);
+          }
+        } else {
+          const int n = un.y + 32 * q + lane;
+          if (A.y_fixed) {  // the reference's accumulation (src/kernels/moe/moe.h:186-192): y_fixed[token] += fixed(w * v)
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (c0 + i < un.w) {
+                const float v = A.pair_weight[un.z + c0 + i] * __uint_as_float(r[i]);
+                atomicAdd(A.y_fixed + size_t(A.pair_token[un.z + c0 + i]) * H + n,
+                          static_cast<unsigned long long>(__float2ll_rn(v * 4294967296.0f)));
+              }
+          } else {
+            // (an epilogue warp gets an issue slot every eight cycles or so: the weights come in one load and reach the
+            // lanes by shuffles, and whole chunks skip the bounds checks)
+            const float pw = c0 + (lane & 15) < un.w ? A.pair_weight[un.z + c0 + (lane & 15)] : 0.0f;
+            float* out = A.yp + size_t(un.z + c0) * H + n;
+            if (c0 + 16 <= un.w) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) out[i * H] = __shfl_sync(0xffffffffu, pw, i) * __uint_as_float(r[i]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float w = __shfl_sync(0xffffffffu, pw, i);
+                if (c0 + i < un.w) out[i * H] = w * __uint_as_float(r[i]);
+              }
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (wide || nb == 0) { if (lane == 0) mbar_arrive(&bars->acc_empty[0]); ++use0; }
+      if (wide || nb == 1) { if (lane == 0) mbar_arrive(&bars->acc_empty[1]); ++use1; }
+      if (!wide) nb ^= 1u;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// Token rows in pair order: xg[p] = x[pair_token[p]], one warp per row. The whole pass is memory traffic: 100 us for
+// 81,920 rows (x stays in the L2 cache, the rows are written once).
+__global__ void __launch_bounds__(256) gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pair_token,
+                                                          const int32_t* __restrict__ n_pairs, __nv_bfloat16* __restrict__ xg) {
+  const int n = *n_pairs, lane = threadIdx.x & 31;
+  for (int p = blockIdx.x * 8 + (threadIdx.x >> 5); p < n; p += gridDim.x * 8) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + size_t(pair_token[p]) * H);
+    uint4* dst = reinterpret_cast<uint4*>(xg + size_t(p) * H);
+    uint4 v[H / 256];
+#pragma unroll
+    for (int i = 0; i < H / 256; ++i) v[i] = __ldg(src + 32 * i + lane);
+#pragma unroll
+    for (int i = 0; i < H / 256; ++i) dst[32 * i + lane] = v[i];
+  }
+}

@@ -190,9 +190,9 @@ int32_t fb_moe_layer_decode_host(const void* router_w_bf16, const fb_moe_expert_
                                  float* logits_scratch, void* x_dev, float* y_dev, float* y_host, void* stream);
 
 /* ---------------------------------------------------------------- prefill (eager, T up to the workspace capacity)
- * MoePrefillWorkspace, src/kernels/moe/moe.h:167-184. Differences: the work list holds the units
- * of both grouped GEMMs ({expert, first weight row of a 128-row tile, first pair, tokens}, up to 256
- * tokens per unit) instead of 64-token tiles; the per-pair results go to `yp` (fp32, routing weight
+ * MoePrefillWorkspace, src/kernels/moe/moe.h:167-184. Differences: the work list holds the token
+ * tiles of both grouped GEMMs ({expert, 0, first pair, tokens}: up to 256 tokens for gate/up, 128 for down)
+ * instead of 64-token tiles; the per-pair results go to `yp` (fp32, routing weight
  * applied) and the combine adds a token's ten rows in ascending-expert order, which replaces the
  * reference's 64-bit fixed-point atomics (moe.h:186-192) as the mechanism that makes the prefill sum
  * independent of scheduling; `token_pair` maps (token, rank) to its pair. */
@@ -210,8 +210,8 @@ typedef struct fb_moe_prefill_workspace {
   int32_t* pair_token;    /* [capacity*10] pairs grouped by expert */
   float* pair_weight;     /* [capacity*10] */
   int32_t* token_pair;    /* [capacity][10] */
-  void* units_gate_up;    /* int4 [max_units_gate_up] */
-  void* units_down;       /* int4 [max_units_down] */
+  void* units_gate_up;    /* int4 token tiles, one per inter / 128 units */
+  void* units_down;       /* int4 token tiles, one per 2560 / 128 units */
   void* h;                /* bf16 [capacity*10 + 256][inter] */
   float* yp;              /* [capacity*10][2560] */
   uint32_t* status;       /* FB_STATUS_* */
