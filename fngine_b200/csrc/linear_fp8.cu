@@ -382,7 +382,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 
   if (warp == 0) {
     // ---------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int tile = blockIdx.x; tile < n_work; tile += gridDim.x) {
         const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
@@ -403,7 +403,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, tl = 0;
       for (int tile = blockIdx.x; tile < n_work; tile += gridDim.x, ++tl) {
         const int ab = tl & 1;
@@ -580,7 +580,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs): own token rows and own weight box, completion on the leader's barrier
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int tile = pair; tile < n_work; tile += n_pairs) {
         const int m_blk = tile % m_tiles, n_blk = tile / m_tiles;
@@ -600,7 +600,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       uint32_t it = 0, tl = 0;
       for (int tile = pair; tile < n_work; tile += n_pairs, ++tl) {
         const int ab = tl & 1;
@@ -1000,7 +1000,7 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer: 128 weight rows (two 64-row boxes) + the 48 piece rows per K block
-    if (lane == 0) {
+    if (elect_one()) {
       // The weight codes do not depend on the kernel launched just before (the activation split), so
       // the first ring's worth of them is requested before waiting for it: under programmatic
       // dependent launch this kernel is resident while the split still runs.
@@ -1040,7 +1040,7 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, seg = 0;
       bool ok = true;
       for (long long pos = begin; pos < end && ok; ++seg) {
