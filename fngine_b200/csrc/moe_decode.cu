@@ -6,12 +6,10 @@
 //   down     partial[pair][n] = w_pair * (down_n . q8(h[pair]))
 //   combine  y[t] = sum of token t's partials in slot order (+ shared, + residual write)
 //
-// gate_up and down of IQ3_S and IQ4_NL experts are one persistent kernel, one CTA per SM
-// (moe_decode_iq3s.cuh): a producer thread streams tiles of the expert blob into a three-stage
-// shared-memory ring with 1-D bulk async copies (TMA, no multicast) signalled through mbarriers;
-// consumer warps decode the blocks from shared memory and accumulate exact int8 dot products (dp4a).
-// (IQ4_NL down at intermediate 640 keeps an earlier two-stage kernel; the other formats have plain
-// kernels, moe_decode_generic.cuh.) Numerics are those of the
+// gate_up and down are one persistent kernel, one CTA per SM (moe_decode_experts.cuh): a producer thread streams
+// tiles of the expert blob into a three-stage shared-memory ring with 1-D bulk async copies (TMA, no multicast)
+// signalled through mbarriers; consumer warps decode the blocks from shared memory and accumulate exact int8 dot
+// products (dp4a). (A Q2_0 down projection has a plain kernel, moe_decode_generic.cuh.) Numerics are those of the
 // reference's CPU expert tier (src/cpu/iq_cpu.h:12-40 of the reference project): Q8_K activations
 // for IQ3_S weights, Q8_0 for IQ4_NL, integer sums per block, one fp32 scale step per block.
 #include "iq_decode.cuh"
@@ -67,10 +65,6 @@ __host__ __device__ constexpr int act_row_bytes_planar(int act, int k) {
 __host__ __device__ constexpr int act_of(int fmt) {
   return fmt == FB_FMT_IQ4_NL || fmt == FB_FMT_Q2_0 ? FB_ACT_Q8_0 : FB_ACT_Q8_K;
 }
-// gate/up formats without a streaming kernel (plain kernels in moe_decode_generic.cuh)
-__host__ __device__ constexpr bool plain_gate_up(int fmt) {
-  return fmt == FB_FMT_IQ3_XXS || fmt == FB_FMT_IQ2_S || fmt == FB_FMT_IQ4_XS;
-}
 // ws.xq holds [2][16][FB_XQ_STRIDE]: the Q8_K rows of the step's tokens, then their Q8_0 rows. A workspace
 // made for a layout gets the one its gate/up format needs; one made without a layout gets both from
 // the stand-alone selection (which does not see the layout).
@@ -79,7 +73,7 @@ __host__ __device__ constexpr size_t xq_offset(int act) { return act == FB_ACT_Q
 __device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + expf(-g)) * u; }
 
 // Planar Q8_K rows: codes [k] | block scales float [k/256] (64 bytes reserved) | code sums of every 32
-// codes, int16 [k/32] (Q8_K's bsums added in pairs; the IQ3_S kernels use them, see moe_decode_iq3s.cuh).
+// codes, int16 [k/32] (Q8_K's bsums added in pairs; the IQ3_S kernels use them, see moe_decode_experts.cuh).
 __host__ __device__ constexpr int q8k_asum_off(int k) { return k + 64; }
 
 // Stores block b of a planar Q8_K row from the calling warp's quantizer output (lane l holds codes
@@ -668,19 +662,6 @@ __global__ void __launch_bounds__(512) select_kernel(const float* __restrict__ l
       slot_of, T, ws, counts, false, true, true, s_work);
 }
 
-// The selection alone, from logits a route kernel stored (one block): for layers whose gate/up format has
-// only plain kernels, which read the device work list.
-__global__ void __launch_bounds__(512) select_only_kernel(SelectArgs sel, fb_moe_decode_workspace ws) {
-  pdl_launch_dependents();
-  pdl_wait_prior();
-  __shared__ WorkCache s_work;
-  select_block(
-      [&](int t, uint2* scratch, int* ids, float* wts) {
-        warp_topk10_pruned([&](int e) { return __ldcg(sel.logits + size_t(t) * sel.stride + e); }, scratch, ids, wts);
-      },
-      sel.slot_of, sel.tokens, ws, nullptr, sel.remote_ok != 0, true, false, s_work);
-}
-
 // What route_kernel needs for an expert-parallel step with peer-memory exchange (n_ranks == 0: none).
 struct EpRouteArgs {
   fb_ep_peers peers;
@@ -897,152 +878,6 @@ struct StageMeta {
   float wgt[kTT];  // routing weights of the pass's pairs (down)
 };
 
-struct Ring {
-  uint64_t* full;   // [2] count 1 + tx bytes
-  uint64_t* empty;  // [2]
-  volatile StageMeta* meta;  // [2]
-  volatile int* abort;
-};
-
-// After a wait has run out every later wait is skipped and all loops end at their next check, so
-// the kernel drains quickly with the status word set; nothing ever waits without a limit.
-__device__ __forceinline__ bool ring_aborted(const Ring& r) { return *r.abort != 0; }
-__device__ __forceinline__ void ring_timeout(const Ring& r, uint32_t* status) {
-  *r.abort = 1;
-  atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
-}
-
-__device__ __forceinline__ void ring_init(const Ring& r, int empty_count) {
-  mbar_init(&r.full[0], 1);
-  mbar_init(&r.full[1], 1);
-  mbar_init(&r.empty[0], empty_count);
-  mbar_init(&r.empty[1], empty_count);
-  r.meta[0].tile = -1;
-  r.meta[1].tile = -1;
-  *r.abort = 0;
-  mbar_fence_init();
-}
-
-// Producer loop of one CTA (one thread): draws tiles from `counter`, stages every pass of each
-// tile through issue(meta, slot), and finally posts the end marker in both slots.
-template <class IssueF>
-__device__ __forceinline__ void producer_loop(const Ring& r, const fb_moe_decode_workspace& ws, const WorkCache& wc,
-                                              int* counter, int n_tiles, int tiles_per_item, int rows_per_tile,
-                                              IssueF issue) {
-  int i = 0;
-  auto slot_free = [&](int s) -> bool {
-    if (ring_aborted(r)) return false;
-    if (i >= 2 && !mbar_wait(&r.empty[s], ((i >> 1) - 1) & 1)) {
-      ring_timeout(r, ws.status);
-      return false;
-    }
-    return true;
-  };
-  int next = int(blockIdx.x);  // a block's first tile needs no ticket; later ones are drawn one step ahead of their use
-  while (true) {
-    const int tile = next;
-    if (tile >= n_tiles) break;
-    next = int(gridDim.x) + atomicAdd(counter, 1);
-    const int pos = tile / tiles_per_item;
-    const int item = wc.order[pos];
-    const int sub = tile - pos * tiles_per_item;
-    const int pb = wc.pair_begin[item];
-    const int ntok = wc.pair_begin[item + 1] - pb;
-    const int slot_id = wc.slot[item];
-    for (int tok0 = 0; tok0 < ntok; tok0 += kTT, ++i) {
-      const int s = i & 1;
-      if (!slot_free(s)) return;
-      volatile StageMeta* m = &r.meta[s];
-      m->tile = tile;
-      m->pair0 = pb + tok0;
-      m->ntp = min(kTT, ntok - tok0);
-      m->row0 = sub * rows_per_tile;
-      m->item = item;
-      m->item_pair0 = pb;
-      m->item_tok = ntok;
-      for (int t = 0; t < kTT; ++t) m->wgt[t] = tok0 + t < ntok ? wc.pair_weight[pb + tok0 + t] : 0.0f;
-      issue(s, slot_id, sub, pb + tok0, min(kTT, ntok - tok0));
-    }
-  }
-  for (int e = 0; e < 2; ++e, ++i) {  // end marker in both slots: every waiting warp sees it
-    const int s = i & 1;
-    if (!slot_free(s)) return;
-    r.meta[s].tile = -1;
-    mbar_arrive(&r.full[s]);
-  }
-}
-
-// ------------------------------------------------------------------------------ per-format tile math
-// One 36-byte IQ4_NL unit (two blocks) against TT interleaved Q8_0 rows; ublk = index of the
-// unit's first block within the row.
-template <int TT>
-__device__ __forceinline__ void iq4nl_unit_dot(const uint32_t* unit, const Iq4nlLevels& L,
-                                               const uint8_t* const (&actrow)[TT], int ublk, int act_k,
-                                               float (&acc)[TT]) {
-  int w[8];
-  {
-    const uint32_t q[4] = {ld4<2>(unit), ld4<6>(unit), ld4<10>(unit), ld4<14>(unit)};
-    iq4nl_decode32(L, q, w);
-    const float d = ld_fp16<0>(unit);
-#pragma unroll
-    for (int t = 0; t < TT; ++t) {
-      const int s = dot32(w, reinterpret_cast<const int8_t*>(actrow[t]) + 32 * ublk);
-      acc[t] = fmaf(float(s), d * reinterpret_cast<const float*>(actrow[t] + act_k)[ublk], acc[t]);
-    }
-  }
-  {
-    const uint32_t q[4] = {unit[5], unit[6], unit[7], unit[8]};
-    iq4nl_decode32(L, q, w);
-    const float d = ld_fp16<18>(unit);
-#pragma unroll
-    for (int t = 0; t < TT; ++t) {
-      const int s = dot32(w, reinterpret_cast<const int8_t*>(actrow[t]) + 32 * (ublk + 1));
-      acc[t] = fmaf(float(s), d * reinterpret_cast<const float*>(actrow[t] + act_k)[ublk + 1], acc[t]);
-    }
-  }
-}
-
-// One IQ4_NL block (18 bytes at row + 18 b, two-byte aligned) against TT interleaved Q8_0 rows, for
-// the gate/up kernel where eight lanes share a row and lane q takes blocks q, q + 8, ...: the
-// block's parity, hence its alignment, is a lane constant (`odd`), so the five aligned words that
-// cover it are read directly and the four code words come out of one PRMT each. The eight lanes
-// read eight consecutive 32-byte activation blocks; lanes 4-7 (`swap`) take the two 16-byte halves in
-// the other order, which puts the eight 128-bit loads of an instruction in eight different bank
-// groups. Integer sums do not depend on that order.
-template <int TT>
-__device__ __forceinline__ void iq4nl_block_dot(const uint8_t* row, int b, bool odd, bool swap, const Iq4nlLevels& L,
-                                                const uint8_t* const (&actrow)[TT], int act_k, float (&acc)[TT]) {
-  const uint32_t* u = reinterpret_cast<const uint32_t*>(row + 18 * b - (odd ? 2 : 0));
-  const uint32_t u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3], u4 = u[4];
-  const uint32_t sel = odd ? 0x7654u : 0x5432u;
-  const uint32_t q[4] = {__byte_perm(u0, u1, sel), __byte_perm(u1, u2, sel), __byte_perm(u2, u3, sel),
-                         __byte_perm(u3, u4, sel)};
-  const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(odd ? (u0 >> 16) : (u0 & 0xFFFFu))));
-  int w[8];
-  iq4nl_decode32(L, q, w);
-  int wa[4], wb[4];  // weights of the half read first / second
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    wa[i] = swap ? w[4 + i] : w[i];
-    wb[i] = swap ? w[i] : w[4 + i];
-  }
-  const int off_a = 32 * b + (swap ? 16 : 0), off_b = 32 * b + (swap ? 0 : 16);
-#pragma unroll
-  for (int t = 0; t < TT; ++t) {
-    const int4 a = *reinterpret_cast<const int4*>(actrow[t] + off_a);
-    const int4 c = *reinterpret_cast<const int4*>(actrow[t] + off_b);
-    int sum = __dp4a(wa[0], a.x, 0);
-    sum = __dp4a(wa[1], a.y, sum);
-    sum = __dp4a(wa[2], a.z, sum);
-    sum = __dp4a(wa[3], a.w, sum);
-    sum = __dp4a(wb[0], c.x, sum);
-    sum = __dp4a(wb[1], c.y, sum);
-    sum = __dp4a(wb[2], c.z, sum);
-    sum = __dp4a(wb[3], c.w, sum);
-    acc[t] = fmaf(float(sum), d * reinterpret_cast<const float*>(actrow[t] + act_k)[b], acc[t]);
-  }
-}
-
 // h of one finished work item -> planar activation rows for the down projection (one warp).
 __device__ __forceinline__ void quantize_item_h(const fb_moe_decode_workspace& ws, int pair_begin, int n_tok,
                                                 int down_act, int I) {
@@ -1101,162 +936,9 @@ __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_works
   }
 }
 
-// Consumer side of the task scheme: draws the next (entry, task) ticket; returns false at the end.
-// seq = entry number of this CTA, s = its ring slot.
-template <int TASKS>
-__device__ __forceinline__ bool draw_task(const Ring& r, int* ticket_ctr, uint32_t* status, int lane, int& s,
-                                          int& task) {
-  int ticket = 0;
-  if (lane == 0) ticket = atomicAdd(ticket_ctr, 1);
-  ticket = __shfl_sync(0xffffffffu, ticket, 0);
-  const int seq = ticket / TASKS;
-  task = ticket - seq * TASKS;
-  s = seq & 1;
-  if (ring_aborted(r)) return false;
-  if (!mbar_wait(&r.full[s], (seq >> 1) & 1)) {
-    ring_timeout(r, status);
-    return false;
-  }
-  return r.meta[s].tile >= 0;
-}
-
-// ------------------------------------------------------------------------------ down kernel
-template <int FMT, int INTER>
-struct Down;
-// IQ4_NL, inter 512: a row is eight 36-byte units, eight lanes per row, four rows per warp step.
-template <>
-struct Down<FB_FMT_IQ4_NL, 512> {
-  static constexpr int kRows = 320, kRowBytes = 288, kWarps = 16, kTasks = 16, kAct = FB_ACT_Q8_0,
-                       kActBytes = 512 + 64;
-  static constexpr int kLanesPerRow = 8, kUnitsPerLane = 1, kUnitA = 1, kUnitB = 0;
-};
-// IQ4_NL, inter 640: a row is ten units, two lanes per row with five consecutive units each.
-template <>
-struct Down<FB_FMT_IQ4_NL, 640> {
-  static constexpr int kRows = 256, kRowBytes = 360, kWarps = 16, kTasks = 16, kAct = FB_ACT_Q8_0,
-                       kActBytes = 640 + 80;
-  static constexpr int kLanesPerRow = 2, kUnitsPerLane = 5, kUnitA = 5, kUnitB = 1;
-};
-
-template <int FMT, int INTER>
-__global__ void __launch_bounds__((Down<FMT, INTER>::kWarps + 1) * 32, 1)
-down_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws) {
-  using C = Down<FMT, INTER>;
-  constexpr int kW = C::kWarps, kStageW = C::kRows * C::kRowBytes;
-  constexpr int kStage = kStageW + kTT * C::kActBytes;
-  extern __shared__ __align__(128) uint8_t smem[];
-  uint8_t* p = smem;
-  uint8_t* stage0 = p;
-  p += 2 * kStage;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p);
-  __shared__ StageMeta s_meta[2];
-  __shared__ int s_misc[4];
-  __shared__ WorkCache s_work;
-  Ring ring{bars, bars + 2, s_meta, s_misc};
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    ring_init(ring, 1);  // one arrival frees a slot: the warp that finishes the entry's last task
-    s_misc[1] = 0;
-    s_misc[2] = 0;
-    s_misc[3] = 0;
-  }
-  __syncthreads();
-  pdl_launch_dependents();
-  pdl_wait_prior();
-
-  const fb_moe_decode_work* work = ws.work;
-  const int n_items = min(max(work->n_items, 0), kMaxPairs);
-  constexpr int tpi = H / C::kRows;
-  const int n_tiles = n_items * tpi;
-
-  if (warp == kW) {
-    work_cache_fill(ws, s_work, n_items);
-    __syncwarp();
-    if (lane == 0) {
-      producer_loop(ring, ws, s_work, ws.sched + kSchedDown, n_tiles, tpi, C::kRows,
-                    [&](int s, int slot_id, int sub, int pair0, int ntp) {
-                      const uint8_t* blob = L.slots + int64_t(slot_id) * L.blob_stride;
-                      uint8_t* st = stage0 + s * kStage;
-                      mbar_expect_tx(&ring.full[s], uint32_t(kStageW + ntp * C::kActBytes));
-                      bulk_g2s(st, blob + L.down_offset + size_t(sub) * kStageW, kStageW, &ring.full[s]);
-                      for (int t = 0; t < ntp; ++t)
-                        bulk_g2s(st + kStageW + t * C::kActBytes, ws.hq + size_t(pair0 + t) * FB_HQ_STRIDE,
-                                 C::kActBytes, &ring.full[s]);
-                    });
-    }
-    return;
-  }
-
-  {
-    const Iq4nlLevels lv = iq4nl_levels();
-    while (true) {  // sixteen tasks per tile, drawn from the ticket: task k takes row steps k, k + 16, ...
-      int s, task;
-      if (!draw_task<C::kTasks>(ring, &s_misc[1], ws.status, lane, s, task)) break;
-      const int ntp = ring.meta[s].ntp, pair0 = ring.meta[s].pair0, r0 = ring.meta[s].row0;
-      const float wgt[kTT] = {ring.meta[s].wgt[0], ring.meta[s].wgt[1]};
-      uint8_t* st = stage0 + s * kStage;
-      const uint8_t* actbase = st + kStageW;
-      constexpr int LPR = C::kLanesPerRow, RPS = 32 / LPR;
-      const int q = lane % LPR, r = lane / LPR;
-      for (int step = task; step < C::kRows / RPS; step += C::kTasks) {
-        const int row = step * RPS + r;
-        const uint8_t* rowp = st + row * C::kRowBytes;
-        float acc[kTT] = {0.0f, 0.0f};
-        if constexpr (INTER == 512) {
-          // eight lanes per row, lane q takes blocks q and q + 8 (conflict-free weight and activation reads)
-          const bool odd = (q & 1) != 0, swap = (q & 4) != 0;
-          if (ntp == 1) {
-            const uint8_t* ar[1] = {actbase};
-            float a1[1] = {0.0f};
-            iq4nl_block_dot<1>(rowp, q, odd, swap, lv, ar, INTER, a1);
-            iq4nl_block_dot<1>(rowp, q + 8, odd, swap, lv, ar, INTER, a1);
-            acc[0] = a1[0];
-          } else {
-            const uint8_t* ar[2] = {actbase, actbase + C::kActBytes};
-            iq4nl_block_dot<2>(rowp, q, odd, swap, lv, ar, INTER, acc);
-            iq4nl_block_dot<2>(rowp, q + 8, odd, swap, lv, ar, INTER, acc);
-          }
-        } else if (ntp == 1) {
-          const uint8_t* ar[1] = {actbase};
-          float a1[1] = {0.0f};
-#pragma unroll
-          for (int it = 0; it < C::kUnitsPerLane; ++it) {
-            const int u = q * C::kUnitA + it * C::kUnitB;
-            iq4nl_unit_dot<1>(reinterpret_cast<const uint32_t*>(rowp + 36 * u), lv, ar, 2 * u, INTER, a1);
-          }
-          acc[0] = a1[0];
-        } else {
-          const uint8_t* ar[2] = {actbase, actbase + C::kActBytes};
-#pragma unroll
-          for (int it = 0; it < C::kUnitsPerLane; ++it) {
-            const int u = q * C::kUnitA + it * C::kUnitB;
-            iq4nl_unit_dot<2>(reinterpret_cast<const uint32_t*>(rowp + 36 * u), lv, ar, 2 * u, INTER, acc);
-          }
-        }
-#pragma unroll
-        for (int t = 0; t < kTT; ++t) {
-          float v = acc[t];
-#pragma unroll
-          for (int o = 1; o < LPR; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (t < ntp && q == 0) ws.partial[size_t(pair0 + t) * H + r0 + row] = wgt[t] * v;
-        }
-      }
-      __syncwarp();
-      int done = 0;
-      if (lane == 0) done = atomicAdd(&s_misc[2 + s], 1);
-      done = __shfl_sync(0xffffffffu, done, 0);
-      if (done == C::kTasks - 1 && lane == 0) {
-        s_misc[2 + s] = 0;
-        mbar_arrive(&ring.empty[s]);
-      }
-    }
-  }
-}
-
-#include "moe_decode_iq3s.cuh"
 #define FB_MOE_DECODE_TU
 #include "moe_decode_generic.cuh"
+#include "moe_decode_experts.cuh"
 
 // ------------------------------------------------------------------------------ combine
 // y[t][n] = partials of token t in slot order (+ y_shared); optional rank-1 ablation of the routed
@@ -1362,19 +1044,14 @@ __global__ void __launch_bounds__(256) ep_combine_exchange_kernel(fb_moe_decode_
 }
 
 // ------------------------------------------------------------------------------ host side
-template <int FMT, int INTER>
-constexpr size_t down_smem() {
-  using C = Down<FMT, INTER>;
-  return 2 * size_t(C::kRows * C::kRowBytes + kTT * C::kActBytes) + 64;
-}
-
 bool layout_ok(const fb_moe_expert_layout* L) {
   if (!L || !L->slots) return false;
   if ((reinterpret_cast<uintptr_t>(L->slots) | uintptr_t(L->blob_stride) | uintptr_t(L->gate_offset) |
        uintptr_t(L->up_offset) | uintptr_t(L->down_offset)) & 15)
     return false;
   if (L->inter != 512 && L->inter != 640) return false;
-  if (L->gate_up_format != FB_FMT_IQ3_S && L->gate_up_format != FB_FMT_IQ4_NL && !plain_gate_up(L->gate_up_format))
+  if (L->gate_up_format != FB_FMT_IQ3_S && L->gate_up_format != FB_FMT_IQ4_NL &&
+      L->gate_up_format != FB_FMT_IQ3_XXS && L->gate_up_format != FB_FMT_IQ2_S && L->gate_up_format != FB_FMT_IQ4_XS)
     return false;
   if (L->down_format == FB_FMT_IQ3_S) return L->inter % 256 == 0;
   return L->down_format == FB_FMT_IQ4_NL || L->down_format == FB_FMT_Q2_0;
@@ -1395,22 +1072,44 @@ bool ws_ok(const fb_moe_decode_workspace* ws) {
   return ws && ws->work && ws->xq && ws->h && ws->hq && ws->partial && ws->item_done && ws->sched && ws->status;
 }
 
-// The streaming expert kernel of a format (IQ3_S or IQ4_NL) over the given phases.
-template <int FMT>
-int32_t launch_experts_fmt(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases,
-                           void* stream, const char* what, const SelectArgs* sel) {
-  using C = ExpertsCfg<FMT>;
+// The streaming expert kernel over the given phases; with `sel` it runs the selection itself.
+template <int GU, int DN, int INTER>
+int32_t launch_experts_as(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases,
+                          void* stream, const char* what, const SelectArgs* sel) {
+  using C = ExpertsCfg<GU, DN, INTER>;
   static PerDeviceOnce once;
-  const cudaError_t attr = per_device_once(once, [] { return opt_in_smem(experts_kernel<FMT>, C::kSmem); });
+  const cudaError_t attr = per_device_once(once, [] { return opt_in_smem(experts_kernel<GU, DN, INTER>, C::kSmem); });
   if (attr != cudaSuccess) {
     set_error("%s: shared-memory opt-in: %s", what, cudaGetErrorString(attr));
     return int32_t(attr);
   }
-  const cudaError_t e = launch_pdl(experts_kernel<FMT>, dim3(sm_count()), dim3((C::kWarps + 1) * 32), C::kSmem,
+  const cudaError_t e = launch_pdl(experts_kernel<GU, DN, INTER>, dim3(sm_count()), dim3((C::kWarps + 1) * 32), C::kSmem,
                                    as_stream(stream), *layout, *ws, sel ? (phases | kPhaseSelect) : phases,
                                    sel ? *sel : SelectArgs{});
   if (e != cudaSuccess) return check_launch(what);
   return 0;
+}
+// Every gate/up format has its kernel with an IQ4_NL down projection at both intermediate sizes; IQ3_S also with its own.
+template <int GU>
+int32_t launch_experts_gu(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases, void* stream,
+                          const char* what, const SelectArgs* sel) {
+  return layout->inter == 512 ? launch_experts_as<GU, FB_FMT_IQ4_NL, 512>(layout, ws, phases, stream, what, sel)
+                              : launch_experts_as<GU, FB_FMT_IQ4_NL, 640>(layout, ws, phases, stream, what, sel);
+}
+int32_t launch_phases(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases, void* stream,
+                      const char* what, const SelectArgs* sel) {
+  const bool dn_iq3s = layout->down_format == FB_FMT_IQ3_S;
+  // a down-only launch does not care for the gate/up format: IQ4_NL's kernel has no table to fill
+  const int gu = phases & kPhaseGateUp ? layout->gate_up_format : dn_iq3s ? FB_FMT_IQ3_S : FB_FMT_IQ4_NL;
+  switch (gu) {
+    case FB_FMT_IQ3_S:
+      if (dn_iq3s) return launch_experts_as<FB_FMT_IQ3_S, FB_FMT_IQ3_S, 512>(layout, ws, phases, stream, what, sel);
+      return launch_experts_gu<FB_FMT_IQ3_S>(layout, ws, phases, stream, what, sel);
+    case FB_FMT_IQ4_NL: return launch_experts_gu<FB_FMT_IQ4_NL>(layout, ws, phases, stream, what, sel);
+    case FB_FMT_IQ2_S: return launch_experts_gu<FB_FMT_IQ2_S>(layout, ws, phases, stream, what, sel);
+    case FB_FMT_IQ3_XXS: return launch_experts_gu<FB_FMT_IQ3_XXS>(layout, ws, phases, stream, what, sel);
+    default: return launch_experts_gu<FB_FMT_IQ4_XS>(layout, ws, phases, stream, what, sel);
+  }
 }
 
 }  // namespace
@@ -1508,34 +1207,10 @@ int32_t fb_moe_select_publish(const float* router_logits, int32_t logits_stride,
   return 0;
 }
 
-// The IQ3_S expert kernel: gate/up tiles, down tiles, or both in one launch (down needs inter 512).
-static int32_t launch_experts_iq3s(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases,
-                                   void* stream, const char* what, const SelectArgs* sel = nullptr) {
-  return launch_experts_fmt<FB_FMT_IQ3_S>(layout, ws, phases, stream, what, sel);
-}
-
 // `sel`: the kernel runs the selection itself (the fused layer call), else it reads the device work list.
 static int32_t launch_gate_up(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream,
                               const SelectArgs* sel) {
-  if (layout->gate_up_format == FB_FMT_IQ3_S)
-    return launch_experts_iq3s(layout, ws, kPhaseGateUp, stream, "hot_gate_up", sel);
-  if (plain_gate_up(layout->gate_up_format)) {  // plain kernels: they read the device work list (sel is not for them)
-    const dim3 pgrid(sm_count() * 8);
-    cudaError_t pe;
-    if (layout->gate_up_format == FB_FMT_IQ3_XXS)
-      pe = launch_pdl(gate_up_generic_kernel<FB_FMT_IQ3_XXS>, pgrid, dim3(256), 0, as_stream(stream), *layout, *ws);
-    else if (layout->gate_up_format == FB_FMT_IQ2_S)
-      pe = launch_pdl(gate_up_generic_kernel<FB_FMT_IQ2_S>, pgrid, dim3(256), 0, as_stream(stream), *layout, *ws);
-    else
-      pe = launch_pdl(gate_up_generic_kernel<FB_FMT_IQ4_XS>, pgrid, dim3(256), 0, as_stream(stream), *layout, *ws);
-    if (pe == cudaSuccess)  // the down projection wants h re-quantized: one warp per pair
-      pe = launch_pdl(requant_h_kernel, dim3(kMaxPairs / 8), dim3(256), 0, as_stream(stream), *layout, *ws);
-    if (pe != cudaSuccess) return check_launch("hot_gate_up");
-    return 0;
-  }
-  if (layout->gate_up_format == FB_FMT_IQ4_NL)
-    return launch_experts_fmt<FB_FMT_IQ4_NL>(layout, ws, kPhaseGateUp, stream, "hot_gate_up", sel);
-  return invalid("hot_gate_up: unsupported gate/up format");
+  return launch_phases(layout, ws, kPhaseGateUp, stream, "hot_gate_up", sel);
 }
 
 int32_t fb_moe_hot_gate_up(const fb_moe_expert_layout* layout, int32_t tokens, const fb_moe_decode_workspace* ws,
@@ -1548,17 +1223,14 @@ int32_t fb_moe_hot_gate_up(const fb_moe_expert_layout* layout, int32_t tokens, c
 
 static int32_t launch_down(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream);
 
-// Both projections of every routed expert: one launch for IQ3_S experts, a gate/up and a down launch otherwise.
+// Both projections of every routed expert: one launch, but for a down format without a shared streaming kernel.
 static int32_t launch_experts(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream,
                               const SelectArgs* sel) {
-  if (layout->gate_up_format == FB_FMT_IQ3_S && layout->down_format == FB_FMT_IQ3_S)
-    return launch_experts_iq3s(layout, ws, kPhaseGateUp | kPhaseDown, stream, "hot_experts", sel);
-  if (layout->gate_up_format == FB_FMT_IQ4_NL && layout->down_format == FB_FMT_IQ4_NL && layout->inter == 512)
-    return launch_experts_fmt<FB_FMT_IQ4_NL>(layout, ws, kPhaseGateUp | kPhaseDown, stream, "hot_experts", sel);
+  if (layout->down_format == FB_FMT_IQ4_NL || (layout->down_format == FB_FMT_IQ3_S && layout->gate_up_format == FB_FMT_IQ3_S))
+    return launch_phases(layout, ws, kPhaseGateUp | kPhaseDown, stream, "hot_experts", sel);
   const int32_t st = launch_gate_up(layout, ws, stream, sel);
   return st ? st : launch_down(layout, ws, stream);
 }
-
 
 int32_t fb_moe_hot_experts(const fb_moe_expert_layout* layout, int32_t tokens, const fb_moe_decode_workspace* ws,
                            void* stream) {
@@ -1569,33 +1241,12 @@ int32_t fb_moe_hot_experts(const fb_moe_expert_layout* layout, int32_t tokens, c
 }
 
 static int32_t launch_down(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream) {
-  if (layout->down_format == FB_FMT_IQ3_S) return launch_experts_iq3s(layout, ws, kPhaseDown, stream, "hot_down");
   if (layout->down_format == FB_FMT_Q2_0) {
     if (launch_pdl(down_q2_0_kernel, dim3(sm_count() * 8), dim3(256), 0, as_stream(stream), *layout, *ws) != cudaSuccess)
       return check_launch("hot_down");
     return 0;
   }
-  if (layout->inter == 512) return launch_experts_fmt<FB_FMT_IQ4_NL>(layout, ws, kPhaseDown, stream, "hot_down", nullptr);
-  static PerDeviceOnce once;
-  const cudaError_t attr = per_device_once(once, [] {
-    cudaError_t a = opt_in_smem(down_kernel<FB_FMT_IQ4_NL, 512>, down_smem<FB_FMT_IQ4_NL, 512>());
-    if (a == cudaSuccess) a = opt_in_smem(down_kernel<FB_FMT_IQ4_NL, 640>, down_smem<FB_FMT_IQ4_NL, 640>());
-    return a;
-  });
-  if (attr != cudaSuccess) {
-    set_error("hot_down: shared-memory opt-in: %s", cudaGetErrorString(attr));
-    return int32_t(attr);
-  }
-  const dim3 grid(sm_count());
-  cudaError_t e;
-  if (layout->inter == 512)
-    e = launch_pdl(down_kernel<FB_FMT_IQ4_NL, 512>, grid, dim3((Down<FB_FMT_IQ4_NL, 512>::kWarps + 1) * 32),
-                   down_smem<FB_FMT_IQ4_NL, 512>(), as_stream(stream), *layout, *ws);
-  else
-    e = launch_pdl(down_kernel<FB_FMT_IQ4_NL, 640>, grid, dim3((Down<FB_FMT_IQ4_NL, 640>::kWarps + 1) * 32),
-                   down_smem<FB_FMT_IQ4_NL, 640>(), as_stream(stream), *layout, *ws);
-  if (e != cudaSuccess) return check_launch("hot_down");
-  return 0;
+  return launch_phases(layout, ws, kPhaseDown, stream, "hot_down", nullptr);
 }
 
 int32_t fb_moe_hot_down(const fb_moe_expert_layout* layout, int32_t tokens, const fb_moe_decode_workspace* ws,
@@ -1653,14 +1304,7 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
                                           : launch(route_kernel<false, false>);
   if (e != cudaSuccess) return check_launch("layer_decode: route");
   const SelectArgs sel{logits_scratch, int(FB_ROUTER_ROWS), slot_of, tokens, remote_ok ? 1 : 0};
-  int32_t st;
-  if (plain_gate_up(layout->gate_up_format)) {  // no streaming kernel to select inside: one more launch
-    if (launch_pdl(select_only_kernel, dim3(1), dim3(512), 0, as_stream(stream), sel, *ws) != cudaSuccess)
-      return check_launch("layer_decode: select");
-    st = launch_experts(layout, ws, stream, nullptr);
-  } else {
-    st = launch_experts(layout, ws, stream, &sel);  // selection + both projections of every routed expert
-  }
+  const int32_t st = launch_experts(layout, ws, stream, &sel);  // selection + both projections of every routed expert
   if (st || !with_combine) return st;
   return fb_moe_combine(ws, nullptr, nullptr, 0, nullptr, nullptr, nullptr, y_out, tokens, 0, nullptr, 0.0f, stream);
 }

@@ -1,7 +1,8 @@
-// The streaming expert kernel of the decode path (gate/up and down of IQ3_S and of IQ4_NL experts), included
-// by moe_decode.cu inside namespace fb's anonymous namespace. Written for IQ3_S, described for IQ3_S; IQ4_NL
-// rides the same skeleton with its own tile sizes and block arithmetic (ExpertsCfg<FB_FMT_IQ4_NL>,
-// iq4nl_task_terms).
+// The streaming expert kernel of the decode path, included by moe_decode.cu inside namespace fb's anonymous namespace:
+// gate/up in IQ3_S, IQ4_NL, IQ2_S, IQ3_XXS or IQ4_XS, down in IQ3_S or IQ4_NL. Written for IQ3_S, described for IQ3_S; the
+// other formats ride the same skeleton with their own tile sizes and block arithmetic (ExpertsCfg, gate_up_sub,
+// iq4nl_task_terms). (Behind plain kernels - a warp per row, lanes = sub-blocks from global memory - an IQ2_S + IQ4_NL
+// layer of five tokens took 129 us in six launches.)
 //
 // One persistent kernel streams the gate, up and down matrices of every routed expert of a layer:
 // first all gate/up tiles (heaviest experts first), then all down tiles, through one three-stage ring
@@ -36,12 +37,7 @@ static_assert(q8k_planar_bytes(2560) % 16 == 0 && q8k_planar_bytes(512) % 16 == 
 
 // ------------------------------------------------------------------------------ codebook for the 2x+1 form
 // Entry i of lane l at word i*32 + l (as iq3s_tables_fill), bytes (g - 1) / 2.
-__device__ __forceinline__ void iq3s_half_tables_fill(uint32_t* gridrep, uint32_t* signtab) {
-  // consecutive threads write consecutive 16-byte pieces (eight per entry): no bank conflicts
-  for (int i = threadIdx.x; i < 512 * 8; i += blockDim.x) {
-    const uint32_t w = (iq3s_grid_entry(i >> 3) >> 1) & 0x07070707u;
-    reinterpret_cast<uint4*>(gridrep)[i] = make_uint4(w, w, w, w);
-  }
+__device__ __forceinline__ void sign_table_fill(uint32_t* signtab) {
   if (threadIdx.x < 16) {
     uint32_t m = 0;
 #pragma unroll
@@ -49,6 +45,14 @@ __device__ __forceinline__ void iq3s_half_tables_fill(uint32_t* gridrep, uint32_
       if (threadIdx.x & (1 << j)) m |= 0xFFu << (8 * j);
     signtab[threadIdx.x] = m;
   }
+}
+__device__ __forceinline__ void iq3s_half_tables_fill(uint32_t* gridrep, uint32_t* signtab) {
+  // consecutive threads write consecutive 16-byte pieces (eight per entry): no bank conflicts
+  for (int i = threadIdx.x; i < 512 * 8; i += blockDim.x) {
+    const uint32_t w = (iq3s_grid_entry(i >> 3) >> 1) & 0x07070707u;
+    reinterpret_cast<uint4*>(gridrep)[i] = make_uint4(w, w, w, w);
+  }
+  sign_table_fill(signtab);
 }
 
 // One 32-weight sub-block: P = sum over its 8 look-ups of dp4a(G ^ m, a) for each of TT tokens.
@@ -168,6 +172,7 @@ __device__ __forceinline__ float iq3s_block_d(const uint32_t* w) {
 // The 64-byte mask table sits on a 256-byte boundary (its address bytes 1-3 ride in a byte-permute)
 // inside an area of kSignArea bytes.
 constexpr int kSignArea = 320;
+constexpr int kIq2sTableBytes = 1024 * 64;  // eight copies of 1024 x 8 bytes
 __device__ __forceinline__ uint32_t* sign_table_at(uint8_t* area) {
   return reinterpret_cast<uint32_t*>(area + ((256u - (smem_u32(area) & 255u)) & 255u));
 }
@@ -240,113 +245,257 @@ __device__ __forceinline__ bool draw_task_n(const RingN<S>& r, int* ticket_ctr, 
 }
 
 // ------------------------------------------------------------------------------ the expert kernel
-// Gate/up tile = 16 intermediate rows: 16 gate rows and the 16 matching up rows (17,600 bytes each);
-// task b (0..9) = block b of all 32 rows, lanes 0-15 the gate rows, lanes 16-31 the up rows; the warp
-// that finishes the tile's last task adds each row's ten block terms in block order, pairs gate with
-// up through a shuffle and applies SwiGLU.
-// Down tile = 160 output rows (35,200 bytes; a row is two blocks); task 2k + b = block b of rows
-// 32k .. 32k+31; the finishing warp adds each row's two block terms and applies the routing weight.
-// Both kinds carry the activation rows of the pass behind the weights.
+// Gate/up tile = 16 intermediate rows: 16 gate rows and the 16 matching up rows; task b (0..9) = block b (256 weights)
+// of all 32 rows, lanes 0-15 the gate rows, lanes 16-31 the up rows; the warp that finishes the tile's last task adds
+// each row's ten block terms in block order, pairs gate with up through a shuffle and applies SwiGLU.
+// Down tile = 160 output rows at intermediate 512, 128 at 640; task 2k + b = half b (256 or 320 weights) of rows
+// 32k .. 32k+31 (at 640 the tasks 8 and 9 are empty); the finishing warp adds each row's two half terms and applies the
+// routing weight. Both kinds carry the activation rows of the pass behind the weights.
+// Bytes of 256 gate/up weights of one row, and the shared-memory table that decodes them (sign masks included).
 template <int FMT>
-struct ExpertsCfg;
+struct GuFmt;
 template <>
-struct ExpertsCfg<FB_FMT_IQ3_S> {
-  static constexpr int kWarps = 24, kTasks = 10, kStages = 3, kInter = 512;
-  static constexpr int kTaskBytes = 110;  // one block of 256 weights
-  static constexpr int kGuRows = 16, kGuRowBytes = 1100, kGuPart = kGuRows * kGuRowBytes;  // 17,600
-  static constexpr int kDnRows = 160, kDnRowBytes = 220, kDnTile = kDnRows * kDnRowBytes;  // 35,200
-  static constexpr int kAct = FB_ACT_Q8_K;
-  static constexpr int kGuAct = q8k_planar_bytes(H), kDnAct = q8k_planar_bytes(kInter);    // 2,784 / 608
-  static constexpr int kSlot = 2 * kGuPart + kTT * kGuAct;                                 // 40,768
-  static constexpr int kDnTilesPerItem = H / kDnRows;                                      // 16
-  static constexpr int kPartialFloats = kStages * kTasks * kTT * 32;
-  static constexpr int kTableBytes = kGridRepBytes + kSignArea;  // codebook replica and sign masks
-  static constexpr size_t kSmem = size_t(kTableBytes) + size_t(kStages) * kSlot + kPartialFloats * 4 + 128;
-};
-// IQ4_NL: the same tile and task shapes with a "block" of eight consecutive 18-byte blocks (256 weights, 144
-// bytes, 16-byte aligned in every row): gate/up tile = 16 + 16 rows of 1440 bytes, down tile = 160 rows of 288.
-// No table: the sixteen levels live in registers.
+struct GuFmt<FB_FMT_IQ3_S> { static constexpr int kBlock = 110, kTable = kGridRepBytes + kSignArea; };
 template <>
-struct ExpertsCfg<FB_FMT_IQ4_NL> {
-  static constexpr int kWarps = 24, kTasks = 10, kStages = 3, kInter = 512;
-  static constexpr int kTaskBytes = 144;
-  static constexpr int kGuRows = 16, kGuRowBytes = 1440, kGuPart = kGuRows * kGuRowBytes;  // 23,040
-  static constexpr int kDnRows = 160, kDnRowBytes = 288, kDnTile = kDnRows * kDnRowBytes;  // 46,080
-  static constexpr int kAct = FB_ACT_Q8_0;
-  static constexpr int kGuAct = H + H / 8, kDnAct = kInter + kInter / 8;                    // 2,880 / 576
-  static constexpr int kSlot = 2 * kGuPart + kTT * kGuAct;                                 // 51,840
+struct GuFmt<FB_FMT_IQ4_NL> { static constexpr int kBlock = 144, kTable = 0; };  // eight 18-byte blocks; levels in registers
+template <>
+struct GuFmt<FB_FMT_IQ2_S> { static constexpr int kBlock = 82, kTable = kIq2sTableBytes + kSignArea; };
+template <>
+struct GuFmt<FB_FMT_IQ3_XXS> { static constexpr int kBlock = 98, kTable = 256 * 32 * 4 + kSignArea; };
+template <>
+struct GuFmt<FB_FMT_IQ4_XS> { static constexpr int kBlock = 136, kTable = 0; };
+
+template <int GU, int DN, int INTER>
+struct ExpertsCfg {
+  static constexpr int kWarps = 24, kTasks = 10, kStages = 3, kInter = INTER;
+  static constexpr int kTaskBytes = GuFmt<GU>::kBlock;
+  static constexpr int kGuRows = 16, kGuRowBytes = kTasks * kTaskBytes, kGuPart = kGuRows * kGuRowBytes;
+  static constexpr int kDnTaskBytes = DN == FB_FMT_IQ3_S ? 110 : INTER / 64 * 18;  // half a row
+  static constexpr int kDnRows = INTER == 512 ? 160 : 128, kDnRowBytes = 2 * kDnTaskBytes, kDnTile = kDnRows * kDnRowBytes;
+  static constexpr int kAct = act_of(GU);
+  static constexpr int kGuAct = kAct == FB_ACT_Q8_K ? q8k_planar_bytes(H) : H + H / 8;
+  static constexpr int kDnAct = DN == FB_FMT_IQ3_S ? q8k_planar_bytes(INTER) : INTER + INTER / 8;
+  static constexpr int kGuBytes = 2 * kGuPart + kTT * kGuAct, kDnBytes = kDnTile + kTT * kDnAct;
+  static constexpr int kSlot = kGuBytes > kDnBytes ? kGuBytes : kDnBytes;
   static constexpr int kDnTilesPerItem = H / kDnRows;
   static constexpr int kPartialFloats = kStages * kTasks * kTT * 32;
-  static constexpr int kTableBytes = 0;
-  static constexpr size_t kSmem = size_t(kStages) * kSlot + kPartialFloats * 4 + 128;
+  static constexpr int kTableBytes = GuFmt<GU>::kTable;
+  static constexpr size_t kSmem = size_t(kTableBytes) + size_t(kStages) * kSlot + kPartialFloats * 4 + 128;
+  static_assert(DN == FB_FMT_IQ4_NL || (DN == FB_FMT_IQ3_S && GU == FB_FMT_IQ3_S && INTER == 512),
+                "IQ3_S down shares the gate/up codebook and needs whole blocks per half row");
+  static_assert(kTableBytes % 16 == 0 && kSlot % 16 == 0 && kGuPart % 16 == 0 && kDnTile % 16 == 0 && kGuAct % 16 == 0 &&
+                    kDnAct % 16 == 0 && H % kDnRows == 0 && kDnRows % 32 == 0 && 2 * (kDnRows / 32) <= kTasks,
+                "tile shapes, bulk-copy sizes");
+  static_assert(kSmem + 14592 <= 232448, "dynamic plus static shared memory of a block");
 };
-using Experts3 = ExpertsCfg<FB_FMT_IQ3_S>;
-template <int FMT>
-constexpr bool experts_cfg_ok() {
-  using C = ExpertsCfg<FMT>;
-  return C::kDnTile + kTT * C::kDnAct <= C::kSlot && C::kSlot % 16 == 0 && C::kGuPart % 16 == 0 && C::kDnTile % 16 == 0 &&
-         C::kGuAct % 16 == 0 && C::kDnAct % 16 == 0 && H % C::kDnRows == 0 && C::kDnRows % 32 == 0 &&
-         C::kGuRowBytes == C::kTasks * C::kTaskBytes && C::kDnRowBytes == 2 * C::kTaskBytes && C::kTaskBytes % 2 == 0;
-}
-static_assert(experts_cfg_ok<FB_FMT_IQ3_S>() && experts_cfg_ok<FB_FMT_IQ4_NL>(), "tile shapes, bulk-copy sizes");
 // kPhaseSelect: the CTA builds the work list itself from the router logits (SelectArgs) instead of
 // reading the device work list a selection kernel left.
 enum { kPhaseGateUp = 1, kPhaseDown = 2, kPhaseSelect = 4 };
 
-// One block (256 weights) of the lane's row against the pass's tokens: term[t] = bsum * d * d_act.
-template <bool MIS>
-__device__ __forceinline__ void expert_block_terms(const uint32_t* w, const uint32_t* grid_lane, uint32_t sign_base,
-                                                   const uint8_t* act0, int act_bytes, int k, int blk, int ntp,
-                                                   float (&term)[kTT]) {
-  const float d = iq3s_block_d<MIS>(w);
-  if (ntp == 1) {
-    const int8_t* a[1] = {reinterpret_cast<const int8_t*>(act0) + 256 * blk};
-    const int16_t* as[1] = {reinterpret_cast<const int16_t*>(act0 + q8k_planar_asum_off(k)) + 8 * blk};
-    int bs[1];
-    iq3s_block_idot2<MIS, 1>(w, grid_lane, sign_base, a, as, bs);
-    term[0] = float(bs[0]) * (d * reinterpret_cast<const float*>(act0 + k)[blk]);
-    term[1] = 0.0f;
-  } else {
-    const uint8_t* act1 = act0 + act_bytes;
-    const int8_t* a[2] = {reinterpret_cast<const int8_t*>(act0) + 256 * blk,
-                          reinterpret_cast<const int8_t*>(act1) + 256 * blk};
-    const int16_t* as[2] = {reinterpret_cast<const int16_t*>(act0 + q8k_planar_asum_off(k)) + 8 * blk,
-                            reinterpret_cast<const int16_t*>(act1 + q8k_planar_asum_off(k)) + 8 * blk};
-    int bs[2];
-    iq3s_block_idot2<MIS, 2>(w, grid_lane, sign_base, a, as, bs);
-    term[0] = float(bs[0]) * (d * reinterpret_cast<const float*>(act0 + k)[blk]);
-    term[1] = float(bs[1]) * (d * reinterpret_cast<const float*>(act1 + k)[blk]);
+// ------------------------------------------------------------------------------ tables of the gate/up formats
+// IQ3_S: the half codebook, replicated per lane. IQ2_S: 1024 entries of eight magnitudes, eight copies (entry i of
+// copy c at byte 64 i + 8 c, a lane reads copy lane % 8: two lanes of a half warp share two bank groups, 3 passes per
+// look-up of eight weights against 6 with one copy). IQ3_XXS: 256 entries of four magnitudes, one copy per lane.
+template <int FMT>
+__device__ __forceinline__ void experts_table_fill(uint32_t* grid, uint32_t* signtab) {
+  if constexpr (FMT == FB_FMT_IQ3_S) {
+    iq3s_half_tables_fill(grid, signtab);
+  } else if constexpr (FMT == FB_FMT_IQ2_S || FMT == FB_FMT_IQ3_XXS) {
+    if constexpr (FMT == FB_FMT_IQ2_S) {
+      for (int i = threadIdx.x; i < 1024 * 4; i += blockDim.x) {  // 16 bytes = two copies of an entry
+        const uint2 w = iq2s_grid_entry(i >> 2);
+        reinterpret_cast<uint4*>(grid)[i] = make_uint4(w.x, w.y, w.x, w.y);
+      }
+    } else {
+      for (int i = threadIdx.x; i < 256 * 8; i += blockDim.x) {
+        const uint32_t w = iq3xxs_grid_entry(i >> 3);
+        reinterpret_cast<uint4*>(grid)[i] = make_uint4(w, w, w, w);
+      }
+    }
+    sign_table_fill(signtab);
   }
 }
 
-// IQ4_NL: one task = eight consecutive blocks (144 bytes at `wp`, 16-byte aligned) of the lane's row against
-// the pass's tokens; blk0 = index of the first of them in the row. Even blocks start on a word (scale in the
-// low half, codes two bytes off: funnel shifts), odd blocks on a half word (scale in the high half, codes
-// aligned). term[t] = sum over the eight blocks, in block order, of isum * (d * d_act).
+// ------------------------------------------------------------------------------ one block against the pass's tokens
+// Four signed int8 weights from magnitudes and a sign mask (0xFF in the bytes of negative weights; magnitudes are at
+// least one, so the byte-wise + 1 never carries).
+__device__ __forceinline__ int signed4(uint32_t mag, uint32_t mask) { return int((mag ^ mask) + (mask & 0x01010101u)); }
+__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+
+// One 32-weight sub-block of the other formats as eight words of int8 weights in natural order. w = the word that holds
+// the block's scale (even blocks: in its low half), as iq3s_stream reads it; IQ4_XS: the block's words.
+template <int FMT, bool EVEN>
+__device__ __forceinline__ void gate_up_sub(const uint32_t* w, int ib, const uint32_t* grid, uint32_t sign_base,
+                                            const Iq4nlLevels& lv, int (&q)[8], int& m0, int& m1) {
+  if constexpr (FMT == FB_FMT_IQ4_XS) {
+    const uint32_t head = w[0], sl = w[1];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint2 v = reinterpret_cast<const uint2*>(w)[1 + 2 * ib + h];
+      const uint32_t qq[2] = {v.x, v.y};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t sel = qq[i] & 0x77777777u, pick = ((qq[i] >> 1) & 0x44444444u) | 0x32103210u;
+        const uint32_t r0 = prmt(prmt(lv.t0, lv.t1, sel), prmt(lv.t2, lv.t3, sel), pick);
+        const uint32_t sel1 = sel >> 16;
+        const uint32_t r1 = prmt(prmt(lv.t0, lv.t1, sel1), prmt(lv.t2, lv.t3, sel1), pick >> 16);
+        q[2 * h + i] = int(prmt(r0, r1, 0x6420u));      // low nibbles: weights 4j .. 4j + 3
+        q[4 + 2 * h + i] = int(prmt(r0, r1, 0x7531u));  // high nibbles: weights 16 + 4j ..
+      }
+    }
+    m0 = m1 = int(((sl >> (8 * (ib >> 1) + 4 * (ib & 1))) & 15u) | (((head >> (16 + 2 * ib)) & 3u) << 4)) - 32;
+  } else {
+    uint32_t g[8], sg;
+    if constexpr (FMT == FB_FMT_IQ2_S) {
+      const uint32_t qs = iq3s_stream<EVEN>(w, ib), qh = (iq3s_stream<EVEN>(w, 16 + (ib >> 2)) >> (8 * (ib & 3))) & 0xFFu;
+      sg = iq3s_stream<EVEN>(w, 8 + ib);
+      const uint32_t sc = iq3s_stream<EVEN>(w, 18 + (ib >> 2)) >> (8 * (ib & 3));
+      m0 = int((sc << 1) & 30u) + 1;
+      m1 = int((sc >> 3) & 30u) + 1;
+      // byte offsets 64 * index + 8 * (lane % 8) of two look-ups per word: the index byte in bits 6..13 (22..29), its two
+      // upper bits, taken from qh by a multiply that lands them on bits 14 and 15 (30 and 31)
+      const uint32_t lane_pat = (threadIdx.x & 7) * 0x00080008u;
+      const uint32_t a02 = ((qs << 6) & 0x3FC03FC0u) | lane_pat | ((qh * 0x04004000u) & 0xC000C000u);
+      const uint32_t a13 = ((qs >> 2) & 0x3FC03FC0u) | lane_pat | ((qh * 0x01001000u) & 0xC000C000u);
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        const uint32_t a = (l & 1) ? a13 : a02;
+        const uint2 v = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(grid) + ((l & 2) ? a >> 16 : a & 0xFFFFu));
+        g[2 * l] = v.x;
+        g[2 * l + 1] = v.y;
+      }
+    } else {
+      const uint32_t aux = iq3s_stream<EVEN>(w, 16 + ib);
+      m0 = m1 = 2 * int(aux >> 28) + 1;
+      // four 7-bit sign indices into bytes, the eighth sign is their parity
+      sg = (aux & 0x7Fu) | ((aux << 1) & 0x7F00u) | ((aux << 2) & 0x7F0000u) | ((aux << 3) & 0x7F000000u);
+      uint32_t p = sg ^ (sg >> 4);
+      p ^= p >> 2;
+      p ^= p >> 1;
+      sg |= (p & 0x01010101u) << 7;
+      const uint32_t lane4 = 4 * (threadIdx.x & 31);
+#pragma unroll
+      for (int l = 0; l < 8; ++l) {
+        const uint32_t qs = iq3s_stream<EVEN>(w, 2 * ib + (l >> 2));
+        g[l] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(grid) +
+                                                  ((((qs >> (8 * (l & 3))) & 0xFFu) << 7) | lane4));
+      }
+    }
+    const uint32_t s_even = (sg << 2) & 0x3C3C3C3Cu, s_odd = (sg >> 2) & 0x3C3C3C3Cu;  // nibbles as byte offsets, see iq3s_sub_dot
+#pragma unroll
+    for (int l = 0; l < 8; ++l)
+      q[l] = signed4(g[l], lds_word(prmt((l & 1) ? s_odd : s_even, sign_base, 0x7650u | uint32_t(l >> 1))));
+  }
+}
+
+template <int FMT, bool EVEN, int TT>
+__device__ __forceinline__ void gate_up_block_idot(const uint32_t* w, const uint32_t* grid, uint32_t sign_base,
+                                                   const Iq4nlLevels& lv, const int8_t* const (&act)[TT], int (&bsum)[TT]) {
+#pragma unroll
+  for (int t = 0; t < TT; ++t) bsum[t] = 0;
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ib = 4 * half + i;
+      int q[8], m0, m1;
+      gate_up_sub<FMT, EVEN>(w, ib, grid, sign_base, lv, q, m0, m1);
+#pragma unroll
+      for (int t = 0; t < TT; ++t) {
+        const int4 a0 = *reinterpret_cast<const int4*>(act[t] + 32 * ib);
+        const int4 a1 = *reinterpret_cast<const int4*>(act[t] + 32 * ib + 16);
+        int s0 = __dp4a(q[0], a0.x, 0);
+        s0 = __dp4a(q[1], a0.y, s0);
+        s0 = __dp4a(q[2], a0.z, s0);
+        s0 = __dp4a(q[3], a0.w, s0);
+        int s1 = __dp4a(q[4], a1.x, FMT == FB_FMT_IQ2_S ? 0 : s0);
+        s1 = __dp4a(q[5], a1.y, s1);
+        s1 = __dp4a(q[6], a1.z, s1);
+        s1 = __dp4a(q[7], a1.w, s1);
+        bsum[t] += FMT == FB_FMT_IQ2_S ? m0 * s0 + m1 * s1 : m0 * s1;
+      }
+    }
+  }
+}
+
+// One block (256 weights) of the lane's row against the pass's tokens: term[t] = bsum * d * d_act. EVEN: the block starts
+// on a word; ablk = index of the Q8_K block it meets in the activation row of k values.
+template <int FMT, bool EVEN>
+__device__ __forceinline__ void gate_up_block_terms(const uint8_t* blk, const uint32_t* grid, uint32_t sign_base,
+                                                    const Iq4nlLevels& lv, const uint8_t* act0, int act_bytes, int ablk,
+                                                    int ntp, float (&term)[kTT], int k = H) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(EVEN || FMT == FB_FMT_IQ4_XS ? blk : blk - 2);
+  constexpr bool kLow = EVEN || FMT == FB_FMT_IQ4_XS;  // the scale sits in the low half of its word
+  constexpr float kFactor = FMT == FB_FMT_IQ2_S ? 0.125f : FMT == FB_FMT_IQ3_XXS ? 0.25f : 1.0f;
+  const float d = iq3s_block_d<kLow>(w) * kFactor;
+  auto dots = [&](auto& a, auto& as, auto& bs) {
+    constexpr int TT = sizeof(bs) / sizeof(int);
+    if constexpr (FMT == FB_FMT_IQ3_S) iq3s_block_idot2<EVEN, TT>(w, grid + (threadIdx.x & 31), sign_base, a, as, bs);
+    else gate_up_block_idot<FMT, EVEN, TT>(w, grid, sign_base, lv, a, bs);
+  };
+  if (ntp == 1) {
+    const int8_t* a[1] = {reinterpret_cast<const int8_t*>(act0) + 256 * ablk};
+    const int16_t* as[1] = {reinterpret_cast<const int16_t*>(act0 + q8k_planar_asum_off(k)) + 8 * ablk};
+    int bs[1];
+    dots(a, as, bs);
+    term[0] = float(bs[0]) * (d * reinterpret_cast<const float*>(act0 + k)[ablk]);
+  } else {
+    const uint8_t* act1 = act0 + act_bytes;
+    const int8_t* a[2] = {reinterpret_cast<const int8_t*>(act0) + 256 * ablk,
+                          reinterpret_cast<const int8_t*>(act1) + 256 * ablk};
+    const int16_t* as[2] = {reinterpret_cast<const int16_t*>(act0 + q8k_planar_asum_off(k)) + 8 * ablk,
+                            reinterpret_cast<const int16_t*>(act1 + q8k_planar_asum_off(k)) + 8 * ablk};
+    int bs[2];
+    dots(a, as, bs);
+    term[0] = float(bs[0]) * (d * reinterpret_cast<const float*>(act0 + k)[ablk]);
+    term[1] = float(bs[1]) * (d * reinterpret_cast<const float*>(act1 + k)[ablk]);
+  }
+}
+
+// IQ4_NL: one task = NB consecutive 18-byte blocks of the lane's row, OFF bytes behind `wp`, against the pass's tokens;
+// blk0 = index of the first of them in the row. Even blocks start on a word (scale in the low half, codes two bytes
+// off: funnel shifts), odd blocks on a half word (scale in the high half, codes aligned). Rows of 1440 and 288 bytes keep
+// eight blocks on 16-byte boundaries, the halves of 360-byte rows start on 8-byte boundaries (the second one four bytes
+// early): the widest loads without bank conflicts. term[t] = sum over the blocks, in block order, of isum * (d * d_act).
+template <int NB, int OFF>
 __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlLevels& lv, const uint8_t* act0,
                                                  int act_bytes, int k, int blk0, int ntp, float (&term)[kTT]) {
-  uint32_t w[36];
+  constexpr int kWords = NB == 8 ? 36 : 46, kOff = OFF / 4;
+  uint32_t w[kWords];
+  if constexpr (NB == 8) {
 #pragma unroll
-  for (int c = 0; c < 9; ++c) {
-    const uint4 v = reinterpret_cast<const uint4*>(wp)[c];
-    w[4 * c] = v.x;
-    w[4 * c + 1] = v.y;
-    w[4 * c + 2] = v.z;
-    w[4 * c + 3] = v.w;
+    for (int c = 0; c < kWords / 4; ++c) {
+      const uint4 v = reinterpret_cast<const uint4*>(wp)[c];
+      w[4 * c] = v.x;
+      w[4 * c + 1] = v.y;
+      w[4 * c + 2] = v.z;
+      w[4 * c + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < kWords / 2; ++c) {
+      const uint2 v = reinterpret_cast<const uint2*>(wp)[c];
+      w[2 * c] = v.x;
+      w[2 * c + 1] = v.y;
+    }
   }
   term[0] = term[1] = 0.0f;
   const uint8_t* act1 = act0 + (ntp == 2 ? act_bytes : 0);
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
+  for (int b = 0; b < NB; ++b) {
     uint32_t q[4];
     float d;
     if (b % 2 == 0) {
-      const int base = 9 * b / 2;
+      const int base = kOff + 9 * b / 2;
       d = __half2float(__ushort_as_half(static_cast<unsigned short>(w[base] & 0xFFFFu)));
 #pragma unroll
       for (int i = 0; i < 4; ++i) q[i] = __funnelshift_r(w[base + i], w[base + i + 1], 16);
     } else {
-      const int base = (18 * b - 2) / 4;
+      const int base = kOff + (18 * b - 2) / 4;
       d = __half2float(__ushort_as_half(static_cast<unsigned short>(w[base] >> 16)));
 #pragma unroll
       for (int i = 0; i < 4; ++i) q[i] = w[base + 1 + i];
@@ -362,16 +511,15 @@ __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlL
     }
   }
 }
-
-template <int FMT>
-__global__ void __launch_bounds__((ExpertsCfg<FMT>::kWarps + 1) * 32, 1)
+template <int GU, int DN, int INTER>
+__global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + 1) * 32, 1)
 experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, SelectArgs sel) {
-  using C = ExpertsCfg<FMT>;
+  using C = ExpertsCfg<GU, DN, INTER>;
   constexpr int S = C::kStages;
-  constexpr bool kIq3s = FMT == FB_FMT_IQ3_S;
+  constexpr bool kSigns = GU == FB_FMT_IQ3_S || GU == FB_FMT_IQ2_S || GU == FB_FMT_IQ3_XXS;
   extern __shared__ __align__(128) uint8_t smem[];
-  uint32_t* gridrep = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* signtab = kIq3s ? sign_table_at(smem + kGridRepBytes) : nullptr;
+  uint32_t* grid = reinterpret_cast<uint32_t*>(smem);  // the gate/up format's codebook, its sign masks behind it
+  uint32_t* signtab = kSigns ? sign_table_at(smem + (C::kTableBytes - kSignArea)) : nullptr;
   uint8_t* stage0 = smem + C::kTableBytes;
   float* partials = reinterpret_cast<float*>(stage0 + S * C::kSlot);
   uint64_t* bars = reinterpret_cast<uint64_t*>(partials + C::kPartialFloats);
@@ -382,7 +530,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   RingN<S> ring{bars, bars + S, s_meta, &s_end};
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if constexpr (kIq3s) iq3s_half_tables_fill(gridrep, signtab);
+  // (a down-only launch of another format than IQ3_S looks nothing up)
+  if (DN == FB_FMT_IQ3_S || (phases & kPhaseGateUp)) experts_table_fill<GU>(grid, signtab);
   if (tid == 0) {
     ringn_init(ring);
     for (int i = 1; i < 3 + S; ++i) s_misc[i] = 0;
@@ -402,9 +551,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   } else {
     n_items = min(max(ws.work->n_items, 0), kMaxPairs);
   }
-  const int I = L.inter;  // gate/up takes 512 or 640; the down phase is for 512 (checked on the host)
   const uint8_t* xq_rows = ws.xq + xq_offset(C::kAct);
-  const int gu_tpi = I / C::kGuRows;
+  constexpr int gu_tpi = INTER / C::kGuRows;
   const int n_gu = (phases & kPhaseGateUp) ? n_items * gu_tpi : 0;
   const int n_dn = (phases & kPhaseDown) ? n_items * C::kDnTilesPerItem : 0;
 
@@ -448,7 +596,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       next2 = first_ticket + atomicAdd(counter, 1);
       const bool down = tile >= n_gu;
       const int tl = down ? tile - n_gu : tile;
-      const int pos = down ? tl / C::kDnTilesPerItem : I == 512 ? tl >> 5 : tl / (640 / C::kGuRows);  // (no run-time division)
+      const int pos = down ? tl / C::kDnTilesPerItem : tl / gu_tpi;
       const int sub = down ? tl - pos * C::kDnTilesPerItem : tl - pos * gu_tpi;
       const int item = s_work.order[pos];
       const int pb = s_work.pair_begin[item];
@@ -512,13 +660,12 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   }
 
   // ---------------- consumers
-  const uint32_t* grid_lane = gridrep + lane;
-  const uint32_t sign_base = kIq3s ? smem_u32(signtab) : 0u;
+  const uint32_t sign_base = kSigns ? smem_u32(signtab) : 0u;
   const Iq4nlLevels lv = iq4nl_levels();
   const int gu_row_off = (lane >> 4) * C::kGuPart + (lane & 15) * C::kGuRowBytes;
-  // Even blocks start on a word boundary (their 27-word stream is 2 bytes off), odd blocks the other
-  // way round: two code paths. A warp keeps to one parity, and since warp w issues on scheduler w % 4,
-  // each scheduler's instruction cache sees one path only.
+  // Even blocks of the formats with 2-byte alignment start on a word boundary (their words behind the scale are 2 bytes
+  // off), odd blocks the other way round: two code paths. A warp keeps to one parity, and since warp w issues on
+  // scheduler w % 4, each scheduler's instruction cache sees one path only.
   const int parity = warp & 1;
   const int down_act = act_of(L.down_format);
   while (true) {
@@ -528,20 +675,31 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     const int ntp = ring.meta[s].ntp;
     const bool down = ring.meta[s].tile != 0;
     uint8_t* st = stage0 + s * C::kSlot;
-    // the lane's block, the activation rows, and which of their blocks it meets
-    const uint8_t* blk = down ? st + (32 * k + lane) * C::kDnRowBytes + parity * C::kTaskBytes
-                              : st + gu_row_off + task * C::kTaskBytes;
-    const uint8_t* act0 = st + (down ? C::kDnTile : 2 * C::kGuPart);
-    const int act_bytes = down ? C::kDnAct : C::kGuAct, act_k = down ? C::kInter : H, ablk = down ? parity : task;
-    float term[kTT];
-    if constexpr (!kIq3s)
-      iq4nl_task_terms(blk, lv, act0, act_bytes, act_k, 8 * ablk, ntp, term);
-    else if (parity == 0)
-      expert_block_terms<true>(reinterpret_cast<const uint32_t*>(blk), grid_lane, sign_base, act0, act_bytes, act_k, ablk,
-                               ntp, term);
-    else
-      expert_block_terms<false>(reinterpret_cast<const uint32_t*>(blk - 2), grid_lane, sign_base, act0, act_bytes, act_k,
-                                ablk, ntp, term);
+    float term[kTT] = {0.0f, 0.0f};
+    if (!down) {
+      const uint8_t* blk = st + gu_row_off + task * C::kTaskBytes;
+      const uint8_t* act0 = st + 2 * C::kGuPart;
+      if constexpr (GU == FB_FMT_IQ4_NL) {
+        iq4nl_task_terms<8, 0>(blk, lv, act0, C::kGuAct, H, 8 * task, ntp, term);
+      } else if (parity == 0) {
+        gate_up_block_terms<GU, true>(blk, grid, sign_base, lv, act0, C::kGuAct, task, ntp, term);
+      } else {
+        gate_up_block_terms<GU, false>(blk, grid, sign_base, lv, act0, C::kGuAct, task, ntp, term);
+      }
+    } else if (k < C::kDnRows / 32) {
+      const uint8_t* half = st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes;
+      const uint8_t* act0 = st + C::kDnTile;
+      if constexpr (DN == FB_FMT_IQ3_S) {
+        if (parity == 0) gate_up_block_terms<GU, true>(half, grid, sign_base, lv, act0, C::kDnAct, 0, ntp, term, INTER);
+        else gate_up_block_terms<GU, false>(half, grid, sign_base, lv, act0, C::kDnAct, 1, ntp, term, INTER);
+      } else if constexpr (INTER == 512) {
+        iq4nl_task_terms<8, 0>(half, lv, act0, C::kDnAct, INTER, 8 * parity, ntp, term);
+      } else if (parity == 0) {
+        iq4nl_task_terms<10, 0>(half, lv, act0, C::kDnAct, INTER, 0, ntp, term);
+      } else {
+        iq4nl_task_terms<10, 4>(half - 4, lv, act0, C::kDnAct, INTER, 10, ntp, term);
+      }
+    }
     float* part = partials + (s * C::kTasks + task) * (kTT * 32);
     part[lane] = term[0];
     part[32 + lane] = term[1];
@@ -563,14 +721,14 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 #pragma unroll
         for (int b = 0; b < C::kTasks; ++b) v += pt[(b * kTT + t) * 32 + lane];
         const float u = __shfl_down_sync(0xffffffffu, v, 16);
-        if (lane < 16) ws.h[size_t(pair0 + t) * I + r0 + lane] = silu_mul(v, u);
+        if (lane < 16) ws.h[size_t(pair0 + t) * INTER + r0 + lane] = silu_mul(v, u);
       }
       __syncwarp();
       if (lane == 0) {
         s_misc[3 + s] = 0;
         mbar_arrive(&ring.empty[s]);
       }
-      item_contribution_done(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act, I, lane);
+      item_contribution_done(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act, INTER, lane);
     } else {
       const float w0 = ring.meta[s].wgt[0], w1 = ring.meta[s].wgt[1];
 #pragma unroll

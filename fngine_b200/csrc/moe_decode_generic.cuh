@@ -4,13 +4,8 @@
 // third_party/ggml-iq/ggml-iq.h:26-78 of the reference. Included by moe_decode.cu (everything) and by
 // probes.cu (the decoders and the dequantization probe only).
 //
-// These are plain kernels, not the streaming skeleton of the IQ3_S / IQ4_NL paths: a warp takes one
-// (work item, row) unit, its lanes the row's 32-weight sub-blocks straight from global memory; every
-// sub-block is decoded once into eight words of int8 weights and met with each token's codes by dp4a.
-// Arithmetic per sub-block and token: d * dA * (m0 * dot(first 16) + m1 * dot(second 16)), the integer
-// part exact; a warp butterfly adds the lanes. They read the device work list a selection kernel left.
-// Not tuned: they are here so that a layer in any of the pack's formats runs on the GPU with the CPU
-// tier's numerics (1e-3), at a fraction of the streaming kernels' rate.
+// The gate/up formats run in the streaming kernel (moe_decode_experts.cuh takes the codebooks from here); Q2_0 has a
+// plain kernel: a warp per pair of rows, lanes = sub-blocks straight from global memory, reading the device work list.
 // (No namespace of its own: included inside namespace fb's unnamed namespace, once per translation unit.)
 #pragma once
 
@@ -19,32 +14,36 @@ static __constant__ uint16_t c_iq2s_grid_packed[1024] = {FB_IQ2S_GRID_PACKED};
 
 constexpr int kGenericGridWords = 2048;  // shared-memory words the largest expanded codebook takes (IQ2_S: 1024 x 8 bytes)
 
+__device__ __forceinline__ uint32_t iq3xxs_grid_entry(int i) {
+  const uint32_t p = c_iq3xxs_grid_packed[i];
+  uint32_t w = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t c = (p >> (3 * j)) & 7u;
+    w |= (4u + 8u * c + (c == 7u ? 2u : 0u)) << (8 * j);  // 4, 12, ..., 52, 62
+  }
+  return w;
+}
+
+__device__ __forceinline__ uint2 iq2s_grid_entry(int i) {
+  const uint32_t p = c_iq2s_grid_packed[i];
+  uint32_t w[2] = {0, 0};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t c = (p >> (2 * j)) & 3u;
+    w[j >> 2] |= (c == 0u ? 8u : c == 1u ? 25u : 43u) << (8 * (j & 3));
+  }
+  return make_uint2(w[0], w[1]);
+}
+
 // Expands the format's codebook into shared memory (called by every thread; caller synchronizes).
 // IQ3_XXS: 256 words of four magnitudes; IQ2_S: 1024 pairs of words of four magnitudes each.
 template <int FMT>
 __device__ __forceinline__ void generic_grid_fill(uint32_t* grid) {
   if constexpr (FMT == FB_FMT_IQ3_XXS) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-      const uint32_t p = c_iq3xxs_grid_packed[i];
-      uint32_t w = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t c = (p >> (3 * j)) & 7u;
-        w |= (4u + 8u * c + (c == 7u ? 2u : 0u)) << (8 * j);  // 4, 12, ..., 52, 62
-      }
-      grid[i] = w;
-    }
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) grid[i] = iq3xxs_grid_entry(i);
   } else if constexpr (FMT == FB_FMT_IQ2_S) {
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) {
-      const uint32_t p = c_iq2s_grid_packed[i >> 1] >> (8 * (i & 1));
-      uint32_t w = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t c = (p >> (2 * j)) & 3u;
-        w |= (c == 0u ? 8u : c == 1u ? 25u : 43u) << (8 * j);
-      }
-      grid[i] = w;
-    }
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x) reinterpret_cast<uint2*>(grid)[i] = iq2s_grid_entry(i);
   }
 }
 
@@ -177,7 +176,7 @@ __device__ __forceinline__ void dequant_sub32(const uint8_t* row, int sub, const
 template <int FMT>
 __global__ void __launch_bounds__(256) dequant_generic_kernel(const uint8_t* __restrict__ rows, int64_t row_bytes,
                                                               int nrows, int k, float* __restrict__ out) {
-  __shared__ uint32_t s_grid[kGenericGridWords];
+  __shared__ __align__(8) uint32_t s_grid[kGenericGridWords];
   generic_grid_fill<FMT>(s_grid);
   __syncthreads();
   const int subs = k / 32;
@@ -191,82 +190,8 @@ __global__ void __launch_bounds__(256) dequant_generic_kernel(const uint8_t* __r
   }
 }
 
-#ifdef FB_MOE_DECODE_TU  // the MoE kernels below need the decode translation unit's workspace helpers
-// dp4a of a decoded sub-block with 32 activation codes in natural order (Q8_K planar rows)
-__device__ __forceinline__ float sub32_dot_natural(const Sub32& s, const int* a, float da) {
-  int s0 = 0, s1 = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) s0 = __dp4a(s.q[j], a[j], s0);
-#pragma unroll
-  for (int j = 4; j < 8; ++j) s1 = __dp4a(s.q[j], a[j], s1);
-  return float(s.m0 * s0 + s.m1 * s1) * (s.d * da);
-}
-
+#ifdef FB_MOE_DECODE_TU  // the MoE kernel below needs the decode translation unit's workspace helpers
 constexpr int kGenTok = 4;  // tokens of an item handled per pass over a row
-
-// gate/up for a Q8_K-paired format: unit = (item, intermediate row); h[pair][j] = silu(gate.x) * (up.x).
-template <int FMT>
-__global__ void __launch_bounds__(256) gate_up_generic_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws) {
-  __shared__ uint32_t s_grid[kGenericGridWords];
-  generic_grid_fill<FMT>(s_grid);
-  __syncthreads();
-  pdl_launch_dependents();
-  pdl_wait_prior();
-  const fb_moe_decode_work* work = ws.work;
-  const int n_items = min(max(work->n_items, 0), kMaxPairs), I = L.inter;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row_bytes = int64_t(H / 256) * (FMT == FB_FMT_IQ3_XXS ? 98 : FMT == FB_FMT_IQ2_S ? 82 : 136);
-  for (int u = blockIdx.x * 8 + warp; u < n_items * I; u += gridDim.x * 8) {
-    const int item = u / I, j = u - item * I;
-    const int pb = work->item_pair_begin[item], ntok = work->item_pair_begin[item + 1] - pb;
-    const uint8_t* blob = L.slots + int64_t(work->item_slot[item]) * L.blob_stride;
-    const uint8_t* grow = blob + L.gate_offset + int64_t(j) * row_bytes;
-    const uint8_t* urow = blob + L.up_offset + int64_t(j) * row_bytes;
-    for (int t0 = 0; t0 < ntok; t0 += kGenTok) {
-      float ag[kGenTok], au[kGenTok];
-      const uint8_t* xq[kGenTok];
-#pragma unroll
-      for (int t = 0; t < kGenTok; ++t) {
-        ag[t] = au[t] = 0.0f;
-        xq[t] = ws.xq + size_t(work->pair_token[pb + min(t0 + t, ntok - 1)]) * FB_XQ_STRIDE;  // Q8_K rows sit first
-      }
-      for (int sub = lane; sub < H / 32; sub += 32) {
-        Sub32 sg, su;
-        decode_sub32<FMT>(grow, sub, s_grid, sg);
-        decode_sub32<FMT>(urow, sub, s_grid, su);
-#pragma unroll
-        for (int t = 0; t < kGenTok; ++t) {
-          const int4* ap = reinterpret_cast<const int4*>(xq[t] + 32 * sub);
-          const int4 a0 = ap[0], a1 = ap[1];
-          const int a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-          const float da = reinterpret_cast<const float*>(xq[t] + H)[sub >> 3];
-          ag[t] += sub32_dot_natural(sg, a, da);
-          au[t] += sub32_dot_natural(su, a, da);
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < kGenTok; ++t) {
-        float g = ag[t], up = au[t];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          g += __shfl_xor_sync(0xffffffffu, g, o);
-          up += __shfl_xor_sync(0xffffffffu, up, o);
-        }
-        if (lane == 0 && t0 + t < ntok) ws.h[size_t(pb + t0 + t) * I + j] = silu_mul(g, up);
-      }
-    }
-  }
-}
-
-// h of every pair -> planar activation rows for the down projection (one warp per pair); the streaming
-// gate/up kernels do this themselves, the generic one leaves it to this launch.
-__global__ void __launch_bounds__(256) requant_h_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws) {
-  pdl_launch_dependents();
-  pdl_wait_prior();
-  const int n_pairs = min(max(ws.work->n_pairs, 0), kMaxPairs);
-  const int p = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (p < n_pairs) quantize_item_h(ws, p, 1, act_of(L.down_format), L.inter);
-}
 
 // down for Q2_0 (Q8_0 activations, stored per 32-block in the order position p <- element (p % 2) * 16 + p / 2):
 // unit = (item, pair of output rows): lanes 0-15 take the 16 sub-blocks of row 2n (inter 512; 20 of 640 wrap),
