@@ -1138,6 +1138,282 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   }
 }
 
+// ------------------------------------------------------------------------------ few row tiles
+// The same projection when the row tiles do not fill the GPU (at most one CTA each: everything but the vocabulary
+// matrix). Bound: latency. The two kernels above spend a launch on the activation split, then a chain of global
+// round trips on partial sums and tickets: 15.5 us for 2560 x 6144 at four tokens, 2.5 us of which is the weights'
+// traffic. Here a CLUSTER owns a row tile, its CTAs equal shares of K; each CTA splits its own part of the activations
+// straight into operand rows in shared memory (the token scale is then the CTA's own, so no pass over whole rows comes
+// first), and the partial tiles meet through distributed shared memory, added in CTA order (fixed: repeated calls are
+// bitwise identical). One launch, no workspace.
+constexpr int kSmallThreads = 512, kSmallMaxKb = 20, kSmallMaxCluster = 8;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallMaxStages = 8;
+struct SmallBars {
+  uint64_t full[kSmallMaxStages], empty[kSmallMaxStages];
+  uint64_t acc;
+  uint32_t tmem_base;
+  int abort;
+  float red[kSmallWarps];
+  float scale[kDecTok];
+};
+constexpr int kSmallPartFloats = 128 * kDecTok;
+__host__ __device__ constexpr int small_smem_of(int nkb, int stages) {
+  return 1024 + stages * kDecStageA + nkb * kDecStageB + kSmallPartFloats * 4 + int(sizeof(SmallBars)) + 16;
+}
+// Weight stages: every K block of the CTA at once if eight do, else what fits beside the operand rows. (Three stages, so
+// that two calls' CTAs share a multiprocessor, were slower: each refill is a round trip to memory.)
+__host__ __device__ constexpr int small_stages(int nkb) {
+  int s = nkb < kSmallMaxStages ? nkb : kSmallMaxStages;
+  while (small_smem_of(nkb, s) > 232448) --s;
+  return s;
+}
+constexpr int small_smem(int nkb) { return small_smem_of(nkb, small_stages(nkb)); }
+static_assert(small_smem(kSmallMaxKb) <= 232448, "shared memory per block");
+
+// Two fp32 values as three E5M2 pairs: each rounds the remainder of the one before (round to nearest, subtract).
+__device__ __forceinline__ void split_pair_e5m2(float a, float b, uint32_t (&c)[3]) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    c[p] = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E5M2);
+    if (p < 2) {
+      const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(c[p]), __NV_E5M2);
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+      a -= f.x;
+      b -= f.y;
+    }
+  }
+}
+
+__device__ __forceinline__ void prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1)
+fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* __restrict__ x,
+                 const __grid_constant__ DecArgs a, int cluster) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const bool swiglu = a.kind == FB_EPI_SWIGLU;
+  const int kbt = a.k / BK, m = int(blockIdx.x) / cluster, rank = int(blockIdx.x) - m * cluster;
+  const int kb0 = kbt * rank / cluster, nkb = kbt * (rank + 1) / cluster - kb0;
+  const int nkb_max = (kbt + cluster - 1) / cluster, S = small_stages(nkb_max);
+  uint8_t* pieces = smem + S * kDecStageA;                                             // [nkb][48][128], swizzled
+  float* part = reinterpret_cast<float*>(pieces + nkb_max * kDecStageB);               // [token][row]
+  SmallBars* bars = reinterpret_cast<SmallBars*>(part + kSmallPartFloats);
+  const int r0 = swiglu ? m * 64 : m * 128, r1 = swiglu ? (a.n >> 1) + m * 64 : m * 128 + 64;
+  pdl_launch_dependents();
+
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+    for (uint32_t i = 0; i < (1u << 21); ++i) {
+      if (mbar_try_wait_hint(bar, parity)) return true;
+      if ((i & 31u) == 31u && *reinterpret_cast<volatile int*>(&bars->abort)) return false;
+    }
+    *reinterpret_cast<volatile int*>(&bars->abort) = 1;
+    atomicMax(a.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+    return false;
+  };
+  // The weights start on their way into L2 before the wait for the preceding kernel (a prefetch reads nothing yet, so
+  // it does not matter whether that kernel writes them).
+  if (warp == 2 && elect_one())
+    for (int i = 0; i < nkb; ++i) {
+      prefetch_2d(&map_w, (kb0 + i) * BK, r0);
+      prefetch_2d(&map_w, (kb0 + i) * BK, r1);
+    }
+  if (tid == 0) {
+    for (int i = 0; i < kSmallMaxStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    mbar_init(&bars->acc, 1);
+    bars->abort = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&bars->tmem_base, 64);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  pdl_wait_prior();
+
+  auto load_stage = [&](int i) {
+    uint8_t* st = smem + (i % S) * kDecStageA;
+    mbar_expect_tx(&bars->full[i % S], kDecStageA);
+    tma_load_2d(st, &map_w, (kb0 + i) * BK, r0, &bars->full[i % S]);
+    tma_load_2d(st + 64 * BK, &map_w, (kb0 + i) * BK, r1, &bars->full[i % S]);
+  };
+  if (warp == 0 && elect_one())
+    for (int i = 0; i < min(nkb, S); ++i) load_stage(i);
+
+  // ---------------- activations: W warps per token, each takes every W-th piece of 256 values of the CTA's K range
+  int tp = 1;
+  while (tp < a.T) tp <<= 1;
+  const int W = kSmallWarps / tp, t = warp / W, sub = warp - t * W, len = nkb * BK;
+  float mx = 0.0f;
+  const __nv_bfloat16* row = x + size_t(t) * a.k + size_t(kb0) * BK;
+  if (t < a.T) {
+#pragma unroll 5
+    for (int el = 256 * sub + 8 * lane; el < len; el += 256 * W) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + el);
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        mx = fmaxf(mx, fmaxf(fabsf(__uint_as_float(u[i] << 16)), fabsf(__uint_as_float(u[i] & 0xFFFF0000u))));
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) bars->red[warp] = mx;
+  }
+  __syncthreads();
+  if (t < a.T) {
+    for (int i = 0; i < W; ++i) mx = fmaxf(mx, bars->red[t * W + i]);
+    // scale = 2^(exponent(max) - 14), as in fp8_split_tokens_kernel
+    uint32_t e = (__float_as_uint(mx) >> 23) & 0xFFu;
+    e = e < 15u ? 15u : (e > 253u ? 253u : e);
+    const float inv = __uint_as_float((268u - e) << 23);
+    if (sub == 0 && lane == 0) bars->scale[t] = __uint_as_float((e - 14u) << 23);
+#pragma unroll 2
+    for (int el = 256 * sub + 8 * lane; el < len; el += 256 * W) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + el);  // (from the L1 cache now)
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+      uint32_t out[3][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t lo[3], hi[3];
+        split_pair_e5m2(__uint_as_float(u[2 * i] << 16) * inv, __uint_as_float(u[2 * i] & 0xFFFF0000u) * inv, lo);
+        split_pair_e5m2(__uint_as_float(u[2 * i + 1] << 16) * inv, __uint_as_float(u[2 * i + 1] & 0xFFFF0000u) * inv, hi);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) out[q][i] = lo[q] | (hi[q] << 16);
+      }
+      uint8_t* tile = pieces + (el >> 7) * kDecStageB;
+      const int chunk = (el & 127) >> 4, half = el & 8;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const int r = q * kDecTok + t;
+        *reinterpret_cast<uint2*>(tile + r * 128 + ((chunk ^ (r & 7)) << 4) + half) = make_uint2(out[q][0], out[q][1]);
+      }
+    }
+  }
+  fence_proxy_async();
+  __syncthreads();
+
+  if (warp == 0) {
+    if (elect_one())
+      for (int i = S; i < nkb; ++i) {
+        if (!wait(&bars->empty[i % S], ((i / S) - 1) & 1)) break;
+        load_stage(i);
+      }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      bool ok = true;
+      for (int i = 0; i < nkb; ++i) {
+        if (!(ok = wait(&bars->full[i % S], (i / S) & 1))) break;
+        const uint64_t da = umma_desc_k128(smem_u32(smem + (i % S) * kDecStageA)),
+                       db = umma_desc_k128(smem_u32(pieces + i * kDecStageB));
+#pragma unroll
+        for (int k4 = 0; k4 < BK / 32; ++k4)
+          umma_f8(tmem_base, da + uint64_t(2 * k4), db + uint64_t(2 * k4), kIdescDec, (i || k4) ? 1u : 0u);
+        if (i + S < nkb) umma_commit(&bars->empty[i % S]);
+      }
+      if (ok) umma_commit(&bars->acc);
+    }
+  } else if (warp >= 4 && warp < 8) {
+    // ---------------- the CTA's partial tile, token scale applied, into shared memory
+    const int q = warp & 3, rl = q * 32 + lane;
+    if (__all_sync(0xffffffffu, wait(&bars->acc, 0))) {
+      tc_fence_after();
+      uint32_t c[kDecN];
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16);
+      tmem_ld16_nowait(taddr, c);
+      tmem_ld16_nowait(taddr + 16, c + 16);
+      tmem_ld16_nowait(taddr + 32, c + 32);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < kDecTok; ++i)
+        if (i < a.T)
+          part[i * 128 + rl] = ((__uint_as_float(c[32 + i]) + __uint_as_float(c[16 + i])) + __uint_as_float(c[i])) * bars->scale[i];
+      tc_fence_before();
+    }
+  }
+  // The outputs of the tile are dealt out over the cluster's threads: consecutive threads, consecutive rows. What an
+  // output needs besides the sum is fetched while the sums are still on their way.
+  const int rows = swiglu ? 64 : 128, n_out = a.T * rows;
+  const int half_n = a.n >> 1;
+  auto sum_of = [&](int tt, int r) -> float {
+    if (cluster == 1) return part[tt * 128 + r];
+    float p[kSmallMaxCluster];
+#pragma unroll
+    for (int c = 0; c < kSmallMaxCluster; ++c) p[c] = c < cluster ? ld_cluster_f32(part + tt * 128 + r, uint32_t(c)) : 0.0f;
+    float s = p[0];
+#pragma unroll
+    for (int c = 1; c < kSmallMaxCluster; ++c) s += p[c];  // (adding + 0.0 behind the last changes nothing)
+    return s;
+  };
+  const int first = rank * kSmallThreads + tid;
+  int tt = first / rows, r = first - tt * rows;  // (rows is 64 or 128)
+  bool live = first < n_out && (swiglu ? m * 64 + r < half_n : m * 128 + r < a.n);
+  float ws0 = 0.0f, ws1 = 0.0f, gate = 1.0f, x4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float4 g4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  auto fetch = [&]() {
+    if (!live) return;
+    if (swiglu) {
+      ws0 = dec_row_scale(a, m * 64 + r);
+      ws1 = dec_row_scale(a, half_n + m * 64 + r);
+      return;
+    }
+    const int n = m * 128 + r;
+    ws0 = dec_row_scale(a, n);
+    if (a.kind == FB_EPI_GR_WRITE) {
+      g4 = *reinterpret_cast<const float4*>(a.inj + size_t(tt) * 4);
+#pragma unroll
+      for (int st = 0; st < 4; ++st) x4[st] = static_cast<const float*>(a.out)[(size_t(tt) * 4 + st) * a.n + n];
+    } else if (a.kind == FB_EPI_SHARED_SCALE) {
+      gate = 1.0f / (1.0f + expf(-a.gate_logit[size_t(tt) * a.gate_stride]));
+    }
+  };
+  fetch();
+  if (cluster > 1) cluster_sync();
+  else __syncthreads();
+  for (int o = first; o < n_out;) {
+    const bool last = o + cluster * kSmallThreads >= n_out;
+    if (live) {
+      float sum = sum_of(tt, r), sum_up = swiglu ? sum_of(tt, r + 64) : 0.0f;
+      if (swiglu) {
+        const float g = sum * ws0, u = sum_up * ws1;
+        static_cast<__nv_bfloat16*>(a.out)[size_t(tt) * half_n + m * 64 + r] = __float2bfloat16_rn(g / (1.0f + expf(-g)) * u);
+      } else {
+        const int n = m * 128 + r;
+        const float val = sum * ws0 * gate;
+        if (a.kind == FB_EPI_GR_WRITE) {
+          float* xs = static_cast<float*>(a.out) + size_t(tt) * 4 * a.n + n;
+          xs[0] = fmaf(g4.x, val, x4[0]);
+          xs[size_t(a.n)] = fmaf(g4.y, val, x4[1]);
+          xs[2 * size_t(a.n)] = fmaf(g4.z, val, x4[2]);
+          xs[3 * size_t(a.n)] = fmaf(g4.w, val, x4[3]);
+        } else if (a.kind == FB_EPI_STORE_BF16) {
+          static_cast<__nv_bfloat16*>(a.out)[size_t(tt) * a.n + n] = __float2bfloat16_rn(val);
+        } else {
+          static_cast<float*>(a.out)[size_t(tt) * a.n + n] = val;  // StoreF32, SharedScale
+        }
+      }
+    }
+    if (last) break;
+    o += cluster * kSmallThreads;
+    tt = o / rows;
+    r = o - tt * rows;
+    live = swiglu ? m * 64 + r < half_n : m * 128 + r < a.n;
+    fetch();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (cluster > 1) cluster_sync();  // no CTA leaves while another may still read its partial tile
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 64);
+  }
+}
+
 // ------------------------------------------------------------------------------ host
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1189,6 +1465,40 @@ int pair_count() {
     cached[dev] = clusters;
   }
   return cached[dev];
+}
+
+// Clusters of 1..8 CTAs of fp8_small_kernel that can be resident at once with one CTA per multiprocessor (clusters do not
+// straddle GPCs, so this is less than multiprocessors / size); asked once per device. nullptr: the kernel cannot run.
+const int* small_clusters() {
+  static PerDeviceOnce once;
+  static int cached[64][kSmallMaxCluster + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  int* table = cached[dev];
+  const cudaError_t e = per_device_once(once, [&] {
+    const cudaError_t a = opt_in_smem(fp8_small_kernel, small_smem(kSmallMaxKb));
+    if (a != cudaSuccess) return a;
+    for (int cl = 1; cl <= kSmallMaxCluster; ++cl) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(unsigned(cl));
+      cfg.blockDim = dim3(kSmallThreads);
+      cfg.dynamicSmemBytes = 120 * 1024;  // one CTA per multiprocessor
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = unsigned(cl);
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, fp8_small_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      table[cl] = cl == 1 ? sm_count() : n;
+    }
+    return cudaSuccess;
+  });
+  return e == cudaSuccess ? table : nullptr;
 }
 
 }  // namespace
@@ -1356,12 +1666,8 @@ int32_t fb_linear_fp8_decode(const void* x_bf16, int32_t tokens, const uint8_t* 
     return int32_t(attr);
   }
   cudaStream_t s = as_stream(stream);
-  fp8_split_tokens_kernel<<<kDecTok, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x_bf16), tokens, k, pieces,
-                                                   tok_scale, tickets, n_tickets, status);
-  int32_t st = check_launch("linear_fp8_decode: split");
-  if (st) return st;
-  CUtensorMap map_w, map_p;
-  if (!make_map_u8(&map_w, w_codes, n, k, 64) || !make_map_u8(&map_p, pieces, kDecN, k, kDecN)) {
+  CUtensorMap map_w;
+  if (!make_map_u8(&map_w, w_codes, n, k, 64)) {
     set_error("linear_fp8_decode: cuTensorMapEncodeTiled failed");
     return int32_t(cudaErrorInvalidValue);
   }
@@ -1381,6 +1687,37 @@ int32_t fb_linear_fp8_decode(const void* x_bf16, int32_t tokens, const uint8_t* 
   a.tickets = tickets;
   a.status = status;
   const int m_tiles = kind == FB_EPI_SWIGLU ? ((n >> 1) + 63) / 64 : (n + 127) / 128;
+  // At most one row tile per multiprocessor: a cluster per tile, the largest (up to the portable size and one K block per
+  // CTA) of which as many as there are tiles are resident at once. (Above kSmallMaxKb blocks per CTA the operand rows do
+  // not fit. Fewer than four tiles, which no projection of the engine has, stay with the streaming kernel: its operand
+  // rows can be read back from the workspace.)
+  const int kb = k / BK;
+  if (m_tiles >= 4 && m_tiles <= sm_count()) {
+    const int* resident = small_clusters();
+    if (!resident) {
+      set_error("linear_fp8_decode: shared-memory opt-in failed");
+      return int32_t(cudaErrorInvalidConfiguration);
+    }
+    int cl = kb < kSmallMaxCluster ? kb : kSmallMaxCluster;
+    while (cl > 1 && resident[cl] < m_tiles) --cl;
+    const int nkb = (kb + cl - 1) / cl;
+    if (nkb <= kSmallMaxKb) {
+      const cudaError_t e = launch_pdl_cluster(fp8_small_kernel, dim3(unsigned(m_tiles * cl)), dim3(kSmallThreads),
+                                               size_t(small_smem(nkb)), s, unsigned(cl), map_w,
+                                               static_cast<const __nv_bfloat16*>(x_bf16), a, cl);
+      const int32_t launched = check_launch("linear_fp8_decode");
+      return launched ? launched : int32_t(e);
+    }
+  }
+  fp8_split_tokens_kernel<<<kDecTok, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x_bf16), tokens, k, pieces,
+                                                   tok_scale, tickets, n_tickets, status);
+  int32_t st = check_launch("linear_fp8_decode: split");
+  if (st) return st;
+  CUtensorMap map_p;
+  if (!make_map_u8(&map_p, pieces, kDecN, k, kDecN)) {
+    set_error("linear_fp8_decode: cuTensorMapEncodeTiled failed");
+    return int32_t(cudaErrorInvalidValue);
+  }
   const long long total = (long long)m_tiles * (k / BK);
   // Row tiles that nearly fill the GPU get one CTA each (whole tiles: no partial sums, whose ticketed
   // reduction costs more than the idle multiprocessors). Otherwise the K blocks are divided evenly,
