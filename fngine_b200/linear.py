@@ -1,6 +1,8 @@
 """Host-side mirror of the reference's FP8-row projection (linear_fp8, src/kernels/linear/linear.h
 of the reference): E4M3 weight codes with one scale per row, bf16 activations, bf16 output.
 Every call goes through the C ABI; torch only owns the device buffers."""
+import ctypes
+
 import torch
 
 from . import lib as L
@@ -14,6 +16,7 @@ class Fp8RowWeight:
         assert scales.is_cuda and scales.dtype in (torch.float32, torch.bfloat16) and scales.numel() == codes.shape[0]
         self.codes, self.scales = codes, scales.contiguous()
         self.n, self.k = codes.shape
+        self.scale_dtype = L.DT_BF16 if scales.dtype == torch.bfloat16 else L.DT_F32
 
 
 def linear_fp8_workspace(weight, max_tokens, device="cuda"):
@@ -28,13 +31,11 @@ def linear_fp8(x, weight, out, workspace, path=L.FP8_PATH_AUTO):
     store_f32, gr_write, swiglu, shared_scale) or, as a shorthand for store_bf16, a bf16 [T][n] tensor.
     path: FP8_PATH_AUTO / FP8_PATH_A16 = exact activations (the reference's default), FP8_PATH_A8 =
     one E4M3 code per activation (faster, 1-4 % rms noise)."""
-    import ctypes
     assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1] == weight.k
     epi = store_bf16(out) if isinstance(out, torch.Tensor) else out
-    dt = L.DT_BF16 if weight.scales.dtype == torch.bfloat16 else L.DT_F32
-    L.check(L.load().fb_linear_fp8(x.data_ptr(), x.shape[0], weight.codes.data_ptr(), weight.scales.data_ptr(), dt,
-                                   weight.n, weight.k, ctypes.byref(epi), workspace.data_ptr(), workspace.numel(),
-                                   torch.cuda.current_stream().cuda_stream, path), "linear_fp8")
+    L.check(L.load().fb_linear_fp8(x.data_ptr(), x.shape[0], weight.codes.data_ptr(), weight.scales.data_ptr(),
+                                   weight.scale_dtype, weight.n, weight.k, ctypes.byref(epi), workspace.data_ptr(), workspace.numel(),
+                                   L.stream(), path), "linear_fp8")
 
 
 def _epilogue(kind, gate_stride, out, inj=None, gate_logit=None):
@@ -88,12 +89,11 @@ def linear_fp8_decode(x, weight, epilogue, workspace):
     x bf16 [T][k]; the output is whatever `epilogue` (store_bf16, store_f32, gr_write, swiglu,
     shared_scale) names."""
     assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1] == weight.k
-    dt = L.DT_BF16 if weight.scales.dtype == torch.bfloat16 else L.DT_F32
-    import ctypes
-    L.check(L.load().fb_linear_fp8_decode(x.data_ptr(), x.shape[0], weight.codes.data_ptr(), weight.scales.data_ptr(),
-                                          dt, weight.n, weight.k, ctypes.byref(epilogue), workspace.data_ptr(),
-                                          workspace.numel(), torch.cuda.current_stream().cuda_stream),
-            "linear_fp8_decode")
+    st = L.load().fb_linear_fp8_decode(x.data_ptr(), x.shape[0], weight.codes.data_ptr(), weight.scales.data_ptr(),
+                                       weight.scale_dtype, weight.n, weight.k, ctypes.byref(epilogue),
+                                       workspace.data_ptr(), workspace.numel(), L.stream())
+    if st:
+        L.check(st, "linear_fp8_decode")
 
 
 def fp8_quantize_tokens(x):
@@ -102,7 +102,7 @@ def fp8_quantize_tokens(x):
     codes = torch.empty(T, k, dtype=torch.uint8, device=x.device)
     scales = torch.empty(T, dtype=torch.float32, device=x.device)
     L.check(L.load().fb_fp8_quantize_tokens(x.data_ptr(), T, k, codes.data_ptr(), scales.data_ptr(),
-                                            torch.cuda.current_stream().cuda_stream), "fp8_quantize_tokens")
+                                            L.stream()), "fp8_quantize_tokens")
     return codes, scales
 
 
@@ -113,5 +113,5 @@ def fp8_split_tokens(x):
     lo = torch.empty(T, k, dtype=torch.uint8, device=x.device)
     scales = torch.empty(T, dtype=torch.float32, device=x.device)
     L.check(L.load().fb_fp8_split_tokens(x.data_ptr(), T, k, hi.data_ptr(), lo.data_ptr(), scales.data_ptr(),
-                                         torch.cuda.current_stream().cuda_stream), "fp8_split_tokens")
+                                         L.stream()), "fp8_split_tokens")
     return hi, lo, scales

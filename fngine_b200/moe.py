@@ -23,8 +23,7 @@ def _ptr(t):
     return t
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = L.stream
 
 
 def _dtype_code(t):
