@@ -420,26 +420,33 @@ __device__ __forceinline__ void warp_topk10(LoadF load_logit, int* ids, float* w
 template <class LoadF>
 __device__ __forceinline__ void warp_topk10_pruned(LoadF load_logit, uint2* scratch, int* out_ids, float* out_w) {
   const int lane = threadIdx.x & 31;
-  uint32_t key[16];
+  float x[16];  // (fmaxf turns a NaN into -infinity; the keys are made for the candidates alone)
 #pragma unroll
-  for (int i = 0; i < 16; ++i) key[i] = logit_key(load_logit(lane + 32 * i));
-  uint32_t lm = key[0];
+  for (int i = 0; i < 16; ++i) x[i] = fmaxf(load_logit(lane + 32 * i), -INFINITY);
+  float lm = x[0];
 #pragma unroll
-  for (int i = 1; i < 16; ++i) lm = max(lm, key[i]);
+  for (int i = 1; i < 16; ++i) lm = fmaxf(lm, x[i]);
   int above = 0;  // lanes whose maximum is larger than this lane's
 #pragma unroll
   for (int j = 0; j < 32; ++j) above += __shfl_sync(0xffffffffu, lm, j) > lm ? 1 : 0;
-  const uint32_t thr = __reduce_min_sync(0xffffffffu, above < FB_TOPK ? lm : 0xffffffffu);
-  int total = 0;
-  const uint32_t below = (1u << lane) - 1u;
+  const float thr = key_logit(__reduce_min_sync(0xffffffffu, above < FB_TOPK ? logit_key(lm) : 0xffffffffu));
+  int mine = 0;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const bool in = key[i] >= thr;
-    const uint32_t m = __ballot_sync(0xffffffffu, in);
-    const int pos = total + __popc(m & below);
-    if (in && pos < 32) scratch[pos] = make_uint2(key[i], uint32_t(lane + 32 * i));
-    total += __popc(m);
+  for (int i = 0; i < 16; ++i) mine += x[i] >= thr ? 1 : 0;
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  int pos = incl - mine;  // (the candidates' order does not matter: they are ranked by key and id)
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (x[i] >= thr) {
+      if (pos < 32) scratch[pos] = make_uint2(logit_key(x[i]), uint32_t(lane + 32 * i));
+      ++pos;
+    }
   if (total > 32) {
     int ids[FB_TOPK];
     float w[FB_TOPK];

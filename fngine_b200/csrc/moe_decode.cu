@@ -17,6 +17,7 @@
 #include <cstring>
 
 #include <cuda_bf16.h>
+#include <cuda_fp8.h>
 
 namespace fb {
 namespace {
@@ -358,10 +359,12 @@ __device__ __forceinline__ void work_cache_fill(const fb_moe_decode_workspace& w
 // the tile and item counters of the streaming kernels (only where no such kernel can be running). The
 // list is a function of the logits alone: every block that runs this on the same logits builds the same
 // list. Every CTA of a decode step waits for this, so it is kept a short chain of six barriers: token
-// masks per physical slot (shared-memory atomics), a scan over the 512 slots (thread = slot), the pairs
-// placed from the scan, and the items ranked by a counting sort on their token counts (warp votes). Few
+// masks per physical slot (shared-memory atomics), one scan over the 512 slots (thread = slot), the items ranked by a
+// counting sort on their token counts (warp matches), and the pairs placed from the scan. Few
 // warps do this work and a warp on its own retires an instruction every few cycles: what counts here is the
-// number of instructions on the longest chain, not the arithmetic. (Up to three tokens: one warp, shuffles.)
+// number of instructions on the longest chain, not the arithmetic. (Up to three tokens: one warp, shuffles. Above, the
+// list took 4.0 us at sixteen tokens with two scans, every thread adding 32 warp totals and a ranking of 80 adds per
+// item.)
 //   items  = distinct selected experts held on this rank, in physical-slot order
 //   pairs  = (item, token), tokens ascending inside an item
 //   order  = items by token count, most first, ties by item index (the streaming kernels' visiting order)
@@ -369,19 +372,19 @@ template <class TopkF>
 __device__ __forceinline__ void select_block(TopkF topk, const int32_t* slot_of, int T,
                                              const fb_moe_decode_workspace& ws, uint32_t* counts, bool remote_ok,
                                              bool publish, bool reset, WorkCache& wc) {
-  static_assert(kMaxPairs % 32 == 0 && kMaxTok % 4 == 0, "the ranking below votes by whole warps and reads 16-byte groups");
+  static_assert(kExperts == 512 && kMaxTok == 16, "sixteen warps of slots, lanes 0..15 hold the token-count classes");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __shared__ int s_id[kMaxTok][kTopK];
   __shared__ float s_w[kMaxTok][kTopK];
   __shared__ int s_pair[kMaxTok][kTopK];
   __shared__ uint32_t s_tok[kExperts];  // physical slot -> mask of the tokens that chose it
   __shared__ int s_begin[kExperts];     // physical slot -> first pair of its item
-  __shared__ int s_scan[2][kExperts / 32];
-  __shared__ __align__(16) int s_item_cnt[kMaxPairs];
-  __shared__ __align__(16) int s_hist[kMaxPairs / 32][kMaxTok];  // [warp of items][token count - 1] -> items
+  __shared__ int s_scan[kExperts / 32];  // [warp of slots] -> its pairs | its items << 16
+  __shared__ int s_hist[kExperts / 32][kMaxTok + 1];  // [warp of slots][token count - 1] -> items (padded: no bank conflicts)
   __shared__ uint2 s_cand[kMaxTok][32];
   fb_moe_decode_work* work = ws.work;
   if (tid < kExperts) s_tok[tid] = 0;
+  if (tid < kExperts / 32 * (kMaxTok + 1)) (&s_hist[0][0])[tid] = 0;
   if (reset) {
     if (tid < kMaxPairs) ws.item_done[tid] = 0;
     if (tid < kSchedOrderBase) ws.sched[tid] = 0;
@@ -498,54 +501,66 @@ __device__ __forceinline__ void select_block(TopkF topk, const int32_t* slot_of,
     if (counts) atomicAdd(&counts[my_e], 1u);
   }
   __syncthreads();
-  // inclusive scans of (tokens, chosen flag) over the 512 slots: inside the warps first
+  // Thread = slot, sixteen warps. Inside the warps: inclusive scan of (pairs, items) in one word, and each item's place
+  // among the warp's items of as many tokens.
   const int c = tid < kExperts ? __popc(s_tok[tid]) : 0;
-  int incl_c = c, incl_n = c > 0 ? 1 : 0;
-  if (tid < kExperts) {  // (whole warps)
+  int incl = c | (c > 0 ? 1 << 16 : 0), peer_rank = 0;
+  if (warp < kExperts / 32) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, incl_c, o), y = __shfl_up_sync(0xffffffffu, incl_n, o);
-      if (lane >= o) {
-        incl_c += x;
-        incl_n += y;
-      }
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
     }
-    if (lane == 31) {
-      s_scan[0][warp] = incl_c;
-      s_scan[1][warp] = incl_n;
-    }
+    if (lane == 31) s_scan[warp] = incl;
+    const uint32_t peers = __match_any_sync(0xffffffffu, c);
+    peer_rank = __popc(peers & ((1u << lane) - 1u));
+    if (c > 0 && peer_rank == 0) s_hist[warp][c - 1] = __popc(peers);
   }
   __syncthreads();
-  int base_c = 0, base_n = 0, n_pairs = 0, n_items = 0;
+  if (warp < kExperts / 32) {
+    const int v = lane < kExperts / 32 ? s_scan[lane] : 0;
+    const int base = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0), total = __reduce_add_sync(0xffffffffu, v);
+    const int n_pairs = total & 0xFFFF, n_items = total >> 16;
+    // Visiting order: items with more tokens first, ties by item index. Lane = token count - 1: items of that count in
+    // all warps and in the warps before this one, then the items of larger counts.
+    int all = 0, before = 0;
 #pragma unroll
-  for (int i = 0; i < kExperts / 32; ++i) {
-    const int sc = s_scan[0][i], sn = s_scan[1][i];
-    base_c += i < warp ? sc : 0;
-    base_n += i < warp ? sn : 0;
-    n_pairs += sc;
-    n_items += sn;
-  }
-  if (c > 0) {  // thread = a chosen slot = an item
-    const int item = base_n + incl_n - 1, pair_begin = base_c + incl_c - c;
-    s_begin[tid] = pair_begin;
-    s_item_cnt[item] = c;
-    wc.slot[item] = tid;
-    wc.pair_begin[item] = pair_begin;
-    if (publish) {
-      work->item_slot[item] = tid;
-      work->item_pair_begin[item] = pair_begin;
+    for (int w = 0; w < kExperts / 32; ++w) {
+      const int h = s_hist[w][lane & 15];
+      all += h;
+      before += w < warp ? h : 0;
     }
-  }
-  if (tid == 0) {
-    wc.pair_begin[n_items] = n_pairs;
-    wc.n_items = n_items;
-    if (publish) {
-      work->item_pair_begin[n_items] = n_pairs;
-      work->n_items = n_items;
-      work->n_pairs = n_pairs;
-      work->n_cold = np - n_pairs;
-      work->tokens = T;
-      if (np - n_pairs && !remote_ok) atomicMax(ws.status, uint32_t(FB_STATUS_BAD_WORK));
+    int larger = lane < kMaxTok ? all : 0;
+#pragma unroll
+    for (int o = 1; o < kMaxTok; o <<= 1) {
+      const int x = __shfl_down_sync(0xffffffffu, larger, o);
+      larger += lane + o < kMaxTok ? x : 0;
+    }
+    const int order_base = __shfl_sync(0xffffffffu, larger - all + before, (c - 1) & 15);
+    if (c > 0) {  // a chosen slot = an item
+      const int first = base + incl;
+      const int item = (first >> 16) - 1, pair_begin = (first & 0xFFFF) - c, rank = order_base + peer_rank;
+      s_begin[tid] = pair_begin;
+      wc.slot[item] = tid;
+      wc.pair_begin[item] = pair_begin;
+      wc.order[rank] = item;
+      if (publish) {
+        work->item_slot[item] = tid;
+        work->item_pair_begin[item] = pair_begin;
+        ws.sched[kSchedOrderBase + rank] = item;
+      }
+    }
+    if (tid == 0) {
+      wc.pair_begin[n_items] = n_pairs;
+      wc.n_items = n_items;
+      if (publish) {
+        work->item_pair_begin[n_items] = n_pairs;
+        work->n_items = n_items;
+        work->n_pairs = n_pairs;
+        work->n_cold = np - n_pairs;
+        work->tokens = T;
+        if (np - n_pairs && !remote_ok) atomicMax(ws.status, uint32_t(FB_STATUS_BAD_WORK));
+      }
     }
   }
   __syncthreads();
@@ -564,42 +579,6 @@ __device__ __forceinline__ void select_block(TopkF topk, const int32_t* slot_of,
     if (publish) {
       work->topk_expert[pt][pk] = my_e;
       work->topk_weight[pt][pk] = s_w[pt][pk];
-    }
-  }
-  // Visiting order: rank of an item = items with more tokens + items with as many tokens and a lower index.
-  // A counting sort on the token count (1..16): every warp of items votes its histogram, then an item adds the
-  // counts above its own, the earlier warps' share of its own count, and its place among its warp's equals.
-  {
-    const bool live = tid < n_items;
-    const int mine = live ? s_item_cnt[tid] : 0;
-    uint32_t equals = 0;
-    if (tid < kMaxPairs) {  // (whole warps: kMaxPairs is a multiple of 32)
-#pragma unroll
-      for (int cnt = 1; cnt <= kMaxTok; ++cnt) {
-        const uint32_t b = __ballot_sync(0xffffffffu, mine == cnt);
-        equals = mine == cnt ? b : equals;
-        if (lane == cnt - 1) s_hist[warp][cnt - 1] = __popc(b);
-      }
-    }
-    __syncthreads();
-    if (live) {
-      int rank = __popc(equals & ((1u << lane) - 1u));
-#pragma unroll
-      for (int wv = 0; wv < kMaxPairs / 32; ++wv) {
-        const int4* hp = reinterpret_cast<const int4*>(s_hist[wv]);
-#pragma unroll
-        for (int g = 0; g < kMaxTok / 4; ++g) {
-          const int4 hv = hp[g];
-          const int hc[4] = {hv.x, hv.y, hv.z, hv.w};
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int cnt = 4 * g + i + 1;
-            rank += (cnt > mine || (cnt == mine && wv < warp)) ? hc[i] : 0;
-          }
-        }
-      }
-      wc.order[rank] = tid;
-      if (publish) ws.sched[kSchedOrderBase + rank] = tid;
     }
   }
   __syncthreads();
@@ -679,19 +658,40 @@ struct EpRouteArgs {
 // x slice of all tokens sits in the CTA's shared memory (sixteen CTAs read each slice: no line of x is
 // wanted by all SMs at once), one warp per row pair (every x value read from shared memory feeds two
 // rows), all tokens in flight at once. The eight slice sums of a logit meet through distributed shared
-// memory: after a cluster barrier CTA q adds the slices of rows 4q..4q+3 in order 0..7 (fixed: repeated
+// memory: after a cluster barrier (the activation quantization sits between its two halves) CTA q adds the slices of rows 4q..4q+3 in order 0..7 (fixed: repeated
 // calls are bitwise identical) and stores the logits. No block waits on device memory for another. Every
 // warp of the grid also quantizes a share of the activation blocks, and block 0 clears the counters of
 // the streaming kernels (none can be running: this kernel waited for its predecessor).
+//
+// With SHARED (the whole decode branch of a layer) the kernel also projects the shared expert's gate/up rows and router
+// row 512, its gate: cluster g takes inter_s / 16 (gate, up) row pairs the same way, FP8 codes widened exactly, and
+// stores h = bf16(silu(gate) * up). Five megabytes spread over 128 blocks that run anyway: as projections of their own
+// on a second stream they cost four launches, two events and, the expert kernel filling every multiprocessor, no overlap.
+struct SharedRouteArgs {
+  const uint8_t* codes;    // [2 inter_s][2560] E4M3
+  const void* scales;      // [2 inter_s], fp32 or bf16
+  int scale_bf16;
+  int inter_s;             // a multiple of 32, at most kSharedMaxInter
+  __nv_bfloat16* h;        // [tokens][inter_s]
+};
+constexpr int kSharedMaxInter = 1024;
+constexpr int kSharedRows = 2 * kSharedMaxInter / 16 + 4;  // of a cluster; the last four: router row 512 and nothing
+__device__ __forceinline__ float fp8_row_scale(const void* scales, int is_bf16, int row) {
+  return is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(scales)[row]) : static_cast<const float*>(scales)[row];
+}
+__device__ __forceinline__ float2 e4m3x2_float2(uint32_t pair) {
+  const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(pair), __NV_E4M3);
+  return __half22float2(*reinterpret_cast<const __half2*>(&hr));
+}
 constexpr int kRouteSplits = 8, kRouteSlice = H / kRouteSplits;  // 320
 constexpr int kRouteGroups = kExperts / 32;                      // 16
 constexpr int kRouteBlocks = kRouteGroups * kRouteSplits;
 static_assert(kRouteSlice == 320, "lane layout below: two 128-element chunks and a 64-element tail");
 
-template <bool XBF16, bool EP>
-__global__ void __launch_bounds__(512) route_kernel(const __nv_bfloat16* __restrict__ w, const void* __restrict__ xv,
+template <bool XBF16, bool EP, bool SHARED = false>
+__global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* __restrict__ w, const void* __restrict__ xv,
                                                     int T, float* __restrict__ logits, int stride,
-                                                    fb_moe_decode_workspace ws, EpRouteArgs ep) {
+                                                    fb_moe_decode_workspace ws, EpRouteArgs ep, SharedRouteArgs sh) {
   pdl_launch_dependents();
   pdl_wait_prior();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -739,74 +739,126 @@ __global__ void __launch_bounds__(512) route_kernel(const __nv_bfloat16* __restr
     }
     reinterpret_cast<float4*>(&s_x[t][0])[c] = v;
   }
-  const int row0 = g * 32 + 2 * warp;
-  float wr[2][10];  // lane holds elements 128c + 4 lane .. +3 (c = 0, 1) and 256 + 2 lane, +1 of the slice
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const __nv_bfloat16* wrow = w + size_t(row0 + r) * H + q * kRouteSlice;
+  __shared__ float s_sh[SHARED ? kSharedRows : 1][kMaxTok];
+  const int n_sh = SHARED ? sh.inter_s / 16 : 0;  // (gate, up) pairs of this cluster
+  // A warp takes four rows and half of the token slots: every value of x read from shared memory feeds four rows. (Two rows
+  // and all tokens per warp: 3 us instead of 1.5 at sixteen tokens, the shared-memory reads.) Lane holds elements
+  // 128c + 4 lane .. +3 (c = 0, 1) and 256 + 2 lane, +1 of the slice.
+  const int quad = warp >> 1, tok0 = (warp & 1) * (kMaxTok / 2);
+  float wr[4][10];
+  auto bf16_row = [&](int row, float (&v)[10]) {
+    const __nv_bfloat16* wrow = w + size_t(row) * H + q * kRouteSlice;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const uint2 u = reinterpret_cast<const uint2*>(wrow)[c * 32 + lane];
-      wr[r][4 * c + 0] = __uint_as_float(u.x << 16);
-      wr[r][4 * c + 1] = __uint_as_float(u.x & 0xFFFF0000u);
-      wr[r][4 * c + 2] = __uint_as_float(u.y << 16);
-      wr[r][4 * c + 3] = __uint_as_float(u.y & 0xFFFF0000u);
+      v[4 * c + 0] = __uint_as_float(u.x << 16);
+      v[4 * c + 1] = __uint_as_float(u.x & 0xFFFF0000u);
+      v[4 * c + 2] = __uint_as_float(u.y << 16);
+      v[4 * c + 3] = __uint_as_float(u.y & 0xFFFF0000u);
     }
     const uint32_t u = reinterpret_cast<const uint32_t*>(wrow + 256)[lane];
-    wr[r][8] = __uint_as_float(u << 16);
-    wr[r][9] = __uint_as_float(u & 0xFFFF0000u);
-  }
+    v[8] = __uint_as_float(u << 16);
+    v[9] = __uint_as_float(u & 0xFFFF0000u);
+  };
+  // Shared expert: a group = two (gate, up) pairs of this cluster = four rows; this lane's codes of group u
+  auto fp8_fetch = [&](int u, uint32_t (&v)[12]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint8_t* wrow = sh.codes + size_t((r & 1 ? sh.inter_s : 0) + g * n_sh + 2 * u + (r >> 1)) * H + q * kRouteSlice;
+      v[3 * r] = reinterpret_cast<const uint32_t*>(wrow)[lane];
+      v[3 * r + 1] = reinterpret_cast<const uint32_t*>(wrow)[32 + lane];
+      v[3 * r + 2] = reinterpret_cast<const uint16_t*>(wrow + 256)[lane];
+    }
+  };
+  auto fp8_widen = [&](const uint32_t (&v)[12]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float2 a = e4m3x2_float2(v[3 * r + c] & 0xFFFFu), b = e4m3x2_float2(v[3 * r + c] >> 16);
+        wr[r][4 * c + 0] = a.x;
+        wr[r][4 * c + 1] = a.y;
+        wr[r][4 * c + 2] = b.x;
+        wr[r][4 * c + 3] = b.y;
+      }
+      const float2 a = e4m3x2_float2(v[3 * r + 2]);
+      wr[r][8] = a.x;
+      wr[r][9] = a.y;
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < 4; ++r) bf16_row(g * 32 + 4 * quad + r, wr[r]);
   __syncthreads();
-  {
-    float acc[2 * kMaxTok];  // [row of the pair][token]
+  // the slice's sums of the four rows in wr over this warp's tokens -> dst[row][token]
+  auto project = [&](float (*dst)[kMaxTok]) {
+#pragma unroll 1
+    for (int tg = tok0; tg < min(tok0 + kMaxTok / 2, T); tg += 4) {  // (four at a time: registers)
+      float acc[16];  // [row][token of the group]
 #pragma unroll
-    for (int t = 0; t < kMaxTok; ++t) {
-      float a0 = 0.0f, a1 = 0.0f;
-      if (t < T) {
+      for (int t = 0; t < 4; ++t) {
+        float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (tg + t < T) {
+          const float* xr = &s_x[tg + t][0];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const float4 x4 = reinterpret_cast<const float4*>(&s_x[t][0])[c * 32 + lane];
-          a0 = fmaf(wr[0][4 * c + 0], x4.x, a0);
-          a1 = fmaf(wr[1][4 * c + 0], x4.x, a1);
-          a0 = fmaf(wr[0][4 * c + 1], x4.y, a0);
-          a1 = fmaf(wr[1][4 * c + 1], x4.y, a1);
-          a0 = fmaf(wr[0][4 * c + 2], x4.z, a0);
-          a1 = fmaf(wr[1][4 * c + 2], x4.z, a1);
-          a0 = fmaf(wr[0][4 * c + 3], x4.w, a0);
-          a1 = fmaf(wr[1][4 * c + 3], x4.w, a1);
+          for (int c = 0; c < 2; ++c) {
+            const float4 x4 = reinterpret_cast<const float4*>(xr)[c * 32 + lane];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              a[r] = fmaf(wr[r][4 * c + 0], x4.x, a[r]);
+              a[r] = fmaf(wr[r][4 * c + 1], x4.y, a[r]);
+              a[r] = fmaf(wr[r][4 * c + 2], x4.z, a[r]);
+              a[r] = fmaf(wr[r][4 * c + 3], x4.w, a[r]);
+            }
+          }
+          const float2 x2 = reinterpret_cast<const float2*>(xr + 256)[lane];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            a[r] = fmaf(wr[r][8], x2.x, a[r]);
+            a[r] = fmaf(wr[r][9], x2.y, a[r]);
+          }
         }
-        const float2 x2 = reinterpret_cast<const float2*>(&s_x[t][256])[lane];
-        a0 = fmaf(wr[0][8], x2.x, a0);
-        a1 = fmaf(wr[1][8], x2.x, a1);
-        a0 = fmaf(wr[0][9], x2.y, a0);
-        a1 = fmaf(wr[1][9], x2.y, a1);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[4 * r + t] = a[r];
       }
-      acc[t] = a0;
-      acc[kMaxTok + t] = a1;
-    }
-    // Sum over the 32 lanes by the butterfly xor 16, 8, 4, 2, 1, halving the values a lane carries
-    // at each step: 31 shuffles for the 32 (row, token) sums. Lane l ends with row l >> 4, token l & 15.
+      // Sum over the 32 lanes by the butterfly xor 16, 8, 4, 2, 1, halving the values a lane carries at each step but the
+      // last: 16 shuffles for the 16 (row, token) sums. Lanes 2i and 2i + 1 end with row i >> 2, token i & 3 of the group.
 #pragma unroll
-    for (int n = 16, o = 16; n >= 1; n >>= 1, o >>= 1) {
-      const bool hi = (lane & o) != 0;
+      for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool hi = (lane & o) != 0;
 #pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const float send = hi ? acc[i] : acc[i + n], keep = hi ? acc[i + n] : acc[i];
-        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        for (int i = 0; i < n; ++i) {
+          const float send = hi ? acc[i] : acc[i + n], keep = hi ? acc[i + n] : acc[i];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
       }
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+      if ((lane & 1) == 0) dst[lane >> 3][tg + ((lane >> 1) & 3)] = acc[0];
     }
-    s_part[2 * warp + (lane >> 4)][lane & 15] = acc[0];
-  }
-  cluster_sync();
-  if (tid < 4 * kMaxTok) {
-    const int r = 4 * q + (tid >> 4), t = tid & 15;
-    if (t < T) {
-      float v = 0.0f;
+  };
+  if constexpr (SHARED) {
+    // the next group's codes are on their way while the current one is projected
+    uint32_t codes[12];
+    const int groups = n_sh / 2;
+    if (quad < groups) fp8_fetch(quad, codes);
+    project(&s_part[4 * quad]);
+#pragma unroll 1
+    for (int u = quad; u < groups; u += 8) {
+      fp8_widen(codes);
+      if (u + 8 < groups) fp8_fetch(u + 8, codes);
+      project(&s_sh[4 * u]);
+    }
+    if (g == 0 && quad == 7) {  // router row 512, with three rows of nothing
+      bf16_row(kExperts, wr[0]);
 #pragma unroll
-      for (int qq = 0; qq < kRouteSplits; ++qq) v += ld_cluster_f32(&s_part[r][t], uint32_t(qq));
-      logits[size_t(t) * stride + g * 32 + r] = v;
+      for (int r = 1; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 10; ++i) wr[r][i] = 0.0f;
+      project(&s_sh[2 * n_sh]);
     }
+  } else {
+    project(&s_part[4 * quad]);
   }
+  cluster_arrive();
   // activation quantization, one warp per ggml block, strided over every warp of the grid (spread over
   // the blocks first: a single token's ten blocks go to ten different SMs)
   {
@@ -851,6 +903,39 @@ __global__ void __launch_bounds__(512) route_kernel(const __nv_bfloat16* __restr
         out[32 * b + q8_0_interleave_index(lane)] = uint8_t(int8_t(qv));
         if (lane == 0) scales[b] = __half2float(__ushort_as_half(dh));
       }
+    }
+  }
+  cluster_wait();
+  if (tid < 4 * kMaxTok) {
+    const int r = 4 * q + (tid >> 4), t = tid & 15;
+    if (t < T) {
+      float v = 0.0f;
+#pragma unroll
+      for (int qq = 0; qq < kRouteSplits; ++qq) v += ld_cluster_f32(&s_part[r][t], uint32_t(qq));
+      logits[size_t(t) * stride + g * 32 + r] = v;
+    }
+  }
+  if constexpr (SHARED) {
+    const int per = (n_sh + kRouteSplits - 1) / kRouteSplits;  // pairs this CTA finishes
+    for (int i = tid; i < per * kMaxTok; i += 512) {
+      const int p = q * per + (i >> 4), t = i & 15;
+      if (t >= T || p >= n_sh) continue;
+      float gv = 0.0f, uv = 0.0f;
+#pragma unroll
+      for (int qq = 0; qq < kRouteSplits; ++qq) {
+        gv += ld_cluster_f32(&s_sh[2 * p][t], uint32_t(qq));
+        uv += ld_cluster_f32(&s_sh[2 * p + 1][t], uint32_t(qq));
+      }
+      const int j = g * n_sh + p;
+      gv *= fp8_row_scale(sh.scales, sh.scale_bf16, j);
+      uv *= fp8_row_scale(sh.scales, sh.scale_bf16, sh.inter_s + j);
+      sh.h[size_t(t) * sh.inter_s + j] = __float2bfloat16_rn(gv / (1.0f + expf(-gv)) * uv);
+    }
+    if (g == 0 && q == kRouteSplits - 1 && tid < T) {
+      float v = 0.0f;
+#pragma unroll
+      for (int qq = 0; qq < kRouteSplits; ++qq) v += ld_cluster_f32(&s_sh[2 * n_sh][tid], uint32_t(qq));
+      logits[size_t(tid) * stride + kExperts] = v;
     }
   }
   cluster_sync();  // no CTA of the cluster leaves while another may still read its slice sums
@@ -922,17 +1007,16 @@ __device__ __forceinline__ void quantize_item_h(const fb_moe_decode_workspace& w
 constexpr int kItemReady = 0x40000000;
 __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_workspace& ws, int item, int pair_begin,
                                                        int n_tok, int expected, int down_act, int inter, int lane) {
-  __threadfence();
+  // (release and acquire ride on the two atomics: at one token this chain is a tenth of the layer)
   __syncwarp();
   int ticket = 0;
-  if (lane == 0) ticket = atomicAdd(&ws.item_done[item], 1);
+  if (lane == 0)
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(&ws.item_done[item]) : "memory");
   ticket = __shfl_sync(0xffffffffu, ticket, 0);
   if (ticket == expected - 1) {
-    __threadfence();
     quantize_item_h(ws, pair_begin, n_tok, down_act, inter);
-    __threadfence();
     __syncwarp();
-    if (lane == 0) atomicOr(&ws.item_done[item], kItemReady);
+    if (lane == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(&ws.item_done[item]), "r"(kItemReady) : "memory");
   }
 }
 
@@ -945,6 +1029,21 @@ __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_works
 // part; X[t][s][n] += inj[t][s] * y (4 residual streams) when X is given; y_out optional.
 // One block per (token, 256-column slice): the projection r . y_routed needs the whole row, so
 // with ablation a block first reduces the row (only then).
+// Column n of token t's partial rows, added in slot order; all loads in flight at once.
+__device__ __forceinline__ float sum_partials(const fb_moe_decode_workspace& ws, int t, int np, int n) {
+  int row[kTopK];
+  float v[kTopK];
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k) row[k] = k < np ? ws.work->token_pairs[t][k] : 0;
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k) v[k] = k < np ? ws.partial[size_t(row[k]) * H + n] : 0.0f;
+  float y = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k)
+    if (k < np) y += v[k];
+  return y;
+}
+
 __global__ void __launch_bounds__(256) combine_kernel(fb_moe_decode_workspace ws, const float* __restrict__ y_shared,
                                                       const float* __restrict__ inj, float* __restrict__ X,
                                                       float* __restrict__ y_out, const float* __restrict__ ablate,
@@ -977,14 +1076,120 @@ __global__ void __launch_bounds__(256) combine_kernel(fb_moe_decode_workspace ws
     proj = s_proj;
   }
   const int n = blockIdx.x * 256 + threadIdx.x;
-  float y = 0.0f;
-  for (int k = 0; k < np; ++k) y += ws.partial[size_t(work->token_pairs[t][k]) * H + n];
+  float y = sum_partials(ws, t, np, n);
   if (ablate) y -= ablate_scale * ablate[n] * proj;
   if (y_shared) y += y_shared[size_t(t) * H + n];
   if (y_out) y_out[size_t(t) * H + n] = y;
   if (X) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) X[(size_t(t) * 4 + s) * H + n] += inj[t * 4 + s] * y;
+  }
+}
+
+// The combine of the whole decode branch: the shared expert's down projection (y_shared[t][n] = sigmoid(gate logit) *
+// scale[n] * sum_k h[t][k] W[n][k], exact products, fp32 sums) for 16 columns and all tokens first, then their sums and
+// residual writes. The 1.6 MB of codes are read once, by 160 blocks; as a projection of its own in front of the combine
+// it took 6 us. Warp = two columns, lanes split K; h of all tokens in shared memory.
+struct SharedDownArgs {
+  const uint8_t* codes;  // [2560][k] E4M3
+  const void* scales;
+  int scale_bf16;
+  int k;                 // a multiple of 128
+  const __nv_bfloat16* h;
+  const float* logits;   // [tokens][stride], the gate in column 512
+  int stride;
+  float* y_shared;
+};
+constexpr int kCsCols = 16, kCsMaxK = kSharedMaxInter;
+__global__ void __launch_bounds__(256) combine_shared_kernel(fb_moe_decode_workspace ws, SharedDownArgs sh, int T,
+                                                             const float* __restrict__ inj, float* __restrict__ X,
+                                                             float* __restrict__ y_out) {
+  extern __shared__ __align__(16) float s_h[];  // [token][k]
+  __shared__ float s_y[kMaxTok][kCsCols];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n0 = blockIdx.x * kCsCols;
+  {  // on their way into L2 while the expert kernel finishes
+    const int bytes = kCsCols * sh.k;
+    for (int i = tid * 128; i < bytes; i += 256 * 128)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(sh.codes + size_t(n0) * sh.k + i));
+  }
+  pdl_wait_prior();
+  // Everything the block reads is asked for before it waits for any of it: its codes, its partial rows and residual
+  // streams (thread = token, column), then h.
+  constexpr int kChunks = kCsMaxK / 128;
+  const int chunks = sh.k / 128, t_out = tid >> 4, n = n0 + (tid & 15);
+  uint32_t codes[kChunks][2];
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c)
+    if (c < chunks) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        codes[c][r] = reinterpret_cast<const uint32_t*>(sh.codes + size_t(n0 + 2 * warp + r) * sh.k)[c * 32 + lane];
+    }
+  float routed = 0.0f, xs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (t_out < T) {
+    routed = sum_partials(ws, t_out, min(max(ws.work->token_pair_count[t_out], 0), kTopK), n);
+    if (X) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) xs[i] = X[(size_t(t_out) * 4 + i) * H + n];
+    }
+  }
+  for (int i = tid; i < T * sh.k / 8; i += 256) {
+    const uint4 u = reinterpret_cast<const uint4*>(sh.h)[i];
+    float4* d = reinterpret_cast<float4*>(s_h) + 2 * i;
+    d[0] = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xFFFF0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xFFFF0000u));
+    d[1] = make_float4(__uint_as_float(u.z << 16), __uint_as_float(u.z & 0xFFFF0000u), __uint_as_float(u.w << 16),
+                       __uint_as_float(u.w & 0xFFFF0000u));
+  }
+  __syncthreads();
+  float acc[32];  // [column of the warp][token]
+#pragma unroll
+  for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    if (c >= chunks) break;
+    float w[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float2 a = e4m3x2_float2(codes[c][r] & 0xFFFFu), b = e4m3x2_float2(codes[c][r] >> 16);
+      w[r][0] = a.x; w[r][1] = a.y; w[r][2] = b.x; w[r][3] = b.y;
+    }
+#pragma unroll
+    for (int t = 0; t < kMaxTok; ++t) {
+      if (t < T) {
+        const float4 hv = reinterpret_cast<const float4*>(s_h + t * sh.k)[c * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          acc[16 * r + t] = fmaf(w[r][3], hv.w, fmaf(w[r][2], hv.z, fmaf(w[r][1], hv.y, fmaf(w[r][0], hv.x, acc[16 * r + t]))));
+      }
+    }
+  }
+  // the butterfly of the route kernel: lane l ends with column l >> 4, token l & 15
+#pragma unroll
+  for (int m = 16, o = 16; m >= 1; m >>= 1, o >>= 1) {
+    const bool hi = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const float send = hi ? acc[i] : acc[i + m], keep = hi ? acc[i + m] : acc[i];
+      acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  {
+    const int t = lane & 15, col = 2 * warp + (lane >> 4);
+    if (t < T)
+      s_y[t][col] = acc[0] * fp8_row_scale(sh.scales, sh.scale_bf16, n0 + col) /
+                    (1.0f + expf(-sh.logits[size_t(t) * sh.stride + kExperts]));
+  }
+  __syncthreads();
+  if (t_out < T) {
+    const float ysh = s_y[t_out][tid & 15], y = routed + ysh;
+    sh.y_shared[size_t(t_out) * H + n] = ysh;
+    if (y_out) y_out[size_t(t_out) * H + n] = y;
+    if (X) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) X[(size_t(t_out) * 4 + i) * H + n] = xs[i] + inj[t_out * 4 + i] * y;
+    }
   }
 }
 
@@ -1275,8 +1480,8 @@ int32_t fb_moe_combine(const fb_moe_decode_workspace* ws, const float* y_shared,
 static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_layout* layout,
                                  const int32_t* slot_of, bool remote_ok, const void* x, int32_t x_dtype,
                                  int32_t tokens, const fb_moe_decode_workspace* ws, float* logits_scratch, float* y_out,
-                                 void* stream, const EpRouteArgs* ep = nullptr) {
-  const bool with_combine = ep == nullptr;
+                                 void* stream, const EpRouteArgs* ep = nullptr, const SharedRouteArgs* shared = nullptr) {
+  const bool with_combine = ep == nullptr && shared == nullptr;
   EpRouteArgs era{};
   if (ep) era = *ep;
   era.act = layout_ok(layout) ? act_of(layout->gate_up_format) : FB_ACT_Q8_K;
@@ -1297,9 +1502,10 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
   auto launch = [&](auto kernel) {
     return launch_pdl_cluster(kernel, grid, block, 0, as_stream(stream), unsigned(kRouteSplits),
                               static_cast<const __nv_bfloat16*>(router_w_bf16), x, tokens, logits_scratch,
-                              int(FB_ROUTER_ROWS), *ws, era);
+                              int(FB_ROUTER_ROWS), *ws, era, shared ? *shared : SharedRouteArgs{});
   };
   cudaError_t e = ep                       ? launch(route_kernel<false, true>)
+                  : shared                 ? launch(route_kernel<true, false, true>)
                   : x_dtype == FB_DT_BF16 ? launch(route_kernel<true, false>)
                                           : launch(route_kernel<false, false>);
   if (e != cudaSuccess) return check_launch("layer_decode: route");
@@ -1314,6 +1520,37 @@ int32_t fb_moe_layer_decode(const void* router_w_bf16, const fb_moe_expert_layou
                             float* y_out, void* stream) {
   return layer_decode_impl(router_w_bf16, layout, nullptr, false, x, x_dtype, tokens, ws, logits_scratch, y_out,
                            stream);
+}
+
+int32_t fb_moe_forward_decode(const void* router_w_bf16, const fb_moe_expert_layout* layout, const fb_shared_expert* shared,
+                              const void* x_bf16, int32_t tokens, const fb_moe_decode_workspace* ws, float* logits,
+                              const float* inj, float* X, float* y_out, void* stream) {
+  if (!shared || !shared->gate_up_codes || !shared->gate_up_scales || !shared->down_codes || !shared->down_scales ||
+      !shared->h_bf16 || !shared->y || tokens < 1 || tokens > kMaxTok || (X && !inj) || (!X && !y_out))
+    return invalid("forward_decode: bad arguments (tokens must be 1..16)");
+  if (shared->inter < 128 || shared->inter > kSharedMaxInter || shared->inter % 128)
+    return invalid("forward_decode: the shared expert's intermediate size must be a multiple of 128, at most %d", kSharedMaxInter);
+  if ((reinterpret_cast<uintptr_t>(shared->gate_up_codes) | reinterpret_cast<uintptr_t>(shared->down_codes) |
+       reinterpret_cast<uintptr_t>(shared->h_bf16) | reinterpret_cast<uintptr_t>(x_bf16)) & 15)
+    return invalid("forward_decode: x, weight codes and h must be 16-byte aligned");
+  const SharedRouteArgs ra{shared->gate_up_codes, shared->gate_up_scales, shared->gate_up_scales_dtype == FB_DT_BF16,
+                           shared->inter, static_cast<__nv_bfloat16*>(shared->h_bf16)};
+  const int32_t st = layer_decode_impl(router_w_bf16, layout, nullptr, false, x_bf16, FB_DT_BF16, tokens, ws, logits,
+                                       nullptr, stream, nullptr, &ra);
+  if (st) return st;
+  const SharedDownArgs da{shared->down_codes, shared->down_scales, shared->down_scales_dtype == FB_DT_BF16, shared->inter,
+                          static_cast<const __nv_bfloat16*>(shared->h_bf16), logits, int(FB_ROUTER_ROWS), shared->y};
+  static PerDeviceOnce once;
+  const cudaError_t attr =
+      per_device_once(once, [] { return opt_in_smem(combine_shared_kernel, size_t(kMaxTok) * kCsMaxK * 4); });
+  if (attr != cudaSuccess) {
+    set_error("forward_decode: shared-memory opt-in: %s", cudaGetErrorString(attr));
+    return int32_t(attr);
+  }
+  const cudaError_t e = launch_pdl(combine_shared_kernel, dim3(H / kCsCols), dim3(256), size_t(tokens) * shared->inter * 4,
+                                   as_stream(stream), *ws, da, tokens, inj, X, y_out);
+  if (e != cudaSuccess) return check_launch("forward_decode: combine");
+  return 0;
 }
 
 int32_t fb_moe_layer_decode_ep(const void* router_w_bf16, const fb_moe_expert_layout* layout,

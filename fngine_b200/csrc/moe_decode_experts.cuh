@@ -640,7 +640,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
                 give_up();
                 break;
               }
-              __nanosleep(200);
+              __nanosleep(50);
             }
             ready = true;
             // the rows were written by another SM's ordinary stores and are read by bulk copies

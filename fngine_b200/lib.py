@@ -68,6 +68,13 @@ class LinearEpilogue(C.Structure):
                 ("gate_logit", C.c_void_p)]
 
 
+class SharedExpert(C.Structure):
+    """fb_shared_expert: weights and intermediate buffers of a layer's shared expert."""
+    _fields_ = [("gate_up_codes", C.c_void_p), ("gate_up_scales", C.c_void_p), ("down_codes", C.c_void_p),
+                ("down_scales", C.c_void_p), ("h_bf16", C.c_void_p), ("y", C.c_void_p), ("gate_up_scales_dtype", C.c_int32),
+                ("down_scales_dtype", C.c_int32), ("inter", C.c_int32), ("reserved", C.c_int32)]
+
+
 EPI_STORE_BF16, EPI_STORE_F32, EPI_GR_WRITE, EPI_SWIGLU, EPI_SHARED_SCALE = range(5)
 FP8_PATH_AUTO, FP8_PATH_A16, FP8_PATH_A8 = range(3)
 
@@ -100,6 +107,8 @@ _SIGNATURES = {
     "fb_moe_layer_decode": (_I32, [_P, C.POINTER(ExpertLayout), _P, _I32, _I32, C.POINTER(DecodeWorkspace), _P, _P, _P]),
     "fb_moe_layer_decode_host": (_I32, [_P, C.POINTER(ExpertLayout), _P, _I32, _I32, C.POINTER(DecodeWorkspace), _P,
                                         _P, _P, _P, _P]),
+    "fb_moe_forward_decode": (_I32, [_P, C.POINTER(ExpertLayout), C.POINTER(SharedExpert), _P, _I32,
+                                     C.POINTER(DecodeWorkspace), _P, _P, _P, _P, _P]),
     "fb_moe_prefill_workspace_bytes": (C.c_size_t, [_I32, _I32]),
     "fb_moe_prefill_workspace_make": (_I32, [_P, _I32, _I32, C.POINTER(PrefillWorkspace)]),
     "fb_moe_route": (_I32, [_P, _I32, _P, _P, _I32, _P, _P, _I32, C.POINTER(PrefillWorkspace), _P]),

@@ -183,6 +183,27 @@ int32_t fb_moe_combine(const fb_moe_decode_workspace* ws, const float* y_shared,
 int32_t fb_moe_layer_decode(const void* router_w_bf16, const fb_moe_expert_layout* layout, const void* x,
                             int32_t x_dtype, int32_t tokens, const fb_moe_decode_workspace* ws, float* logits_scratch,
                             float* y_out, void* stream);
+/* The whole decode branch of Forward::moe (src/model/forward.cpp:333,356-376), shared expert included, in three launches:
+ * 513-row router and the shared expert's gate/up (its h goes to `h_bf16` [tokens][inter], the gate logit to column 512 of
+ * `logits`), the routed experts, and the combine with the shared expert's down projection (y [tokens][2560]) and the
+ * residual write. Weights as Fp8RowWeight (src/kernels/linear/linear.h:57-62): gate_up (2 inter, 2560), down (2560,
+ * inter), inter a multiple of 128 up to 1024. x is bf16; X [tokens][4][2560] with inj [tokens][4], or y_out, or both. No
+ * reference counterpart as a single function. */
+typedef struct fb_shared_expert {
+  const uint8_t* gate_up_codes;
+  const void* gate_up_scales;
+  const uint8_t* down_codes;
+  const void* down_scales;
+  void* h_bf16;
+  float* y;
+  int32_t gate_up_scales_dtype;
+  int32_t down_scales_dtype;
+  int32_t inter;
+  int32_t reserved;
+} fb_shared_expert;
+int32_t fb_moe_forward_decode(const void* router_w_bf16, const fb_moe_expert_layout* layout, const fb_shared_expert* shared,
+                              const void* x_bf16, int32_t tokens, const fb_moe_decode_workspace* ws, float* logits,
+                              const float* inj, float* X, float* y_out, void* stream);
 /* Same with HOST x and y: copies x in, runs the layer, copies y back and waits for it. `x_dev`
  * ([tokens][2560] of x_dtype) and `y_dev` (fp32) are caller-owned device staging buffers. */
 int32_t fb_moe_layer_decode_host(const void* router_w_bf16, const fb_moe_expert_layout* layout, const void* x_host,
