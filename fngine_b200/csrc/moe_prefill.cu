@@ -175,49 +175,76 @@ __global__ void __launch_bounds__(256) pf_import_kernel(const int32_t* __restric
 // Exclusive scan of the counts and the token-tile lists of both grouped GEMMs (one block of 512): tile = {expert, 0,
 // first pair, tokens}; a tile stands for inter / 128 (down: 2560 / 128) units of 128 weight rows, which the GEMM kernel
 // counts out itself. (Lists of units cost this single block 17 us at 8192 tokens.)
+// Tiles are listed by token count, most first (in steps of sixteen; a bucket's order is whatever the atomics give, results
+// do not depend on it): the GEMM's blocks take units in turn, and with tiles in expert order, a block's share of some forty
+// units of unequal cost was up to a sixth above the mean.
+constexpr int kTileBuckets = kTileN / 16;
+template <int TILE>
+__device__ __forceinline__ void list_tiles(int expert, int first_pair, int count, int* s_cursor, int4* __restrict__ tiles,
+                                           int max_tiles) {
+  const int full = count / TILE, rest = count - full * TILE;
+  if (full) {
+    const int at = atomicAdd(&s_cursor[0], full);
+    for (int t = 0; t < full; ++t)
+      if (at + t < max_tiles) tiles[at + t] = make_int4(expert, 0, first_pair + t * TILE, TILE);
+  }
+  if (rest) {
+    const int at = atomicAdd(&s_cursor[(TILE - rest) / 16], 1);
+    if (at < max_tiles) tiles[at] = make_int4(expert, 0, first_pair + full * TILE, rest);
+  }
+}
 __global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* __restrict__ count, int32_t* __restrict__ offset,
                                                       int32_t* __restrict__ cursor, int4* __restrict__ tiles_gu,
                                                       int4* __restrict__ tiles_dn, int32_t* __restrict__ meta,
                                                       int inter, int max_units_gu, int max_units_dn) {
-  __shared__ int s_scan[3][16];
+  __shared__ int s_scan[16];
+  __shared__ int s_bucket[2][kTileBuckets], s_cursor[2][kTileBuckets];  // bucket b: TILE - 16 b - 15 .. TILE - 16 b tokens
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < 2 * kTileBuckets) (&s_bucket[0][0])[tid] = 0;
   const int c = count[tid];
-  const int own[3] = {c, (c + kTileN - 1) / kTileN, (c + kTileNDown - 1) / kTileNDown};  // pairs, tiles of either kind
-  int incl[3] = {own[0], own[1], own[2]}, before[3] = {0, 0, 0}, total[3] = {0, 0, 0};
+  int incl = c;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += a;
+  }
+  if (lane == 31) s_scan[warp] = incl;
+  __syncthreads();
+  auto tally = [&](int tile, int* bucket) {
+    const int full = c / tile, rest = c - full * tile;
+    if (full) atomicAdd(&bucket[0], full);
+    if (rest) atomicAdd(&bucket[(tile - rest) / 16], 1);
+  };
+  tally(kTileN, s_bucket[0]);
+  tally(kTileNDown, s_bucket[1]);
+  int first = incl - c, total = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int a = __shfl_up_sync(0xffffffffu, incl[k], o);
-      if (lane >= o) incl[k] += a;
+  for (int i = 0; i < 16; ++i) {
+    first += i < warp ? s_scan[i] : 0;
+    total += s_scan[i];
+  }
+  offset[tid] = first;
+  cursor[tid] = 0;
+  __syncthreads();
+  const int mg = inter / kTileM, md = H / kTileM;
+  if (warp < 2) {  // warp k: list k
+    const int n = lane < kTileBuckets ? s_bucket[warp][lane] : 0;
+    int upto = n;
+#pragma unroll
+    for (int o = 1; o < kTileBuckets; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += a;
     }
-    if (lane == 31) s_scan[k][warp] = incl[k];
+    if (lane < kTileBuckets) s_cursor[warp][lane] = upto - n;
+    if (lane == kTileBuckets - 1) meta[warp] = min(upto * (warp ? md : mg), warp ? max_units_dn : max_units_gu);
+  }
+  if (tid == 0) {
+    offset[kExperts] = total;
+    meta[2] = total;
   }
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      before[k] += i < warp ? s_scan[k][i] : 0;
-      total[k] += s_scan[k][i];
-    }
-    before[k] += incl[k] - own[k];
-  }
-  offset[tid] = before[0];
-  cursor[tid] = 0;
-  const int mg = inter / kTileM, md = H / kTileM;
-  if (tid == 0) {
-    offset[kExperts] = total[0];
-    meta[0] = min(total[1] * mg, max_units_gu);
-    meta[1] = min(total[2] * md, max_units_dn);
-    meta[2] = total[0];
-  }
-  for (int t = 0; t < own[1]; ++t)
-    if ((before[1] + t + 1) * mg <= max_units_gu)
-      tiles_gu[before[1] + t] = make_int4(tid, 0, before[0] + t * kTileN, min(kTileN, c - t * kTileN));
-  for (int t = 0; t < own[2]; ++t)
-    if ((before[2] + t + 1) * md <= max_units_dn)
-      tiles_dn[before[2] + t] = make_int4(tid, 0, before[0] + t * kTileNDown, min(kTileNDown, c - t * kTileNDown));
+  list_tiles<kTileN>(tid, first, c, s_cursor[0], tiles_gu, max_units_gu / mg);
+  list_tiles<kTileNDown>(tid, first, c, s_cursor[1], tiles_dn, max_units_dn / md);
 }
 
 // Pairs grouped by expert. The order inside an expert depends on the atomics, the results do not:
@@ -260,47 +287,92 @@ __global__ void __launch_bounds__(256) ep_scatter_sum_kernel(const float* __rest
 
 // ------------------------------------------------------------------------------ combine
 // y[t][n] = sum over token t's ten pairs, in ascending expert id, of yp[pair][n] (+ shared);
-// X[t][s][n] += inj[t][s] * y when X is given.
-__global__ void __launch_bounds__(256) pf_combine_kernel(const int32_t* __restrict__ topk_e,
-                                                         const int32_t* __restrict__ token_pair,
-                                                         const float* __restrict__ yp, const float* __restrict__ y_shared,
-                                                         const float* __restrict__ inj, float* __restrict__ X,
-                                                         float* __restrict__ y_out, const long long* __restrict__ y_fixed) {
-  const int t = blockIdx.y;
+// X[t][s][n] += inj[t][s] * y when X is given. Bound: the ten rows per token from memory. One block per token, thread = four
+// columns, all ten 16-byte loads in flight (ten blocks per token with 4-byte loads: 198 us at 8192 tokens, 0.72 of the
+// copy rate).
+constexpr int kPcThreads = H / 4;  // 640
+template <bool ALIGNED>  // y_shared, X and y_out on 16-byte boundaries (single words otherwise)
+__device__ __forceinline__ float4 load4(const float* p) {
+  if constexpr (ALIGNED) return *reinterpret_cast<const float4*>(p);
+  else return make_float4(p[0], p[1], p[2], p[3]);
+}
+template <bool ALIGNED>
+__device__ __forceinline__ void store4(float* p, const float4& v) {
+  if constexpr (ALIGNED) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    p[0] = v.x;
+    p[1] = v.y;
+    p[2] = v.z;
+    p[3] = v.w;
+  }
+}
+template <bool ALIGNED>
+__global__ void __launch_bounds__(kPcThreads) pf_combine_kernel(const int32_t* __restrict__ topk_e,
+                                                                const int32_t* __restrict__ token_pair,
+                                                                const float* __restrict__ yp, const float* __restrict__ y_shared,
+                                                                const float* __restrict__ inj, float* __restrict__ X,
+                                                                float* __restrict__ y_out,
+                                                                const long long* __restrict__ y_fixed) {
+  const int t = blockIdx.x, n4 = threadIdx.x, lane = threadIdx.x & 31;
+  float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (y_fixed) {  // fixed-point sums: one rounding, the scale is exact (moe_y_fixed_to_float of the reference)
-    const int n = blockIdx.x * 256 + threadIdx.x;
-    float y = static_cast<float>(y_fixed[size_t(t) * H + n]) * (1.0f / 4294967296.0f);
-    if (y_shared) y += y_shared[size_t(t) * H + n];
-    if (y_out) y_out[size_t(t) * H + n] = y;
-    if (X) {
-#pragma unroll
-      for (int s = 0; s < 4; ++s) X[(size_t(t) * 4 + s) * H + n] += inj[t * 4 + s] * y;
+    const longlong2* f = reinterpret_cast<const longlong2*>(y_fixed + size_t(t) * H) + 2 * n4;
+    const longlong2 a = f[0], b = f[1];
+    constexpr float kScale = 1.0f / 4294967296.0f;
+    y = make_float4(float(a.x) * kScale, float(a.y) * kScale, float(b.x) * kScale, float(b.y) * kScale);
+  } else {
+    // Every warp orders the token's pairs by expert id (lane = list entry; the ids are distinct); entries without a local
+    // pair (expert-parallel shards) sort last.
+    int e = 0x7fffffff, pair = -1;
+    if (lane < kTopK) {
+      e = topk_e[t * kTopK + lane];
+      pair = token_pair[t * kTopK + lane];
+      if (e < 0) e = kExperts + lane;
     }
-    return;
-  }
-  __shared__ int s_order[kTopK];
-  if (threadIdx.x < kTopK) {
-    // ascending expert id; entries without a local pair (expert-parallel shards) sort last
-    auto key = [&](int k) {
-      const int e = topk_e[t * kTopK + k];
-      return e < 0 ? kExperts + k : e;
-    };
-    const int mine = key(threadIdx.x);
     int rank = 0;
-    for (int k = 0; k < kTopK; ++k) rank += key(k) < mine ? 1 : 0;
-    s_order[rank] = token_pair[t * kTopK + threadIdx.x];
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) rank += __shfl_sync(0xffffffffu, e, k) < e ? 1 : 0;
+    int row[kTopK];
+    float4 v[kTopK];
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) {
+      const uint32_t who = __ballot_sync(0xffffffffu, lane < kTopK && rank == k);
+      row[k] = __shfl_sync(0xffffffffu, pair, __ffs(who) - 1);
+    }
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k)
+      if (row[k] >= 0) v[k] = __ldcs(reinterpret_cast<const float4*>(yp + size_t(row[k]) * H) + n4);
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k)
+      if (row[k] >= 0) {
+        y.x += v[k].x;
+        y.y += v[k].y;
+        y.z += v[k].z;
+        y.w += v[k].w;
+      }
   }
-  __syncthreads();
-  const int n = blockIdx.x * 256 + threadIdx.x;
-  float y = 0.0f;
-#pragma unroll
-  for (int k = 0; k < kTopK; ++k)
-    if (s_order[k] >= 0) y += yp[size_t(s_order[k]) * H + n];
-  if (y_shared) y += y_shared[size_t(t) * H + n];
-  if (y_out) y_out[size_t(t) * H + n] = y;
+  if (y_shared) {
+    const float4 s = load4<ALIGNED>(y_shared + size_t(t) * H + 4 * n4);
+    y.x += s.x;
+    y.y += s.y;
+    y.z += s.z;
+    y.w += s.w;
+  }
+  if (y_out) store4<ALIGNED>(y_out + size_t(t) * H + 4 * n4, y);
   if (X) {
+    float4 x[4];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) X[(size_t(t) * 4 + s) * H + n] += inj[t * 4 + s] * y;
+    for (int s = 0; s < 4; ++s) x[s] = load4<ALIGNED>(X + (size_t(t) * 4 + s) * H + 4 * n4);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const float g = inj[t * 4 + s];
+      x[s].x += g * y.x;
+      x[s].y += g * y.y;
+      x[s].z += g * y.z;
+      x[s].w += g * y.w;
+      store4<ALIGNED>(X + (size_t(t) * 4 + s) * H + 4 * n4, x[s]);
+    }
   }
 }
 
@@ -536,8 +608,8 @@ int32_t fb_moe_grouped_gate_up(const fb_moe_expert_layout* layout, const uint8_t
   auto* xg = reinterpret_cast<__nv_bfloat16*>(ws->yp + size_t(ws->capacity) * kTopK * (H / 2));
   CUtensorMap map_b;
   if (const int32_t st = rows_map(&map_b, xg, H, ws->capacity, "grouped_gate_up")) return st;
-  gather_rows_kernel<<<min(8 * sm_count(), (tokens * kTopK + 7) / 8), 256, 0, as_stream(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x_bf16), ws->pair_token, ws->meta + 2, xg);
+  scatter_rows_kernel<<<(tokens + 7) / 8, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x_bf16),
+                                                                      ws->token_pair, tokens, xg);
   GgArgs a{};
   a.L = *layout;
   a.expert_blob = expert_blob;
@@ -592,7 +664,10 @@ int32_t fb_moe_prefill_combine(const fb_moe_prefill_workspace* ws, const float* 
   if (control) return invalid("prefill_combine: no CPU expert tier exists behind these kernels; control must be NULL");
   if (ablate_direction) return invalid("prefill_combine: the rank-1 ablation is not built for the prefill path");
   if (!pf_ws_ok(ws, tokens) || (X && !inj) || (!X && !y_out)) return invalid("prefill_combine: bad arguments");
-  pf_combine_kernel<<<dim3(H / 256, tokens), 256, 0, as_stream(stream)>>>(
+  const bool aligned = ((reinterpret_cast<uintptr_t>(y_shared) | reinterpret_cast<uintptr_t>(X) |
+                         reinterpret_cast<uintptr_t>(y_out)) & 15) == 0;
+  auto* kernel = aligned ? pf_combine_kernel<true> : pf_combine_kernel<false>;
+  kernel<<<tokens, kPcThreads, 0, as_stream(stream)>>>(
       ws->topk_expert, ws->token_pair, ws->yp, y_shared, inj, X, y_out,
       g_prefill_fixed ? reinterpret_cast<const long long*>(ws->yp) : nullptr);
   return check_launch("prefill_combine");

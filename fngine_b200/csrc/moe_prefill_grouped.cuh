@@ -13,7 +13,7 @@
 // stored swizzled tiles into a three-stage shared-memory ring: 8 weights per clock and SM.)
 //
 // The B operand comes by TMA from rows in pair order: h for the down projection; for gate/up the token rows are first
-// copied into that order (gather_rows_kernel). (Gathered by cp.async inside this kernel, a unit of 256 tokens cost
+// copied into that order (scatter_rows_kernel). (Gathered by cp.async inside this kernel, a unit of 256 tokens cost
 // 2048 load/store cycles per 256 K beside the decoding's thousand; by TMA gather, 52 cycles per four rows.)
 //
 // Roles: warp 0 issues the MMAs, warp 1 the TMA copies, two warps copy raw weight bytes with cp.async; 16 decoding
@@ -620,17 +620,23 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
   }
 }
 
-// Token rows in pair order: xg[p] = x[pair_token[p]], one warp per row. The whole pass is memory traffic: 100 us for
-// 81,920 rows (x stays in the L2 cache, the rows are written once).
-__global__ void __launch_bounds__(256) gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pair_token,
-                                                          const int32_t* __restrict__ n_pairs, __nv_bfloat16* __restrict__ xg) {
-  const int n = *n_pairs, lane = threadIdx.x & 31;
-  for (int p = blockIdx.x * 8 + (threadIdx.x >> 5); p < n; p += gridDim.x * 8) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + size_t(pair_token[p]) * H);
-    uint4* dst = reinterpret_cast<uint4*>(xg + size_t(p) * H);
-    uint4 v[H / 256];
+// Token rows in pair order: xg[p] = x[token of p]. One warp per token reads its row once and writes it to the token's
+// pairs: the writes (420 MB at 8192 tokens) are the cost. (A warp per pair took 100 us there.)
+__global__ void __launch_bounds__(256) scatter_rows_kernel(const __nv_bfloat16* __restrict__ x,
+                                                           const int32_t* __restrict__ token_pair, int tokens,
+                                                           __nv_bfloat16* __restrict__ xg) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= tokens) return;
+  const uint4* src = reinterpret_cast<const uint4*>(x + size_t(t) * H);
+  const int mine = lane < kTopK ? token_pair[t * kTopK + lane] : -1;
+  uint4 v[H / 256];
 #pragma unroll
-    for (int i = 0; i < H / 256; ++i) v[i] = __ldg(src + 32 * i + lane);
+  for (int i = 0; i < H / 256; ++i) v[i] = __ldg(src + 32 * i + lane);
+#pragma unroll
+  for (int k = 0; k < kTopK; ++k) {
+    const int p = __shfl_sync(0xffffffffu, mine, k);
+    if (p < 0) continue;  // a pair of another rank
+    uint4* dst = reinterpret_cast<uint4*>(xg + size_t(p) * H);
 #pragma unroll
     for (int i = 0; i < H / 256; ++i) dst[32 * i + lane] = v[i];
   }
