@@ -283,6 +283,29 @@ __device__ __forceinline__ int q8_0_block_warp(float v, unsigned short& d_half) 
   return int(roundf(__fmul_rn(v, id)));
 }
 
+// Eight Q8_0 blocks (256 values) by one warp: lane l holds elements 8l..8l+7 in v, four lanes a block. Same arithmetic as
+// q8_0_block_warp. Codes go to out[0..255] in the interleaved order (16-byte stores by two lanes of four), the fp16-rounded
+// scales widened to scales[0..7]. `live` = this lane's block exists (its four lanes agree).
+__device__ __forceinline__ void q8_0_eight_blocks_warp(const float (&v)[8], bool live, uint8_t* out, float* scales) {
+  const int lane = threadIdx.x & 31;
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  const float d = __fdiv_rn(amax, 127.0f);
+  const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+  uint32_t w[2] = {0u, 0u}, o[2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i >> 2] |= uint32_t(uint8_t(int8_t(int(roundf(__fmul_rn(v[i], id)))))) << (8 * (i & 3));
+#pragma unroll
+  for (int i = 0; i < 2; ++i) o[i] = __shfl_xor_sync(0xffffffffu, w[i], 2);
+  if (live && (lane & 2) == 0)  // elements e and, from the lane two up, e + 16
+    *reinterpret_cast<uint4*>(out + 32 * (lane >> 2) + 16 * (lane & 1)) =
+        make_uint4(prmt(w[0], o[0], 0x5140u), prmt(w[0], o[0], 0x7362u), prmt(w[1], o[1], 0x5140u), prmt(w[1], o[1], 0x7362u));
+  if (live && (lane & 3) == 0) scales[lane >> 2] = __half2float(__float2half_rn(d));
+}
+
 // ------------------------------------------------------------------------------ routing
 // Top-10 of 512 logits by one warp (lane l holds logits l + 32 i): value descending, ties to the
 // lower id, NaN never wins, -0 == +0; weights = softmax over the winners in fp32, summed in rank

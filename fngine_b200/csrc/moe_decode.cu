@@ -963,41 +963,36 @@ struct StageMeta {
   float wgt[kTT];  // routing weights of the pass's pairs (down)
 };
 
-// h of one finished work item -> planar activation rows for the down projection (one warp).
-__device__ __forceinline__ void quantize_item_h(const fb_moe_decode_workspace& ws, int pair_begin, int n_tok,
-                                                int down_act, int I) {
+// One row of h -> a planar activation row of the down projection, by the calling warp; all of the row's loads are in
+// flight before the first block is quantized (the finishing warp waits on this chain: Q8_0 rows taken block by block, twenty
+// round trips at 640, cost a layer of one token 8 us). `out` in global or shared memory, 16-byte aligned.
+template <int I>
+__device__ __forceinline__ void quantize_h_row(const float* __restrict__ h, int down_act, uint8_t* out) {
+  constexpr int kPasses = (I + 255) / 256;
   const int lane = threadIdx.x & 31;
-  for (int p = pair_begin; p < pair_begin + n_tok; ++p) {
-    const float* h = ws.h + size_t(p) * I;
-    uint8_t* out = ws.hq + size_t(p) * FB_HQ_STRIDE;
-    if (down_act == FB_ACT_Q8_K) {
-      for (int b0 = 0; b0 < I / 256; b0 += 2) {  // two blocks' loads in flight: the finishing warp waits on this chain
-        const int nb = min(2, I / 256 - b0);
-        float4 a[2], c[2];
+  float v[kPasses][8];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-          if (i < nb) {
-            a[i] = __ldcg(reinterpret_cast<const float4*>(h + 256 * (b0 + i) + 8 * lane));
-            c[i] = __ldcg(reinterpret_cast<const float4*>(h + 256 * (b0 + i) + 8 * lane) + 1);
-          }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-          if (i < nb) {
-            float v[8] = {a[i].x, a[i].y, a[i].z, a[i].w, c[i].x, c[i].y, c[i].z, c[i].w};
-            int q[8], ps;
-            const float d = q8k_block_warp(v, q, ps);
-            store_q8k_block_planar(out, I, b0 + i, q, ps, d);
-          }
-      }
-    } else {
-      float* scales = reinterpret_cast<float*>(out + I);
-      for (int b = 0; b < I / 32; ++b) {
-        unsigned short dh;
-        const int q = q8_0_block_warp(__ldcg(h + 32 * b + lane), dh);
-        out[32 * b + q8_0_interleave_index(lane)] = uint8_t(int8_t(q));
-        if (lane == 0) scales[b] = __half2float(__ushort_as_half(dh));
-      }
+  for (int p = 0; p < kPasses; ++p) {
+    const int e = 256 * p + 8 * lane;
+    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = a;
+    if (e < I) {
+      a = __ldcg(reinterpret_cast<const float4*>(h + e));
+      c = __ldcg(reinterpret_cast<const float4*>(h + e) + 1);
     }
+    v[p][0] = a.x; v[p][1] = a.y; v[p][2] = a.z; v[p][3] = a.w;
+    v[p][4] = c.x; v[p][5] = c.y; v[p][6] = c.z; v[p][7] = c.w;
+  }
+  if (I % 256 == 0 && down_act == FB_ACT_Q8_K) {
+#pragma unroll
+    for (int p = 0; p < kPasses; ++p) {
+      int q[8], ps;
+      const float d = q8k_block_warp(v[p], q, ps);
+      store_q8k_block_planar(out, I, p, q, ps, d);
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < kPasses; ++p)
+      q8_0_eight_blocks_warp(v[p], 256 * p + 8 * lane < I, out + 256 * p, reinterpret_cast<float*>(out + I) + 8 * p);
   }
 }
 
@@ -1005,8 +1000,9 @@ __device__ __forceinline__ void quantize_item_h(const fb_moe_decode_workspace& w
 // down projection and then sets kItemReady in the item's counter (a fused gate/up + down launch polls
 // it before staging the item's rows). `expected` = contributions per item.
 constexpr int kItemReady = 0x40000000;
+template <int I>
 __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_workspace& ws, int item, int pair_begin,
-                                                       int n_tok, int expected, int down_act, int inter, int lane) {
+                                                       int n_tok, int expected, int down_act, int lane) {
   // (release and acquire ride on the two atomics: at one token this chain is a tenth of the layer)
   __syncwarp();
   int ticket = 0;
@@ -1014,7 +1010,8 @@ __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_works
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(&ws.item_done[item]) : "memory");
   ticket = __shfl_sync(0xffffffffu, ticket, 0);
   if (ticket == expected - 1) {
-    quantize_item_h(ws, pair_begin, n_tok, down_act, inter);
+    for (int p = pair_begin; p < pair_begin + n_tok; ++p)
+      quantize_h_row<I>(ws.h + size_t(p) * I, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
     __syncwarp();
     if (lane == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(&ws.item_done[item]), "r"(kItemReady) : "memory");
   }

@@ -728,7 +728,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         s_misc[3 + s] = 0;
         mbar_arrive(&ring.empty[s]);
       }
-      item_contribution_done(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act, INTER, lane);
+      item_contribution_done<INTER>(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act, lane);
     } else {
       const float w0 = ring.meta[s].wgt[0], w1 = ring.meta[s].wgt[1];
 #pragma unroll
