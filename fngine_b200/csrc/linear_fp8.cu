@@ -721,10 +721,6 @@ __device__ __forceinline__ bool dec_wait(DecBars* b, uint64_t* bar, uint32_t par
   atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
   return false;
 }
-// Adds to the pending byte count of a barrier without arriving on it.
-__device__ __forceinline__ void mbar_expect_tx_only(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 // All `threads` threads of named barrier `id` learn whether every one of them passed `ok`.
 __device__ __forceinline__ bool named_bar_all(int id, int threads, bool ok) {
   uint32_t r;

@@ -58,7 +58,9 @@ __device__ __forceinline__ float2 ll_read(const uint4* line, uint32_t step, uint
   atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
   return make_float2(0.0f, 0.0f);
 }
-constexpr int kSchedInts = 256;
+// ws.sched behind the order: [token][down tile] finished partial tiles (the expert kernel's own combine)
+constexpr int kSchedParts = 192, kMaxDnTiles = H / 128;
+constexpr int kSchedInts = kSchedParts + kMaxTok * kMaxDnTiles;
 
 __host__ __device__ constexpr int act_row_bytes_planar(int act, int k) {
   return act == FB_ACT_Q8_K ? k + 64 : k + k / 8;
@@ -352,8 +354,16 @@ __device__ __forceinline__ void work_cache_fill(const fb_moe_decode_workspace& w
 }
 
 // ------------------------------------------------------------------------------ select
-// topk(t, scratch, ids, weights): the calling warp writes token t's top-10 (ids and softmax weights, rank
-// order) to ids / weights in shared memory; scratch = 32 entries of shared memory for that warp.
+struct SelectScratch {
+  uint2 cand[kMaxTok][32];               // a token's candidates: key, id
+  int id[kMaxTok][kTopK];
+  float w[kMaxTok][kTopK];
+  uint32_t tok[kExperts];                // physical slot -> mask of the tokens that chose it
+  int begin[kExperts];                   // physical slot -> first pair of its item
+  int hist[kExperts / 32][kMaxTok + 1];  // [warp of slots][token count - 1] -> items (padded: no bank conflicts)
+  int scan[kExperts / 32];               // [warp of slots] -> its pairs | its items << 16
+};
+// load(t, e): logit e of token t. `scratch`: shared memory that is free until the call returns.
 // Called by every thread of a block of 512 or more threads. The work list goes to `wc` in shared memory
 // (complete when the call returns) and, with `publish`, to the device work list as well; `reset` clears
 // the tile and item counters of the streaming kernels (only where no such kernel can be running). The
@@ -368,20 +378,14 @@ __device__ __forceinline__ void work_cache_fill(const fb_moe_decode_workspace& w
 //   items  = distinct selected experts held on this rank, in physical-slot order
 //   pairs  = (item, token), tokens ascending inside an item
 //   order  = items by token count, most first, ties by item index (the streaming kernels' visiting order)
-template <class TopkF>
-__device__ __forceinline__ void select_block(TopkF topk, const int32_t* slot_of, int T,
+template <class LoadF>
+__device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of, int T,
                                              const fb_moe_decode_workspace& ws, uint32_t* counts, bool remote_ok,
-                                             bool publish, bool reset, WorkCache& wc) {
+                                             bool publish, bool reset, WorkCache& wc, SelectScratch& scratch) {
   static_assert(kExperts == 512 && kMaxTok == 16, "sixteen warps of slots, lanes 0..15 hold the token-count classes");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ int s_id[kMaxTok][kTopK];
-  __shared__ float s_w[kMaxTok][kTopK];
-  __shared__ int s_pair[kMaxTok][kTopK];
-  __shared__ uint32_t s_tok[kExperts];  // physical slot -> mask of the tokens that chose it
-  __shared__ int s_begin[kExperts];     // physical slot -> first pair of its item
-  __shared__ int s_scan[kExperts / 32];  // [warp of slots] -> its pairs | its items << 16
-  __shared__ int s_hist[kExperts / 32][kMaxTok + 1];  // [warp of slots][token count - 1] -> items (padded: no bank conflicts)
-  __shared__ uint2 s_cand[kMaxTok][32];
+  __shared__ int s_pair[kMaxTok][kTopK];  // (block 0 reads it behind the last barrier)
+  auto& [s_cand, s_id, s_w, s_tok, s_begin, s_hist, s_scan] = scratch;
   fb_moe_decode_work* work = ws.work;
   if (tid < kExperts) s_tok[tid] = 0;
   if (tid < kExperts / 32 * (kMaxTok + 1)) (&s_hist[0][0])[tid] = 0;
@@ -389,7 +393,9 @@ __device__ __forceinline__ void select_block(TopkF topk, const int32_t* slot_of,
     if (tid < kMaxPairs) ws.item_done[tid] = 0;
     if (tid < kSchedOrderBase) ws.sched[tid] = 0;
   }
-  if (warp < T) topk(warp, s_cand[warp], s_id[warp], s_w[warp]);
+  // (One warp per token. All sixteen warps on each token's slices - maxima, threshold, candidates and ranking behind a
+  // barrier each - was slower at every batch: 3.3 against 2.5 us at one token, 6 against 3 at sixteen.)
+  if (warp < T) warp_topk10_pruned([&](int e) { return load(warp, e); }, s_cand[warp], s_id[warp], s_w[warp]);
   __syncthreads();
   const int np = T * kTopK;
   if (np <= 32) {
@@ -611,6 +617,7 @@ struct SelectArgs {
   const int32_t* slot_of;
   int tokens;
   int remote_ok;
+  float* y_out;  // not null: the kernel adds up the token's partial rows itself (every expert held here)
 };
 
 // Stand-alone selection (the reference's moe_select_publish): block 0 routes, blocks 1..T quantize
@@ -634,11 +641,9 @@ __global__ void __launch_bounds__(512) select_kernel(const float* __restrict__ l
     return;
   }
   __shared__ WorkCache s_work;  // the streaming kernels of this path read the device work list instead
-  select_block(
-      [&](int t, uint2* scratch, int* ids, float* wts) {
-        warp_topk10_pruned([&](int e) { return logits[size_t(t) * logits_stride + e]; }, scratch, ids, wts);
-      },
-      slot_of, T, ws, counts, false, true, true, s_work);
+  __shared__ SelectScratch s_scratch;
+  select_block([&](int t, int e) { return logits[size_t(t) * logits_stride + e]; },
+               slot_of, T, ws, counts, false, true, true, s_work, s_scratch);
 }
 
 // What route_kernel needs for an expert-parallel step with peer-memory exchange (n_ranks == 0: none).
@@ -717,6 +722,7 @@ __global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* __re
   if (blockIdx.x == 0) {
     if (tid < kMaxPairs) ws.item_done[tid] = 0;
     if (tid < kSchedOrderBase) ws.sched[tid] = 0;
+    if (tid < kMaxTok * kMaxDnTiles) ws.sched[kSchedParts + tid] = 0;
   }
   __shared__ __align__(16) float s_x[kMaxTok][kRouteSlice];  // x slice [token][320]
   __shared__ float s_part[32][kMaxTok];                       // this slice's sums [row of the group][token]
@@ -951,17 +957,27 @@ __global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* __re
 constexpr int kSchedGateUp = 0, kSchedDown = 1, kSchedOrder = kSchedOrderBase;
 
 // What the producer tells the consumers about the entry staged in a ring slot (shared memory).
-struct StageMeta {
-  int tile;        // -1: no more work
+struct alignas(16) StageMeta {
+  int seq;         // entry number of this CTA
+  int tile;        // entry kind: 0 gate/up, 1 down
   int pair0;       // first pair (row of h / partial) of this pass
   int ntp;         // tokens in this pass (1..kTT)
   int row0;        // first intermediate row (gate/up) or output row (down) of the tile
   int item;        // work item
   int item_pair0;  // first pair of the item
   int item_tok;    // tokens of the item
-  int seq;         // entry number of this CTA (the multi-stage rings check it)
   float wgt[kTT];  // routing weights of the pass's pairs (down)
+  __device__ __forceinline__ void store(int seq_, int tile_, int pair0_, int ntp_, int row0_, int item_, int item_pair0_,
+                                        int item_tok_, const float (&wgt_)[kTT]) {
+    const uint32_t a = smem_u32(this);
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a + 32), "f"(wgt_[0]), "f"(wgt_[1]) : "memory");
+    asm volatile("st.shared.v4.s32 [%0], {%1, %2, %3, %4};" ::"r"(a + 16), "r"(row0_), "r"(item_), "r"(item_pair0_),
+                 "r"(item_tok_)
+                 : "memory");
+    asm volatile("st.shared.v4.s32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(seq_), "r"(tile_), "r"(pair0_), "r"(ntp_) : "memory");
+  }
 };
+static_assert(kTT == 2 && sizeof(StageMeta) == 48, "three vector stores");
 
 // One row of h -> a planar activation row of the down projection, by the calling warp; all of the row's loads are in
 // flight before the first block is quantized (the finishing warp waits on this chain: Q8_0 rows taken block by block, twenty
@@ -1425,10 +1441,13 @@ int32_t fb_moe_hot_gate_up(const fb_moe_expert_layout* layout, int32_t tokens, c
 
 static int32_t launch_down(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream);
 
+static bool one_launch(const fb_moe_expert_layout* layout) {
+  return layout->down_format == FB_FMT_IQ4_NL || (layout->down_format == FB_FMT_IQ3_S && layout->gate_up_format == FB_FMT_IQ3_S);
+}
 // Both projections of every routed expert: one launch, but for a down format without a shared streaming kernel.
 static int32_t launch_experts(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream,
                               const SelectArgs* sel) {
-  if (layout->down_format == FB_FMT_IQ4_NL || (layout->down_format == FB_FMT_IQ3_S && layout->gate_up_format == FB_FMT_IQ3_S))
+  if (one_launch(layout))
     return launch_phases(layout, ws, kPhaseGateUp | kPhaseDown, stream, "hot_experts", sel);
   const int32_t st = launch_gate_up(layout, ws, stream, sel);
   return st ? st : launch_down(layout, ws, stream);
@@ -1506,9 +1525,10 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
                   : x_dtype == FB_DT_BF16 ? launch(route_kernel<true, false>)
                                           : launch(route_kernel<false, false>);
   if (e != cudaSuccess) return check_launch("layer_decode: route");
-  const SelectArgs sel{logits_scratch, int(FB_ROUTER_ROWS), slot_of, tokens, remote_ok ? 1 : 0};
+  const bool own_combine = with_combine && !slot_of && one_launch(layout);
+  const SelectArgs sel{logits_scratch, int(FB_ROUTER_ROWS), slot_of, tokens, remote_ok ? 1 : 0, own_combine ? y_out : nullptr};
   const int32_t st = launch_experts(layout, ws, stream, &sel);  // selection + both projections of every routed expert
-  if (st || !with_combine) return st;
+  if (st || !with_combine || own_combine) return st;
   return fb_moe_combine(ws, nullptr, nullptr, 0, nullptr, nullptr, nullptr, y_out, tokens, 0, nullptr, 0.0f, stream);
 }
 

@@ -286,7 +286,8 @@ struct ExpertsCfg {
   static_assert(kTableBytes % 16 == 0 && kSlot % 16 == 0 && kGuPart % 16 == 0 && kDnTile % 16 == 0 && kGuAct % 16 == 0 &&
                     kDnAct % 16 == 0 && H % kDnRows == 0 && kDnRows % 32 == 0 && 2 * (kDnRows / 32) <= kTasks,
                 "tile shapes, bulk-copy sizes");
-  static_assert(kSmem + 14592 <= 232448, "dynamic plus static shared memory of a block");
+  static_assert(sizeof(SelectScratch) <= kSlot * kStages, "the selection borrows the ring");
+  static_assert(kSmem + 9216 <= 232448, "dynamic plus static shared memory of a block");
 };
 // kPhaseSelect: the CTA builds the work list itself from the router logits (SelectArgs) instead of
 // reading the device work list a selection kernel left.
@@ -511,6 +512,60 @@ __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlL
     }
   }
 }
+// The combine of the fused layer call, by the warps that finish down tiles: a tile's rows of a token are counted, and the
+// warp that brings the last of the token's pairs adds the columns' partial rows in slot order (the order, hence the
+// bits, of combine_kernel). A launch of its own behind this kernel cost a layer of one token 4 us.
+template <int ROWS>
+__device__ __forceinline__ void combine_tile(const fb_moe_decode_workspace& ws, const SelectArgs& sel, const WorkCache& wc,
+                                             int pair0, int ntp, int r0, int lane, int* rows) {
+  int mine = 0;
+  if (lane < ntp) {  // release and acquire ride on the atomic; the warp's stores are ordered before it by the __syncwarp
+    int* counter = ws.sched + kSchedParts + wc.pair_token[pair0 + lane] * kMaxDnTiles + r0 / ROWS;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(mine) : "l"(counter) : "memory");
+  }
+  const int n_pairs = wc.pair_begin[wc.n_items];
+  for (int i = 0; i < ntp; ++i) {
+    const int before = __shfl_sync(0xffffffffu, mine, i);
+    if (before != kTopK - 1) continue;
+    const int t = wc.pair_token[pair0 + i];
+    int n = 0;
+    for (int b = 0; b < n_pairs; b += 32) {  // the token's pairs in pair order = slot order
+      const bool in = b + lane < n_pairs && wc.pair_token[b + lane] == t;
+      const uint32_t m = __ballot_sync(0xffffffffu, in);
+      if (in) rows[n + __popc(m & ((1u << lane) - 1u))] = b + lane;
+      n += __popc(m);
+    }
+    __syncwarp();
+    int row[kTopK];
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) row[k] = rows[k];
+    __syncwarp();
+    for (int c = 4 * lane; c < ROWS; c += 128) {
+      float4 v[kTopK];
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k)
+        v[k] = __ldcg(reinterpret_cast<const float4*>(ws.partial + size_t(row[k]) * H + r0 + c));
+      float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k) {
+        y.x += v[k].x;
+        y.y += v[k].y;
+        y.z += v[k].z;
+        y.w += v[k].w;
+      }
+      float* out = sel.y_out + size_t(t) * H + r0 + c;  // (any 4-byte alignment)
+      if ((reinterpret_cast<uintptr_t>(sel.y_out) & 15) == 0) {
+        *reinterpret_cast<float4*>(out) = y;
+      } else {
+        out[0] = y.x;
+        out[1] = y.y;
+        out[2] = y.z;
+        out[3] = y.w;
+      }
+    }
+  }
+}
+
 template <int GU, int DN, int INTER>
 __global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + 1) * 32, 1)
 experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, SelectArgs sel) {
@@ -526,6 +581,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   __shared__ StageMeta s_meta[S];
   __shared__ int s_misc[3 + S];  // [1..2] task tickets (even / odd blocks), [3..] finished tasks per slot
   __shared__ int s_end;
+  __shared__ int s_rows[C::kWarps][kTopK];
   __shared__ WorkCache s_work;
   RingN<S> ring{bars, bars + S, s_meta, &s_end};
 
@@ -542,11 +598,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 
   int n_items;
   if (phases & kPhaseSelect) {
-    select_block(
-        [&](int t, uint2* scratch, int* ids, float* wts) {
-          warp_topk10_pruned([&](int e) { return __ldcg(sel.logits + size_t(t) * sel.stride + e); }, scratch, ids, wts);
-        },
-        sel.slot_of, sel.tokens, ws, nullptr, sel.remote_ok != 0, blockIdx.x == 0, false, s_work);
+    select_block([&](int t, int e) { return __ldcg(sel.logits + size_t(t) * sel.stride + e); }, sel.slot_of, sel.tokens, ws,
+                 nullptr, sel.remote_ok != 0, blockIdx.x == 0, false, s_work, *reinterpret_cast<SelectScratch*>(stage0));
     n_items = s_work.n_items;
   } else {
     n_items = min(max(ws.work->n_items, 0), kMaxPairs);
@@ -555,6 +608,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   constexpr int gu_tpi = INTER / C::kGuRows;
   const int n_gu = (phases & kPhaseGateUp) ? n_items * gu_tpi : 0;
   const int n_dn = (phases & kPhaseDown) ? n_items * C::kDnTilesPerItem : 0;
+  const int down_act = act_of(L.down_format);
 
   if (warp == C::kWarps) {
     // ---------------- producer: one lane draws tiles (two steps ahead of their use) and issues their
@@ -564,6 +618,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       __syncwarp();
     }
     if (lane != 0) return;
+    fence_proxy_async();  // the selection used the ring's memory through ordinary accesses
     int* counter = ws.sched + ((phases & kPhaseGateUp) ? kSchedGateUp : kSchedDown);
     const int n_tiles = n_gu + n_dn;
     int i = 0;
@@ -586,6 +641,10 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       }
       return true;
     };
+    // With three slots, whatever lies between a slot's release and its next copy is lost streaming time (an exchange of a
+    // few values with the idle lanes of this warp here cost a sixteen-token layer 11 us of 84): an entry is made up before
+    // the wait, and behind it come the copies first, then the entry's description, then the arrival that publishes both.
+    int s = 0;
     // a block's first two tiles need no ticket; the counter hands out the tiles behind those
     const int first_ticket = 2 * int(gridDim.x);
     int next = int(blockIdx.x), next2 = int(blockIdx.x + gridDim.x);
@@ -602,33 +661,34 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       const int pb = s_work.pair_begin[item];
       const int ntok = s_work.pair_begin[item + 1] - pb;
       const uint8_t* blob = L.slots + int64_t(s_work.slot[item]) * L.blob_stride;
+      const uint8_t* w0 = blob + (down ? L.down_offset + size_t(sub) * C::kDnTile : L.gate_offset + size_t(sub) * C::kGuPart);
+      const uint8_t* w1 = blob + L.up_offset + size_t(sub) * C::kGuPart;  // (gate/up)
+      const int row0 = sub * (down ? C::kDnRows : C::kGuRows);
       bool ready = !down || !(phases & kPhaseGateUp);  // a down-only launch runs behind a finished gate/up launch
       for (int tok0 = 0; tok0 < ntok; tok0 += kTT, ++i) {
-        const int s = i % S;
-        if (!slot_free(s)) return;
-        const int ntp = min(kTT, ntok - tok0);
-        volatile StageMeta* m = &ring.meta[s];
-        m->seq = i;
-        m->tile = down ? 1 : 0;  // entry kind
-        m->pair0 = pb + tok0;
-        m->ntp = ntp;
-        m->row0 = sub * (down ? C::kDnRows : C::kGuRows);
-        m->item = item;
-        m->item_pair0 = pb;
-        m->item_tok = ntok;
-        for (int t = 0; t < kTT; ++t) m->wgt[t] = tok0 + t < ntok ? s_work.pair_weight[pb + tok0 + t] : 0.0f;
+        const int ntp = min(kTT, ntok - tok0), pair0 = pb + tok0;
+        float wgt[kTT];
+        const uint8_t* act[kTT];
+#pragma unroll
+        for (int t = 0; t < kTT; ++t) {
+          const int p = pair0 + (t < ntp ? t : 0);
+          wgt[t] = s_work.pair_weight[p];
+          act[t] = down ? ws.hq + size_t(p) * FB_HQ_STRIDE : xq_rows + size_t(s_work.pair_token[p]) * FB_XQ_STRIDE;
+        }
         uint8_t* st = stage0 + s * C::kSlot;
+        uint64_t* full = &ring.full[s];
+        StageMeta* m = const_cast<StageMeta*>(&ring.meta[s]);
+        if (!slot_free(s)) return;
         if (!down) {
-          mbar_expect_tx(&ring.full[s], uint32_t(2 * C::kGuPart + ntp * C::kGuAct));
-          const size_t off = size_t(sub) * C::kGuPart;
-          bulk_g2s(st, blob + L.gate_offset + off, C::kGuPart, &ring.full[s]);
-          bulk_g2s(st + C::kGuPart, blob + L.up_offset + off, C::kGuPart, &ring.full[s]);
-          for (int t = 0; t < ntp; ++t)
-            bulk_g2s(st + 2 * C::kGuPart + t * C::kGuAct,
-                     xq_rows + size_t(s_work.pair_token[pb + tok0 + t]) * FB_XQ_STRIDE, C::kGuAct, &ring.full[s]);
+          mbar_expect_tx_only(full, uint32_t(2 * C::kGuPart + ntp * C::kGuAct));
+          bulk_g2s(st, w0, C::kGuPart, full);
+          bulk_g2s(st + C::kGuPart, w1, C::kGuPart, full);
+#pragma unroll
+          for (int t = 0; t < kTT; ++t)
+            if (t < ntp) bulk_g2s(st + 2 * C::kGuPart + t * C::kGuAct, act[t], C::kGuAct, full);
         } else {
-          mbar_expect_tx(&ring.full[s], uint32_t(C::kDnTile + ntp * C::kDnAct));
-          bulk_g2s(st, blob + L.down_offset + size_t(sub) * C::kDnTile, C::kDnTile, &ring.full[s]);
+          mbar_expect_tx_only(full, uint32_t(C::kDnTile + ntp * C::kDnAct));
+          bulk_g2s(st, w0, C::kDnTile, full);
           if (!ready) {  // the item's h must have been re-quantized (bounded poll of its flag)
             const int* flag = ws.item_done + item;
             uint32_t tries = 0;
@@ -646,14 +706,17 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
             // the rows were written by another SM's ordinary stores and are read by bulk copies
             asm volatile("fence.proxy.async.global;" ::: "memory");
           }
-          for (int t = 0; t < ntp; ++t)
-            bulk_g2s(st + C::kDnTile + t * C::kDnAct, ws.hq + size_t(pb + tok0 + t) * FB_HQ_STRIDE, C::kDnAct,
-                     &ring.full[s]);
-          if (failed) {  // nobody will use the entry: see its copies land (bounded), then leave
-            mbar_wait_hint(&ring.full[s], (i / S) & 1);
-            return;
-          }
+#pragma unroll
+          for (int t = 0; t < kTT; ++t)
+            if (t < ntp) bulk_g2s(st + C::kDnTile + t * C::kDnAct, act[t], C::kDnAct, full);
         }
+        m->store(i, down ? 1 : 0, pair0, ntp, row0, item, pb, ntok, wgt);
+        mbar_arrive(full);
+        if (failed) {  // nobody will use the entry: see its copies land (bounded), then leave
+          mbar_wait_hint(full, (i / S) & 1);
+          return;
+        }
+        if (++s == S) s = 0;
       }
     }
     return;
@@ -667,7 +730,6 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   // off), odd blocks the other way round: two code paths. A warp keeps to one parity, and since warp w issues on
   // scheduler w % 4, each scheduler's instruction cache sees one path only.
   const int parity = warp & 1;
-  const int down_act = act_of(L.down_format);
   while (true) {
     int s, k;
     if (!draw_task_n<S, C::kTasks / 2>(ring, &s_misc[1 + parity], ws.status, lane, s, k)) break;
@@ -676,7 +738,15 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     const bool down = ring.meta[s].tile != 0;
     uint8_t* st = stage0 + s * C::kSlot;
     float term[kTT] = {0.0f, 0.0f};
-    if (!down) {
+    if constexpr (DN == FB_FMT_IQ3_S) {
+      // one copy of the decode for both projections: the two parities' loops fill the instruction cache as it is
+      const uint8_t* blk = down ? st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes
+                                : st + gu_row_off + task * C::kTaskBytes;
+      const uint8_t* act0 = st + (down ? C::kDnTile : 2 * C::kGuPart);
+      const int act_bytes = down ? C::kDnAct : C::kGuAct, act_k = down ? INTER : H, ablk = down ? parity : task;
+      if (parity == 0) gate_up_block_terms<GU, true>(blk, grid, sign_base, lv, act0, act_bytes, ablk, ntp, term, act_k);
+      else gate_up_block_terms<GU, false>(blk, grid, sign_base, lv, act0, act_bytes, ablk, ntp, term, act_k);
+    } else if (!down) {
       const uint8_t* blk = st + gu_row_off + task * C::kTaskBytes;
       const uint8_t* act0 = st + 2 * C::kGuPart;
       if constexpr (GU == FB_FMT_IQ4_NL) {
@@ -689,10 +759,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     } else if (k < C::kDnRows / 32) {
       const uint8_t* half = st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes;
       const uint8_t* act0 = st + C::kDnTile;
-      if constexpr (DN == FB_FMT_IQ3_S) {
-        if (parity == 0) gate_up_block_terms<GU, true>(half, grid, sign_base, lv, act0, C::kDnAct, 0, ntp, term, INTER);
-        else gate_up_block_terms<GU, false>(half, grid, sign_base, lv, act0, C::kDnAct, 1, ntp, term, INTER);
-      } else if constexpr (INTER == 512) {
+      if constexpr (INTER == 512) {
         iq4nl_task_terms<8, 0>(half, lv, act0, C::kDnAct, INTER, 8 * parity, ntp, term);
       } else if (parity == 0) {
         iq4nl_task_terms<10, 0>(half, lv, act0, C::kDnAct, INTER, 0, ntp, term);
@@ -745,6 +812,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         s_misc[3 + s] = 0;
         mbar_arrive(&ring.empty[s]);
       }
+      if (sel.y_out) combine_tile<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane, s_rows[warp]);
     }
   }
 }
