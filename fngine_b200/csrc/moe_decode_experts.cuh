@@ -265,9 +265,10 @@ struct GuFmt<FB_FMT_IQ3_XXS> { static constexpr int kBlock = 98, kTable = 256 * 
 template <>
 struct GuFmt<FB_FMT_IQ4_XS> { static constexpr int kBlock = 136, kTable = 0; };
 
+constexpr int kStaticSmem = 6144;  // the kernel's own shared variables, at most
 template <int GU, int DN, int INTER>
 struct ExpertsCfg {
-  static constexpr int kWarps = 24, kTasks = 10, kStages = 3, kInter = INTER;
+  static constexpr int kWarps = 24, kTasks = 10, kInter = INTER;
   static constexpr int kTaskBytes = GuFmt<GU>::kBlock;
   static constexpr int kGuRows = 16, kGuRowBytes = kTasks * kTaskBytes, kGuPart = kGuRows * kGuRowBytes;
   static constexpr int kDnTaskBytes = DN == FB_FMT_IQ3_S ? 110 : INTER / 64 * 18;  // half a row
@@ -278,16 +279,22 @@ struct ExpertsCfg {
   static constexpr int kGuBytes = 2 * kGuPart + kTT * kGuAct, kDnBytes = kDnTile + kTT * kDnAct;
   static constexpr int kSlot = kGuBytes > kDnBytes ? kGuBytes : kDnBytes;
   static constexpr int kDnTilesPerItem = H / kDnRows;
-  static constexpr int kPartialFloats = kStages * kTasks * kTT * 32;
   static constexpr int kTableBytes = GuFmt<GU>::kTable;
-  static constexpr size_t kSmem = size_t(kTableBytes) + size_t(kStages) * kSlot + kPartialFloats * 4 + 128;
+  static constexpr size_t smem_of(int stages) {
+    return size_t(kTableBytes) + size_t(stages) * (kSlot + kTasks * kTT * 32 * 4) + 128;
+  }
+  // 24 warps work on 2.4 tiles at a time, so of three slots little more than a half is in flight from memory: four where
+  // they fit (the formats without a table)
+  static constexpr int kStages = smem_of(4) + kStaticSmem <= 232448 ? 4 : 3;
+  static constexpr int kPartialFloats = kStages * kTasks * kTT * 32;
+  static constexpr size_t kSmem = smem_of(kStages);
   static_assert(DN == FB_FMT_IQ4_NL || (DN == FB_FMT_IQ3_S && GU == FB_FMT_IQ3_S && INTER == 512),
                 "IQ3_S down shares the gate/up codebook and needs whole blocks per half row");
   static_assert(kTableBytes % 16 == 0 && kSlot % 16 == 0 && kGuPart % 16 == 0 && kDnTile % 16 == 0 && kGuAct % 16 == 0 &&
                     kDnAct % 16 == 0 && H % kDnRows == 0 && kDnRows % 32 == 0 && 2 * (kDnRows / 32) <= kTasks,
                 "tile shapes, bulk-copy sizes");
   static_assert(sizeof(SelectScratch) <= kSlot * kStages, "the selection borrows the ring");
-  static_assert(kSmem + 9216 <= 232448, "dynamic plus static shared memory of a block");
+  static_assert(kSmem + kStaticSmem <= 232448, "dynamic plus static shared memory of a block");
 };
 // kPhaseSelect: the CTA builds the work list itself from the router logits (SelectArgs) instead of
 // reading the device work list a selection kernel left.
