@@ -147,7 +147,9 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t pair) {
 __global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfloat16* __restrict__ x, int K,
                                                                   uint8_t* __restrict__ codes,
                                                                   uint8_t* __restrict__ codes_lo,
-                                                                  float* __restrict__ scales) {
+                                                                  float* __restrict__ scales, uint32_t* status) {
+  pdl_launch_dependents();
+  if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;  // of the GEMM that follows
   const int t = blockIdx.x;
   const __nv_bfloat16* row = x + size_t(t) * K;
   __shared__ float s_red[8];
@@ -1400,6 +1402,207 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   }
 }
 
+// ------------------------------------------------------------------------------ middle widths
+// The GEMM where its output tiles do not fill the GPU (a few tens to a few hundred tokens, or a narrow matrix). Bound:
+// latency and the rate at which one CTA takes operands in; with 128 x 256 output tiles, 2560 x 6144 at 40 tokens ran on ten
+// multiprocessors for 73 us. Here 128 weight rows are the M side of the MMA and up to 256 tokens the N side, and K is
+// shared by the CTAs of a cluster, whose partial tiles meet through distributed shared memory as in fp8_small_kernel
+// (added in CTA order: repeated calls are bitwise identical).
+#ifndef MID_PAIR_NUM
+#define MID_PAIR_NUM 2
+#endif
+constexpr int kMidThreads = 512, kMidTok = 256, kMidMaxStages = 8;
+struct MidBars {
+  uint64_t full[kMidMaxStages], empty[kMidMaxStages];
+  uint64_t acc;
+  uint32_t tmem_base;
+  int abort;
+};
+constexpr int kMidSmemMax = 232448;
+// Shared memory of a stage (16 KB of weights, `pieces` tiles of `tok` tokens) and of the whole block; the partial tile
+// reuses the stages.
+inline int mid_stage(int pieces, int tok) { return kDecStageA + pieces * tok * BK; }
+inline int mid_smem(int pieces, int tok, int stages) {
+  const int ring = stages * mid_stage(pieces, tok), part = tok * 128 * 4;
+  return 1024 + (ring > part ? ring : part) + int(sizeof(MidBars)) + 16;
+}
+struct MidArgs {
+  int cluster, stages, tok;  // CTAs per unit, ring stages, token slots of a stage (a multiple of 32)
+  int m_tiles;
+};
+
+template <int PIECES>
+__global__ void __launch_bounds__(kMidThreads, 1)
+fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const GemmArgs a,
+               const MidArgs g) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cluster = g.cluster, S = g.stages;
+  const int unit = int(blockIdx.x) / cluster, rank = int(blockIdx.x) - unit * cluster;
+  const int tile = unit / g.m_tiles, m = unit - tile * g.m_tiles;
+  const int t0 = tile * kMidTok, nt = min(kMidTok, a.M - t0), n16 = (nt + 15) & ~15;
+  const bool swiglu = a.kind == FB_EPI_SWIGLU;
+  const int kbt = a.K / BK, kb0 = kbt * rank / cluster, nkb = kbt * (rank + 1) / cluster - kb0;
+  const int stage = kDecStageA + PIECES * g.tok * BK, half_n = a.N >> 1;
+  const int r0 = swiglu ? m * 64 : m * 128, r1 = swiglu ? half_n + m * 64 : m * 128 + 64;
+  float* part = reinterpret_cast<float*>(smem);  // [token][row], behind the last MMA
+  const int ring = S * stage, part_bytes = g.tok * 128 * 4;
+  MidBars* bars = reinterpret_cast<MidBars*>(smem + (ring > part_bytes ? ring : part_bytes));
+  pdl_launch_dependents();
+  if (tid == 0) {
+    for (int i = 0; i < kMidMaxStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    mbar_init(&bars->acc, 1);
+    bars->abort = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&bars->tmem_base, 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+    for (uint32_t i = 0; i < (1u << 21); ++i) {
+      if (mbar_try_wait_hint(bar, parity)) return true;
+      if ((i & 31u) == 31u && *reinterpret_cast<volatile int*>(&bars->abort)) return false;
+    }
+    *reinterpret_cast<volatile int*>(&bars->abort) = 1;
+    atomicMax(a.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+    return false;
+  };
+
+  bool done = true;
+  if (warp == 0) {
+    if (elect_one()) {
+      const int boxes = (nt + 31) >> 5;
+      auto weights = [&](int i) {
+        uint8_t* st = smem + (i % S) * stage;
+        tma_load_2d(st, &map_w, (kb0 + i) * BK, r0, &bars->full[i % S]);
+        tma_load_2d(st + 64 * BK, &map_w, (kb0 + i) * BK, r1, &bars->full[i % S]);
+      };
+      const uint32_t bytes = uint32_t(kDecStageA + PIECES * boxes * 32 * BK);
+      // the weights do not come from the kernel launched just before (the activation pieces do)
+      const int pre = min(nkb, S);
+      for (int i = 0; i < pre; ++i) {
+        mbar_expect_tx(&bars->full[i], bytes);
+        weights(i);
+      }
+      pdl_wait_prior();
+      for (int i = 0; i < nkb; ++i) {
+        if (i >= pre) {
+          if (!wait(&bars->empty[i % S], ((i / S) - 1) & 1)) break;
+          mbar_expect_tx(&bars->full[i % S], bytes);
+          weights(i);
+        }
+        uint8_t* xs = smem + (i % S) * stage + kDecStageA;
+#pragma unroll
+        for (int p = 0; p < PIECES; ++p)
+          for (int b = 0; b < boxes; ++b)
+            tma_load_2d(xs + (p * g.tok + 32 * b) * BK, &map_x, (kb0 + i) * BK, p * a.lo_row0 + t0 + 32 * b,
+                        &bars->full[i % S]);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      // D fp32, A and B E4M3, both K-major, M = 128, N = n16
+      const uint32_t idesc = (1u << 4) | (uint32_t(n16 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+      bool ok = true;
+      for (int i = 0; i < nkb; ++i) {
+        if (!(ok = wait(&bars->full[i % S], (i / S) & 1))) break;
+        uint8_t* st = smem + (i % S) * stage;
+        const uint64_t da = umma_desc_k128(smem_u32(st));
+#pragma unroll
+        for (int p = 0; p < PIECES; ++p) {
+          const uint64_t db = umma_desc_k128(smem_u32(st + kDecStageA + p * g.tok * BK));
+#pragma unroll
+          for (int k4 = 0; k4 < BK / 32; ++k4)
+            umma_f8(tmem_base, da + uint64_t(2 * k4), db + uint64_t(2 * k4), idesc, (i | p | k4) ? 1u : 0u);
+        }
+        if (i + S < nkb) umma_commit(&bars->empty[i % S]);
+      }
+      if (ok) umma_commit(&bars->acc);
+    }
+  }
+  __syncwarp();
+  pdl_wait_prior();  // (token scales, and nothing is written before the preceding kernels are done)
+  {
+    // ---------------- the partial tile into shared memory: lane quarter = warp % 4, its four warps take chunks of 16 tokens
+    const int q = warp & 3, rl = q * 32 + lane;
+    done = __all_sync(0xffffffffu, wait(&bars->acc, 0));
+    if (done) {
+      tc_fence_after();
+      for (int c0 = 16 * (warp >> 2); c0 < n16; c0 += 64) {
+        uint32_t c[16];
+        tmem_ld16_nowait(tmem_base + (uint32_t(q * 32) << 16) + uint32_t(c0), c);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (c0 + i < nt) part[(c0 + i) * 128 + rl] = __uint_as_float(c[i]);
+      }
+      tc_fence_before();
+    }
+  }
+  if (cluster > 1) cluster_sync();
+  else __syncthreads();
+  // ---------------- outputs, dealt out over the cluster's threads: consecutive threads, consecutive rows
+  auto sum_of = [&](int t, int r) -> float {
+    if (cluster == 1) return part[t * 128 + r];
+    float p[kSmallMaxCluster];
+#pragma unroll
+    for (int c = 0; c < kSmallMaxCluster; ++c) p[c] = c < cluster ? ld_cluster_f32(part + t * 128 + r, uint32_t(c)) : 0.0f;
+    float v = p[0];
+#pragma unroll
+    for (int c = 1; c < kSmallMaxCluster; ++c) v += p[c];  // (adding + 0.0 behind the last changes nothing)
+    return v;
+  };
+  auto row_scale = [&](int n) -> float {
+    return a.scale_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.w_scale)[n])
+                        : static_cast<const float*>(a.w_scale)[n];
+  };
+  const int rows = swiglu ? 64 : 128, r = tid & (rows - 1);  // a thread keeps its row (the stride is a multiple of it)
+  const int n = (swiglu ? m * 64 : m * 128) + r, limit = swiglu ? half_n : a.N;
+  if (n < limit) {
+    const float ws0 = row_scale(n), ws1 = swiglu ? row_scale(half_n + n) : 0.0f;
+    const int per = kMidThreads / rows;  // tokens per turn of a CTA
+#pragma unroll 2
+    for (int t = rank * per + tid / rows; t < nt; t += cluster * per) {
+      const int row = t0 + t;
+      const float sa = a.act_scale[row];
+      if (a.kind == FB_EPI_GR_WRITE) {
+        float* X = static_cast<float*>(a.out) + size_t(row) * 4 * a.N + n;
+        float x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = X[size_t(i) * a.N];
+        const float4 inj = *reinterpret_cast<const float4*>(a.inj + size_t(row) * 4);
+        const float v = sum_of(t, r) * sa * ws0;
+        X[0] = fmaf(inj.x, v, x[0]);
+        X[size_t(a.N)] = fmaf(inj.y, v, x[1]);
+        X[2 * size_t(a.N)] = fmaf(inj.z, v, x[2]);
+        X[3 * size_t(a.N)] = fmaf(inj.w, v, x[3]);
+      } else if (swiglu) {
+        const float gv = sum_of(t, r) * sa * ws0, uv = sum_of(t, r + 64) * sa * ws1;
+        static_cast<__nv_bfloat16*>(a.out)[size_t(row) * half_n + n] = __float2bfloat16_rn(gv / (1.0f + expf(-gv)) * uv);
+      } else if (a.kind == FB_EPI_STORE_BF16) {
+        static_cast<__nv_bfloat16*>(a.out)[size_t(row) * a.N + n] = __float2bfloat16_rn(sum_of(t, r) * sa * ws0);
+      } else {
+        float v = sum_of(t, r) * sa * ws0;
+        if (a.kind == FB_EPI_SHARED_SCALE) v /= 1.0f + expf(-a.gate_logit[size_t(row) * a.gate_stride]);
+        static_cast<float*>(a.out)[size_t(row) * a.N + n] = v;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (cluster > 1) cluster_sync();  // no CTA leaves while another may still read its partial tile
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 256);
+  }
+}
+
 // ------------------------------------------------------------------------------ host
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1507,7 +1710,7 @@ int32_t fb_fp8_quantize_tokens(const void* x_bf16, int32_t tokens, int32_t k, ui
   if (!x_bf16 || !codes || !scales || tokens <= 0 || k <= 0 || k % 8)
     return invalid("fp8_quantize_tokens: bad arguments (k must be a multiple of 8)");
   fp8_quantize_tokens_kernel<<<tokens, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x_bf16), k, codes,
-                                                                    nullptr, scales);
+                                                                    nullptr, scales, nullptr);
   return check_launch("fp8_quantize_tokens");
 }
 
@@ -1516,7 +1719,7 @@ int32_t fb_fp8_split_tokens(const void* x_bf16, int32_t tokens, int32_t k, uint8
   if (!x_bf16 || !codes_hi || !codes_lo || !scales || tokens <= 0 || k <= 0 || k % 8)
     return invalid("fp8_split_tokens: bad arguments (k must be a multiple of 8)");
   fp8_quantize_tokens_kernel<<<tokens, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x_bf16), k, codes_hi,
-                                                                    codes_lo, scales);
+                                                                    codes_lo, scales, nullptr);
   return check_launch("fp8_split_tokens");
 }
 
@@ -1551,7 +1754,7 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
   float* a_scales = reinterpret_cast<float*>(a_codes + align256(size_t(2) * size_t(tokens) * size_t(k)));
   uint32_t* status = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(a_scales) + align256(size_t(tokens) * 4));
   fp8_quantize_tokens_kernel<<<tokens, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x_bf16), k, a_codes,
-                                                                    a_lo, a_scales);
+                                                                    a_lo, a_scales, status);
   int32_t st = check_launch("linear_fp8: activation pieces");
   if (st) return st;
   static PerDeviceOnce once;
@@ -1560,20 +1763,27 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
     if (a == cudaSuccess) a = opt_in_smem(fp8_gemm_kernel<2>, kGemmSmem);
     if (a == cudaSuccess) a = opt_in_smem(fp8_gemm_pair_kernel<1>, kGemmSmem2);
     if (a == cudaSuccess) a = opt_in_smem(fp8_gemm_pair_kernel<2>, kGemmSmem2);
+    if (a == cudaSuccess) a = opt_in_smem(fp8_mid_kernel<1>, kMidSmemMax);
+    if (a == cudaSuccess) a = opt_in_smem(fp8_mid_kernel<2>, kMidSmemMax);
     return a;
   });
   if (attr != cudaSuccess) {
     set_error("linear_fp8: shared-memory opt-in: %s", cudaGetErrorString(attr));
     return int32_t(attr);
   }
-  cudaError_t e = cudaMemsetAsync(status, 0, 4, as_stream(stream));
-  if (e != cudaSuccess) return check_launch("linear_fp8: status clear");
   // Two-SM tiles (256 x 256 per CTA pair) once there are enough rows to fill them; the single-CTA
   // kernel (128 x 256) below that and when FB_FP8_SINGLE_CTA is set (for comparisons).
   static const bool force_single = getenv("FB_FP8_SINGLE_CTA") != nullptr;
   const bool pair = tokens >= BM2 && !force_single;
+  // Middle widths (fp8_mid_kernel): where fewer output tiles than half of the CTA pairs would run (below 256 tokens: than
+  // two waves of 128-row tiles).
+  const int m_tiles_mid = kind == FB_EPI_SWIGLU ? ((n >> 1) + 63) / 64 : (n + 127) / 128;
+  const int units = m_tiles_mid * ((tokens + kMidTok - 1) / kMidTok);
+  const int pair_work = ((tokens + BM2 - 1) / BM2) * (kind == FB_EPI_SWIGLU ? ((n >> 1) + 127) / 128 : (n + BN - 1) / BN);
+  const bool mid = !force_single && (pair ? MID_PAIR_NUM * pair_work <= pair_count() : units <= 2 * sm_count());
   CUtensorMap map_a, map_b;
-  if (!make_map_u8(&map_a, a_codes, int64_t(pieces) * tokens, k, 128) || !make_map_u8(&map_b, w_codes, n, k, 128)) {
+  if (!make_map_u8(&map_a, a_codes, int64_t(pieces) * tokens, k, mid ? 32 : 128) ||
+      !make_map_u8(&map_b, w_codes, n, k, mid ? 64 : 128)) {
     set_error("linear_fp8: cuTensorMapEncodeTiled failed");
     return int32_t(cudaErrorInvalidValue);
   }
@@ -1591,6 +1801,30 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
   ga.N = n;
   ga.K = k;
   ga.lo_row0 = tokens;
+  if (mid) {
+    const int* resident = small_clusters();
+    if (!resident) {
+      set_error("linear_fp8: shared-memory opt-in failed");
+      return int32_t(cudaErrorInvalidConfiguration);
+    }
+    const int kb = k / BK;
+    MidArgs g;
+    g.cluster = kb < kSmallMaxCluster ? kb : kSmallMaxCluster;
+    while (g.cluster > 1 && resident[g.cluster] < units) --g.cluster;
+    g.tok = ((tokens < kMidTok ? tokens : kMidTok) + 31) & ~31;
+    g.m_tiles = m_tiles_mid;
+    g.stages = (kb + g.cluster - 1) / g.cluster;
+    if (g.stages > kMidMaxStages) g.stages = kMidMaxStages;
+    while (g.stages > 1 && mid_smem(pieces, g.tok, g.stages) > kMidSmemMax) --g.stages;
+    const dim3 grid(unsigned(units * g.cluster)), block(kMidThreads);
+    const size_t smem = size_t(mid_smem(pieces, g.tok, g.stages));
+    const cudaError_t e = pieces == 2 ? launch_pdl_cluster(fp8_mid_kernel<2>, grid, block, smem, as_stream(stream),
+                                                           unsigned(g.cluster), map_a, map_b, ga, g)
+                                      : launch_pdl_cluster(fp8_mid_kernel<1>, grid, block, smem, as_stream(stream),
+                                                           unsigned(g.cluster), map_a, map_b, ga, g);
+    st = check_launch("linear_fp8");
+    return st ? st : int32_t(e);
+  }
   const int n_tiles = kind == FB_EPI_SWIGLU ? ((n >> 1) + 127) / 128 : (n + BN - 1) / BN;
   if (pair) {
     const int work = ((tokens + BM2 - 1) / BM2) * n_tiles;
