@@ -1408,9 +1408,6 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
 // multiprocessors for 73 us. Here 128 weight rows are the M side of the MMA and up to 256 tokens the N side, and K is
 // shared by the CTAs of a cluster, whose partial tiles meet through distributed shared memory as in fp8_small_kernel
 // (added in CTA order: repeated calls are bitwise identical).
-#ifndef MID_PAIR_NUM
-#define MID_PAIR_NUM 2
-#endif
 constexpr int kMidThreads = 512, kMidTok = 256, kMidMaxStages = 8;
 struct MidBars {
   uint64_t full[kMidMaxStages], empty[kMidMaxStages];
@@ -1528,6 +1525,13 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   }
   __syncwarp();
   pdl_wait_prior();  // (token scales, and nothing is written before the preceding kernels are done)
+  if (a.kind == FB_EPI_GR_WRITE && lane == 0 && m * 128 + 32 * (warp & 3) < a.N) {  // residual streams into L2 meanwhile
+    for (int t = rank * 4 + (warp >> 2); t < nt; t += cluster * 4)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const float*>(a.out) + (size_t(t0 + t) * 4 + i) * a.N + m * 128 +
+                                                     32 * (warp & 3)));
+  }
   {
     // ---------------- the partial tile into shared memory: lane quarter = warp % 4, its four warps take chunks of 16 tokens
     const int q = warp & 3, rl = q * 32 + lane;
@@ -1775,12 +1779,13 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
   // kernel (128 x 256) below that and when FB_FP8_SINGLE_CTA is set (for comparisons).
   static const bool force_single = getenv("FB_FP8_SINGLE_CTA") != nullptr;
   const bool pair = tokens >= BM2 && !force_single;
-  // Middle widths (fp8_mid_kernel): where fewer output tiles than half of the CTA pairs would run (below 256 tokens: than
-  // two waves of 128-row tiles).
+  // Middle widths (fp8_mid_kernel): where fewer output tiles than half of the CTA pairs would run (measured at 300 - 1003
+  // tokens: 1.3 - 2.2 times faster below that line, up to 2.4 times slower above it); below 256 tokens up to two waves of
+  // 128-row tiles.
   const int m_tiles_mid = kind == FB_EPI_SWIGLU ? ((n >> 1) + 63) / 64 : (n + 127) / 128;
   const int units = m_tiles_mid * ((tokens + kMidTok - 1) / kMidTok);
   const int pair_work = ((tokens + BM2 - 1) / BM2) * (kind == FB_EPI_SWIGLU ? ((n >> 1) + 127) / 128 : (n + BN - 1) / BN);
-  const bool mid = !force_single && (pair ? MID_PAIR_NUM * pair_work <= pair_count() : units <= 2 * sm_count());
+  const bool mid = !force_single && (pair ? 2 * pair_work <= pair_count() : units <= 2 * sm_count());
   CUtensorMap map_a, map_b;
   if (!make_map_u8(&map_a, a_codes, int64_t(pieces) * tokens, k, mid ? 32 : 128) ||
       !make_map_u8(&map_b, w_codes, n, k, mid ? 64 : 128)) {
