@@ -15,6 +15,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 namespace fb {
 namespace {
 
@@ -415,9 +417,9 @@ int32_t rows_map(CUtensorMap* map, void* rows, int width, int capacity, const ch
 template <int FMT, bool DOWN>
 cudaError_t launch_grouped(const GgArgs& a, const CUtensorMap& map_b, cudaStream_t stream) {
   static PerDeviceOnce once;
-  const cudaError_t e = per_device_once(once, [] { return opt_in_smem(grouped_kernel<FMT, DOWN>, gg_smem<FMT>()); });
+  const cudaError_t e = per_device_once(once, [] { return opt_in_smem(grouped_kernel<FMT, DOWN>, gg_smem<FMT, DOWN>()); });
   if (e != cudaSuccess) return e;
-  grouped_kernel<FMT, DOWN><<<sm_count(), kGgThreads, gg_smem<FMT>(), stream>>>(a, map_b);
+  grouped_kernel<FMT, DOWN><<<sm_count(), kGgThreads, gg_smem<FMT, DOWN>(), stream>>>(a, map_b);
   return cudaSuccess;
 }
 

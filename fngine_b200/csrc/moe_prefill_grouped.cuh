@@ -38,32 +38,46 @@ struct GgBars {
   int abort;
 };
 
-// Raw bytes of a round (256 weights) of one row in shared memory. IQ3_S: the 28 words that cover the 110-byte block,
-// 29 words apart (an odd number: 32 lanes reading the same word of 32 rows meet 32 banks). IQ4_NL: 144 bytes,
-// back to back (16-byte reads of eight neighbouring rows cover all banks).
 static __constant__ int8_t c_iq4nl_levels[16] = {FB_IQ4NL_LEVELS};
 
-template <int FMT>
+// Raw weight bytes in shared memory.
+// gate/up: a slot = one round (256 weights) of the unit's 128 rows, copied row piece by row piece. IQ3_S: the 28 words that
+//   cover a row's 110-byte block, 29 words apart (an odd number: 32 lanes reading the same word of 32 rows meet 32
+//   banks). IQ4_NL: 144 bytes, back to back (16-byte reads of eight neighbouring rows cover all banks).
+// down: a slot = the whole unit, 128 complete rows, which lie back to back in the matrix: one bulk copy. (Cut into pieces like
+//   gate/up, rows of 360 bytes came in 8-byte copies, and the copying warps were the pace: 382 us instead of 233 at 1003
+//   tokens.)
+template <int FMT, bool DOWN>
 struct GgRaw;
 template <>
-struct GgRaw<FB_FMT_IQ3_S> {
-  static constexpr int kPiece = 110, kPitch = 116, kSlots = 6;
+struct GgRaw<FB_FMT_IQ3_S, false> {
+  static constexpr int kPiece = 110, kPitch = 116, kSlots = 6, kSlot = kTileM * kPitch;
 };
 template <>
-struct GgRaw<FB_FMT_IQ4_NL> {
-  static constexpr int kPiece = 144, kPitch = 144, kSlots = 5;
+struct GgRaw<FB_FMT_IQ4_NL, false> {
+  static constexpr int kPiece = 144, kPitch = 144, kSlots = 5, kSlot = kTileM * kPitch;
+};
+template <>
+struct GgRaw<FB_FMT_IQ3_S, true> {
+  static constexpr int kPiece = 110, kPitch = 220, kSlots = 3, kSlot = kTileM * kPitch;  // (intermediate 512 only)
+};
+template <>
+struct GgRaw<FB_FMT_IQ4_NL, true> {
+  static constexpr int kPiece = 144, kPitch = 360, kSlots = 2, kSlot = kTileM * kPitch;  // (288-byte rows: pitch 288)
 };
 // IQ3_S selectors, 16 bits per index and lane: entry i of lane l at byte 64 i + 2 l. Two lanes share a bank, so a
 // warp's look-up takes two passes at most where one shared copy takes three to four.
 // IQ4_NL level pairs, entry b of lane l at byte 128 b + 4 l.
 template <int FMT>
 constexpr int kGgTableBytes = FMT == FB_FMT_IQ3_S ? 512 * 64 : 256 * 128;
-template <int FMT>
+template <int FMT, bool DOWN>
 constexpr int gg_smem() {
-  return 1024 + kGgBStages * kTileB + GgRaw<FMT>::kSlots * kTileM * GgRaw<FMT>::kPitch + kGgTableBytes<FMT> +
+  return 1024 + kGgBStages * kTileB + GgRaw<FMT, DOWN>::kSlots * GgRaw<FMT, DOWN>::kSlot + kGgTableBytes<FMT> +
          int(sizeof(GgBars)) + 64;
 }
-static_assert(gg_smem<FB_FMT_IQ3_S>() <= 232448 && gg_smem<FB_FMT_IQ4_NL>() <= 232448, "shared memory per block");
+static_assert(gg_smem<FB_FMT_IQ3_S, false>() <= 232448 && gg_smem<FB_FMT_IQ4_NL, false>() <= 232448 &&
+                  gg_smem<FB_FMT_IQ3_S, true>() <= 232448 && gg_smem<FB_FMT_IQ4_NL, true>() <= 232448,
+              "shared memory per block");
 
 __device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
   uint32_t v;
@@ -165,10 +179,7 @@ __device__ __forceinline__ void gg_decode_iq4nl(float d, const uint32_t (&q)[4],
 struct GgDecodeConst {
   uint32_t table, lane_pat;  // window address of the format's table, this lane's address bits in it
 };
-template <int FMT>
-struct GgStep;
-template <>
-struct GgStep<FB_FMT_IQ3_S> {
+struct GgStepIq3s {
   uint32_t qs[4], sg[2], qh, sc;
   float d;
   // `row` = the row's words of the round, `shift` = 2 if the block starts in the middle of the first word, pos = K step.
@@ -196,29 +207,50 @@ struct GgStep<FB_FMT_IQ3_S> {
                    c.lane_pat, out);
   }
 };
-template <>
-struct GgStep<FB_FMT_IQ4_NL> {
-  uint32_t w[9];  // two 18-byte blocks
-  __device__ __forceinline__ void load(uint32_t row, int, int pos) {
-    const uint32_t b = row + 36 * pos;
+// IQ4_NL: W words of the lane's row. gate/up fetches one K step (two 18-byte blocks, nine words) at a time; down both steps of
+// its half round (72 bytes) in wide loads: 16 bytes where rows keep that alignment, 8 for rows of 360 bytes. (Rows are 288
+// bytes apart there, single words of 32 rows meet in four banks. For gate/up, rows 144 bytes apart, the wide forms cost
+// registers and gained nothing.)
+template <int W>
+struct GgWords {
+  uint32_t w[W];
+  __device__ __forceinline__ void load_step(uint32_t b) {
     w[0] = lds_u32<0>(b); w[1] = lds_u32<4>(b); w[2] = lds_u32<8>(b); w[3] = lds_u32<12>(b); w[4] = lds_u32<16>(b);
     w[5] = lds_u32<20>(b); w[6] = lds_u32<24>(b); w[7] = lds_u32<28>(b); w[8] = lds_u32<32>(b);
   }
-  template <int HALF>
-  __device__ __forceinline__ void decode(const GgDecodeConst& c, uint32_t (&out)[16]) const {
-    if constexpr (HALF == 0) {
-      const uint32_t q[4] = {__funnelshift_r(w[0], w[1], 16), __funnelshift_r(w[1], w[2], 16),
-                             __funnelshift_r(w[2], w[3], 16), __funnelshift_r(w[3], w[4], 16)};
-      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[0] & 0xFFFFu))), q, c.table, c.lane_pat, out);
+  __device__ __forceinline__ void load_half(uint32_t row, int m, bool by16) {  // half m of the 144 bytes at `row`
+    if (by16) {
+      uint32_t v[20];
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v[4 * i]), "=r"(v[4 * i + 1]), "=r"(v[4 * i + 2]), "=r"(v[4 * i + 3])
+                     : "r"(row + 64 * m + 16 * i)
+                     : "memory");
+#pragma unroll
+      for (int i = 0; i < 18; ++i) w[i] = m ? v[i + 2] : v[i];
     } else {
-      const uint32_t q[4] = {w[5], w[6], w[7], w[8]};
-      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[4] >> 16))), q, c.table, c.lane_pat, out);
+#pragma unroll
+      for (int i = 0; i < 9; ++i)
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[2 * i]), "=r"(w[2 * i + 1]) : "r"(row + 72 * m + 8 * i) : "memory");
+    }
+  }
+  template <int B>  // block B of those fetched
+  __device__ __forceinline__ void decode(const GgDecodeConst& c, uint32_t (&out)[16]) const {
+    constexpr int k = 9 * B / 2;
+    if constexpr (B % 2 == 0) {
+      const uint32_t q[4] = {__funnelshift_r(w[k], w[k + 1], 16), __funnelshift_r(w[k + 1], w[k + 2], 16),
+                             __funnelshift_r(w[k + 2], w[k + 3], 16), __funnelshift_r(w[k + 3], w[k + 4], 16)};
+      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[k] & 0xFFFFu))), q, c.table, c.lane_pat, out);
+    } else {
+      const uint32_t q[4] = {w[k + 1], w[k + 2], w[k + 3], w[k + 4]};
+      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[k] >> 16))), q, c.table, c.lane_pat, out);
     }
   }
 };
 
 // ------------------------------------------------------------------------------ raw bytes into shared memory
-// One loader warp copies the pieces of 32 rows (`bytes` of each) into its part of a raw slot. row_at(r) = address of
+// gate/up: one loader warp copies the pieces of 32 rows (`bytes` of each) into its part of a raw slot. row_at(r) = address of
 // the piece of row r (IQ3_S: of the word that holds its first byte). Copy size: the largest the alignment allows; pieces two bytes off word alignment (an expert
 // table may hold any even address) go through registers. Returns true if the copies are asynchronous.
 template <int B, class RowF>
@@ -232,19 +264,19 @@ __device__ __forceinline__ void gg_copy_pieces(uint32_t dst, int pitch, int byte
 }
 template <int FMT, class RowF>
 __device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t align, int lane, const uint8_t* base,
-                                            const int (&piece)[9], uint32_t short_mask, RowF row_at) {
+                                            const int (&piece)[9], RowF row_at) {
   if constexpr (FMT == FB_FMT_IQ3_S) {
     // 28 words from the word that holds the block's first byte (never one that starts behind the matrix)
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
       if (lane < 28)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + r * GgRaw<FMT>::kPitch + 4 * lane),
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + r * GgRaw<FMT, false>::kPitch + 4 * lane),
                      "l"(row_at(r) + 4 * lane)
                      : "memory");
     }
     return true;
   } else {
-    constexpr int P = GgRaw<FMT>::kPitch;
+    constexpr int P = GgRaw<FMT, false>::kPitch;
     if ((align & 15u) == 0 && bytes == P) {
       // 16-byte pieces, nine per row: piece id -> shared-memory byte 16 id. `piece[i]` = where this lane's i-th piece
       // lies from the first row's, the same for every round: recomputing it made the two loader warps, which get an
@@ -252,18 +284,6 @@ __device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t al
 #pragma unroll
       for (int i = 0; i < 9; ++i)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * lane + 512 * i), "l"(base + piece[i]) : "memory");
-    } else if ((align & 15u) == 8) {
-      // rows of 360 bytes: 8-byte pieces, eighteen per row, sixteen rows per nine instructions; a short last round
-      // keeps the first nine of each row
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const uint8_t* b = hf ? row_at(16) : base;
-#pragma unroll
-        for (int i = 0; i < 9; ++i)
-          if (bytes == P || ((short_mask >> i) & 1u))
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8 * lane + 256 * i + 16 * P * hf),
-                         "l"(b + piece[i]) : "memory");
-      }
     } else if ((align & 7u) == 0) {
       gg_copy_pieces<8>(dst, P, bytes, lane, row_at);
     } else if ((align & 3u) == 0) {
@@ -302,13 +322,13 @@ struct GgArgs {
 template <int FMT, bool DOWN>
 __global__ void __launch_bounds__(kGgThreads, 1)
 grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
-  using R = GgRaw<FMT>;
+  using R = GgRaw<FMT, DOWN>;
   constexpr bool kIq3s = FMT == FB_FMT_IQ3_S;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* ringb = smem;
   uint8_t* rawb = smem + kGgBStages * kTileB;
-  uint8_t* table = rawb + R::kSlots * kTileM * R::kPitch;
+  uint8_t* table = rawb + R::kSlots * R::kSlot;
   GgBars* bars = reinterpret_cast<GgBars*>(table + kGgTableBytes<FMT>);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int I = A.L.inter;
@@ -342,8 +362,8 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
       mbar_init(&bars->a_empty[i], 1);
     }
     for (int i = 0; i < R::kSlots; ++i) {
-      mbar_init(&bars->raw_full[i], 32 * kGgRawWarps);
-      mbar_init(&bars->raw_empty[i], 8);
+      mbar_init(&bars->raw_full[i], DOWN ? 1 : 32 * kGgRawWarps);
+      mbar_init(&bars->raw_empty[i], DOWN ? kGgDecodeWarps : 8);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->acc_full[i], 1);
@@ -438,89 +458,115 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
       }
     }
   } else if (warp < kGgFirstDecode) {
-    // ---------------- raw weight bytes, up to three rounds ahead of the decoding; a warp copies 64 of the 128 rows
-    constexpr int kRows = kTileM / kGgRawWarps;
-    const int row0 = kRows * (warp - 2);
-    int piece[9] = {};  // IQ4_NL, see gg_load_raw
-    uint32_t short_mask = 0;
-    if constexpr (!kIq3s) {
-      const int per_row = row_bytes % 16 == 0 ? 9 : 18, bytes = 144 / per_row;
-#pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        const int id = lane + 32 * i, r = id / per_row, c = id - per_row * r;
-        piece[i] = bytes * c + (DOWN ? r * row_bytes : (r >> 1) * row_bytes + ((r & 1) ? int(A.L.up_offset - A.L.gate_offset) : 0));
-        short_mask |= (c < 9 ? 1u : 0u) << i;
-      }
-    }
-    uint32_t rcount = 0;
-    int4 un = unit_or_none(blockIdx.x), un_next;
-    bool ok = true;
-    for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, un = un_next) {
-      un_next = unit_or_none(u + gridDim.x);
-      const uint8_t* blob = blob_of(un.x);
-      const uint8_t* rg = DOWN ? blob + A.L.down_offset + size_t(un.y + row0) * row_bytes  // first gate (down) row
-                               : blob + A.L.gate_offset + size_t(un.y + row0 / 2) * row_bytes;
-      const uint8_t* rup = DOWN ? rg : blob + A.L.up_offset + size_t(un.y + row0 / 2) * row_bytes;  // first up row
-      for (int rd = 0; rd < rounds; ++rd, ++rcount) {
-        const uint32_t s = rcount % R::kSlots;
-        if (!(ok = ab.wait_warp(&bars->raw_empty[s], ((rcount / R::kSlots) & 1) ^ 1))) break;
-        const int off = rd * R::kPiece;
-        const int bytes = min(R::kPitch, row_bytes - off);
-        const uint8_t *pg = rg + off, *pu = rup + off;
-        uint32_t align = uint32_t(reinterpret_cast<uintptr_t>(pg) | reinterpret_cast<uintptr_t>(pu)) | uint32_t(row_bytes);
-        if constexpr (kIq3s) {
-          pg -= reinterpret_cast<uintptr_t>(pg) & 3;
-          pu -= reinterpret_cast<uintptr_t>(pu) & 3;
-        }
-        bool async = true;
-        for (int hf = 0; hf < kRows / 32; ++hf) {
-          const uint32_t dst = smem_u32(rawb) + (s * kTileM + row0 + 32 * hf) * R::kPitch;
-          if constexpr (DOWN) {
-            const uint8_t* p = pg + size_t(32 * hf) * row_bytes;
-            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece, short_mask, [&](int r) { return p + r * row_bytes; });
-          } else {
-            const uint8_t *p = pg + 16 * hf * row_bytes, *p2 = pu + 16 * hf * row_bytes;
-            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece, short_mask,
-                                     [&](int r) { return ((r & 1) ? p2 : p) + (r >> 1) * row_bytes; });
+    if constexpr (DOWN) {
+      // ---------------- raw weight bytes of whole units, a unit or two ahead of the decoding (one warp)
+      if (warp == 2) {
+        uint32_t n = 0;
+        const uint32_t bytes = uint32_t(kTileM * row_bytes);
+        for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++n) {
+          const int4 un = unit_at(u);
+          const uint8_t* src = blob_of(un.x) + A.L.down_offset + size_t(un.y) * row_bytes;
+          const uint32_t s = n % R::kSlots;
+          uint8_t* dst = rawb + s * R::kSlot;
+          if (!ab.wait_warp(&bars->raw_empty[s], ((n / R::kSlots) & 1) ^ 1)) break;
+          if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+            if (lane == 0) {
+              mbar_expect_tx(&bars->raw_full[s], bytes);
+              bulk_g2s(dst, src, bytes, &bars->raw_full[s]);
+            }
+          } else {  // an expert table may hold any even address
+            for (uint32_t i = lane; i < bytes / 2; i += 32)
+              reinterpret_cast<unsigned short*>(dst)[i] = __ldg(reinterpret_cast<const unsigned short*>(src) + i);
+            fence_proxy_async();  // (a later unit's bulk copy will write here)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->raw_full[s]);
           }
         }
-        if (async) cp_async_arrive_noinc(&bars->raw_full[s]);
-        else mbar_arrive(&bars->raw_full[s]);
       }
+    } else {
+      // ---------------- raw weight bytes, a few rounds ahead of the decoding; a warp copies 64 of the 128 rows
+      constexpr int kRows = kTileM / kGgRawWarps;
+      const int row0 = kRows * (warp - 2);
+      int piece[9] = {};  // IQ4_NL, see gg_load_raw
+      if constexpr (!kIq3s) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+          const int id = lane + 32 * i, r = id / 9, c = id - 9 * r;
+          piece[i] = 16 * c + (r >> 1) * row_bytes + ((r & 1) ? int(A.L.up_offset - A.L.gate_offset) : 0);
+        }
+      }
+      uint32_t rcount = 0;
+      int4 un = unit_or_none(blockIdx.x), un_next;
+      bool ok = true;
+      for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, un = un_next) {
+        un_next = unit_or_none(u + gridDim.x);
+        const uint8_t* blob = blob_of(un.x);
+        const uint8_t* rg = blob + A.L.gate_offset + size_t(un.y + row0 / 2) * row_bytes;   // first gate row
+        const uint8_t* rup = blob + A.L.up_offset + size_t(un.y + row0 / 2) * row_bytes;  // first up row
+        for (int rd = 0; rd < rounds; ++rd, ++rcount) {
+          const uint32_t s = rcount % R::kSlots;
+          if (!(ok = ab.wait_warp(&bars->raw_empty[s], ((rcount / R::kSlots) & 1) ^ 1))) break;
+          const int off = rd * R::kPiece;
+          const int bytes = min(R::kPitch, row_bytes - off);
+          const uint8_t *pg = rg + off, *pu = rup + off;
+          uint32_t align = uint32_t(reinterpret_cast<uintptr_t>(pg) | reinterpret_cast<uintptr_t>(pu)) | uint32_t(row_bytes);
+          if constexpr (kIq3s) {
+            pg -= reinterpret_cast<uintptr_t>(pg) & 3;
+            pu -= reinterpret_cast<uintptr_t>(pu) & 3;
+          }
+          bool async = true;
+          for (int hf = 0; hf < kRows / 32; ++hf) {
+            const uint32_t dst = smem_u32(rawb) + s * R::kSlot + (row0 + 32 * hf) * R::kPitch;
+            const uint8_t *p = pg + 16 * hf * row_bytes, *p2 = pu + 16 * hf * row_bytes;
+            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece,
+                                     [&](int r) { return ((r & 1) ? p2 : p) + (r >> 1) * row_bytes; });
+          }
+          if (async) cp_async_arrive_noinc(&bars->raw_full[s]);
+          else mbar_arrive(&bars->raw_full[s]);
+        }
+      }
+      cp_async_wait_all();
     }
-    cp_async_wait_all();
   } else if (warp < kGgFirstEpi) {
     // ---------------- decoding warps: lane = row 32 q + lane. Two groups of eight warps take alternate rounds of 256 K
     // and own one A stage each: while one group waits (raw bytes, its stage, its tensor-memory stores) the other one
     // decodes. In a group, a quarter's two warps take 128 K each. (Sixteen warps on every round ran in phase and waited
     // in phase; four groups on 128 K each double the hand-offs of the MMA thread, which then paces the kernel.)
     const int q = warp & 3, j = (warp - kGgFirstDecode) >> 2, grp = j >> 1;
-    const uint32_t raw_row = smem_u32(rawb) + (32 * q + lane) * R::kPitch;
+    const uint32_t raw_row = smem_u32(rawb) + (32 * q + lane) * (DOWN ? row_bytes : R::kPitch);
     const uint32_t ta = tmem_base + (uint32_t(32 * q) << 16) + kGgABase + grp * 128;
     const GgDecodeConst dc{smem_u32(table), uint32_t(lane) * (kIq3s ? 0x00020002u : 0x00040004u)};
-    // bytes from the covering word to the first block of the lane's row (IQ3_S: 0 or 2; rows are multiples of 4 apart)
+    // gate/up: bytes from the covering word to the first block of the lane's row (IQ3_S: 0 or 2; rows are multiples of 4
+    // apart)
     auto row_shift = [&](const int4& w) -> int {
-      if constexpr (!kIq3s) return 0;
-      const int64_t off = DOWN ? A.L.down_offset : (lane & 1) ? A.L.up_offset : A.L.gate_offset;
-      return int(reinterpret_cast<uintptr_t>(blob_of(w.x) + off)) & 3;
+      if constexpr (!kIq3s || DOWN) return 0;
+      return int(reinterpret_cast<uintptr_t>(blob_of(w.x) + ((lane & 1) ? A.L.up_offset : A.L.gate_offset))) & 3;
     };
-    uint32_t r0 = 0;  // rounds before this unit
+    uint32_t r0 = 0, n = 0;  // rounds, units before this unit
     int4 un_next = unit_or_none(blockIdx.x);
-    for (int u = blockIdx.x; u < n_units; u += gridDim.x, r0 += rounds) {
+    for (int u = blockIdx.x; u < n_units; u += gridDim.x, r0 += rounds, ++n) {
       const int shift0 = row_shift(un_next);
       un_next = unit_or_none(u + gridDim.x);
       bool ok = true;
+      if constexpr (DOWN) {
+        if (!ab.wait_warp(&bars->raw_full[n % R::kSlots], (n / R::kSlots) & 1)) break;
+      }
       for (int rd = (grp ^ int(r0)) & 1; rd < rounds; rd += 2) {
-        const uint32_t rc = r0 + rd, rs = rc % R::kSlots, pa = ((rc / kGgAStages) & 1) ^ 1;
+        const uint32_t rc = r0 + rd, rs = (DOWN ? n : rc) % R::kSlots, pa = ((rc / kGgAStages) & 1) ^ 1;
         const int m = (j ^ int(rc >> 1)) & 1;  // this warp's half of the round (a short round's only half changes hands)
-        const uint32_t row = raw_row + rs * (kTileM * R::kPitch), tcol = ta + m * 64;
-        const int shift = (shift0 + rd * R::kPiece) & 3;
-        if (!(ok = ab.wait_warp(&bars->raw_full[rs], (rc / R::kSlots) & 1))) break;
+        const int at = DOWN ? rd * R::kPiece : 0;
+        const uint32_t row = raw_row + rs * R::kSlot + (at & ~3), tcol = ta + m * 64;
+        const int shift = DOWN ? at & 3 : (shift0 + rd * R::kPiece) & 3;
+        if constexpr (!DOWN) {
+          if (!(ok = ab.wait_warp(&bars->raw_full[rs], (rc / R::kSlots) & 1))) break;
+        }
         const bool mine = 4 * rd + 2 * m < k_steps;
-        GgStep<FMT> raw;
+        std::conditional_t<kIq3s, GgStepIq3s, GgWords<DOWN ? 18 : 9>> raw;
         uint32_t out[16];
         if (mine) {
-          raw.load(row, shift, 2 * m);
+          if constexpr (kIq3s) raw.load(row, shift, 2 * m);
+          else if constexpr (DOWN) raw.load_half(row, m, (row_bytes & 15) == 0);
+          else raw.load_step(row + 72 * m);
           raw.template decode<0>(dc, out);
         }
         if (!(ok = ab.wait_warp(&bars->a_empty[grp], pa))) break;
@@ -529,10 +575,11 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
           tmem_st16(tcol, out);
           raw.template decode<1>(dc, out);
           tmem_st16(tcol + 16, out);
-          raw.load(row, shift, 2 * m + 1);
-          raw.template decode<0>(dc, out);
+          if constexpr (kIq3s) raw.load(row, shift, 2 * m + 1);
+          else if constexpr (!DOWN) raw.load_step(row + 72 * m + 36);
+          raw.template decode<!kIq3s && DOWN ? 2 : 0>(dc, out);
           tmem_st16(tcol + 32, out);
-          raw.template decode<1>(dc, out);
+          raw.template decode<!kIq3s && DOWN ? 3 : 1>(dc, out);
           tmem_st16(tcol + 48, out);
           tmem_st_wait();
         }
@@ -540,10 +587,14 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&bars->a_full[grp]);
-          mbar_arrive(&bars->raw_empty[rs]);
+          if (!DOWN) mbar_arrive(&bars->raw_empty[rs]);
         }
       }
       if (!ok) break;
+      if (DOWN) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->raw_empty[n % R::kSlots]);
+      }
     }
   } else {
     // ---------------- epilogue: lane quarter = warp % 4, two warps per quarter take alternate chunks of 16 tokens
