@@ -86,8 +86,10 @@ struct Abort {
   volatile int* flag;
   uint32_t* status;
   __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) const {
-    // each try may sleep in the instruction for about a microsecond: two dozen waiting warps share the issue slots
-    // with the decoding ones
+    // The first probe of a barrier does not wait (a try with a time limit takes longer even when the phase is complete).
+    // Each later one may sleep in the instruction for about a microsecond: two dozen waiting warps share the issue slots
+    // with the decoding ones.
+    if (mbar_test_wait(bar, parity)) return true;
     for (uint32_t i = 0; i < (1u << 21); ++i) {
       if (mbar_try_wait_hint(bar, parity)) return true;
       if ((i & 31u) == 31u && *flag) return false;  // another role gave up: fall through every later wait
@@ -96,11 +98,17 @@ struct Abort {
     atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
     return false;
   }
-  // The same for a whole warp: one lane polls (the barrier is read once, not by 32 lanes in turn).
+  // The same for a whole warp. All lanes try: a lane that polls for the others (a branch, then a shuffle) made a wait on a
+  // barrier that is ready cost some 400 cycles (gate/up of 96 IQ3_S tokens 278 us, 253 so); all decisions are the warp's.
   __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) const {
-    bool ok = true;
-    if ((threadIdx.x & 31) == 0) ok = wait(bar, parity);
-    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
+    for (uint32_t i = 0; i < (1u << 21); ++i) {
+      if (__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity))) return true;
+      if ((i & 31u) == 31u && __any_sync(0xffffffffu, *flag != 0)) return false;
+    }
+    *flag = 1;
+    if ((threadIdx.x & 31) == 0) atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+    return false;
   }
 };
 

@@ -65,8 +65,8 @@ template <>
 struct GgRaw<FB_FMT_IQ4_NL, true> {
   static constexpr int kPiece = 144, kPitch = 360, kSlots = 2, kSlot = kTileM * kPitch;  // (288-byte rows: pitch 288)
 };
-// IQ3_S selectors, 16 bits per index and lane: entry i of lane l at byte 64 i + 2 l. Two lanes share a bank, so a
-// warp's look-up takes two passes at most where one shared copy takes three to four.
+// IQ3_S selectors, 16 bits per index and lane: entry i of lane l at byte 128 (i % 256) + 64 (i / 256) + 2 l. Two lanes
+// share a bank, so a warp's look-up takes two passes at most where one shared copy takes three to four.
 // IQ4_NL level pairs, entry b of lane l at byte 128 b + 4 l.
 template <int FMT>
 constexpr int kGgTableBytes = FMT == FB_FMT_IQ3_S ? 512 * 64 : 256 * 128;
@@ -108,65 +108,69 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------ decoding
+// Byte B of `word` times `weight` plus `acc`: one integer dot product, which runs on the multiply pipe. The decoders are
+// bound by the half-rate integer pipe and by issue (74 and 72 % busy in IQ3_S gate/up with shifts and masks here), so table
+// addresses and sign masks are formed this way: gate/up of 96 tokens 306 -> 278 us.
+template <int B>
+__device__ __forceinline__ uint32_t byte_mad(uint32_t word, uint32_t weight, uint32_t acc) {
+  return __dp4a(word, weight << (8 * B), acc);
+}
 // IQ3_S, one sub-block (32 weights). A weight is db * g * sign with g one of the 8 odd magnitudes 1..15, so the 8
 // possible bf16 values of the sub-block are computed once (db * (2k+1) is exact in fp32, then rounded like the
 // reference rounds) and kept as two byte planes in four registers; the codebook table holds, per 9-bit index, the
 // four 3-bit magnitude numbers as PRMT selector nibbles, so one PRMT per plane picks four weights, one XOR flips
 // their signs (bit 7 of the high bytes; rounding is sign-symmetric) and two PRMTs interleave the planes into bf16
-// pairs. B = the sub-block's eight ninth index bits, lane_pat = 2 * lane in both halves of the word.
+// pairs. B = the sub-block's eight ninth index bits, lane_table = the lane's entry 0.
+template <int L>
+__device__ __forceinline__ void gg_iq3s_lookup(uint32_t qs, uint32_t bits, uint32_t s_even, uint32_t s_odd, uint32_t lane_table,
+                                               const uint32_t (&plane)[4], uint32_t (&out)[16]) {
+  constexpr int b = L & 3;
+  const uint32_t sel = lds_u16<0>(byte_mad<b>(qs, 128u, byte_mad<b>(bits, 4u, lane_table)));
+  // the four sign bits -> bit 7 of the four bytes
+  const uint32_t sx = (L & 1) ? byte_mad<L / 2>(s_odd, 4u, 0u) * 0x00408102u : byte_mad<L / 2>(s_even, 128u, 0u) * 0x00204081u;
+  const uint32_t lo4 = prmt(plane[0], plane[1], sel);
+  const uint32_t hi4 = prmt(plane[2], plane[3], sel) ^ (sx & 0x80808080u);
+  out[2 * L] = prmt(lo4, hi4, 0x5140u);
+  out[2 * L + 1] = prmt(lo4, hi4, 0x7362u);
+}
 __device__ __forceinline__ void gg_decode_iq3s(float db, uint32_t qs_lo, uint32_t qs_hi, uint32_t B, uint32_t sg,
-                                               uint32_t sel_base, uint32_t lane_pat, uint32_t (&out)[16]) {
-  const float db2 = db + db;
+                                               uint32_t lane_table, uint32_t (&out)[16]) {
   float pv[8];
   pv[0] = db;
 #pragma unroll
   for (int k = 1; k < 8; ++k) pv[k] = fmaf(float(2 * k), db, db);  // exact: (2k+1) * db has at most 20 significant bits
-  (void)db2;
   const uint32_t t01 = pack_bf16(pv[0], pv[1]), t23 = pack_bf16(pv[2], pv[3]);
   const uint32_t t45 = pack_bf16(pv[4], pv[5]), t67 = pack_bf16(pv[6], pv[7]);
-  const uint32_t lo_a = prmt(t01, t23, 0x6420u), hi_a = prmt(t01, t23, 0x7531u);
-  const uint32_t lo_b = prmt(t45, t67, 0x6420u), hi_b = prmt(t45, t67, 0x7531u);
-  // Table byte offsets (64 * index + 2 * lane) of two look-ups per word: qs byte in bits 6..13 (22..29), the ninth
-  // index bit, taken from B by a multiply that lands it on bit 14 (30).
-  constexpr uint32_t kM = 0x3FC03FC0u, kM2 = 0x40004000u;
-  uint32_t a[4];
-  a[0] = (((qs_lo << 6) & kM) | lane_pat) | ((B * 0x10004000u) & kM2);  // look-ups 0, 2
-  a[1] = (((qs_lo >> 2) & kM) | lane_pat) | ((B * 0x08002000u) & kM2);  // look-ups 1, 3
-  a[2] = (((qs_hi << 6) & kM) | lane_pat) | ((B * 0x01000400u) & kM2);  // look-ups 4, 6
-  a[3] = (((qs_hi >> 2) & kM) | lane_pat) | ((B * 0x00800200u) & kM2);  // look-ups 5, 7
-  const uint32_t s_even = sg & 0x0F0F0F0Fu, s_odd = (sg >> 4) & 0x0F0F0F0Fu;
-#pragma unroll
-  for (int l = 0; l < 8; ++l) {
-    const uint32_t aw = a[2 * (l >> 2) + (l & 1)];
-    const uint32_t off = (l & 2) ? (aw >> 16) : (aw & 0xFFFFu);
-    const uint32_t sel = lds_u16<0>(sel_base + off);
-    const uint32_t nib = prmt((l & 1) ? s_odd : s_even, 0u, 0x4440u | uint32_t(l >> 1));
-    const uint32_t sx = nib * 0x10204080u;  // sign bit j -> bit 7 of byte j
-    const uint32_t lo4 = prmt(lo_a, lo_b, sel);
-    const uint32_t hi4 = prmt(hi_a, hi_b, sel) ^ (sx & 0x80808080u);
-    out[2 * l] = prmt(lo4, hi4, 0x5140u);
-    out[2 * l + 1] = prmt(lo4, hi4, 0x7362u);
-  }
+  const uint32_t plane[4] = {prmt(t01, t23, 0x6420u), prmt(t45, t67, 0x6420u), prmt(t01, t23, 0x7531u), prmt(t45, t67, 0x7531u)};
+  // ninth index bits, one per byte (bit 4): look-ups 0..3 and 4..7. (The dot products share two weights, 4 and 128, so their
+  // eight constants stay in registers: 2 % against four weights.)
+  const uint32_t b_lo = ((B & 0x0Fu) * 0x02040810u) & 0x10101010u, b_hi = ((B & 0xF0u) * 0x00204081u) & 0x10101010u;
+  const uint32_t s_even = sg & 0x0F0F0F0Fu, s_odd = sg & 0xF0F0F0F0u;
+  gg_iq3s_lookup<0>(qs_lo, b_lo, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<1>(qs_lo, b_lo, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<2>(qs_lo, b_lo, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<3>(qs_lo, b_lo, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<4>(qs_hi, b_hi, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<5>(qs_hi, b_hi, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<6>(qs_hi, b_hi, s_even, s_odd, lane_table, plane, out);
+  gg_iq3s_lookup<7>(qs_hi, b_hi, s_even, s_odd, lane_table, plane, out);
 }
 
 // IQ4_NL, one block (32 weights) from its scale and 16 code bytes. A byte holds the codes of elements i and i + 16; a
 // table in shared memory (one copy per lane: a look-up takes one pass) gives both levels as a bf16 pair (exact:
 // |level| <= 127), which widen to fp32 by a shift and a mask; d * level is exact in fp32 (19 significant bits) and
-// rounded once to bf16. Two operations of the half-rate integer pipe per weight; looking the levels up by byte-permutes
-// and converting them through the mantissa took 3.5.
-__device__ __forceinline__ void gg_decode_iq4nl(float d, const uint32_t (&q)[4], uint32_t pair_base, uint32_t lane_pat,
-                                                uint32_t (&out)[16]) {
+// rounded once to bf16. One operation of the half-rate integer pipe per weight (two with the table addresses formed by
+// shifts and masks: gate/up of 96 tokens 297 us against 262).
+__device__ __forceinline__ void gg_decode_iq4nl(float d, const uint32_t (&q)[4], uint32_t lane_table, uint32_t (&out)[16]) {
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
-    // byte offsets 128 * code byte + 4 * lane of two look-ups per word
-    const uint32_t a02 = ((q[m] * 128u) & 0x7F807F80u) | lane_pat, a13 = ((q[m] >> 1) & 0x7F807F80u) | lane_pat;
+    const uint32_t v[4] = {lds_u32<0>(byte_mad<0>(q[m], 128u, lane_table)), lds_u32<0>(byte_mad<1>(q[m], 128u, lane_table)),
+                           lds_u32<0>(byte_mad<2>(q[m], 128u, lane_table)), lds_u32<0>(byte_mad<3>(q[m], 128u, lane_table))};
     float lo[4], hi[4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const uint32_t a = (b & 1) ? a13 : a02;
-      const uint32_t v = lds_u32<0>(pair_base + ((b & 2) ? a >> 16 : a & 0xFFFFu));
-      lo[b] = __fmul_rn(d, __uint_as_float(v * 65536u));
-      hi[b] = __fmul_rn(d, __uint_as_float(v & 0xFFFF0000u));
+      lo[b] = __fmul_rn(d, __uint_as_float(v[b] * 65536u));
+      hi[b] = __fmul_rn(d, __uint_as_float(v[b] & 0xFFFF0000u));
     }
     out[2 * m] = pack_bf16(lo[0], lo[1]);
     out[2 * m + 1] = pack_bf16(lo[2], lo[3]);
@@ -176,9 +180,6 @@ __device__ __forceinline__ void gg_decode_iq4nl(float d, const uint32_t (&q)[4],
 }
 
 // The raw words of one warp step (64 weights of the lane's row), in registers, and their decoding half by half.
-struct GgDecodeConst {
-  uint32_t table, lane_pat;  // window address of the format's table, this lane's address bits in it
-};
 struct GgStepIq3s {
   uint32_t qs[4], sg[2], qh, sc;
   float d;
@@ -200,11 +201,11 @@ struct GgStepIq3s {
     sg[1] = __funnelshift_r(g1, g2, sh);
   }
   template <int HALF>
-  __device__ __forceinline__ void decode(const GgDecodeConst& c, uint32_t (&out)[16]) const {
+  __device__ __forceinline__ void decode(uint32_t lane_table, uint32_t (&out)[16]) const {
     // multiplier 2 s + 1 as a float through the mantissa of 2^23
     const float m = __uint_as_float(0x4B000001u | ((HALF ? sc >> 4 : sc & 15u) << 1)) - 8388608.0f;
-    gg_decode_iq3s(__fmul_rn(d, m), qs[2 * HALF], qs[2 * HALF + 1], HALF ? qh >> 8 : qh & 0xFFu, sg[HALF], c.table,
-                   c.lane_pat, out);
+    gg_decode_iq3s(__fmul_rn(d, m), qs[2 * HALF], qs[2 * HALF + 1], HALF ? qh >> 8 : qh & 0xFFu, sg[HALF], lane_table,
+                   out);
   }
 };
 // IQ4_NL: W words of the lane's row. gate/up fetches one K step (two 18-byte blocks, nine words) at a time; down both steps of
@@ -236,15 +237,15 @@ struct GgWords {
     }
   }
   template <int B>  // block B of those fetched
-  __device__ __forceinline__ void decode(const GgDecodeConst& c, uint32_t (&out)[16]) const {
+  __device__ __forceinline__ void decode(uint32_t lane_table, uint32_t (&out)[16]) const {
     constexpr int k = 9 * B / 2;
     if constexpr (B % 2 == 0) {
       const uint32_t q[4] = {__funnelshift_r(w[k], w[k + 1], 16), __funnelshift_r(w[k + 1], w[k + 2], 16),
                              __funnelshift_r(w[k + 2], w[k + 3], 16), __funnelshift_r(w[k + 3], w[k + 4], 16)};
-      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[k] & 0xFFFFu))), q, c.table, c.lane_pat, out);
+      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[k] & 0xFFFFu))), q, lane_table, out);
     } else {
       const uint32_t q[4] = {w[k + 1], w[k + 2], w[k + 3], w[k + 4]};
-      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[k] >> 16))), q, c.table, c.lane_pat, out);
+      gg_decode_iq4nl(__half2float(__ushort_as_half(static_cast<unsigned short>(w[k] >> 16))), q, lane_table, out);
     }
   }
 };
@@ -341,7 +342,7 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
 
   if constexpr (kIq3s) {
     for (int i = tid; i < 512 * 4; i += kGgThreads) {  // 16 bytes = eight lanes' copies of an entry
-      const uint32_t p = c_iq3s_grid_packed[i >> 2];
+      const uint32_t p = c_iq3s_grid_packed[(i >> 3) | ((i & 4) << 6)];
       const uint32_t e = (p & 7u) | (((p >> 3) & 7u) << 4) | (((p >> 6) & 7u) << 8) | (((p >> 9) & 7u) << 12);
       const uint32_t w = e * 0x00010001u;
       reinterpret_cast<uint4*>(table)[i] = make_uint4(w, w, w, w);
@@ -411,14 +412,19 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
         const uint32_t b_step = (kTileB >> 4) / S;  // descriptor distance of a stage's K steps
         for (int rd = 0; rd < rounds; ++rd, ++ra) {
           const uint32_t sa = ra % kGgAStages;
-          if (!(ok = ab.wait(&bars->a_full[sa], (ra / kGgAStages) & 1))) break;
           const int steps = min(4, k_steps - 4 * rd);
           uint32_t la = tmem_base + kGgABase + sa * 128;
           for (int k0 = 0; k0 < steps; k0 += S, ++sbc) {
             const uint32_t sb = sbc % kGgBStages;
             if (!(ok = ab.wait(&bars->b_full[sb], (sbc / kGgBStages) & 1))) break;
+            if (k0 == 0 && !(ok = ab.wait(&bars->a_full[sa], (ra / kGgAStages) & 1))) break;  // (the later of the two)
             tc_fence_after();
             uint32_t lb = ring_lo + sb * (kTileB >> 4);
+            if (S == 4 && steps == 4) {  // (constant operand distances and predicates: fewer instructions per MMA)
+#pragma unroll
+              for (int k = 0; k < 16; ++k)
+                umma_bf16_ts(dcol, la + 8 * k, lb + (k >> 2) * (kTileB >> 6) + 2 * (k & 3), idesc, (rd | k) ? 1u : 0u);
+            } else
             for (int k = k0; k < min(k0 + S, steps); ++k, la += 32, lb += b_step) {
               umma_bf16_ts(dcol, la, lb, idesc, (rd | k) ? 1u : 0u);
 #pragma unroll
@@ -535,7 +541,7 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
     const int q = warp & 3, j = (warp - kGgFirstDecode) >> 2, grp = j >> 1;
     const uint32_t raw_row = smem_u32(rawb) + (32 * q + lane) * (DOWN ? row_bytes : R::kPitch);
     const uint32_t ta = tmem_base + (uint32_t(32 * q) << 16) + kGgABase + grp * 128;
-    const GgDecodeConst dc{smem_u32(table), uint32_t(lane) * (kIq3s ? 0x00020002u : 0x00040004u)};
+    const uint32_t lane_table = smem_u32(table) + uint32_t(lane) * (kIq3s ? 2 : 4);
     // gate/up: bytes from the covering word to the first block of the lane's row (IQ3_S: 0 or 2; rows are multiples of 4
     // apart)
     auto row_shift = [&](const int4& w) -> int {
@@ -567,19 +573,19 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
           if constexpr (kIq3s) raw.load(row, shift, 2 * m);
           else if constexpr (DOWN) raw.load_half(row, m, (row_bytes & 15) == 0);
           else raw.load_step(row + 72 * m);
-          raw.template decode<0>(dc, out);
+          raw.template decode<0>(lane_table, out);
         }
         if (!(ok = ab.wait_warp(&bars->a_empty[grp], pa))) break;
         tc_fence_after();
         if (mine) {
           tmem_st16(tcol, out);
-          raw.template decode<1>(dc, out);
+          raw.template decode<1>(lane_table, out);
           tmem_st16(tcol + 16, out);
           if constexpr (kIq3s) raw.load(row, shift, 2 * m + 1);
           else if constexpr (!DOWN) raw.load_step(row + 72 * m + 36);
-          raw.template decode<!kIq3s && DOWN ? 2 : 0>(dc, out);
+          raw.template decode<!kIq3s && DOWN ? 2 : 0>(lane_table, out);
           tmem_st16(tcol + 32, out);
-          raw.template decode<!kIq3s && DOWN ? 3 : 1>(dc, out);
+          raw.template decode<!kIq3s && DOWN ? 3 : 1>(lane_table, out);
           tmem_st16(tcol + 48, out);
           tmem_st_wait();
         }
