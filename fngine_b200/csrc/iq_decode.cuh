@@ -196,6 +196,7 @@ __host__ __device__ constexpr int iq4nl_level(int i) {
   constexpr int lv[16] = {FB_IQ4NL_LEVELS};
   return lv[i];
 }
+__device__ __forceinline__ uint32_t upper_half(uint32_t w) { return __dp2a_lo(w, 0x0100u, 0u); }
 // One 32-weight block from its 16 nibble bytes (4 words). Output word 2m+h (m = word, h = half)
 // holds weights of elements {4m+2h, 4m+2h+16, 4m+2h+1, 4m+2h+17}: activations are stored in
 // that interleaved order (see q8_0_interleave_index). A byte-permute looks at the low 16 bits of its selector only, so
@@ -205,7 +206,8 @@ __device__ __forceinline__ void iq4nl_decode32(const Iq4nlLevels& L, const uint3
   for (int m = 0; m < 4; ++m) {
     const uint32_t sel = q[m] & 0x77777777u, pick = ((q[m] >> 1) & 0x44444444u) | 0x32103210u;
     w[2 * m] = int(prmt(prmt(L.t0, L.t1, sel), prmt(L.t2, L.t3, sel), pick));
-    const uint32_t sel1 = sel >> 16, pick1 = pick >> 16;
+    // (upper halves by a dot product with 0 and 1: the shift's pipe is the one the permutes keep busy; 1 to 3 % of a layer)
+    const uint32_t sel1 = upper_half(sel), pick1 = upper_half(pick);
     w[2 * m + 1] = int(prmt(prmt(L.t0, L.t1, sel1), prmt(L.t2, L.t3, sel1), pick1));
   }
 }

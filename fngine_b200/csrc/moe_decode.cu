@@ -9,7 +9,7 @@
 // gate_up and down are one persistent kernel, one CTA per SM (moe_decode_experts.cuh): a producer thread streams
 // tiles of the expert blob into a three-stage shared-memory ring with 1-D bulk async copies (TMA, no multicast)
 // signalled through mbarriers; consumer warps decode the blocks from shared memory and accumulate exact int8 dot
-// products (dp4a). (A Q2_0 down projection has a plain kernel, moe_decode_generic.cuh.) Numerics are those of the
+// products (dp4a). Numerics are those of the
 // reference's CPU expert tier (src/cpu/iq_cpu.h:12-40 of the reference project): Q8_K activations
 // for IQ3_S weights, Q8_0 for IQ4_NL, integer sums per block, one fp32 scale step per block.
 #include "iq_decode.cuh"
@@ -1033,7 +1033,6 @@ __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_works
   }
 }
 
-#define FB_MOE_DECODE_TU
 #include "moe_decode_generic.cuh"
 #include "moe_decode_experts.cuh"
 
@@ -1307,10 +1306,14 @@ int32_t launch_experts_as(const fb_moe_expert_layout* layout, const fb_moe_decod
   if (e != cudaSuccess) return check_launch(what);
   return 0;
 }
-// Every gate/up format has its kernel with an IQ4_NL down projection at both intermediate sizes; IQ3_S also with its own.
+// Every gate/up format has its kernel with an IQ4_NL or Q2_0 down projection at both intermediate sizes; IQ3_S also with
+// its own.
 template <int GU>
 int32_t launch_experts_gu(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases, void* stream,
                           const char* what, const SelectArgs* sel) {
+  if (layout->down_format == FB_FMT_Q2_0)
+    return layout->inter == 512 ? launch_experts_as<GU, FB_FMT_Q2_0, 512>(layout, ws, phases, stream, what, sel)
+                                : launch_experts_as<GU, FB_FMT_Q2_0, 640>(layout, ws, phases, stream, what, sel);
   return layout->inter == 512 ? launch_experts_as<GU, FB_FMT_IQ4_NL, 512>(layout, ws, phases, stream, what, sel)
                               : launch_experts_as<GU, FB_FMT_IQ4_NL, 640>(layout, ws, phases, stream, what, sel);
 }
@@ -1442,9 +1445,9 @@ int32_t fb_moe_hot_gate_up(const fb_moe_expert_layout* layout, int32_t tokens, c
 static int32_t launch_down(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream);
 
 static bool one_launch(const fb_moe_expert_layout* layout) {
-  return layout->down_format == FB_FMT_IQ4_NL || (layout->down_format == FB_FMT_IQ3_S && layout->gate_up_format == FB_FMT_IQ3_S);
+  return layout->down_format != FB_FMT_IQ3_S || layout->gate_up_format == FB_FMT_IQ3_S;
 }
-// Both projections of every routed expert: one launch, but for a down format without a shared streaming kernel.
+// Both projections of every routed expert: one launch, but for IQ3_S down behind another gate/up format.
 static int32_t launch_experts(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream,
                               const SelectArgs* sel) {
   if (one_launch(layout))
@@ -1462,11 +1465,6 @@ int32_t fb_moe_hot_experts(const fb_moe_expert_layout* layout, int32_t tokens, c
 }
 
 static int32_t launch_down(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, void* stream) {
-  if (layout->down_format == FB_FMT_Q2_0) {
-    if (launch_pdl(down_q2_0_kernel, dim3(sm_count() * 8), dim3(256), 0, as_stream(stream), *layout, *ws) != cudaSuccess)
-      return check_launch("hot_down");
-    return 0;
-  }
   return launch_phases(layout, ws, kPhaseDown, stream, "hot_down", nullptr);
 }
 
@@ -1501,10 +1499,11 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
   EpRouteArgs era{};
   if (ep) era = *ep;
   era.act = layout_ok(layout) ? act_of(layout->gate_up_format) : FB_ACT_Q8_K;
-  // Three launches for IQ3_S experts (four otherwise): route (router projection + activation quantization),
-  // the expert kernel (every CTA runs the selection on the stored logits, then gate/up and down tiles in
-  // one persistent launch; the other formats take a gate/up and a down launch), combine. The expert
-  // arithmetic is that of the separate entry points. The route kernel sums a logit as eight K slices of
+  // Two launches: route (router projection + activation quantization) and the expert kernel (every CTA runs the
+  // selection on the stored logits, then gate/up and down tiles in one persistent launch, whose warps also combine a
+  // token's rows when its last one is there). IQ3_S down behind another gate/up format takes a gate/up and a down launch,
+  // and a caller with a table of resident slots a combine launch. The expert arithmetic is that of the separate entry
+  // points. The route kernel sums a logit as eight K slices of
   // 320 added in slice order, where fb_router_logits sums 80 values per lane and then the lanes: the two
   // projections agree to fp32 rounding (a few ulp), not bit for bit, so a near-tie between the tenth and
   // eleventh expert may resolve differently. Only rows 0..511 of logits_scratch are written: row 512

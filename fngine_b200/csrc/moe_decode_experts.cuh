@@ -1,8 +1,8 @@
 // The streaming expert kernel of the decode path, included by moe_decode.cu inside namespace fb's anonymous namespace:
-// gate/up in IQ3_S, IQ4_NL, IQ2_S, IQ3_XXS or IQ4_XS, down in IQ3_S or IQ4_NL. Written for IQ3_S, described for IQ3_S; the
+// gate/up in IQ3_S, IQ4_NL, IQ2_S, IQ3_XXS or IQ4_XS, down in IQ3_S, IQ4_NL or Q2_0. Written for IQ3_S, described for IQ3_S; the
 // other formats ride the same skeleton with their own tile sizes and block arithmetic (ExpertsCfg, gate_up_sub,
-// iq4nl_task_terms). (Behind plain kernels - a warp per row, lanes = sub-blocks from global memory - an IQ2_S + IQ4_NL
-// layer of five tokens took 129 us in six launches.)
+// iq4nl_task_terms, q2_0_task_terms). (Behind plain kernels - a warp per row, lanes = sub-blocks from global memory - an
+// IQ2_S + IQ4_NL layer of five tokens took 129 us in six launches.)
 //
 // One persistent kernel streams the gate, up and down matrices of every routed expert of a layer:
 // first all gate/up tiles (heaviest experts first), then all down tiles, through one three-stage ring
@@ -271,7 +271,7 @@ struct ExpertsCfg {
   static constexpr int kWarps = 24, kTasks = 10, kInter = INTER;
   static constexpr int kTaskBytes = GuFmt<GU>::kBlock;
   static constexpr int kGuRows = 16, kGuRowBytes = kTasks * kTaskBytes, kGuPart = kGuRows * kGuRowBytes;
-  static constexpr int kDnTaskBytes = DN == FB_FMT_IQ3_S ? 110 : INTER / 64 * 18;  // half a row
+  static constexpr int kDnTaskBytes = DN == FB_FMT_IQ3_S ? 110 : INTER / (DN == FB_FMT_Q2_0 ? 128 : 64) * 18;  // half a row
   static constexpr int kDnRows = INTER == 512 ? 160 : 128, kDnRowBytes = 2 * kDnTaskBytes, kDnTile = kDnRows * kDnRowBytes;
   static constexpr int kAct = act_of(GU);
   static constexpr int kGuAct = kAct == FB_ACT_Q8_K ? q8k_planar_bytes(H) : H + H / 8;
@@ -288,7 +288,7 @@ struct ExpertsCfg {
   static constexpr int kStages = smem_of(4) + kStaticSmem <= 232448 ? 4 : 3;
   static constexpr int kPartialFloats = kStages * kTasks * kTT * 32;
   static constexpr size_t kSmem = smem_of(kStages);
-  static_assert(DN == FB_FMT_IQ4_NL || (DN == FB_FMT_IQ3_S && GU == FB_FMT_IQ3_S && INTER == 512),
+  static_assert(DN == FB_FMT_IQ4_NL || DN == FB_FMT_Q2_0 || (DN == FB_FMT_IQ3_S && GU == FB_FMT_IQ3_S && INTER == 512),
                 "IQ3_S down shares the gate/up codebook and needs whole blocks per half row");
   static_assert(kTableBytes % 16 == 0 && kSlot % 16 == 0 && kGuPart % 16 == 0 && kDnTile % 16 == 0 && kGuAct % 16 == 0 &&
                     kDnAct % 16 == 0 && H % kDnRows == 0 && kDnRows % 32 == 0 && 2 * (kDnRows / 32) <= kTasks,
@@ -349,8 +349,8 @@ __device__ __forceinline__ void gate_up_sub(const uint32_t* w, int ib, const uin
       for (int i = 0; i < 2; ++i) {
         const uint32_t sel = qq[i] & 0x77777777u, pick = ((qq[i] >> 1) & 0x44444444u) | 0x32103210u;
         const uint32_t r0 = prmt(prmt(lv.t0, lv.t1, sel), prmt(lv.t2, lv.t3, sel), pick);
-        const uint32_t sel1 = sel >> 16;
-        const uint32_t r1 = prmt(prmt(lv.t0, lv.t1, sel1), prmt(lv.t2, lv.t3, sel1), pick >> 16);
+        const uint32_t sel1 = upper_half(sel);
+        const uint32_t r1 = prmt(prmt(lv.t0, lv.t1, sel1), prmt(lv.t2, lv.t3, sel1), upper_half(pick));
         q[2 * h + i] = int(prmt(r0, r1, 0x6420u));      // low nibbles: weights 4j .. 4j + 3
         q[4 + 2 * h + i] = int(prmt(r0, r1, 0x7531u));  // high nibbles: weights 16 + 4j ..
       }
@@ -516,6 +516,65 @@ __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlL
     if (ntp == 2) {
       const int s1 = dot32(wq, reinterpret_cast<const int8_t*>(act1) + 32 * blk);
       term[1] = fmaf(float(s1), d * reinterpret_cast<const float*>(act1 + k)[blk], term[1]);
+    }
+  }
+}
+// Q2_0: one task = NB consecutive 18-byte blocks (64 weights, codes 0..3 for -1..2) of the lane's row, OFF (0 or 2) bytes
+// behind the word `wp`. A code is a byte-permute's selector into the four levels once every other code of a byte is masked
+// off; eight more permutes put sixteen weights into the activations' interleaved order. Rows of 180 bytes (45 words) are
+// read without bank conflicts word by word, rows of 144 bytes in pairs of words.
+template <int NB, int OFF>
+__device__ __forceinline__ void q2_0_task_terms(const uint8_t* wp, const uint8_t* act0, int act_bytes, int k, int sub0,
+                                                int ntp, float (&term)[kTT]) {
+  constexpr int kWords = (OFF + 18 * NB + 3) / 4;
+  constexpr uint32_t kLevels = 0x020100FFu, kPairs = 0x33333333u;
+  uint32_t w[kWords];
+  if constexpr (NB == 4) {
+#pragma unroll
+    for (int c = 0; c < kWords / 2; ++c) {
+      const uint2 v = reinterpret_cast<const uint2*>(wp)[c];
+      w[2 * c] = v.x;
+      w[2 * c + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < kWords; ++c) w[c] = reinterpret_cast<const uint32_t*>(wp)[c];
+  }
+  term[0] = term[1] = 0.0f;
+  const uint8_t* act1 = act0 + (ntp == 2 ? act_bytes : 0);
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int at = OFF + 18 * b;  // even: the block's scale is the low or the high half of its word
+    const uint32_t head = w[at / 4];
+    const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(at % 4 ? head >> 16 : head & 0xFFFFu)));
+#pragma unroll
+    for (int sub = 0; sub < 2; ++sub) {
+      uint32_t c[2];  // codes 0..15 and 16..31 of the sub-block
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int n = at / 4 + 2 * sub + i;
+        c[i] = at % 4 ? w[n + 1] : __funnelshift_r(w[n], w[n + 1], 16);
+      }
+      // selectors of the even and of the odd weights
+      const uint32_t e0 = c[0] & kPairs, o0 = (c[0] >> 2) & kPairs, e1 = c[1] & kPairs, o1 = (c[1] >> 2) & kPairs;
+      int wq[8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t A = prmt(kLevels, 0u, h ? upper_half(e0) : e0), B = prmt(kLevels, 0u, h ? upper_half(o0) : o0);
+        const uint32_t C = prmt(kLevels, 0u, h ? upper_half(e1) : e1), D = prmt(kLevels, 0u, h ? upper_half(o1) : o1);
+        const uint32_t ac0 = prmt(A, C, 0x5140u), ac1 = prmt(A, C, 0x7362u), bd0 = prmt(B, D, 0x5140u), bd1 = prmt(B, D, 0x7362u);
+        wq[4 * h] = int(prmt(ac0, bd0, 0x5410u));  // weights 2j, 2j + 16, 2j + 1, 2j + 17
+        wq[4 * h + 1] = int(prmt(ac0, bd0, 0x7632u));
+        wq[4 * h + 2] = int(prmt(ac1, bd1, 0x5410u));
+        wq[4 * h + 3] = int(prmt(ac1, bd1, 0x7632u));
+      }
+      const int blk = sub0 + 2 * b + sub;
+      const int s0 = dot32(wq, reinterpret_cast<const int8_t*>(act0) + 32 * blk);
+      term[0] = fmaf(float(s0), d * reinterpret_cast<const float*>(act0 + k)[blk], term[0]);
+      if (ntp == 2) {
+        const int s1 = dot32(wq, reinterpret_cast<const int8_t*>(act1) + 32 * blk);
+        term[1] = fmaf(float(s1), d * reinterpret_cast<const float*>(act1 + k)[blk], term[1]);
+      }
     }
   }
 }
@@ -766,7 +825,11 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     } else if (k < C::kDnRows / 32) {
       const uint8_t* half = st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes;
       const uint8_t* act0 = st + C::kDnTile;
-      if constexpr (INTER == 512) {
+      if constexpr (DN == FB_FMT_Q2_0) {
+        if constexpr (INTER == 512) q2_0_task_terms<4, 0>(half, act0, C::kDnAct, INTER, 8 * parity, ntp, term);
+        else if (parity == 0) q2_0_task_terms<5, 0>(half, act0, C::kDnAct, INTER, 0, ntp, term);
+        else q2_0_task_terms<5, 2>(half - 2, act0, C::kDnAct, INTER, 10, ntp, term);
+      } else if constexpr (INTER == 512) {
         iq4nl_task_terms<8, 0>(half, lv, act0, C::kDnAct, INTER, 8 * parity, ntp, term);
       } else if (parity == 0) {
         iq4nl_task_terms<10, 0>(half, lv, act0, C::kDnAct, INTER, 0, ntp, term);

@@ -1,11 +1,7 @@
-// Decode-width projections for the reference's other expert formats: IQ3_XXS, IQ2_S and IQ4_XS as
-// gate/up formats (256-weight super-blocks, paired with Q8_K activations) and Q2_0 as a down format
-// (64-weight blocks, paired with Q8_0), src/kernels/moe/iq_device.cuh:171-288 and
-// third_party/ggml-iq/ggml-iq.h:26-78 of the reference. Included by moe_decode.cu (everything) and by
-// probes.cu (the decoders and the dequantization probe only).
-//
-// The gate/up formats run in the streaming kernel (moe_decode_experts.cuh takes the codebooks from here); Q2_0 has a
-// plain kernel: a warp per pair of rows, lanes = sub-blocks straight from global memory, reading the device work list.
+// The reference's other expert formats: IQ3_XXS, IQ2_S and IQ4_XS as gate/up formats (256-weight super-blocks, paired with
+// Q8_K activations) and Q2_0 as a down format (64-weight blocks, paired with Q8_0), src/kernels/moe/iq_device.cuh:171-288
+// and third_party/ggml-iq/ggml-iq.h:26-78 of the reference: codebooks, which the streaming kernel
+// (moe_decode_experts.cuh) uses too, and the dequantization probe's decoders. Included by moe_decode.cu and probes.cu.
 // (No namespace of its own: included inside namespace fb's unnamed namespace, once per translation unit.)
 #pragma once
 
@@ -189,59 +185,3 @@ __global__ void __launch_bounds__(256) dequant_generic_kernel(const uint8_t* __r
     for (int i = 0; i < 8; ++i) o[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
   }
 }
-
-#ifdef FB_MOE_DECODE_TU  // the MoE kernel below needs the decode translation unit's workspace helpers
-constexpr int kGenTok = 4;  // tokens of an item handled per pass over a row
-
-// down for Q2_0 (Q8_0 activations, stored per 32-block in the order position p <- element (p % 2) * 16 + p / 2):
-// unit = (item, pair of output rows): lanes 0-15 take the 16 sub-blocks of row 2n (inter 512; 20 of 640 wrap),
-// lanes 16-31 those of row 2n + 1. partial[pair][n] = w_pair * (down_n . q8(h[pair])).
-__global__ void __launch_bounds__(256) down_q2_0_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws) {
-  pdl_launch_dependents();
-  pdl_wait_prior();
-  const fb_moe_decode_work* work = ws.work;
-  const int n_items = min(max(work->n_items, 0), kMaxPairs), I = L.inter;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, hl = lane & 15;
-  const int64_t row_bytes = int64_t(I / 64) * 18;
-  for (int u = blockIdx.x * 8 + warp; u < n_items * (H / 2); u += gridDim.x * 8) {
-    const int item = u / (H / 2), n = 2 * (u - item * (H / 2)) + half;
-    const int pb = work->item_pair_begin[item], ntok = work->item_pair_begin[item + 1] - pb;
-    const uint8_t* row = L.slots + int64_t(work->item_slot[item]) * L.blob_stride + L.down_offset + int64_t(n) * row_bytes;
-    for (int t0 = 0; t0 < ntok; t0 += kGenTok) {
-      float acc[kGenTok];
-#pragma unroll
-      for (int t = 0; t < kGenTok; ++t) acc[t] = 0.0f;
-      for (int sub = hl; sub < I / 32; sub += 16) {
-        Sub32 s;
-        decode_sub32<FB_FMT_Q2_0>(row, sub, nullptr, s);
-        // weights into the activation rows' order: word w <- weights (2w, 2w + 16, 2w + 1, 2w + 17)
-        int wq[8];
-#pragma unroll
-        for (int wv = 0; wv < 8; ++wv) {
-          const uint32_t lo = uint32_t(s.q[wv >> 1]), hi = uint32_t(s.q[4 + (wv >> 1)]);
-          wq[wv] = int(__byte_perm(lo, hi, (wv & 1) ? 0x7362 : 0x5140));
-        }
-#pragma unroll
-        for (int t = 0; t < kGenTok; ++t) {
-          const uint8_t* hq = ws.hq + size_t(pb + min(t0 + t, ntok - 1)) * FB_HQ_STRIDE;
-          const int4* ap = reinterpret_cast<const int4*>(hq + 32 * sub);
-          const int4 a0 = ap[0], a1 = ap[1];
-          const int a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-          int sum = 0;
-#pragma unroll
-          for (int wv = 0; wv < 8; ++wv) sum = __dp4a(wq[wv], a[wv], sum);
-          acc[t] = fmaf(float(sum), s.d * reinterpret_cast<const float*>(hq + I)[sub], acc[t]);
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < kGenTok; ++t) {
-        float v = acc[t];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (hl == 0 && t0 + t < ntok) ws.partial[size_t(pb + t0 + t) * H + n] = work->pair_weight[pb + t0 + t] * v;
-      }
-    }
-  }
-}
-
-#endif  // FB_MOE_DECODE_TU
