@@ -766,3 +766,65 @@ def test_decode_layer_against_the_reference_expert_pool():
     err = max(rel_l2(got[t], want[t]) for t in range(tokens))
     print("decode layer vs cpu::ExpertPool (inter 640, IQ3_S + IQ4_NL): max rel L2 %.2e" % err)
     assert err <= TOL, err
+
+
+@pytest.mark.parametrize("fg,fd,inter,tokens", [(IQ3_S, IQ3_S, 512, 16), (IQ4_XS, IQ4_NL, 512, 3), (IQ4_XS, IQ4_NL, 640, 16),
+                                                (IQ3_XXS, Q2_0, 640, 16), (IQ2_S, IQ4_NL, 512, 1), (IQ4_NL, Q2_0, 512, 2)])
+def test_fused_layer_into_any_output_address(fg, fd, inter, tokens):
+    """Format pairs and sizes of the streaming expert kernel against the CPU expert path, and the combine that runs in
+    it: the same bits in an output that is only 4-byte aligned."""
+    torch = _torch()
+    from fngine_b200 import moe
+    seed = 3100 + inter + fg
+    layer = moe.synth_layer(fg, fd, inter, 512, seed)
+    ws = moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(306, rows=512).view(np.int16)).cuda().view(torch.bfloat16)
+    x = synth.activations(530 + tokens, tokens)
+    xd = torch.from_numpy(x).cuda()
+    flat = torch.full((tokens * H + 1,), float("nan"), dtype=torch.float32, device="cuda")
+    ys = [torch.full((tokens, H), float("nan"), dtype=torch.float32, device="cuda"), flat[1:].view(tokens, H)]
+    for y in ys:
+        moe.moe_layer_decode(wr, layer, xd, ws, y)
+    torch.cuda.synchronize()
+    assert ws.status() == 0
+    ids, w = O.topk(ws.logits.cpu().numpy()[:tokens * 513].reshape(tokens, 513)[:, :512])
+    want = oracle_layer(fg, fd, inter, seed, x, ids, w)
+    got = ys[0].cpu().numpy()
+    # fp32 rounding, but where an element of some expert's h lies so near a rounding boundary of its 8-bit code that the
+    # two sides' sums fall on different sides: one step is at most 1/127 of the largest |h| of its block, so of |h|, and
+    # columns of the down matrix have like norms (IQ3_XXS at 640, sixteen tokens: one row at 1.07e-3, the others 1.5e-7)
+    errs = [rel_l2(got[t], want[t]) for t in range(tokens)]
+    assert float(np.median(errs)) <= 1e-5 and max(errs) <= 1.0 / 127, errs
+    assert np.array_equal(ys[1].cpu().numpy().view(np.uint32), got.view(np.uint32))
+
+
+@pytest.mark.parametrize("inter_s,tokens", [(128, 1), (128, 16), (1024, 2), (1024, 16)])
+def test_one_call_branch_at_the_sizes_of_its_shared_expert(inter_s, tokens):
+    """The decode branch in one call with the smallest and the largest shared expert it takes, without residual
+    streams: y against the routed experts alone plus an fp64 shared expert."""
+    torch = _torch()
+    from fngine_b200 import linear, moe
+    layer = moe.synth_layer(IQ3_S, IQ4_NL, 640, 512, 4343)
+    ws, ws_plain = moe.DecodeWorkspace(layer), moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(910, rows=513).view(np.int16)).cuda().view(torch.bfloat16)
+    gu_c, gu_s = synth.fp8_row_weight(33, 2 * inter_s, H)
+    dn_c, dn_s = synth.fp8_row_weight(34, H, inter_s)
+    gu_s = gu_s * np.float32(10.0)
+    shared = moe.SharedExpert(linear.Fp8RowWeight(torch.from_numpy(gu_c).cuda(), torch.from_numpy(gu_s).cuda()),
+                              linear.Fp8RowWeight(torch.from_numpy(dn_c).cuda(), torch.from_numpy(dn_s).cuda()))
+    xb = synth.to_bf16_bits(synth.activations(78 + tokens, tokens))
+    xd = torch.from_numpy(xb.view(np.int16)).cuda().view(torch.bfloat16)
+    y, routed = (torch.full((tokens, H), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2))
+    moe.forward_moe_decode(wr, shared, layer, xd, ws, None, None, y)
+    moe.moe_layer_decode(wr[:512].contiguous(), layer, xd, ws_plain, routed)
+    torch.cuda.synchronize()
+    assert ws.status() == 0
+    logits = ws.logits.cpu().numpy()[:tokens * 513].reshape(tokens, 513)
+    assert np.array_equal(logits[:, :512], ws_plain.logits.cpu().numpy()[:tokens * 513].reshape(tokens, 513)[:, :512])
+    h = O.linear_fp8_a16(xb, gu_c, gu_s, kind="swiglu")
+    ysh = O.linear_fp8_a16(synth.to_bf16_bits(h.astype(np.float32)), dn_c, dn_s, kind="shared_scale", gate_logit=logits[:, 512])
+    got, ysh_gpu = y.cpu().numpy(), shared.y[:tokens].cpu().numpy()
+    assert max(rel_l2(ysh_gpu[t], ysh[t]) for t in range(tokens)) <= TOL
+    # the routed sum of the same call is the plain layer's: one fp32 addition lies between them
+    total = routed.cpu().numpy() + ysh_gpu
+    assert np.all(np.abs(got - total) <= 2.0 ** -22 * (np.abs(routed.cpu().numpy()) + np.abs(ysh_gpu) + np.abs(got)))

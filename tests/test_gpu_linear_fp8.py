@@ -279,3 +279,58 @@ def test_linear_fp8_argument_errors():
     assert lib.fb_linear_fp8(p, 32, p, p, 0, 192, 256, ctypes.byref(sw), p, 1 << 20, None, 0) == 1  # SwiGlu n % 128
     sh = fblib.LinearEpilogue(fblib.EPI_SHARED_SCALE, 513, p, None, None)
     assert lib.fb_linear_fp8(p, 32, p, p, 0, 128, 256, ctypes.byref(sh), p, 1 << 20, None, 0) == 1  # no gate logit
+
+
+def epilogue_case(torch, kind, T, n, acc):
+    """(maker of the epilogue with a fresh output, reference, whether bf16) over fp64 accumulators [T][n]."""
+    from fngine_b200 import linear
+    g = torch.Generator(device="cuda").manual_seed(T + n)
+    nan = lambda w, dt: torch.full((T, w), float("nan"), dtype=dt, device="cuda")
+    if kind == "store_bf16":
+        return lambda: linear.store_bf16(nan(n, torch.bfloat16)), acc, True
+    if kind == "store_f32":
+        return lambda: linear.store_f32(nan(n, torch.float32)), acc, False
+    if kind == "swiglu":
+        gg, uu = acc[:, :n // 2], acc[:, n // 2:]
+        return lambda: linear.swiglu(nan(n // 2, torch.bfloat16)), gg / (1.0 + torch.exp(-gg)) * uu, True
+    if kind == "shared_scale":
+        logit = torch.randn(T, 513, device="cuda", generator=g)
+        return (lambda: linear.shared_scale(nan(n, torch.float32), logit[:, 512:], 513),
+                acc * torch.sigmoid(logit[:, 512].double())[:, None], False)
+    inj, x0 = torch.randn(T, 4, device="cuda", generator=g), torch.randn(T, 4, n, device="cuda", generator=g)
+    return lambda: linear.gr_write(x0.clone(), inj), x0.double() + inj.double()[:, :, None] * acc[:, None, :], False
+
+
+@pytest.mark.parametrize("path", ["auto", "a8"])
+@pytest.mark.parametrize("T,n,k,kind", [
+    (17, 64, 128, "store_f32"),        # smallest: half a row tile, one K block, one CTA
+    (32, 128, 640, "swiglu"),          # one tile of 64 gate and 64 up rows, five K blocks over a cluster
+    (33, 960, 384, "gr_write"),        # ragged rows, one token behind a multiple of 32, three K blocks
+    (255, 2560, 896, "gr_write"),      # a token short of the two-SM kernel, seven K blocks
+    (256, 1280, 2560, "swiglu"),       # exactly one token tile, few output tiles
+    (257, 2560, 128, "shared_scale"),  # a second token tile of one token, K too short to share
+    (700, 640, 1152, "store_bf16"),    # three token tiles, nine K blocks over a cluster
+    (40, 19008, 128, "store_bf16"),    # more 128-row tiles than multiprocessors
+    (1, 512, 640, "store_f32"),        # decode width: the fewest row tiles that share K in a cluster, five K blocks
+    (16, 448, 1152, "gr_write"),       # decode width: a ragged fourth row tile, nine K blocks
+])
+def test_linear_fp8_small_and_middle_widths(T, n, k, kind, path):
+    """The kernels of small and middle widths at the edges of their tiles and K shares, both routes, every epilogue."""
+    torch = _torch()
+    from fngine_b200 import linear
+    weight = make_weight(torch, 7000 + T, n, k, T % 2 == 0)
+    x = bf16_tensor(torch, synth.activations(70 + T, T, hidden=k))
+    a = x.double()
+    if path == "a8":
+        xq, xs = linear.fp8_quantize_tokens(x)
+        a = torch.from_numpy(O.e4m3_table().astype(np.float64)).cuda()[xq.long()] * xs.double()[:, None]
+    make, ref, bf16_out = epilogue_case(torch, kind, T, n, exact_acc(torch, a, weight))
+    work = linear.linear_fp8_workspace(weight, T)
+    route = linear.L.FP8_PATH_A8 if path == "a8" else linear.L.FP8_PATH_AUTO
+    epis = [make(), make()]
+    for epi in epis:
+        linear.linear_fp8(x, weight, epi, work, path=route)
+    torch.cuda.synchronize()
+    out, again = (e._keep[0] for e in epis)
+    compare(torch, out, ref, bf16_out)
+    assert torch.equal(out.view(torch.uint8), again.view(torch.uint8))  # repeated calls are bitwise identical

@@ -359,3 +359,70 @@ def test_forward_moe_prefill_with_shared_expert(T):
     assert rel_l2(X.cpu().numpy(), wantX) <= 1e-6
     print("forward moe prefill T=%d: shared/routed norm %.2f, end to end median %.2e max %.2e" %
           (T, float(np.linalg.norm(ysh) / np.linalg.norm(routed)), float(np.median(errs)), max(errs)))
+
+
+def edge_counts_logits(counts, T):
+    """Router logits that send tokens 0 .. counts[e]-1 to expert e; the other choices of a token go to the ten experts
+    behind those, so every expert's token count is known."""
+    lg = np.full((T, 512), -30.0, np.float32)
+    for t in range(T):
+        chosen = [e for e, c in enumerate(counts) if t < c]
+        chosen += [len(counts) + i for i in range(10 - len(chosen))]
+        lg[t, chosen] = (synth.normal(700 + t, 10) * 0.5).astype(np.float32)
+    return lg
+
+
+@pytest.mark.parametrize("fg,fd,inter", [(IQ3_S, IQ3_S, 512), (IQ4_NL, IQ4_NL, 512), (IQ3_S, IQ4_NL, 640)])
+def test_grouped_gemms_at_the_edges_of_token_tiles(fg, fd, inter):
+    """Experts with 1, 16, 17, 64, 65, 128, 129, 256 and 257 tokens (the widths where the grouped kernel's token ring,
+    its accumulators and its tiles change), against fp64 products of the bf16-rounded weights; then the same bits from
+    an expert table of blobs at any even address, into an output row that is not 16-byte aligned."""
+    torch = _torch()
+    from fngine_b200 import moe, prefill
+    counts = [1, 16, 17, 64, 65, 128, 129, 256, 257]
+    T, n_exp = 257, len(counts) + 9  # (every token has the last expert of the list, so nine others at most)
+    layer = moe.synth_layer(fg, fd, inter, n_exp, 5150)
+    ws = prefill.PrefillWorkspace(T, inter)
+    logits = edge_counts_logits(counts, T)
+    xd = torch.from_numpy(synth.to_bf16_bits(synth.activations(41, T)).view(np.int16)).cuda().view(torch.bfloat16)
+    y = run_prefill(torch, layer, ws, torch.from_numpy(logits).cuda(), xd, T)
+    assert ws.status() == 0
+    off = ws.ints(ws.ws.expert_offset, 513)
+    assert [int(off[e + 1] - off[e]) for e in range(len(counts))] == counts
+    ptok = torch.from_numpy(ws.ints(ws.ws.pair_token, T * 10)).cuda().long()
+    pw = torch.from_numpy(ws.floats(ws.ws.pair_weight, T * 10)).cuda().double()
+    hb = ws.h(T * 10)
+    h = torch.from_numpy(synth.bf16_bits_to_f32(hb)).cuda().double()
+    stride, gate = layer.layout.blob_stride, inter * O.row_bytes(fg, H)
+    want, room = torch.zeros(T, H, dtype=torch.float64, device="cuda"), torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for e in range(n_exp):
+        blob = layer.slots[e * stride:(e + 1) * stride]
+        wgu = moe.dequant_rows(fg, blob[:2 * gate], 2 * inter, H).to(torch.bfloat16).double()
+        wdn = moe.dequant_rows(fd, blob[2 * gate:], H, inter).to(torch.bfloat16).double()
+        p0, p1 = int(off[e]), int(off[e + 1])
+        acc = xd[ptok[p0:p1]].double() @ wgu.T
+        g, u = acc[:, :inter], acc[:, inter:]
+        href = g / (1.0 + torch.exp(-g)) * u
+        # one bf16 step, and the same allowance near zero as the oracle comparison above
+        err = (h[p0:p1] - href).abs() / (href.abs() + 1e-2 * href.abs().amax(dim=1, keepdim=True))
+        assert float(err.max()) <= 2 ** -7, (e, float(err.max()))
+        want.index_add_(0, ptok[p0:p1], pw[p0:p1, None] * (h[p0:p1] @ wdn.T))
+        room.index_add_(0, ptok[p0:p1], pw[p0:p1, None] * (h[p0:p1].abs() @ wdn.abs().T))
+    # fp32 sums of `inter` exact products, one product with the weight, ten additions: at most one unit in the last
+    # place of the sum of magnitudes each
+    excess = ((y.double() - want).abs() / room).max()
+    assert float(excess) <= (inter + 11) * 2.0 ** -23, float(excess)
+    ybits = y.cpu().numpy().view(np.uint32)
+    for shift in (2, 4, 8):
+        buf = torch.zeros(n_exp * stride + 32, dtype=torch.uint8, device="cuda")
+        at = (-buf.data_ptr()) % 16 + shift
+        buf[at:at + n_exp * stride] = layer.slots
+        table = torch.full((512,), buf.data_ptr() + at, dtype=torch.int64, device="cuda")
+        table[:n_exp] += torch.arange(n_exp, device="cuda") * stride
+        prefill.moe_grouped_gate_up(layer, table, xd, T, ws)
+        assert np.array_equal(ws.h(T * 10), hb), shift
+        prefill.moe_grouped_down(layer, table, T, ws)
+        out = torch.full((T * H + 1,), float("nan"), dtype=torch.float32, device="cuda")[1:].view(T, H)
+        prefill.moe_prefill_combine(ws, None, None, 0, None, None, None, out, T)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), ybits), shift
+    assert ws.status() == 0
