@@ -302,10 +302,10 @@ __device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t al
   }
 }
 
-// A stage of the token ring holds this many 64-wide K steps: 256 / n rounded down to 1, 2 or 4. A unit of few tokens
-// then takes one hand-off per 256 K instead of four: a wait costs the MMA thread a few hundred cycles, as much as a
+// A stage of the token ring holds this many 64-wide K steps: 256 / n rounded down to 1, 2, 4 or 8. A unit of few tokens
+// then takes one hand-off per 512 K instead of eight: a wait costs the MMA thread a few hundred cycles, as much as a
 // whole K step of such a unit.
-__device__ __forceinline__ int gg_b_steps(int n) { return n <= 64 ? 4 : n <= 128 ? 2 : 1; }
+__device__ __forceinline__ int gg_b_steps(int n) { return n <= 32 ? 8 : n <= 64 ? 4 : n <= 128 ? 2 : 1; }
 
 struct GgArgs {
   fb_moe_expert_layout L;
@@ -410,27 +410,43 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
         const uint32_t dcol = tmem_base + (wide ? 0u : nb * 128u);
         const int S = gg_b_steps(n);
         const uint32_t b_step = (kTileB >> 4) / S;  // descriptor distance of a stage's K steps
+        int in_stage = 0;                           // steps used of the current stage
         for (int rd = 0; rd < rounds; ++rd, ++ra) {
           const uint32_t sa = ra % kGgAStages;
           const int steps = min(4, k_steps - 4 * rd);
           uint32_t la = tmem_base + kGgABase + sa * 128;
-          for (int k0 = 0; k0 < steps; k0 += S, ++sbc) {
+          for (int k = 0; k < steps;) {
             const uint32_t sb = sbc % kGgBStages;
-            if (!(ok = ab.wait(&bars->b_full[sb], (sbc / kGgBStages) & 1))) break;
-            if (k0 == 0 && !(ok = ab.wait(&bars->a_full[sa], (ra / kGgAStages) & 1))) break;  // (the later of the two)
+            if (in_stage == 0 && !(ok = ab.wait(&bars->b_full[sb], (sbc / kGgBStages) & 1))) break;
+            if (k == 0 && !(ok = ab.wait(&bars->a_full[sa], (ra / kGgAStages) & 1))) break;  // (the later of the two)
             tc_fence_after();
-            uint32_t lb = ring_lo + sb * (kTileB >> 4);
-            if (S == 4 && steps == 4) {  // (constant operand distances and predicates: fewer instructions per MMA)
+            uint32_t lb = ring_lo + sb * (kTileB >> 4) + in_stage * b_step;
+            if (S >= 4) {  // the round's steps lie in one stage, and a stage of eight lasts for two rounds
+              if (steps == 4) {  // (unrolled: fewer instructions per MMA)
 #pragma unroll
-              for (int k = 0; k < 16; ++k)
-                umma_bf16_ts(dcol, la + 8 * k, lb + (k >> 2) * (kTileB >> 6) + 2 * (k & 3), idesc, (rd | k) ? 1u : 0u);
-            } else
-            for (int k = k0; k < min(k0 + S, steps); ++k, la += 32, lb += b_step) {
-              umma_bf16_ts(dcol, la, lb, idesc, (rd | k) ? 1u : 0u);
+                for (int i = 0; i < 4; ++i, lb += b_step)
 #pragma unroll
-              for (int k4 = 1; k4 < 4; ++k4) umma_bf16_ts(dcol, la + 8 * k4, lb + 2 * k4, idesc, 1u);
+                  for (int k4 = 0; k4 < 4; ++k4)
+                    umma_bf16_ts(dcol, la + 32 * i + 8 * k4, lb + 2 * k4, idesc, (rd | i | k4) ? 1u : 0u);
+              } else {
+                for (int i = 0; i < steps; ++i, la += 32, lb += b_step)
+#pragma unroll
+                  for (int k4 = 0; k4 < 4; ++k4)
+                    umma_bf16_ts(dcol, la + 8 * k4, lb + 2 * k4, idesc, (rd | i | k4) ? 1u : 0u);
+              }
+              k = steps;
+              in_stage += steps;
+              if (in_stage < S && 4 * rd + steps < k_steps) continue;  // (= the round's end)
+              in_stage = 0;
+            } else {
+              for (int k1 = min(k + S, steps); k < k1; ++k, la += 32, lb += b_step) {
+                umma_bf16_ts(dcol, la, lb, idesc, (rd | k) ? 1u : 0u);
+#pragma unroll
+                for (int k4 = 1; k4 < 4; ++k4) umma_bf16_ts(dcol, la + 8 * k4, lb + 2 * k4, idesc, 1u);
+              }
             }
             umma_commit(&bars->b_empty[sb]);
+            ++sbc;
           }
           if (!ok) break;
           umma_commit(&bars->a_empty[sa]);
