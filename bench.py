@@ -218,7 +218,7 @@ def single_expert_section(torch, layers, routers, steps):
 def iq4nl_section(torch, steps, n_layers=4, fg=20, fd=20, inter=INTER, batches=(1, 8)):
     """The IQ4_NL resident-expert variant (18-byte blocks, Q8_0 activations): the same decode layer at batch
     1 and 8, four rotating layers (4.5 GB, larger than L2), CUDA-graph replays, device time. With other
-    formats: the same measurement for a layer of the reference's other expert formats (plain kernels)."""
+    formats: the same measurement for a layer of the reference's other expert formats."""
     from fngine_b200 import moe, synth
     blob = synth.blob_bytes(fg, fd, inter)
     layers = [moe.synth_layer(fg, fd, inter, EXPERTS, 6000 + l) for l in range(n_layers)]
@@ -257,7 +257,7 @@ def iq4nl_section(torch, steps, n_layers=4, fg=20, fd=20, inter=INTER, batches=(
         res["workload"] = "512 IQ4_NL experts per layer (2,211,840 B each), Q8_0 activations, %d rotating layers" % n_layers
     else:
         res["workload"] = "512 experts per layer, gate/up ggml type %d, down type %d, intermediate %d (%d B each), %d " \
-                          "rotating layers; plain (untuned) kernels for the formats beside IQ3_S and IQ4_NL" % (fg, fd, inter, blob, n_layers)
+                          "rotating layers" % (fg, fd, inter, blob, n_layers)
     res["device_status"] = ws.status()
     del layers
     torch.cuda.empty_cache()
@@ -837,7 +837,7 @@ def run_ours(args, rank, world, local_rank):
                 "h2d_bytes_per_step": B * HIDDEN * 4 * Lr, "d2h_bytes_per_step": B * HIDDEN * 4 * Lr,
                 "ms_per_step": e2e_ms / args.steps,
                 "api": "fb_moe_layer_decode_host per layer: pinned host x in, host y out, stream wait inside"},
-        "gpu_launches": args.steps * Lr * 3,
+        "gpu_launches": args.steps * Lr * 2,  # route, experts (selection and combine inside)
         "other_batches": other,
         "single_expert": single,
         "iq4nl_decode": iq4,

@@ -4,10 +4,9 @@ tensors `blk.N.ffn_{gate,up,down}_exps.weight` of a GGUF v3 file (tools/gguf.py:
 layer, 512 blobs `gate | up | down` of raw ggml blocks; `load_layer` puts them in HBM as the slot array
 the kernels read (stride kept from the pack, 4096-aligned).
 
-The decode kernels take gate/up in IQ3_S, IQ4_NL, IQ3_XXS, IQ2_S or IQ4_XS and down in IQ3_S, IQ4_NL or Q2_0
-(IQ3_S and IQ4_NL through the streaming kernels, the others through plain ones). A layer in another
-combination of the pack spec's formats is described and validated like the rest, and refused by `load_layer`
-with a PackError that names it. Everything here is host code; device memory comes from torch."""
+The decode kernels take gate/up in IQ3_S, IQ4_NL, IQ3_XXS, IQ2_S or IQ4_XS and down in IQ3_S, IQ4_NL or Q2_0.
+A layer in another combination of the pack spec's formats is described and validated like the rest, and refused
+by `load_layer` with a PackError that names it. Everything here is host code; device memory comes from torch."""
 import json
 import os
 import struct

@@ -34,9 +34,9 @@
 extern "C" {
 #endif
 
-/* ggml type ids of the expert formats (src/kernels/moe/moe.h:48-55). IQ3_S and IQ4_NL have the streaming
- * decode kernels and the prefill kernels; IQ3_XXS, IQ2_S and IQ4_XS (gate/up) and Q2_0 (down) run at decode
- * width through plain, untuned kernels (no prefill path). */
+/* ggml type ids of the expert formats (src/kernels/moe/moe.h:48-55). All of them run in the
+ * streaming decode kernel, IQ3_XXS, IQ2_S and IQ4_XS as gate/up, Q2_0 as down, IQ3_S and IQ4_NL as both; the prefill
+ * kernels take IQ3_S and IQ4_NL. */
 enum { FB_FMT_IQ3_XXS = 18, FB_FMT_IQ4_NL = 20, FB_FMT_IQ3_S = 21, FB_FMT_IQ2_S = 22, FB_FMT_IQ4_XS = 23, FB_FMT_Q2_0 = 42 };
 /* element types of activation inputs */
 enum { FB_DT_F32 = 0, FB_DT_BF16 = 1 };
@@ -111,7 +111,8 @@ typedef struct fb_moe_decode_work {
  * Q8_0 codes are stored per block in the order 2*(e%16) + e/16 that the IQ4_NL nibble decode
  * produces). `hq` is h re-quantized for the down projection, `item_done` counts finished gate/up
  * tiles per work item, `sched` holds the dynamic tile counters ([0] gate/up, [1] down) and from
- * [8] on the work items ordered by token count (heaviest first), `status` is one device word set
+ * [8] on the work items ordered by token count (heaviest first), from [192] on the counters of finished
+ * down rows per token and column tile, `status` is one device word set
  * when a bounded wait runs out. */
 typedef struct fb_moe_decode_workspace {
   fb_moe_decode_work* work;
@@ -120,7 +121,7 @@ typedef struct fb_moe_decode_workspace {
   uint8_t* hq;        /* [160 pairs][FB_HQ_STRIDE] */
   float* partial;     /* [160 pairs][2560], routing weight applied */
   int32_t* item_done; /* [160] */
-  int32_t* sched;     /* [8 + 160] */
+  int32_t* sched;     /* [192 + 16 * 20] */
   uint32_t* status;   /* FB_STATUS_* */
   int32_t gate_up_format;
   int32_t down_format;
@@ -159,10 +160,9 @@ int32_t fb_moe_hot_gate_up(const fb_moe_expert_layout* layout, int32_t tokens, c
 /* moe_hot_down, src/kernels/moe/moe.h:141-142: partial[pair][n] = w_pair * (down_n . q8(h[pair])). */
 int32_t fb_moe_hot_down(const fb_moe_expert_layout* layout, int32_t tokens, const fb_moe_decode_workspace* ws,
                         void* stream);
-/* moe_hot_gate_up followed by moe_hot_down as ONE launch where the formats allow it (IQ3_S gate/up and
- * down: a persistent kernel streams all gate/up tiles and then all down tiles through one pipeline, an
- * expert's down tiles waiting for its re-quantized h); otherwise the two launches. Same results as the
- * two calls, bit for bit. No counterpart in the reference as a single function. */
+/* moe_hot_gate_up followed by moe_hot_down as ONE launch (a persistent kernel streams all gate/up tiles
+ * and then all down tiles through one pipeline, an expert's down tiles waiting for its re-quantized h); two launches
+ * for IQ3_S down behind another gate/up format. Same results as the two calls, bit for bit. No counterpart in the reference as a single function. */
 int32_t fb_moe_hot_experts(const fb_moe_expert_layout* layout, int32_t tokens, const fb_moe_decode_workspace* ws,
                            void* stream);
 /* moe_combine, src/kernels/moe/moe.h:154-158: y[t] = sum of token t's partials in slot order
