@@ -188,9 +188,8 @@ __global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* __rest
 
 // The same logits, bit for bit, at prefill width (tokens > kMaxTok). Bound: the fp32 pipe (tokens x rows x 2560
 // multiply-adds). router_kernel above re-reads x for every row and keeps four tokens in flight: 0.96 us per token,
-// 963 us at 1003 tokens; this kernel takes 105 us there (fp32 pipe 43 % busy, 3.7 waves of blocks) and 27 us for up
-// to 256 tokens.
-// A block owns 32 rows x 32 tokens; its sixteen warps split K the way router_kernel's lanes do: the partial sum of
+// 963 us at 1003 tokens; this kernel takes 103 us there (fp32 pipe 43 % busy, 3.7 waves of blocks).
+// A block owns 32 rows (ROWS) x 32 tokens; its sixteen warps split K the way router_kernel's lanes do: the partial sum of
 // lane l (elements 256 c + 8 l + i, added over c, then i) belongs to warp l mod 16, which adds those of lanes l and
 // l + 16; the sixteen results meet in shared memory in the butterfly's order. A thread accumulates 8 rows x 4 tokens
 // in packed pairs of rows (fma.rn.f32x2: two multiply-adds per instruction, each rounded as fmaf is). 256-wide K
@@ -198,15 +197,19 @@ __global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* __rest
 // row's eight elements of a lane class, and the widening to fp32 (a shift or a mask) shares the issue slots that the
 // packed multiply-adds leave. (A K-major copy in fp32, widened while staging, took 142 us: its global loads touched
 // 32 rows per instruction.)
-constexpr int kRtRows = 32, kRtTok = 32, kRtChunk = 256, kRtBufs = 3;
+// ROWS (32, 16 or 8): few tokens do not fill the GPU with tiles of 32 rows, and a block's time follows its rows; see
+// fb_router_logits.
+constexpr int kRtTok = 32, kRtChunk = 256, kRtBufs = 3;
 template <bool XBF16>
 constexpr int router_tile_pitch() { return kRtChunk * (XBF16 ? 2 : 4) + 16; }  // bytes between token rows
 constexpr int kRtWPitch = kRtChunk * 2 + 16;                                  // and between weight rows
-template <bool XBF16>
-constexpr int router_tile_buf() { return kRtRows * kRtWPitch + kRtTok * router_tile_pitch<XBF16>(); }
-template <bool XBF16>
-constexpr int router_tile_smem() { return kRtBufs * router_tile_buf<XBF16>(); }
-static_assert(16 * kRtRows * kRtTok * 4 <= router_tile_smem<true>(), "the warps' partial tiles reuse the buffers");
+template <bool XBF16, int ROWS>
+constexpr int router_tile_buf() { return ROWS * kRtWPitch + kRtTok * router_tile_pitch<XBF16>(); }
+template <bool XBF16, int ROWS>
+constexpr int router_tile_smem() {
+  const int ring = kRtBufs * router_tile_buf<XBF16, ROWS>(), part = 16 * ROWS * kRtTok * 4;
+  return ring > part ? ring : part;  // the warps' partial tiles reuse the buffers
+}
 
 __device__ __forceinline__ void fma_f32x2(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
@@ -220,16 +223,16 @@ __device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
 }
 
-template <bool XBF16>
+template <bool XBF16, int ROWS>
 __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16* __restrict__ w, int rows,
                                                              const void* __restrict__ xv, int tokens,
                                                              float* __restrict__ logits, int stride) {
   extern __shared__ __align__(128) uint8_t smem[];
-  constexpr int kXPitch = router_tile_pitch<XBF16>(), kBuf = router_tile_buf<XBF16>(), kChunks = H / kRtChunk;
+  constexpr int kXPitch = router_tile_pitch<XBF16>(), kBuf = router_tile_buf<XBF16, ROWS>(), kChunks = H / kRtChunk;
   pdl_launch_dependents();
   pdl_wait_prior();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row_base = blockIdx.x * kRtRows, tok_base = blockIdx.y * kRtTok;
+  const int row_base = blockIdx.x * ROWS, tok_base = blockIdx.y * kRtTok;
   // a warp copies two weight rows and two token rows of a chunk; rows and tokens beyond the end repeat the last one
   // (they are computed and not stored)
   auto fetch = [&](int c) {
@@ -237,8 +240,8 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       const int r = warp + 16 * p;
-      cp_async_16(buf + r * kRtWPitch + 16 * lane, w + size_t(min(row_base + r, rows - 1)) * H + kRtChunk * c + 8 * lane);
-      uint8_t* xd = buf + kRtRows * kRtWPitch + r * kXPitch + 16 * lane;
+      if (r < ROWS) cp_async_16(buf + r * kRtWPitch + 16 * lane, w + size_t(min(row_base + r, rows - 1)) * H + kRtChunk * c + 8 * lane);
+      uint8_t* xd = buf + ROWS * kRtWPitch + r * kXPitch + 16 * lane;
       const size_t at = size_t(min(tok_base + r, tokens - 1)) * H + kRtChunk * c;
       if constexpr (XBF16) {
         cp_async_16(xd, static_cast<const __nv_bfloat16*>(xv) + at + 8 * lane);
@@ -249,13 +252,13 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // thread = rows rg + 4 j (j = 0..7, pairs of neighbouring j) x tokens tg + 8 t (t = 0..3)
+  // thread = rows rg + 4 j (j = 0..ROWS / 4 - 1, pairs of neighbouring j) x tokens tg + 8 t (t = 0..3)
   const int rg = lane >> 3, tg = lane & 7;
-  uint64_t acc[2][4][4];  // [lane class warp, warp + 16][row pair][token]
+  uint64_t acc[2][ROWS / 8][4];  // [lane class warp, warp + 16][row pair][token]
 #pragma unroll
   for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < ROWS / 8; ++r)
 #pragma unroll
       for (int t = 0; t < 4; ++t) acc[c][r][t] = 0;
   fetch(0);
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
       uint64_t xx[4][4];                  // token values, both halves alike: made once, used by four row pairs
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const uint8_t* xp = buf + kRtRows * kRtWPitch + (tg + 8 * t) * kXPitch + (8 * piece + e) * (XBF16 ? 2 : 4);
+        const uint8_t* xp = buf + ROWS * kRtWPitch + (tg + 8 * t) * kXPitch + (8 * piece + e) * (XBF16 ? 2 : 4);
         uint32_t v[4];
         if constexpr (XBF16) {
           const uint2 a = *reinterpret_cast<const uint2*>(xp);
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
         for (int i = 0; i < 4; ++i) xx[t][i] = pack_f32x2(v[i], v[i]);
       }
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < ROWS / 8; ++r) {
         const uint2 a = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r) * kRtWPitch + 16 * piece + 2 * e);
         const uint2 b = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r + 4) * kRtWPitch + 16 * piece + 2 * e);
         const uint64_t wp[4] = {pack_f32x2(a.x << 16, b.x << 16), pack_f32x2(a.x & 0xFFFF0000u, b.x & 0xFFFF0000u),
@@ -301,24 +304,24 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
   __syncthreads();
   float* part = reinterpret_cast<float*>(smem);  // [warp][token][row]
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < ROWS / 8; ++r)
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const float2 a = *reinterpret_cast<const float2*>(&acc[0][r][t]), b = *reinterpret_cast<const float2*>(&acc[1][r][t]);
-      float* q = part + (warp * kRtTok + tg + 8 * t) * kRtRows + rg + 8 * r;
+      float* q = part + (warp * kRtTok + tg + 8 * t) * ROWS + rg + 8 * r;
       q[0] = a.x + b.x;
       q[4] = a.y + b.y;
     }
   __syncthreads();
-  for (int o = tid; o < kRtRows * kRtTok; o += 512) {
+  for (int o = tid; o < ROWS * kRtTok; o += 512) {
     float v[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = part[i * kRtRows * kRtTok + o];
+    for (int i = 0; i < 16; ++i) v[i] = part[i * ROWS * kRtTok + o];
 #pragma unroll
     for (int n = 8; n >= 1; n >>= 1)
 #pragma unroll
       for (int i = 0; i < n; ++i) v[i] += v[i + n];
-    const int t = tok_base + o / kRtRows, r = row_base + (o & (kRtRows - 1));
+    const int t = tok_base + o / ROWS, r = row_base + (o & (ROWS - 1));
     if (t < tokens && r < rows) logits[size_t(t) * stride + r] = v[0];
   }
 }
@@ -1380,25 +1383,30 @@ int32_t fb_router_logits(const void* w_bf16, int32_t rows, const void* x, int32_
   if (!w_bf16 || !x || !logits || rows <= 0 || tokens <= 0 || logits_stride < rows)
     return invalid("router_logits: bad arguments");
   if (tokens > kMaxTok) {
-    static PerDeviceOnce once;
-    const cudaError_t attr = per_device_once(once, [] {
-      cudaError_t a = opt_in_smem(router_tile_kernel<true>, router_tile_smem<true>());
-      return a == cudaSuccess ? opt_in_smem(router_tile_kernel<false>, router_tile_smem<false>()) : a;
-    });
-    if (attr != cudaSuccess) {
-      set_error("router_logits: shared-memory opt-in: %s", cudaGetErrorString(attr));
-      return int32_t(attr);
-    }
-    const dim3 tiles((rows + kRtRows - 1) / kRtRows, (tokens + kRtTok - 1) / kRtTok);
-    const auto* wb = static_cast<const __nv_bfloat16*>(w_bf16);
+    // Tiles of fewer rows while they run as one wave (513 rows, us: 17 tokens 26.7 -> 14.6, 40 27.1 -> 19.2, 100 28.0 ->
+    // 20.2); beyond that each wave of smaller blocks costs as much as it saves.
+    const int tok_tiles = (tokens + kRtTok - 1) / kRtTok;
+    auto tiles = [&](int r) { return ((rows + r - 1) / r) * tok_tiles; };
+    auto launch = [&](auto kernel, PerDeviceOnce& once, int r, int smem) {
+      cudaError_t a = per_device_once(once, [&] { return opt_in_smem(kernel, smem); });
+      if (a == cudaSuccess)
+        a = launch_pdl(kernel, dim3((rows + r - 1) / r, tok_tiles), dim3(512), size_t(smem), as_stream(stream),
+                       static_cast<const __nv_bfloat16*>(w_bf16), rows, x, tokens, logits, logits_stride);
+      return a;
+    };
+    static PerDeviceOnce once[6];
+    const bool bf = x_dtype == FB_DT_BF16;
     const cudaError_t e =
-        x_dtype == FB_DT_BF16
-            ? launch_pdl(router_tile_kernel<true>, tiles, dim3(512), size_t(router_tile_smem<true>()), as_stream(stream),
-                         wb, rows, x, tokens, logits, logits_stride)
-            : launch_pdl(router_tile_kernel<false>, tiles, dim3(512), size_t(router_tile_smem<false>()),
-                         as_stream(stream), wb, rows, x, tokens, logits, logits_stride);
-    if (e != cudaSuccess) return check_launch("router_logits");
-    return 0;
+        tiles(8) <= sm_count()    ? bf ? launch(router_tile_kernel<true, 8>, once[0], 8, router_tile_smem<true, 8>())
+                                       : launch(router_tile_kernel<false, 8>, once[1], 8, router_tile_smem<false, 8>())
+        : tiles(16) <= sm_count() ? bf ? launch(router_tile_kernel<true, 16>, once[2], 16, router_tile_smem<true, 16>())
+                                       : launch(router_tile_kernel<false, 16>, once[3], 16, router_tile_smem<false, 16>())
+        : bf                      ? launch(router_tile_kernel<true, 32>, once[4], 32, router_tile_smem<true, 32>())
+                                  : launch(router_tile_kernel<false, 32>, once[5], 32, router_tile_smem<false, 32>());
+    if (e == cudaSuccess) return 0;
+    set_error("router_logits: %s", cudaGetErrorString(e));
+    cudaGetLastError();
+    return int32_t(e);
   }
   const dim3 grid((rows + 3) / 4), block(128);
   cudaError_t e = x_dtype == FB_DT_BF16

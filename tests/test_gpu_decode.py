@@ -828,3 +828,10 @@ def test_one_call_branch_at_the_sizes_of_its_shared_expert(inter_s, tokens):
     # the routed sum of the same call is the plain layer's: one fp32 addition lies between them
     total = routed.cpu().numpy() + ysh_gpu
     assert np.all(np.abs(got - total) <= 2.0 ** -22 * (np.abs(routed.cpu().numpy()) + np.abs(ysh_gpu) + np.abs(got)))
+
+
+@pytest.mark.parametrize("rows,tokens,bf16", [(513, 64, False), (513, 97, True), (513, 128, False), (513, 129, True), (72, 530, True)])
+def test_wide_router_at_the_edges_of_its_tile_heights(rows, tokens, bf16):
+    """The last token counts of the 8- and 16-row tiles, the first of the next height, and a ragged last tile of each:
+    the bits of slices of at most 16 tokens."""
+    test_wide_router_gives_the_bits_of_the_narrow_one(rows, tokens, bf16)
