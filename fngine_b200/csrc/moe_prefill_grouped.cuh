@@ -334,12 +334,12 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int I = A.L.inter;
   const int k_steps = (DOWN ? I : H) / kBK, rounds = (k_steps + 3) / 4;
-  // gate/up: 128 intermediate rows are two units here, of 64 gate and 64 up rows each
-  const int n_units = DOWN ? *A.n_units : 2 * *A.n_units;
   // (IQ3_S down comes at intermediate 512 only: its row length is a constant of the copies' addresses)
   const int row_bytes = kIq3s ? (DOWN ? 512 : H) / 256 * 110 : (DOWN ? I : H) / 32 * 18;
   const Abort ab{&bars->abort, A.status};
 
+  // (not from down: combine blocks that sit early on the multiprocessors that are done first made 8192 tokens 1.5 % slower)
+  if constexpr (!DOWN) pdl_launch_dependents();
   if constexpr (kIq3s) {
     for (int i = tid; i < 512 * 4; i += kGgThreads) {  // 16 bytes = eight lanes' copies of an entry
       const uint32_t p = c_iq3s_grid_packed[(i >> 3) | ((i & 4) << 6)];
@@ -378,6 +378,9 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  pdl_wait_prior();
+  // gate/up: 128 intermediate rows are two units here, of 64 gate and 64 up rows each
+  const int n_units = DOWN ? *A.n_units : 2 * *A.n_units;
   auto unit_at = [&](int u) -> int4 {  // {expert, first weight row, first pair, tokens}
     const int per_tile = DOWN ? H / kTileM : I / 64, tile = DOWN ? u / (H / kTileM) : I == 512 ? u / 8 : u / 10;
     int4 un = A.tiles[tile];
@@ -693,24 +696,28 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
   }
 }
 
-// Token rows in pair order: xg[p] = x[token of p]. One warp per token reads its row once and writes it to the token's
-// pairs: the writes (420 MB at 8192 tokens) are the cost. (A warp per pair took 100 us there.)
-__global__ void __launch_bounds__(256) scatter_rows_kernel(const __nv_bfloat16* __restrict__ x,
-                                                           const int32_t* __restrict__ token_pair, int tokens,
-                                                           __nv_bfloat16* __restrict__ xg) {
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+// Token rows in pair order: xg[p] = x[token of p]. A warp reads its token's row (1 / PARTS of it) once and writes it to the
+// token's pairs: the writes (420 MB at 8192 tokens) are the cost. (A warp per pair took 100 us there.)
+template <int PARTS>
+__global__ void __launch_bounds__(128) scatter_rows_kernel(const __nv_bfloat16* x, const int32_t* token_pair, int tokens,
+                                                           __nv_bfloat16* xg) {
+  pdl_launch_dependents();
+  pdl_wait_prior();
+  constexpr int kPieces = H / 256 / PARTS;
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), t = w / PARTS, lane = threadIdx.x & 31;
   if (t >= tokens) return;
-  const uint4* src = reinterpret_cast<const uint4*>(x + size_t(t) * H);
+  const int at = 32 * kPieces * (w - t * PARTS) + lane;
+  const uint4* src = reinterpret_cast<const uint4*>(x + size_t(t) * H) + at;
   const int mine = lane < kTopK ? token_pair[t * kTopK + lane] : -1;
-  uint4 v[H / 256];
+  uint4 v[kPieces];
 #pragma unroll
-  for (int i = 0; i < H / 256; ++i) v[i] = __ldg(src + 32 * i + lane);
+  for (int i = 0; i < kPieces; ++i) v[i] = src[32 * i];
 #pragma unroll
   for (int k = 0; k < kTopK; ++k) {
     const int p = __shfl_sync(0xffffffffu, mine, k);
     if (p < 0) continue;  // a pair of another rank
-    uint4* dst = reinterpret_cast<uint4*>(xg + size_t(p) * H);
+    uint4* dst = reinterpret_cast<uint4*>(xg + size_t(p) * H) + at;
 #pragma unroll
-    for (int i = 0; i < H / 256; ++i) dst[32 * i + lane] = v[i];
+    for (int i = 0; i < kPieces; ++i) dst[32 * i] = v[i];
   }
 }
