@@ -147,7 +147,9 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t pair) {
 __global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfloat16* x, int K, uint8_t* codes,
                                                                   uint8_t* codes_lo, float* scales, uint32_t* status) {
   pdl_wait_prior();
-  pdl_launch_dependents();  // (behind the wait: ahead of it the GEMM's early loads compete with the call before)
+  // (behind the wait: fp8_mid_kernel asks for its weights, which the kernel ahead of this one may have written, before it
+  // waits for this one; nor do its early loads compete with the call before)
+  pdl_launch_dependents();
   if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;  // of the GEMM that follows
   const int t = blockIdx.x;
   const __nv_bfloat16* row = x + size_t(t) * K;
@@ -758,8 +760,10 @@ constexpr int kSplitPer = 5;  // 16-byte pieces of a row a thread keeps in regis
 __global__ void __launch_bounds__(256) fp8_split_tokens_kernel(const __nv_bfloat16* x, int T, int K, uint8_t* pieces,
                                                                float* tok_scale, int32_t* tickets, int n_tickets,
                                                                uint32_t* status) {
-  pdl_launch_dependents();
+  // The trigger stands behind the wait: the projection asks for its weights before it waits for this kernel, and the
+  // kernel ahead of this one may have written them.
   pdl_wait_prior();
+  pdl_launch_dependents();
   const int t = blockIdx.x, tid = threadIdx.x;
   if (t == 0) {
     for (int i = tid; i < n_tickets; i += 256) tickets[i] = 0;
@@ -999,7 +1003,8 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (elect_one()) {
       // The weight codes do not depend on the kernel launched just before (the activation split), so
       // the first ring's worth of them is requested before waiting for it: under programmatic
-      // dependent launch this kernel is resident while the split still runs.
+      // dependent launch this kernel is resident while the split still runs. (All kernels ahead of the split are
+      // complete: it waits for them before it lets this one start.)
       const int pre = end - begin < kDecStages ? int(end - begin) : kDecStages;
       for (int i = 0; i < pre; ++i) {
         const long long pos = begin + i;
@@ -1482,7 +1487,8 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         tma_load_2d(st + 64 * BK, &map_w, (kb0 + i) * BK, r1, &bars->full[i % S]);
       };
       const uint32_t bytes = uint32_t(kDecStageA + PIECES * boxes * 32 * BK);
-      // the weights do not come from the kernel launched just before (the activation pieces do)
+      // the weights do not come from the kernel launched just before (the activation pieces do), and all kernels ahead of
+      // that one are complete: it waits for them before it lets this one start
       const int pre = min(nkb, S);
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(&bars->full[i], bytes);

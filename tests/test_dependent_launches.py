@@ -1,0 +1,55 @@
+"""Rules that the CUDA sources keep where launches are chained by programmatic dependent launch. A kernel launched that way
+may start while its predecessor runs, so what keeps its reads in order is in the source and can be checked there (a
+race on the GPU shows by chance only). No GPU."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "fngine_b200", "csrc")
+KERNEL = re.compile(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)\s*)?(\w+)\s*\(")
+
+
+def _block(text, at, opening, closing):
+    """The text from the bracket at `at` to its match, and the position behind it."""
+    depth = 0
+    for i in range(at, len(text)):
+        if text[i] == opening:
+            depth += 1
+        elif text[i] == closing:
+            depth -= 1
+            if depth == 0:
+                return text[at:i + 1], i + 1
+    raise AssertionError("unbalanced source")
+
+
+def kernels():
+    """name -> (parameters, body) of every kernel, comments removed."""
+    found = {}
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        with open(os.path.join(CSRC, name)) as f:
+            text = re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+        for m in KERNEL.finditer(text):
+            params, end = _block(text, m.end() - 1, "(", ")")
+            body, _ = _block(text, text.index("{", end), "{", "}")
+            found[m.group(1)] = (params, body)
+    return found
+
+
+KERNELS = kernels()
+CHAINED = sorted(n for n, (_, body) in KERNELS.items() if "pdl_wait_prior()" in body)
+
+
+def test_the_sources_are_read():
+    assert len(KERNELS) > 25 and {"experts_kernel", "grouped_kernel", "fp8_mid_kernel", "pf_combine_kernel"} <= set(CHAINED)
+
+
+@pytest.mark.parametrize("split", ["fp8_split_tokens_kernel", "fp8_quantize_tokens_kernel"])
+def test_a_split_waits_before_it_lets_the_projection_start(split):
+    """fp8_decode_kernel and fp8_mid_kernel ask for weight codes before their own wait. That is in order only if everything
+    ahead of the activation split, which may have written the codes, is complete when the split lets them start."""
+    body = KERNELS[split][1]
+    assert body.count("pdl_wait_prior()") == 1 and body.count("pdl_launch_dependents()") == 1
+    assert body.index("pdl_wait_prior()") < body.index("pdl_launch_dependents()")

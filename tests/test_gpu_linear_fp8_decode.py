@@ -154,6 +154,31 @@ def test_activation_pieces_are_exact():
     assert np.all(np.log2(scales[[0, 1, 3, 4, 5]]) == np.round(np.log2(scales[[0, 1, 3, 4, 5]])))  # powers of two
 
 
+@pytest.mark.parametrize("T,n,k", [(1, 24832, 1024), (9, 19080, 2560)])
+def test_projection_right_behind_the_kernel_that_wrote_its_weights(T, n, k):
+    """More row tiles than multiprocessors, whose kernel asks for weight codes ahead of its own wait: codes copied in by
+    the call before on the same stream, no synchronization between, give the bits of synchronized calls."""
+    torch = _torch()
+    from fngine_b200 import linear
+    weights = [make_weight(torch, 40 + i, n, k, False) for i in range(2)]
+    x = bf16_tensor(torch, synth.activations(700 + T, T, hidden=k))
+    work = linear.linear_fp8_decode_workspace(weights[0])
+    want = [torch.empty(T, n, dtype=torch.float32, device="cuda") for _ in weights]
+    for w, o in zip(weights, want):
+        linear.linear_fp8_decode(x, w, linear.store_f32(o), work)
+        torch.cuda.synchronize()
+    live = linear.Fp8RowWeight(weights[0].codes.clone(), weights[0].scales.clone())
+    outs = [torch.empty_like(want[0]) for _ in range(12)]
+    for i, o in enumerate(outs):
+        live.codes.copy_(weights[i % 2].codes)
+        live.scales.copy_(weights[i % 2].scales)
+        live.codes[-1:].copy_(weights[i % 2].codes[-1:])  # (the last kernel ahead of the projection writes codes)
+        linear.linear_fp8_decode(x, live, linear.store_f32(o), work)
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        assert torch.equal(o, want[i % 2]), i
+
+
 def test_linear_fp8_decode_argument_errors():
     torch = _torch()
     import ctypes
