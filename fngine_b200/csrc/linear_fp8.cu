@@ -913,7 +913,7 @@ __device__ __forceinline__ void dec_emit(const DecArgs& a, int m, int rl, int et
       for (int t = 0; t < 8; ++t)
         if (h + t < a.T) {
           const float val = v[h + t] * ts[h + t] * ws;
-          const float4 g = __ldg(reinterpret_cast<const float4*>(a.inj + size_t(h + t) * 4));
+          const float4 g = *reinterpret_cast<const float4*>(a.inj + size_t(h + t) * 4);
           xs[(size_t(h + t) * 4 + 0) * n] = fmaf(g.x, val, x4[t][0]);
           xs[(size_t(h + t) * 4 + 1) * n] = fmaf(g.y, val, x4[t][1]);
           xs[(size_t(h + t) * 4 + 2) * n] = fmaf(g.z, val, x4[t][2]);
@@ -1073,14 +1073,14 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     float ts[kDecTok];
 #pragma unroll
     for (int t4 = 0; t4 < kDecTok / 4; ++t4) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(a.tok_scale) + t4);
+      const float4 f = reinterpret_cast<const float4*>(a.tok_scale)[t4];
       ts[4 * t4] = f.x, ts[4 * t4 + 1] = f.y, ts[4 * t4 + 2] = f.z, ts[4 * t4 + 3] = f.w;
     }
     if (a.kind == FB_EPI_SHARED_SCALE) {  // sigmoid(gate logit) folded into the token scale
       float gl[kDecTok];
 #pragma unroll
       for (int t = 0; t < kDecTok; ++t)  // all loads first: the division below branches, and loads do not move across it
-        gl[t] = __ldg(a.gate_logit + size_t(t < a.T ? t : 0) * a.gate_stride);
+        gl[t] = a.gate_logit[size_t(t < a.T ? t : 0) * a.gate_stride];
 #pragma unroll
       for (int t = 0; t < kDecTok; ++t) ts[t] /= 1.0f + expf(-gl[t]);
     }
@@ -1187,7 +1187,7 @@ __device__ __forceinline__ void split_pair_e5m2(float a, float b, uint32_t (&c)[
 }
 
 __global__ void __launch_bounds__(kSmallThreads, 1)
-fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* __restrict__ x,
+fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* x,
                  const __grid_constant__ DecArgs a, int cluster) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

@@ -6,6 +6,10 @@
 //   down     partial[pair][n] = w_pair * (down_n . q8(h[pair]))
 //   combine  y[t] = sum of token t's partials in slot order (+ shared, + residual write)
 //
+// Kernels of this path start while their predecessor runs out (programmatic dependent launch) and wait for it before they
+// touch global memory. None of them reads through const __restrict__ pointers or __ldg: such loads count as invariant
+// and may be moved ahead of the wait.
+//
 // gate_up and down are one persistent kernel, one CTA per SM (moe_decode_experts.cuh): a producer thread streams
 // tiles of the expert blob into a three-stage shared-memory ring with 1-D bulk async copies (TMA, no multicast)
 // signalled through mbarriers; consumer warps decode the blocks from shared memory and accumulate exact int8 dot
@@ -126,9 +130,8 @@ __device__ __forceinline__ void quantize_row_planar(int act, int k, LoadF load, 
 // weights held in registers, tokens taken four at a time so that their loads overlap; the 32 lane
 // sums are added by a butterfly. Fixed order: repeated calls are bitwise identical.
 template <bool XBF16>
-__global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* __restrict__ w, int rows,
-                                                     const void* __restrict__ xv, int tokens,
-                                                     float* __restrict__ logits, int stride) {
+__global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* w, int rows, const void* xv, int tokens,
+                                                     float* logits, int stride) {
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -224,9 +227,8 @@ __device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
 }
 
 template <bool XBF16, int ROWS>
-__global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16* __restrict__ w, int rows,
-                                                             const void* __restrict__ xv, int tokens,
-                                                             float* __restrict__ logits, int stride) {
+__global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16* w, int rows, const void* xv,
+                                                             int tokens, float* logits, int stride) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kXPitch = router_tile_pitch<XBF16>(), kBuf = router_tile_buf<XBF16, ROWS>(), kChunks = H / kRtChunk;
   pdl_launch_dependents();
@@ -626,10 +628,9 @@ struct SelectArgs {
 // Stand-alone selection (the reference's moe_select_publish): block 0 routes, blocks 1..T quantize
 // one token's activations each.
 template <bool XBF16>
-__global__ void __launch_bounds__(512) select_kernel(const float* __restrict__ logits, int logits_stride,
-                                                     const void* __restrict__ xv, const int32_t* __restrict__ slot_of,
-                                                     int T, fb_moe_decode_workspace ws,
-                                                     uint32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(512) select_kernel(const float* logits, int logits_stride, const void* xv,
+                                                     const int32_t* slot_of, int T, fb_moe_decode_workspace ws,
+                                                     uint32_t* counts) {
   pdl_launch_dependents();
   pdl_wait_prior();
   if (blockIdx.x > 0) {
@@ -697,9 +698,9 @@ constexpr int kRouteBlocks = kRouteGroups * kRouteSplits;
 static_assert(kRouteSlice == 320, "lane layout below: two 128-element chunks and a 64-element tail");
 
 template <bool XBF16, bool EP, bool SHARED = false>
-__global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* __restrict__ w, const void* __restrict__ xv,
-                                                    int T, float* __restrict__ logits, int stride,
-                                                    fb_moe_decode_workspace ws, EpRouteArgs ep, SharedRouteArgs sh) {
+__global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* w, const void* xv, int T, float* logits,
+                                                       int stride, fb_moe_decode_workspace ws, EpRouteArgs ep,
+                                                       SharedRouteArgs sh) {
   pdl_launch_dependents();
   pdl_wait_prior();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -986,7 +987,7 @@ static_assert(kTT == 2 && sizeof(StageMeta) == 48, "three vector stores");
 // flight before the first block is quantized (the finishing warp waits on this chain: Q8_0 rows taken block by block, twenty
 // round trips at 640, cost a layer of one token 8 us). `out` in global or shared memory, 16-byte aligned.
 template <int I>
-__device__ __forceinline__ void quantize_h_row(const float* __restrict__ h, int down_act, uint8_t* out) {
+__device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uint8_t* out) {
   constexpr int kPasses = (I + 255) / 256;
   const int lane = threadIdx.x & 31;
   float v[kPasses][8];
@@ -1059,9 +1060,8 @@ __device__ __forceinline__ float sum_partials(const fb_moe_decode_workspace& ws,
   return y;
 }
 
-__global__ void __launch_bounds__(256) combine_kernel(fb_moe_decode_workspace ws, const float* __restrict__ y_shared,
-                                                      const float* __restrict__ inj, float* __restrict__ X,
-                                                      float* __restrict__ y_out, const float* __restrict__ ablate,
+__global__ void __launch_bounds__(256) combine_kernel(fb_moe_decode_workspace ws, const float* y_shared,
+                                                      const float* inj, float* X, float* y_out, const float* ablate,
                                                       float ablate_scale) {
   pdl_launch_dependents();
   pdl_wait_prior();
@@ -1094,10 +1094,18 @@ __global__ void __launch_bounds__(256) combine_kernel(fb_moe_decode_workspace ws
   float y = sum_partials(ws, t, np, n);
   if (ablate) y -= ablate_scale * ablate[n] * proj;
   if (y_shared) y += y_shared[size_t(t) * H + n];
+  float x[4], g[4];  // (all loads ahead of the stores: they may meet for all the compiler knows)
+  if (X) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      x[s] = X[(size_t(t) * 4 + s) * H + n];
+      g[s] = inj[t * 4 + s];
+    }
+  }
   if (y_out) y_out[size_t(t) * H + n] = y;
   if (X) {
 #pragma unroll
-    for (int s = 0; s < 4; ++s) X[(size_t(t) * 4 + s) * H + n] += inj[t * 4 + s] * y;
+    for (int s = 0; s < 4; ++s) X[(size_t(t) * 4 + s) * H + n] = x[s] + g[s] * y;
   }
 }
 
@@ -1117,8 +1125,7 @@ struct SharedDownArgs {
 };
 constexpr int kCsCols = 16, kCsMaxK = kSharedMaxInter;
 __global__ void __launch_bounds__(256) combine_shared_kernel(fb_moe_decode_workspace ws, SharedDownArgs sh, int T,
-                                                             const float* __restrict__ inj, float* __restrict__ X,
-                                                             float* __restrict__ y_out) {
+                                                             const float* inj, float* X, float* y_out) {
   extern __shared__ __align__(16) float s_h[];  // [token][k]
   __shared__ float s_y[kMaxTok][kCsCols];
   pdl_launch_dependents();
@@ -1141,12 +1148,15 @@ __global__ void __launch_bounds__(256) combine_shared_kernel(fb_moe_decode_works
       for (int r = 0; r < 2; ++r)
         codes[c][r] = reinterpret_cast<const uint32_t*>(sh.codes + size_t(n0 + 2 * warp + r) * sh.k)[c * 32 + lane];
     }
-  float routed = 0.0f, xs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float routed = 0.0f, xs[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   if (t_out < T) {
     routed = sum_partials(ws, t_out, min(max(ws.work->token_pair_count[t_out], 0), kTopK), n);
     if (X) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) xs[i] = X[(size_t(t_out) * 4 + i) * H + n];
+      for (int i = 0; i < 4; ++i) {
+        xs[i] = X[(size_t(t_out) * 4 + i) * H + n];
+        gs[i] = inj[t_out * 4 + i];
+      }
     }
   }
   for (int i = tid; i < T * sh.k / 8; i += 256) {
@@ -1203,7 +1213,7 @@ __global__ void __launch_bounds__(256) combine_shared_kernel(fb_moe_decode_works
     if (y_out) y_out[size_t(t_out) * H + n] = y;
     if (X) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) X[(size_t(t_out) * 4 + i) * H + n] = xs[i] + inj[t_out * 4 + i] * y;
+      for (int i = 0; i < 4; ++i) X[(size_t(t_out) * 4 + i) * H + n] = xs[i] + gs[i] * y;
     }
   }
 }
@@ -1235,7 +1245,7 @@ __global__ void __launch_bounds__(256) sum_ranks_kernel(const float* __restrict_
 // this rank owns then read the partial rows of all ranks and add them in rank order.
 __global__ void __launch_bounds__(256) ep_combine_exchange_kernel(fb_moe_decode_workspace ws, fb_ep_peers peers, int tpr,
                                                                   int parity, uint32_t step, uint32_t spin_limit,
-                                                                  float* __restrict__ y_local) {
+                                                                  float* y_local) {
   pdl_launch_dependents();
   pdl_wait_prior();
   const int t = blockIdx.y;

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) pf_import_kernel(const int32_t* in_e, con
 // units of unequal cost was up to a sixth above the mean.
 constexpr int kTileBuckets = kTileN / 16;
 template <int TILE>
-__device__ __forceinline__ void list_tiles(int expert, int first_pair, int count, int* s_cursor, int4* __restrict__ tiles,
+__device__ __forceinline__ void list_tiles(int expert, int first_pair, int count, int* s_cursor, int4* tiles,
                                            int max_tiles) {
   const int full = count / TILE, rest = count - full * TILE;
   if (full) {

@@ -501,7 +501,7 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
             }
           } else {  // an expert table may hold any even address
             for (uint32_t i = lane; i < bytes / 2; i += 32)
-              reinterpret_cast<unsigned short*>(dst)[i] = __ldg(reinterpret_cast<const unsigned short*>(src) + i);
+              reinterpret_cast<unsigned short*>(dst)[i] = reinterpret_cast<const unsigned short*>(src)[i];
             fence_proxy_async();  // (a later unit's bulk copy will write here)
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->raw_full[s]);

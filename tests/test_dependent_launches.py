@@ -53,3 +53,22 @@ def test_a_split_waits_before_it_lets_the_projection_start(split):
     body = KERNELS[split][1]
     assert body.count("pdl_wait_prior()") == 1 and body.count("pdl_launch_dependents()") == 1
     assert body.index("pdl_wait_prior()") < body.index("pdl_launch_dependents()")
+
+
+@pytest.mark.parametrize("name", CHAINED)
+def test_no_load_of_a_chained_kernel_may_move_ahead_of_its_wait(name):
+    """Loads through const __restrict__ parameters and by __ldg count as invariant: the compiler may move them ahead of the
+    wait, where the predecessor's data is not there yet."""
+    params, body = KERNELS[name]
+    assert "__restrict__" not in params and "__ldg(" not in body
+
+
+def test_no_helper_of_the_chained_kernels_uses_invariant_loads():
+    for name in sorted(os.listdir(CSRC)):
+        if name == "probes.cu":  # (ordinary launches)
+            continue
+        with open(os.path.join(CSRC, name)) as f:
+            text = re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+        assert "__ldg(" not in text, name
+        for m in re.finditer(r"__device__ __forceinline__[^;{]*\([^{;]*\{", text):
+            assert "__restrict__" not in m.group(0), (name, m.group(0)[:80])

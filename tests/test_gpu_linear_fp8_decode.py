@@ -179,6 +179,42 @@ def test_projection_right_behind_the_kernel_that_wrote_its_weights(T, n, k):
         assert torch.equal(o, want[i % 2]), i
 
 
+@pytest.mark.parametrize("T", [1, 5, 16])
+def test_projection_reads_what_the_kernel_ahead_of_it_wrote(T):
+    """A projection whose activations the projection before it writes, chained in a CUDA graph and replayed on changing
+    inputs: the bits of synchronized calls every time."""
+    torch = _torch()
+    from fngine_b200 import linear
+    gu, dn = make_weight(torch, 61, 1280, 2560, True), make_weight(torch, 62, 2560, 640, True)
+    works = [linear.linear_fp8_decode_workspace(w) for w in (gu, dn)]
+    x = torch.empty(T, 2560, dtype=torch.bfloat16, device="cuda")
+    h = torch.empty(T, 640, dtype=torch.bfloat16, device="cuda")
+    y = torch.empty(T, 2560, dtype=torch.float32, device="cuda")
+    inputs = [bf16_tensor(torch, synth.activations(900 + i, T, hidden=2560) * np.float32(2.0 ** (3 * (i % 3)))) for i in range(16)]
+    epis = linear.swiglu(h), linear.store_f32(y)
+    want = []
+    for v in inputs:
+        x.copy_(v)
+        torch.cuda.synchronize()
+        for src, w, e, k in zip((x, h), (gu, dn), epis, works):
+            linear.linear_fp8_decode(src, w, e, k)
+            torch.cuda.synchronize()
+        want.append(y.clone())
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        for src, w, e, k in zip((x, h), (gu, dn), epis, works):
+            linear.linear_fp8_decode(src, w, e, k)
+    for turn in range(4):
+        got = []
+        for v in inputs:
+            x.copy_(v)
+            graph.replay()
+            got.append(y.clone())
+        torch.cuda.synchronize()
+        for i, g in enumerate(got):
+            assert torch.equal(g, want[i]), (turn, i)
+
+
 def test_linear_fp8_decode_argument_errors():
     torch = _torch()
     import ctypes
