@@ -163,6 +163,13 @@ __device__ __forceinline__ float ld_cluster_f32(const float* local, uint32_t cta
   return v;
 }
 
+// A 4-byte store into the shared memory of the CTA with rank `cta`, at the address `local` has in this CTA's window.
+__device__ __forceinline__ void st_cluster_u32(const void* local, uint32_t cta, uint32_t v) {
+  uint32_t addr;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(cta));
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float(uint32_t(b) << 16); }
 
 // Launch with the programmatic-stream-serialization attribute (the kernel calls pdl_wait_prior()

@@ -1146,7 +1146,8 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // traffic. Here a CLUSTER owns a row tile, its CTAs equal shares of K; each CTA splits its own part of the activations
 // straight into operand rows in shared memory (the token scale is then the CTA's own, so no pass over whole rows comes
 // first), and the partial tiles meet through distributed shared memory, added in CTA order (fixed: repeated calls are
-// bitwise identical). One launch, no workspace.
+// bitwise identical). One launch; of the workspace it uses the status word only. A CTA whose wait runs out tells the
+// others of its cluster ahead of the barrier that ends the sums, and none of them stores anything.
 constexpr int kSmallThreads = 512, kSmallMaxKb = 20, kSmallMaxCluster = 8;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallMaxStages = 8;
@@ -1154,7 +1155,8 @@ struct SmallBars {
   uint64_t full[kSmallMaxStages], empty[kSmallMaxStages];
   uint64_t acc;
   uint32_t tmem_base;
-  int abort;
+  int abort;   // a wait of this CTA has run out
+  int failed;  // a partial tile of the cluster is missing: nothing is stored
   float red[kSmallWarps];
   float scale[kDecTok];
 };
@@ -1219,7 +1221,7 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
       mbar_init(&bars->empty[i], 1);
     }
     mbar_init(&bars->acc, 1);
-    bars->abort = 0;
+    bars->abort = bars->failed = 0;
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&bars->tmem_base, 64);
@@ -1227,7 +1229,9 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+  cluster_arrive();  // (`failed` is cleared: the peers may write it behind their half of this barrier)
   pdl_wait_prior();
+  if (blockIdx.x == 0 && tid == 0) *a.status = 0;  // (the limits of the waits are seconds away)
 
   auto load_stage = [&](int i) {
     uint8_t* st = smem + (i % S) * kDecStageA;
@@ -1290,6 +1294,7 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   }
   fence_proxy_async();
   __syncthreads();
+  cluster_wait();
 
   if (warp == 0) {
     if (elect_one())
@@ -1327,6 +1332,8 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
         if (i < a.T)
           part[i * 128 + rl] = ((__uint_as_float(c[32 + i]) + __uint_as_float(c[16 + i])) + __uint_as_float(c[i])) * bars->scale[i];
       tc_fence_before();
+    } else if (lane < cluster) {
+      st_cluster_u32(&bars->failed, uint32_t(lane), 1u);
     }
   }
   // The outputs of the tile are dealt out over the cluster's threads: consecutive threads, consecutive rows. What an
@@ -1366,9 +1373,10 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
     }
   };
   fetch();
-  if (cluster > 1) cluster_sync();
-  else __syncthreads();
-  for (int o = first; o < n_out;) {
+  __syncwarp();  // (warps 0 and 1 came through one lane's branches: the barrier wants them whole)
+  cluster_sync();
+  const bool complete = *reinterpret_cast<volatile int*>(&bars->failed) == 0;
+  for (int o = first; complete && o < n_out;) {
     const bool last = o + cluster * kSmallThreads >= n_out;
     if (live) {
       float sum = sum_of(tt, r), sum_up = swiglu ? sum_of(tt, r + 64) : 0.0f;
@@ -1400,7 +1408,7 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   }
   tc_fence_before();
   __syncthreads();
-  if (cluster > 1) cluster_sync();  // no CTA leaves while another may still read its partial tile
+  cluster_sync();  // no CTA leaves while another may still read its partial tile
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 64);
@@ -1418,7 +1426,7 @@ struct MidBars {
   uint64_t full[kMidMaxStages], empty[kMidMaxStages];
   uint64_t acc;
   uint32_t tmem_base;
-  int abort;
+  int abort, failed;  // as in SmallBars
 };
 constexpr int kMidSmemMax = 232448;
 // Shared memory of a stage (16 KB of weights, `pieces` tiles of `tok` tokens) and of the whole block; the partial tile
@@ -1458,13 +1466,14 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       mbar_init(&bars->empty[i], 1);
     }
     mbar_init(&bars->acc, 1);
-    bars->abort = 0;
+    bars->abort = bars->failed = 0;
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&bars->tmem_base, 256);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  cluster_arrive();  // (`failed` is cleared: the peers may write it behind their half of this barrier)
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
     if (mbar_test_wait(bar, parity)) return true;
@@ -1477,7 +1486,6 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     return false;
   };
 
-  bool done = true;
   if (warp == 0) {
     if (elect_one()) {
       const int boxes = (nt + 31) >> 5;
@@ -1531,6 +1539,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     }
   }
   __syncwarp();
+  cluster_wait();
   pdl_wait_prior();  // (token scales, and nothing is written before the preceding kernels are done)
   if (a.kind == FB_EPI_GR_WRITE && lane == 0 && m * 128 + 32 * (warp & 3) < a.N) {  // residual streams into L2 meanwhile
     for (int t = rank * 4 + (warp >> 2); t < nt; t += cluster * 4)
@@ -1542,8 +1551,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   {
     // ---------------- the partial tile into shared memory: lane quarter = warp % 4, its four warps take chunks of 16 tokens
     const int q = warp & 3, rl = q * 32 + lane;
-    done = __all_sync(0xffffffffu, wait(&bars->acc, 0));
-    if (done) {
+    if (__all_sync(0xffffffffu, wait(&bars->acc, 0))) {
       tc_fence_after();
       for (int c0 = 16 * (warp >> 2); c0 < n16; c0 += 64) {
         uint32_t c[16];
@@ -1554,10 +1562,13 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           if (c0 + i < nt) part[(c0 + i) * 128 + rl] = __uint_as_float(c[i]);
       }
       tc_fence_before();
+    } else if (lane < cluster) {
+      st_cluster_u32(&bars->failed, uint32_t(lane), 1u);
     }
+    __syncwarp();
   }
-  if (cluster > 1) cluster_sync();
-  else __syncthreads();
+  cluster_sync();
+  const bool complete = *reinterpret_cast<volatile int*>(&bars->failed) == 0;  // (else nothing is stored)
   // ---------------- outputs, dealt out over the cluster's threads: consecutive threads, consecutive rows
   auto sum_of = [&](int t, int r) -> float {
     if (cluster == 1) return part[t * 128 + r];
@@ -1575,7 +1586,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   };
   const int rows = swiglu ? 64 : 128, r = tid & (rows - 1);  // a thread keeps its row (the stride is a multiple of it)
   const int n = (swiglu ? m * 64 : m * 128) + r, limit = swiglu ? half_n : a.N;
-  if (n < limit) {
+  if (complete && n < limit) {
     const float ws0 = row_scale(n), ws1 = swiglu ? row_scale(half_n + n) : 0.0f;
     const int per = kMidThreads / rows;  // tokens per turn of a CTA
 #pragma unroll 2
@@ -1607,7 +1618,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
-  if (cluster > 1) cluster_sync();  // no CTA leaves while another may still read its partial tile
+  cluster_sync();  // no CTA leaves while another may still read its partial tile
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 256);

@@ -1,6 +1,6 @@
 """Rules that the CUDA sources keep where launches are chained by programmatic dependent launch. A kernel launched that way
 may start while its predecessor runs, so what keeps its reads in order is in the source and can be checked there (a
-race on the GPU shows by chance only). No GPU."""
+race on the GPU shows by chance only). The same for what a kernel does once a bounded wait has run out. No GPU."""
 import os
 import re
 
@@ -72,3 +72,18 @@ def test_no_helper_of_the_chained_kernels_uses_invariant_loads():
         assert "__ldg(" not in text, name
         for m in re.finditer(r"__device__ __forceinline__[^;{]*\([^{;]*\{", text):
             assert "__restrict__" not in m.group(0), (name, m.group(0)[:80])
+
+
+@pytest.mark.parametrize("name", ["fp8_small_kernel", "fp8_mid_kernel"])
+def test_a_cluster_with_a_missing_partial_tile_stores_nothing(name):
+    """Every CTA learns of an expired wait anywhere in its cluster at the barrier that ends the sums, and the outputs
+    stand behind that."""
+    body = KERNELS[name][1]
+    tell, learn = body.find("st_cluster_u32(&bars->failed"), body.find("bool complete")
+    assert 0 <= tell < learn
+    barrier = body.rindex("cluster_sync()", 0, learn)
+    guard = re.search(r"(for|if) \([^{]*\bcomplete &&[^{]*\{", body)
+    assert tell < barrier and learn < guard.start()
+    _, end = _block(body, guard.end() - 1, "{", "}")
+    stores = [m.start() for m in re.finditer(r"static_cast<(?:__nv_bfloat16|float)\*>\(a\.out\)", body) if m.start() > barrier]
+    assert stores and all(guard.start() < at < end for at in stores)

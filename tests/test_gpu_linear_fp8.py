@@ -334,3 +334,25 @@ def test_linear_fp8_small_and_middle_widths(T, n, k, kind, path):
     out, again = (e._keep[0] for e in epis)
     compare(torch, out, ref, bf16_out)
     assert torch.equal(out.view(torch.uint8), again.view(torch.uint8))  # repeated calls are bitwise identical
+
+
+@pytest.mark.parametrize("T,n,k", [(1, 640, 512),       # decode width, few row tiles
+                                   (16, 19072, 128),    # decode width, more row tiles than multiprocessors
+                                   (17, 256, 256),      # middle widths
+                                   (1100, 2560, 256)])  # the GEMM of two-SM tiles
+def test_the_status_word_of_a_call_is_its_own(T, n, k):
+    """Workspaces are not initialised by the caller: the status word, where an expired wait is recorded, reads 0 after a
+    call on one full of ones."""
+    torch = _torch()
+    from fngine_b200 import linear
+    weight = make_weight(torch, 5, n, k, False)
+    x = bf16_tensor(torch, synth.activations(6, T, hidden=k))
+    work = linear.linear_fp8_workspace(weight, T)
+    work.fill_(255)
+    out = torch.empty(T, n, dtype=torch.float32, device="cuda")
+    linear.linear_fp8(x, weight, linear.store_f32(out), work)
+    torch.cuda.synchronize()
+    up = lambda v: (v + 255) // 256 * 256
+    at = up(48 * k) + 256 if T <= 16 else up(2 * T * k) + up(4 * T)
+    assert int(work[at:at + 4].view(torch.int32)) == 0
+    compare(torch, out, exact_acc(torch, x.double(), weight), False)
