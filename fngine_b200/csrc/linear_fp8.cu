@@ -1942,8 +1942,15 @@ int32_t fb_linear_fp8_decode(const void* x_bf16, int32_t tokens, const uint8_t* 
   // not fit. A tile that gets one CTA alone splits whole activation rows in every CTA: 13.3 - 16.2 us for 16384 x 2560 at
   // 4 - 16 tokens against 12.1 - 13.4 of the streaming kernel, which keeps it. Fewer than four tiles, which no projection of the engine has, stay with the streaming kernel: its operand
   // rows can be read back from the workspace.)
+  // An output that lies in the activations' memory also stays with the streaming kernel, whose split has read all of them
+  // when the first output is written.
+  const size_t out_values = size_t(tokens) * size_t(n);
+  const size_t out_bytes = kind == FB_EPI_GR_WRITE ? 16 * out_values : kind == FB_EPI_STORE_BF16 ? 2 * out_values
+                           : kind == FB_EPI_SWIGLU ? out_values : 4 * out_values;
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x_bf16), out0 = reinterpret_cast<uintptr_t>(epilogue->out);
+  const bool in_place = out0 < x0 + size_t(tokens) * size_t(k) * 2 && x0 < out0 + out_bytes;
   const int kb = k / BK;
-  if (m_tiles >= 4 && m_tiles <= sm_count()) {
+  if (m_tiles >= 4 && m_tiles <= sm_count() && !in_place) {
     const int* resident = small_clusters();
     if (!resident) {
       set_error("linear_fp8_decode: shared-memory opt-in failed");

@@ -215,6 +215,30 @@ def test_projection_reads_what_the_kernel_ahead_of_it_wrote(T):
             assert torch.equal(g, want[i]), (turn, i)
 
 
+@pytest.mark.parametrize("T,n,k,kind", [(1, 2560, 2560, "store_bf16"), (16, 2560, 2560, "store_bf16"), (7, 1280, 2560, "store_f32"),
+                                        (4, 512, 2560, "swiglu")])
+def test_projection_into_the_memory_of_its_activations(T, n, k, kind):
+    """The activations are read before anything is written: an output that starts inside them holds the product."""
+    torch = _torch()
+    from fngine_b200 import linear
+    weight = make_weight(torch, 88, n, k, True)
+    x = bf16_tensor(torch, synth.activations(31 + T, T, hidden=k))
+    work = linear.linear_fp8_decode_workspace(weight)
+    make = {"store_bf16": linear.store_bf16, "store_f32": linear.store_f32, "swiglu": linear.swiglu}[kind]
+    shape, dt = (T, n // 2 if kind == "swiglu" else n), torch.float32 if kind == "store_f32" else torch.bfloat16
+    values, ref = shape[0] * shape[1], exact_acc(torch, x, weight)
+    if kind == "swiglu":
+        ref = ref[:, :n // 2] / (1.0 + torch.exp(-ref[:, :n // 2])) * ref[:, n // 2:]
+    for first in (0, 16 * (x.numel() // 32)):  # the output at the start of the activations, and from their middle on
+        room = torch.empty(x.numel() + 16 + 2 * values, dtype=torch.bfloat16, device="cuda")
+        xin = room[:x.numel()].view(T, k)
+        xin.copy_(x)
+        out = room[first:first + values * dt.itemsize // 2].view(dt).view(shape)
+        linear.linear_fp8_decode(xin, weight, make(out), work)
+        torch.cuda.synchronize()
+        compare(torch, out, ref, dt == torch.bfloat16)
+
+
 def test_linear_fp8_decode_argument_errors():
     torch = _torch()
     import ctypes
