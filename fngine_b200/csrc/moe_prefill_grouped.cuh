@@ -265,7 +265,7 @@ __device__ __forceinline__ void gg_copy_pieces(uint32_t dst, int pitch, int byte
 }
 template <int FMT, class RowF>
 __device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t align, int lane, const uint8_t* base,
-                                            const int (&piece)[9], RowF row_at) {
+                                            const int (&piece)[9], bool near, RowF row_at) {
   if constexpr (FMT == FB_FMT_IQ3_S) {
     // 28 words from the word that holds the block's first byte (never one that starts behind the matrix)
 #pragma unroll
@@ -278,7 +278,7 @@ __device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t al
     return true;
   } else {
     constexpr int P = GgRaw<FMT, false>::kPitch;
-    if ((align & 15u) == 0 && bytes == P) {
+    if ((align & 15u) == 0 && bytes == P && near) {
       // 16-byte pieces, nine per row: piece id -> shared-memory byte 16 id. `piece[i]` = where this lane's i-th piece
       // lies from the first row's, the same for every round: recomputing it made the two loader warps, which get an
       // issue slot every eight cycles or so, the pace of the kernel (2400 cycles per round).
@@ -513,11 +513,14 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
       constexpr int kRows = kTileM / kGgRawWarps;
       const int row0 = kRows * (warp - 2);
       int piece[9] = {};  // IQ4_NL, see gg_load_raw
+      // (32-bit distances: matrices further apart, as separate tensors may be, take the copies by row address)
+      const int64_t apart = A.L.up_offset - A.L.gate_offset;
+      const bool near = apart > -(int64_t(1) << 30) && apart < (int64_t(1) << 30);
       if constexpr (!kIq3s) {
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
           const int id = lane + 32 * i, r = id / 9, c = id - 9 * r;
-          piece[i] = 16 * c + (r >> 1) * row_bytes + ((r & 1) ? int(A.L.up_offset - A.L.gate_offset) : 0);
+          piece[i] = 16 * c + (r >> 1) * row_bytes + ((r & 1) && near ? int(apart) : 0);
         }
       }
       uint32_t rcount = 0;
@@ -543,7 +546,7 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
           for (int hf = 0; hf < kRows / 32; ++hf) {
             const uint32_t dst = smem_u32(rawb) + s * R::kSlot + (row0 + 32 * hf) * R::kPitch;
             const uint8_t *p = pg + 16 * hf * row_bytes, *p2 = pu + 16 * hf * row_bytes;
-            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece,
+            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece, near,
                                      [&](int r) { return ((r & 1) ? p2 : p) + (r >> 1) * row_bytes; });
           }
           if (async) cp_async_arrive_noinc(&bars->raw_full[s]);

@@ -426,3 +426,31 @@ def test_grouped_gemms_at_the_edges_of_token_tiles(fg, fd, inter):
         prefill.moe_prefill_combine(ws, None, None, 0, None, None, None, out, T)
         assert np.array_equal(out.cpu().numpy().view(np.uint32), ybits), shift
     assert ws.status() == 0
+
+
+@pytest.mark.parametrize("up_first", [False, True])
+@pytest.mark.parametrize("fg,fd,inter", [(IQ4_NL, IQ4_NL, 512), (IQ3_S, IQ4_NL, 640)])
+def test_matrices_further_apart_than_31_bits(fg, fd, inter, up_first):
+    """Gate and up matrices as separate tensors more than 2 GiB apart, in either order: the bits of packed blobs."""
+    torch = _torch()
+    from fngine_b200 import moe, prefill
+    T, n_exp = 40, 10
+    layer = moe.synth_layer(fg, fd, inter, n_exp, 5151)
+    ws = prefill.PrefillWorkspace(T, inter)
+    logits = torch.from_numpy(edge_counts_logits([T], T)).cuda()
+    xd = torch.from_numpy(synth.to_bf16_bits(synth.activations(43, T)).view(np.int16)).cuda().view(torch.bfloat16)
+    y = run_prefill(torch, layer, ws, logits, xd, T).clone()
+    stride, gate = layer.layout.blob_stride, inter * O.row_bytes(fg, H)
+    far = (1 << 31) + 65536
+    buf = torch.zeros(far + n_exp * stride, dtype=torch.uint8, device="cuda")
+    first, second = buf[:n_exp * stride].view(n_exp, stride), buf[far:].view(n_exp, stride)
+    blobs = layer.slots.view(n_exp, stride)
+    gates, ups = (second, first) if up_first else (first, second)
+    gates[:, :gate], ups[:, :gate] = blobs[:, :gate], blobs[:, gate:2 * gate]
+    first[:, 2 * gate:] = blobs[:, 2 * gate:]
+    apart = moe.ExpertLayer(buf, fg, fd, inter)
+    for name in ("slots", "blob_stride", "down_offset"):  # (stands: down matrices in the first array)
+        assert getattr(apart.layout, name) == (buf.data_ptr() if name == "slots" else getattr(layer.layout, name))
+    apart.layout.gate_offset, apart.layout.up_offset = (far, 0) if up_first else (0, far)
+    got = run_prefill(torch, apart, ws, logits, xd, T)
+    assert ws.status() == 0 and torch.equal(got, y)
