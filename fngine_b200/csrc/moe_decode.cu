@@ -32,8 +32,9 @@ constexpr int kExperts = FB_EXPERTS;
 constexpr int kMaxTok = FB_DECODE_MAX_TOKENS;
 constexpr int kMaxPairs = FB_DECODE_MAX_PAIRS;
 constexpr int kTT = 2;  // tokens of one work item handled per pass over a staged tile
-// ws.sched: [0] gate/up tile counter, [1] down tile counter, [8..168) item order
-constexpr int kSchedOrderBase = 8;
+// ws.sched: [0] gate/up tile counter, [1] down tile counter, [2] producers that have staged their last tile,
+// [8..168) item order
+constexpr int kSchedLeft = 2, kSchedOrderBase = 8;
 constexpr int kEpMaxRanks = FB_EP_MAX_RANKS;
 constexpr uint32_t kPeerSpinLimit = 1u << 20;  // default polls of a peer-written flag before giving up (about a second)
 
@@ -395,7 +396,7 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
   if (tid < kExperts) s_tok[tid] = 0;
   if (tid < kExperts / 32 * (kMaxTok + 1)) (&s_hist[0][0])[tid] = 0;
   if (reset) {
-    if (tid < kMaxPairs) ws.item_done[tid] = 0;
+    if (tid < 2 * kMaxPairs) ws.item_done[tid] = 0;
     if (tid < kSchedOrderBase) ws.sched[tid] = 0;
   }
   // (One warp per token. All sixteen warps on each token's slices - maxima, threshold, candidates and ranking behind a
@@ -724,7 +725,7 @@ __global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* w, c
     x_lines = static_cast<const uint4*>(ep.peers.x_all[ep.peers.rank]) + size_t(ep.parity) * kMaxTok * (H / 2);
   }
   if (blockIdx.x == 0) {
-    if (tid < kMaxPairs) ws.item_done[tid] = 0;
+    if (tid < 2 * kMaxPairs) ws.item_done[tid] = 0;
     if (tid < kSchedOrderBase) ws.sched[tid] = 0;
     if (tid < kMaxTok * kMaxDnTiles) ws.sched[kSchedParts + tid] = 0;
   }
@@ -958,7 +959,7 @@ __global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* w, c
 // than kTT tokens is staged once per group of kTT tokens (its weights come back from L2). Every
 // output element is still written by exactly one thread after a fixed-order reduction: results do
 // not depend on which CTA or warp ran which piece.
-constexpr int kSchedGateUp = 0, kSchedDown = 1, kSchedOrder = kSchedOrderBase;
+constexpr int kSchedGateUp = 0, kSchedDown = 1;
 
 // What the producer tells the consumers about the entry staged in a ring slot (shared memory).
 struct alignas(16) StageMeta {
@@ -1017,23 +1018,23 @@ __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uin
 }
 
 // Counts one finished contribution to an item's h; the last one re-quantizes that item's h for the
-// down projection and then sets kItemReady in the item's counter (a fused gate/up + down launch polls
-// it before staging the item's rows). `expected` = contributions per item.
-constexpr int kItemReady = 0x40000000;
+// down projection and then sets the item's flag, ws.item_done[kMaxPairs + item], to `ready` (1 in a fused gate/up + down
+// launch, which polls it before staging the item's rows). `expected` = contributions per item; the counter wraps to zero
+// behind the last one.
 template <int I>
 __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_workspace& ws, int item, int pair_begin,
-                                                       int n_tok, int expected, int down_act, int lane) {
+                                                       int n_tok, int expected, int down_act, int ready, int lane) {
   // (release and acquire ride on the two atomics: at one token this chain is a tenth of the layer)
   __syncwarp();
   int ticket = 0;
   if (lane == 0)
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(&ws.item_done[item]) : "memory");
+    asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(ticket) : "l"(&ws.item_done[item]), "r"(expected - 1) : "memory");
   ticket = __shfl_sync(0xffffffffu, ticket, 0);
   if (ticket == expected - 1) {
     for (int p = pair_begin; p < pair_begin + n_tok; ++p)
       quantize_h_row<I>(ws.h + size_t(p) * I, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
     __syncwarp();
-    if (lane == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(&ws.item_done[item]), "r"(kItemReady) : "memory");
+    if (lane == 0) asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(&ws.item_done[kMaxPairs + item]), "r"(ready) : "memory");
   }
 }
 
@@ -1357,7 +1358,7 @@ size_t fb_moe_decode_workspace_bytes(int32_t inter) {
   (void)inter;
   auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
   return up(sizeof(fb_moe_decode_work)) + up(size_t(2 * kMaxTok) * FB_XQ_STRIDE) + up(size_t(kMaxPairs) * 640 * 4) +
-         up(size_t(kMaxPairs) * FB_HQ_STRIDE) + up(size_t(kMaxPairs) * H * 4) + up(kMaxPairs * 4) +
+         up(size_t(kMaxPairs) * FB_HQ_STRIDE) + up(size_t(kMaxPairs) * H * 4) + up(2 * kMaxPairs * 4) +
          up(kSchedInts * 4) + 256;
 }
 
@@ -1377,7 +1378,7 @@ int32_t fb_moe_decode_workspace_make(void* base, const fb_moe_expert_layout* lay
   out->partial = reinterpret_cast<float*>(p);
   p += up(size_t(kMaxPairs) * H * 4);
   out->item_done = reinterpret_cast<int32_t*>(p);
-  p += up(kMaxPairs * 4);
+  p += up(2 * kMaxPairs * 4);
   out->sched = reinterpret_cast<int32_t*>(p);
   p += up(kSchedInts * 4);
   out->status = reinterpret_cast<uint32_t*>(p);

@@ -756,12 +756,12 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
           mbar_expect_tx_only(full, uint32_t(C::kDnTile + ntp * C::kDnAct));
           bulk_g2s(st, w0, C::kDnTile, full);
           if (!ready) {  // the item's h must have been re-quantized (bounded poll of its flag)
-            const int* flag = ws.item_done + item;
+            const int* flag = ws.item_done + kMaxPairs + item;
             uint32_t tries = 0;
             while (true) {
               int v;
               asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-              if (v & kItemReady) break;
+              if (v) break;
               if (++tries > (1u << 22) || *ring.end_seq == 0) {
                 give_up();
                 break;
@@ -784,6 +784,19 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         }
         if (++s == S) s = 0;
       }
+    }
+    if (phases & kPhaseSelect) return;
+    // Behind a selection of its own, the last producer of the launch clears the tile counters and the items' flags (all of
+    // which have been seen by then), so that the next launch on the same work list (another layer's weights, say) starts
+    // like the first; the items' counters wrap to zero. (The fused call's route kernel clears them all.)
+    int before;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(ws.sched + kSchedLeft) : "memory");
+    if (before != int(gridDim.x) - 1) return;
+#pragma unroll 1
+    for (int k = 0; k < kSchedOrderBase; ++k) ws.sched[k] = 0;
+    if (phases & kPhaseDown) {
+#pragma unroll 1
+      for (int k = 0; k < kMaxPairs; ++k) ws.item_done[kMaxPairs + k] = 0;
     }
     return;
   }
@@ -865,7 +878,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         s_misc[3 + s] = 0;
         mbar_arrive(&ring.empty[s]);
       }
-      item_contribution_done<INTER>(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act, lane);
+      item_contribution_done<INTER>(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act,
+                                    phases & kPhaseDown ? 1 : 0, lane);
     } else {
       const float w0 = ring.meta[s].wgt[0], w1 = ring.meta[s].wgt[1];
 #pragma unroll

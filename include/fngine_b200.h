@@ -110,7 +110,9 @@ typedef struct fb_moe_decode_work {
  * codes first, then the block scales as fp32 (Q8_0 scales are the fp16-rounded values widened;
  * Q8_0 codes are stored per block in the order 2*(e%16) + e/16 that the IQ4_NL nibble decode
  * produces). `hq` is h re-quantized for the down projection, `item_done` counts finished gate/up
- * tiles per work item, `sched` holds the dynamic tile counters ([0] gate/up, [1] down) and from
+ * tiles per work item (from [160] on: its h is re-quantized), `sched` holds the dynamic tile counters ([0] gate/up, [1]
+ * down). A launch behind a selection of its own leaves all of these cleared: gate/up and down may run repeatedly on one
+ * work list. In `sched` follow from
  * [8] on the work items ordered by token count (heaviest first), from [192] on the counters of finished
  * down rows per token and column tile, `status` is one device word set
  * when a bounded wait runs out. */
@@ -120,7 +122,7 @@ typedef struct fb_moe_decode_workspace {
   float* h;           /* [160 pairs][inter] fp32 silu(g)*u */
   uint8_t* hq;        /* [160 pairs][FB_HQ_STRIDE] */
   float* partial;     /* [160 pairs][2560], routing weight applied */
-  int32_t* item_done; /* [160] */
+  int32_t* item_done; /* [2][160] */
   int32_t* sched;     /* [192 + 16 * 20] */
   uint32_t* status;   /* FB_STATUS_* */
   int32_t gate_up_format;

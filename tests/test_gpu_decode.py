@@ -835,3 +835,47 @@ def test_wide_router_at_the_edges_of_its_tile_heights(rows, tokens, bf16):
     """The last token counts of the 8- and 16-row tiles, the first of the next height, and a ragged last tile of each:
     the bits of slices of at most 16 tokens."""
     test_wide_router_gives_the_bits_of_the_narrow_one(rows, tokens, bf16)
+
+
+@pytest.mark.parametrize("fg,fd,inter", [(IQ2_S, Q2_0, 640), (IQ4_XS, IQ4_NL, 512), (IQ3_S, IQ3_S, 512), (IQ4_NL, IQ3_S, 512)])
+@pytest.mark.parametrize("one_launch", [False, True])
+def test_experts_of_several_layers_behind_one_selection(fg, fd, inter, one_launch):
+    """The work list is a function of the logits alone: gate/up and down of another layer's weights, called again behind
+    the same selection, give the bits they give behind a selection of their own."""
+    torch = _torch()
+    from fngine_b200 import moe
+    tokens = 9
+    layers = [moe.synth_layer(fg, fd, inter, 512, 640 + i) for i in range(3)]
+    wr = torch.from_numpy(synth.router_weights(41, rows=513).view(np.int16)).cuda().view(torch.bfloat16)
+    x = torch.from_numpy(synth.activations(47, tokens)).cuda()
+    ws = moe.DecodeWorkspace(layers[0])
+
+    def select():
+        moe.router_logits(wr, x, ws.logits)
+        moe.moe_select_publish(ws.logits, x, None, 0, None, None, tokens, ws)
+
+    def experts(layer):
+        y = torch.empty(tokens, H, dtype=torch.float32, device="cuda")
+        if one_launch:
+            moe.moe_hot_experts(layer, tokens, ws)
+        else:
+            moe.moe_hot_gate_up(layer, tokens, ws)
+            moe.moe_hot_down(layer, tokens, ws)
+        moe.moe_combine(ws, None, None, 0, None, None, None, y, tokens)
+        return y
+
+    want = []
+    for layer in layers:
+        select()
+        want.append(experts(layer))
+    select()
+    got = [experts(layer) for layer in layers]
+    moe.moe_hot_gate_up(layers[1], tokens, ws)  # (no down projection behind this one)
+    got += [experts(layer) for layer in layers]
+    moe.moe_layer_decode(wr[:512].contiguous(), layers[0], x, ws, torch.empty(tokens, H, dtype=torch.float32, device="cuda"))
+    select()
+    got += [experts(layer) for layer in layers]
+    torch.cuda.synchronize()
+    assert ws.status() == 0 and not torch.equal(want[0], want[1])
+    for g, w in zip(got, want + want + want):
+        assert torch.equal(g, w)
