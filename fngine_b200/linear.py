@@ -16,7 +16,10 @@ class Fp8RowWeight:
         assert scales.is_cuda and scales.dtype in (torch.float32, torch.bfloat16) and scales.numel() == codes.shape[0]
         self.codes, self.scales = codes, scales.contiguous()
         self.n, self.k = codes.shape
-        self.scale_dtype = L.DT_BF16 if scales.dtype == torch.bfloat16 else L.DT_F32
+
+    @property
+    def scale_dtype(self):
+        return L.DT_BF16 if self.scales.dtype == torch.bfloat16 else L.DT_F32
 
 
 def linear_fp8_workspace(weight, max_tokens, device="cuda"):

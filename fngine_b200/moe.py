@@ -195,12 +195,18 @@ class SharedExpert:
         self.work_dn = linear.linear_fp8_decode_workspace(down)
         self.h = torch.empty(max_tokens, down.k, dtype=torch.bfloat16, device=gate_up.codes.device)
         self.y = torch.empty(max_tokens, down.n, dtype=torch.float32, device=gate_up.codes.device)
-        # the one-call branch takes intermediate sizes in steps of 128 up to 1024; others run as separate projections
-        self.args = None
-        if gate_up.k == L.HIDDEN and down.k % 128 == 0 and down.k <= 1024:
-            self.args = L.SharedExpert(gate_up.codes.data_ptr(), gate_up.scales.data_ptr(), down.codes.data_ptr(),
-                                       down.scales.data_ptr(), self.h.data_ptr(), self.y.data_ptr(), gate_up.scale_dtype,
-                                       down.scale_dtype, down.k, 0)
+
+    def args(self):
+        """fb_shared_expert of the tensors as they are now, or None: the one-call branch takes intermediate sizes in steps
+        of 128 up to 1024, others run as separate projections."""
+        gate_up, down = self.gate_up, self.down
+        if gate_up.k != L.HIDDEN or down.k % 128 or down.k > 1024:
+            return None
+        assert gate_up.n == 2 * down.k and down.n == L.HIDDEN
+        assert self.h.dtype == torch.bfloat16 and self.h.shape[1] == down.k
+        assert self.y.dtype == torch.float32 and self.y.shape[1] == down.n and self.y.shape[0] >= self.h.shape[0]
+        return L.SharedExpert(_ptr(gate_up.codes), _ptr(gate_up.scales), _ptr(down.codes), _ptr(down.scales), _ptr(self.h),
+                              _ptr(self.y), gate_up.scale_dtype, down.scale_dtype, down.k, 0)
 
 
 def forward_moe_decode(w_router, shared, layer, x, ws, inj, X, y_out=None, aux_stream=None):
@@ -209,10 +215,12 @@ def forward_moe_decode(w_router, shared, layer, x, ws, inj, X, y_out=None, aux_s
     experts on `aux_stream` (its down epilogue reads the shared-gate logit), gate/up, down, and the
     combine that adds y_shared and writes the residual streams X += inj * y. x: bf16 [T][2560]."""
     T = x.shape[0]
-    assert x.dtype == torch.bfloat16 and w_router.shape[0] == L.ROUTER_ROWS and T <= shared.h.shape[0]
-    if shared.args is not None:
+    assert x.dtype == torch.bfloat16 and x.shape[1] == shared.gate_up.k
+    assert w_router.shape[0] == L.ROUTER_ROWS and T <= shared.h.shape[0]
+    args = shared.args()
+    if args is not None:
         # one call: the shared expert rides in the launches of the routed ones (nothing is left for aux_stream)
-        L.check(L.load().fb_moe_forward_decode(_ptr(w_router), C.byref(layer.layout), C.byref(shared.args), _ptr(x), T,
+        L.check(L.load().fb_moe_forward_decode(_ptr(w_router), C.byref(layer.layout), C.byref(args), _ptr(x), T,
                                                C.byref(ws.ws), _ptr(ws.logits), _ptr(inj), _ptr(X), _ptr(y_out), _stream()),
                 "moe_forward_decode")
         return

@@ -879,3 +879,36 @@ def test_experts_of_several_layers_behind_one_selection(fg, fd, inter, one_launc
     assert ws.status() == 0 and not torch.equal(want[0], want[1])
     for g, w in zip(got, want + want + want):
         assert torch.equal(g, w)
+
+
+def test_branch_uses_the_shared_expert_as_it_is_now():
+    """Weights, row scales and buffers of a shared expert may be replaced after it was made: a call takes those that are
+    there, as separate projections do."""
+    torch = _torch()
+    from fngine_b200 import linear, moe
+    tokens, inter_s = 3, 640
+    layer = moe.synth_layer(IQ3_S, IQ4_NL, 640, 512, 4344)
+    ws = moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(910, rows=513).view(np.int16)).cuda().view(torch.bfloat16)
+
+    def weight(seed, n, k):
+        codes, scales = synth.fp8_row_weight(seed, n, k)
+        return linear.Fp8RowWeight(torch.from_numpy(codes).cuda(), torch.from_numpy(scales * np.float32(4.0)).cuda())
+
+    xb = synth.to_bf16_bits(synth.activations(79, tokens))
+    xd = torch.from_numpy(xb.view(np.int16)).cuda().view(torch.bfloat16)
+    first = (weight(33, 2 * inter_s, H), weight(34, H, inter_s))
+    gu, dn = weight(35, 2 * inter_s, H), weight(36, H, inter_s)
+    dn.scales = dn.scales.to(torch.bfloat16)
+    used, fresh = moe.SharedExpert(*first), moe.SharedExpert(gu, dn)
+    old = used.h, used.y
+    used.gate_up, used.down = gu, dn
+    used.h, used.y = torch.full_like(old[0], float("nan")), torch.full_like(old[1], float("nan"))
+    ys = [torch.full((tokens, H), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2)]
+    for shared, y in zip((fresh, used), ys):
+        moe.forward_moe_decode(wr, shared, layer, xd, ws, None, None, y)
+    torch.cuda.synchronize()
+    assert torch.equal(ys[0], ys[1])
+    assert torch.equal(used.h[:tokens], fresh.h[:tokens]) and torch.equal(used.y[:tokens], fresh.y[:tokens])
+    with pytest.raises(AssertionError):  # rows of another width
+        moe.forward_moe_decode(wr, used, layer, xd[:, :2048].contiguous(), ws, None, None, ys[0])
