@@ -1031,6 +1031,7 @@ __device__ __forceinline__ void item_contribution_done(const fb_moe_decode_works
     asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(ticket) : "l"(&ws.item_done[item]), "r"(expected - 1) : "memory");
   ticket = __shfl_sync(0xffffffffu, ticket, 0);
   if (ticket == expected - 1) {
+    __syncwarp();  // (the shuffle orders no memory: the other lanes read h behind lane 0's acquire by this)
     for (int p = pair_begin; p < pair_begin + n_tok; ++p)
       quantize_h_row<I>(ws.h + size_t(p) * I, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
     __syncwarp();

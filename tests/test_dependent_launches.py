@@ -87,3 +87,12 @@ def test_a_cluster_with_a_missing_partial_tile_stores_nothing(name):
     _, end = _block(body, guard.end() - 1, "{", "}")
     stores = [m.start() for m in re.finditer(r"static_cast<(?:__nv_bfloat16|float)\*>\(a\.out\)", body) if m.start() > barrier]
     assert stores and all(guard.start() < at < end for at in stores)
+
+
+def test_lanes_read_behind_the_acquire_of_lane_0():
+    """A shuffle orders no memory: between lane 0's acquiring atomic and the other lanes' loads stands a __syncwarp."""
+    with open(os.path.join(CSRC, "moe_decode.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    body, _ = _block(text, text.index("{", text.index("void item_contribution_done")), "{", "}")
+    behind = body[body.index("atom.acq_rel"):body.index("quantize_h_row")]
+    assert "__syncwarp();" in behind
