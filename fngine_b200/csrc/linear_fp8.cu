@@ -1938,10 +1938,10 @@ int32_t fb_linear_fp8_decode(const void* x_bf16, int32_t tokens, const uint8_t* 
   a.status = status;
   const int m_tiles = kind == FB_EPI_SWIGLU ? ((n >> 1) + 63) / 64 : (n + 127) / 128;
   // At most one row tile per multiprocessor: a cluster per tile, the largest (up to the portable size and one K block per
-  // CTA) of which as many as there are tiles are resident at once. (Above kSmallMaxKb blocks per CTA the operand rows do
-  // not fit. A tile that gets one CTA alone splits whole activation rows in every CTA: 13.3 - 16.2 us for 16384 x 2560 at
-  // 4 - 16 tokens against 12.1 - 13.4 of the streaming kernel, which keeps it. Fewer than four tiles, which no projection of the engine has, stay with the streaming kernel: its operand
-  // rows can be read back from the workspace.)
+  // CTA) of which as many as there are tiles are resident at once. (us per call, four tokens, against the streaming kernel:
+  // 128 x 2560 4.9 and 7.0, 256 x 1024 4.6 and 6.7, 384 x 10240 7.7 and 9.8, 512 x 6144 6.2.) Above kSmallMaxKb blocks per
+  // CTA the operand rows do not fit. A tile that gets one CTA alone splits whole activation rows in every CTA: 13.3 - 16.2
+  // us for 16384 x 2560 at 4 - 16 tokens against 12.1 - 13.4 of the streaming kernel, which keeps it.
   // An output that lies in the activations' memory also stays with the streaming kernel, whose split has read all of them
   // when the first output is written.
   const size_t out_values = size_t(tokens) * size_t(n);
@@ -1950,7 +1950,7 @@ int32_t fb_linear_fp8_decode(const void* x_bf16, int32_t tokens, const uint8_t* 
   const uintptr_t x0 = reinterpret_cast<uintptr_t>(x_bf16), out0 = reinterpret_cast<uintptr_t>(epilogue->out);
   const bool in_place = out0 < x0 + size_t(tokens) * size_t(k) * 2 && x0 < out0 + out_bytes;
   const int kb = k / BK;
-  if (m_tiles >= 4 && m_tiles <= sm_count() && !in_place) {
+  if (m_tiles <= sm_count() && !in_place) {
     const int* resident = small_clusters();
     if (!resident) {
       set_error("linear_fp8_decode: shared-memory opt-in failed");

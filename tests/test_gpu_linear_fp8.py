@@ -311,7 +311,7 @@ def epilogue_case(torch, kind, T, n, acc):
     (257, 2560, 128, "shared_scale"),  # a second token tile of one token, K too short to share
     (700, 640, 1152, "store_bf16"),    # three token tiles, nine K blocks over a cluster
     (40, 19008, 128, "store_bf16"),    # more 128-row tiles than multiprocessors
-    (1, 512, 640, "store_f32"),        # decode width: the fewest row tiles that share K in a cluster, five K blocks
+    (1, 512, 640, "store_f32"),        # decode width: four row tiles, five K blocks shared in a cluster
     (16, 448, 1152, "gr_write"),       # decode width: a ragged fourth row tile, nine K blocks
 ])
 def test_linear_fp8_small_and_middle_widths(T, n, k, kind, path):

@@ -124,10 +124,11 @@ def test_linear_fp8_decode_matches_the_exact_product(T, n, k, kind, bf16_scales)
 
 def test_activation_pieces_are_exact():
     """scale[t] * (p0 + p1 + p2) reproduces the bf16 activations bit for bit over a 2^23 dynamic range
-    inside a row; an all-zero token, a tiny token, and unused token slots left as zero rows."""
+    inside a row; an all-zero token, a tiny token, and unused token slots left as zero rows. The pieces of the streaming
+    kernel, which more row tiles than multiprocessors take: they can be read back from the workspace."""
     torch = _torch()
     from fngine_b200 import linear
-    T, n, k = 6, 256, 1024
+    T, n, k = 6, 19080, 1024
     weight = make_weight(torch, 11, n, k, False)
     x = synth.activations(99, T, hidden=k) * np.exp2(np.linspace(-12, 4, k, dtype=np.float32))[None, :]
     x[2] = 0.0
@@ -237,6 +238,38 @@ def test_projection_into_the_memory_of_its_activations(T, n, k, kind):
         linear.linear_fp8_decode(xin, weight, make(out), work)
         torch.cuda.synchronize()
         compare(torch, out, ref, dt == torch.bfloat16)
+
+
+@pytest.mark.parametrize("T,n,k", [(6, 1024, 1024),     # eight row tiles, clusters of eight CTAs with one K block each
+                                   (16, 2560, 2560),    # twenty row tiles, twenty K blocks: uneven shares
+                                   (1, 8192, 1024),     # sixty-four row tiles: two CTAs each
+                                   (9, 8, 10240),       # one ragged row tile, ten K blocks per CTA
+                                   (5, 256, 640)])      # two row tiles, clusters of five
+def test_activations_reach_the_sums_exactly(T, n, k):
+    """The cluster kernel's own activation split, through its outputs: weight rows with a single 1 make each output one
+    activation, bit for bit over a 2^23 dynamic range inside a row (below that to 2^-30 of the row's maximum, as above);
+    an all-zero token, a tiny token."""
+    torch = _torch()
+    from fngine_b200 import linear
+    at = torch.arange(n) % k if n >= k else torch.randperm(k, generator=torch.Generator().manual_seed(n))[:n]
+    codes = torch.zeros(n, k, dtype=torch.uint8)
+    codes[torch.arange(n), at] = 0x38  # E4M3 1.0
+    weight = linear.Fp8RowWeight(codes.cuda(), torch.ones(n, dtype=torch.float32, device="cuda"))
+    x = synth.activations(99, T, hidden=k) * np.exp2(np.linspace(-12, 4, k, dtype=np.float32))[None, :]
+    if T > 4:
+        x[2] = 0.0
+        x[4] *= np.float32(1e-6)
+    xb = bf16_tensor(torch, x)
+    out = torch.full((T, n), float("nan"), dtype=torch.float32, device="cuda")
+    linear.linear_fp8_decode(xb, weight, linear.store_f32(out), linear.linear_fp8_decode_workspace(weight))
+    torch.cuda.synchronize()
+    rows = xb.float().cpu().numpy().astype(np.float64)
+    want, got = rows[:, at.numpy()], out.cpu().numpy().astype(np.float64)
+    rowmax = np.abs(rows).max(axis=1, keepdims=True)
+    err = np.abs(got - want)
+    assert np.all((err == 0) | (np.abs(want) < rowmax * 2.0 ** -23))
+    assert np.all(err <= rowmax * 2.0 ** -30)
+    assert (err == 0).mean() > 0.99
 
 
 def test_linear_fp8_decode_argument_errors():
