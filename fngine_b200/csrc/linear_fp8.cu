@@ -1145,7 +1145,7 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // round trips on partial sums and tickets: 15.5 us for 2560 x 6144 at four tokens, 2.5 us of which is the weights'
 // traffic. Here a CLUSTER owns a row tile, its CTAs equal shares of K; each CTA splits its own part of the activations
 // straight into operand rows in shared memory (the token scale is then the CTA's own, so no pass over whole rows comes
-// first), and the partial tiles meet through distributed shared memory, added in CTA order (fixed: repeated calls are
+// first), and the partial tiles meet through distributed shared memory, added in a fixed order (repeated calls are
 // bitwise identical). One launch; of the workspace it uses the status word only. A CTA whose wait runs out tells the
 // others of its cluster ahead of the barrier that ends the sums, and none of them stores anything.
 constexpr int kSmallThreads = 512, kSmallMaxKb = 20, kSmallMaxCluster = 8;
@@ -1345,15 +1345,14 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
     float p[kSmallMaxCluster];
 #pragma unroll
     for (int c = 0; c < kSmallMaxCluster; ++c) p[c] = c < cluster ? ld_cluster_f32(part + tt * 128 + r, uint32_t(c)) : 0.0f;
-    float s = p[0];
-#pragma unroll
-    for (int c = 1; c < kSmallMaxCluster; ++c) s += p[c];  // (adding + 0.0 behind the last changes nothing)
-    return s;
+    // In pairs: closer than one by one, and a shorter chain (2560 x 6144 at four tokens 10.0 -> 9.7 us per call). With
+    // compensated or fp64 additions 10.2 and 10.3 us.
+    return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
   };
   const int first = rank * kSmallThreads + tid;
   int tt = first / rows, r = first - tt * rows;  // (rows is 64 or 128)
   bool live = first < n_out && (swiglu ? m * 64 + r < half_n : m * 128 + r < a.n);
-  float ws0 = 0.0f, ws1 = 0.0f, gate = 1.0f, x4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float ws0 = 0.0f, ws1 = 0.0f, x4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   float4 g4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   auto fetch = [&]() {
     if (!live) return;
@@ -1369,7 +1368,9 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
 #pragma unroll
       for (int st = 0; st < 4; ++st) x4[st] = static_cast<const float*>(a.out)[(size_t(tt) * 4 + st) * a.n + n];
     } else if (a.kind == FB_EPI_SHARED_SCALE) {
-      gate = 1.0f / (1.0f + expf(-a.gate_logit[size_t(tt) * a.gate_stride]));
+      // (one rounding for both factors, where a reciprocal and two products had three: with five partial tiles 7.2e-8 from
+      // an fp64 product, now 6.6e-8)
+      ws0 /= 1.0f + expf(-a.gate_logit[size_t(tt) * a.gate_stride]);
     }
   };
   fetch();
@@ -1385,7 +1386,7 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
         static_cast<__nv_bfloat16*>(a.out)[size_t(tt) * half_n + m * 64 + r] = __float2bfloat16_rn(g / (1.0f + expf(-g)) * u);
       } else {
         const int n = m * 128 + r;
-        const float val = sum * ws0 * gate;
+        const float val = sum * ws0;
         if (a.kind == FB_EPI_GR_WRITE) {
           float* xs = static_cast<float*>(a.out) + size_t(tt) * 4 * a.n + n;
           xs[0] = fmaf(g4.x, val, x4[0]);

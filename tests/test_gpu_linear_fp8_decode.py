@@ -272,6 +272,28 @@ def test_activations_reach_the_sums_exactly(T, n, k):
     assert (err == 0).mean() > 0.99
 
 
+@pytest.mark.parametrize("T", [4, 15])
+def test_distance_of_a_shared_sum_from_the_exact_product(T):
+    """Five partial tiles, one per CTA, and the shared-gate factor (2560 x 640): in relative L2 not further from the fp64
+    product than the 7.0e-8 of a kernel that adds two or three partial tiles of two K blocks each. (Added one by one in
+    fp32, with a reciprocal and two products behind, 7.1e-8 to 7.3e-8.)"""
+    torch = _torch()
+    from fngine_b200 import linear
+    num = den = 0.0
+    for seed in range(8):
+        weight = make_weight(torch, 8800 + seed, 2560, 640, True)
+        x = bf16_tensor(torch, synth.activations(8900 + seed + T, T, hidden=640))
+        gate = torch.randn(T, 513, generator=torch.Generator().manual_seed(seed)).cuda()
+        out = torch.empty(T, 2560, dtype=torch.float32, device="cuda")
+        work = linear.linear_fp8_decode_workspace(weight)
+        linear.linear_fp8_decode(x, weight, linear.shared_scale(out, gate[:, 512:], 513), work)
+        torch.cuda.synchronize()
+        ref = exact_acc(torch, x, weight) * torch.sigmoid(gate[:, 512].double())[:, None]
+        num, den = num + float((out.double() - ref).norm()) ** 2, den + float(ref.norm()) ** 2
+    print("distance %.3e" % (num / den) ** 0.5)
+    assert (num / den) ** 0.5 <= 7.0e-8
+
+
 def test_linear_fp8_decode_argument_errors():
     torch = _torch()
     import ctypes
