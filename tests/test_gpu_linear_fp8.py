@@ -356,3 +356,24 @@ def test_the_status_word_of_a_call_is_its_own(T, n, k):
     at = up(48 * k) + 256 if T <= 16 else up(2 * T * k) + up(4 * T)
     assert int(work[at:at + 4].view(torch.int32)) == 0
     compare(torch, out, exact_acc(torch, x.double(), weight), False)
+
+
+@pytest.mark.parametrize("path", ["auto", "a8"])
+@pytest.mark.parametrize("T,n,k,kind", [
+    # two-SM tiles of 256 tokens x 256 rows, more of them than half of the GPU's pairs
+    (1030, 5056, 384, "store_bf16"),    # ragged tokens and rows, three K blocks
+    (1030, 5056, 384, "store_f32"),
+    (769, 5056, 1152, "gr_write"),      # one token in the last tile
+    (1025, 4736, 640, "shared_scale"),
+    (1280, 4864, 256, "swiglu"),        # exact token tiles, a ragged last tile of 128 gate and 128 up rows
+    (257, 19008, 128, "store_bf16"),    # the fewest tokens with a second tile, one K block
+    # one-SM tiles: fewer tokens than such a tile takes, more than two waves of 128-row tiles
+    (17, 38016, 128, "store_f32"),
+    (130, 38080, 256, "store_bf16"),    # a second token tile of two tokens, a ragged last row tile
+    (255, 38272, 128, "swiglu"),
+    (129, 38080, 128, "shared_scale"),
+    (40, 38080, 384, "gr_write"),
+])
+def test_linear_fp8_wide_tiles(T, n, k, kind, path):
+    """The two GEMM kernels that middle widths do not take, at the edges of their tiles, both routes, every epilogue."""
+    test_linear_fp8_small_and_middle_widths(T, n, k, kind, path)
