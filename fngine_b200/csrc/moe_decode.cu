@@ -67,9 +67,6 @@ __device__ __forceinline__ float2 ll_read(const uint4* line, uint32_t step, uint
 constexpr int kSchedParts = 192, kMaxDnTiles = H / 128;
 constexpr int kSchedInts = kSchedParts + kMaxTok * kMaxDnTiles;
 
-__host__ __device__ constexpr int act_row_bytes_planar(int act, int k) {
-  return act == FB_ACT_Q8_K ? k + 64 : k + k / 8;
-}
 __host__ __device__ constexpr int act_of(int fmt) {
   return fmt == FB_FMT_IQ4_NL || fmt == FB_FMT_Q2_0 ? FB_ACT_Q8_0 : FB_ACT_Q8_K;
 }
