@@ -11,7 +11,7 @@
 // and may be moved ahead of the wait.
 //
 // gate_up and down are one persistent kernel, one CTA per SM (moe_decode_experts.cuh): a producer thread streams
-// tiles of the expert blob into a three-stage shared-memory ring with 1-D bulk async copies (TMA, no multicast)
+// tiles of the expert blob into a shared-memory ring of three or four slots with 1-D bulk async copies (TMA, no multicast)
 // signalled through mbarriers; consumer warps decode the blocks from shared memory and accumulate exact int8 dot
 // products (dp4a). Numerics are those of the
 // reference's CPU expert tier (src/cpu/iq_cpu.h:12-40 of the reference project): Q8_K activations
@@ -1611,8 +1611,8 @@ int32_t fb_moe_layer_decode_ep_p2p(const void* router_w_bf16, const fb_moe_exper
       return invalid("layer_decode_ep_p2p: a peer buffer address is missing");
   const int R = peers->n_ranks, tpr = tokens / R, parity = int(step & 1u);
   cudaStream_t s = as_stream(stream);
-  // Four launches, chained like the single-GPU layer: route (publishes this rank's rows, waits for
-  // everyone's), gate/up, down, combine (sends partial rows, waits, sums).
+  // Three launches, chained like the single-GPU layer: route (publishes this rank's rows, waits for everyone's), experts
+  // (selection, gate/up, down; IQ3_S down behind another gate/up format: two), combine (sends partial rows, waits, sums).
   EpRouteArgs era{};
   era.peers = *peers;
   era.x_local = x_local;
@@ -1789,7 +1789,7 @@ int32_t fb_moe_layer_decode_static(const void* router_w_bf16, const fb_moe_exper
   if (st) return st;
   sc.status = ws.status;
   float* logits = reinterpret_cast<float*>(sc.base + kStaticWorkspaceBytes);
-  // the sticky status word and the scheduler words (tile counters, route tickets) are the only state a call inherits
+  // the sticky status word and the scheduler words (tile counters) are the only state a call inherits
   e = cudaMemsetAsync(ws.status, 0, sizeof(uint32_t), as_stream(stream));
   if (e == cudaSuccess) e = cudaMemsetAsync(ws.sched, 0, kSchedInts * sizeof(int32_t), as_stream(stream));
   if (e != cudaSuccess) {

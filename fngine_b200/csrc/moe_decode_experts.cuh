@@ -5,8 +5,8 @@
 // IQ2_S + IQ4_NL layer of five tokens took 129 us in six launches.)
 //
 // One persistent kernel streams the gate, up and down matrices of every routed expert of a layer:
-// first all gate/up tiles (heaviest experts first), then all down tiles, through one three-stage ring
-// of 40 KB slots, so the codebook set-up, the work-list copy and the pipeline fill are paid once per
+// first all gate/up tiles (heaviest experts first), then all down tiles, through one ring of three
+// 40 KB slots (four where no table takes the space), so the codebook set-up, the work-list copy and the pipeline fill are paid once per
 // layer and HBM keeps streaming across the gate/up -> down boundary. A down tile needs its expert's h
 // re-quantized, which the warp that finishes the expert's last gate/up tile does and then flags; the
 // producer asks for a down tile's weights first and polls that flag (a bounded number of times) only

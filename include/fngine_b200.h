@@ -446,7 +446,8 @@ int32_t fb_fp8_split_tokens(const void* x_bf16, int32_t tokens, int32_t k, uint8
 /* linear_fp8 at decode width, the reference's "A16" path for T <= 16 (src/kernels/linear/linear.h:27-31,
  * :137-139; fp8/fp8_gemv.cuh, fp8/fp8_a16_ksplit_mma.cuh): bf16 activations are kept exactly (three
  * E5M2 pieces per value), E4M3 weights are used exactly, fp32 accumulation, one multiplication by the
- * row scale, then the epilogue. tokens 1..16, k % 128 == 0, n % 8 == 0 (n % 16 for SwiGlu). */
+ * row scale, then the epilogue. tokens 1..16, k % 128 == 0, n % 8 == 0 (n % 16 for SwiGlu). `out` may lie in the memory
+ * of x: all activations are read before the first output is written. */
 size_t fb_linear_fp8_decode_workspace_bytes(int32_t n, int32_t k);
 int32_t fb_linear_fp8_decode(const void* x_bf16, int32_t tokens, const uint8_t* w_codes, const void* w_scales,
                              int32_t w_scales_dtype, int32_t n, int32_t k, const fb_linear_epilogue* epilogue,
