@@ -1180,7 +1180,8 @@ def run_ours_multi(args, rank, world, local_rank):
                 "e2e": {"value": step_bytes * args.steps / (e2e_ms * 1e-3) / 1e9, "unit": "GB/s",
                         "h2d_bytes_per_step": (hi - lo) * HIDDEN * 4 * Lr * world,
                         "d2h_bytes_per_step": (hi - lo) * HIDDEN * 4 * Lr * world, "ms_per_step": e2e_ms / args.steps},
-                "gpu_launches": args.steps * Lr * 4 * world, "parity_vs_cpu_max_rel_l2": parity,
+                "gpu_launches": args.steps * Lr * 3 * world,  # route, experts, combine + exchange
+                "parity_vs_cpu_max_rel_l2": parity,
                 "device_status": status, "clocks": clocks, "prefill_stack": pre,
                 "cpu_baseline": None}
         print(json.dumps(line))
