@@ -22,6 +22,7 @@
 //     CTAs, each CTA staging its 128 token rows (one or two pieces) and its 128 weight rows per K
 //     step (32 / 48 KB, six / four stages);
 //   * single CTA: 128 x 256 tiles, 48 / 64 KB per K step, four / three stages.
+// Where their tiles do not fill the GPU a third kernel shares K among the CTAs of a cluster, see "middle widths" below.
 // What the measurements said (B200, 4096 x 9216 x 2560, one piece): operand traffic is not the limit
 // (a run that skips every load after the first ring fill takes the same time); the per-K-step work of
 // the MMA-issuing thread is. A tcgen05 fence after each full-barrier wait and a shared-memory flag load
@@ -31,7 +32,8 @@
 //
 // A second operation lives here: the same weights at decode width (T <= 16) with the bf16 activations
 // kept exactly and the same epilogues, a stream over the weight codes that reaches 0.9 of the HBM copy
-// rate; see "decode-width projection" below. fb_linear_fp8 routes T <= 16 there.
+// rate; see "decode-width projection" below, and "few row tiles" for the cluster kernel that takes all matrices of at most
+// one row tile per multiprocessor. fb_linear_fp8 routes T <= 16 there.
 #include "common.cuh"
 
 #include <cuda.h>
