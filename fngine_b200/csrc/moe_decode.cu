@@ -660,29 +660,30 @@ struct EpRouteArgs {
 };
 
 // Router projection and activation quantization in one launch (the head of the fused layer call; the
-// selection runs inside the streaming kernel that follows, see SelectArgs). 128 blocks in sixteen
-// clusters of eight: cluster g owns router rows 32g..32g+31, its CTA q the K slice [320q, 320q+320). The
-// x slice of all tokens sits in the CTA's shared memory (sixteen CTAs read each slice: no line of x is
-// wanted by all SMs at once), one warp per row pair (every x value read from shared memory feeds two
-// rows), all tokens in flight at once. The eight slice sums of a logit meet through distributed shared
-// memory: after a cluster barrier (the activation quantization sits between its two halves) CTA q adds the slices of rows 4q..4q+3 in order 0..7 (fixed: repeated
-// calls are bitwise identical) and stores the logits. No block waits on device memory for another. Every
-// warp of the grid also quantizes a share of the activation blocks, and block 0 clears the counters of
-// the streaming kernels (none can be running: this kernel waited for its predecessor).
+// selection runs inside the streaming kernel that follows, see SelectArgs). Bound: latency, from the predecessor's end to the
+// logits. 128 blocks in clusters of four: cluster g owns router rows 16g..16g+15, its CTA q K elements [640q, 640q+640),
+// two of the eight slices whose sums make a logit. The weights are asked into L2 ahead of the dependency wait, into
+// registers behind it together with the x share, which goes to shared memory; every CTA sends the slice sums of rows
+// 4i..4i+3 to CTA i of its cluster through distributed shared memory, and behind one cluster barrier CTA i adds them in
+// slice order 0..7 (fixed: repeated calls are bitwise identical) and stores the logits. Two more warps of every block
+// quantize the activation rows meanwhile, and block 0 clears the counters of the streaming kernels (none can be running:
+// this kernel waited for its predecessor). From the wait to the last block's end, before -> now: one token 4.5 -> 2.3 us,
+// sixteen 8.8 -> 4.2, four with the shared rows 9.8 -> 5.6. (Before: clusters of eight, of which only fifteen find a
+// multiprocessor per CTA where 33 of four do; x was loaded in turns ahead of the weights, quantization stood behind the
+// projection, and slice sums were read out of the other CTAs, which had to wait for that.)
 //
 // With SHARED (the whole decode branch of a layer) the kernel also projects the shared expert's gate/up rows and router
-// row 512, its gate: cluster g takes inter_s / 16 (gate, up) row pairs the same way, FP8 codes widened exactly, and
+// row 512, its gate: cluster g takes inter_s / 32 (gate, up) row pairs the same way, FP8 codes widened exactly, and
 // stores h = bf16(silu(gate) * up). Five megabytes spread over 128 blocks that run anyway: as projections of their own
 // on a second stream they cost four launches, two events and, the expert kernel filling every multiprocessor, no overlap.
 struct SharedRouteArgs {
   const uint8_t* codes;    // [2 inter_s][2560] E4M3
   const void* scales;      // [2 inter_s], fp32 or bf16
   int scale_bf16;
-  int inter_s;             // a multiple of 32, at most kSharedMaxInter
+  int inter_s;             // a multiple of 128, at most kSharedMaxInter
   __nv_bfloat16* h;        // [tokens][inter_s]
 };
 constexpr int kSharedMaxInter = 1024;
-constexpr int kSharedRows = 2 * kSharedMaxInter / 16 + 4;  // of a cluster; the last four: router row 512 and nothing
 __device__ __forceinline__ float fp8_row_scale(const void* scales, int is_bf16, int row) {
   return is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(scales)[row]) : static_cast<const float*>(scales)[row];
 }
@@ -691,17 +692,38 @@ __device__ __forceinline__ float2 e4m3x2_float2(uint32_t pair) {
   return __half22float2(*reinterpret_cast<const __half2*>(&hr));
 }
 constexpr int kRouteSplits = 8, kRouteSlice = H / kRouteSplits;  // 320
-constexpr int kRouteGroups = kExperts / 32;                      // 16
-constexpr int kRouteBlocks = kRouteGroups * kRouteSplits;
+constexpr int kRouteCluster = 4, kRouteSpan = H / kRouteCluster;  // a CTA's share of K: two slices
+constexpr int kRouteRows = 4 * kRouteCluster;                     // router rows of a cluster
+constexpr int kRouteBlocks = kExperts / kRouteRows * kRouteCluster;
+constexpr int kRouteWarps = 16, kRouteThreads = (kRouteWarps + 2) * 32;  // projection; two warps quantize beside it
 static_assert(kRouteSlice == 320, "lane layout below: two 128-element chunks and a 64-element tail");
+static_assert(2 * kRouteBlocks >= kMaxTok * (H / 256), "a quantizing warp takes one 256-value piece");
 
 template <bool XBF16, bool EP, bool SHARED = false>
-__global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* w, const void* xv, int T, float* logits,
-                                                       int stride, fb_moe_decode_workspace ws, EpRouteArgs ep,
-                                                       SharedRouteArgs sh) {
+__global__ void __launch_bounds__(kRouteThreads, 1) route_kernel(const __nv_bfloat16* w, const void* xv, int T, float* logits,
+                                                                 int stride, fb_moe_decode_workspace ws, EpRouteArgs ep,
+                                                                 SharedRouteArgs sh) {
   pdl_launch_dependents();
-  pdl_wait_prior();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = blockIdx.x / kRouteCluster, q = int(cluster_cta_rank());  // (clusters are four consecutive blocks)
+  const int n_sh = SHARED ? sh.inter_s / (kRouteBlocks / kRouteCluster) : 0;  // (gate, up) pairs of this cluster
+  cluster_arrive();  // (its other half stands before the first store into another CTA's shared memory)
+  {
+    // The weights on their way into L2 while the kernel before this one runs out (nothing is read ahead of the wait).
+    const void* src = nullptr;
+    uint32_t bytes = 0;
+    if (tid < kRouteRows) {
+      src = w + size_t(g * kRouteRows + tid) * H + q * kRouteSpan;
+      bytes = kRouteSpan * 2;
+    } else if (SHARED && tid - kRouteRows < 2 * n_sh) {
+      const int i = tid - kRouteRows, row = g * n_sh + (i < n_sh ? i : sh.inter_s + i - n_sh);
+      src = sh.codes + size_t(row) * H + q * kRouteSpan;
+      bytes = kRouteSpan;
+    }
+    if (src && (reinterpret_cast<uintptr_t>(src) & 15) == 0)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+  }
+  pdl_wait_prior();
   constexpr bool ep_mode = EP;  // the single-GPU instantiation carries none of the exchange code
   const uint4* x_lines = nullptr;  // this rank's copy of all tokens' rows, as exchange lines
   if constexpr (EP) {
@@ -714,124 +736,161 @@ __global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* w, c
     uint4* dst = static_cast<uint4*>(ep.peers.x_all[d]) +
                  (size_t(ep.parity) * kMaxTok + size_t(ep.peers.rank) * ep.tpr) * (H / 2);
     const float4* src = reinterpret_cast<const float4*>(ep.x_local);
-    for (int i = lo + tid; i < hi; i += 512) {
+    for (int i = lo + tid; i < hi; i += kRouteThreads) {
       const float4 v = src[i];
       ll_store(dst + 2 * i, v.x, v.y, ep.step);
       ll_store(dst + 2 * i + 1, v.z, v.w, ep.step);
     }
     x_lines = static_cast<const uint4*>(ep.peers.x_all[ep.peers.rank]) + size_t(ep.parity) * kMaxTok * (H / 2);
   }
-  if (blockIdx.x == 0) {
-    if (tid < 2 * kMaxPairs) ws.item_done[tid] = 0;
-    if (tid < kSchedOrderBase) ws.sched[tid] = 0;
-    if (tid < kMaxTok * kMaxDnTiles) ws.sched[kSchedParts + tid] = 0;
-  }
-  __shared__ __align__(16) float s_x[kMaxTok][kRouteSlice];  // x slice [token][320]
-  __shared__ float s_part[32][kMaxTok];                       // this slice's sums [row of the group][token]
-  const int g = blockIdx.x / kRouteSplits, q = int(cluster_cta_rank());  // (clusters are eight consecutive blocks)
-  for (int i = tid; i < T * (kRouteSlice / 4); i += 512) {
-    const int t = i / (kRouteSlice / 4), c = i - t * (kRouteSlice / 4);
-    float4 v;
+  // Four or eight values (the size of v) of token t from element e on, as fp32; e a multiple of four.
+  auto load_x = [&](int t, int e, auto& v) {
+    constexpr int n = sizeof(v) / sizeof(float);
     if constexpr (ep_mode) {
-      const uint4* ln = x_lines + (size_t(t) * H + q * kRouteSlice) / 2 + 2 * c;
-      const float2 a = ll_read(ln, ep.step, ws.status, ep.spin_limit),
-                   b2 = ll_read(ln + 1, ep.step, ws.status, ep.spin_limit);
-      v = make_float4(a.x, a.y, b2.x, b2.y);
-    } else if constexpr (XBF16) {
-      const uint2 u = reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(xv) + size_t(t) * H +
-                                                     q * kRouteSlice)[c];
-      v = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xFFFF0000u), __uint_as_float(u.y << 16),
-                      __uint_as_float(u.y & 0xFFFF0000u));
-    } else {
-      v = reinterpret_cast<const float4*>(static_cast<const float*>(xv) + size_t(t) * H + q * kRouteSlice)[c];
-    }
-    reinterpret_cast<float4*>(&s_x[t][0])[c] = v;
-  }
-  __shared__ float s_sh[SHARED ? kSharedRows : 1][kMaxTok];
-  const int n_sh = SHARED ? sh.inter_s / 16 : 0;  // (gate, up) pairs of this cluster
-  // A warp takes four rows and half of the token slots: every value of x read from shared memory feeds four rows. (Two rows
-  // and all tokens per warp: 3 us instead of 1.5 at sixteen tokens, the shared-memory reads.) Lane holds elements
-  // 128c + 4 lane .. +3 (c = 0, 1) and 256 + 2 lane, +1 of the slice.
-  const int quad = warp >> 1, tok0 = (warp & 1) * (kMaxTok / 2);
-  float wr[4][10];
-  auto bf16_row = [&](int row, float (&v)[10]) {
-    const __nv_bfloat16* wrow = w + size_t(row) * H + q * kRouteSlice;
+      const uint4* ln = x_lines + (size_t(t) * H + e) / 2;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const uint2 u = reinterpret_cast<const uint2*>(wrow)[c * 32 + lane];
-      v[4 * c + 0] = __uint_as_float(u.x << 16);
-      v[4 * c + 1] = __uint_as_float(u.x & 0xFFFF0000u);
-      v[4 * c + 2] = __uint_as_float(u.y << 16);
-      v[4 * c + 3] = __uint_as_float(u.y & 0xFFFF0000u);
+      for (int i = 0; i < n / 2; ++i) {
+        const float2 f = ll_read(ln + i, ep.step, ws.status, ep.spin_limit);
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+      }
+    } else if constexpr (XBF16) {
+      const uint2* src = reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(xv) + size_t(t) * H + e);
+#pragma unroll
+      for (int i = 0; i < n / 4; ++i) {
+        const uint2 u = src[i];
+        v[4 * i] = __uint_as_float(u.x << 16);
+        v[4 * i + 1] = __uint_as_float(u.x & 0xFFFF0000u);
+        v[4 * i + 2] = __uint_as_float(u.y << 16);
+        v[4 * i + 3] = __uint_as_float(u.y & 0xFFFF0000u);
+      }
+    } else {
+      const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(xv) + size_t(t) * H + e);
+#pragma unroll
+      for (int i = 0; i < n / 4; ++i) {
+        const float4 u = src[i];
+        v[4 * i] = u.x;
+        v[4 * i + 1] = u.y;
+        v[4 * i + 2] = u.z;
+        v[4 * i + 3] = u.w;
+      }
     }
-    const uint32_t u = reinterpret_cast<const uint32_t*>(wrow + 256)[lane];
-    v[8] = __uint_as_float(u << 16);
-    v[9] = __uint_as_float(u & 0xFFFF0000u);
   };
-  // Shared expert: a group = two (gate, up) pairs of this cluster = four rows; this lane's codes of group u
-  auto fp8_fetch = [&](int u, uint32_t (&v)[12]) {
+  extern __shared__ __align__(16) float s_x[];  // this CTA's part of x [token][640]
+  // what the cluster's CTAs send this one: [K slice][row][token] of the rows it finishes
+  __shared__ float s_in[kRouteSplits][4][kMaxTok];
+  constexpr int kShPer = SHARED ? kSharedMaxInter / kRouteBlocks : 1;  // (gate, up) pairs a CTA finishes, at most
+  __shared__ float s_sh[kRouteSplits][2 * kShPer][kMaxTok];
+  __shared__ float s_gate[SHARED ? kRouteSplits : 1][kMaxTok];
+  const int per = n_sh / kRouteCluster;  // pairs a CTA finishes
+
+  // Row groups of this cluster: four of four router rows; SHARED: n_sh / 2 of two (gate, up) pairs, then (cluster 0) router
+  // row 512 with three rows of nothing. An item is a group and one of the CTA's two K slices; a warp takes an item for
+  // every value of x it reads from shared memory to feed four rows. (Two rows and all tokens per warp: 3 us instead of
+  // 1.5 at sixteen tokens, the shared-memory reads.) Without shared groups there are items for half of the warps: above two
+  // tokens warps i and i + 8 share item i and take alternate pairs of tokens (neighbours would leave two schedulers idle up
+  // to two tokens). Lane holds elements 128c + 4 lane .. +3 (c = 0, 1) and 256 + 2 lane, +1 of the slice.
+  const int item0 = SHARED ? warp : warp & 7, tok0 = SHARED ? 0 : 2 * (warp >> 3), tok_step = SHARED ? 2 : 4;
+  const int half = item0 & 1, slice = 2 * q + half, k0 = slice * kRouteSlice;  // (a warp's items are all on one slice)
+  uint32_t raw[20];  // a group's rows as loaded
+  float wr[4][10];
+  auto fetch = [&](int row, int n) {  // n router rows
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const uint8_t* wrow = sh.codes + size_t((r & 1 ? sh.inter_s : 0) + g * n_sh + 2 * u + (r >> 1)) * H + q * kRouteSlice;
-      v[3 * r] = reinterpret_cast<const uint32_t*>(wrow)[lane];
-      v[3 * r + 1] = reinterpret_cast<const uint32_t*>(wrow)[32 + lane];
-      v[3 * r + 2] = reinterpret_cast<const uint16_t*>(wrow + 256)[lane];
+      if (r >= n) break;
+      const __nv_bfloat16* wrow = w + size_t(row + r) * H + k0;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const uint2 u = reinterpret_cast<const uint2*>(wrow)[c * 32 + lane];
+        raw[5 * r + 2 * c] = u.x;
+        raw[5 * r + 2 * c + 1] = u.y;
+      }
+      raw[5 * r + 4] = reinterpret_cast<const uint32_t*>(wrow + 256)[lane];
     }
   };
-  auto fp8_widen = [&](const uint32_t (&v)[12]) {
+  auto widen = [&](int n) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        wr[r][2 * i] = r < n ? __uint_as_float(raw[5 * r + i] << 16) : 0.0f;
+        wr[r][2 * i + 1] = r < n ? __uint_as_float(raw[5 * r + i] & 0xFFFF0000u) : 0.0f;
+      }
+  };
+  auto fetch_shared = [&](int u) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint8_t* wrow = sh.codes + size_t((r & 1 ? sh.inter_s : 0) + g * n_sh + 2 * u + (r >> 1)) * H + k0;
+      raw[3 * r] = reinterpret_cast<const uint32_t*>(wrow)[lane];
+      raw[3 * r + 1] = reinterpret_cast<const uint32_t*>(wrow)[32 + lane];
+      raw[3 * r + 2] = reinterpret_cast<const uint16_t*>(wrow + 256)[lane];
+    }
+  };
+  auto widen_shared = [&]() {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        const float2 a = e4m3x2_float2(v[3 * r + c] & 0xFFFFu), b = e4m3x2_float2(v[3 * r + c] >> 16);
+        const float2 a = e4m3x2_float2(raw[3 * r + c] & 0xFFFFu), b = e4m3x2_float2(raw[3 * r + c] >> 16);
         wr[r][4 * c + 0] = a.x;
         wr[r][4 * c + 1] = a.y;
         wr[r][4 * c + 2] = b.x;
         wr[r][4 * c + 3] = b.y;
       }
-      const float2 a = e4m3x2_float2(v[3 * r + 2]);
+      const float2 a = e4m3x2_float2(raw[3 * r + 2]);
       wr[r][8] = a.x;
       wr[r][9] = a.y;
     }
   };
-#pragma unroll
-  for (int r = 0; r < 4; ++r) bf16_row(g * 32 + 4 * quad + r, wr[r]);
-  __syncthreads();
-  // the slice's sums of the four rows in wr over this warp's tokens -> dst[row][token]
-  auto project = [&](float (*dst)[kMaxTok]) {
+  // the slice's sums of the rows in wr over this warp's tokens, into the shared memory of the CTA that finishes the row
+  auto project = [&](int group) {
+    // lanes 4i end with row i >> 1 (of four), token i & 1 of a pair of tokens
+    const int r = lane >> 3;
+    const float* dst = &s_in[slice][r][0];
+    uint32_t owner = uint32_t(group);
+    bool live = (lane & 3) == 0;
+    if (SHARED && group == 4 + n_sh / 2) {
+      dst = s_gate[SHARED ? slice : 0];
+      owner = kRouteCluster - 1;
+      live = live && r == 0;
+    } else if (SHARED && group >= 4) {
+      const int p = 2 * (group - 4) + (r >> 1);
+      owner = uint32_t(p / per);
+      dst = &s_sh[slice][2 * (p - int(owner) * per) + (r & 1)][0];
+    }
 #pragma unroll 1
-    for (int tg = tok0; tg < min(tok0 + kMaxTok / 2, T); tg += 4) {  // (four at a time: registers)
-      float acc[16];  // [row][token of the group]
+    for (int tg = tok0; tg < T; tg += tok_step) {  // (two at a time: registers)
+      float acc[8];  // [row][token of the pair]
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
+      for (int t = 0; t < 2; ++t) {
         float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (tg + t < T) {
-          const float* xr = &s_x[tg + t][0];
+          const float* xr = s_x + (tg + t) * kRouteSpan + half * kRouteSlice;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const float4 x4 = reinterpret_cast<const float4*>(xr)[c * 32 + lane];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-              a[r] = fmaf(wr[r][4 * c + 0], x4.x, a[r]);
-              a[r] = fmaf(wr[r][4 * c + 1], x4.y, a[r]);
-              a[r] = fmaf(wr[r][4 * c + 2], x4.z, a[r]);
-              a[r] = fmaf(wr[r][4 * c + 3], x4.w, a[r]);
+            for (int i = 0; i < 4; ++i) {
+              a[i] = fmaf(wr[i][4 * c + 0], x4.x, a[i]);
+              a[i] = fmaf(wr[i][4 * c + 1], x4.y, a[i]);
+              a[i] = fmaf(wr[i][4 * c + 2], x4.z, a[i]);
+              a[i] = fmaf(wr[i][4 * c + 3], x4.w, a[i]);
             }
           }
           const float2 x2 = reinterpret_cast<const float2*>(xr + 256)[lane];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            a[r] = fmaf(wr[r][8], x2.x, a[r]);
-            a[r] = fmaf(wr[r][9], x2.y, a[r]);
+          for (int i = 0; i < 4; ++i) {
+            a[i] = fmaf(wr[i][8], x2.x, a[i]);
+            a[i] = fmaf(wr[i][9], x2.y, a[i]);
           }
         }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) acc[4 * r + t] = a[r];
+        for (int i = 0; i < 4; ++i) acc[2 * i + t] = a[i];
       }
-      // Sum over the 32 lanes by the butterfly xor 16, 8, 4, 2, 1, halving the values a lane carries at each step but the
-      // last: 16 shuffles for the 16 (row, token) sums. Lanes 2i and 2i + 1 end with row i >> 2, token i & 3 of the group.
+      // Sum over the 32 lanes by the butterfly xor 16, 8, 4, 2, 1, halving the values a lane carries at its first three
+      // steps: nine shuffles for the eight (row, token) sums.
 #pragma unroll
-      for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
+      for (int n = 4, o = 16; n >= 1; n >>= 1, o >>= 1) {
         const bool hi = (lane & o) != 0;
 #pragma unroll
         for (int i = 0; i < n; ++i) {
@@ -839,114 +898,107 @@ __global__ void __launch_bounds__(512, 2) route_kernel(const __nv_bfloat16* w, c
           acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
       }
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
       acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-      if ((lane & 1) == 0) dst[lane >> 3][tg + ((lane >> 1) & 3)] = acc[0];
+      if (live) st_cluster_u32(dst + tg + ((lane >> 2) & 1), owner, __float_as_uint(acc[0]));
     }
   };
-  if constexpr (SHARED) {
-    // the next group's codes are on their way while the current one is projected
-    uint32_t codes[12];
-    const int groups = n_sh / 2;
-    if (quad < groups) fp8_fetch(quad, codes);
-    project(&s_part[4 * quad]);
-#pragma unroll 1
-    for (int u = quad; u < groups; u += 8) {
-      fp8_widen(codes);
-      if (u + 8 < groups) fp8_fetch(u + 8, codes);
-      project(&s_sh[4 * u]);
+
+  // Everything is asked for before anything is waited for: this warp's first rows, then its share of the x slice.
+  if (warp < kRouteWarps) {
+    if (!SHARED || item0 < 8) fetch(g * kRouteRows + 4 * (item0 >> 1), 4);
+    else if (item0 < 8 + n_sh) fetch_shared((item0 - 8) >> 1);
+    constexpr int kMaxX = kMaxTok * (kRouteSpan / 4) / (kRouteWarps * 32);
+    float xs[kMaxX][4];
+#pragma unroll
+    for (int j = 0; j < kMaxX; ++j) {
+      const int i = tid + j * kRouteWarps * 32, t = i / (kRouteSpan / 4), c = i - t * (kRouteSpan / 4);
+      if (t < T) load_x(t, q * kRouteSpan + 4 * c, xs[j]);
     }
-    if (g == 0 && quad == 7) {  // router row 512, with three rows of nothing
-      bf16_row(kExperts, wr[0]);
 #pragma unroll
-      for (int r = 1; r < 4; ++r)
-#pragma unroll
-        for (int i = 0; i < 10; ++i) wr[r][i] = 0.0f;
-      project(&s_sh[2 * n_sh]);
+    for (int j = 0; j < kMaxX; ++j) {
+      const int i = tid + j * kRouteWarps * 32;
+      if (i < T * (kRouteSpan / 4)) reinterpret_cast<float4*>(s_x)[i] = make_float4(xs[j][0], xs[j][1], xs[j][2], xs[j][3]);
+    }
+    named_bar_sync(1, kRouteWarps * 32);
+    cluster_wait();  // every CTA of the cluster runs: its shared memory may be written
+    if (!SHARED || item0 < 8) {
+      widen(4);
+      project(item0 >> 1);
+    }
+    if constexpr (SHARED) {
+#pragma unroll 1
+      for (int i = item0 < 8 ? item0 + kRouteWarps : item0; i < 8 + n_sh; i += kRouteWarps) {
+        if (i != item0) fetch_shared((i - 8) >> 1);
+        widen_shared();
+        project(i >> 1);
+      }
+      if (g == 0 && (item0 >> 1) == (4 + n_sh / 2) % (kRouteWarps / 2)) {
+        fetch(kExperts, 1);
+        widen(1);
+        project(4 + n_sh / 2);
+      }
     }
   } else {
-    project(&s_part[4 * quad]);
-  }
-  cluster_arrive();
-  // activation quantization, one warp per ggml block, strided over every warp of the grid (spread over
-  // the blocks first: a single token's ten blocks go to ten different SMs)
-  {
-    const int act = ep.act;
-    const int per_tok = act == FB_ACT_Q8_K ? H / 256 : H / 32;
-    const int n_warps = gridDim.x * 16;
-    for (int task = warp * gridDim.x + blockIdx.x; task < T * per_tok; task += n_warps) {
-      const int t = task / per_tok, b = task - t * per_tok;
-      auto load = [&](int i) -> float {
-        if constexpr (XBF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(xv)[size_t(t) * H + i]);
-        else return static_cast<const float*>(xv)[size_t(t) * H + i];
-      };
-      uint8_t* out = ws.xq + xq_offset(act) + size_t(t) * FB_XQ_STRIDE;
-      float* scales = reinterpret_cast<float*>(out + H);
-      if (act == FB_ACT_Q8_K) {
-        float v[8];
-        if constexpr (EP) {
-          const uint4* ln = x_lines + (size_t(t) * H + 256 * b + 8 * lane) / 2;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 f = ll_read(ln + i, ep.step, ws.status, ep.spin_limit);
-            v[2 * i] = f.x;
-            v[2 * i + 1] = f.y;
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = load(256 * b + 8 * lane + i);
-        }
+    // activation quantization: one warp per 256 values (spread over the blocks first: a single token's ten pieces go to
+    // ten different SMs); block 0 clears the counters of the streaming kernel
+    const int task = (warp - kRouteWarps) * kRouteBlocks + int(blockIdx.x), t = task / (H / 256), b = task - t * (H / 256);
+    if (t < T) {
+      float v[8];
+      load_x(t, 256 * b + 8 * lane, v);
+      uint8_t* out = ws.xq + xq_offset(ep.act) + size_t(t) * FB_XQ_STRIDE;
+      if (ep.act == FB_ACT_Q8_K) {
         int qv[8], ps;
         const float d = q8k_block_warp(v, qv, ps);
         store_q8k_block_planar(out, H, b, qv, ps, d);
       } else {
-        unsigned short dh;
-        float xv1;
-        if constexpr (EP) {
-          const float2 f = ll_read(x_lines + (size_t(t) * H + 32 * b + lane) / 2, ep.step, ws.status, ep.spin_limit);
-          xv1 = (lane & 1) ? f.y : f.x;
-        } else {
-          xv1 = load(32 * b + lane);
-        }
-        const int qv = q8_0_block_warp(xv1, dh);
-        out[32 * b + q8_0_interleave_index(lane)] = uint8_t(int8_t(qv));
-        if (lane == 0) scales[b] = __half2float(__ushort_as_half(dh));
+        q8_0_eight_blocks_warp(v, true, out + 256 * b, reinterpret_cast<float*>(out + H) + 8 * b);
       }
     }
+    if (blockIdx.x == 0) {
+      static_assert(kSchedOrderBase <= 2 * kMaxPairs && kMaxTok * kMaxDnTiles <= 2 * kMaxPairs, "one loop clears all");
+      for (int i = tid - kRouteWarps * 32; i < 2 * kMaxPairs; i += 64) {
+        ws.item_done[i] = 0;
+        if (i < kSchedOrderBase) ws.sched[i] = 0;
+        if (i < kMaxTok * kMaxDnTiles) ws.sched[kSchedParts + i] = 0;
+      }
+    }
+    __syncwarp();
+    cluster_wait();
   }
-  cluster_wait();
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();  // the sums of all slices are here; nobody reads another CTA's memory from now on
   if (tid < 4 * kMaxTok) {
-    const int r = 4 * q + (tid >> 4), t = tid & 15;
+    const int r = tid >> 4, t = tid & 15;
     if (t < T) {
       float v = 0.0f;
 #pragma unroll
-      for (int qq = 0; qq < kRouteSplits; ++qq) v += ld_cluster_f32(&s_part[r][t], uint32_t(qq));
-      logits[size_t(t) * stride + g * 32 + r] = v;
+      for (int qq = 0; qq < kRouteSplits; ++qq) v += s_in[qq][r][t];
+      logits[size_t(t) * stride + g * kRouteRows + 4 * q + r] = v;
     }
   }
   if constexpr (SHARED) {
-    const int per = (n_sh + kRouteSplits - 1) / kRouteSplits;  // pairs this CTA finishes
-    for (int i = tid; i < per * kMaxTok; i += 512) {
-      const int p = q * per + (i >> 4), t = i & 15;
-      if (t >= T || p >= n_sh) continue;
+    for (int i = tid; i < per * kMaxTok; i += kRouteThreads) {
+      const int p = i >> 4, j = g * n_sh + q * per + p, t = i & 15;
+      if (t >= T) continue;
       float gv = 0.0f, uv = 0.0f;
 #pragma unroll
       for (int qq = 0; qq < kRouteSplits; ++qq) {
-        gv += ld_cluster_f32(&s_sh[2 * p][t], uint32_t(qq));
-        uv += ld_cluster_f32(&s_sh[2 * p + 1][t], uint32_t(qq));
+        gv += s_sh[qq][2 * p][t];
+        uv += s_sh[qq][2 * p + 1][t];
       }
-      const int j = g * n_sh + p;
       gv *= fp8_row_scale(sh.scales, sh.scale_bf16, j);
       uv *= fp8_row_scale(sh.scales, sh.scale_bf16, sh.inter_s + j);
       sh.h[size_t(t) * sh.inter_s + j] = __float2bfloat16_rn(gv / (1.0f + expf(-gv)) * uv);
     }
-    if (g == 0 && q == kRouteSplits - 1 && tid < T) {
+    if (g == 0 && q == kRouteCluster - 1 && tid < T) {
       float v = 0.0f;
 #pragma unroll
-      for (int qq = 0; qq < kRouteSplits; ++qq) v += ld_cluster_f32(&s_sh[2 * n_sh][tid], uint32_t(qq));
+      for (int qq = 0; qq < kRouteSplits; ++qq) v += s_gate[SHARED ? qq : 0][tid];
       logits[size_t(tid) * stride + kExperts] = v;
     }
   }
-  cluster_sync();  // no CTA of the cluster leaves while another may still read its slice sums
 }
 
 // ------------------------------------------------------------------------------ streaming skeleton
@@ -1530,9 +1582,23 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
     return invalid("layer_decode: bad arguments (tokens must be 1..16, logits scratch [tokens][513] required)");
   if (!ws_fits(ws, layout, true, true))
     return invalid("layer_decode: workspace was made for a different layout");
-  const dim3 grid(kRouteBlocks), block(512);
+  const dim3 grid(kRouteBlocks), block(kRouteThreads);
+  // (one opt-in per kernel and device: the x share of sixteen tokens and the shared expert's sums pass 48 KB together)
+  static PerDeviceOnce once;
+  const cudaError_t attr = per_device_once(once, [] {
+    constexpr size_t most = size_t(kMaxTok) * kRouteSpan * 4;
+    cudaError_t a = opt_in_smem(route_kernel<false, false>, most);
+    if (a == cudaSuccess) a = opt_in_smem(route_kernel<true, false>, most);
+    if (a == cudaSuccess) a = opt_in_smem(route_kernel<false, true>, most);
+    if (a == cudaSuccess) a = opt_in_smem(route_kernel<true, false, true>, most);
+    return a;
+  });
+  if (attr != cudaSuccess) {
+    set_error("layer_decode: shared-memory opt-in: %s", cudaGetErrorString(attr));
+    return int32_t(attr);
+  }
   auto launch = [&](auto kernel) {
-    return launch_pdl_cluster(kernel, grid, block, 0, as_stream(stream), unsigned(kRouteSplits),
+    return launch_pdl_cluster(kernel, grid, block, size_t(tokens) * kRouteSpan * 4, as_stream(stream), unsigned(kRouteCluster),
                               static_cast<const __nv_bfloat16*>(router_w_bf16), x, tokens, logits_scratch,
                               int(FB_ROUTER_ROWS), *ws, era, shared ? *shared : SharedRouteArgs{});
   };
