@@ -24,13 +24,13 @@ constexpr int kSignTabWords = 16;
 // One copy per translation unit (internal linkage), initialised at load time.
 static __constant__ uint16_t c_iq3s_grid_packed[512] = {FB_IQ3S_GRID_PACKED};
 
-__device__ __forceinline__ uint32_t iq3s_grid_entry(int i) {
-  const uint32_t p = c_iq3s_grid_packed[i];
+__device__ __forceinline__ uint32_t iq3s_expand(uint32_t p) {
   uint32_t w = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) w |= (2u * ((p >> (3 * j)) & 7u) + 1u) << (8 * j);
   return w;
 }
+__device__ __forceinline__ uint32_t iq3s_grid_entry(int i) { return iq3s_expand(c_iq3s_grid_packed[i]); }
 
 // Called by every thread of the block; caller synchronizes afterwards.
 __device__ __forceinline__ void iq3s_tables_fill(uint32_t* gridrep, uint32_t* signtab) {
@@ -375,26 +375,33 @@ __device__ __forceinline__ void warp_topk10(LoadF load_logit, int* ids, float* w
   topk_softmax(vals, weights);
 }
 
-// The same selection as a short dependent chain (a decode step runs it in every CTA). The tenth largest
-// of the 32 lanes' own maxima is a lower bound of the tenth largest logit (ten different logits reach it),
-// so only logits at or above it can win; they are compacted into `scratch` (32 entries of this warp, shared
-// memory), one per lane, every lane ranks its candidate against the others through shuffles (larger key,
-// then lower id: a strict order), and ranks 0..9 are the winners. More than 32 survivors (many equal
-// logits) take the general path. Same winners, same order, same weights as warp_topk10; out_ids / out_w
-// (ten entries each, shared memory) are complete after the caller's next barrier.
+// The same selection as a short dependent chain (a decode step runs it in every CTA): winners and their logits; the
+// weights are top10_weights below. The tenth largest of the maxima of the sixteen lane pairs is a lower bound of the tenth
+// largest logit (ten different logits reach it), so only logits at or above it can win (fourteen on average); they are
+// compacted into `scratch` (32 entries of this warp, shared memory, 16-byte aligned), one per lane, every lane ranks its
+// candidate against the others (larger logit, then lower id: a strict order), and ranks 0..9 are the winners. More than 32
+// survivors (many equal logits), or a bound of -infinity (which NaN counts as), take the general path. Same winners, same
+// order as warp_topk10; out_ids / out_vals (ten entries each, shared memory) are complete after the caller's next barrier.
+// Bound: instructions on one warp's chain. With 32 lane maxima, ranks by shuffles and the softmax in the chain the whole
+// selection took 2.8 us at one token and 4.1 at sixteen, now 2.1 and 3.3.
 template <class LoadF>
-__device__ __forceinline__ void warp_topk10_pruned(LoadF load_logit, uint2* scratch, int* out_ids, float* out_w) {
+__device__ __forceinline__ void warp_top10_pruned(LoadF load_logit, uint2* scratch, int* out_ids, float* out_vals) {
   const int lane = threadIdx.x & 31;
-  float x[16];  // (fmaxf turns a NaN into -infinity; the keys are made for the candidates alone)
+  float x[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) x[i] = fmaxf(load_logit(lane + 32 * i), -INFINITY);
-  float lm = x[0];
+  for (int i = 0; i < 16; ++i) x[i] = load_logit(lane + 32 * i);
+  float pm = -INFINITY;  // (fmaxf passes a NaN over; the comparisons below are false for it)
 #pragma unroll
-  for (int i = 1; i < 16; ++i) lm = fmaxf(lm, x[i]);
-  int above = 0;  // lanes whose maximum is larger than this lane's
+  for (int i = 0; i < 16; ++i) pm = fmaxf(pm, x[i]);
+  pm = fmaxf(pm, __shfl_xor_sync(0xffffffffu, pm, 1));
+  int above = 0;  // lane pairs whose maximum is larger than this pair's
 #pragma unroll
-  for (int j = 0; j < 32; ++j) above += __shfl_sync(0xffffffffu, lm, j) > lm ? 1 : 0;
-  const float thr = key_logit(__reduce_min_sync(0xffffffffu, above < FB_TOPK ? logit_key(lm) : 0xffffffffu));
+  for (int j = 0; j < 16; ++j) above += __shfl_sync(0xffffffffu, pm, 2 * j) > pm ? 1 : 0;
+  float thr;
+  {
+    const float v = above < FB_TOPK ? pm : INFINITY;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(thr) : "f"(v));
+  }
   int mine = 0;
 #pragma unroll
   for (int i = 0; i < 16; ++i) mine += x[i] >= thr ? 1 : 0;
@@ -405,14 +412,7 @@ __device__ __forceinline__ void warp_topk10_pruned(LoadF load_logit, uint2* scra
     if (lane >= o) incl += v;
   }
   const int total = __shfl_sync(0xffffffffu, incl, 31);
-  int pos = incl - mine;  // (the candidates' order does not matter: they are ranked by key and id)
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-    if (x[i] >= thr) {
-      if (pos < 32) scratch[pos] = make_uint2(logit_key(x[i]), uint32_t(lane + 32 * i));
-      ++pos;
-    }
-  if (total > 32) {
+  if (total > 32 || thr == -INFINITY) {
     int ids[FB_TOPK];
     float w[FB_TOPK];
     warp_topk10(load_logit, ids, w);
@@ -420,33 +420,36 @@ __device__ __forceinline__ void warp_topk10_pruned(LoadF load_logit, uint2* scra
     for (int k = 0; k < FB_TOPK; ++k)
       if (lane == k) {
         out_ids[k] = ids[k];
-        out_w[k] = w[k];
+        out_vals[k] = key_logit(logit_key(load_logit(ids[k])));
       }
     return;
   }
+  uint2* at = scratch + (incl - mine);  // (the candidates' order does not matter)
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (x[i] >= thr) *at++ = make_uint2(__float_as_uint(x[i]), uint32_t(lane + 32 * i));
+  if (lane == 31 && (total & 1)) *at = make_uint2(0xff800000u, 0x7fffffffu);  // (read in pairs; -infinity beats nobody)
   __syncwarp();
-  uint32_t ck = 0u, cid = 0xffffffffu;  // padding lanes lose to every candidate
-  if (lane < total) {
-    const uint2 c = scratch[lane];
-    ck = c.x;
-    cid = c.y;
-  }
-  int rank = 0;  // (only the real candidates take a turn: a lone warp pays a few cycles per instruction)
+  const uint2 c = scratch[lane < total ? lane : 0];
+  const float cv = __uint_as_float(c.x);
+  int rank = 0;
 #pragma unroll 4
-  for (int j = 0; j < total; ++j) {
-    const uint32_t ok = __shfl_sync(0xffffffffu, ck, j), oi = __shfl_sync(0xffffffffu, cid, j);
-    rank += (ok > ck || (ok == ck && oi < cid)) ? 1 : 0;
+  for (int j = 0; j < total; j += 2) {
+    const uint4 o = *reinterpret_cast<const uint4*>(scratch + j);
+    const float a = __uint_as_float(o.x), b = __uint_as_float(o.z);
+    rank += a > cv || (a == cv && o.y < c.y) ? 1 : 0;
+    rank += b > cv || (b == cv && o.w < c.y) ? 1 : 0;
   }
-  if (lane >= total) rank = 32;
-  __syncwarp();  // every lane holds its candidate: the scratch entries can carry the winners' logits now
-  float* vals = reinterpret_cast<float*>(scratch);
-  if (rank < FB_TOPK) {
-    out_ids[rank] = int(cid);
-    vals[rank] = key_logit(ck);
+  if (lane < total && rank < FB_TOPK) {
+    out_ids[rank] = int(c.y);
+    out_vals[rank] = cv;
   }
-  __syncwarp();
-  // softmax over the winners exactly as topk_softmax: exp(v - top), summed in rank order. Lane k computes
-  // the k-th term; the ten terms then reach every lane through shuffles and are added in the same order.
+}
+
+// Softmax over the winners exactly as topk_softmax: exp(v - top), summed in rank order, by one warp. Lane k computes the
+// k-th term; the ten terms then reach every lane through shuffles and are added in the same order.
+__device__ __forceinline__ void top10_weights(const float* vals, float* out_w) {
+  const int lane = threadIdx.x & 31;
   const float e = expf(vals[lane < FB_TOPK ? lane : 0] - vals[0]);
   float sum = 0.0f;
 #pragma unroll

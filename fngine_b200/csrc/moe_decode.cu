@@ -336,6 +336,7 @@ struct WorkCache {
   int slot[kMaxPairs];
   int pair_token[kMaxPairs];
   float pair_weight[kMaxPairs];
+  int token_row[kMaxTok][kTopK];  // a token's pairs in slot order (only by the CTA's own selection)
   int n_items;
 };
 // Called by the 32 lanes of the producer warp (the only reader) after the wait on the preceding kernel;
@@ -358,15 +359,19 @@ __device__ __forceinline__ void work_cache_fill(const fb_moe_decode_workspace& w
 
 // ------------------------------------------------------------------------------ select
 struct SelectScratch {
-  uint2 cand[kMaxTok][32];               // a token's candidates: key, id
-  int id[kMaxTok][kTopK];
-  float w[kMaxTok][kTopK];
+  union {
+    uint2 cand[kMaxTok][32];  // a token's candidates: logit, id
+    struct {  // behind those
+      int begin[kExperts];         // physical slot -> first pair of its item
+      int slot[kMaxTok][kTopK];    // physical slots of the winners, -1: not held here
+    };
+  };
+  float val[kMaxTok][kTopK];             // the winners' logits
   uint32_t tok[kExperts];                // physical slot -> mask of the tokens that chose it
-  int begin[kExperts];                   // physical slot -> first pair of its item
   int hist[kExperts / 32][kMaxTok + 1];  // [warp of slots][token count - 1] -> items (padded: no bank conflicts)
   int scan[kExperts / 32];               // [warp of slots] -> its pairs | its items << 16
 };
-// load(t, e): logit e of token t. `scratch`: shared memory that is free until the call returns.
+// load(t, e): logit e of token t. `scratch`: shared memory (16-byte aligned) that is free until the call returns.
 // Called by every thread of a block of 512 or more threads. The work list goes to `wc` in shared memory
 // (complete when the call returns) and, with `publish`, to the device work list as well; `reset` clears
 // the tile and item counters of the streaming kernels (only where no such kernel can be running). The
@@ -375,9 +380,9 @@ struct SelectScratch {
 // masks per physical slot (shared-memory atomics), one scan over the 512 slots (thread = slot), the items ranked by a
 // counting sort on their token counts (warp matches), and the pairs placed from the scan. Few
 // warps do this work and a warp on its own retires an instruction every few cycles: what counts here is the
-// number of instructions on the longest chain, not the arithmetic. (Up to three tokens: one warp, shuffles. Above, the
-// list took 4.0 us at sixteen tokens with two scans, every thread adding 32 warp totals and a ranking of 80 adds per
-// item.)
+// number of instructions on the longest chain, not the arithmetic. So the routing weights are computed by warps that
+// the list does not need, and the device work list is written behind the last barrier. (Up to three tokens: one warp,
+// shuffles.)
 //   items  = distinct selected experts held on this rank, in physical-slot order
 //   pairs  = (item, token), tokens ascending inside an item
 //   order  = items by token count, most first, ties by item index (the streaming kernels' visiting order)
@@ -386,10 +391,16 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
                                              const fb_moe_decode_workspace& ws, uint32_t* counts, bool remote_ok,
                                              bool publish, bool reset, WorkCache& wc, SelectScratch& scratch) {
   static_assert(kExperts == 512 && kMaxTok == 16, "sixteen warps of slots, lanes 0..15 hold the token-count classes");
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ int s_pair[kMaxTok][kTopK];  // (block 0 reads it behind the last barrier)
-  auto& [s_cand, s_id, s_w, s_tok, s_begin, s_hist, s_scan] = scratch;
-  fb_moe_decode_work* work = ws.work;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  // (these three outlive the scratch memory)
+  __shared__ int s_pair[kMaxTok][kTopK];
+  __shared__ int s_id[kMaxTok][kTopK];
+  __shared__ float s_w[kMaxTok][kTopK];
+  auto& s_val = scratch.val;
+  auto& s_tok = scratch.tok;
+  auto& s_begin = scratch.begin;
+  auto& s_hist = scratch.hist;
+  auto& s_scan = scratch.scan;
   if (tid < kExperts) s_tok[tid] = 0;
   if (tid < kExperts / 32 * (kMaxTok + 1)) (&s_hist[0][0])[tid] = 0;
   if (reset) {
@@ -398,24 +409,29 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
   }
   // (One warp per token. All sixteen warps on each token's slices - maxima, threshold, candidates and ranking behind a
   // barrier each - was slower at every batch: 3.3 against 2.5 us at one token, 6 against 3 at sixteen.)
-  if (warp < T) warp_topk10_pruned([&](int e) { return load(warp, e); }, s_cand[warp], s_id[warp], s_w[warp]);
+  if (warp < T) warp_top10_pruned([&](int e) { return load(warp, e); }, scratch.cand[warp], s_id[warp], s_val[warp]);
   __syncthreads();
   const int np = T * kTopK;
-  if (np <= 32) {
-    // Up to three tokens: the pairs fit one warp, which builds the whole list through shuffles (lane = pair),
-    // two barriers in all instead of five. Same list as the general path below.
+  const bool small = np <= 32;
+  {
+    const int first = small ? 1 : warps > kMaxTok ? kMaxTok : 0;
+    if (warp >= first)
+      for (int t = warp - first; t < T; t += warps - first) top10_weights(s_val[t], s_w[t]);
+  }
+  const bool valid = tid < np;
+  const int pt = tid / kTopK, pk = tid - pt * kTopK;
+  if (small) {
+    // Up to three tokens: the pairs fit one warp, which builds the whole list through shuffles (lane = pair).
+    // Same list as the general path below.
     if (warp == 0) {
-      const bool pv = lane < np;
-      const int t = lane / kTopK, k = lane - t * kTopK;
-      const int e = pv ? s_id[t][k] : 0;
-      int slot = !pv ? -1 : slot_of ? slot_of[e] : e;
+      const int e = valid ? s_id[pt][pk] : 0;
+      int slot = !valid ? -1 : slot_of ? slot_of[e] : e;
       if (slot >= kExperts) slot = -1;
-      const float wt = pv ? s_w[t][k] : 0.0f;
-      const int key = slot >= 0 ? slot * kMaxTok + t : 0x7fffffff;  // pairs not held here sort last
+      const int key = slot >= 0 ? slot * kMaxTok + pt : 0x7fffffff;  // pairs not held here sort last
       // (a lone warp runs at a few cycles per instruction: the loops below take np turns, not 32, and a single
       // token, whose ten pairs are ten different experts, needs only the first)
       int idx = 0, trank = 0, cnt = 0;
-#pragma unroll 2
+#pragma unroll 5
       for (int j = 0; j < np; ++j) {
         const int kj = __shfl_sync(0xffffffffu, key, j);
         const bool same = kj != 0x7fffffff && (kj / kMaxTok) == slot;
@@ -441,173 +457,147 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
           rank += ((first_m >> j) & 1u) && (cj > cnt || (cj == cnt && ij < item)) ? 1 : 0;
         }
       }
-      if (hot) {
-        wc.pair_token[idx] = t;
-        wc.pair_weight[idx] = wt;
-        if (publish) {
-          work->pair_token[idx] = t;
-          work->pair_weight[idx] = wt;
-        }
-      }
+      if (hot) wc.pair_token[idx] = pt;
       if (first) {
         wc.slot[item] = slot;
         wc.pair_begin[item] = idx;
         wc.order[rank] = item;
-        if (publish) {
-          work->item_slot[item] = slot;
-          work->item_pair_begin[item] = idx;
-          ws.sched[kSchedOrderBase + rank] = item;
-        }
       }
       if (lane == 0) {
         wc.pair_begin[n_items] = n_pairs;
         wc.n_items = n_items;
       }
-      if (pv && counts) atomicAdd(&counts[e], 1u);
-      if (publish) {
-        if (pv) {
-          work->topk_expert[t][k] = e;
-          work->topk_weight[t][k] = wt;
-        }
-        // a token's held pairs in pair order (= slot order)
-        int prank = idx, nh = n_pairs;
-        if (T > 1) {
-          prank = nh = 0;
-#pragma unroll 2
-          for (int j = 0; j < np; ++j) {
-            const int kj = __shfl_sync(0xffffffffu, key, j), ixj = __shfl_sync(0xffffffffu, idx, j);
-            const bool mine = j / kTopK == t && kj != 0x7fffffff;
-            nh += mine ? 1 : 0;
-            prank += mine && ixj < idx ? 1 : 0;
-          }
-        }
-        if (hot) work->token_pairs[t][prank] = idx;
-        if (pv && k == 0) {
-          work->token_pair_count[t] = nh;
-          work->token_cold_count[t] = kTopK - nh;
-        }
-        if (lane == 0) {
-          work->item_pair_begin[n_items] = n_pairs;
-          work->n_items = n_items;
-          work->n_pairs = n_pairs;
-          work->n_cold = np - n_pairs;
-          work->tokens = T;
-          if (np - n_pairs && !remote_ok) atomicMax(ws.status, uint32_t(FB_STATUS_BAD_WORK));
-        }
+      if (valid) {
+        s_pair[pt][pk] = hot ? idx : -1;
+        if (counts) atomicAdd(&counts[e], 1u);
       }
     }
     __syncthreads();
-    return;
+    if (valid) {
+      const int idx = s_pair[pt][pk];
+      if (idx >= 0) wc.pair_weight[idx] = s_w[pt][pk];
+    }
+    if (warp == 1 && lane < np) {  // a token's pairs in slot order = pair order
+      const int t = lane / kTopK, idx = s_pair[t][lane - t * kTopK];
+      int rank = 0;
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k) rank += uint32_t(s_pair[t][k]) < uint32_t(idx) ? 1 : 0;  // (-1 is the largest)
+      if (idx >= 0) wc.token_row[t][rank] = idx;
+    }
+  } else {
+    int my_slot = -1;
+    if (valid) {
+      const int e = s_id[pt][pk];
+      my_slot = slot_of ? slot_of[e] : e;
+      if (my_slot >= kExperts) my_slot = -1;
+      scratch.slot[pt][pk] = my_slot;
+      if (my_slot >= 0) atomicOr(&s_tok[my_slot], 1u << pt);
+      if (counts) atomicAdd(&counts[e], 1u);
+    }
+    __syncthreads();
+    // Thread = slot, sixteen warps. Inside the warps: inclusive scan of (pairs, items) in one word, and each item's place
+    // among the warp's items of as many tokens.
+    const int c = tid < kExperts ? __popc(s_tok[tid]) : 0;
+    int incl = c | (c > 0 ? 1 << 16 : 0), peer_rank = 0;
+    if (warp < kExperts / 32) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+      }
+      if (lane == 31) s_scan[warp] = incl;
+      const uint32_t peers = __match_any_sync(0xffffffffu, c);
+      peer_rank = __popc(peers & ((1u << lane) - 1u));
+      if (c > 0 && peer_rank == 0) s_hist[warp][c - 1] = __popc(peers);
+    }
+    __syncthreads();
+    if (warp < kExperts / 32) {
+      const int v = lane < kExperts / 32 ? s_scan[lane] : 0;
+      const int base = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0), total = __reduce_add_sync(0xffffffffu, v);
+      const int n_pairs = total & 0xFFFF, n_items = total >> 16;
+      // Visiting order: items with more tokens first, ties by item index. Lane = token count - 1: items of that count in
+      // all warps and in the warps before this one, then the items of larger counts.
+      int all = 0, before = 0;
+#pragma unroll
+      for (int w = 0; w < kExperts / 32; ++w) {
+        const int h = s_hist[w][lane & 15];
+        all += h;
+        before += w < warp ? h : 0;
+      }
+      int larger = lane < kMaxTok ? all : 0;
+#pragma unroll
+      for (int o = 1; o < kMaxTok; o <<= 1) {
+        const int x = __shfl_down_sync(0xffffffffu, larger, o);
+        larger += lane + o < kMaxTok ? x : 0;
+      }
+      const int order_base = __shfl_sync(0xffffffffu, larger - all + before, (c - 1) & 15);
+      if (c > 0) {  // a chosen slot = an item
+        const int first = base + incl;
+        const int item = (first >> 16) - 1, pair_begin = (first & 0xFFFF) - c;
+        s_begin[tid] = pair_begin;
+        wc.slot[item] = tid;
+        wc.pair_begin[item] = pair_begin;
+        wc.order[order_base + peer_rank] = item;
+      }
+      if (tid == 0) {
+        wc.pair_begin[n_items] = n_pairs;
+        wc.n_items = n_items;
+      }
+    }
+    // thread = pair, of the first warps, and for the pairs' places in their tokens of the last ones (of all there are)
+    const int p2 = tid - (blockDim.x >= 512 + kMaxPairs ? 512 : 0), t2 = p2 / kTopK;
+    int slot2 = -1, rank2 = 0;
+    if (p2 >= 0 && p2 < np) {
+      slot2 = scratch.slot[t2][p2 - t2 * kTopK];
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k) rank2 += uint32_t(scratch.slot[t2][k]) < uint32_t(slot2) ? 1 : 0;
+    }
+    __syncthreads();
+    auto pair_of = [&](int slot, int t) {  // tokens ascending inside an item
+      return s_begin[slot] + __popc(s_tok[slot] & ((1u << t) - 1u));
+    };
+    if (valid) {
+      int idx = -1;
+      if (my_slot >= 0) {
+        idx = pair_of(my_slot, pt);
+        wc.pair_token[idx] = pt;
+        wc.pair_weight[idx] = s_w[pt][pk];
+      }
+      s_pair[pt][pk] = idx;
+    }
+    if (slot2 >= 0) wc.token_row[t2][rank2] = pair_of(slot2, t2);
   }
-  const bool valid = tid < np;
-  const int pt = tid / kTopK, pk = tid - pt * kTopK;
-  int my_e = 0, my_slot = -1;
+  __syncthreads();
+  if (!publish || tid >= kExperts) return;  // (the device list is behind everything the streaming waits for)
+  fb_moe_decode_work* work = ws.work;
+  const int n_items = wc.n_items, n_pairs = wc.pair_begin[n_items];
+  if (tid < n_items) {
+    work->item_slot[tid] = wc.slot[tid];
+    ws.sched[kSchedOrderBase + tid] = wc.order[tid];
+  }
+  if (tid <= n_items) work->item_pair_begin[tid] = wc.pair_begin[tid];
+  if (tid < n_pairs) {
+    work->pair_token[tid] = wc.pair_token[tid];
+    work->pair_weight[tid] = wc.pair_weight[tid];
+  }
   if (valid) {
-    my_e = s_id[pt][pk];
-    my_slot = slot_of ? slot_of[my_e] : my_e;
-    if (my_slot >= kExperts) my_slot = -1;
-    if (my_slot >= 0) atomicOr(&s_tok[my_slot], 1u << pt);
-    if (counts) atomicAdd(&counts[my_e], 1u);
-  }
-  __syncthreads();
-  // Thread = slot, sixteen warps. Inside the warps: inclusive scan of (pairs, items) in one word, and each item's place
-  // among the warp's items of as many tokens.
-  const int c = tid < kExperts ? __popc(s_tok[tid]) : 0;
-  int incl = c | (c > 0 ? 1 << 16 : 0), peer_rank = 0;
-  if (warp < kExperts / 32) {
+    work->topk_expert[pt][pk] = s_id[pt][pk];
+    work->topk_weight[pt][pk] = s_w[pt][pk];
+    int held = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += x;
-    }
-    if (lane == 31) s_scan[warp] = incl;
-    const uint32_t peers = __match_any_sync(0xffffffffu, c);
-    peer_rank = __popc(peers & ((1u << lane) - 1u));
-    if (c > 0 && peer_rank == 0) s_hist[warp][c - 1] = __popc(peers);
-  }
-  __syncthreads();
-  if (warp < kExperts / 32) {
-    const int v = lane < kExperts / 32 ? s_scan[lane] : 0;
-    const int base = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0), total = __reduce_add_sync(0xffffffffu, v);
-    const int n_pairs = total & 0xFFFF, n_items = total >> 16;
-    // Visiting order: items with more tokens first, ties by item index. Lane = token count - 1: items of that count in
-    // all warps and in the warps before this one, then the items of larger counts.
-    int all = 0, before = 0;
-#pragma unroll
-    for (int w = 0; w < kExperts / 32; ++w) {
-      const int h = s_hist[w][lane & 15];
-      all += h;
-      before += w < warp ? h : 0;
-    }
-    int larger = lane < kMaxTok ? all : 0;
-#pragma unroll
-    for (int o = 1; o < kMaxTok; o <<= 1) {
-      const int x = __shfl_down_sync(0xffffffffu, larger, o);
-      larger += lane + o < kMaxTok ? x : 0;
-    }
-    const int order_base = __shfl_sync(0xffffffffu, larger - all + before, (c - 1) & 15);
-    if (c > 0) {  // a chosen slot = an item
-      const int first = base + incl;
-      const int item = (first >> 16) - 1, pair_begin = (first & 0xFFFF) - c, rank = order_base + peer_rank;
-      s_begin[tid] = pair_begin;
-      wc.slot[item] = tid;
-      wc.pair_begin[item] = pair_begin;
-      wc.order[rank] = item;
-      if (publish) {
-        work->item_slot[item] = tid;
-        work->item_pair_begin[item] = pair_begin;
-        ws.sched[kSchedOrderBase + rank] = item;
-      }
-    }
-    if (tid == 0) {
-      wc.pair_begin[n_items] = n_pairs;
-      wc.n_items = n_items;
-      if (publish) {
-        work->item_pair_begin[n_items] = n_pairs;
-        work->n_items = n_items;
-        work->n_pairs = n_pairs;
-        work->n_cold = np - n_pairs;
-        work->tokens = T;
-        if (np - n_pairs && !remote_ok) atomicMax(ws.status, uint32_t(FB_STATUS_BAD_WORK));
-      }
+    for (int k = 0; k < kTopK; ++k) held += s_pair[pt][k] >= 0 ? 1 : 0;
+    if (pk < held) work->token_pairs[pt][pk] = wc.token_row[pt][pk];
+    if (pk == 0) {
+      work->token_pair_count[pt] = held;
+      work->token_cold_count[pt] = kTopK - held;
     }
   }
-  __syncthreads();
-  if (valid) {
-    int idx = -1;
-    if (my_slot >= 0) {
-      idx = s_begin[my_slot] + __popc(s_tok[my_slot] & ((1u << pt) - 1u));  // tokens ascending inside an item
-      wc.pair_token[idx] = pt;
-      wc.pair_weight[idx] = s_w[pt][pk];
-      if (publish) {
-        work->pair_token[idx] = pt;
-        work->pair_weight[idx] = s_w[pt][pk];
-      }
-    }
-    s_pair[pt][pk] = idx;
-    if (publish) {
-      work->topk_expert[pt][pk] = my_e;
-      work->topk_weight[pt][pk] = s_w[pt][pk];
-    }
-  }
-  __syncthreads();
-  if (publish && tid < T) {
-    int idx10[kTopK];
-#pragma unroll
-    for (int k = 0; k < kTopK; ++k) idx10[k] = s_pair[tid][k];
-    int nh = 0;
-#pragma unroll
-    for (int k = 0; k < kTopK; ++k) {
-      if (idx10[k] >= 0) {
-        int rank = 0;
-#pragma unroll
-        for (int k2 = 0; k2 < kTopK; ++k2) rank += (idx10[k2] >= 0 && idx10[k2] < idx10[k]) ? 1 : 0;
-        work->token_pairs[tid][rank] = idx10[k];  // slot order == pair order
-        ++nh;
-      }
-    }
-    work->token_pair_count[tid] = nh;
-    work->token_cold_count[tid] = kTopK - nh;
+  if (tid == 0) {
+    work->n_items = n_items;
+    work->n_pairs = n_pairs;
+    work->n_cold = np - n_pairs;
+    work->tokens = T;
+    if (np - n_pairs && !remote_ok) atomicMax(ws.status, uint32_t(FB_STATUS_BAD_WORK));
   }
 }
 
@@ -643,7 +633,7 @@ __global__ void __launch_bounds__(512) select_kernel(const float* logits, int lo
     return;
   }
   __shared__ WorkCache s_work;  // the streaming kernels of this path read the device work list instead
-  __shared__ SelectScratch s_scratch;
+  __shared__ __align__(16) SelectScratch s_scratch;
   select_block([&](int t, int e) { return logits[size_t(t) * logits_stride + e]; },
                slot_of, T, ws, counts, false, true, true, s_work, s_scratch);
 }

@@ -46,15 +46,6 @@ __device__ __forceinline__ void sign_table_fill(uint32_t* signtab) {
     signtab[threadIdx.x] = m;
   }
 }
-__device__ __forceinline__ void iq3s_half_tables_fill(uint32_t* gridrep, uint32_t* signtab) {
-  // consecutive threads write consecutive 16-byte pieces (eight per entry): no bank conflicts
-  for (int i = threadIdx.x; i < 512 * 8; i += blockDim.x) {
-    const uint32_t w = (iq3s_grid_entry(i >> 3) >> 1) & 0x07070707u;
-    reinterpret_cast<uint4*>(gridrep)[i] = make_uint4(w, w, w, w);
-  }
-  sign_table_fill(signtab);
-}
-
 // One 32-weight sub-block: P = sum over its 8 look-ups of dp4a(G ^ m, a) for each of TT tokens.
 // qs_lo/qs_hi = its 8 index bytes, qh = a word whose bits [sh, sh+8) are the ninth index bits, sg = its
 // 32 sign bits (nibble l = look-up l). sign_base = shared-window address of the 16-word mask table
@@ -265,7 +256,7 @@ struct GuFmt<FB_FMT_IQ3_XXS> { static constexpr int kBlock = 98, kTable = 256 * 
 template <>
 struct GuFmt<FB_FMT_IQ4_XS> { static constexpr int kBlock = 136, kTable = 0; };
 
-constexpr int kStaticSmem = 6144;  // the kernel's own shared variables, at most
+constexpr int kStaticSmem = 7168;  // the kernel's own shared variables, at most
 template <int GU, int DN, int INTER>
 struct ExpertsCfg {
   static constexpr int kWarps = 24, kTasks = 10, kInter = INTER;
@@ -280,20 +271,24 @@ struct ExpertsCfg {
   static constexpr int kSlot = kGuBytes > kDnBytes ? kGuBytes : kDnBytes;
   static constexpr int kDnTilesPerItem = H / kDnRows;
   static constexpr int kTableBytes = GuFmt<GU>::kTable;
+  // block terms of the tasks in flight; before the first task the selection's scratch memory
+  static constexpr size_t partials_of(int stages) {
+    const size_t terms = size_t(stages) * kTasks * kTT * 32 * 4, scratch = (sizeof(SelectScratch) + 15) & ~size_t(15);
+    return terms > scratch ? terms : scratch;
+  }
   static constexpr size_t smem_of(int stages) {
-    return size_t(kTableBytes) + size_t(stages) * (kSlot + kTasks * kTT * 32 * 4) + 128;
+    return size_t(kTableBytes) + size_t(stages) * kSlot + partials_of(stages) + 128;
   }
   // 24 warps work on 2.4 tiles at a time, so of three slots little more than a half is in flight from memory: four where
   // they fit (the formats without a table)
   static constexpr int kStages = smem_of(4) + kStaticSmem <= 232448 ? 4 : 3;
-  static constexpr int kPartialFloats = kStages * kTasks * kTT * 32;
+  static constexpr int kPartialFloats = int(partials_of(kStages) / 4);
   static constexpr size_t kSmem = smem_of(kStages);
   static_assert(DN == FB_FMT_IQ4_NL || DN == FB_FMT_Q2_0 || (DN == FB_FMT_IQ3_S && GU == FB_FMT_IQ3_S && INTER == 512),
                 "IQ3_S down shares the gate/up codebook and needs whole blocks per half row");
   static_assert(kTableBytes % 16 == 0 && kSlot % 16 == 0 && kGuPart % 16 == 0 && kDnTile % 16 == 0 && kGuAct % 16 == 0 &&
                     kDnAct % 16 == 0 && H % kDnRows == 0 && kDnRows % 32 == 0 && 2 * (kDnRows / 32) <= kTasks,
                 "tile shapes, bulk-copy sizes");
-  static_assert(sizeof(SelectScratch) <= kSlot * kStages, "the selection borrows the ring");
   static_assert(kSmem + kStaticSmem <= 232448, "dynamic plus static shared memory of a block");
 };
 // kPhaseSelect: the CTA builds the work list itself from the router logits (SelectArgs) instead of
@@ -301,23 +296,37 @@ struct ExpertsCfg {
 enum { kPhaseGateUp = 1, kPhaseDown = 2, kPhaseSelect = 4 };
 
 // ------------------------------------------------------------------------------ tables of the gate/up formats
+// The packed codebooks once more in global memory: a warp reads 32 different entries, which constant memory would deliver
+// one by one.
+static __device__ uint16_t g_iq3s_grid_packed[512] = {FB_IQ3S_GRID_PACKED};
+static __device__ uint16_t g_iq3xxs_grid_packed[256] = {FB_IQ3XXS_GRID_PACKED};
+static __device__ uint16_t g_iq2s_grid_packed[1024] = {FB_IQ2S_GRID_PACKED};
 // IQ3_S: the half codebook, replicated per lane. IQ2_S: 1024 entries of eight magnitudes, eight copies (entry i of
 // copy c at byte 64 i + 8 c, a lane reads copy lane % 8: two lanes of a half warp share two bank groups, 3 passes per
 // look-up of eight weights against 6 with one copy). IQ3_XXS: 256 entries of four magnitudes, one copy per lane.
+// A warp expands 32 entries, one per lane, and its lanes then write consecutive 16-byte pieces of the copies (no bank
+// conflicts), the values coming through shuffles. (With a constant-memory read and an expansion per 16 bytes written the
+// fill took 1.0 us for IQ3_S and up to 3.0 for IQ2_S and stood between the route kernel's end and the selection on the
+// multiprocessors that the route kernel left last: now 0.8 and 1.3.)
 template <int FMT>
 __device__ __forceinline__ void experts_table_fill(uint32_t* grid, uint32_t* signtab) {
-  if constexpr (FMT == FB_FMT_IQ3_S) {
-    iq3s_half_tables_fill(grid, signtab);
-  } else if constexpr (FMT == FB_FMT_IQ2_S || FMT == FB_FMT_IQ3_XXS) {
-    if constexpr (FMT == FB_FMT_IQ2_S) {
-      for (int i = threadIdx.x; i < 1024 * 4; i += blockDim.x) {  // 16 bytes = two copies of an entry
-        const uint2 w = iq2s_grid_entry(i >> 2);
-        reinterpret_cast<uint4*>(grid)[i] = make_uint4(w.x, w.y, w.x, w.y);
-      }
-    } else {
-      for (int i = threadIdx.x; i < 256 * 8; i += blockDim.x) {
-        const uint32_t w = iq3xxs_grid_entry(i >> 3);
-        reinterpret_cast<uint4*>(grid)[i] = make_uint4(w, w, w, w);
+  if constexpr (FMT == FB_FMT_IQ3_S || FMT == FB_FMT_IQ2_S || FMT == FB_FMT_IQ3_XXS) {
+    constexpr int kEntries = FMT == FB_FMT_IQ3_S ? 512 : FMT == FB_FMT_IQ2_S ? 1024 : 256;
+    constexpr int kPieces = FMT == FB_FMT_IQ2_S ? 4 : 8;  // 16-byte pieces of an entry's copies
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int e0 = 32 * (threadIdx.x >> 5); e0 < kEntries; e0 += int(blockDim.x)) {
+      uint2 w = make_uint2(0u, 0u);
+      if constexpr (FMT == FB_FMT_IQ3_S) w.x = (iq3s_expand(g_iq3s_grid_packed[e0 + lane]) >> 1) & 0x07070707u;
+      else if constexpr (FMT == FB_FMT_IQ2_S) w = iq2s_expand(g_iq2s_grid_packed[e0 + lane]);
+      else w.x = iq3xxs_expand(g_iq3xxs_grid_packed[e0 + lane]);
+      uint4* out = reinterpret_cast<uint4*>(grid) + size_t(e0) * kPieces + lane;
+#pragma unroll
+      for (int k = 0; k < kPieces; ++k) {
+        const int src = (32 * k + lane) / kPieces;
+        const uint32_t x = __shfl_sync(0xffffffffu, w.x, src);
+        const uint32_t y = FMT == FB_FMT_IQ2_S ? __shfl_sync(0xffffffffu, w.y, src) : x;
+        out[32 * k] = make_uint4(x, y, x, y);
       }
     }
     sign_table_fill(signtab);
@@ -583,29 +592,20 @@ __device__ __forceinline__ void q2_0_task_terms(const uint8_t* wp, const uint8_t
 // bits, of combine_kernel). A launch of its own behind this kernel cost a layer of one token 4 us.
 template <int ROWS>
 __device__ __forceinline__ void combine_tile(const fb_moe_decode_workspace& ws, const SelectArgs& sel, const WorkCache& wc,
-                                             int pair0, int ntp, int r0, int lane, int* rows) {
+                                             int pair0, int ntp, int r0, int lane) {
   int mine = 0;
   if (lane < ntp) {  // release and acquire ride on the atomic; the warp's stores are ordered before it by the __syncwarp
     int* counter = ws.sched + kSchedParts + wc.pair_token[pair0 + lane] * kMaxDnTiles + r0 / ROWS;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(mine) : "l"(counter) : "memory");
   }
-  const int n_pairs = wc.pair_begin[wc.n_items];
   for (int i = 0; i < ntp; ++i) {
     const int before = __shfl_sync(0xffffffffu, mine, i);
     if (before != kTopK - 1) continue;
+    __syncwarp();  // (the shuffle orders no memory: the other lanes read the partial rows behind their lane's acquire by this)
     const int t = wc.pair_token[pair0 + i];
-    int n = 0;
-    for (int b = 0; b < n_pairs; b += 32) {  // the token's pairs in pair order = slot order
-      const bool in = b + lane < n_pairs && wc.pair_token[b + lane] == t;
-      const uint32_t m = __ballot_sync(0xffffffffu, in);
-      if (in) rows[n + __popc(m & ((1u << lane) - 1u))] = b + lane;
-      n += __popc(m);
-    }
-    __syncwarp();
     int row[kTopK];
 #pragma unroll
-    for (int k = 0; k < kTopK; ++k) row[k] = rows[k];
-    __syncwarp();
+    for (int k = 0; k < kTopK; ++k) row[k] = wc.token_row[t][k];
     for (int c = 4 * lane; c < ROWS; c += 128) {
       float4 v[kTopK];
 #pragma unroll
@@ -647,7 +647,6 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   __shared__ StageMeta s_meta[S];
   __shared__ int s_misc[3 + S];  // [1..2] task tickets (even / odd blocks), [3..] finished tasks per slot
   __shared__ int s_end;
-  __shared__ int s_rows[C::kWarps][kTopK];
   __shared__ WorkCache s_work;
   RingN<S> ring{bars, bars + S, s_meta, &s_end};
 
@@ -665,7 +664,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   int n_items;
   if (phases & kPhaseSelect) {
     select_block([&](int t, int e) { return __ldcg(sel.logits + size_t(t) * sel.stride + e); }, sel.slot_of, sel.tokens, ws,
-                 nullptr, sel.remote_ok != 0, blockIdx.x == 0, false, s_work, *reinterpret_cast<SelectScratch*>(stage0));
+                 nullptr, sel.remote_ok != 0, blockIdx.x == 0, false, s_work, *reinterpret_cast<SelectScratch*>(partials));
     n_items = s_work.n_items;
   } else {
     n_items = min(max(ws.work->n_items, 0), kMaxPairs);
@@ -684,7 +683,6 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       __syncwarp();
     }
     if (lane != 0) return;
-    fence_proxy_async();  // the selection used the ring's memory through ordinary accesses
     int* counter = ws.sched + ((phases & kPhaseGateUp) ? kSchedGateUp : kSchedDown);
     const int n_tiles = n_gu + n_dn;
     int i = 0;
@@ -711,14 +709,15 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     // few values with the idle lanes of this warp here cost a sixteen-token layer 11 us of 84): an entry is made up before
     // the wait, and behind it come the copies first, then the entry's description, then the arrival that publishes both.
     int s = 0;
-    // a block's first two tiles need no ticket; the counter hands out the tiles behind those
+    // a block's first two tiles need no ticket; the counter hands out the tiles behind those (a ticket's value is not touched
+    // before its tile's turn)
     const int first_ticket = 2 * int(gridDim.x);
-    int next = int(blockIdx.x), next2 = int(blockIdx.x + gridDim.x);
+    int next = int(blockIdx.x) - first_ticket, next2 = int(blockIdx.x + gridDim.x) - first_ticket;
     while (true) {
-      const int tile = next;
+      const int tile = first_ticket + next;
       if (tile >= n_tiles) break;
       next = next2;
-      next2 = first_ticket + atomicAdd(counter, 1);
+      next2 = atomicAdd(counter, 1);
       const bool down = tile >= n_gu;
       const int tl = down ? tile - n_gu : tile;
       const int pos = down ? tl / C::kDnTilesPerItem : tl / gu_tpi;
@@ -896,7 +895,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         s_misc[3 + s] = 0;
         mbar_arrive(&ring.empty[s]);
       }
-      if (sel.y_out) combine_tile<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane, s_rows[warp]);
+      if (sel.y_out) combine_tile<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane);
     }
   }
 }

@@ -10,8 +10,7 @@ static __constant__ uint16_t c_iq2s_grid_packed[1024] = {FB_IQ2S_GRID_PACKED};
 
 constexpr int kGenericGridWords = 2048;  // shared-memory words the largest expanded codebook takes (IQ2_S: 1024 x 8 bytes)
 
-__device__ __forceinline__ uint32_t iq3xxs_grid_entry(int i) {
-  const uint32_t p = c_iq3xxs_grid_packed[i];
+__device__ __forceinline__ uint32_t iq3xxs_expand(uint32_t p) {
   uint32_t w = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -21,8 +20,7 @@ __device__ __forceinline__ uint32_t iq3xxs_grid_entry(int i) {
   return w;
 }
 
-__device__ __forceinline__ uint2 iq2s_grid_entry(int i) {
-  const uint32_t p = c_iq2s_grid_packed[i];
+__device__ __forceinline__ uint2 iq2s_expand(uint32_t p) {
   uint32_t w[2] = {0, 0};
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -37,9 +35,9 @@ __device__ __forceinline__ uint2 iq2s_grid_entry(int i) {
 template <int FMT>
 __device__ __forceinline__ void generic_grid_fill(uint32_t* grid) {
   if constexpr (FMT == FB_FMT_IQ3_XXS) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) grid[i] = iq3xxs_grid_entry(i);
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) grid[i] = iq3xxs_expand(c_iq3xxs_grid_packed[i]);
   } else if constexpr (FMT == FB_FMT_IQ2_S) {
-    for (int i = threadIdx.x; i < 1024; i += blockDim.x) reinterpret_cast<uint2*>(grid)[i] = iq2s_grid_entry(i);
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x) reinterpret_cast<uint2*>(grid)[i] = iq2s_expand(c_iq2s_grid_packed[i]);
   }
 }
 
