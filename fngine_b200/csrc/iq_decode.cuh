@@ -235,17 +235,10 @@ __device__ __forceinline__ float q8k_block_warp(const float (&v)[8], int (&q)[8]
       idx = 8 * lane + i;
     }
   }
-  if (amax == 0.0f) idx = 0x7fffffff;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (oa > amax || (oa == amax && oi < idx)) {
-      amax = oa;
-      idx = oi;
-    }
-  }
-  if (amax == 0.0f) {
+  // (magnitudes, never NaN here, order like their bits; the first of the largest is the one with the smallest index)
+  const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  idx = int(__reduce_min_sync(0xffffffffu, amax == most ? uint32_t(idx) : 0x7fffffffu));
+  if (most == 0.0f) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] = 0;
     pair_sum = 0;

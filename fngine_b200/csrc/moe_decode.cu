@@ -638,6 +638,12 @@ __global__ void __launch_bounds__(512) select_kernel(const float* logits, int lo
                slot_of, T, ws, counts, false, true, true, s_work, s_scratch);
 }
 
+// Up to here values carry their own arrival flags (direct_store). Eight layers, us, by counters and so: IQ3_S 512 at one
+// token 168 and 154, two 218 and 198, three 251 and 249; IQ4_NL 512 at three 246 and 231; IQ3_S + IQ4_NL 640 at one 183 and
+// 176, two 240 and 262, IQ2_S + IQ4_NL 640 at two 247 and 263: rows of 640 take the quantizing warp longer than a tile.
+__host__ __device__ constexpr int direct_tokens(int inter) { return inter == 512 ? 3 : 1; }
+constexpr uint32_t kNotYet = 0xFFFFFFFFu;
+
 // What route_kernel needs for an expert-parallel step with peer-memory exchange (n_ranks == 0: none).
 struct EpRouteArgs {
   fb_ep_peers peers;
@@ -647,6 +653,7 @@ struct EpRouteArgs {
   uint32_t step;
   uint32_t spin_limit;  // polls per awaited line
   int act;              // activation format the layer's gate/up weights pair with (set for every launch)
+  int clear_h, clear_partial;  // floats at ws.h and ws.partial to set to kNotYet (multiples of four)
 };
 
 // Router projection and activation quantization in one launch (the head of the fused layer call; the
@@ -953,6 +960,10 @@ __global__ void __launch_bounds__(kRouteThreads, 1) route_kernel(const __nv_bflo
         if (i < kMaxTok * kMaxDnTiles) ws.sched[kSchedParts + i] = 0;
       }
     }
+    for (int i = int(blockIdx.x) * 64 + tid - kRouteWarps * 32; i < (ep.clear_h + ep.clear_partial) / 4; i += kRouteBlocks * 64) {
+      float* dst = i < ep.clear_h / 4 ? ws.h + 4 * size_t(i) : ws.partial + 4 * size_t(i - ep.clear_h / 4);
+      *reinterpret_cast<uint4*>(dst) = make_uint4(kNotYet, kNotYet, kNotYet, kNotYet);
+    }
     __syncwarp();
     cluster_wait();
   }
@@ -1027,6 +1038,24 @@ static_assert(kTT == 2 && sizeof(StageMeta) == 48, "three vector stores");
 // flight before the first block is quantized (the finishing warp waits on this chain: Q8_0 rows taken block by block, twenty
 // round trips at 640, cost a layer of one token 8 us). `out` in global or shared memory, 16-byte aligned.
 template <int I>
+__device__ __forceinline__ void quantize_h_values(const float (&v)[(I + 255) / 256][8], int down_act, uint8_t* out) {
+  constexpr int kPasses = (I + 255) / 256;
+  const int lane = threadIdx.x & 31;
+  if (I % 256 == 0 && down_act == FB_ACT_Q8_K) {
+#pragma unroll
+    for (int p = 0; p < kPasses; ++p) {
+      int q[8], ps;
+      const float d = q8k_block_warp(v[p], q, ps);
+      store_q8k_block_planar(out, I, p, q, ps, d);
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < kPasses; ++p)
+      q8_0_eight_blocks_warp(v[p], 256 * p + 8 * lane < I, out + 256 * p, reinterpret_cast<float*>(out + I) + 8 * p);
+  }
+}
+
+template <int I>
 __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uint8_t* out) {
   constexpr int kPasses = (I + 255) / 256;
   const int lane = threadIdx.x & 31;
@@ -1042,19 +1071,29 @@ __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uin
     v[p][0] = a.x; v[p][1] = a.y; v[p][2] = a.z; v[p][3] = a.w;
     v[p][4] = c.x; v[p][5] = c.y; v[p][6] = c.z; v[p][7] = c.w;
   }
-  if (I % 256 == 0 && down_act == FB_ACT_Q8_K) {
-#pragma unroll
-    for (int p = 0; p < kPasses; ++p) {
-      int q[8], ps;
-      const float d = q8k_block_warp(v[p], q, ps);
-      store_q8k_block_planar(out, I, p, q, ps, d);
-    }
-  } else {
-#pragma unroll
-    for (int p = 0; p < kPasses; ++p)
-      q8_0_eight_blocks_warp(v[p], 256 * p + 8 * lane < I, out + 256 * p, reinterpret_cast<float*>(out + I) + 8 * p);
-  }
+  quantize_h_values<I>(v, down_act, out);
 }
+
+// Few tokens (direct_tokens): values that are their own arrival flags. The route kernel fills the rows with kNotYet, a NaN
+// that no arithmetic produces; a value is stored once, by one relaxed store, and a reader polls the values it needs (a
+// bounded number of times). Nothing else is read on the strength of a value, so no fence and no counter stand between a
+// store and its reader: release, counter, a last contributor that re-quantizes a row, its flag, the row's copy into shared
+// memory were four dependent round trips.
+__device__ __forceinline__ void direct_store(float* p, float v) {
+  const uint32_t b = __float_as_uint(v);
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(b == kNotYet ? 0x7FFFFFFFu : b) : "memory");
+}
+// Four values; `all` goes false where one is not there yet.
+__device__ __forceinline__ float4 direct_load4(const float* p, bool& all) {
+  uint4 u;
+  asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+               : "l"(p)
+               : "memory");
+  all = all && u.x != kNotYet && u.y != kNotYet && u.z != kNotYet && u.w != kNotYet;
+  return make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w));
+}
+constexpr uint32_t kDirectPolls = 1u << 20;  // about a second
 
 // Counts one finished contribution to an item's h; the last one re-quantizes that item's h for the
 // down projection and then sets the item's flag, ws.item_done[kMaxPairs + item], to `ready` (1 in a fused gate/up + down
@@ -1365,17 +1404,21 @@ template <int GU, int DN, int INTER>
 int32_t launch_experts_as(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases,
                           void* stream, const char* what, const SelectArgs* sel) {
   using C = ExpertsCfg<GU, DN, INTER>;
-  static PerDeviceOnce once;
-  const cudaError_t attr = per_device_once(once, [] { return opt_in_smem(experts_kernel<GU, DN, INTER>, C::kSmem); });
-  if (attr != cudaSuccess) {
-    set_error("%s: shared-memory opt-in: %s", what, cudaGetErrorString(attr));
-    return int32_t(attr);
-  }
-  const cudaError_t e = launch_pdl(experts_kernel<GU, DN, INTER>, dim3(sm_count()), dim3((C::kWarps + 1) * 32), C::kSmem,
-                                   as_stream(stream), *layout, *ws, sel ? (phases | kPhaseSelect) : phases,
-                                   sel ? *sel : SelectArgs{});
-  if (e != cudaSuccess) return check_launch(what);
-  return 0;
+  auto launch = [&](auto kernel, PerDeviceOnce& once, int warps) -> int32_t {
+    const cudaError_t attr = per_device_once(once, [&] { return opt_in_smem(kernel, C::kSmem); });
+    if (attr != cudaSuccess) {
+      set_error("%s: shared-memory opt-in: %s", what, cudaGetErrorString(attr));
+      return int32_t(attr);
+    }
+    const cudaError_t e = launch_pdl(kernel, dim3(sm_count()), dim3(warps * 32), C::kSmem, as_stream(stream), *layout, *ws,
+                                     sel ? (phases | kPhaseSelect) : phases, sel ? *sel : SelectArgs{});
+    return e != cudaSuccess ? check_launch(what) : 0;
+  };
+  static PerDeviceOnce once[2];
+  // the fused call's few tokens (the route kernel has filled h and the partial rows: layer_decode_impl)
+  if (sel && sel->tokens <= direct_tokens(INTER) && phases == (kPhaseGateUp | kPhaseDown))
+    return launch(experts_kernel<GU, DN, INTER, true>, once[1], C::kWarps + 2);
+  return launch(experts_kernel<GU, DN, INTER, false>, once[0], C::kWarps + 1);
 }
 // Every gate/up format has its kernel with an IQ4_NL or Q2_0 down projection at both intermediate sizes; IQ3_S also with
 // its own.
@@ -1575,6 +1618,11 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
   EpRouteArgs era{};
   if (ep) era = *ep;
   era.act = layout_ok(layout) ? act_of(layout->gate_up_format) : FB_ACT_Q8_K;
+  const bool own_combine = with_combine && !slot_of && layout_ok(layout) && one_launch(layout);
+  if (layout_ok(layout) && tokens <= direct_tokens(layout->inter) && one_launch(layout)) {
+    era.clear_h = tokens * kTopK * layout->inter;
+    era.clear_partial = own_combine ? tokens * kTopK * H : 0;
+  }
   // Two launches: route (router projection + activation quantization) and the expert kernel (every CTA runs the
   // selection on the stored logits, then gate/up and down tiles in one persistent launch, whose warps also combine a
   // token's rows when its last one is there). IQ3_S down behind another gate/up format takes a gate/up and a down launch,
@@ -1614,7 +1662,6 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
                   : x_dtype == FB_DT_BF16 ? launch(route_kernel<true, false>)
                                           : launch(route_kernel<false, false>);
   if (e != cudaSuccess) return check_launch("layer_decode: route");
-  const bool own_combine = with_combine && !slot_of && one_launch(layout);
   const SelectArgs sel{logits_scratch, int(FB_ROUTER_ROWS), slot_of, tokens, remote_ok ? 1 : 0, own_combine ? y_out : nullptr};
   const int32_t st = launch_experts(layout, ws, stream, &sel);  // selection + both projections of every routed expert
   if (st || !with_combine || own_combine) return st;

@@ -171,7 +171,7 @@ __device__ __forceinline__ uint32_t* sign_table_at(uint8_t* area) {
 // ------------------------------------------------------------------------------ multi-stage ring
 template <int S>
 struct RingN {
-  uint64_t* full;   // [S] count 1 + tx bytes
+  uint64_t* full;   // [S] count 1 (DIRECT: 2) + tx bytes
   uint64_t* empty;  // [S]
   volatile StageMeta* meta;  // [S]
   // number of entries the producer staged in all; INT_MAX while it is still staging; 0 after a time-out
@@ -186,9 +186,9 @@ __device__ __forceinline__ bool mbar_wait_hint(uint64_t* bar, uint32_t parity) {
 }
 
 template <int S>
-__device__ __forceinline__ void ringn_init(const RingN<S>& r) {
+__device__ __forceinline__ void ringn_init(const RingN<S>& r, int arrivals) {
   for (int s = 0; s < S; ++s) {
-    mbar_init(&r.full[s], 1);
+    mbar_init(&r.full[s], arrivals);
     mbar_init(&r.empty[s], 1);  // one arrival frees a slot: the warp that finishes the entry's last task
     r.meta[s].tile = -1;
     r.meta[s].seq = -1;
@@ -632,8 +632,70 @@ __device__ __forceinline__ void combine_tile(const fb_moe_decode_workspace& ws, 
   }
 }
 
-template <int GU, int DN, int INTER>
-__global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + 1) * 32, 1)
+// The same, few tokens: the warp that finished the tile of the token's last pair polls the other pairs' rows (false: a wait
+// has run out). Every warp that polls holds a finished tile, of which a CTA has a handful, so the others go on working.
+template <int ROWS>
+__device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspace& ws, const SelectArgs& sel,
+                                                    const WorkCache& wc, int pair0, int ntp, int r0, int lane,
+                                                    volatile int* end_seq) {
+  for (int i = 0; i < ntp; ++i) {
+    const int t = wc.pair_token[pair0 + i];
+    if (wc.token_row[t][kTopK - 1] != pair0 + i) continue;
+    int row[kTopK];
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) row[k] = wc.token_row[t][k];
+#pragma unroll 1
+    for (int c0 = 0; c0 < ROWS; c0 += 128) {
+      const int c = c0 + 4 * lane;
+      float4 y;
+      uint32_t tries = 0;
+      while (true) {
+        bool all = true;
+        y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (c < ROWS) {
+          float4 v[kTopK];
+#pragma unroll
+          for (int k = 0; k < kTopK; ++k) v[k] = direct_load4(ws.partial + size_t(row[k]) * H + r0 + c, all);
+#pragma unroll
+          for (int k = 0; k < kTopK; ++k) {
+            y.x += v[k].x;
+            y.y += v[k].y;
+            y.z += v[k].z;
+            y.w += v[k].w;
+          }
+        }
+        if (__all_sync(0xffffffffu, all)) break;
+        if (++tries > kDirectPolls || __shfl_sync(0xffffffffu, *end_seq, 0) == 0) {
+          if (lane == 0) {
+            *end_seq = 0;
+            atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+          }
+          return false;
+        }
+        __nanosleep(20);
+      }
+      if (c >= ROWS) continue;
+      float* out = sel.y_out + size_t(t) * H + r0 + c;  // (any 4-byte alignment)
+      if ((reinterpret_cast<uintptr_t>(sel.y_out) & 15) == 0) {
+        *reinterpret_cast<float4*>(out) = y;
+      } else {
+        out[0] = y.x;
+        out[1] = y.y;
+        out[2] = y.z;
+        out[3] = y.w;
+      }
+    }
+  }
+  return true;
+}
+
+// DIRECT (all phases, up to direct_tokens): h and the partial rows are their own arrival flags (direct_store), and one
+// more warp quantizes the h rows of this CTA's down entries as they arrive (one token: from the last gate/up tile to the
+// down tasks 4.2 -> 3 us, from the last down tile to y 2.5 -> 1.4). (As a run-time switch it cost sixteen tokens 2 to 3 %;
+// with more tokens the down tiles of the first experts cover the hand-off of the last ones, and every tile's own
+// quantization costs more than it saves.)
+template <int GU, int DN, int INTER, bool DIRECT>
+__global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + (DIRECT ? 2 : 1)) * 32, 1)
 experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, SelectArgs sel) {
   using C = ExpertsCfg<GU, DN, INTER>;
   constexpr int S = C::kStages;
@@ -654,7 +716,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   // (a down-only launch of another format than IQ3_S looks nothing up)
   if (DN == FB_FMT_IQ3_S || (phases & kPhaseGateUp)) experts_table_fill<GU>(grid, signtab);
   if (tid == 0) {
-    ringn_init(ring);
+    ringn_init(ring, DIRECT ? 2 : 1);
     for (int i = 1; i < 3 + S; ++i) s_misc[i] = 0;
   }
   __syncthreads();
@@ -751,6 +813,10 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 #pragma unroll
           for (int t = 0; t < kTT; ++t)
             if (t < ntp) bulk_g2s(st + 2 * C::kGuPart + t * C::kGuAct, act[t], C::kGuAct, full);
+          if constexpr (DIRECT) mbar_arrive(full);  // (in the place of the warp that quantizes h rows)
+        } else if constexpr (DIRECT) {
+          mbar_expect_tx_only(full, uint32_t(C::kDnTile));
+          bulk_g2s(st, w0, C::kDnTile, full);
         } else {
           mbar_expect_tx_only(full, uint32_t(C::kDnTile + ntp * C::kDnAct));
           bulk_g2s(st, w0, C::kDnTile, full);
@@ -775,7 +841,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
           for (int t = 0; t < kTT; ++t)
             if (t < ntp) bulk_g2s(st + C::kDnTile + t * C::kDnAct, act[t], C::kDnAct, full);
         }
-        m->store(i, down ? 1 : 0, pair0, ntp, row0, item, pb, ntok, wgt);
+        m->store(i, !down ? 0 : DIRECT && sub == 0 ? 2 : 1, pair0, ntp, row0, item, pb, ntok, wgt);
         mbar_arrive(full);
         if (failed) {  // nobody will use the entry: see its copies land (bounded), then leave
           mbar_wait_hint(full, (i / S) & 1);
@@ -798,6 +864,73 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       for (int k = 0; k < kMaxPairs; ++k) ws.item_done[kMaxPairs + k] = 0;
     }
     return;
+  }
+
+  if (DIRECT && warp == C::kWarps + 1) {
+    // ---------------- the h rows of every down entry, quantized into its slot as they arrive
+    for (int seq = 0;; ++seq) {
+      const int s = seq % S;
+      int e_seq, kind, pair0, ntp;
+      uint32_t tries = 0;
+      while (true) {
+        asm volatile("ld.volatile.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(e_seq), "=r"(kind), "=r"(pair0), "=r"(ntp)
+                     : "r"(smem_u32(const_cast<StageMeta*>(&s_meta[s])))
+                     : "memory");
+        e_seq = __shfl_sync(0xffffffffu, e_seq, 0);
+        kind = __shfl_sync(0xffffffffu, kind, 0);
+        pair0 = __shfl_sync(0xffffffffu, pair0, 0);
+        ntp = __shfl_sync(0xffffffffu, ntp, 0);
+        if (e_seq >= seq) break;
+        if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) <= seq) return;
+        if (++tries > kDirectPolls) {
+          if (lane == 0) {
+            *ring.end_seq = 0;
+            atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+          }
+          return;
+        }
+        __nanosleep(100);
+      }
+      if (e_seq != seq || kind == 0) continue;  // gate/up (its slot may have gone to a later entry already)
+      uint8_t* out = stage0 + s * C::kSlot + C::kDnTile;
+      for (int t = 0; t < ntp; ++t, out += C::kDnAct) {
+        constexpr int kPasses = (INTER + 255) / 256;
+        const float* h = ws.h + size_t(pair0 + t) * INTER;
+        float v[kPasses][8];
+        tries = 0;
+        while (true) {
+          bool all = true;
+#pragma unroll
+          for (int p = 0; p < kPasses; ++p) {
+            const int e = 256 * p + 8 * lane;
+            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = a;
+            if (e < INTER) {
+              a = direct_load4(h + e, all);
+              c = direct_load4(h + e + 4, all);
+            }
+            v[p][0] = a.x; v[p][1] = a.y; v[p][2] = a.z; v[p][3] = a.w;
+            v[p][4] = c.x; v[p][5] = c.y; v[p][6] = c.z; v[p][7] = c.w;
+          }
+          if (__all_sync(0xffffffffu, all)) break;
+          if (++tries > kDirectPolls || __shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) {
+            if (lane == 0) {
+              *ring.end_seq = 0;
+              atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+            }
+            return;
+          }
+          __nanosleep(20);
+        }
+        quantize_h_values<INTER>(v, down_act, out);
+      }
+      fence_proxy_async();  // (a later entry's bulk copies will write here)
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ring.full[s]);
+      if (kind == 2)  // an item's first tile: its rows in the workspace too, where the other form of this kernel leaves them
+        for (int p = pair0; p < pair0 + ntp; ++p)
+          quantize_h_row<INTER>(ws.h + size_t(p) * INTER, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
+    }
   }
 
   // ---------------- consumers
@@ -870,24 +1003,10 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 #pragma unroll
         for (int b = 0; b < C::kTasks; ++b) v += pt[(b * kTT + t) * 32 + lane];
         const float u = __shfl_down_sync(0xffffffffu, v, 16);
-        if (lane < 16) ws.h[size_t(pair0 + t) * INTER + r0 + lane] = silu_mul(v, u);
-      }
-      __syncwarp();
-      if (lane == 0) {
-        s_misc[3 + s] = 0;
-        mbar_arrive(&ring.empty[s]);
-      }
-      item_contribution_done<INTER>(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act,
-                                    phases & kPhaseDown ? 1 : 0, lane);
-    } else {
-      const float w0 = ring.meta[s].wgt[0], w1 = ring.meta[s].wgt[1];
-#pragma unroll
-      for (int g = 0; g < C::kDnRows / 32; ++g) {
-        const float v0 = pt[((2 * g) * kTT + 0) * 32 + lane] + pt[((2 * g + 1) * kTT + 0) * 32 + lane];
-        ws.partial[size_t(pair0) * H + r0 + 32 * g + lane] = w0 * v0;
-        if (ntp == 2) {
-          const float v1 = pt[((2 * g) * kTT + 1) * 32 + lane] + pt[((2 * g + 1) * kTT + 1) * 32 + lane];
-          ws.partial[size_t(pair0 + 1) * H + r0 + 32 * g + lane] = w1 * v1;
+        float* out = ws.h + size_t(pair0 + t) * INTER + r0 + lane;
+        if (lane < 16) {
+          if constexpr (DIRECT) direct_store(out, silu_mul(v, u));
+          else *out = silu_mul(v, u);
         }
       }
       __syncwarp();
@@ -895,7 +1014,32 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         s_misc[3 + s] = 0;
         mbar_arrive(&ring.empty[s]);
       }
-      if (sel.y_out) combine_tile<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane);
+      if constexpr (!DIRECT)
+        item_contribution_done<INTER>(ws, item, ipb, itok, gu_tpi * ((itok + kTT - 1) / kTT), down_act,
+                                      phases & kPhaseDown ? 1 : 0, lane);
+    } else {
+      const float w0 = ring.meta[s].wgt[0], w1 = ring.meta[s].wgt[1];
+#pragma unroll
+      for (int g = 0; g < C::kDnRows / 32; ++g) {
+        const float v0 = pt[((2 * g) * kTT + 0) * 32 + lane] + pt[((2 * g + 1) * kTT + 0) * 32 + lane];
+        float* out = ws.partial + size_t(pair0) * H + r0 + 32 * g + lane;
+        if constexpr (DIRECT) direct_store(out, w0 * v0);
+        else *out = w0 * v0;
+        if (ntp == 2) {
+          const float v1 = pt[((2 * g) * kTT + 1) * 32 + lane] + pt[((2 * g + 1) * kTT + 1) * 32 + lane];
+          if constexpr (DIRECT) direct_store(out + H, w1 * v1);
+          else out[H] = w1 * v1;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        s_misc[3 + s] = 0;
+        mbar_arrive(&ring.empty[s]);
+      }
+      if (sel.y_out) {
+        if constexpr (!DIRECT) combine_tile<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane);
+        else if (!combine_tile_direct<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane, ring.end_seq)) break;
+      }
     }
   }
 }
