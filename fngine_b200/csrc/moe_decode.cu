@@ -337,6 +337,7 @@ struct WorkCache {
   int pair_token[kMaxPairs];
   float pair_weight[kMaxPairs];
   int token_row[kMaxTok][kTopK];  // a token's pairs in slot order (only by the CTA's own selection)
+  int last_pair[kMaxTok];         // the one of them whose item is visited last (the same)
   int n_items;
 };
 // Called by the 32 lanes of the producer warp (the only reader) after the wait on the preceding kernel;
@@ -364,6 +365,7 @@ struct SelectScratch {
     struct {  // behind those
       int begin[kExperts];         // physical slot -> first pair of its item
       int slot[kMaxTok][kTopK];    // physical slots of the winners, -1: not held here
+      int16_t rank[kExperts];      // physical slot -> its item's place in the visiting order
     };
   };
   float val[kMaxTok][kTopK];             // the winners' logits
@@ -457,6 +459,13 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
           rank += ((first_m >> j) & 1u) && (cj > cnt || (cj == cnt && ij < item)) ? 1 : 0;
         }
       }
+      {  // (the lanes of an item agree on its rank)
+        const int mine = hot ? rank : -1;
+        int most = -1;
+#pragma unroll
+        for (int k = 0; k < kTopK; ++k) most = max(most, __shfl_sync(0xffffffffu, mine, min(31, kTopK * (valid ? pt : 0) + k)));
+        if (valid && hot && mine == most) wc.last_pair[pt] = idx;
+      }
       if (hot) wc.pair_token[idx] = pt;
       if (first) {
         wc.slot[item] = slot;
@@ -538,6 +547,7 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
         wc.slot[item] = tid;
         wc.pair_begin[item] = pair_begin;
         wc.order[order_base + peer_rank] = item;
+        scratch.rank[tid] = int16_t(order_base + peer_rank);
       }
       if (tid == 0) {
         wc.pair_begin[n_items] = n_pairs;
@@ -565,7 +575,17 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
       }
       s_pair[pt][pk] = idx;
     }
-    if (slot2 >= 0) wc.token_row[t2][rank2] = pair_of(slot2, t2);
+    if (slot2 >= 0) {
+      const int pair = pair_of(slot2, t2), mine = scratch.rank[slot2];
+      bool last = true;
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k) {
+        const int other = scratch.slot[t2][k];
+        last = last && (other < 0 || scratch.rank[other] <= mine);
+      }
+      wc.token_row[t2][rank2] = pair;
+      if (last) wc.last_pair[t2] = pair;
+    }
   }
   __syncthreads();
   if (!publish || tid >= kExperts) return;  // (the device list is behind everything the streaming waits for)
@@ -639,9 +659,13 @@ __global__ void __launch_bounds__(512) select_kernel(const float* logits, int lo
 }
 
 // Up to here values carry their own arrival flags (direct_store). Eight layers, us, by counters and so: IQ3_S 512 at one
-// token 168 and 154, two 218 and 198, three 251 and 249; IQ4_NL 512 at three 246 and 231; IQ3_S + IQ4_NL 640 at one 183 and
-// 176, two 240 and 262, IQ2_S + IQ4_NL 640 at two 247 and 263: rows of 640 take the quantizing warp longer than a tile.
-__host__ __device__ constexpr int direct_tokens(int inter) { return inter == 512 ? 3 : 1; }
+// token 168 and 146, two 218 and 187, three 251 and 230, four 253 and 255, sixteen 630 and 662; IQ4_NL 512 (four ring slots:
+// the quantizing warps run further ahead) at one 161 and 144, four 254 and 233, eight 371 and 359, sixteen 612 and 597;
+// IQ3_S + IQ4_NL 640 at one 183 and 160, two 237 and 240, IQ4_XS + IQ4_NL 640 at two 244 and 244, four 340 and 365: rows of
+// 640 take the quantizing warps longer than a tile of 128 rows takes the others.
+__host__ __device__ constexpr int direct_tokens(int gate_up, int inter) {
+  return inter != 512 ? 1 : gate_up == FB_FMT_IQ4_NL ? kMaxTok : 3;
+}
 constexpr uint32_t kNotYet = 0xFFFFFFFFu;
 
 // What route_kernel needs for an expert-parallel step with peer-memory exchange (n_ranks == 0: none).
@@ -1037,24 +1061,17 @@ static_assert(kTT == 2 && sizeof(StageMeta) == 48, "three vector stores");
 // One row of h -> a planar activation row of the down projection, by the calling warp; all of the row's loads are in
 // flight before the first block is quantized (the finishing warp waits on this chain: Q8_0 rows taken block by block, twenty
 // round trips at 640, cost a layer of one token 8 us). `out` in global or shared memory, 16-byte aligned.
+// Piece p of a row: lane l holds elements 256 p + 8 l .. + 7 (none behind the row's end).
 template <int I>
-__device__ __forceinline__ void quantize_h_values(const float (&v)[(I + 255) / 256][8], int down_act, uint8_t* out) {
-  constexpr int kPasses = (I + 255) / 256;
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void quantize_h_piece(const float (&v)[8], int p, int down_act, uint8_t* out) {
   if (I % 256 == 0 && down_act == FB_ACT_Q8_K) {
-#pragma unroll
-    for (int p = 0; p < kPasses; ++p) {
-      int q[8], ps;
-      const float d = q8k_block_warp(v[p], q, ps);
-      store_q8k_block_planar(out, I, p, q, ps, d);
-    }
+    int q[8], ps;
+    const float d = q8k_block_warp(v, q, ps);
+    store_q8k_block_planar(out, I, p, q, ps, d);
   } else {
-#pragma unroll
-    for (int p = 0; p < kPasses; ++p)
-      q8_0_eight_blocks_warp(v[p], 256 * p + 8 * lane < I, out + 256 * p, reinterpret_cast<float*>(out + I) + 8 * p);
+    q8_0_eight_blocks_warp(v, 256 * p + 8 * int(threadIdx.x & 31) < I, out + 256 * p, reinterpret_cast<float*>(out + I) + 8 * p);
   }
 }
-
 template <int I>
 __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uint8_t* out) {
   constexpr int kPasses = (I + 255) / 256;
@@ -1071,10 +1088,11 @@ __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uin
     v[p][0] = a.x; v[p][1] = a.y; v[p][2] = a.z; v[p][3] = a.w;
     v[p][4] = c.x; v[p][5] = c.y; v[p][6] = c.z; v[p][7] = c.w;
   }
-  quantize_h_values<I>(v, down_act, out);
+#pragma unroll
+  for (int p = 0; p < kPasses; ++p) quantize_h_piece<I>(v[p], p, down_act, out);
 }
 
-// Few tokens (direct_tokens): values that are their own arrival flags. The route kernel fills the rows with kNotYet, a NaN
+// Up to direct_tokens: values that are their own arrival flags. The route kernel fills the rows with kNotYet, a NaN
 // that no arithmetic produces; a value is stored once, by one relaxed store, and a reader polls the values it needs (a
 // bounded number of times). Nothing else is read on the strength of a value, so no fence and no counter stand between a
 // store and its reader: release, counter, a last contributor that re-quantizes a row, its flag, the row's copy into shared
@@ -1093,7 +1111,21 @@ __device__ __forceinline__ float4 direct_load4(const float* p, bool& all) {
   all = all && u.x != kNotYet && u.y != kNotYet && u.z != kNotYet && u.w != kNotYet;
   return make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w));
 }
+// Eight values of a row from element `at` on (zeros behind the row's end): false where one is not there yet.
+__device__ __forceinline__ bool direct_load8(const float* row, int at, int n, float (&v)[8]) {
+  bool all = true;
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = a;
+  if (at < n) {
+    a = direct_load4(row + at, all);
+    c = direct_load4(row + at + 4, all);
+  }
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+  return all;
+}
 constexpr uint32_t kDirectPolls = 1u << 20;  // about a second
+// Warps that quantize the h rows of a CTA's down entries, each its piece of 256 values.
+constexpr int direct_warps(int inter) { return (inter + 255) / 256; }
 
 // Counts one finished contribution to an item's h; the last one re-quantizes that item's h for the
 // down projection and then sets the item's flag, ws.item_done[kMaxPairs + item], to `ready` (1 in a fused gate/up + down
@@ -1416,8 +1448,8 @@ int32_t launch_experts_as(const fb_moe_expert_layout* layout, const fb_moe_decod
   };
   static PerDeviceOnce once[2];
   // the fused call's few tokens (the route kernel has filled h and the partial rows: layer_decode_impl)
-  if (sel && sel->tokens <= direct_tokens(INTER) && phases == (kPhaseGateUp | kPhaseDown))
-    return launch(experts_kernel<GU, DN, INTER, true>, once[1], C::kWarps + 2);
+  if (sel && sel->tokens <= direct_tokens(GU, INTER) && phases == (kPhaseGateUp | kPhaseDown))
+    return launch(experts_kernel<GU, DN, INTER, true>, once[1], C::kWarps + 1 + direct_warps(INTER));
   return launch(experts_kernel<GU, DN, INTER, false>, once[0], C::kWarps + 1);
 }
 // Every gate/up format has its kernel with an IQ4_NL or Q2_0 down projection at both intermediate sizes; IQ3_S also with
@@ -1619,7 +1651,7 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
   if (ep) era = *ep;
   era.act = layout_ok(layout) ? act_of(layout->gate_up_format) : FB_ACT_Q8_K;
   const bool own_combine = with_combine && !slot_of && layout_ok(layout) && one_launch(layout);
-  if (layout_ok(layout) && tokens <= direct_tokens(layout->inter) && one_launch(layout)) {
+  if (layout_ok(layout) && tokens <= direct_tokens(layout->gate_up_format, layout->inter) && one_launch(layout)) {
     era.clear_h = tokens * kTopK * layout->inter;
     era.clear_partial = own_combine ? tokens * kTopK * H : 0;
   }

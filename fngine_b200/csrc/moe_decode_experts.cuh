@@ -171,7 +171,7 @@ __device__ __forceinline__ uint32_t* sign_table_at(uint8_t* area) {
 // ------------------------------------------------------------------------------ multi-stage ring
 template <int S>
 struct RingN {
-  uint64_t* full;   // [S] count 1 (DIRECT: 2) + tx bytes
+  uint64_t* full;   // [S] count 1 (DIRECT: and one for every quantizing warp) + tx bytes
   uint64_t* empty;  // [S]
   volatile StageMeta* meta;  // [S]
   // number of entries the producer staged in all; INT_MAX while it is still staging; 0 after a time-out
@@ -632,15 +632,16 @@ __device__ __forceinline__ void combine_tile(const fb_moe_decode_workspace& ws, 
   }
 }
 
-// The same, few tokens: the warp that finished the tile of the token's last pair polls the other pairs' rows (false: a wait
-// has run out). Every warp that polls holds a finished tile, of which a CTA has a handful, so the others go on working.
+// The same where rows are their own arrival flags: the warp that finished the tile of the token's pair that is visited last
+// polls the other pairs' rows (false: a wait has run out). What it waits for comes before its own tile in the order in which
+// tiles are drawn and tasks taken, so the earliest unfinished tile never waits for a polling warp.
 template <int ROWS>
 __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspace& ws, const SelectArgs& sel,
                                                     const WorkCache& wc, int pair0, int ntp, int r0, int lane,
                                                     volatile int* end_seq) {
   for (int i = 0; i < ntp; ++i) {
     const int t = wc.pair_token[pair0 + i];
-    if (wc.token_row[t][kTopK - 1] != pair0 + i) continue;
+    if (wc.last_pair[t] != pair0 + i) continue;
     int row[kTopK];
 #pragma unroll
     for (int k = 0; k < kTopK; ++k) row[k] = wc.token_row[t][k];
@@ -689,13 +690,13 @@ __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspac
   return true;
 }
 
-// DIRECT (all phases, up to direct_tokens): h and the partial rows are their own arrival flags (direct_store), and one
-// more warp quantizes the h rows of this CTA's down entries as they arrive (one token: from the last gate/up tile to the
-// down tasks 4.2 -> 3 us, from the last down tile to y 2.5 -> 1.4). (As a run-time switch it cost sixteen tokens 2 to 3 %;
-// with more tokens the down tiles of the first experts cover the hand-off of the last ones, and every tile's own
+// DIRECT (all phases, up to direct_tokens): h and the partial rows are their own arrival flags (direct_store), and two or
+// three more warps, each its 256 values, quantize the h rows of this CTA's down entries as they arrive. One token of IQ3_S:
+// by counters 168 us for eight layers, with one quantizing warp 154, now 146. (As a run-time switch it cost sixteen tokens 2
+// to 3 %; beyond direct_tokens the down tiles of the first experts cover the hand-off of the last ones, and every tile's own
 // quantization costs more than it saves.)
 template <int GU, int DN, int INTER, bool DIRECT>
-__global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + (DIRECT ? 2 : 1)) * 32, 1)
+__global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + 1 + (DIRECT ? direct_warps(INTER) : 0)) * 32, 1)
 experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, SelectArgs sel) {
   using C = ExpertsCfg<GU, DN, INTER>;
   constexpr int S = C::kStages;
@@ -716,7 +717,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   // (a down-only launch of another format than IQ3_S looks nothing up)
   if (DN == FB_FMT_IQ3_S || (phases & kPhaseGateUp)) experts_table_fill<GU>(grid, signtab);
   if (tid == 0) {
-    ringn_init(ring, DIRECT ? 2 : 1);
+    ringn_init(ring, DIRECT ? 1 + direct_warps(INTER) : 1);
     for (int i = 1; i < 3 + S; ++i) s_misc[i] = 0;
   }
   __syncthreads();
@@ -813,7 +814,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 #pragma unroll
           for (int t = 0; t < kTT; ++t)
             if (t < ntp) bulk_g2s(st + 2 * C::kGuPart + t * C::kGuAct, act[t], C::kGuAct, full);
-          if constexpr (DIRECT) mbar_arrive(full);  // (in the place of the warp that quantizes h rows)
+          if constexpr (DIRECT) mbar_arrive_n(full, direct_warps(INTER));  // (in the place of the warps that quantize h rows)
         } else if constexpr (DIRECT) {
           mbar_expect_tx_only(full, uint32_t(C::kDnTile));
           bulk_g2s(st, w0, C::kDnTile, full);
@@ -866,8 +867,9 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     return;
   }
 
-  if (DIRECT && warp == C::kWarps + 1) {
-    // ---------------- the h rows of every down entry, quantized into its slot as they arrive
+  if (DIRECT && warp > C::kWarps) {
+    // ---------------- a piece of the h rows of every down entry, quantized into its slot as they arrive
+    const int piece = warp - (C::kWarps + 1), at = 256 * piece + 8 * lane;
     for (int seq = 0;; ++seq) {
       const int s = seq % S;
       int e_seq, kind, pair0, ntp;
@@ -895,23 +897,11 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       if (e_seq != seq || kind == 0) continue;  // gate/up (its slot may have gone to a later entry already)
       uint8_t* out = stage0 + s * C::kSlot + C::kDnTile;
       for (int t = 0; t < ntp; ++t, out += C::kDnAct) {
-        constexpr int kPasses = (INTER + 255) / 256;
         const float* h = ws.h + size_t(pair0 + t) * INTER;
-        float v[kPasses][8];
+        float v[8];
         tries = 0;
         while (true) {
-          bool all = true;
-#pragma unroll
-          for (int p = 0; p < kPasses; ++p) {
-            const int e = 256 * p + 8 * lane;
-            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = a;
-            if (e < INTER) {
-              a = direct_load4(h + e, all);
-              c = direct_load4(h + e + 4, all);
-            }
-            v[p][0] = a.x; v[p][1] = a.y; v[p][2] = a.z; v[p][3] = a.w;
-            v[p][4] = c.x; v[p][5] = c.y; v[p][6] = c.z; v[p][7] = c.w;
-          }
+          const bool all = direct_load8(h, at, INTER, v);
           if (__all_sync(0xffffffffu, all)) break;
           if (++tries > kDirectPolls || __shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) {
             if (lane == 0) {
@@ -922,14 +912,17 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
           }
           __nanosleep(20);
         }
-        quantize_h_values<INTER>(v, down_act, out);
+        quantize_h_piece<INTER>(v, piece, down_act, out);
       }
       fence_proxy_async();  // (a later entry's bulk copies will write here)
       __syncwarp();
       if (lane == 0) mbar_arrive(&ring.full[s]);
       if (kind == 2)  // an item's first tile: its rows in the workspace too, where the other form of this kernel leaves them
-        for (int p = pair0; p < pair0 + ntp; ++p)
-          quantize_h_row<INTER>(ws.h + size_t(p) * INTER, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
+        for (int p = pair0; p < pair0 + ntp; ++p) {
+          float v[8];
+          direct_load8(ws.h + size_t(p) * INTER, at, INTER, v);
+          quantize_h_piece<INTER>(v, piece, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
+        }
     }
   }
 

@@ -9,7 +9,7 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 H = 2560
-IQ3_S, IQ4_NL, IQ2_S, Q2_0 = L.FMT_IQ3_S, L.FMT_IQ4_NL, L.FMT_IQ2_S, L.FMT_Q2_0
+IQ3_S, IQ4_NL, IQ2_S, IQ4_XS, Q2_0 = L.FMT_IQ3_S, L.FMT_IQ4_NL, L.FMT_IQ2_S, L.FMT_IQ4_XS, L.FMT_Q2_0
 
 
 def _torch():
@@ -22,11 +22,14 @@ def _bits(t):
     return t.contiguous().view(-1).cpu().numpy().view(np.uint32)
 
 
-@pytest.mark.parametrize("fg,fd,inter", [(IQ3_S, IQ3_S, 512), (IQ3_S, IQ4_NL, 640), (IQ4_NL, IQ4_NL, 512), (IQ2_S, Q2_0, 640)])
-@pytest.mark.parametrize("tokens", [1, 2, 3, 4])
-def test_fused_layer_equals_the_four_calls_at_few_tokens(fg, fd, inter, tokens):
-    """Three and four tokens are the two sides of a line. Several calls on one workspace with other activations, so that a
-    value of the call before would show; in one of them all tokens are alike (experts with every token, two passes)."""
+@pytest.mark.parametrize("fg,fd,inter,tokens", [(IQ3_S, IQ3_S, 512, t) for t in (1, 2, 3, 4)] +
+                         [(IQ3_S, IQ4_NL, 640, t) for t in (1, 2)] + [(IQ2_S, Q2_0, 640, t) for t in (1, 3)] +
+                         [(IQ4_NL, IQ4_NL, 512, t) for t in (1, 3, 4, 11, 16)] + [(IQ4_XS, IQ4_NL, 640, t) for t in (1, 2)] +
+                         [(IQ4_NL, Q2_0, 512, 7)])
+def test_fused_layer_equals_the_four_calls(fg, fd, inter, tokens):
+    """Both sides of the lines up to which values are their own arrival flags. Several calls on one workspace with other
+    activations, so that a value of the call before would show; in one of them most tokens are alike (experts with many
+    tokens, several passes; the pair visited last is not the one in the last slot)."""
     torch = _torch()
     from fngine_b200 import moe
     layer = moe.synth_layer(fg, fd, inter, 512, 40 + inter)
@@ -36,7 +39,7 @@ def test_fused_layer_equals_the_four_calls_at_few_tokens(fg, fd, inter, tokens):
     for call in range(5):
         x = torch.from_numpy(synth.activations(70 + call, tokens)).cuda()
         if call == 2:
-            x[:] = x[0].clone()
+            x[:tokens - tokens // 4] = x[0].clone()
         if call == 3:
             x = x.to(torch.bfloat16)
         y.fill_(float("nan"))
