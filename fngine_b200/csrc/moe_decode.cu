@@ -373,7 +373,7 @@ struct SelectScratch {
   int hist[kExperts / 32][kMaxTok + 1];  // [warp of slots][token count - 1] -> items (padded: no bank conflicts)
   int scan[kExperts / 32];               // [warp of slots] -> its pairs | its items << 16
 };
-// load(t, e): logit e of token t. `scratch`: shared memory (16-byte aligned) that is free until the call returns.
+// LAST: wc.last_pair is wanted. load(t, e): logit e of token t. `scratch`: shared memory (16-byte aligned) that is free until the call returns.
 // Called by every thread of a block of 512 or more threads. The work list goes to `wc` in shared memory
 // (complete when the call returns) and, with `publish`, to the device work list as well; `reset` clears
 // the tile and item counters of the streaming kernels (only where no such kernel can be running). The
@@ -388,7 +388,7 @@ struct SelectScratch {
 //   items  = distinct selected experts held on this rank, in physical-slot order
 //   pairs  = (item, token), tokens ascending inside an item
 //   order  = items by token count, most first, ties by item index (the streaming kernels' visiting order)
-template <class LoadF>
+template <bool LAST, class LoadF>
 __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of, int T,
                                              const fb_moe_decode_workspace& ws, uint32_t* counts, bool remote_ok,
                                              bool publish, bool reset, WorkCache& wc, SelectScratch& scratch) {
@@ -459,7 +459,7 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
           rank += ((first_m >> j) & 1u) && (cj > cnt || (cj == cnt && ij < item)) ? 1 : 0;
         }
       }
-      {  // (the lanes of an item agree on its rank)
+      if constexpr (LAST) {  // (the lanes of an item agree on its rank)
         const int mine = hot ? rank : -1;
         int most = -1;
 #pragma unroll
@@ -547,7 +547,7 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
         wc.slot[item] = tid;
         wc.pair_begin[item] = pair_begin;
         wc.order[order_base + peer_rank] = item;
-        scratch.rank[tid] = int16_t(order_base + peer_rank);
+        if constexpr (LAST) scratch.rank[tid] = int16_t(order_base + peer_rank);
       }
       if (tid == 0) {
         wc.pair_begin[n_items] = n_pairs;
@@ -576,15 +576,18 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
       s_pair[pt][pk] = idx;
     }
     if (slot2 >= 0) {
-      const int pair = pair_of(slot2, t2), mine = scratch.rank[slot2];
-      bool last = true;
-#pragma unroll
-      for (int k = 0; k < kTopK; ++k) {
-        const int other = scratch.slot[t2][k];
-        last = last && (other < 0 || scratch.rank[other] <= mine);
-      }
+      const int pair = pair_of(slot2, t2);
       wc.token_row[t2][rank2] = pair;
-      if (last) wc.last_pair[t2] = pair;
+      if constexpr (LAST) {
+        const int mine = scratch.rank[slot2];
+        bool last = true;
+#pragma unroll
+        for (int k = 0; k < kTopK; ++k) {
+          const int other = scratch.slot[t2][k];
+          last = last && (other < 0 || scratch.rank[other] <= mine);
+        }
+        if (last) wc.last_pair[t2] = pair;
+      }
     }
   }
   __syncthreads();
@@ -654,7 +657,7 @@ __global__ void __launch_bounds__(512) select_kernel(const float* logits, int lo
   }
   __shared__ WorkCache s_work;  // the streaming kernels of this path read the device work list instead
   __shared__ __align__(16) SelectScratch s_scratch;
-  select_block([&](int t, int e) { return logits[size_t(t) * logits_stride + e]; },
+  select_block<false>([&](int t, int e) { return logits[size_t(t) * logits_stride + e]; },
                slot_of, T, ws, counts, false, true, true, s_work, s_scratch);
 }
 

@@ -726,7 +726,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 
   int n_items;
   if (phases & kPhaseSelect) {
-    select_block([&](int t, int e) { return __ldcg(sel.logits + size_t(t) * sel.stride + e); }, sel.slot_of, sel.tokens, ws,
+    select_block<DIRECT>([&](int t, int e) { return __ldcg(sel.logits + size_t(t) * sel.stride + e); }, sel.slot_of, sel.tokens, ws,
                  nullptr, sel.remote_ok != 0, blockIdx.x == 0, false, s_work, *reinterpret_cast<SelectScratch*>(partials));
     n_items = s_work.n_items;
   } else {
