@@ -1439,21 +1439,21 @@ template <int GU, int DN, int INTER>
 int32_t launch_experts_as(const fb_moe_expert_layout* layout, const fb_moe_decode_workspace* ws, int phases,
                           void* stream, const char* what, const SelectArgs* sel) {
   using C = ExpertsCfg<GU, DN, INTER>;
-  auto launch = [&](auto kernel, PerDeviceOnce& once, int warps) -> int32_t {
+  auto launch = [&](auto kernel, PerDeviceOnce& once, int threads) -> int32_t {
     const cudaError_t attr = per_device_once(once, [&] { return opt_in_smem(kernel, C::kSmem); });
     if (attr != cudaSuccess) {
       set_error("%s: shared-memory opt-in: %s", what, cudaGetErrorString(attr));
       return int32_t(attr);
     }
-    const cudaError_t e = launch_pdl(kernel, dim3(sm_count()), dim3(warps * 32), C::kSmem, as_stream(stream), *layout, *ws,
+    const cudaError_t e = launch_pdl(kernel, dim3(sm_count()), dim3(threads), C::kSmem, as_stream(stream), *layout, *ws,
                                      sel ? (phases | kPhaseSelect) : phases, sel ? *sel : SelectArgs{});
     return e != cudaSuccess ? check_launch(what) : 0;
   };
   static PerDeviceOnce once[2];
   // the fused call's few tokens (the route kernel has filled h and the partial rows: layer_decode_impl)
   if (sel && sel->tokens <= direct_tokens(GU, INTER) && phases == (kPhaseGateUp | kPhaseDown))
-    return launch(experts_kernel<GU, DN, INTER, true>, once[1], C::kWarps + 1 + direct_warps(INTER));
-  return launch(experts_kernel<GU, DN, INTER, false>, once[0], C::kWarps + 1);
+    return launch(experts_kernel<GU, DN, INTER, true>, once[1], C::threads(true));
+  return launch(experts_kernel<GU, DN, INTER, false>, once[0], C::threads(false));
 }
 // Every gate/up format has its kernel with an IQ4_NL or Q2_0 down projection at both intermediate sizes; IQ3_S also with
 // its own.

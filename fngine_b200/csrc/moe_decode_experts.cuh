@@ -260,6 +260,8 @@ constexpr int kStaticSmem = 7168;  // the kernel's own shared variables, at most
 template <int GU, int DN, int INTER>
 struct ExpertsCfg {
   static constexpr int kWarps = 24, kTasks = 10, kInter = INTER;
+  // consumers, the producer, and where h rows carry their own arrival flags the warps that quantize them
+  static constexpr int threads(bool direct) { return (kWarps + 1 + (direct ? direct_warps(INTER) : 0)) * 32; }
   static constexpr int kTaskBytes = GuFmt<GU>::kBlock;
   static constexpr int kGuRows = 16, kGuRowBytes = kTasks * kTaskBytes, kGuPart = kGuRows * kGuRowBytes;
   static constexpr int kDnTaskBytes = DN == FB_FMT_IQ3_S ? 110 : INTER / (DN == FB_FMT_Q2_0 ? 128 : 64) * 18;  // half a row
@@ -696,7 +698,7 @@ __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspac
 // to 3 %; beyond direct_tokens the down tiles of the first experts cover the hand-off of the last ones, and every tile's own
 // quantization costs more than it saves.)
 template <int GU, int DN, int INTER, bool DIRECT>
-__global__ void __launch_bounds__((ExpertsCfg<GU, DN, INTER>::kWarps + 1 + (DIRECT ? direct_warps(INTER) : 0)) * 32, 1)
+__global__ void __launch_bounds__(ExpertsCfg<GU, DN, INTER>::threads(DIRECT), 1)
 experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, SelectArgs sel) {
   using C = ExpertsCfg<GU, DN, INTER>;
   constexpr int S = C::kStages;
