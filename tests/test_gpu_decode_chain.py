@@ -145,3 +145,63 @@ def test_host_activations_that_take_the_copy(kind, bf16):
         torch.cuda.synchronize()
         assert np.array_equal(yh.numpy().view(np.uint32), y2.cpu().numpy().view(np.uint32))
         assert torch.equal(xd.cpu(), x)
+
+
+def test_host_buffers_over_two_registrations():
+    """x and y that each lie in two neighbouring page-locked ranges: read and written in place, the same bits."""
+    torch = _torch()
+    import mmap
+    from fngine_b200 import moe
+    tokens = 2
+    layer = moe.synth_layer(IQ3_S, IQ3_S, 512, 512, 9)
+    ws = moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(303, rows=512).view(np.int16)).cuda().view(torch.bfloat16)
+    x = torch.from_numpy(synth.activations(13, tokens))
+    mem = torch.frombuffer(mmap.mmap(-1, 16 * 4096), dtype=torch.float32)  # x and y: five pages each
+    xh, yh = mem[:tokens * H].view(tokens, H), mem[5 * 1024:5 * 1024 + tokens * H].view(tokens, H)
+    xh.copy_(x)
+    cudart, base, pages = torch.cuda.cudart(), mem.data_ptr(), [0, 2, 7, 10]
+    for a, b in zip(pages, pages[1:]):
+        assert int(cudart.cudaHostRegister(base + 4096 * a, 4096 * (b - a), 0)) == 0
+    try:
+        xd = torch.zeros(tokens, H, dtype=torch.float32, device="cuda")
+        yd, y2 = (torch.empty(tokens, H, dtype=torch.float32, device="cuda") for _ in range(2))
+        yd.fill_(7.0)
+        moe.moe_layer_decode_host(wr, layer, xh, ws, xd, yd, yh)
+        moe.moe_layer_decode(wr, layer, x.cuda(), ws, y2)
+        torch.cuda.synchronize()
+        assert np.array_equal(yh.numpy().view(np.uint32), y2.cpu().numpy().view(np.uint32))
+        assert torch.equal(xd.cpu(), x) and bool((yd == 7.0).all())  # (the result went past the device buffer)
+    finally:
+        torch.cuda.synchronize()
+        for a in pages[:-1]:
+            cudart.cudaHostUnregister(base + 4096 * a)
+
+
+def test_page_locked_buffers_on_a_thread_without_a_context():
+    torch = _torch()
+    import ctypes as C
+    import threading
+    from fngine_b200 import moe
+    tokens = 1
+    layer = moe.synth_layer(IQ3_S, IQ3_S, 512, 512, 9)
+    ws = moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(303, rows=512).view(np.int16)).cuda().view(torch.bfloat16)
+    xh = torch.from_numpy(synth.activations(14, tokens)).pin_memory()
+    xd = torch.zeros(tokens, H, dtype=torch.float32, device="cuda")
+    yd, y2 = (torch.full((tokens, H), 7.0, dtype=torch.float32, device="cuda") for _ in range(2))
+    yh = torch.empty(tokens, H, dtype=torch.float32).pin_memory()
+    torch.cuda.synchronize()
+    status = []
+
+    def call():
+        status.append(L.load().fb_moe_layer_decode_host(wr.data_ptr(), C.byref(layer.layout), xh.data_ptr(), L.DT_F32, tokens,
+                                                        C.byref(ws.ws), ws.logits.data_ptr(), xd.data_ptr(), yd.data_ptr(),
+                                                        yh.data_ptr(), None))
+    t = threading.Thread(target=call)
+    t.start()
+    t.join()
+    moe.moe_layer_decode(wr, layer, xh.cuda(), ws, y2)
+    torch.cuda.synchronize()
+    assert status == [0] and bool((yd == 7.0).all())
+    assert np.array_equal(yh.numpy().view(np.uint32), y2.cpu().numpy().view(np.uint32))
