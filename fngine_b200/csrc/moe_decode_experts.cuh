@@ -173,6 +173,7 @@ template <int S>
 struct RingN {
   uint64_t* full;   // [S] count 1 (DIRECT: and one for every quantizing warp) + tx bytes
   uint64_t* empty;  // [S]
+  uint64_t* staged;  // [S] DIRECT: the entry's description stands (count 1, the producer)
   volatile StageMeta* meta;  // [S]
   // number of entries the producer staged in all; INT_MAX while it is still staging; 0 after a time-out
   volatile int* end_seq;
@@ -190,6 +191,7 @@ __device__ __forceinline__ void ringn_init(const RingN<S>& r, int arrivals) {
   for (int s = 0; s < S; ++s) {
     mbar_init(&r.full[s], arrivals);
     mbar_init(&r.empty[s], 1);  // one arrival frees a slot: the warp that finishes the entry's last task
+    mbar_init(&r.staged[s], 1);
     r.meta[s].tile = -1;
     r.meta[s].seq = -1;
   }
@@ -713,7 +715,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   __shared__ int s_misc[3 + S];  // [1..2] task tickets (even / odd blocks), [3..] finished tasks per slot
   __shared__ int s_end;
   __shared__ WorkCache s_work;
-  RingN<S> ring{bars, bars + S, s_meta, &s_end};
+  static_assert(3 * S * sizeof(uint64_t) <= 128, "barriers behind the block terms");
+  RingN<S> ring{bars, bars + S, bars + 2 * S, s_meta, &s_end};
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // (a down-only launch of another format than IQ3_S looks nothing up)
@@ -816,7 +819,6 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 #pragma unroll
           for (int t = 0; t < kTT; ++t)
             if (t < ntp) bulk_g2s(st + 2 * C::kGuPart + t * C::kGuAct, act[t], C::kGuAct, full);
-          if constexpr (DIRECT) mbar_arrive_n(full, direct_warps(INTER));  // (in the place of the warps that quantize h rows)
         } else if constexpr (DIRECT) {
           mbar_expect_tx_only(full, uint32_t(C::kDnTile));
           bulk_g2s(st, w0, C::kDnTile, full);
@@ -845,6 +847,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
             if (t < ntp) bulk_g2s(st + C::kDnTile + t * C::kDnAct, act[t], C::kDnAct, full);
         }
         m->store(i, !down ? 0 : DIRECT && sub == 0 ? 2 : 1, pair0, ntp, row0, item, pb, ntok, wgt);
+        if constexpr (DIRECT) mbar_arrive(&ring.staged[s]);
         mbar_arrive(full);
         if (failed) {  // nobody will use the entry: see its copies land (bounded), then leave
           mbar_wait_hint(full, (i / S) & 1);
@@ -871,32 +874,31 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
 
   if (DIRECT && warp > C::kWarps) {
     // ---------------- a piece of the h rows of every down entry, quantized into its slot as they arrive
+    // These warps arrive on every entry's full barrier, gate/up entries included, so the producer cannot lap them and an
+    // entry's phase of `staged` is its own. That barrier is what orders their reads of the description behind the producer's
+    // stores, and their writes into the slot behind the consumers' reads of the entry before (those arrive on `empty`, which
+    // the producer has waited for). (Probes with short naps: a try with a time limit wakes so late that eight layers of one
+    // token take 152.4 us instead of 146.4.)
     const int piece = warp - (C::kWarps + 1), at = 256 * piece + 8 * lane;
     for (int seq = 0;; ++seq) {
       const int s = seq % S;
-      int e_seq, kind, pair0, ntp;
       uint32_t tries = 0;
-      while (true) {
-        asm volatile("ld.volatile.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(e_seq), "=r"(kind), "=r"(pair0), "=r"(ntp)
-                     : "r"(smem_u32(const_cast<StageMeta*>(&s_meta[s])))
-                     : "memory");
-        e_seq = __shfl_sync(0xffffffffu, e_seq, 0);
-        kind = __shfl_sync(0xffffffffu, kind, 0);
-        pair0 = __shfl_sync(0xffffffffu, pair0, 0);
-        ntp = __shfl_sync(0xffffffffu, ntp, 0);
-        if (e_seq >= seq) break;
+      while (!__all_sync(0xffffffffu, mbar_test_wait(&ring.staged[s], (seq / S) & 1))) {
         if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) <= seq) return;
-        if (++tries > kDirectPolls) {
+        if (++tries > 4 * kDirectPolls) {
           if (lane == 0) {
             *ring.end_seq = 0;
             atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
           }
           return;
         }
-        __nanosleep(100);
+        __nanosleep(40);
       }
-      if (e_seq != seq || kind == 0) continue;  // gate/up (its slot may have gone to a later entry already)
+      const int kind = ring.meta[s].tile, pair0 = ring.meta[s].pair0, ntp = ring.meta[s].ntp;
+      if (kind == 0) {  // gate/up: nothing to add
+        if (lane == 0) mbar_arrive(&ring.full[s]);
+        continue;
+      }
       uint8_t* out = stage0 + s * C::kSlot + C::kDnTile;
       for (int t = 0; t < ntp; ++t, out += C::kDnAct) {
         const float* h = ws.h + size_t(pair0 + t) * INTER;
