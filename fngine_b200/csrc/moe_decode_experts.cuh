@@ -175,15 +175,42 @@ struct RingN {
   uint64_t* empty;  // [S]
   uint64_t* staged;  // [S] DIRECT: the entry's description stands (count 1, the producer)
   volatile StageMeta* meta;  // [S]
-  // number of entries the producer staged in all; INT_MAX while it is still staging; 0 after a time-out
+  // number of entries the producer staged in all; kRingOpen while it is still staging; 0 from a time-out on
   volatile int* end_seq;
+  volatile int* staged_seq;  // -1, then the entries staged when the producer stopped, whatever made it stop
 };
+constexpr int kRingOpen = 0x7fffffff;
+constexpr uint32_t kStopPolls = 1u << 26;  // polls of shared memory with naps of 40 ns or more: some five seconds
 
 // Bounded: 2^21 tries of at most about a microsecond each.
 __device__ __forceinline__ bool mbar_wait_hint(uint64_t* bar, uint32_t parity) {
   for (uint32_t i = 0; i < (1u << 21); ++i)
     if (mbar_try_wait_hint(bar, parity)) return true;
   return false;
+}
+
+// A wait has run out: warps that look at the end mark leave. It stays 0: the producer's count only ever takes the place of
+// kRingOpen.
+template <int S>
+__device__ __forceinline__ void ring_abort(const RingN<S>& r, uint32_t* status) {
+  *r.end_seq = 0;
+  atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+}
+template <int S>
+__device__ __forceinline__ void ring_close(const RingN<S>& r, int entries) {
+  *r.staged_seq = entries;
+  __threadfence_block();
+  atomicCAS(const_cast<int*>(r.end_seq), kRingOpen, entries);
+}
+// By one lane of the warp whose wait ran out: warps that leave early leave entries behind, and no block may end with copies
+// on their way into its shared memory. Waits (bounded) until the producer has stopped, then for the last entries' barriers.
+// The producer may be in its wait for a slot, some two seconds at most, which does not look at the end mark (eight layers of
+// one token take 148.5 us where it does, 146.5 as it is; a look at the end of every warp costs them 1 us as well).
+template <int S>
+__device__ __noinline__ void ring_drain(const RingN<S>& r) {
+  for (uint32_t i = 0; *r.staged_seq < 0 && i < kStopPolls; ++i) __nanosleep(100);
+  const int n = *r.staged_seq;
+  for (int e = max(0, n - S); e < n; ++e) mbar_wait_hint(&r.full[e % S], (e / S) & 1);
 }
 
 template <int S>
@@ -195,7 +222,8 @@ __device__ __forceinline__ void ringn_init(const RingN<S>& r, int arrivals) {
     r.meta[s].tile = -1;
     r.meta[s].seq = -1;
   }
-  *r.end_seq = 0x7fffffff;
+  *r.end_seq = kRingOpen;
+  *r.staged_seq = -1;
   mbar_fence_init();
 }
 
@@ -204,8 +232,7 @@ __device__ __forceinline__ void ringn_init(const RingN<S>& r, int arrivals) {
 // is being filled with, and the barrier's one-bit phase cannot tell those apart. So the warp first waits
 // (polling one shared-memory word, asleep in between) until the producer has written this entry's number
 // into the slot, which it does before it arms the barrier; only then is the barrier's current phase the
-// entry's own, and the warp can sleep inside try_wait. On a time-out the producer sets end_seq to 0, which
-// releases every waiting warp.
+// entry's own, and the warp can sleep inside try_wait.
 template <int S, int TASKS>
 __device__ __forceinline__ bool draw_task_n(const RingN<S>& r, int* ticket_ctr, uint32_t* status, int lane, int& s,
                                             int& task) {
@@ -219,8 +246,8 @@ __device__ __forceinline__ bool draw_task_n(const RingN<S>& r, int* ticket_ctr, 
   while (r.meta[s].seq != seq) {
     if (*r.end_seq <= seq) return false;
     if (++tries > (1u << 20)) {  // bounded: about a second
-      *r.end_seq = 0;
-      atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+      ring_abort(r, status);
+      if (lane == 0) ring_drain(r);
       return false;
     }
     // (the producer is behind only at the start of a phase; the nap is short because at one to three tokens this
@@ -232,8 +259,8 @@ __device__ __forceinline__ bool draw_task_n(const RingN<S>& r, int* ticket_ctr, 
     if (mbar_try_wait_hint(&r.full[s], parity)) return true;
     if (*r.end_seq <= seq) return false;
   }
-  *r.end_seq = 0;
-  atomicMax(status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+  ring_abort(r, status);
+  if (lane == 0) ring_drain(r);
   return false;
 }
 
@@ -639,10 +666,10 @@ __device__ __forceinline__ void combine_tile(const fb_moe_decode_workspace& ws, 
 // The same where rows are their own arrival flags: the warp that finished the tile of the token's pair that is visited last
 // polls the other pairs' rows (false: a wait has run out). What it waits for comes before its own tile in the order in which
 // tiles are drawn and tasks taken, so the earliest unfinished tile never waits for a polling warp.
-template <int ROWS>
+template <int ROWS, int S>
 __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspace& ws, const SelectArgs& sel,
                                                     const WorkCache& wc, int pair0, int ntp, int r0, int lane,
-                                                    volatile int* end_seq) {
+                                                    const RingN<S>& ring) {
   for (int i = 0; i < ntp; ++i) {
     const int t = wc.pair_token[pair0 + i];
     if (wc.last_pair[t] != pair0 + i) continue;
@@ -670,10 +697,11 @@ __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspac
           }
         }
         if (__all_sync(0xffffffffu, all)) break;
-        if (++tries > kDirectPolls || __shfl_sync(0xffffffffu, *end_seq, 0) == 0) {
+        if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) return false;
+        if (++tries > kDirectPolls) {
           if (lane == 0) {
-            *end_seq = 0;
-            atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+            ring_abort(ring, ws.status);
+            ring_drain(ring);
           }
           return false;
         }
@@ -713,10 +741,10 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
   uint64_t* bars = reinterpret_cast<uint64_t*>(partials + C::kPartialFloats);
   __shared__ StageMeta s_meta[S];
   __shared__ int s_misc[3 + S];  // [1..2] task tickets (even / odd blocks), [3..] finished tasks per slot
-  __shared__ int s_end;
+  __shared__ int s_end, s_staged;
   __shared__ WorkCache s_work;
   static_assert(3 * S * sizeof(uint64_t) <= 128, "barriers behind the block terms");
-  RingN<S> ring{bars, bars + S, bars + 2 * S, s_meta, &s_end};
+  RingN<S> ring{bars, bars + S, bars + 2 * S, s_meta, &s_end, &s_staged};
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // (a down-only launch of another format than IQ3_S looks nothing up)
@@ -755,18 +783,24 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     const int n_tiles = n_gu + n_dn;
     int i = 0;
     bool failed = false;
-    struct EndMark {  // whichever way the loop is left, waiting consumers learn how many entries exist
+    struct EndMark {  // whichever way the loop is left, waiting warps learn how many entries exist
       const RingN<S>& r;
       const int& i;
       const bool& failed;
-      __device__ ~EndMark() { *r.end_seq = failed ? 0 : i; }
+      __device__ ~EndMark() {
+        ring_close(r, i);
+        if (failed) ring_drain(r);
+      }
     } end_mark{ring, i, failed};
     auto give_up = [&]() {
       failed = true;
-      atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
+      ring_abort(ring, ws.status);
     };
     auto slot_free = [&](int s) -> bool {
-      if (*ring.end_seq == 0) return false;  // a consumer gave up
+      if (*ring.end_seq == 0) {  // another warp gave up
+        failed = true;
+        return false;
+      }
       if (i >= S && !mbar_wait_hint(&ring.empty[s], ((i / S) - 1) & 1)) {
         give_up();
         return false;
@@ -849,8 +883,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         m->store(i, !down ? 0 : DIRECT && sub == 0 ? 2 : 1, pair0, ntp, row0, item, pb, ntok, wgt);
         if constexpr (DIRECT) mbar_arrive(&ring.staged[s]);
         mbar_arrive(full);
-        if (failed) {  // nobody will use the entry: see its copies land (bounded), then leave
-          mbar_wait_hint(full, (i / S) & 1);
+        if (failed) {  // (the entry is complete all the same: its copies are under way)
+          ++i;
           return;
         }
         if (++s == S) s = 0;
@@ -880,20 +914,25 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
     // the producer has waited for). (Probes with short naps: a try with a time limit wakes so late that eight layers of one
     // token take 152.4 us instead of 146.4.)
     const int piece = warp - (C::kWarps + 1), at = 256 * piece + 8 * lane;
+    // Behind an expired wait they go on to the last entry that has been staged, with whatever h holds: the block's last wait
+    // for its copies (ring_drain) needs their arrivals.
+    bool expired = false;
     for (int seq = 0;; ++seq) {
       const int s = seq % S;
       uint32_t tries = 0;
+      bool end = false;
       while (!__all_sync(0xffffffffu, mbar_test_wait(&ring.staged[s], (seq / S) & 1))) {
-        if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) <= seq) return;
-        if (++tries > 4 * kDirectPolls) {
-          if (lane == 0) {
-            *ring.end_seq = 0;
-            atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
-          }
-          return;
+        end = uint32_t(__shfl_sync(0xffffffffu, *ring.staged_seq, 0)) <= uint32_t(seq);  // (-1: not known yet)
+        if (end) break;
+        if (++tries > kStopPolls) {
+          if (expired) return;  // (the producer does not answer)
+          expired = true;
+          tries = 0;
+          if (lane == 0) ring_abort(ring, ws.status);
         }
         __nanosleep(40);
       }
+      if (end) break;
       const int kind = ring.meta[s].tile, pair0 = ring.meta[s].pair0, ntp = ring.meta[s].ntp;
       if (kind == 0) {  // gate/up: nothing to add
         if (lane == 0) mbar_arrive(&ring.full[s]);
@@ -904,15 +943,12 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         const float* h = ws.h + size_t(pair0 + t) * INTER;
         float v[8];
         tries = 0;
-        while (true) {
-          const bool all = direct_load8(h, at, INTER, v);
-          if (__all_sync(0xffffffffu, all)) break;
-          if (++tries > kDirectPolls || __shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) {
-            if (lane == 0) {
-              *ring.end_seq = 0;
-              atomicMax(ws.status, uint32_t(FB_STATUS_PIPELINE_TIMEOUT));
-            }
-            return;
+        while (!__all_sync(0xffffffffu, direct_load8(h, at, INTER, v))) {
+          if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) break;
+          if (++tries > kDirectPolls) {
+            expired = true;
+            if (lane == 0) ring_abort(ring, ws.status);
+            break;
           }
           __nanosleep(20);
         }
@@ -928,6 +964,8 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
           quantize_h_piece<INTER>(v, piece, down_act, ws.hq + size_t(p) * FB_HQ_STRIDE);
         }
     }
+    if (expired && lane == 0) ring_drain(ring);
+    return;
   }
 
   // ---------------- consumers
@@ -1035,7 +1073,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       }
       if (sel.y_out) {
         if constexpr (!DIRECT) combine_tile<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane);
-        else if (!combine_tile_direct<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane, ring.end_seq)) break;
+        else if (!combine_tile_direct<C::kDnRows>(ws, sel, s_work, pair0, ntp, r0, lane, ring)) break;
       }
     }
   }
