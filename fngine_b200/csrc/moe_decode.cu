@@ -1128,7 +1128,13 @@ __device__ __forceinline__ bool direct_load8(const float* row, int at, int n, fl
   v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
   return all;
 }
-constexpr uint32_t kDirectPolls = 1u << 20;  // about a second
+// Polls of a value (or of an item's flag) that other multiprocessors write, unless the workspace names a number: each takes a
+// round trip to L2 and a nap of 20 ns or more, two to three seconds in all. A layer may share the GPU with another stream's
+// kernel, and the blocks that it waits for start behind that.
+constexpr uint32_t kValuePolls = 1u << 22;
+__device__ __forceinline__ uint32_t value_polls(const fb_moe_decode_workspace& ws) {
+  return ws.wait_polls > 0 ? uint32_t(ws.wait_polls) : kValuePolls;
+}
 // Warps that quantize the h rows of a CTA's down entries, each its piece of 256 values.
 constexpr int direct_warps(int inter) { return (inter + 255) / 256; }
 
@@ -1546,7 +1552,7 @@ int32_t fb_moe_decode_workspace_make(void* base, const fb_moe_expert_layout* lay
   out->gate_up_format = layout ? layout->gate_up_format : 0;  // 0: any (the selection quantizes x both ways)
   out->down_format = layout ? layout->down_format : 0;
   out->inter = layout ? layout->inter : 0;
-  out->reserved = 0;
+  out->wait_polls = 0;
   return 0;
 }
 

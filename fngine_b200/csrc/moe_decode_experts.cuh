@@ -245,7 +245,7 @@ __device__ __forceinline__ bool draw_task_n(const RingN<S>& r, int* ticket_ctr, 
   uint32_t tries = 0;
   while (r.meta[s].seq != seq) {
     if (*r.end_seq <= seq) return false;
-    if (++tries > (1u << 20)) {  // bounded: about a second
+    if (++tries > (1u << 20)) {  // bounded: a quarter of a second
       ring_abort(r, status);
       if (lane == 0) ring_drain(r);
       return false;
@@ -698,7 +698,7 @@ __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspac
         }
         if (__all_sync(0xffffffffu, all)) break;
         if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) return false;
-        if (++tries > kDirectPolls) {
+        if (++tries > value_polls(ws)) {
           if (lane == 0) {
             ring_abort(ring, ws.status);
             ring_drain(ring);
@@ -866,7 +866,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
               int v;
               asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
               if (v) break;
-              if (++tries > (1u << 22) || *ring.end_seq == 0) {
+              if (++tries > value_polls(ws) || *ring.end_seq == 0) {
                 give_up();
                 break;
               }
@@ -945,7 +945,7 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         tries = 0;
         while (!__all_sync(0xffffffffu, direct_load8(h, at, INTER, v))) {
           if (__shfl_sync(0xffffffffu, *ring.end_seq, 0) == 0) break;
-          if (++tries > kDirectPolls) {
+          if (++tries > value_polls(ws)) {
             expired = true;
             if (lane == 0) ring_abort(ring, ws.status);
             break;

@@ -128,7 +128,12 @@ typedef struct fb_moe_decode_workspace {
   int32_t gate_up_format;
   int32_t down_format;
   int32_t inter;
-  int32_t reserved;
+  union {
+    int32_t reserved;
+    /* 0, or the polls that the expert kernel gives a value written by another multiprocessor (h, partial rows, an item's
+     * flag) before it gives up and sets FB_STATUS_PIPELINE_TIMEOUT; 0: some two to three seconds' worth. */
+    int32_t wait_polls;
+  };
 } fb_moe_decode_workspace;
 enum { FB_XQ_STRIDE = 2880, FB_HQ_STRIDE = 720 };
 

@@ -205,3 +205,43 @@ def test_page_locked_buffers_on_a_thread_without_a_context():
     torch.cuda.synchronize()
     assert status == [0] and bool((yd == 7.0).all())
     assert np.array_equal(yh.numpy().view(np.uint32), y2.cpu().numpy().view(np.uint32))
+
+
+@pytest.mark.parametrize("fg,fd,inter", [(IQ3_S, IQ3_S, 512), (IQ4_NL, IQ4_NL, 512), (IQ3_S, IQ4_NL, 640)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_a_value_that_does_not_arrive_in_time(fg, fd, inter, fused):
+    """One poll for what other multiprocessors write instead of millions, at one token, where h is never there when the first
+    down tile wants it: rows that are their own arrival flags (the fused layer) and an item's flag (behind a stand-alone
+    selection). The layer ends by itself in a few seconds, the status says why, and the next layer on the workspace gives the
+    right bits."""
+    torch = _torch()
+    import time
+    from fngine_b200 import moe
+    layer = moe.synth_layer(fg, fd, inter, 512, 21)
+    ws = moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(303, rows=512).view(np.int16)).cuda().view(torch.bfloat16)
+    x = torch.from_numpy(synth.activations(15, 1)).cuda()
+    want, y = (torch.empty(1, H, dtype=torch.float32, device="cuda") for _ in range(2))
+
+    def run(out):
+        if fused:
+            moe.moe_layer_decode(wr, layer, x, ws, out)
+        else:
+            moe.moe_select_publish(ws.logits, x, None, 0, None, None, 1, ws)
+            moe.moe_hot_experts(layer, 1, ws)
+            moe.moe_combine(ws, None, None, 0, None, None, None, out, 1)
+        torch.cuda.synchronize()
+
+    moe.moe_layer_decode(wr, layer, x, ws, want)
+    run(y)
+    assert ws.status() == 0 and torch.equal(y, want)
+    ws.ws.wait_polls = 1
+    began = time.monotonic()
+    run(y)
+    assert time.monotonic() - began < 10.0
+    assert ws.status() == L.STATUS_PIPELINE_TIMEOUT
+    ws.ws.wait_polls = 0
+    ws._view(ws.ws.status, 4).zero_()
+    y.fill_(float("nan"))
+    run(y)
+    assert ws.status() == 0 and torch.equal(y, want)
