@@ -1237,9 +1237,11 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
   cluster_arrive();  // (`failed` is cleared: the peers may write it behind their half of this barrier)
   // Few tokens on a matrix whose traffic counts: the weights on their way into L2 while the call before runs out (nothing
-  // is read yet). Eight calls, us, without and with: 2560 x 6144 at one token 70.1 and 67.1, two 77.7 and 73.7, four 79.3
-  // and 75.8, but six 82.6 and 83.7, sixteen 94.5 and 99.6 (the activations and residual streams queue behind them);
-  // 9216 x 2560 at one 78.0 and 74.2, eight 89.5 and 92.8; 1280 x 2560 at four 49.5 and 53.2.
+  // is read yet). Eight calls of a chain whose weights come from memory, us, without and with: 2560 x 6144 at one token 66.0
+  // and 62.8, four 69.2 and 65.1; 4096 x 2560 57.4 and 55.3, 60.0 and 57.5; 3328 x 2560 (8.5 MB) 56.1 and 54.4, 61.9 and
+  // 59.9; below the line 2560 x 2560 53.3 and 53.2, 58.4 and 58.1, and where eight calls' weights stay in L2 it costs: 1280 x
+  // 2560 at four 49.5 and 53.2. More tokens: 2560 x 6144 at six 82.6 and 83.7, sixteen 94.5 and 99.6, 9216 x 2560 at eight
+  // 89.5 and 92.8 (the activations and residual streams queue behind the weights).
   if (warp == 0 && a.T <= 4 && size_t(a.n) * a.k >= (size_t(8) << 20)) {
     if (elect_one())
       for (int i = 0; i < nkb; ++i) {

@@ -663,13 +663,18 @@ __global__ void __launch_bounds__(512) select_kernel(const float* logits, int lo
                slot_of, T, ws, counts, false, true, true, s_work, s_scratch);
 }
 
-// Up to here values carry their own arrival flags (direct_store). Eight layers, us, by counters and so: IQ3_S 512 at one
-// token 168 and 146, two 218 and 187, three 251 and 230, four 253 and 255, sixteen 630 and 662; IQ4_NL 512 (four ring slots:
-// the quantizing warps run further ahead) at one 161 and 144, four 254 and 233, eight 371 and 359, sixteen 612 and 597;
-// IQ3_S + IQ4_NL 640 at one 183 and 160, two 237 and 240, IQ4_XS + IQ4_NL 640 at two 244 and 244, four 340 and 365: rows of
-// 640 take the quantizing warps longer than a tile of 128 rows takes the others.
-__host__ __device__ constexpr int direct_tokens(int gate_up, int inter) {
-  return inter != 512 ? 1 : gate_up == FB_FMT_IQ4_NL ? kMaxTok : 3;
+// Up to here values carry their own arrival flags (direct_store). At one token that is 7 to 13 % of a layer in every pair of
+// formats, because the hand-off of h stands in the layer's chain; with more tokens the down tiles of the first experts cover
+// the hand-off of the last ones, and each down tile quantizes its item's rows again. Eight layers, us, by counters and so:
+//   512, IQ3_S + IQ3_S     one 161 144   three 245 230   four 253 253   six 312 326   sixteen 627 658
+//        IQ4_NL + IQ4_NL   one 166 145   three 246 219   four 255 236   six 311 300   eight 377 363   sixteen 616 596
+//        IQ4_NL + Q2_0     one 158 140   three 233 215   four 239 229   six 287 292   eight 343 349   sixteen 563 572
+//        the other eight at one 158 to 174 and 137 to 155, at three 239 to 266 and 219 to 247; the lines are not drawn
+//        further for them: six tokens +2 to -2 %
+//   640, IQ3_S + IQ4_NL    one 178 154   two 237 227   three 292 287
+//        the other nine at one 163 to 185 and 146 to 164, at two 212 to 249 and 201 to 247
+__host__ __device__ constexpr int direct_tokens(int gate_up, int down, int inter) {
+  return inter != 512 ? 1 : gate_up != FB_FMT_IQ4_NL ? 3 : down == FB_FMT_IQ4_NL ? kMaxTok : 4;
 }
 constexpr uint32_t kNotYet = 0xFFFFFFFFu;
 
@@ -1483,7 +1488,7 @@ int32_t launch_experts_as(const fb_moe_expert_layout* layout, const fb_moe_decod
   };
   static PerDeviceOnce once[2];
   // the fused call's few tokens (the route kernel has filled h and the partial rows: layer_decode_impl)
-  if (sel && sel->tokens <= direct_tokens(GU, INTER) && phases == (kPhaseGateUp | kPhaseDown))
+  if (sel && sel->tokens <= direct_tokens(GU, DN, INTER) && phases == (kPhaseGateUp | kPhaseDown))
     return launch(experts_kernel<GU, DN, INTER, true>, once[1], C::threads(true));
   return launch(experts_kernel<GU, DN, INTER, false>, once[0], C::threads(false));
 }
@@ -1686,7 +1691,7 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
   if (ep) era = *ep;
   era.act = layout_ok(layout) ? act_of(layout->gate_up_format) : FB_ACT_Q8_K;
   const bool own_combine = with_combine && !slot_of && layout_ok(layout) && one_launch(layout);
-  if (layout_ok(layout) && tokens <= direct_tokens(layout->gate_up_format, layout->inter) && one_launch(layout)) {
+  if (layout_ok(layout) && tokens <= direct_tokens(layout->gate_up_format, layout->down_format, layout->inter) && one_launch(layout)) {
     era.clear_h = tokens * kTopK * layout->inter;
     era.clear_partial = own_combine ? tokens * kTopK * H : 0;
   }

@@ -60,6 +60,12 @@ def test_fused_layer_equals_the_four_calls(fg, fd, inter, tokens):
             assert list(a.token_pairs[t]) == list(b.token_pairs[t]) and list(a.topk_weight[t]) == list(b.topk_weight[t])
 
 
+@pytest.mark.parametrize("tokens", [4, 5])
+def test_fused_layer_equals_the_four_calls_with_q2_0_down(tokens):
+    """The two sides of the line of IQ4_NL + Q2_0 at 512."""
+    test_fused_layer_equals_the_four_calls(IQ4_NL, Q2_0, 512, tokens)
+
+
 def test_values_that_are_not_numbers_arrive_too():
     """Rows of h that are NaN or infinite (an activation at the top of the range) must not be taken for missing ones."""
     torch = _torch()
