@@ -375,8 +375,8 @@ __device__ __forceinline__ void warp_topk10(LoadF load_logit, int* ids, float* w
 // candidate against the others (larger logit, then lower id: a strict order), and ranks 0..9 are the winners. More than 32
 // survivors (many equal logits), or a bound of -infinity (which NaN counts as), take the general path. Same winners, same
 // order as warp_topk10; out_ids / out_vals (ten entries each, shared memory) are complete after the caller's next barrier.
-// Bound: instructions on one warp's chain. With 32 lane maxima, ranks by shuffles and the softmax in the chain the whole
-// selection took 2.8 us at one token and 4.1 at sixteen, now 2.1 and 3.3.
+// Bound: instructions on one warp's chain. The whole selection takes 2.1 us at one token and 3.3 at sixteen, 2.8 and 4.1 with
+// 32 lane maxima, ranks by shuffles and the softmax in the chain.
 template <class LoadF>
 __device__ __forceinline__ void warp_top10_pruned(LoadF load_logit, uint2* scratch, int* out_ids, float* out_vals) {
   const int lane = threadIdx.x & 31;

@@ -375,7 +375,8 @@ struct SelectScratch {
   int hist[kExperts / 32][kMaxTok + 1];  // [warp of slots][token count - 1] -> items (padded: no bank conflicts)
   int scan[kExperts / 32];               // [warp of slots] -> its pairs | its items << 16
 };
-// LAST: wc.last_pair is wanted. load(t, e): logit e of token t. `scratch`: shared memory (16-byte aligned) that is free until the call returns.
+// LAST: wc.last_pair is wanted. load(t, e): logit e of token t. `scratch`: shared memory (16-byte aligned) that is free until
+// the call returns.
 // Called by every thread of a block of 512 or more threads. The work list goes to `wc` in shared memory
 // (complete when the call returns) and, with `publish`, to the device work list as well; `reset` clears
 // the tile and item counters of the streaming kernels (only where no such kernel can be running). The
@@ -698,10 +699,10 @@ struct EpRouteArgs {
 // 4i..4i+3 to CTA i of its cluster through distributed shared memory, and behind one cluster barrier CTA i adds them in
 // slice order 0..7 (fixed: repeated calls are bitwise identical) and stores the logits. Two more warps of every block
 // quantize the activation rows meanwhile, and block 0 clears the counters of the streaming kernels (none can be running:
-// this kernel waited for its predecessor). From the wait to the last block's end, before -> now: one token 4.5 -> 2.3 us,
-// sixteen 8.8 -> 4.2, four with the shared rows 9.8 -> 5.6. (Before: clusters of eight, of which only fifteen find a
-// multiprocessor per CTA where 33 of four do; x was loaded in turns ahead of the weights, quantization stood behind the
-// projection, and slice sums were read out of the other CTAs, which had to wait for that.)
+// this kernel waited for its predecessor). From the wait to the last block's end: one token 2.3 us, sixteen 4.2, four with
+// the shared rows 5.6; 4.5, 8.8 and 9.8 with clusters of eight (only fifteen of those find a multiprocessor per CTA, 33 of
+// four do), x loaded in turns ahead of the weights, quantization behind the projection, and slice sums read out of the other
+// CTAs, which then wait for their readers.
 //
 // With SHARED (the whole decode branch of a layer) the kernel also projects the shared expert's gate/up rows and router
 // row 512, its gate: cluster g takes inter_s / 32 (gate, up) row pairs the same way, FP8 codes widened exactly, and
@@ -1045,10 +1046,12 @@ __global__ void __launch_bounds__(kRouteThreads, 1) route_kernel(const __nv_bflo
 // not depend on which CTA or warp ran which piece.
 constexpr int kSchedGateUp = 0, kSchedDown = 1;
 
-// What the producer tells the consumers about the entry staged in a ring slot (shared memory).
+// What the producer tells the consumers about the entry staged in a ring slot (shared memory). A reader acquires it through
+// the barrier on which the producer arrives behind store() (`full`, or `staged`); the entry number alone is also polled, to
+// learn that the slot's barrier has reached the entry's phase (draw_task_n), and is therefore stored last.
 struct alignas(16) StageMeta {
   int seq;         // entry number of this CTA
-  int tile;        // entry kind: 0 gate/up, 1 down
+  int tile;        // entry kind: 0 gate/up, 1 down, 2 down and its item's first tile
   int pair0;       // first pair (row of h / partial) of this pass
   int ntp;         // tokens in this pass (1..kTT)
   int row0;        // first intermediate row (gate/up) or output row (down) of the tile
@@ -1068,10 +1071,8 @@ struct alignas(16) StageMeta {
 };
 static_assert(kTT == 2 && sizeof(StageMeta) == 48, "three vector stores");
 
-// One row of h -> a planar activation row of the down projection, by the calling warp; all of the row's loads are in
-// flight before the first block is quantized (the finishing warp waits on this chain: Q8_0 rows taken block by block, twenty
-// round trips at 640, cost a layer of one token 8 us). `out` in global or shared memory, 16-byte aligned.
-// Piece p of a row: lane l holds elements 256 p + 8 l .. + 7 (none behind the row's end).
+// Piece p of a row of h -> its place in a planar activation row of the down projection, by the calling warp: lane l holds
+// elements 256 p + 8 l .. + 7 (none behind the row's end). `out`: the row, in global or shared memory, 16-byte aligned.
 template <int I>
 __device__ __forceinline__ void quantize_h_piece(const float (&v)[8], int p, int down_act, uint8_t* out) {
   if (I % 256 == 0 && down_act == FB_ACT_Q8_K) {
@@ -1082,6 +1083,8 @@ __device__ __forceinline__ void quantize_h_piece(const float (&v)[8], int p, int
     q8_0_eight_blocks_warp(v, 256 * p + 8 * int(threadIdx.x & 31) < I, out + 256 * p, reinterpret_cast<float*>(out + I) + 8 * p);
   }
 }
+// A whole row; all of its loads are in flight before the first block is quantized (the finishing warp waits on this chain:
+// Q8_0 rows taken block by block, twenty round trips at 640, cost a layer of one token 8 us).
 template <int I>
 __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uint8_t* out) {
   constexpr int kPasses = (I + 255) / 256;
@@ -1102,7 +1105,7 @@ __device__ __forceinline__ void quantize_h_row(const float* h, int down_act, uin
   for (int p = 0; p < kPasses; ++p) quantize_h_piece<I>(v[p], p, down_act, out);
 }
 
-// Up to direct_tokens: values that are their own arrival flags. The route kernel fills the rows with kNotYet, a NaN
+// Up to direct_tokens, values are their own arrival flags. The route kernel fills the rows with kNotYet, a NaN
 // that no arithmetic produces; a value is stored once, by one relaxed store, and a reader polls the values it needs (a
 // bounded number of times). Nothing else is read on the strength of a value, so no fence and no counter stand between a
 // store and its reader: release, counter, a last contributor that re-quantizes a row, its flag, the row's copy into shared
@@ -1691,7 +1694,8 @@ static int32_t layer_decode_impl(const void* router_w_bf16, const fb_moe_expert_
   if (ep) era = *ep;
   era.act = layout_ok(layout) ? act_of(layout->gate_up_format) : FB_ACT_Q8_K;
   const bool own_combine = with_combine && !slot_of && layout_ok(layout) && one_launch(layout);
-  if (layout_ok(layout) && tokens <= direct_tokens(layout->gate_up_format, layout->down_format, layout->inter) && one_launch(layout)) {
+  if (layout_ok(layout) && one_launch(layout) &&
+      tokens <= direct_tokens(layout->gate_up_format, layout->down_format, layout->inter)) {
     era.clear_h = tokens * kTopK * layout->inter;
     era.clear_partial = own_combine ? tokens * kTopK * H : 0;
   }

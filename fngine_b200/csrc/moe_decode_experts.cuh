@@ -10,8 +10,8 @@
 // layer and HBM keeps streaming across the gate/up -> down boundary. A down tile needs its expert's h
 // re-quantized, which the warp that finishes the expert's last gate/up tile does and then flags; the
 // producer asks for a down tile's weights first and polls that flag (a bounded number of times) only
-// before it asks for the activation rows. The same kernel runs one phase alone behind the separate
-// gate/up and down entry points.
+// before it asks for the activation rows. (With few tokens values carry their own arrival flags instead: DIRECT, below.) The
+// same kernel runs one phase alone behind the separate gate/up and down entry points.
 //
 // Shape of the work. A lane owns a weight row; a warp task is one 110-byte block (256 weights) of 32
 // rows (gate/up: 16 gate rows + the 16 matching up rows, ten blocks; down: five groups of 32 rows, two
@@ -336,9 +336,9 @@ static __device__ uint16_t g_iq2s_grid_packed[1024] = {FB_IQ2S_GRID_PACKED};
 // copy c at byte 64 i + 8 c, a lane reads copy lane % 8: two lanes of a half warp share two bank groups, 3 passes per
 // look-up of eight weights against 6 with one copy). IQ3_XXS: 256 entries of four magnitudes, one copy per lane.
 // A warp expands 32 entries, one per lane, and its lanes then write consecutive 16-byte pieces of the copies (no bank
-// conflicts), the values coming through shuffles. (With a constant-memory read and an expansion per 16 bytes written the
-// fill took 1.0 us for IQ3_S and up to 3.0 for IQ2_S and stood between the route kernel's end and the selection on the
-// multiprocessors that the route kernel left last: now 0.8 and 1.3.)
+// conflicts), the values coming through shuffles: 0.8 us for IQ3_S, up to 1.3 for IQ2_S, between the route kernel's end and
+// the selection on the multiprocessors that the route kernel leaves last (1.0 and 3.0 with a constant-memory read and an
+// expansion per 16 bytes written).
 template <int FMT>
 __device__ __forceinline__ void experts_table_fill(uint32_t* grid, uint32_t* signtab) {
   if constexpr (FMT == FB_FMT_IQ3_S || FMT == FB_FMT_IQ2_S || FMT == FB_FMT_IQ3_XXS) {
@@ -724,9 +724,8 @@ __device__ __forceinline__ bool combine_tile_direct(const fb_moe_decode_workspac
 
 // DIRECT (all phases, up to direct_tokens): h and the partial rows are their own arrival flags (direct_store), and two or
 // three more warps, each its 256 values, quantize the h rows of this CTA's down entries as they arrive. One token of IQ3_S:
-// by counters 168 us for eight layers, with one quantizing warp 154, now 146. (As a run-time switch it cost sixteen tokens 2
-// to 3 %; beyond direct_tokens the down tiles of the first experts cover the hand-off of the last ones, and every tile's own
-// quantization costs more than it saves.)
+// by counters 161 us for eight layers, with one quantizing warp 154, with two 147. (As a run-time switch it cost sixteen
+// tokens 2 to 3 %.)
 template <int GU, int DN, int INTER, bool DIRECT>
 __global__ void __launch_bounds__(ExpertsCfg<GU, DN, INTER>::threads(DIRECT), 1)
 experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, SelectArgs sel) {

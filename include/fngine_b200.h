@@ -115,7 +115,8 @@ typedef struct fb_moe_decode_work {
  * work list. In `sched` follow from
  * [8] on the work items ordered by token count (heaviest first), from [192] on the counters of finished
  * down rows per token and column tile, `status` is one device word set
- * when a bounded wait runs out. */
+ * when a bounded wait runs out. The fused layer calls of few tokens leave `item_done` and those counters clear: there h and
+ * the partial rows hold the bits 0xFFFFFFFF (a NaN that the library never stores) until a value arrives. */
 typedef struct fb_moe_decode_workspace {
   fb_moe_decode_work* work;
   uint8_t* xq;        /* [2][16][FB_XQ_STRIDE]: Q8_K rows, then Q8_0 rows */
