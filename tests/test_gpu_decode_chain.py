@@ -66,6 +66,26 @@ def test_fused_layer_equals_the_four_calls_with_q2_0_down(tokens):
     test_fused_layer_equals_the_four_calls(IQ4_NL, Q2_0, 512, tokens)
 
 
+@pytest.mark.parametrize("fg,fd,inter,tokens", [(IQ3_S, IQ3_S, 512, 1), (IQ3_S, IQ3_S, 512, 4), (IQ4_NL, IQ4_NL, 512, 16),
+                                                (IQ2_S, Q2_0, 640, 1), (IQ3_S, IQ4_NL, 640, 2)])
+def test_down_alone_behind_the_fused_layer(fg, fd, inter, tokens):
+    """Both forms of the hand-off leave h re-quantized in the workspace: the down projection, run again by itself, gives the
+    partial rows once more."""
+    torch = _torch()
+    from fngine_b200 import moe
+    layer = moe.synth_layer(fg, fd, inter, 512, 60 + inter)
+    ws = moe.DecodeWorkspace(layer)
+    wr = torch.from_numpy(synth.router_weights(303, rows=512).view(np.int16)).cuda().view(torch.bfloat16)
+    x = torch.from_numpy(synth.activations(77, tokens)).cuda()
+    y, y2 = (torch.empty(tokens, H, dtype=torch.float32, device="cuda") for _ in range(2))
+    moe.moe_layer_decode(wr, layer, x, ws, y)
+    ws._view(ws.ws.partial, 10 * tokens * H * 4).fill_(255)
+    moe.moe_hot_down(layer, tokens, ws)
+    moe.moe_combine(ws, None, None, 0, None, None, None, y2, tokens)
+    torch.cuda.synchronize()
+    assert ws.status() == 0 and torch.equal(y, y2)
+
+
 def test_values_that_are_not_numbers_arrive_too():
     """Rows of h that are NaN or infinite (an activation at the top of the range) must not be taken for missing ones."""
     torch = _torch()
