@@ -41,9 +41,11 @@ struct GgBars {
 static __constant__ int8_t c_iq4nl_levels[16] = {FB_IQ4NL_LEVELS};
 
 // Raw weight bytes in shared memory.
-// gate/up: a slot = one round (256 weights) of the unit's 128 rows, copied row piece by row piece. IQ3_S: the 28 words that
-//   cover a row's 110-byte block, 29 words apart (an odd number: 32 lanes reading the same word of 32 rows meet 32
-//   banks). IQ4_NL: 144 bytes, back to back (16-byte reads of eight neighbouring rows cover all banks).
+// gate/up: a slot = one round (256 weights) of the unit's 128 rows, copied row piece by row piece. IQ3_S: the up to eight
+//   16-byte words that cover a row's 110-byte block (single 4-byte words took four times the copies: with them the two copying
+//   warps alone needed 200 us for gate/up of 96 tokens, which went from 241 to 213 us). Rows lie 1100 bytes apart, so a block starts at word 0..3 of its first 16 bytes,
+//   by turns; the rows of 32 lanes are laid out so that the same word of their blocks meets 32 banks (gg_iq3s_slot_row).
+//   IQ4_NL: 144 bytes, back to back (16-byte reads of eight neighbouring rows cover all banks).
 // down: a slot = the whole unit, 128 complete rows, which lie back to back in the matrix: one bulk copy. (Cut into pieces like
 //   gate/up, rows of 360 bytes came in 8-byte copies, and the copying warps were the pace: 382 us instead of 233 at 1003
 //   tokens.)
@@ -51,7 +53,7 @@ template <int FMT, bool DOWN>
 struct GgRaw;
 template <>
 struct GgRaw<FB_FMT_IQ3_S, false> {
-  static constexpr int kPiece = 110, kPitch = 116, kSlots = 6, kSlot = kTileM * kPitch;
+  static constexpr int kPiece = 110, kPitch = 132, kSlots = 5, kSlot = kTileM * kPitch;  // (128 + 16 bytes per four rows)
 };
 template <>
 struct GgRaw<FB_FMT_IQ4_NL, false> {
@@ -78,6 +80,14 @@ constexpr int gg_smem() {
 static_assert(gg_smem<FB_FMT_IQ3_S, false>() <= 232448 && gg_smem<FB_FMT_IQ4_NL, false>() <= 232448 &&
                   gg_smem<FB_FMT_IQ3_S, true>() <= 232448 && gg_smem<FB_FMT_IQ4_NL, true>() <= 232448,
               "shared memory per block");
+
+// Byte of an IQ3_S gate/up slot where the piece of lane l (row l / 2 of gate or up) of a lane quarter begins. Places are taken
+// in the order of g = l / 8 + 4 (l % 2), four rows each, 128 bytes per row and another 16 after every four: the 16-byte words
+// of a g start in bank 4 g, and its four rows' blocks in the four banks from there.
+__device__ __forceinline__ uint32_t gg_iq3s_slot_row(int l) {
+  const int g = (l >> 3) + 4 * (l & 1), p = 4 * g + ((l >> 1) & 3);
+  return uint32_t(128 * p + 16 * g);
+}
 
 __device__ __forceinline__ uint32_t lds_u8(uint32_t a) {
   uint32_t v;
@@ -258,8 +268,8 @@ struct GgWords {
 };
 
 // ------------------------------------------------------------------------------ raw bytes into shared memory
-// gate/up: one loader warp copies the pieces of 32 rows (`bytes` of each) into its part of a raw slot. row_at(r) = address of
-// the piece of row r (IQ3_S: of the word that holds its first byte). Copy size: the largest the alignment allows; pieces two bytes off word alignment (an expert
+// gate/up, IQ4_NL: one loader warp copies the pieces of 32 rows (`bytes` of each) into its part of a raw slot. row_at(r) =
+// address of the piece of row r. Copy size: the largest the alignment allows; pieces two bytes off word alignment (an expert
 // table may hold any even address) go through registers. Returns true if the copies are asynchronous.
 template <int B, class RowF>
 __device__ __forceinline__ void gg_copy_pieces(uint32_t dst, int pitch, int bytes, int lane, RowF row_at) {
@@ -270,43 +280,31 @@ __device__ __forceinline__ void gg_copy_pieces(uint32_t dst, int pitch, int byte
                  : "memory");
   }
 }
-template <int FMT, class RowF>
-__device__ __forceinline__ bool gg_load_raw(uint32_t dst, int bytes, uint32_t align, int lane, const uint8_t* base,
-                                            const int (&piece)[9], bool near, RowF row_at) {
-  if constexpr (FMT == FB_FMT_IQ3_S) {
-    // 28 words from the word that holds the block's first byte (never one that starts behind the matrix)
+template <class RowF>
+__device__ __forceinline__ bool gg_load_iq4nl(uint32_t dst, int bytes, uint32_t align, int lane, const uint8_t* base,
+                                              const int (&piece)[9], bool near, RowF row_at) {
+  constexpr int P = GgRaw<FB_FMT_IQ4_NL, false>::kPitch;
+  if ((align & 15u) == 0 && bytes == P && near) {
+    // 16-byte pieces, nine per row: piece id -> shared-memory byte 16 id. `piece[i]` = where this lane's i-th piece
+    // lies from the first row's, the same for every round: recomputing it made the two loader warps, which get an
+    // issue slot every eight cycles or so, the pace of the kernel (2400 cycles per round).
 #pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      if (lane < 28)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + r * GgRaw<FMT, false>::kPitch + 4 * lane),
-                     "l"(row_at(r) + 4 * lane)
-                     : "memory");
-    }
-    return true;
+    for (int i = 0; i < 9; ++i)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * lane + 512 * i), "l"(base + piece[i]) : "memory");
+  } else if ((align & 7u) == 0) {
+    gg_copy_pieces<8>(dst, P, bytes, lane, row_at);
+  } else if ((align & 3u) == 0) {
+    gg_copy_pieces<4>(dst, P, bytes, lane, row_at);
   } else {
-    constexpr int P = GgRaw<FMT, false>::kPitch;
-    if ((align & 15u) == 0 && bytes == P && near) {
-      // 16-byte pieces, nine per row: piece id -> shared-memory byte 16 id. `piece[i]` = where this lane's i-th piece
-      // lies from the first row's, the same for every round: recomputing it made the two loader warps, which get an
-      // issue slot every eight cycles or so, the pace of the kernel (2400 cycles per round).
-#pragma unroll
-      for (int i = 0; i < 9; ++i)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * lane + 512 * i), "l"(base + piece[i]) : "memory");
-    } else if ((align & 7u) == 0) {
-      gg_copy_pieces<8>(dst, P, bytes, lane, row_at);
-    } else if ((align & 3u) == 0) {
-      gg_copy_pieces<4>(dst, P, bytes, lane, row_at);
-    } else {
-      const int per_row = bytes / 4;
-      for (int id = lane; id < 32 * per_row; id += 32) {
-        const int r = id / per_row, c = id - r * per_row;
-        const unsigned short* p = reinterpret_cast<const unsigned short*>(row_at(r) + 4 * c);
-        sts_u32<0>(dst + r * P + 4 * c, uint32_t(p[0]) | (uint32_t(p[1]) << 16));
-      }
-      return false;
+    const int per_row = bytes / 4;
+    for (int id = lane; id < 32 * per_row; id += 32) {
+      const int r = id / per_row, c = id - r * per_row;
+      const unsigned short* p = reinterpret_cast<const unsigned short*>(row_at(r) + 4 * c);
+      sts_u32<0>(dst + r * P + 4 * c, uint32_t(p[0]) | (uint32_t(p[1]) << 16));
     }
-    return true;
+    return false;
   }
+  return true;
 }
 
 // A stage of the token ring holds this many 64-wide K steps: 256 / n rounded down to 1, 2, 4 or 8. A unit of few tokens
@@ -543,19 +541,36 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
           const uint32_t s = rcount % R::kSlots;
           if (!(ok = ab.wait_warp(&bars->raw_empty[s], ((rcount / R::kSlots) & 1) ^ 1))) break;
           const int off = rd * R::kPiece;
-          const int bytes = min(R::kPitch, row_bytes - off);
-          const uint8_t *pg = rg + off, *pu = rup + off;
-          uint32_t align = uint32_t(reinterpret_cast<uintptr_t>(pg) | reinterpret_cast<uintptr_t>(pu)) | uint32_t(row_bytes);
-          if constexpr (kIq3s) {
-            pg -= reinterpret_cast<uintptr_t>(pg) & 3;
-            pu -= reinterpret_cast<uintptr_t>(pu) & 3;
-          }
+          const uint32_t slot = smem_u32(rawb) + s * R::kSlot + row0 * R::kPitch;
           bool async = true;
-          for (int hf = 0; hf < kRows / 32; ++hf) {
-            const uint32_t dst = smem_u32(rawb) + s * R::kSlot + (row0 + 32 * hf) * R::kPitch;
-            const uint8_t *p = pg + 16 * hf * row_bytes, *p2 = pu + 16 * hf * row_bytes;
-            async = gg_load_raw<FMT>(dst, bytes, align, lane, p, piece, near,
-                                     [&](int r) { return ((r & 1) ? p2 : p) + (r >> 1) * row_bytes; });
+          if constexpr (kIq3s) {
+            // lane = 16-byte word c of a block in row i of four; rows 4 k + i lie 4400 bytes apart, so they are cut alike
+            const int i = lane >> 3, c = lane & 7;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              const uint8_t* p = (m ? rup : rg) + off + i * row_bytes;
+              const int in = int(reinterpret_cast<uintptr_t>(p) & 15);
+              p += 16 * c - in;
+              if (16 * c < in + R::kPiece) {  // (no copy of 16 bytes without one of the block's)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                  for (int hf = 0; hf < kRows / 32; ++hf)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                 ::"r"(slot + 32 * hf * R::kPitch + (4 * (4 * m + k) + i) * 128 + 16 * (4 * m + k) + 16 * c),
+                                 "l"(p + (16 * hf + 4 * k) * row_bytes)
+                                 : "memory");
+              }
+            }
+          } else {
+            const int bytes = min(R::kPitch, row_bytes - off);
+            const uint8_t *pg = rg + off, *pu = rup + off;
+            const uint32_t align = uint32_t(reinterpret_cast<uintptr_t>(pg) | reinterpret_cast<uintptr_t>(pu)) | uint32_t(row_bytes);
+            for (int hf = 0; hf < kRows / 32; ++hf) {
+              const uint8_t *p = pg + 16 * hf * row_bytes, *p2 = pu + 16 * hf * row_bytes;
+              async = gg_load_iq4nl(slot + 32 * hf * R::kPitch, bytes, align, lane, p, piece, near,
+                                    [&](int r) { return ((r & 1) ? p2 : p) + (r >> 1) * row_bytes; });
+            }
           }
           if (async) cp_async_arrive_noinc(&bars->raw_full[s]);
           else mbar_arrive(&bars->raw_full[s]);
@@ -569,19 +584,21 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
     // decodes. In a group, a quarter's two warps take 128 K each. (Sixteen warps on every round ran in phase and waited
     // in phase; four groups on 128 K each double the hand-offs of the MMA thread, which then paces the kernel.)
     const int q = warp & 3, j = (warp - kGgFirstDecode) >> 2, grp = j >> 1;
-    const uint32_t raw_row = smem_u32(rawb) + (32 * q + lane) * (DOWN ? row_bytes : R::kPitch);
+    const uint32_t raw_row = smem_u32(rawb) + (!DOWN && kIq3s ? 32 * q * R::kPitch + gg_iq3s_slot_row(lane)
+                                                              : (32 * q + lane) * (DOWN ? row_bytes : R::kPitch));
     const uint32_t ta = tmem_base + (uint32_t(32 * q) << 16) + kGgABase + grp * 128;
     const uint32_t lane_table = smem_u32(table) + uint32_t(lane) * (kIq3s ? 2 : 4);
-    // gate/up: bytes from the covering word to the first block of the lane's row (IQ3_S: 0 or 2; rows are multiples of 4
-    // apart)
-    auto row_shift = [&](const int4& w) -> int {
+    // IQ3_S gate/up: where the lane's row begins in its first 16 bytes (units and lane quarters are multiples of four rows
+    // apart, which are multiples of 16 bytes)
+    auto row_start = [&](const int4& w) -> int {
       if constexpr (!kIq3s || DOWN) return 0;
-      return int(reinterpret_cast<uintptr_t>(blob_of(w.x) + ((lane & 1) ? A.L.up_offset : A.L.gate_offset))) & 3;
+      const int64_t at = ((lane & 1) ? A.L.up_offset : A.L.gate_offset) + ((lane >> 1) & 3) * row_bytes;
+      return int(reinterpret_cast<uintptr_t>(blob_of(w.x) + at)) & 15;
     };
     uint32_t r0 = 0, n = 0;  // rounds, units before this unit
     int4 un_next = unit_or_none(blockIdx.x);
     for (int u = blockIdx.x; u < n_units; u += gridDim.x, r0 += rounds, ++n) {
-      const int shift0 = row_shift(un_next);
+      const int start0 = row_start(un_next);
       un_next = unit_or_none(u + gridDim.x);
       bool ok = true;
       if constexpr (DOWN) {
@@ -590,9 +607,9 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
       for (int rd = (grp ^ int(r0)) & 1; rd < rounds; rd += 2) {
         const uint32_t rc = r0 + rd, rs = (DOWN ? n : rc) % R::kSlots, pa = ((rc / kGgAStages) & 1) ^ 1;
         const int m = (j ^ int(rc >> 1)) & 1;  // this warp's half of the round (a short round's only half changes hands)
-        const int at = DOWN ? rd * R::kPiece : 0;
+        const int at = DOWN ? rd * R::kPiece : kIq3s ? (start0 + rd * R::kPiece) & 15 : 0;
         const uint32_t row = raw_row + rs * R::kSlot + (at & ~3), tcol = ta + m * 64;
-        const int shift = DOWN ? at & 3 : (shift0 + rd * R::kPiece) & 3;
+        const int shift = at & 3;
         if constexpr (!DOWN) {
           if (!(ok = ab.wait_warp(&bars->raw_full[rs], (rc / R::kSlots) & 1))) break;
         }

@@ -454,3 +454,53 @@ def test_matrices_further_apart_than_31_bits(fg, fd, inter, up_first):
     apart.layout.gate_offset, apart.layout.up_offset = (far, 0) if up_first else (0, far)
     got = run_prefill(torch, apart, ws, logits, xd, T)
     assert ws.status() == 0 and torch.equal(got, y)
+
+
+@pytest.mark.parametrize("fg,fd,inter", [(IQ3_S, IQ3_S, 512), (IQ4_NL, IQ4_NL, 512), (IQ3_S, IQ4_NL, 640)])
+def test_token_boxes_and_gate_up_matrices_at_any_even_address(fg, fd, inter):
+    """Experts with 31 to 225 tokens (where the copies of token rows change their boxes) against fp64 products of the
+    bf16-rounded weights; then the same bits with the gate and up matrices at any even address, each cut differently into
+    16-byte words."""
+    torch = _torch()
+    from fngine_b200 import moe, prefill
+    counts = [31, 32, 33, 48, 96, 97, 192, 193, 225]
+    T, n_exp = 225, len(counts) + 9
+    layer = moe.synth_layer(fg, fd, inter, n_exp, 5152)
+    ws = prefill.PrefillWorkspace(T, inter)
+    lg = torch.from_numpy(edge_counts_logits(counts, T)).cuda()
+    xd = torch.from_numpy(synth.to_bf16_bits(synth.activations(44, T)).view(np.int16)).cuda().view(torch.bfloat16)
+    y = run_prefill(torch, layer, ws, lg, xd, T).clone()
+    off = ws.ints(ws.ws.expert_offset, 513)
+    assert [int(off[e + 1] - off[e]) for e in range(len(counts))] == counts
+    ptok = torch.from_numpy(ws.ints(ws.ws.pair_token, T * 10)).cuda().long()
+    pw = torch.from_numpy(ws.floats(ws.ws.pair_weight, T * 10)).cuda().double()
+    h = torch.from_numpy(synth.bf16_bits_to_f32(ws.h(T * 10))).cuda().double()
+    stride, gate = layer.layout.blob_stride, inter * O.row_bytes(fg, H)
+    want, room = torch.zeros(T, H, dtype=torch.float64, device="cuda"), torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for e in range(n_exp):
+        blob = layer.slots[e * stride:(e + 1) * stride]
+        wgu = moe.dequant_rows(fg, blob[:2 * gate], 2 * inter, H).to(torch.bfloat16).double()
+        wdn = moe.dequant_rows(fd, blob[2 * gate:], H, inter).to(torch.bfloat16).double()
+        p0, p1 = int(off[e]), int(off[e + 1])
+        acc = xd[ptok[p0:p1]].double() @ wgu.T
+        href = acc[:, :inter] / (1.0 + torch.exp(-acc[:, :inter])) * acc[:, inter:]
+        err = (h[p0:p1] - href).abs() / (href.abs() + 1e-2 * href.abs().amax(dim=1, keepdim=True))
+        assert float(err.max()) <= 2 ** -7, (e, float(err.max()))  # one bf16 step
+        want.index_add_(0, ptok[p0:p1], pw[p0:p1, None] * (h[p0:p1] @ wdn.T))
+        room.index_add_(0, ptok[p0:p1], pw[p0:p1, None] * (h[p0:p1].abs() @ wdn.abs().T))
+    # one unit in the last place of the sum of magnitudes for each of `inter` sums, the weight and ten additions
+    assert float(((y.double() - want).abs() / room).max()) <= (inter + 11) * 2.0 ** -23
+    blobs = layer.slots.view(n_exp, stride)
+    for g_at, u_at in ((6, 12), (10, 2), (14, 0), (0, 8)):
+        wide = stride + 64
+        buf = torch.zeros(n_exp * wide, dtype=torch.uint8, device="cuda")
+        rows = buf.view(n_exp, wide)
+        rows[:, g_at:g_at + gate] = blobs[:, :gate]
+        up = gate + 16 + u_at
+        rows[:, up:up + gate] = blobs[:, gate:2 * gate]
+        down = 2 * gate + 48
+        rows[:, down:down + stride - 2 * gate] = blobs[:, 2 * gate:]
+        apart = moe.ExpertLayer(buf, fg, fd, inter)
+        apart.layout.blob_stride, apart.layout.gate_offset, apart.layout.up_offset, apart.layout.down_offset = wide, g_at, up, down
+        got = run_prefill(torch, apart, ws, lg, xd, T)
+        assert ws.status() == 0 and torch.equal(got, y), (g_at, u_at)
