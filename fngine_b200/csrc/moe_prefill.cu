@@ -57,10 +57,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
       : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
@@ -409,32 +409,35 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// Rows of pairs as a 2-D bf16 tensor [pairs][width], boxes of 64 x 32, 128-byte swizzle; a box that reaches behind the
-// last pair reads the zero fill.
-int32_t rows_map(CUtensorMap* map, void* rows, int width, int capacity, const char* what) {
+// Rows of pairs as a bf16 tensor [K steps][pairs][64], 128-byte swizzle; a box that reaches behind the last pair or the last
+// K step reads the zero fill.
+int32_t rows_maps(GgMaps* maps, void* rows, int width, int capacity, const char* what) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) {
     set_error("%s: cuTensorMapEncodeTiled is not available", what);
     return int32_t(cudaErrorNotSupported);
   }
-  const cuuint64_t dims[2] = {cuuint64_t(width), cuuint64_t(size_t(capacity) * kTopK)};
-  const cuuint64_t strides[1] = {cuuint64_t(width) * 2};
-  const cuuint32_t box[2] = {cuuint32_t(kBK), cuuint32_t(kGgBox)};
-  const cuuint32_t elem[2] = {1, 1};
-  if (fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-    set_error("%s: cuTensorMapEncodeTiled failed", what);
-    return int32_t(cudaErrorInvalidValue);
+  static const cuuint32_t boxes[kBoxes][2] = {{32, 1}, {64, 1}, {128, 1}, {32, 8}, {64, 4}};
+  const cuuint64_t dims[3] = {cuuint64_t(kBK), cuuint64_t(size_t(capacity) * kTopK), cuuint64_t(width / kBK)};
+  const cuuint64_t strides[2] = {cuuint64_t(width) * 2, cuuint64_t(kBK) * 2};
+  const cuuint32_t elem[3] = {1, 1, 1};
+  for (int i = 0; i < kBoxes; ++i) {
+    const cuuint32_t box[3] = {cuuint32_t(kBK), boxes[i][0], boxes[i][1]};
+    if (fn(&maps->m[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, rows, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+      set_error("%s: cuTensorMapEncodeTiled failed", what);
+      return int32_t(cudaErrorInvalidValue);
+    }
   }
   return 0;
 }
 
 template <int FMT, bool DOWN>
-cudaError_t launch_grouped(const GgArgs& a, const CUtensorMap& map_b, cudaStream_t stream) {
+cudaError_t launch_grouped(const GgArgs& a, const GgMaps& maps, cudaStream_t stream) {
   static PerDeviceOnce once;
   const cudaError_t e = per_device_once(once, [] { return opt_in_smem(grouped_kernel<FMT, DOWN>, gg_smem<FMT, DOWN>()); });
   if (e != cudaSuccess) return e;
-  return launch_pdl(grouped_kernel<FMT, DOWN>, dim3(sm_count()), dim3(kGgThreads), size_t(gg_smem<FMT, DOWN>()), stream, a, map_b);
+  return launch_pdl(grouped_kernel<FMT, DOWN>, dim3(sm_count()), dim3(kGgThreads), size_t(gg_smem<FMT, DOWN>()), stream, a, maps);
 }
 
 // Offsets, token tiles and pair lists from the counts and the top-10 entries of `rows` tokens.
@@ -625,8 +628,8 @@ int32_t fb_moe_grouped_gate_up(const fb_moe_expert_layout* layout, const uint8_t
   // The token rows in pair order use the upper half of yp, which nothing needs before the down projection writes it
   // (the fixed-point sums, cleared by the route call, sit in its first fifth).
   auto* xg = reinterpret_cast<__nv_bfloat16*>(ws->yp + size_t(ws->capacity) * kTopK * (H / 2));
-  CUtensorMap map_b;
-  if (const int32_t st = rows_map(&map_b, xg, H, ws->capacity, "grouped_gate_up")) return st;
+  GgMaps maps;
+  if (const int32_t st = rows_maps(&maps, xg, H, ws->capacity, "grouped_gate_up")) return st;
   // a few tokens: a fifth of a row per warp, so that there are enough of them (9.3 us at 96 tokens with whole rows)
   const int parts = tokens <= 1024 ? 5 : 1;
   cudaError_t e = launch_pdl(parts == 5 ? scatter_rows_kernel<5> : scatter_rows_kernel<1>, dim3((tokens * parts + 3) / 4),
@@ -643,8 +646,8 @@ int32_t fb_moe_grouped_gate_up(const fb_moe_expert_layout* layout, const uint8_t
   a.n_units = ws->meta;
   a.h = static_cast<__nv_bfloat16*>(ws->h);
   a.status = ws->status;
-  e = layout->gate_up_format == FB_FMT_IQ3_S ? launch_grouped<FB_FMT_IQ3_S, false>(a, map_b, as_stream(stream))
-                                             : launch_grouped<FB_FMT_IQ4_NL, false>(a, map_b, as_stream(stream));
+  e = layout->gate_up_format == FB_FMT_IQ3_S ? launch_grouped<FB_FMT_IQ3_S, false>(a, maps, as_stream(stream))
+                                             : launch_grouped<FB_FMT_IQ4_NL, false>(a, maps, as_stream(stream));
   if (e != cudaSuccess) {
     set_error("grouped_gate_up: %s", cudaGetErrorString(e));
     return int32_t(e);
@@ -656,8 +659,8 @@ int32_t fb_moe_grouped_down(const fb_moe_expert_layout* layout, const uint8_t* c
                             const fb_moe_prefill_workspace* ws, void* stream) {
   if (!pf_layout_ok(layout, expert_blob) || !pf_ws_ok(ws, tokens) || layout->inter != ws->inter)
     return invalid("grouped_down: bad arguments");
-  CUtensorMap map_b;
-  if (const int32_t st = rows_map(&map_b, ws->h, ws->inter, ws->capacity, "grouped_down")) return st;
+  GgMaps maps;
+  if (const int32_t st = rows_maps(&maps, ws->h, ws->inter, ws->capacity, "grouped_down")) return st;
   GgArgs a{};
   a.L = *layout;
   a.expert_blob = expert_blob;
@@ -669,8 +672,8 @@ int32_t fb_moe_grouped_down(const fb_moe_expert_layout* layout, const uint8_t* c
   a.y_fixed = g_prefill_fixed ? reinterpret_cast<unsigned long long*>(ws->yp) : nullptr;
   a.status = ws->status;
   const cudaError_t e = layout->down_format == FB_FMT_IQ3_S
-                            ? launch_grouped<FB_FMT_IQ3_S, true>(a, map_b, as_stream(stream))
-                            : launch_grouped<FB_FMT_IQ4_NL, true>(a, map_b, as_stream(stream));
+                            ? launch_grouped<FB_FMT_IQ3_S, true>(a, maps, as_stream(stream))
+                            : launch_grouped<FB_FMT_IQ4_NL, true>(a, maps, as_stream(stream));
   if (e != cudaSuccess) {
     set_error("grouped_down: %s", cudaGetErrorString(e));
     return int32_t(e);

@@ -27,7 +27,12 @@ constexpr int kGgRawWarps = 2, kGgDecodeWarps = 16, kGgEpiWarps = 8;
 constexpr int kGgFirstDecode = 2 + kGgRawWarps, kGgFirstEpi = kGgFirstDecode + kGgDecodeWarps;
 constexpr int kGgThreads = (kGgFirstEpi + kGgEpiWarps) * 32;
 constexpr int kGgABase = 256;  // first tensor-memory column of the A slots
-constexpr int kGgBox = 32;     // token (h) rows per TMA box
+// TMA boxes of token (h) rows x K steps: a stage of one or two K steps is filled with the fewest boxes of 128, 64 and 32
+// rows, a stage of four or eight steps by one box.
+enum { kBox32, kBox64, kBox128, kBox32x8, kBox64x4, kBoxes };
+struct GgMaps {
+  CUtensorMap m[kBoxes];
+};
 
 struct GgBars {
   uint64_t b_full[kGgBStages], b_empty[kGgBStages];
@@ -310,6 +315,8 @@ __device__ __forceinline__ bool gg_load_iq4nl(uint32_t dst, int bytes, uint32_t 
 // A stage of the token ring holds this many 64-wide K steps: 256 / n rounded down to 1, 2, 4 or 8. A unit of few tokens
 // then takes one hand-off per 512 K instead of eight: a wait costs the MMA thread a few hundred cycles, as much as a
 // whole K step of such a unit.
+// (What a copy costs is the issuing thread's instructions: its warp gets an issue slot every eight cycles or so beside the
+// decoding ones, and eight boxes of one K step each took it 2000 cycles, more than the 512 K they feed.)
 __device__ __forceinline__ int gg_b_steps(int n) { return n <= 32 ? 8 : n <= 64 ? 4 : n <= 128 ? 2 : 1; }
 
 struct GgArgs {
@@ -327,7 +334,7 @@ struct GgArgs {
 
 template <int FMT, bool DOWN>
 __global__ void __launch_bounds__(kGgThreads, 1)
-grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
+grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
   using R = GgRaw<FMT, DOWN>;
   constexpr bool kIq3s = FMT == FB_FMT_IQ3_S;
   extern __shared__ uint8_t smem_raw[];
@@ -402,64 +409,67 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
   if (warp == 0) {
     // ---------------- MMA issuer. A unit of at most 128 tokens takes one of two 128-column accumulators, so its
     // epilogue overlaps the next unit's K loop; a wider unit takes both.
+    // (Its instructions are on the path from hand-off to hand-off, an issue slot every eight cycles or so: the loop exists once
+    // for every number of K steps a token stage holds, with all addresses a constant away from two. With the token rows in
+    // few boxes, a layer of 1003 tokens went from 507 to 484 us, of 8192 from 1259 to 1240.)
     if (elect_one()) {
       const uint32_t ring_lo = umma_desc_lo_k128(smem_u32(ringb));
-      uint32_t ra = 0, sbc = 0, use0 = 0, use1 = 0, nb = 0;
+      uint32_t sa = 0, pa = 0, sb = 0, pb = 0;  // A and token stage, their phases
+      uint32_t use0 = 0, use1 = 0, nb = 0;
+      bool ok = true;
+      auto unit = [&](auto steps_per_stage, uint32_t dcol, uint32_t idesc) {
+        constexpr int S = decltype(steps_per_stage)::value, kGroup = S < 4 ? S : 4;  // K steps from one wait to the next
+        constexpr uint32_t kStep = (kTileB >> 4) / S;                               // descriptor distance of K steps
+        for (int rd = 0; rd < rounds; ++rd) {
+          const int steps = min(4, k_steps - 4 * rd);
+          const uint32_t la = tmem_base + kGgABase + sa * 128;
+#pragma unroll
+          for (int k = 0; k < 4; k += kGroup) {
+            if (k >= steps) break;
+            if (S < 8 || (rd & 1) == 0) {
+              if (!(ok = ab.wait(&bars->b_full[sb], pb))) return;
+            }
+            if (k == 0 && !(ok = ab.wait(&bars->a_full[sa], pa))) return;  // (the later of the two)
+            tc_fence_after();
+            const uint32_t lb = ring_lo + sb * (kTileB >> 4) + (S == 8 ? (rd & 1) * (4 * kStep) : 0u);
+            {
+#pragma unroll
+              for (int i = 0; i < kGroup; ++i) {
+                if (kGroup > 2 && i >= steps) break;
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4)
+                  umma_bf16_ts(dcol, la + 32 * (k + i) + 8 * k4, lb + i * kStep + 2 * k4, idesc, k + i + k4 ? 1u : uint32_t(rd));
+              }
+              if (S < 8 || (rd & 1) || rd == rounds - 1) umma_commit(&bars->b_empty[sb]);
+            }
+            if (S < 8 || (rd & 1) || rd == rounds - 1) {
+              if (++sb == kGgBStages) {
+                sb = 0;
+                pb ^= 1u;
+              }
+            }
+          }
+          umma_commit(&bars->a_empty[sa]);
+          pa ^= sa;
+          sa ^= 1u;
+        }
+      };
       int tokens = unit_or_none(blockIdx.x).w;
       for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
         const int n = (tokens + 15) & ~15;
         tokens = unit_or_none(u + gridDim.x).w;
         const bool wide = n > 128;
         const uint32_t idesc = idesc_bf16(n);
-        bool ok = true;
         if (wide || nb == 0) ok = ab.wait(&bars->acc_empty[0], (use0 & 1) ^ 1);
         if (ok && (wide || nb == 1)) ok = ab.wait(&bars->acc_empty[1], (use1 & 1) ^ 1);
         if (!ok) break;
         tc_fence_after();
         const uint32_t dcol = tmem_base + (wide ? 0u : nb * 128u);
         const int S = gg_b_steps(n);
-        const uint32_t b_step = (kTileB >> 4) / S;  // descriptor distance of a stage's K steps
-        int in_stage = 0;                           // steps used of the current stage
-        for (int rd = 0; rd < rounds; ++rd, ++ra) {
-          const uint32_t sa = ra % kGgAStages;
-          const int steps = min(4, k_steps - 4 * rd);
-          uint32_t la = tmem_base + kGgABase + sa * 128;
-          for (int k = 0; k < steps;) {
-            const uint32_t sb = sbc % kGgBStages;
-            if (in_stage == 0 && !(ok = ab.wait(&bars->b_full[sb], (sbc / kGgBStages) & 1))) break;
-            if (k == 0 && !(ok = ab.wait(&bars->a_full[sa], (ra / kGgAStages) & 1))) break;  // (the later of the two)
-            tc_fence_after();
-            uint32_t lb = ring_lo + sb * (kTileB >> 4) + in_stage * b_step;
-            if (S >= 4) {  // the round's steps lie in one stage, and a stage of eight lasts for two rounds
-              if (steps == 4) {  // (unrolled: fewer instructions per MMA)
-#pragma unroll
-                for (int i = 0; i < 4; ++i, lb += b_step)
-#pragma unroll
-                  for (int k4 = 0; k4 < 4; ++k4)
-                    umma_bf16_ts(dcol, la + 32 * i + 8 * k4, lb + 2 * k4, idesc, (rd | i | k4) ? 1u : 0u);
-              } else {
-                for (int i = 0; i < steps; ++i, la += 32, lb += b_step)
-#pragma unroll
-                  for (int k4 = 0; k4 < 4; ++k4)
-                    umma_bf16_ts(dcol, la + 8 * k4, lb + 2 * k4, idesc, (rd | i | k4) ? 1u : 0u);
-              }
-              k = steps;
-              in_stage += steps;
-              if (in_stage < S && 4 * rd + steps < k_steps) continue;  // (= the round's end)
-              in_stage = 0;
-            } else {
-              for (int k1 = min(k + S, steps); k < k1; ++k, la += 32, lb += b_step) {
-                umma_bf16_ts(dcol, la, lb, idesc, (rd | k) ? 1u : 0u);
-#pragma unroll
-                for (int k4 = 1; k4 < 4; ++k4) umma_bf16_ts(dcol, la + 8 * k4, lb + 2 * k4, idesc, 1u);
-              }
-            }
-            umma_commit(&bars->b_empty[sb]);
-            ++sbc;
-          }
-          if (!ok) break;
-          umma_commit(&bars->a_empty[sa]);
-        }
+        if (S == 8) unit(std::integral_constant<int, 8>{}, dcol, idesc);
+        else if (S == 4) unit(std::integral_constant<int, 4>{}, dcol, idesc);
+        else if (S == 2) unit(std::integral_constant<int, 2>{}, dcol, idesc);
+        else unit(std::integral_constant<int, 1>{}, dcol, idesc);
         if (!ok) break;
         if (wide || nb == 0) { umma_commit(&bars->acc_full[0]); ++use0; }
         if (wide || nb == 1) { umma_commit(&bars->acc_full[1]); ++use1; }
@@ -467,24 +477,36 @@ grouped_kernel(const GgArgs A, const __grid_constant__ CUtensorMap map_b) {
       }
     }
   } else if (warp == 1) {
-    // ---------------- token (h) rows of the unit's pairs: boxes of 32 rows by TMA (one thread)
+    // ---------------- token (h) rows of the unit's pairs by TMA (one thread)
     if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       int4 un = unit_or_none(blockIdx.x), un_next;
       for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, un = un_next) {
         un_next = unit_or_none(u + gridDim.x);
-        const int boxes = (un.w + kGgBox - 1) / kGgBox;
         const int S = gg_b_steps((un.w + 15) & ~15);
+        const int rows = (un.w + 31) & ~31;
         for (int k0 = 0; k0 < k_steps; k0 += S, ++it) {
           const uint32_t s = it % kGgBStages;
           if (!(ok = ab.wait(&bars->b_empty[s], ((it / kGgBStages) & 1) ^ 1))) break;
-          const int k1 = min(k0 + S, k_steps);
-          mbar_expect_tx(&bars->b_full[s], uint32_t((k1 - k0) * boxes) * (kGgBox * 128));
-          for (int k = k0; k < k1; ++k)
-            for (int b = 0; b < boxes; ++b)
-              tma_load_2d(ringb + s * kTileB + (k - k0) * (kTileB / S) + b * (kGgBox * 128), &map_b, k * kBK,
-                          un.z + b * kGgBox, &bars->b_full[s]);
+          uint64_t* full = &bars->b_full[s];
+          uint8_t* dst = ringb + s * kTileB;
+          if (S >= 4) {  // (steps behind the last one are filled with zeros and not used)
+            mbar_expect_tx(full, kTileB);
+            tma_load_3d(dst, &maps.m[S == 8 ? kBox32x8 : kBox64x4], 0, un.z, k0, full);
+          } else {
+            const int k1 = min(k0 + S, k_steps);
+            mbar_expect_tx(full, uint32_t((k1 - k0) * rows) * 128);
+            for (int k = k0; k < k1; ++k, dst += kTileB / 2) {
+              int r = 0;
+              for (; rows - r >= 128; r += 128) tma_load_3d(dst + r * 128, &maps.m[kBox128], 0, un.z + r, k, full);
+              if (rows - r >= 64) {
+                tma_load_3d(dst + r * 128, &maps.m[kBox64], 0, un.z + r, k, full);
+                r += 64;
+              }
+              if (rows > r) tma_load_3d(dst + r * 128, &maps.m[kBox32], 0, un.z + r, k, full);
+            }
+          }
         }
       }
     }
