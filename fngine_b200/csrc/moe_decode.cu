@@ -191,15 +191,17 @@ __global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* w, int
 
 // The same logits, bit for bit, at prefill width (tokens > kMaxTok). Bound: the fp32 pipe (tokens x rows x 2560
 // multiply-adds). router_kernel above re-reads x for every row and keeps four tokens in flight: 0.96 us per token,
-// 963 us at 1003 tokens; this kernel takes 103 us there (fp32 pipe 43 % busy, 3.7 waves of blocks).
+// 963 us at 1003 tokens; this kernel takes 90 us there (3.7 waves of blocks).
 // A block owns 32 rows (ROWS) x 32 tokens; its sixteen warps split K the way router_kernel's lanes do: the partial sum of
 // lane l (elements 256 c + 8 l + i, added over c, then i) belongs to warp l mod 16, which adds those of lanes l and
-// l + 16; the sixteen results meet in shared memory in the butterfly's order. A thread accumulates 8 rows x 4 tokens
-// in packed pairs of rows (fma.rn.f32x2: two multiply-adds per instruction, each rounded as fmaf is). 256-wide K
-// chunks lie row-major in three cp.async buffers, rows 16 bytes apart modulo the banks: one 16-byte load brings a
-// row's eight elements of a lane class, and the widening to fp32 (a shift or a mask) shares the issue slots that the
-// packed multiply-adds leave. (A K-major copy in fp32, widened while staging, took 142 us: its global loads touched
-// 32 rows per instruction.)
+// l + 16; the sixteen results meet in shared memory in the butterfly's order. A thread accumulates 8 rows x 4 tokens. bf16
+// activations: multiply-adds of two bf16 numbers into fp32, which take the halves of the packed words as they lie (one
+// rounding, as fmaf). What bounds it is their three register operands: an instruction takes some 1.5 cycles of a scheduler.
+// Packed fp32 multiply-adds of widened values (fma.rn.f32x2, half the instructions, and as many again to widen) took 103 us,
+// values widened on their way into shared memory 103, half-warps on a lane class each with 8 x 8 values per thread 100.
+// fp32 activations: packed pairs of rows. 256-wide K chunks lie row-major in three cp.async buffers, rows 16 bytes apart
+// modulo the banks: one 16-byte load brings a row's eight elements of a lane class. (A K-major copy in fp32, widened while
+// staging, took 142 us: its global loads touched 32 rows per instruction.)
 // ROWS (32, 16 or 8): few tokens do not fill the GPU with tiles of 32 rows, and a block's time follows its rows; see
 // fb_router_logits.
 constexpr int kRtTok = 32, kRtChunk = 256, kRtBufs = 3;
@@ -216,6 +218,13 @@ constexpr int router_tile_smem() {
 
 __device__ __forceinline__ void fma_f32x2(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+// acc += lo(w) lo(x), then hi(w) hi(x), of bf16 pairs
+__device__ __forceinline__ void fma_bf16_pair(float& acc, uint32_t w, uint32_t x) {
+  asm("{\n\t.reg .b16 wl, wh, xl, xh;\n\tmov.b32 {wl, wh}, %1;\n\tmov.b32 {xl, xh}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, wl, xl, %0;\n\tfma.rn.f32.bf16 %0, wh, xh, %0;\n\t}"
+      : "+f"(acc)
+      : "r"(w), "r"(x));
 }
 __device__ __forceinline__ uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
   uint64_t d;
@@ -254,13 +263,14 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // thread = rows rg + 4 j (j = 0..ROWS / 4 - 1, pairs of neighbouring j) x tokens tg + 8 t (t = 0..3)
+  // thread = rows rg + 4 j (j = 0..ROWS / 4 - 1; fp32: pairs of neighbouring j) x tokens tg + 8 t (t = 0..3)
   const int rg = lane >> 3, tg = lane & 7;
-  uint64_t acc[2][ROWS / 8][4];  // [lane class warp, warp + 16][row pair][token]
+  constexpr int kAcc = XBF16 ? ROWS / 4 : ROWS / 8;
+  std::conditional_t<XBF16, float, uint64_t> acc[2][kAcc][4];  // [lane class warp, warp + 16][row or row pair][token]
 #pragma unroll
   for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int r = 0; r < ROWS / 8; ++r)
+    for (int r = 0; r < kAcc; ++r)
 #pragma unroll
       for (int t = 0; t < 4; ++t) acc[c][r][t] = 0;
   fetch(0);
@@ -271,48 +281,69 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
     __syncthreads();  // chunk c is in place, and nobody reads the buffer that the next fetch fills
     if (c + 2 < kChunks) fetch(c + 2);
     const uint8_t* buf = smem + (c % kRtBufs) * kBuf;
+    if constexpr (XBF16) {
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-      const int cls = ch >> 1, e = 4 * (ch & 1);
-      const int piece = warp + 16 * cls;  // elements 8 piece + e .. + 3 of the chunk
-      uint64_t xx[4][4];                  // token values, both halves alike: made once, used by four row pairs
+      for (int cls = 0; cls < 2; ++cls) {
+        const int piece = warp + 16 * cls;  // elements 8 piece .. + 7 of the chunk
+        uint4 x[4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint8_t* xp = buf + ROWS * kRtWPitch + (tg + 8 * t) * kXPitch + (8 * piece + e) * (XBF16 ? 2 : 4);
-        uint32_t v[4];
-        if constexpr (XBF16) {
-          const uint2 a = *reinterpret_cast<const uint2*>(xp);
-          v[0] = a.x << 16; v[1] = a.x & 0xFFFF0000u; v[2] = a.y << 16; v[3] = a.y & 0xFFFF0000u;
-        } else {
-          const uint4 a = *reinterpret_cast<const uint4*>(xp);
-          v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        for (int t = 0; t < 4; ++t)
+          x[t] = *reinterpret_cast<const uint4*>(buf + ROWS * kRtWPitch + (tg + 8 * t) * kXPitch + 16 * piece);
+#pragma unroll
+        for (int r = 0; r < ROWS / 4; ++r) {
+          const uint4 wv = *reinterpret_cast<const uint4*>(buf + (rg + 4 * r) * kRtWPitch + 16 * piece);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            fma_bf16_pair(acc[cls][r][t], wv.x, x[t].x);
+            fma_bf16_pair(acc[cls][r][t], wv.y, x[t].y);
+            fma_bf16_pair(acc[cls][r][t], wv.z, x[t].z);
+            fma_bf16_pair(acc[cls][r][t], wv.w, x[t].w);
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) {
+        const int cls = ch >> 1, e = 4 * (ch & 1);
+        const int piece = warp + 16 * cls;  // elements 8 piece + e .. + 3 of the chunk
+        uint64_t xx[4][4];                  // token values, both halves alike: made once, used by four row pairs
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const uint8_t* xp = buf + ROWS * kRtWPitch + (tg + 8 * t) * kXPitch + (8 * piece + e) * 4;
+          const uint4 v = *reinterpret_cast<const uint4*>(xp);
+          xx[t][0] = pack_f32x2(v.x, v.x);
+          xx[t][1] = pack_f32x2(v.y, v.y);
+          xx[t][2] = pack_f32x2(v.z, v.z);
+          xx[t][3] = pack_f32x2(v.w, v.w);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) xx[t][i] = pack_f32x2(v[i], v[i]);
-      }
+        for (int r = 0; r < ROWS / 8; ++r) {
+          const uint2 a = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r) * kRtWPitch + 16 * piece + 2 * e);
+          const uint2 b = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r + 4) * kRtWPitch + 16 * piece + 2 * e);
+          const uint64_t wp[4] = {pack_f32x2(a.x << 16, b.x << 16), pack_f32x2(a.x & 0xFFFF0000u, b.x & 0xFFFF0000u),
+                                  pack_f32x2(a.y << 16, b.y << 16), pack_f32x2(a.y & 0xFFFF0000u, b.y & 0xFFFF0000u)};
 #pragma unroll
-      for (int r = 0; r < ROWS / 8; ++r) {
-        const uint2 a = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r) * kRtWPitch + 16 * piece + 2 * e);
-        const uint2 b = *reinterpret_cast<const uint2*>(buf + (rg + 8 * r + 4) * kRtWPitch + 16 * piece + 2 * e);
-        const uint64_t wp[4] = {pack_f32x2(a.x << 16, b.x << 16), pack_f32x2(a.x & 0xFFFF0000u, b.x & 0xFFFF0000u),
-                                pack_f32x2(a.y << 16, b.y << 16), pack_f32x2(a.y & 0xFFFF0000u, b.y & 0xFFFF0000u)};
+          for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int t = 0; t < 4; ++t) fma_f32x2(acc[cls][r][t], wp[i], xx[t][i]);
+            for (int t = 0; t < 4; ++t) fma_f32x2(acc[cls][r][t], wp[i], xx[t][i]);
+        }
       }
     }
   }
   __syncthreads();
   float* part = reinterpret_cast<float*>(smem);  // [warp][token][row]
 #pragma unroll
-  for (int r = 0; r < ROWS / 8; ++r)
+  for (int r = 0; r < kAcc; ++r)
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const float2 a = *reinterpret_cast<const float2*>(&acc[0][r][t]), b = *reinterpret_cast<const float2*>(&acc[1][r][t]);
-      float* q = part + (warp * kRtTok + tg + 8 * t) * ROWS + rg + 8 * r;
-      q[0] = a.x + b.x;
-      q[4] = a.y + b.y;
+      float* q = part + (warp * kRtTok + tg + 8 * t) * ROWS + rg;
+      if constexpr (XBF16) {
+        q[4 * r] = acc[0][r][t] + acc[1][r][t];
+      } else {
+        const float2 a = *reinterpret_cast<const float2*>(&acc[0][r][t]), b = *reinterpret_cast<const float2*>(&acc[1][r][t]);
+        q[8 * r] = a.x + b.x;
+        q[8 * r + 4] = a.y + b.y;
+      }
     }
   __syncthreads();
   for (int o = tid; o < ROWS * kRtTok; o += 512) {
