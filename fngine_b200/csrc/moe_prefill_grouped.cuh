@@ -332,6 +332,41 @@ struct GgArgs {
   uint32_t* status;
 };
 
+// SwiGLU of the accumulators of one lane quarter, chunks of 16 tokens from `chunk0` on, into rows of h. Even lanes hold gate
+// rows, odd lanes the matching up rows: an even lane finishes tokens 0..7 of a chunk, its neighbour tokens 8..15. A unit of 256
+// tokens waits for this with its accumulators (the next one needs both), so the path is short: constant row distances, no
+// bounds checks in whole chunks, exponential and reciprocal as the hardware gives them (their error, a few fp32 ulp, is far
+// below the bf16 step of h).
+template <int I>
+__device__ __forceinline__ void gg_store_h(__nv_bfloat16* h, const int4& un, int q, int lane, int chunk0, uint32_t dcol) {
+  const bool odd = (lane & 1) != 0;
+  const int first = odd ? 8 : 0;
+  for (int c0 = chunk0; c0 < un.w; c0 += 4 * kGgEpiWarps) {
+    uint32_t r[16];
+    tmem_ld16(dcol + uint32_t(c0), r);
+    tmem_ld_wait();
+    __nv_bfloat16* out = h + size_t(un.z + c0 + first) * I + un.y + 16 * q + (lane >> 1);
+    __nv_bfloat16 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? r[i] : r[8 + i], 1);
+      const float gv = __uint_as_float(odd ? got : r[i]), uv = __uint_as_float(odd ? r[8 + i] : got);
+      float e, d;
+      asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(gv * -1.4426950408889634f));
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(1.0f + e));
+      v[i] = __float2bfloat16_rn(gv * d * uv);
+    }
+    if (c0 + 16 <= un.w) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out[i * I] = v[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + first + i < un.w) out[i * I] = v[i];
+    }
+  }
+}
+
 template <int FMT, bool DOWN>
 __global__ void __launch_bounds__(kGgThreads, 1)
 grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
@@ -685,25 +720,14 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
       if (!ok) break;
       tc_fence_after();
       const uint32_t dcol = tmem_base + (uint32_t(32 * q) << 16) + (wide ? 0u : nb * 128u);
-      for (int c0 = chunk0; c0 < un.w; c0 += 4 * kGgEpiWarps) {
-        uint32_t r[16];
-        tmem_ld16(dcol + uint32_t(c0), r);
-        tmem_ld_wait();
-        if constexpr (!DOWN) {
-          // even lanes hold gate rows, odd lanes the matching up rows: an even lane finishes tokens 0..7 of the chunk,
-          // its neighbour tokens 8..15
-          const bool odd = (lane & 1) != 0;
-          const int j = un.y + 16 * q + (lane >> 1);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? r[i] : r[8 + i], 1);
-            const float gv = __uint_as_float(odd ? got : r[i]), uv = __uint_as_float(odd ? r[8 + i] : got);
-            const int t = c0 + i + (odd ? 8 : 0);
-            // silu(g) * u; fast exp and divide: their error (a few fp32 ulp) is far below the bf16 step of h
-            const float hv = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
-            if (t < un.w) A.h[size_t(un.z + t) * I + j] = __float2bfloat16_rn(hv);
-          }
-        } else {
+      if constexpr (!DOWN) {
+        if (I == 512) gg_store_h<512>(A.h, un, q, lane, chunk0, dcol);
+        else gg_store_h<640>(A.h, un, q, lane, chunk0, dcol);
+      } else {
+        for (int c0 = chunk0; c0 < un.w; c0 += 4 * kGgEpiWarps) {
+          uint32_t r[16];
+          tmem_ld16(dcol + uint32_t(c0), r);
+          tmem_ld_wait();
           const int n = un.y + 32 * q + lane;
           if (A.y_fixed) {  // the reference's accumulation (src/kernels/moe/moe.h:186-192): y_fixed[token] += fixed(w * v)
 #pragma unroll
