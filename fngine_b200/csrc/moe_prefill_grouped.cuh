@@ -22,7 +22,7 @@
 // All hand-offs are mbarriers with bounded waits.
 #pragma once
 
-constexpr int kGgBStages = 3, kGgAStages = 2, kGgMaxRawSlots = 6;
+constexpr int kGgAStages = 2, kGgMaxRawSlots = 5, kGgMaxBStages = 4;
 constexpr int kGgRawWarps = 2, kGgDecodeWarps = 16, kGgEpiWarps = 8;
 constexpr int kGgFirstDecode = 2 + kGgRawWarps, kGgFirstEpi = kGgFirstDecode + kGgDecodeWarps;
 constexpr int kGgThreads = (kGgFirstEpi + kGgEpiWarps) * 32;
@@ -35,7 +35,7 @@ struct GgMaps {
 };
 
 struct GgBars {
-  uint64_t b_full[kGgBStages], b_empty[kGgBStages];
+  uint64_t b_full[kGgMaxBStages], b_empty[kGgMaxBStages];
   uint64_t a_full[kGgAStages], a_empty[kGgAStages];
   uint64_t raw_full[kGgMaxRawSlots], raw_empty[kGgMaxRawSlots];
   uint64_t acc_full[2], acc_empty[2];
@@ -51,6 +51,9 @@ static __constant__ int8_t c_iq4nl_levels[16] = {FB_IQ4NL_LEVELS};
 //   warps alone needed 200 us for gate/up of 96 tokens, which went from 241 to 213 us). Rows lie 1100 bytes apart, so a block starts at word 0..3 of its first 16 bytes,
 //   by turns; the rows of 32 lanes are laid out so that the same word of their blocks meets 32 banks (gg_iq3s_slot_row).
 //   IQ4_NL: 144 bytes, back to back (16-byte reads of eight neighbouring rows cover all banks).
+//   kBStages: token stages of 32 KB. A unit of 256 tokens drains one in 512 cycles, and the L2 answers later than three of them
+//   last: with the fourth in the place of a raw slot a layer of 8192 IQ3_S tokens went from 1216 to 1192 us. (With three raw
+//   slots gate/up of 96 tokens lost 7 to 15 %: IQ4_NL, whose raw slots are larger, keeps three token stages.)
 // down: a slot = the whole unit, 128 complete rows, which lie back to back in the matrix: one bulk copy. (Cut into pieces like
 //   gate/up, rows of 360 bytes came in 8-byte copies, and the copying warps were the pace: 382 us instead of 233 at 1003
 //   tokens.)
@@ -58,19 +61,19 @@ template <int FMT, bool DOWN>
 struct GgRaw;
 template <>
 struct GgRaw<FB_FMT_IQ3_S, false> {
-  static constexpr int kPiece = 110, kPitch = 132, kSlots = 5, kSlot = kTileM * kPitch;  // (128 + 16 bytes per four rows)
+  static constexpr int kPiece = 110, kPitch = 132, kSlots = 4, kSlot = kTileM * kPitch, kBStages = 4;  // (128 + 16 bytes per four rows)
 };
 template <>
 struct GgRaw<FB_FMT_IQ4_NL, false> {
-  static constexpr int kPiece = 144, kPitch = 144, kSlots = 5, kSlot = kTileM * kPitch;
+  static constexpr int kPiece = 144, kPitch = 144, kSlots = 5, kSlot = kTileM * kPitch, kBStages = 3;
 };
 template <>
 struct GgRaw<FB_FMT_IQ3_S, true> {
-  static constexpr int kPiece = 110, kPitch = 220, kSlots = 3, kSlot = kTileM * kPitch;  // (intermediate 512 only)
+  static constexpr int kPiece = 110, kPitch = 220, kSlots = 3, kSlot = kTileM * kPitch, kBStages = 3;  // (intermediate 512 only)
 };
 template <>
 struct GgRaw<FB_FMT_IQ4_NL, true> {
-  static constexpr int kPiece = 144, kPitch = 360, kSlots = 2, kSlot = kTileM * kPitch;  // (288-byte rows: pitch 288)
+  static constexpr int kPiece = 144, kPitch = 360, kSlots = 2, kSlot = kTileM * kPitch, kBStages = 3;  // (288-byte rows: pitch 288)
 };
 // IQ3_S selectors (of an entry's weights 3, 2, 1, 0), 16 bits per index and lane: entry i of lane l at byte 64 i + 2 l. Two
 // lanes share a bank, so a warp's look-up takes two passes at most where one shared copy takes three to four.
@@ -79,7 +82,7 @@ template <int FMT>
 constexpr int kGgTableBytes = FMT == FB_FMT_IQ3_S ? 512 * 64 : 256 * 128;
 template <int FMT, bool DOWN>
 constexpr int gg_smem() {
-  return 1024 + kGgBStages * kTileB + GgRaw<FMT, DOWN>::kSlots * GgRaw<FMT, DOWN>::kSlot + kGgTableBytes<FMT> +
+  return GgRaw<FMT, DOWN>::kBStages * kTileB + GgRaw<FMT, DOWN>::kSlots * GgRaw<FMT, DOWN>::kSlot + kGgTableBytes<FMT> +
          int(sizeof(GgBars)) + 64;
 }
 static_assert(gg_smem<FB_FMT_IQ3_S, false>() <= 232448 && gg_smem<FB_FMT_IQ4_NL, false>() <= 232448 &&
@@ -372,10 +375,10 @@ __global__ void __launch_bounds__(kGgThreads, 1)
 grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
   using R = GgRaw<FMT, DOWN>;
   constexpr bool kIq3s = FMT == FB_FMT_IQ3_S;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* ringb = smem;
-  uint8_t* rawb = smem + kGgBStages * kTileB;
+  constexpr int kBStages = R::kBStages;
+  extern __shared__ __align__(1024) uint8_t gg_smem_base[];  // (operand tiles start on swizzle atoms)
+  uint8_t* ringb = gg_smem_base;
+  uint8_t* rawb = ringb + kBStages * kTileB;
   uint8_t* table = rawb + R::kSlots * R::kSlot;
   GgBars* bars = reinterpret_cast<GgBars*>(table + kGgTableBytes<FMT>);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -402,7 +405,7 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
     }
   }
   if (tid == 0) {
-    for (int i = 0; i < kGgBStages; ++i) {
+    for (int i = 0; i < kBStages; ++i) {
       mbar_init(&bars->b_full[i], 1);
       mbar_init(&bars->b_empty[i], 1);
     }
@@ -478,7 +481,7 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
               if (S < 8 || (rd & 1) || rd == rounds - 1) umma_commit(&bars->b_empty[sb]);
             }
             if (S < 8 || (rd & 1) || rd == rounds - 1) {
-              if (++sb == kGgBStages) {
+              if (++sb == kBStages) {
                 sb = 0;
                 pb ^= 1u;
               }
@@ -522,8 +525,8 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
         const int S = gg_b_steps((un.w + 15) & ~15);
         const int rows = (un.w + 31) & ~31;
         for (int k0 = 0; k0 < k_steps; k0 += S, ++it) {
-          const uint32_t s = it % kGgBStages;
-          if (!(ok = ab.wait(&bars->b_empty[s], ((it / kGgBStages) & 1) ^ 1))) break;
+          const uint32_t s = it % kBStages;
+          if (!(ok = ab.wait(&bars->b_empty[s], ((it / kBStages) & 1) ^ 1))) break;
           uint64_t* full = &bars->b_full[s];
           uint8_t* dst = ringb + s * kTileB;
           if (S >= 4) {  // (steps behind the last one are filled with zeros and not used)
