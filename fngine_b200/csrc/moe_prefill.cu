@@ -142,29 +142,71 @@ __device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) {
 // global memory (so all earlier ones are complete too), and data of a predecessor is never read through const __restrict__
 // pointers, which would allow the load ahead of the wait. Layers of 96 IQ4_NL
 // tokens 373 -> 355 us, of 50 tokens at 640 268 -> 248.
-// Top-10 per token (one warp each), per-expert pair counts.
-__global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int stride, int T, int32_t* topk_e, float* topk_w,
-                                                      int32_t* count) {
-  pdl_launch_dependents();
-  pdl_wait_prior();
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (t >= T) return;
-  int ids[kTopK];
-  float w[kTopK];
-  warp_topk10([&](int e) { return logits[size_t(t) * stride + e]; }, ids, w);
-  if (lane < kTopK) {
-    int id = 0;
-    float wt = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kTopK; ++k)
-      if (lane == k) {
-        id = ids[k];
-        wt = w[k];
-      }
-    topk_e[t * kTopK + lane] = id;
-    topk_w[t * kTopK + lane] = wt;
-    if (count) atomicAdd(&count[id], 1);
+// Pairs are counted and numbered in one pass: a block counts its pairs in shared memory (the count a pair finds is its number
+// within the block), adds the sums to the expert's count once, and the value it meets there plus the block's number is the
+// pair's number within its expert, left in token_pair for the scatter kernel. (One atomic per pair, in two kernels, met a
+// popular expert's counter 4000 times at 8192 tokens.)
+struct PairNumbers {
+  int count[kExperts];  // pairs of the block, then the pairs of blocks before it
+  __device__ __forceinline__ void clear(int threads) {
+    for (int e = threadIdx.x; e < kExperts; e += threads) count[e] = 0;
   }
+  __device__ __forceinline__ int add(int e) { return atomicAdd(&count[e], 1); }
+  __device__ __forceinline__ void publish(int32_t* total, int threads) {
+    for (int e = threadIdx.x; e < kExperts; e += threads) {
+      const int c = count[e];
+      if (c) count[e] = atomicAdd(&total[e], c);
+    }
+  }
+};
+
+// Top-10 per token (one warp each, PER_WARP in turn), per-expert pair counts and the pairs' numbers (token_pair, may be absent).
+// PER_WARP 4 from 4096 tokens on: fewer meetings on a popular expert's counter; below that single tokens fill the GPU.
+// The routing launches of 8192 tokens together: 45 us, 25 so (selection by the pruned search and numbering).
+template <int PER_WARP>
+__global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int stride, int T, int32_t* topk_e, float* topk_w,
+                                                      int32_t* count, int32_t* token_pair) {
+  __shared__ PairNumbers s_num;
+  __shared__ __align__(16) uint2 s_scratch[8][32];
+  __shared__ int s_ids[8][kTopK];
+  __shared__ float s_vals[8][kTopK];
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = (blockIdx.x * 8 + warp) * PER_WARP;
+  if (token_pair) {
+    s_num.clear(256);
+    __syncthreads();
+  }
+  pdl_wait_prior();
+  int id[PER_WARP], number[PER_WARP];
+#pragma unroll
+  for (int i = 0; i < PER_WARP; ++i) {
+    const int t = t0 + i;
+    if (t >= T) break;
+    warp_top10_pruned([&](int e) { return logits[size_t(t) * stride + e]; }, s_scratch[warp], s_ids[warp], s_vals[warp]);
+    __syncwarp();
+    float vals[kTopK], w[kTopK];
+#pragma unroll
+    for (int k = 0; k < kTopK; ++k) vals[k] = s_vals[warp][k];
+    topk_softmax(vals, w);
+    if (lane < kTopK) {
+      id[i] = s_ids[warp][lane];
+      float wt = 0.0f;
+#pragma unroll
+      for (int k = 0; k < kTopK; ++k)
+        if (lane == k) wt = w[k];
+      topk_e[t * kTopK + lane] = id[i];
+      topk_w[t * kTopK + lane] = wt;
+      if (token_pair) number[i] = s_num.add(id[i]);
+    }
+    __syncwarp();
+  }
+  if (!token_pair) return;
+  __syncthreads();
+  s_num.publish(count, 256);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < PER_WARP; ++i)
+    if (t0 + i < T && lane < kTopK) token_pair[(t0 + i) * kTopK + lane] = s_num.count[id[i]] + number[i];
 }
 
 // Expert-parallel routing: the (expert, weight) lists arrive with the dispatched rows; entries of
@@ -173,20 +215,30 @@ __global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int s
 // (n << 8) | i = this rank holds copy i of n and takes the rows r with r % n == i.
 __global__ void __launch_bounds__(256) pf_import_kernel(const int32_t* in_e, const float* in_w, int lo, int hi,
                                                         const int32_t* share, int n, int32_t* topk_e, float* topk_w,
-                                                        int32_t* count) {
+                                                        int32_t* count, int32_t* token_pair) {
+  __shared__ PairNumbers s_num;
   pdl_launch_dependents();
+  s_num.clear(256);
+  __syncthreads();
   pdl_wait_prior();
   const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const int e = in_e[i];
-  bool local = e >= lo && e < hi;
-  if (share) {
-    const int sh = e >= 0 && e < kExperts ? share[e] : -1;
-    local = sh >= 0 && (i / kTopK) % max(sh >> 8, 1) == (sh & 255);
+  int e = -1, number = 0;
+  if (i < n) {
+    e = in_e[i];
+    bool local = e >= lo && e < hi;
+    if (share) {
+      const int sh = e >= 0 && e < kExperts ? share[e] : -1;
+      local = sh >= 0 && (i / kTopK) % max(sh >> 8, 1) == (sh & 255);
+    }
+    if (!local) e = -1;
+    topk_e[i] = e;
+    topk_w[i] = in_w[i];
+    if (local) number = s_num.add(e);
   }
-  topk_e[i] = local ? e : -1;
-  topk_w[i] = in_w[i];
-  if (local) atomicAdd(&count[e], 1);
+  __syncthreads();
+  s_num.publish(count, 256);
+  __syncthreads();
+  if (e >= 0) token_pair[i] = s_num.count[e] + number;
 }
 
 // Exclusive scan of the counts and the token-tile lists of both grouped GEMMs (one block of 512): tile = {expert, 0,
@@ -210,7 +262,7 @@ __device__ __forceinline__ void list_tiles(int expert, int first_pair, int count
     if (at < max_tiles) tiles[at] = make_int4(expert, 0, first_pair + full * TILE, rest);
   }
 }
-__global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int32_t* offset, int32_t* cursor, int4* tiles_gu,
+__global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int32_t* offset, int4* tiles_gu,
                                                       int4* tiles_dn, int32_t* meta, int inter, int max_units_gu,
                                                       int max_units_dn) {
   pdl_launch_dependents();
@@ -242,7 +294,6 @@ __global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int3
     total += s_scan[i];
   }
   offset[tid] = first;
-  cursor[tid] = 0;
   __syncthreads();
   const int mg = inter / kTileM, md = H / kTileM;
   if (warp < 2) {  // warp k: list k
@@ -265,12 +316,11 @@ __global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int3
   list_tiles<kTileNDown>(tid, first, c, s_cursor[1], tiles_dn, max_units_dn / md);
 }
 
-// Pairs grouped by expert. The order inside an expert depends on the atomics, the results do not:
-// every pair's h and y rows depend only on (token, expert) and the combine adds a token's ten rows
-// in ascending-expert order.
+// Pairs grouped by expert, a pair's place being its number within the expert. The numbers depend on the atomics, the results do
+// not: every pair's h and y rows depend only on (token, expert) and the combine adds a token's ten rows in ascending-expert
+// order.
 __global__ void __launch_bounds__(256) pf_scatter_kernel(const int32_t* topk_e, const float* topk_w, const int32_t* offset,
-                                                         int32_t* cursor, int32_t* pair_token, float* pair_weight,
-                                                         int32_t* token_pair, int T) {
+                                                         int32_t* pair_token, float* pair_weight, int32_t* token_pair, int T) {
   pdl_launch_dependents();
   pdl_wait_prior();
   const int i = blockIdx.x * 256 + threadIdx.x;
@@ -280,7 +330,7 @@ __global__ void __launch_bounds__(256) pf_scatter_kernel(const int32_t* topk_e, 
     token_pair[i] = -1;
     return;
   }
-  const int pos = offset[e] + atomicAdd(&cursor[e], 1);
+  const int pos = offset[e] + token_pair[i];
   pair_token[pos] = i / kTopK;
   pair_weight[pos] = topk_w[i];
   token_pair[i] = pos;
@@ -443,11 +493,11 @@ cudaError_t launch_grouped(const GgArgs& a, const GgMaps& maps, cudaStream_t str
 // Offsets, token tiles and pair lists from the counts and the top-10 entries of `rows` tokens.
 cudaError_t launch_pair_lists(const fb_moe_prefill_workspace* ws, int rows, cudaStream_t s) {
   const cudaError_t e = launch_pdl(pf_scan_kernel, dim3(1), dim3(512), 0, s, ws->expert_count, ws->expert_offset,
-                                   ws->expert_cursor, static_cast<int4*>(ws->units_gate_up), static_cast<int4*>(ws->units_down),
+                                   static_cast<int4*>(ws->units_gate_up), static_cast<int4*>(ws->units_down),
                                    ws->meta, ws->inter, ws->max_units_gate_up, ws->max_units_down);
   if (e != cudaSuccess) return e;
   return launch_pdl(pf_scatter_kernel, dim3((rows * kTopK + 255) / 256), dim3(256), 0, s, ws->topk_expert, ws->topk_weight,
-                    ws->expert_offset, ws->expert_cursor, ws->pair_token, ws->pair_weight, ws->token_pair, rows);
+                    ws->expert_offset, ws->pair_token, ws->pair_weight, ws->token_pair, rows);
 }
 
 size_t up256(size_t v) { return (v + 255) & ~size_t(255); }
@@ -565,8 +615,9 @@ int32_t fb_moe_route(const float* router_logits, int32_t logits_stride, const vo
   cudaError_t e = cudaMemsetAsync(ws->expert_count, 0, kExperts * 4, s);
   if (e == cudaSuccess) e = clear_fixed(ws, tokens, s);
   if (e != cudaSuccess) return check_launch("route: memset");
-  e = launch_pdl(pf_topk_kernel, dim3((tokens + 7) / 8), dim3(256), 0, s, router_logits, logits_stride, tokens, ws->topk_expert,
-                 ws->topk_weight, ws->expert_count);
+  const int per_warp = tokens >= 4096 ? 4 : 1;
+  e = launch_pdl(per_warp == 4 ? pf_topk_kernel<4> : pf_topk_kernel<1>, dim3((tokens + 8 * per_warp - 1) / (8 * per_warp)), dim3(256),
+                 0, s, router_logits, logits_stride, tokens, ws->topk_expert, ws->topk_weight, ws->expert_count, ws->token_pair);
   if (e == cudaSuccess) e = launch_pair_lists(ws, tokens, s);
   const int32_t st = check_launch("route");
   return st ? st : int32_t(e);
@@ -576,8 +627,9 @@ int32_t fb_moe_topk(const float* router_logits, int32_t logits_stride, int32_t t
                     float* topk_weight, void* stream) {
   if (!router_logits || logits_stride < kExperts || tokens < 1 || !topk_expert || !topk_weight)
     return invalid("topk: bad arguments");
-  const cudaError_t e = launch_pdl(pf_topk_kernel, dim3((tokens + 7) / 8), dim3(256), 0, as_stream(stream), router_logits,
-                                   logits_stride, tokens, topk_expert, topk_weight, static_cast<int32_t*>(nullptr));
+  const cudaError_t e = launch_pdl(pf_topk_kernel<1>, dim3((tokens + 7) / 8), dim3(256), 0, as_stream(stream), router_logits,
+                                   logits_stride, tokens, topk_expert, topk_weight, static_cast<int32_t*>(nullptr),
+                                   static_cast<int32_t*>(nullptr));
   const int32_t st = check_launch("topk");
   return st ? st : int32_t(e);
 }
@@ -607,7 +659,7 @@ static int32_t route_ep_impl(const int32_t* topk_expert, const float* topk_weigh
   if (e != cudaSuccess) return check_launch("route_ep: memset");
   const int n = rows * kTopK;
   e = launch_pdl(pf_import_kernel, dim3((n + 255) / 256), dim3(256), 0, s, topk_expert, topk_weight, expert_lo, expert_hi, share,
-                 n, ws->topk_expert, ws->topk_weight, ws->expert_count);
+                 n, ws->topk_expert, ws->topk_weight, ws->expert_count, ws->token_pair);
   if (e == cudaSuccess) e = launch_pair_lists(ws, rows, s);
   const int32_t st = check_launch("route_ep");
   return st ? st : int32_t(e);

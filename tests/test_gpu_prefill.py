@@ -504,3 +504,46 @@ def test_token_boxes_and_gate_up_matrices_at_any_even_address(fg, fd, inter):
         apart.layout.blob_stride, apart.layout.gate_offset, apart.layout.up_offset, apart.layout.down_offset = wide, g_at, up, down
         got = run_prefill(torch, apart, ws, lg, xd, T)
         assert ws.status() == 0 and torch.equal(got, y), (g_at, u_at)
+
+
+@pytest.mark.parametrize("T", [1, 31, 4095, 4099])
+def test_route_numbers_every_pair_once(T):
+    """Selection and pair lists of one and of four tokens per warp, ragged: the ten largest logits (NaN never wins, equal
+    logits go to the lower id), every pair in its expert's range exactly once; the same for the half of the experts that a
+    shard holds."""
+    torch = _torch()
+    from fngine_b200 import lib as L, prefill
+    import ctypes as C
+    g = torch.Generator(device="cuda").manual_seed(T)
+    lg = torch.randn(T, 513, generator=g, device="cuda")
+    lg[:, 7] += 3.0  # a popular expert
+    lg[0, :512] = 1.5  # all equal
+    lg[T // 2, 40:300] = float("nan")
+    lg[T - 1, 100:140] = 9.0
+    key = torch.where(torch.isnan(lg[:, :512]), torch.full_like(lg[:, :512], -float("inf")), lg[:, :512])
+    want = torch.sort(key, dim=1, descending=True, stable=True).indices[:, :10]
+    ws = prefill.PrefillWorkspace(T, 512)
+    prefill.moe_route(lg, lg, None, 0, None, None, T, ws, logits_stride=513)
+    torch.cuda.synchronize()
+
+    def check(local):
+        e = ws.ints(ws.ws.topk_expert, T * 10).reshape(T, 10)
+        off, pair = ws.ints(ws.ws.expert_offset, 513), ws.ints(ws.ws.token_pair, T * 10).reshape(T, 10)
+        ids = want.cpu().numpy()
+        assert np.array_equal(e, np.where(local[ids], ids, -1))
+        counts = np.bincount(ids[local[ids]], minlength=512)
+        assert np.array_equal(np.diff(off), counts)
+        held = pair[e >= 0]
+        assert np.array_equal(np.sort(held), np.arange(off[512])) and np.all(pair[e < 0] == -1)
+        assert np.all((held >= off[e[e >= 0]]) & (held < off[e[e >= 0] + 1]))
+        tok = ws.ints(ws.ws.pair_token, T * 10)
+        assert np.array_equal(tok[held], np.repeat(np.arange(T), 10).reshape(T, 10)[e >= 0])
+        w, pw = ws.floats(ws.ws.topk_weight, T * 10).reshape(T, 10), ws.floats(ws.ws.pair_weight, T * 10)
+        assert np.array_equal(pw[held].view(np.uint32), w[e >= 0].view(np.uint32))
+
+    check(np.ones(512, bool))
+    e, w = ws.ints(ws.ws.topk_expert, T * 10), ws.floats(ws.ws.topk_weight, T * 10)
+    ed, wd = torch.from_numpy(e.copy()).cuda(), torch.from_numpy(w.copy()).cuda()
+    L.check(L.load().fb_moe_route_ep(ed.data_ptr(), wd.data_ptr(), 0, 256, T, C.byref(ws.ws), torch.cuda.current_stream().cuda_stream), "route_ep")
+    torch.cuda.synchronize()
+    check(np.arange(512) < 256)
