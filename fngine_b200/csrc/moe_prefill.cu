@@ -355,10 +355,11 @@ __global__ void __launch_bounds__(256) ep_scatter_sum_kernel(const float* __rest
 
 // ------------------------------------------------------------------------------ combine
 // y[t][n] = sum over token t's ten pairs, in ascending expert id, of yp[pair][n] (+ shared);
-// X[t][s][n] += inj[t][s] * y when X is given. Bound: the ten rows per token from memory. One block per token, thread = four
-// columns, all ten 16-byte loads in flight (ten blocks per token with 4-byte loads: 198 us at 8192 tokens, 0.72 of the
-// copy rate).
-constexpr int kPcThreads = H / 4;  // 640
+// X[t][s][n] += inj[t][s] * y when X is given. Bound: the ten rows per token from memory. Four blocks per token, thread = four
+// columns, all ten 16-byte loads in flight. (8192 tokens: 147 us, 0.97 of the copy rate. One block of 640 threads per token
+// took 210: with its registers two of them share a multiprocessor, and while one orders its pairs only the other one loads.
+// Two blocks of 320: 150; blocks of 640 that stay and fetch the next token's pairs ahead: 151.)
+constexpr int kPcParts = 4, kPcThreads = H / 4 / kPcParts;  // 160
 template <bool ALIGNED>  // y_shared, X and y_out on 16-byte boundaries (single words otherwise)
 __device__ __forceinline__ float4 load4(const float* p) {
   if constexpr (ALIGNED) return *reinterpret_cast<const float4*>(p);
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(kPcThreads) pf_combine_kernel(const int32_t* t
                                                                 float* y_out, const long long* y_fixed) {
   pdl_launch_dependents();
   pdl_wait_prior();
-  const int t = blockIdx.x, n4 = threadIdx.x, lane = threadIdx.x & 31;
+  const int t = blockIdx.x / kPcParts, n4 = (blockIdx.x % kPcParts) * kPcThreads + threadIdx.x, lane = threadIdx.x & 31;
   float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (y_fixed) {  // fixed-point sums: one rounding, the scale is exact (moe_y_fixed_to_float of the reference)
     const longlong2* f = reinterpret_cast<const longlong2*>(y_fixed + size_t(t) * H) + 2 * n4;
@@ -747,7 +748,7 @@ int32_t fb_moe_prefill_combine(const fb_moe_prefill_workspace* ws, const float* 
   const bool aligned = ((reinterpret_cast<uintptr_t>(y_shared) | reinterpret_cast<uintptr_t>(X) |
                          reinterpret_cast<uintptr_t>(y_out)) & 15) == 0;
   auto* kernel = aligned ? pf_combine_kernel<true> : pf_combine_kernel<false>;
-  const cudaError_t e = launch_pdl(kernel, dim3(tokens), dim3(kPcThreads), 0, as_stream(stream), ws->topk_expert, ws->token_pair,
+  const cudaError_t e = launch_pdl(kernel, dim3(unsigned(tokens) * kPcParts), dim3(kPcThreads), 0, as_stream(stream), ws->topk_expert, ws->token_pair,
                                    ws->yp, y_shared, inj, X, y_out,
                                    g_prefill_fixed ? reinterpret_cast<const long long*>(ws->yp) : nullptr);
   const int32_t st = check_launch("prefill_combine");
