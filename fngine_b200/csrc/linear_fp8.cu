@@ -141,26 +141,29 @@ __device__ __forceinline__ bool gemm_wait(GemmBars* b, uint64_t* bar, uint32_t p
 // range (|x| >= 2^-9..2^-10 of the row maximum); smaller elements lose bits below 2^-17 of the row
 // maximum. scale * (hi + lo) therefore IS the bf16 activation: the two-piece GEMM has the numerics of
 // the reference's bf16-activation path (src/kernels/linear/linear.h:27-31) on the FP8 tensor cores.
-// Each thread keeps up to kQPer 16-byte pieces of the row in registers between the two phases (rows up
-// to 256 * 8 * kQPer elements are read from memory once); longer rows re-read the remainder.
-constexpr int kQPer = 2;
+// GROUP threads work on a token: a block, or from kSplitWarpTokens tokens on a warp (eight tokens per block). Each thread keeps
+// up to kPer 16-byte pieces of the row in registers between the two phases (rows of 4096, 2560 elements are read from memory
+// once); longer rows re-read the remainder. What bounds it is a token's chain of load,
+// reduction, store: see launch_split.
 
 __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t pair) {
   const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(pair), __NV_E4M3);
   return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
-__global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfloat16* x, int K, uint8_t* codes,
+template <int GROUP>
+__global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfloat16* x, int tokens, int K, uint8_t* codes,
                                                                   uint8_t* codes_lo, float* scales, uint32_t* status) {
+  constexpr int kPer = GROUP == 256 ? 2 : 10;
   pdl_wait_prior();
   // (behind the wait: fp8_mid_kernel asks for its weights, which the kernel ahead of this one may have written, before it
   // waits for this one; nor do its early loads compete with the call before)
   pdl_launch_dependents();
   if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;  // of the GEMM that follows
-  const int t = blockIdx.x;
+  const int me = threadIdx.x % GROUP, t = blockIdx.x * (256 / GROUP) + threadIdx.x / GROUP;
+  if (GROUP < 256 && t >= tokens) return;
   const __nv_bfloat16* row = x + size_t(t) * K;
-  __shared__ float s_red[8];
-  uint4 held[kQPer];
+  uint4 held[kPer];
   float m = 0.0f;
   auto absmax = [&](const uint4& v) {
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
@@ -171,19 +174,22 @@ __global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfl
     }
   };
 #pragma unroll
-  for (int p = 0; p < kQPer; ++p) {
-    const int i = (p * 256 + threadIdx.x) * 8;
+  for (int p = 0; p < kPer; ++p) {
+    const int i = (p * GROUP + me) * 8;
     held[p] = i < K ? *reinterpret_cast<const uint4*>(row + i) : make_uint4(0, 0, 0, 0);
     absmax(held[p]);
   }
-  for (int i = (kQPer * 256 + threadIdx.x) * 8; i < K; i += 256 * 8) absmax(*reinterpret_cast<const uint4*>(row + i));
+  for (int i = (kPer * GROUP + me) * 8; i < K; i += GROUP * 8) absmax(*reinterpret_cast<const uint4*>(row + i));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  m = s_red[0];
+  if constexpr (GROUP == 256) {
+    __shared__ float s_red[8];
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = s_red[0];
 #pragma unroll
-  for (int i = 1; i < 8; ++i) m = fmaxf(m, s_red[i]);
+    for (int i = 1; i < 8; ++i) m = fmaxf(m, s_red[i]);
+  }
   const bool two = codes_lo != nullptr;
   float scale, inv;
   if (two) {
@@ -196,7 +202,7 @@ __global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfl
     scale = m > 0.0f ? __fdiv_rn(m, 448.0f) : 0.0f;
     inv = scale > 0.0f ? __fdiv_rn(1.0f, scale) : 0.0f;
   }
-  if (threadIdx.x == 0) scales[t] = scale;
+  if (me == 0) scales[t] = scale;
   auto encode = [&](const uint4& v, int i) {
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
     uint32_t o[2] = {0, 0}, ol[2] = {0, 0};
@@ -216,11 +222,11 @@ __global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfl
     if (two) *reinterpret_cast<uint2*>(codes_lo + size_t(t) * K + i) = make_uint2(ol[0], ol[1]);
   };
 #pragma unroll
-  for (int p = 0; p < kQPer; ++p) {
-    const int i = (p * 256 + threadIdx.x) * 8;
+  for (int p = 0; p < kPer; ++p) {
+    const int i = (p * GROUP + me) * 8;
     if (i < K) encode(held[p], i);
   }
-  for (int i = (kQPer * 256 + threadIdx.x) * 8; i < K; i += 256 * 8) encode(*reinterpret_cast<const uint4*>(row + i), i);
+  for (int i = (kPer * GROUP + me) * 8; i < K; i += GROUP * 8) encode(*reinterpret_cast<const uint4*>(row + i), i);
 }
 
 // ------------------------------------------------------------------------------ GEMM: tiles and epilogues
@@ -1735,6 +1741,21 @@ const int* small_clusters() {
   return e == cudaSuccess ? table : nullptr;
 }
 
+// The activation kernel of `tokens` rows; `chained`: it may start while the call before runs out. A warp per token where there
+// are enough of them for all warps and a row fits its registers (us per call: 9216 x 2560 at 4096 tokens 135.1 -> 133.5,
+// 1280 x 2560 at 4000 50.0 -> 48.5, at 1003 22.6 -> 22.2; level at 600 and 1200); a block per token elsewhere (with warps,
+// 2560 x 6144 at 300 36.9 -> 41.0, 16384 x 2560 at 30 16.0 -> 17.0).
+constexpr int kSplitWarpTokens = 1000;
+cudaError_t launch_split(bool chained, const __nv_bfloat16* x, int tokens, int k, uint8_t* codes, uint8_t* codes_lo, float* scales,
+                         uint32_t* status, cudaStream_t stream) {
+  const bool warps = tokens >= kSplitWarpTokens && k <= 2560;
+  auto* kernel = warps ? fp8_quantize_tokens_kernel<32> : fp8_quantize_tokens_kernel<256>;
+  const dim3 grid(unsigned(warps ? (tokens + 7) / 8 : tokens));
+  if (chained) return launch_pdl(kernel, grid, dim3(256), 0, stream, x, tokens, k, codes, codes_lo, scales, status);
+  kernel<<<grid, 256, 0, stream>>>(x, tokens, k, codes, codes_lo, scales, status);
+  return cudaSuccess;
+}
+
 }  // namespace
 }  // namespace fb
 
@@ -1754,8 +1775,7 @@ int32_t fb_fp8_quantize_tokens(const void* x_bf16, int32_t tokens, int32_t k, ui
                                void* stream) {
   if (!x_bf16 || !codes || !scales || tokens <= 0 || k <= 0 || k % 8)
     return invalid("fp8_quantize_tokens: bad arguments (k must be a multiple of 8)");
-  fp8_quantize_tokens_kernel<<<tokens, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x_bf16), k, codes,
-                                                                    nullptr, scales, nullptr);
+  launch_split(false, static_cast<const __nv_bfloat16*>(x_bf16), tokens, k, codes, nullptr, scales, nullptr, as_stream(stream));
   return check_launch("fp8_quantize_tokens");
 }
 
@@ -1763,8 +1783,7 @@ int32_t fb_fp8_split_tokens(const void* x_bf16, int32_t tokens, int32_t k, uint8
                             float* scales, void* stream) {
   if (!x_bf16 || !codes_hi || !codes_lo || !scales || tokens <= 0 || k <= 0 || k % 8)
     return invalid("fp8_split_tokens: bad arguments (k must be a multiple of 8)");
-  fp8_quantize_tokens_kernel<<<tokens, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x_bf16), k, codes_hi,
-                                                                    codes_lo, scales, nullptr);
+  launch_split(false, static_cast<const __nv_bfloat16*>(x_bf16), tokens, k, codes_hi, codes_lo, scales, nullptr, as_stream(stream));
   return check_launch("fp8_split_tokens");
 }
 
@@ -1802,11 +1821,7 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
   // 16384 x 2560 at 300 38.7 -> 38.2); not behind GrWrite's residual streams, where 100 tokens got slower (16.3 -> 16.8).
   cudaError_t launched = cudaSuccess;
   const auto* xb = static_cast<const __nv_bfloat16*>(x_bf16);
-  if (kind == FB_EPI_GR_WRITE)
-    fp8_quantize_tokens_kernel<<<tokens, 256, 0, as_stream(stream)>>>(xb, k, a_codes, a_lo, a_scales, status);
-  else
-    launched = launch_pdl(fp8_quantize_tokens_kernel, dim3(tokens), dim3(256), 0, as_stream(stream), xb, k, a_codes, a_lo,
-                          a_scales, status);
+  launched = launch_split(kind != FB_EPI_GR_WRITE, xb, tokens, k, a_codes, a_lo, a_scales, status, as_stream(stream));
   int32_t st = check_launch("linear_fp8: activation pieces");
   if (st || launched != cudaSuccess) return st ? st : int32_t(launched);
   // The GEMM kernels too start while the pieces are made (us per call: 9216 x 2560 at 600 tokens 39.8 -> 37.9, at 4096 137.6 ->
