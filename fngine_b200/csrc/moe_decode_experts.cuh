@@ -46,6 +46,12 @@ __device__ __forceinline__ void sign_table_fill(uint32_t* signtab) {
     signtab[threadIdx.x] = m;
   }
 }
+__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+
 // One 32-weight sub-block: P = sum over its 8 look-ups of dp4a(G ^ m, a) for each of TT tokens.
 // qs_lo/qs_hi = its 8 index bytes, qh = a word whose bits [sh, sh+8) are the ninth index bits, sg = its
 // 32 sign bits (nibble l = look-up l). sign_base = shared-window address of the 16-word mask table
@@ -61,22 +67,22 @@ __device__ __forceinline__ void iq3s_sub_dot(uint32_t qs_lo, uint32_t qs_hi, uin
   // sign nibbles pre-scaled by 4 (byte offsets into the mask table)
   const uint32_t s_even = (sg << 2) & 0x3C3C3C3Cu;  // look-ups 0,2,4,6
   const uint32_t s_odd = (sg >> 2) & 0x3C3C3C3Cu;   // look-ups 1,3,5,7
+  // An index byte and its ninth bit side by side, times 128 (the bytes of an entry), plus the lane's entry 0: one two-way dot
+  // product, which runs on the multiply pipe beside the busier integer one (a byte-permute and a shifted add each: eight
+  // layers of one token 147.0 -> 145.5 us, of sixteen 630.6 -> 626.3).
+  const uint32_t grid_at = smem_u32(grid_lane);
+  const uint32_t idx[4] = {prmt(qs_lo, h_lo, 0x5140u), prmt(qs_lo, h_lo, 0x7362u), prmt(qs_hi, h_hi, 0x5140u),
+                           prmt(qs_hi, h_hi, 0x7362u)};
   uint32_t x[8];
 #pragma unroll
   for (int l = 0; l < 8; ++l) {
-    const int b = l & 3;
-    // byte0 = qs byte b, byte1 = spread bit b, bytes 2-3 = 0 (sign-replicate of a 0/1 byte)
-    const uint32_t sel = uint32_t(b) | (uint32_t(4 + b) << 4) | (uint32_t(0xC + b) << 8) | (uint32_t(0xC + b) << 12);
-    const uint32_t idx = prmt(l < 4 ? qs_lo : qs_hi, l < 4 ? h_lo : h_hi, sel);
-    const uint32_t g = grid_lane[idx * 32];
+    const uint32_t g = lds_word(__dp2a_lo(idx[l >> 1], (l & 1) ? 0x8000u : 0x0080u, grid_at));
     // byte0 = the pre-scaled nibble of look-up l, bytes 1-3 = the table's address bytes
     // (computing the masks instead - isolate the nibble, one wide multiply that sends bit j to the top of
     // byte j, one sign-replicating byte-permute - frees a third of the shared-memory wavefronts but the
     // multiplies queue up in the dispatch stage: measured 96 us against 80 us per layer launch)
     const uint32_t maddr = prmt((l & 1) ? s_odd : s_even, sign_base, 0x7650u | uint32_t(l >> 1));
-    uint32_t m;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(m) : "r"(maddr));
-    x[l] = g ^ m;
+    x[l] = g ^ lds_word(maddr);
   }
 #pragma unroll
   for (int t = 0; t < TT; ++t) {
@@ -368,11 +374,6 @@ __device__ __forceinline__ void experts_table_fill(uint32_t* grid, uint32_t* sig
 // Four signed int8 weights from magnitudes and a sign mask (0xFF in the bytes of negative weights; magnitudes are at
 // least one, so the byte-wise + 1 never carries).
 __device__ __forceinline__ int signed4(uint32_t mag, uint32_t mask) { return int((mag ^ mask) + (mask & 0x01010101u)); }
-__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
-  uint32_t v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-  return v;
-}
 
 // One 32-weight sub-block of the other formats as eight words of int8 weights in natural order. w = the word that holds
 // the block's scale (even blocks: in its low half), as iq3s_stream reads it; IQ4_XS: the block's words.
