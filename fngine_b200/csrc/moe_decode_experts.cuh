@@ -371,15 +371,14 @@ __device__ __forceinline__ void experts_table_fill(uint32_t* grid, uint32_t* sig
 }
 
 // ------------------------------------------------------------------------------ one block against the pass's tokens
-// Four signed int8 weights from magnitudes and a sign mask (0xFF in the bytes of negative weights; magnitudes are at
-// least one, so the byte-wise + 1 never carries).
-__device__ __forceinline__ int signed4(uint32_t mag, uint32_t mask) { return int((mag ^ mask) + (mask & 0x01010101u)); }
-
 // One 32-weight sub-block of the other formats as eight words of int8 weights in natural order. w = the word that holds
-// the block's scale (even blocks: in its low half), as iq3s_stream reads it; IQ4_XS: the block's words.
+// the block's scale (even blocks: in its low half), as iq3s_stream reads it; IQ4_XS: the block's words. With a codebook, q =
+// magnitudes ^ mask (0xFF in the bytes of negative weights): a negative weight's byte is one less than the weight, and the
+// caller takes dp4a(mask, a) off. (Two more integer operations per four weights made the weights themselves: four layers
+// of eight IQ3_XXS tokens 280 -> 276 us.)
 template <int FMT, bool EVEN>
 __device__ __forceinline__ void gate_up_sub(const uint32_t* w, int ib, const uint32_t* grid, uint32_t sign_base,
-                                            const Iq4nlLevels& lv, int (&q)[8], int& m0, int& m1) {
+                                            const Iq4nlLevels& lv, int (&q)[8], int (&mask)[8], int& m0, int& m1) {
   if constexpr (FMT == FB_FMT_IQ4_XS) {
     const uint32_t head = w[0], sl = w[1];
 #pragma unroll
@@ -407,15 +406,13 @@ __device__ __forceinline__ void gate_up_sub(const uint32_t* w, int ib, const uin
       m1 = int((sc >> 3) & 30u) + 1;
       // byte offsets 64 * index + 8 * (lane % 8) of two look-ups per word: the index byte in bits 6..13 (22..29), its two
       // upper bits, taken from qh by a multiply that lands them on bits 14 and 15 (30 and 31)
-      const uint32_t lane_pat = (threadIdx.x & 7) * 0x00080008u;
+      const uint32_t lane_pat = (threadIdx.x & 7) * 0x00080008u, grid_at = smem_u32(grid);
       const uint32_t a02 = ((qs << 6) & 0x3FC03FC0u) | lane_pat | ((qh * 0x04004000u) & 0xC000C000u);
       const uint32_t a13 = ((qs >> 2) & 0x3FC03FC0u) | lane_pat | ((qh * 0x01001000u) & 0xC000C000u);
 #pragma unroll
       for (int l = 0; l < 4; ++l) {
-        const uint32_t a = (l & 1) ? a13 : a02;
-        const uint2 v = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(grid) + ((l & 2) ? a >> 16 : a & 0xFFFFu));
-        g[2 * l] = v.x;
-        g[2 * l + 1] = v.y;
+        const uint32_t at = __dp2a_lo((l & 1) ? a13 : a02, (l & 2) ? 0x0100u : 0x0001u, grid_at);
+        asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(g[2 * l]), "=r"(g[2 * l + 1]) : "r"(at));
       }
     } else {
       const uint32_t aux = iq3s_stream<EVEN>(w, 16 + ib);
@@ -426,18 +423,27 @@ __device__ __forceinline__ void gate_up_sub(const uint32_t* w, int ib, const uin
       p ^= p >> 2;
       p ^= p >> 1;
       sg |= (p & 0x01010101u) << 7;
-      const uint32_t lane4 = 4 * (threadIdx.x & 31);
+      const uint32_t grid_at = smem_u32(grid) + 4 * (threadIdx.x & 31);
 #pragma unroll
-      for (int l = 0; l < 8; ++l) {
-        const uint32_t qs = iq3s_stream<EVEN>(w, 2 * ib + (l >> 2));
-        g[l] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(grid) +
-                                                  ((((qs >> (8 * (l & 3))) & 0xFFu) << 7) | lane4));
-      }
+      for (int l = 0; l < 8; ++l)  // (byte times 128 plus base in one dot product: 276 -> 259 us)
+        g[l] = lds_word(__dp4a(iq3s_stream<EVEN>(w, 2 * ib + (l >> 2)), 128u << (8 * (l & 3)), grid_at));
     }
     const uint32_t s_even = (sg << 2) & 0x3C3C3C3Cu, s_odd = (sg >> 2) & 0x3C3C3C3Cu;  // nibbles as byte offsets, see iq3s_sub_dot
 #pragma unroll
-    for (int l = 0; l < 8; ++l)
-      q[l] = signed4(g[l], lds_word(prmt((l & 1) ? s_odd : s_even, sign_base, 0x7650u | uint32_t(l >> 1))));
+    for (int l = 0; l < 8; ++l) {
+      uint32_t m;
+      if constexpr (FMT == FB_FMT_IQ2_S) {
+        // Shared memory is the busy unit here (look-ups of eight bytes in three passes), so the mask is made: a sign byte times
+        // 0x80402010 has bit 3 - j at bit 7 of byte j, times 0x08040201 bit 7 - j, and a byte-permute spreads them over the
+        // bytes and turns them round. (Eight layers of five tokens 383 -> 371 us. The others, whose look-ups take one
+        // pass, lose by it: IQ3_XXS 259 -> 262, IQ3_S at sixteen tokens 626 -> 640.)
+        m = prmt(__dp4a(sg, 1u << (8 * (l >> 1)), 0u) * ((l & 1) ? 0x08040201u : 0x80402010u), 0u, 0x89ABu);
+      } else {
+        m = lds_word(prmt((l & 1) ? s_odd : s_even, sign_base, 0x7650u | uint32_t(l >> 1)));
+      }
+      q[l] = int(g[l] ^ m);
+      mask[l] = int(m);
+    }
   }
 }
 
@@ -451,8 +457,8 @@ __device__ __forceinline__ void gate_up_block_idot(const uint32_t* w, const uint
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int ib = 4 * half + i;
-      int q[8], m0, m1;
-      gate_up_sub<FMT, EVEN>(w, ib, grid, sign_base, lv, q, m0, m1);
+      int q[8], mask[8], m0, m1;
+      gate_up_sub<FMT, EVEN>(w, ib, grid, sign_base, lv, q, mask, m0, m1);
 #pragma unroll
       for (int t = 0; t < TT; ++t) {
         const int4 a0 = *reinterpret_cast<const int4*>(act[t] + 32 * ib);
@@ -465,6 +471,18 @@ __device__ __forceinline__ void gate_up_block_idot(const uint32_t* w, const uint
         s1 = __dp4a(q[5], a1.y, s1);
         s1 = __dp4a(q[6], a1.z, s1);
         s1 = __dp4a(q[7], a1.w, s1);
+        if constexpr (FMT != FB_FMT_IQ4_XS) {
+          int c0 = __dp4a(mask[0], a0.x, 0);
+          c0 = __dp4a(mask[1], a0.y, c0);
+          c0 = __dp4a(mask[2], a0.z, c0);
+          c0 = __dp4a(mask[3], a0.w, c0);
+          int c1 = __dp4a(mask[4], a1.x, FMT == FB_FMT_IQ2_S ? 0 : c0);
+          c1 = __dp4a(mask[5], a1.y, c1);
+          c1 = __dp4a(mask[6], a1.z, c1);
+          c1 = __dp4a(mask[7], a1.w, c1);
+          s0 -= c0;
+          s1 -= c1;
+        }
         bsum[t] += FMT == FB_FMT_IQ2_S ? m0 * s0 + m1 * s1 : m0 * s1;
       }
     }
