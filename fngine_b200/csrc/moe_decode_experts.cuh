@@ -525,7 +525,7 @@ __device__ __forceinline__ void gate_up_block_terms(const uint8_t* blk, const ui
 
 // IQ4_NL: one task = NB consecutive 18-byte blocks of the lane's row, OFF bytes behind `wp`, against the pass's tokens;
 // blk0 = index of the first of them in the row. Even blocks start on a word (scale in the low half, codes two bytes
-// off: funnel shifts), odd blocks on a half word (scale in the high half, codes aligned). Rows of 1440 and 288 bytes keep
+// off), odd blocks on a half word (scale in the high half, codes aligned). Rows of 1440 and 288 bytes keep
 // eight blocks on 16-byte boundaries, the halves of 360-byte rows start on 8-byte boundaries (the second one four bytes
 // early): the widest loads without bank conflicts. term[t] = sum over the blocks, in block order, of isum * (d * d_act).
 template <int NB, int OFF>
@@ -554,26 +554,15 @@ __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlL
   const uint8_t* act1 = act0 + (ntp == 2 ? act_bytes : 0);
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
-    uint32_t q[4];
-    float d;
-    if (b % 2 == 0) {
-      const int base = kOff + 9 * b / 2;
-      d = __half2float(__ushort_as_half(static_cast<unsigned short>(w[base] & 0xFFFFu)));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = __funnelshift_r(w[base + i], w[base + i + 1], 16);
-    } else {
-      const int base = kOff + (18 * b - 2) / 4;
-      d = __half2float(__ushort_as_half(static_cast<unsigned short>(w[base] >> 16)));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = w[base + 1 + i];
-    }
-    int wq[8];
-    iq4nl_decode32(lv, q, wq);
+    const int base = b % 2 == 0 ? kOff + 9 * b / 2 : kOff + (18 * b - 2) / 4;  // the word with the scale
+    const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(b % 2 == 0 ? w[base] & 0xFFFFu : w[base] >> 16)));
+    int lo[8], hi[8];
+    iq4nl_addends32(lv, w, 2 * base + (b % 2 == 0 ? 1 : 2), lo, hi);
     const int blk = blk0 + b;
-    const int s0 = dot32(wq, reinterpret_cast<const int8_t*>(act0) + 32 * blk);
+    const int s0 = dot32(lo, hi, reinterpret_cast<const int8_t*>(act0) + 32 * blk);
     term[0] = fmaf(float(s0), d * reinterpret_cast<const float*>(act0 + k)[blk], term[0]);
     if (ntp == 2) {
-      const int s1 = dot32(wq, reinterpret_cast<const int8_t*>(act1) + 32 * blk);
+      const int s1 = dot32(lo, hi, reinterpret_cast<const int8_t*>(act1) + 32 * blk);
       term[1] = fmaf(float(s1), d * reinterpret_cast<const float*>(act1 + k)[blk], term[1]);
     }
   }
