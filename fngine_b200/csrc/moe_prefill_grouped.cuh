@@ -717,6 +717,16 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
     for (int u = blockIdx.x; u < n_units; u += gridDim.x, un = un_next) {
       un_next = unit_or_none(u + gridDim.x);
       const bool wide = ((un.w + 15) & ~15) > 128;
+      // (the routing weights of the warp's chunks, asked for ahead of the wait: a load per chunk behind it cost as much as the
+      // rest of the chunk)
+      float pw[kTileNDown / 32];
+      if constexpr (DOWN) {
+#pragma unroll
+        for (int i = 0; i < kTileNDown / 32; ++i) {
+          const int t = chunk0 + 32 * i + (lane & 15);
+          pw[i] = t < un.w && !A.y_fixed ? A.pair_weight[un.z + t] : 0.0f;
+        }
+      }
       bool ok = true;
       if (wide || nb == 0) ok = ab.wait_warp(&bars->acc_full[0], use0 & 1);
       if (ok && (wide || nb == 1)) ok = ab.wait_warp(&bars->acc_full[1], use1 & 1);
@@ -727,7 +737,10 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
         if (I == 512) gg_store_h<512>(A.h, un, q, lane, chunk0, dcol);
         else gg_store_h<640>(A.h, un, q, lane, chunk0, dcol);
       } else {
-        for (int c0 = chunk0; c0 < un.w; c0 += 4 * kGgEpiWarps) {
+#pragma unroll
+        for (int c = 0; c < kTileNDown / 32; ++c) {
+          const int c0 = chunk0 + 32 * c;
+          if (c0 >= un.w) break;
           uint32_t r[16];
           tmem_ld16(dcol + uint32_t(c0), r);
           tmem_ld_wait();
@@ -741,17 +754,16 @@ grouped_kernel(const GgArgs A, const __grid_constant__ GgMaps maps) {
                           static_cast<unsigned long long>(__float2ll_rn(v * 4294967296.0f)));
               }
           } else {
-            // (an epilogue warp gets an issue slot every eight cycles or so: the weights come in one load and reach the
-            // lanes by shuffles, and whole chunks skip the bounds checks)
-            const float pw = c0 + (lane & 15) < un.w ? A.pair_weight[un.z + c0 + (lane & 15)] : 0.0f;
+            // (an epilogue warp gets an issue slot every eight cycles or so: the weights reach the lanes by shuffles, and whole
+            // chunks skip the bounds checks)
             float* out = A.yp + size_t(un.z + c0) * H + n;
             if (c0 + 16 <= un.w) {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) out[i * H] = __shfl_sync(0xffffffffu, pw, i) * __uint_as_float(r[i]);
+              for (int i = 0; i < 16; ++i) out[i * H] = __shfl_sync(0xffffffffu, pw[c], i) * __uint_as_float(r[i]);
             } else {
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
-                const float w = __shfl_sync(0xffffffffu, pw, i);
+                const float w = __shfl_sync(0xffffffffu, pw[c], i);
                 if (c0 + i < un.w) out[i * H] = w * __uint_as_float(r[i]);
               }
             }
