@@ -1467,7 +1467,7 @@ inline int mid_smem(int pieces, int tok, int stages) {
 }
 struct MidArgs {
   int cluster, stages, tok;  // CTAs per unit, ring stages, token slots of a stage (a multiple of 32)
-  int m_tiles;
+  int m_tiles, tile;         // row tiles, tokens of a unit
 };
 
 template <int PIECES>
@@ -1480,7 +1480,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const int cluster = g.cluster, S = g.stages;
   const int unit = int(blockIdx.x) / cluster, rank = int(blockIdx.x) - unit * cluster;
   const int tile = unit / g.m_tiles, m = unit - tile * g.m_tiles;
-  const int t0 = tile * kMidTok, nt = min(kMidTok, a.M - t0), n16 = (nt + 15) & ~15;
+  const int t0 = tile * g.tile, nt = min(g.tile, a.M - t0), n16 = (nt + 15) & ~15;
   const bool swiglu = a.kind == FB_EPI_SWIGLU;
   const int kbt = a.K / BK, kb0 = kbt * rank / cluster, nkb = kbt * (rank + 1) / cluster - kb0;
   const int stage = kDecStageA + PIECES * g.tok * BK, half_n = a.N >> 1;
@@ -1848,7 +1848,8 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
   // tokens: 1.3 - 2.2 times faster below that line, up to 2.4 times slower above it); below 256 tokens up to two waves of
   // 128-row tiles.
   const int m_tiles_mid = kind == FB_EPI_SWIGLU ? ((n >> 1) + 63) / 64 : (n + 127) / 128;
-  const int units = m_tiles_mid * ((tokens + kMidTok - 1) / kMidTok);
+  auto mid_units = [&](int tile) { return m_tiles_mid * ((tokens + tile - 1) / tile); };
+  const int units = mid_units(kMidTok);
   const int pair_work = ((tokens + BM2 - 1) / BM2) * (kind == FB_EPI_SWIGLU ? ((n >> 1) + 127) / 128 : (n + BN - 1) / BN);
   const bool mid = !force_single && (pair ? 2 * pair_work <= pair_count() : units <= 2 * sm_count());
   CUtensorMap map_a, map_b;
@@ -1879,14 +1880,29 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
     }
     const int kb = k / BK;
     MidArgs g;
-    g.cluster = kb < kSmallMaxCluster ? kb : kSmallMaxCluster;
-    while (g.cluster > 1 && resident[g.cluster] < units) --g.cluster;
-    g.tok = ((tokens < kMidTok ? tokens : kMidTok) + 31) & ~31;
+    auto cluster_of = [&](int tile) {
+      int c = kb < kSmallMaxCluster ? kb : kSmallMaxCluster;
+      while (c > 1 && resident[c] < mid_units(tile)) --c;
+      return c;
+    };
+    auto slots_of = [&](int tile) { return ((tokens < tile ? tokens : tile) + 31) & ~31; };
+    auto intake = [&](int tile) { return kb * mid_stage(pieces, slots_of(tile)) / cluster_of(tile); };
+    // Tokens of a unit: 256, but where few hundred tokens make one wave of smaller units, 128, or 64 where K is short, if a CTA
+    // takes in no more than 100 KB in addition for it: the partial tile and the outputs are then shared out more evenly. (us
+    // per call, 256 and smaller: 1280 x 2560 at 200 tokens 13.1 and 12.0, at 300 16.6 and 13.0, at 512 17.5 and 15.5; 2560 x 640
+    // at 300 23.4 and 16.8; 2560 x 6144 at 300 36.9 and 33.1. Beyond that line: 2560 x 6144 at 400 39.0 and 52.9, 9216 x 2560 at
+    // 140 19.9 and 23.2, 2560 x 640 at 512 25.8 and 29.0; above 640 tokens level or slower.)
+    g.tile = kMidTok;
+    if (tokens > 160 && tokens <= 640)
+      for (int tile = k <= 1024 ? 64 : 128; tile < kMidTok && g.tile == kMidTok; tile *= 2)
+        if (mid_units(tile) <= sm_count() && intake(tile) <= intake(kMidTok) + 100 * 1024) g.tile = tile;
+    g.cluster = cluster_of(g.tile);
+    g.tok = slots_of(g.tile);
     g.m_tiles = m_tiles_mid;
     g.stages = (kb + g.cluster - 1) / g.cluster;
     if (g.stages > kMidMaxStages) g.stages = kMidMaxStages;
     while (g.stages > 1 && mid_smem(pieces, g.tok, g.stages) > kMidSmemMax) --g.stages;
-    const dim3 grid(unsigned(units * g.cluster)), block(kMidThreads);
+    const dim3 grid(unsigned(mid_units(g.tile) * g.cluster)), block(kMidThreads);
     const size_t smem = size_t(mid_smem(pieces, g.tok, g.stages));
     const cudaError_t e = pieces == 2 ? launch_pdl_cluster(fp8_mid_kernel<2>, grid, block, smem, as_stream(stream),
                                                            unsigned(g.cluster), map_a, map_b, ga, g)

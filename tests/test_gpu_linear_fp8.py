@@ -377,3 +377,19 @@ def test_the_status_word_of_a_call_is_its_own(T, n, k):
 def test_linear_fp8_wide_tiles(T, n, k, kind, path):
     """The two GEMM kernels that middle widths do not take, at the edges of their tiles, both routes, every epilogue."""
     test_linear_fp8_small_and_middle_widths(T, n, k, kind, path)
+
+
+@pytest.mark.parametrize("path", ["auto", "a8"])
+@pytest.mark.parametrize("T,n,k,kind", [
+    (161, 1280, 2560, "swiglu"),        # units of 128 tokens: the first count that takes them, a ragged second unit
+    (300, 2560, 6144, "gr_write"),      # three units, K over a cluster of two
+    (193, 2560, 640, "shared_scale"),   # units of 64 tokens, the last one of one token
+    (640, 2560, 640, "shared_scale"),   # the last count, too many units of 64 tokens for one wave: 128
+    (255, 192, 128, "store_f32"),       # one K block, no cluster, half a row tile
+    (999, 256, 2560, "store_bf16"),     # the activation kernel's last count with a block per token
+    (1001, 256, 2560, "store_f32"),     # and its first with a warp per token, a ragged last block
+    (1000, 384, 384, "store_bf16"),     # rows shorter than a warp's registers
+])
+def test_units_and_splits_chosen_by_the_token_count(T, n, k, kind, path):
+    """The smaller units of the middle widths and the two forms of the activation kernel, at the counts where they change."""
+    test_linear_fp8_small_and_middle_widths(T, n, k, kind, path)
