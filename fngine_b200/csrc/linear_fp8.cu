@@ -1516,7 +1516,7 @@ inline int mid_smem(int pieces, int tok, int stages) {
 }
 struct MidArgs {
   int cluster, stages, tok;  // CTAs per unit, ring stages, token slots of a stage (a multiple of 32)
-  int m_tiles, tile;         // row tiles, tokens of a unit
+  int m_tiles, tile;         // row tiles, tokens of a unit (kMidTok or a power of two below it)
 };
 
 template <int PIECES>
@@ -1532,6 +1532,8 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const int t0 = tile * g.tile, nt = min(g.tile, a.M - t0), n16 = (nt + 15) & ~15;
   const bool swiglu = a.kind == FB_EPI_SWIGLU;
   const int kbt = a.K / BK, kb0 = kbt * rank / cluster, nkb = kbt * (rank + 1) / cluster - kb0;
+  // Smaller units sum their K in as many chains as fit the 256 columns, one behind the other, added in order at the end.
+  const int chains = min(nkb, kMidTok / g.tile);
   const int stage = kDecStageA + PIECES * g.tok * BK, half_n = a.N >> 1;
   const int r0 = swiglu ? m * 64 : m * 128, r1 = swiglu ? half_n + m * 64 : m * 128 + 64;
   float* part = reinterpret_cast<float*>(smem);  // [token][row], behind the last MMA
@@ -1600,7 +1602,12 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       // D fp32, A and B E4M3, both K-major, M = 128, N = n16
       const uint32_t idesc = (1u << 4) | (uint32_t(n16 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
       bool ok = true;
+      int chain = 0, begin = 0, end = nkb / chains;  // K blocks of the chain
       for (int i = 0; i < nkb; ++i) {
+        if (i == end) {
+          begin = end;
+          end = nkb * (++chain + 1) / chains;
+        }
         if (!(ok = wait(&bars->full[i % S], (i / S) & 1))) break;
         uint8_t* st = smem + (i % S) * stage;
         const uint64_t da = umma_desc_k128(smem_u32(st));
@@ -1609,7 +1616,8 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           const uint64_t db = umma_desc_k128(smem_u32(st + kDecStageA + p * g.tok * BK));
 #pragma unroll
           for (int k4 = 0; k4 < BK / 32; ++k4)
-            umma_f8(tmem_base, da + uint64_t(2 * k4), db + uint64_t(2 * k4), idesc, (i | p | k4) ? 1u : 0u);
+            umma_f8(tmem_base + uint32_t(chain * g.tile), da + uint64_t(2 * k4), db + uint64_t(2 * k4), idesc,
+                    ((i - begin) | p | k4) ? 1u : 0u);
         }
         if (i + S < nkb) umma_commit(&bars->empty[i % S]);
       }
@@ -1632,9 +1640,17 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     if (__all_sync(0xffffffffu, wait(&bars->acc, 0))) {
       tc_fence_after();
       for (int c0 = 16 * (warp >> 2); c0 < n16; c0 += 64) {
+        const uint32_t col = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(c0);
         uint32_t c[16];
-        tmem_ld16_nowait(tmem_base + (uint32_t(q * 32) << 16) + uint32_t(c0), c);
+        tmem_ld16_nowait(col, c);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int k = 1; k < chains; ++k) {
+          uint32_t d[16];
+          tmem_ld16_nowait(col + uint32_t(k * g.tile), d);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 16; ++i) c[i] = __float_as_uint(__uint_as_float(c[i]) + __uint_as_float(d[i]));
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           if (c0 + i < nt) part[(c0 + i) * 128 + rl] = __uint_as_float(c[i]);
@@ -1937,14 +1953,21 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
     auto slots_of = [&](int tile) { return ((tokens < tile ? tokens : tile) + 31) & ~31; };
     auto intake = [&](int tile) { return kb * mid_stage(pieces, slots_of(tile)) / cluster_of(tile); };
     // Tokens of a unit: 256, but where few hundred tokens make one wave of smaller units, 128, or 64 where K is short, if a CTA
-    // takes in no more than 100 KB in addition for it: the partial tile and the outputs are then shared out more evenly. (us
-    // per call, 256 and smaller: 1280 x 2560 at 200 tokens 13.1 and 12.0, at 300 16.6 and 13.0, at 512 17.5 and 15.5; 2560 x 640
-    // at 300 23.4 and 16.8; 2560 x 6144 at 300 36.9 and 33.1. Beyond that line: 2560 x 6144 at 400 39.0 and 52.9, 9216 x 2560 at
-    // 140 19.9 and 23.2, 2560 x 640 at 512 25.8 and 29.0; above 640 tokens level or slower.)
+    // takes in no more than 100 KB in addition for it and K is summed in no fewer chains (the error against fp64 grows with
+    // a chain's length: 2560 x 6144 at 300 tokens 1.10e-6 in three, 1.27e-6 in two). The partial tile and the outputs are then
+    // shared out more evenly. (us per call, 256 and smaller: 1280 x 2560 at 200 tokens 13.1 and 12.0, at 300 16.6 and 13.1;
+    // 2560 x 640 at 300 23.4 and 16.9, at 640 29.0 and 22.4; 2560 x 6144 at 300 36.9 and 33.3. Beyond the first line: 2560 x 6144
+    // at 400 39.0 and 52.9, 9216 x 2560 at 140 19.9 and 23.2, 2560 x 640 at 512 25.8 and 29.0; above 640 tokens level or
+    // slower.)
+    auto chains_of = [&](int tile) {
+      const int c = cluster_of(tile) * (kMidTok / tile);
+      return c < kb ? c : kb;
+    };
     g.tile = kMidTok;
     if (tokens > 160 && tokens <= 640)
       for (int tile = k <= 1024 ? 64 : 128; tile < kMidTok && g.tile == kMidTok; tile *= 2)
-        if (mid_units(tile) <= sm_count() && intake(tile) <= intake(kMidTok) + 100 * 1024) g.tile = tile;
+        if (mid_units(tile) <= sm_count() && intake(tile) <= intake(kMidTok) + 100 * 1024 && chains_of(tile) >= chains_of(kMidTok))
+          g.tile = tile;
     g.cluster = cluster_of(g.tile);
     g.tok = slots_of(g.tile);
     g.m_tiles = m_tiles_mid;
