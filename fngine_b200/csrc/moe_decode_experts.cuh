@@ -999,6 +999,13 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       const int act_bytes = down ? C::kDnAct : C::kGuAct, act_k = down ? INTER : H, ablk = down ? parity : task;
       if (parity == 0) gate_up_block_terms<GU, true>(blk, grid, sign_base, lv, act0, act_bytes, ablk, ntp, term, act_k);
       else gate_up_block_terms<GU, false>(blk, grid, sign_base, lv, act0, act_bytes, ablk, ntp, term, act_k);
+    } else if constexpr (GU == FB_FMT_IQ4_NL && DN == FB_FMT_IQ4_NL && INTER == 512) {
+      // one copy here too: instructions are what the warps wait for most (the two copies before: eight layers of
+      // eight tokens 357.3 us, 354.8 so)
+      if (!down || k < C::kDnRows / 32)
+        iq4nl_task_terms<8, 0>(down ? st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes : st + gu_row_off + task * C::kTaskBytes,
+                               lv, st + (down ? C::kDnTile : 2 * C::kGuPart), down ? C::kDnAct : C::kGuAct, down ? INTER : H,
+                               8 * (down ? parity : task), ntp, term);
     } else if (!down) {
       const uint8_t* blk = st + gu_row_off + task * C::kTaskBytes;
       const uint8_t* act0 = st + 2 * C::kGuPart;
