@@ -523,38 +523,27 @@ __device__ __forceinline__ void gate_up_block_terms(const uint8_t* blk, const ui
   }
 }
 
-// IQ4_NL: one task = NB consecutive 18-byte blocks of the lane's row, OFF bytes behind `wp`, against the pass's tokens;
-// blk0 = index of the first of them in the row. Even blocks start on a word (scale in the low half, codes two bytes
-// off), odd blocks on a half word (scale in the high half, codes aligned). Rows of 1440 and 288 bytes keep
-// eight blocks on 16-byte boundaries, the halves of 360-byte rows start on 8-byte boundaries (the second one four bytes
-// early): the widest loads without bank conflicts. term[t] = sum over the blocks, in block order, of isum * (d * d_act).
-template <int NB, int OFF>
+// IQ4_NL: one task = eight consecutive 18-byte blocks of the lane's row at `wp`, against the pass's tokens; blk0 = index of the
+// first of them in the row. Even blocks start on a word (scale in the low half, codes two bytes off), odd blocks on a half word
+// (scale in the high half, codes aligned). Rows of 1440 and 288 bytes keep eight blocks on 16-byte boundaries: the widest
+// loads. term[t] = sum over the blocks, in block order, of isum * (d * d_act). (Four blocks at a time, with their words moved
+// into place: half the code, eight layers of eight tokens 354.6 -> 351.8 us, but of one 132.8 -> 136.0.)
 __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlLevels& lv, const uint8_t* act0,
                                                  int act_bytes, int k, int blk0, int ntp, float (&term)[kTT]) {
-  constexpr int kWords = NB == 8 ? 36 : 46, kOff = OFF / 4;
-  uint32_t w[kWords];
-  if constexpr (NB == 8) {
+  uint32_t w[36];
 #pragma unroll
-    for (int c = 0; c < kWords / 4; ++c) {
-      const uint4 v = reinterpret_cast<const uint4*>(wp)[c];
-      w[4 * c] = v.x;
-      w[4 * c + 1] = v.y;
-      w[4 * c + 2] = v.z;
-      w[4 * c + 3] = v.w;
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < kWords / 2; ++c) {
-      const uint2 v = reinterpret_cast<const uint2*>(wp)[c];
-      w[2 * c] = v.x;
-      w[2 * c + 1] = v.y;
-    }
+  for (int c = 0; c < 9; ++c) {
+    const uint4 v = reinterpret_cast<const uint4*>(wp)[c];
+    w[4 * c] = v.x;
+    w[4 * c + 1] = v.y;
+    w[4 * c + 2] = v.z;
+    w[4 * c + 3] = v.w;
   }
   term[0] = term[1] = 0.0f;
   const uint8_t* act1 = act0 + (ntp == 2 ? act_bytes : 0);
 #pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    const int base = b % 2 == 0 ? kOff + 9 * b / 2 : kOff + (18 * b - 2) / 4;  // the word with the scale
+  for (int b = 0; b < 8; ++b) {
+    const int base = b % 2 == 0 ? 9 * b / 2 : (18 * b - 2) / 4;  // the word with the scale
     const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(b % 2 == 0 ? w[base] & 0xFFFFu : w[base] >> 16)));
     int lo[8], hi[8];
     iq4nl_addends32(lv, w, 2 * base + (b % 2 == 0 ? 1 : 2), lo, hi);
@@ -564,6 +553,33 @@ __device__ __forceinline__ void iq4nl_task_terms(const uint8_t* wp, const Iq4nlL
     if (ntp == 2) {
       const int s1 = dot32(lo, hi, reinterpret_cast<const int8_t*>(act1) + 32 * blk);
       term[1] = fmaf(float(s1), d * reinterpret_cast<const float*>(act1 + k)[blk], term[1]);
+    }
+  }
+}
+// The same for half a row of 640: ten blocks, two at a time from single words (rows of 360 bytes: two lanes share a bank), so
+// that the code stands in the kernel once and is short. (The warps waited for instructions most: with all ten blocks unrolled, once
+// for either half, eight layers of five IQ2_S + IQ4_NL tokens took 363 us, 327 so; the decode branch of four tokens 420, 378.)
+__device__ __forceinline__ void iq4nl_half_row_terms(const uint8_t* half, const Iq4nlLevels& lv, const uint8_t* act0, int act_bytes,
+                                                     int k, int blk0, int ntp, float (&term)[kTT]) {
+  term[0] = term[1] = 0.0f;
+  const uint8_t* act1 = act0 + (ntp == 2 ? act_bytes : 0);
+#pragma unroll 1
+  for (int p = 0; p < 5; ++p) {
+    uint32_t w[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) w[i] = reinterpret_cast<const uint32_t*>(half)[9 * p + i];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(b == 0 ? w[0] & 0xFFFFu : w[4] >> 16)));
+      int lo[8], hi[8];
+      iq4nl_addends32(lv, w, b == 0 ? 1 : 10, lo, hi);
+      const int blk = blk0 + 2 * p + b;
+      const int s0 = dot32(lo, hi, reinterpret_cast<const int8_t*>(act0) + 32 * blk);
+      term[0] = fmaf(float(s0), d * reinterpret_cast<const float*>(act0 + k)[blk], term[0]);
+      if (ntp == 2) {
+        const int s1 = dot32(lo, hi, reinterpret_cast<const int8_t*>(act1) + 32 * blk);
+        term[1] = fmaf(float(s1), d * reinterpret_cast<const float*>(act1 + k)[blk], term[1]);
+      }
     }
   }
 }
@@ -1003,14 +1019,14 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
       // one copy here too: instructions are what the warps wait for most (the two copies before: eight layers of
       // eight tokens 357.3 us, 354.8 so)
       if (!down || k < C::kDnRows / 32)
-        iq4nl_task_terms<8, 0>(down ? st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes : st + gu_row_off + task * C::kTaskBytes,
+        iq4nl_task_terms(down ? st + (32 * k + lane) * C::kDnRowBytes + parity * C::kDnTaskBytes : st + gu_row_off + task * C::kTaskBytes,
                                lv, st + (down ? C::kDnTile : 2 * C::kGuPart), down ? C::kDnAct : C::kGuAct, down ? INTER : H,
                                8 * (down ? parity : task), ntp, term);
     } else if (!down) {
       const uint8_t* blk = st + gu_row_off + task * C::kTaskBytes;
       const uint8_t* act0 = st + 2 * C::kGuPart;
       if constexpr (GU == FB_FMT_IQ4_NL) {
-        iq4nl_task_terms<8, 0>(blk, lv, act0, C::kGuAct, H, 8 * task, ntp, term);
+        iq4nl_task_terms(blk, lv, act0, C::kGuAct, H, 8 * task, ntp, term);
       } else if (parity == 0) {
         gate_up_block_terms<GU, true>(blk, grid, sign_base, lv, act0, C::kGuAct, task, ntp, term);
       } else {
@@ -1024,11 +1040,9 @@ experts_kernel(fb_moe_expert_layout L, fb_moe_decode_workspace ws, int phases, S
         else if (parity == 0) q2_0_task_terms<5, 0>(half, act0, C::kDnAct, INTER, 0, ntp, term);
         else q2_0_task_terms<5, 2>(half - 2, act0, C::kDnAct, INTER, 10, ntp, term);
       } else if constexpr (INTER == 512) {
-        iq4nl_task_terms<8, 0>(half, lv, act0, C::kDnAct, INTER, 8 * parity, ntp, term);
-      } else if (parity == 0) {
-        iq4nl_task_terms<10, 0>(half, lv, act0, C::kDnAct, INTER, 0, ntp, term);
+        iq4nl_task_terms(half, lv, act0, C::kDnAct, INTER, 8 * parity, ntp, term);
       } else {
-        iq4nl_task_terms<10, 4>(half - 4, lv, act0, C::kDnAct, INTER, 10, ntp, term);
+        iq4nl_half_row_terms(half, lv, act0, C::kDnAct, INTER, 10 * parity, ntp, term);
       }
     }
     float* part = partials + (s * C::kTasks + task) * (kTT * 32);
