@@ -1519,7 +1519,11 @@ struct MidArgs {
   int m_tiles, tile;         // row tiles, tokens of a unit (kMidTok or a power of two below it)
 };
 
-template <int PIECES>
+// CHAINS: units of fewer than kMidTok tokens, which sum their K in as many chains as fit the 256 columns, one behind the other,
+// added in order at the end. A kernel of its own: with the number of chains a variable of one kernel, units of kMidTok tokens took
+// up to 1.4 % longer (us per call, in a captured graph of such calls on different weights: 16384 x 2560 at 17 tokens 15.12 and
+// 15.33, 2560 x 6144 GrWrite at 70 14.66 and 14.83).
+template <int PIECES, bool CHAINS>
 __global__ void __launch_bounds__(kMidThreads, 1)
 fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const GemmArgs a,
                const MidArgs g) {
@@ -1529,11 +1533,11 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const int cluster = g.cluster, S = g.stages;
   const int unit = int(blockIdx.x) / cluster, rank = int(blockIdx.x) - unit * cluster;
   const int tile = unit / g.m_tiles, m = unit - tile * g.m_tiles;
-  const int t0 = tile * g.tile, nt = min(g.tile, a.M - t0), n16 = (nt + 15) & ~15;
+  const int unit_tok = CHAINS ? g.tile : kMidTok;
+  const int t0 = tile * unit_tok, nt = min(unit_tok, a.M - t0), n16 = (nt + 15) & ~15;
   const bool swiglu = a.kind == FB_EPI_SWIGLU;
   const int kbt = a.K / BK, kb0 = kbt * rank / cluster, nkb = kbt * (rank + 1) / cluster - kb0;
-  // Smaller units sum their K in as many chains as fit the 256 columns, one behind the other, added in order at the end.
-  const int chains = min(nkb, kMidTok / g.tile);
+  const int chains = CHAINS ? min(nkb, kMidTok / g.tile) : 1;
   const int stage = kDecStageA + PIECES * g.tok * BK, half_n = a.N >> 1;
   const int r0 = swiglu ? m * 64 : m * 128, r1 = swiglu ? half_n + m * 64 : m * 128 + 64;
   float* part = reinterpret_cast<float*>(smem);  // [token][row], behind the last MMA
@@ -1604,7 +1608,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       bool ok = true;
       int chain = 0, begin = 0, end = nkb / chains;  // K blocks of the chain
       for (int i = 0; i < nkb; ++i) {
-        if (i == end) {
+        if (CHAINS && i == end) {
           begin = end;
           end = nkb * (++chain + 1) / chains;
         }
@@ -1616,7 +1620,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           const uint64_t db = umma_desc_k128(smem_u32(st + kDecStageA + p * g.tok * BK));
 #pragma unroll
           for (int k4 = 0; k4 < BK / 32; ++k4)
-            umma_f8(tmem_base + uint32_t(chain * g.tile), da + uint64_t(2 * k4), db + uint64_t(2 * k4), idesc,
+            umma_f8(tmem_base + (CHAINS ? uint32_t(chain * g.tile) : 0u), da + uint64_t(2 * k4), db + uint64_t(2 * k4), idesc,
                     ((i - begin) | p | k4) ? 1u : 0u);
         }
         if (i + S < nkb) umma_commit(&bars->empty[i % S]);
@@ -1644,7 +1648,7 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         uint32_t c[16];
         tmem_ld16_nowait(col, c);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        for (int k = 1; k < chains; ++k) {
+        for (int k = 1; CHAINS && k < chains; ++k) {
           uint32_t d[16];
           tmem_ld16_nowait(col + uint32_t(k * g.tile), d);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -1680,14 +1684,18 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   };
   const int rows = swiglu ? 64 : 128, r = tid & (rows - 1);  // a thread keeps its row (the stride is a multiple of it)
   const int n = (swiglu ? m * 64 : m * 128) + r, limit = swiglu ? half_n : a.N;
+  // (Two loops, the one with loads ahead of the sum two tokens at a time, the other one token at a time. One loop for all
+  // kinds, two tokens at a time, in us as above: 2560 x 6144 GrWrite at 17 tokens 12.76 -> 12.35, at 450 37.8 -> 37.3, 16384 x 2560 at 40
+  // 16.6 -> 16.1, at 140 24.6 -> 24.1, 1280 x 2560 SwiGlu at 70 9.0 -> 8.5. GrWrite with the token's scale asked for behind the residual
+  // streams: 2560 x 6144 at 450 39.9.)
   if (complete && n < limit) {
     const float ws0 = row_scale(n), ws1 = swiglu ? row_scale(half_n + n) : 0.0f;
     const int per = kMidThreads / rows;  // tokens per turn of a CTA
+    if (a.kind == FB_EPI_GR_WRITE) {
 #pragma unroll 2
-    for (int t = rank * per + tid / rows; t < nt; t += cluster * per) {
-      const int row = t0 + t;
-      const float sa = a.act_scale[row];
-      if (a.kind == FB_EPI_GR_WRITE) {
+      for (int t = rank * per + tid / rows; t < nt; t += cluster * per) {
+        const int row = t0 + t;
+        const float sa = a.act_scale[row];
         float* X = static_cast<float*>(a.out) + size_t(row) * 4 * a.N + n;
         float x[4];
 #pragma unroll
@@ -1698,15 +1706,22 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         X[size_t(a.N)] = fmaf(inj.y, v, x[1]);
         X[2 * size_t(a.N)] = fmaf(inj.z, v, x[2]);
         X[3 * size_t(a.N)] = fmaf(inj.w, v, x[3]);
-      } else if (swiglu) {
-        const float gv = sum_of(t, r) * sa * ws0, uv = sum_of(t, r + 64) * sa * ws1;
-        static_cast<__nv_bfloat16*>(a.out)[size_t(row) * half_n + n] = __float2bfloat16_rn(gv / (1.0f + expf(-gv)) * uv);
-      } else if (a.kind == FB_EPI_STORE_BF16) {
-        static_cast<__nv_bfloat16*>(a.out)[size_t(row) * a.N + n] = __float2bfloat16_rn(sum_of(t, r) * sa * ws0);
-      } else {
-        float v = sum_of(t, r) * sa * ws0;
-        if (a.kind == FB_EPI_SHARED_SCALE) v /= 1.0f + expf(-a.gate_logit[size_t(row) * a.gate_stride]);
-        static_cast<float*>(a.out)[size_t(row) * a.N + n] = v;
+      }
+    } else {
+#pragma unroll 1
+      for (int t = rank * per + tid / rows; t < nt; t += cluster * per) {
+        const int row = t0 + t;
+        const float sa = a.act_scale[row];
+        if (swiglu) {
+          const float gv = sum_of(t, r) * sa * ws0, uv = sum_of(t, r + 64) * sa * ws1;
+          static_cast<__nv_bfloat16*>(a.out)[size_t(row) * half_n + n] = __float2bfloat16_rn(gv / (1.0f + expf(-gv)) * uv);
+        } else if (a.kind == FB_EPI_STORE_BF16) {
+          static_cast<__nv_bfloat16*>(a.out)[size_t(row) * a.N + n] = __float2bfloat16_rn(sum_of(t, r) * sa * ws0);
+        } else {
+          float v = sum_of(t, r) * sa * ws0;
+          if (a.kind == FB_EPI_SHARED_SCALE) v /= 1.0f + expf(-a.gate_logit[size_t(row) * a.gate_stride]);
+          static_cast<float*>(a.out)[size_t(row) * a.N + n] = v;
+        }
       }
     }
   }
@@ -1897,8 +1912,8 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
     if (a == cudaSuccess) a = opt_in_smem(fp8_gemm_kernel<2>, kGemmSmem);
     if (a == cudaSuccess) a = opt_in_smem(fp8_gemm_pair_kernel<1>, kGemmSmem2);
     if (a == cudaSuccess) a = opt_in_smem(fp8_gemm_pair_kernel<2>, kGemmSmem2);
-    if (a == cudaSuccess) a = opt_in_smem(fp8_mid_kernel<1>, kMidSmemMax);
-    if (a == cudaSuccess) a = opt_in_smem(fp8_mid_kernel<2>, kMidSmemMax);
+    for (auto* mid : {fp8_mid_kernel<1, false>, fp8_mid_kernel<2, false>, fp8_mid_kernel<1, true>, fp8_mid_kernel<2, true>})
+      if (a == cudaSuccess) a = opt_in_smem(mid, kMidSmemMax);
     return a;
   });
   if (attr != cudaSuccess) {
@@ -1976,10 +1991,9 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
     while (g.stages > 1 && mid_smem(pieces, g.tok, g.stages) > kMidSmemMax) --g.stages;
     const dim3 grid(unsigned(mid_units(g.tile) * g.cluster)), block(kMidThreads);
     const size_t smem = size_t(mid_smem(pieces, g.tok, g.stages));
-    const cudaError_t e = pieces == 2 ? launch_pdl_cluster(fp8_mid_kernel<2>, grid, block, smem, as_stream(stream),
-                                                           unsigned(g.cluster), map_a, map_b, ga, g)
-                                      : launch_pdl_cluster(fp8_mid_kernel<1>, grid, block, smem, as_stream(stream),
-                                                           unsigned(g.cluster), map_a, map_b, ga, g);
+    auto* kernel = g.tile < kMidTok ? (pieces == 2 ? fp8_mid_kernel<2, true> : fp8_mid_kernel<1, true>)
+                                    : (pieces == 2 ? fp8_mid_kernel<2, false> : fp8_mid_kernel<1, false>);
+    const cudaError_t e = launch_pdl_cluster(kernel, grid, block, smem, as_stream(stream), unsigned(g.cluster), map_a, map_b, ga, g);
     st = check_launch("linear_fp8");
     return st ? st : int32_t(e);
   }
