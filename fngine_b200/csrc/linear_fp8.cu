@@ -1687,7 +1687,8 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   // (Two loops, the one with loads ahead of the sum two tokens at a time, the other one token at a time. One loop for all
   // kinds, two tokens at a time, in us as above: 2560 x 6144 GrWrite at 17 tokens 12.76 -> 12.35, at 450 37.8 -> 37.3, 16384 x 2560 at 40
   // 16.6 -> 16.1, at 140 24.6 -> 24.1, 1280 x 2560 SwiGlu at 70 9.0 -> 8.5. GrWrite with the token's scale asked for behind the residual
-  // streams: 2560 x 6144 at 450 39.9.)
+  // streams: 2560 x 6144 at 450 39.9. bf16 outputs of a whole K, which have one partial tile, in a loop of their own: 16384 x 2560 at
+  // 100 20.9 -> 20.1, at 230 34.0 -> 31.6, and 0.3 to 0.7 % on the other calls.)
   if (complete && n < limit) {
     const float ws0 = row_scale(n), ws1 = swiglu ? row_scale(half_n + n) : 0.0f;
     const int per = kMidThreads / rows;  // tokens per turn of a CTA
@@ -1707,6 +1708,10 @@ fp8_mid_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         X[2 * size_t(a.N)] = fmaf(inj.z, v, x[2]);
         X[3 * size_t(a.N)] = fmaf(inj.w, v, x[3]);
       }
+    } else if (a.kind == FB_EPI_STORE_BF16 && cluster == 1) {
+#pragma unroll 1
+      for (int t = tid / rows; t < nt; t += per)
+        static_cast<__nv_bfloat16*>(a.out)[size_t(t0 + t) * a.N + n] = __float2bfloat16_rn(part[t * 128 + r] * a.act_scale[t0 + t] * ws0);
     } else {
 #pragma unroll 1
       for (int t = rank * per + tid / rows; t < nt; t += cluster * per) {
