@@ -108,13 +108,6 @@ __device__ __forceinline__ uint32_t mbar_test_wait(uint64_t* bar, uint32_t parit
       : "memory");
   return ok;
 }
-// Returns false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
 // 1-D bulk async copy global -> this CTA's shared memory, completion counted in bytes on `bar`.
 // Both addresses 16-byte aligned, bytes a multiple of 16. No multicast.
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
@@ -169,8 +162,6 @@ __device__ __forceinline__ void st_cluster_u32(const void* local, uint32_t cta, 
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(cta));
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-
-__device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float(uint32_t(b) << 16); }
 
 // Launch with the programmatic-stream-serialization attribute (the kernel calls pdl_wait_prior()
 // before touching memory written by its predecessor).

@@ -1,6 +1,6 @@
 // Device routines for the GGUF expert formats: codebook tables in shared memory, exact integer
 // decode of IQ3_S / IQ4_NL sub-blocks into dp4a operands, and the Q8_K / Q8_0 activation
-// quantizers. The GEMV kernels and the parity probes call the same functions.
+// quantizers. What the GEMV kernels and the parity probes share is said at the probes.
 //
 // Format definitions follow third_party/ggml-iq/ggml-iq.h:81-96 and the reference dequantizers
 // third_party/ggml-iq/ggml-iq.c:231-288 of the reference project.
@@ -93,21 +93,6 @@ __device__ __forceinline__ void iq3s_decode_sub(uint32_t qs_lo, uint32_t qs_hi, 
 // because every magnitude is odd.
 __device__ __forceinline__ int iq3s_signed(uint32_t g, uint32_t m) { return int((g ^ m) + (m & 0x01010101u)); }
 
-// sum_i s_i g_i a_i over 32 weights for one token: with x = g ^ m (negated bytes become -g-1),
-// sum s g a = dp4a(x, a) - dp4a(m, a) since m's 0xFF bytes are -1.
-__device__ __forceinline__ int iq3s_dot32(const uint32_t (&g)[8], const uint32_t (&m)[8], const int8_t* a) {
-  const int4 a0 = *reinterpret_cast<const int4*>(a);
-  const int4 a1 = *reinterpret_cast<const int4*>(a + 16);
-  const int av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-  int p = 0, n = 0;
-#pragma unroll
-  for (int l = 0; l < 8; ++l) {
-    p = __dp4a(int(g[l] ^ m[l]), av[l], p);
-    n = __dp4a(int(m[l]), av[l], n);
-  }
-  return p - n;
-}
-
 // dp4a of 8 signed weight words with 32 int8 activations at `a` (16-byte aligned shared memory).
 __device__ __forceinline__ int dot32(const int (&w)[8], const int8_t* a) {
   const int4 a0 = *reinterpret_cast<const int4*>(a);
@@ -137,18 +122,6 @@ __device__ __forceinline__ int dot32(const int (&w)[8], const int (&v)[8], const
   return s + t;
 }
 
-// 4 bytes at a static byte offset (a multiple of 2) of a word-aligned unit in shared memory.
-template <int OFF>
-__device__ __forceinline__ uint32_t ld4(const uint32_t* u) {
-  if constexpr (OFF % 4 == 0) return u[OFF / 4];
-  else return __byte_perm(u[OFF / 4], u[OFF / 4 + 1], 0x5432);
-}
-template <int OFF>
-__device__ __forceinline__ float ld_fp16(const uint32_t* u) {
-  const uint32_t v = u[OFF / 4] >> (8 * (OFF % 4));
-  return __half2float(__ushort_as_half(static_cast<unsigned short>(v & 0xFFFFu)));
-}
-
 // An IQ3_S block is a 2-byte scale followed by 27 words: 16 of index bytes, 2 of ninth bits, 8 of
 // signs, 1 of sub-block scales. In a 220-byte unit (two blocks, word aligned) the first block's
 // 27 words sit 2 bytes off word alignment, the second block's are aligned: S<MIS>(w, k) reads
@@ -157,34 +130,6 @@ template <bool MIS>
 __device__ __forceinline__ uint32_t iq3s_stream(const uint32_t* w, int k) {
   if constexpr (MIS) return __byte_perm(w[k], w[k + 1], 0x5432);
   else return w[k + 1];
-}
-
-// Integer dot of one IQ3_S block with TT activation blocks: bsum[t] = sum over its 8 sub-blocks of
-// (2*s+1) * sum_i w_i * a_t,i, exact in int32 (|bsum| < 2^24, so float(bsum) is exact).
-// act[t] points at the 256 int8 of the matching Q8_K block. Two runtime halves of four unrolled
-// sub-blocks keep the loop body inside the instruction cache.
-template <bool MIS, int TT>
-__device__ __forceinline__ void iq3s_block_idot(const uint32_t* w, const uint32_t* grid_lane,
-                                                const uint32_t* signtab, const int8_t* const (&act)[TT],
-                                                int (&bsum)[TT]) {
-  const uint32_t sc = iq3s_stream<MIS>(w, 26);
-#pragma unroll
-  for (int t = 0; t < TT; ++t) bsum[t] = 0;
-#pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    const uint32_t qh = iq3s_stream<MIS>(w, 16 + half);
-    const uint32_t sch = sc >> (16 * half);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int ib = 4 * half + i;
-      uint32_t g[8], m[8];
-      iq3s_decode_sub(iq3s_stream<MIS>(w, 2 * ib), iq3s_stream<MIS>(w, 2 * ib + 1), qh, 8 * i,
-                      iq3s_stream<MIS>(w, 18 + ib), grid_lane, signtab, g, m);
-      const int mult = 2 * int((sch >> (4 * i)) & 0xFu) + 1;
-#pragma unroll
-      for (int t = 0; t < TT; ++t) bsum[t] += iq3s_dot32(g, m, act[t] + 32 * ib) * mult;
-    }
-  }
 }
 
 // ------------------------------------------------------------------------------ IQ4_NL
@@ -215,28 +160,15 @@ __host__ __device__ constexpr int iq4nl_level(int i) {
   return lv[i];
 }
 __device__ __forceinline__ uint32_t upper_half(uint32_t w) { return __dp2a_lo(w, 0x0100u, 0u); }
-// One 32-weight block from its 16 nibble bytes (4 words). Output word 2m+h (m = word, h = half)
-// holds weights of elements {4m+2h, 4m+2h+16, 4m+2h+1, 4m+2h+17}: activations are stored in
-// that interleaved order (see q8_0_interleave_index). A byte-permute looks at the low 16 bits of its selector only, so
-// the selectors of both halves of a word are made at once: 11 operations per eight weights (13 half by half).
-__device__ __forceinline__ void iq4nl_decode32(const Iq4nlLevels& L, const uint32_t (&q)[4], int (&w)[8]) {
-#pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    const uint32_t sel = q[m] & 0x77777777u, pick = ((q[m] >> 1) & 0x44444444u) | 0x32103210u;
-    w[2 * m] = int(prmt(prmt(L.t0, L.t1, sel), prmt(L.t2, L.t3, sel), pick));
-    // (upper halves by a dot product with 0 and 1: the shift's pipe is the one the permutes keep busy; 1 to 3 % of a layer)
-    const uint32_t sel1 = upper_half(sel), pick1 = upper_half(pick);
-    w[2 * m + 1] = int(prmt(prmt(L.t0, L.t1, sel1), prmt(L.t2, L.t3, sel1), pick1));
-  }
-}
-
-// The same weights as two addends each, for dot products: with the upper bit of a code as a permute's sign-replicating bit, a
-// permute of the lower eight levels (all negative) gives the level, or -1 for an upper code; one of the upper eight levels
-// plus one (all positive), by the code with that bit turned round, gives level + 1, or 0 for a lower code. So
-// sum of level * a = dp4a(lo, a) + dp4a(hi, a), and nothing has to be picked. Codes = eight half words from half word `half0`
-// of `w` on (a permute looks at the low 16 bits of its selector, so halves need no alignment): 45 instructions per 32 weights
-// and token, 21 of them on the integer pipe, which was the busy one, where iq4nl_decode32 and one dp4a per four weights made
-// 54 and 38 (eight IQ4_NL layers of one token 143 -> 133 us, of eight 364 -> 356, of sixteen 599 -> 585).
+// One 32-weight block from its 16 code bytes, as two addends of every weight, for dot products. Word 2 m + h of either (m = word
+// of the codes, h = half) holds the elements {4m+2h, 4m+2h+16, 4m+2h+1, 4m+2h+17}: activations are stored in that interleaved
+// order (q8_0_interleave_index). With the upper bit of a code as a permute's sign-replicating bit, a permute of the lower eight
+// levels (all negative) gives the level, or -1 for an upper code; one of the upper eight levels plus one (all positive), by the
+// code with that bit turned round, gives level + 1, or 0 for a lower code. So sum of level * a = dp4a(lo, a) + dp4a(hi, a), and
+// nothing has to be picked. Codes = eight half words from half word `half0` of `w` on (a permute looks at the low 16 bits of its
+// selector, so halves need no alignment): 45 instructions per 32 weights and token, 21 of them on the integer pipe, which was the
+// busy one, where picking the level out of two permutes by a third, and one dp4a per four weights, made 54 and 38 (eight IQ4_NL
+// layers of one token 143 -> 133 us, of eight 364 -> 356, of sixteen 599 -> 585).
 constexpr bool iq4nl_signs_split() {
   for (int i = 0; i < 16; ++i)
     if (i < 8 ? iq4nl_level(i) >= 0 : iq4nl_level(i) <= 0 || iq4nl_level(i) > 126) return false;

@@ -1,6 +1,8 @@
-// Parity probes and the seeded expert-byte generator. The probes run the same device routines the
-// GEMV kernels use (iq_decode.cuh) and write results in the reference's own layouts, so dequantized
-// weights and int8 activations can be compared bit for bit with the CPU reference.
+// Parity probes and the seeded expert-byte generator. The probes write results in the reference's own layouts, so that
+// dequantized weights and int8 activations can be compared bit for bit with the CPU reference. The activation quantizers
+// and the IQ4_NL decoder (iq4nl_addends32) are the routines that the decode kernels run. The other weight formats are decoded here
+// from the same codebooks, but by plain look-ups: the kernels' own forms (iq3s_sub_dot, gate_up_sub, the prefill tables) never
+// make a weight by itself and are checked through the layers.
 #include "iq_decode.cuh"
 
 #include <cuda_bf16.h>
@@ -54,18 +56,25 @@ __global__ void __launch_bounds__(256) dequant_iq4nl_kernel(const uint8_t* __res
     const uint8_t* row = rows + int64_t(r) * row_bytes;
     for (int b = lane; b < k / 32; b += 32) {
       const uint8_t* blk = row + b * 18;
-      auto rd16 = [&](int off) { return uint32_t(blk[off]) | (uint32_t(blk[off + 1]) << 8); };
-      const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(rd16(0))));
-      uint32_t q[4];
+      // as the kernels meet a row of 18-byte blocks: even blocks start on a word, odd ones on a half word
+      uint32_t w[5];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) q[m] = rd16(2 + 4 * m) | (rd16(4 + 4 * m) << 16);
-      int w[8];
-      iq4nl_decode32(lv, q, w);
+      for (int i = 0; i < 5; ++i) {
+        const int at = 4 * i - (b & 1 ? 2 : 0);
+        const uint32_t lower = at >= 0 ? uint32_t(blk[at]) | (uint32_t(blk[at + 1]) << 8) : 0u;
+        const uint32_t upper = at + 2 < 18 ? uint32_t(blk[at + 2]) | (uint32_t(blk[at + 3]) << 8) : 0u;
+        w[i] = lower | (upper << 16);
+      }
+      const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(b & 1 ? w[0] >> 16 : w[0] & 0xFFFFu)));
+      int lo[8], hi[8];
+      if (b & 1) iq4nl_addends32(lv, w, 2, lo, hi);
+      else iq4nl_addends32(lv, w, 1, lo, hi);
       float* o = out + int64_t(r) * k + 32 * b;
 #pragma unroll
       for (int e = 0; e < 32; ++e) {
         const int pos = q8_0_interleave_index(e);
-        o[e] = __fmul_rn(d, float(int8_t(uint32_t(w[pos >> 2]) >> (8 * (pos & 3)))));
+        const int level = int8_t(uint32_t(lo[pos >> 2]) >> (8 * (pos & 3))) + int8_t(uint32_t(hi[pos >> 2]) >> (8 * (pos & 3)));
+        o[e] = __fmul_rn(d, float(level));
       }
     }
   }
