@@ -35,6 +35,7 @@
 // rate; see "decode-width projection" below, and "few row tiles" for the cluster kernel that takes all matrices of at most
 // one row tile per multiprocessor. fb_linear_fp8 routes T <= 16 there.
 #include "common.cuh"
+#include "mid_units.h"
 
 #include <cuda.h>
 
@@ -1211,7 +1212,7 @@ fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // first), and the partial tiles meet through distributed shared memory, added in a fixed order (repeated calls are
 // bitwise identical). One launch; of the workspace it uses the status word only. A CTA whose wait runs out tells the
 // others of its cluster ahead of the barrier that ends the sums, and none of them stores anything.
-constexpr int kSmallThreads = 512, kSmallMaxKb = 20, kSmallMaxCluster = 8;
+constexpr int kSmallThreads = 512, kSmallMaxKb = 20, kSmallMaxCluster = kMidMaxCluster;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallMaxStages = 8;
 struct SmallBars {
@@ -1499,7 +1500,7 @@ fp8_small_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16*
 // multiprocessors for 73 us. Here 128 weight rows are the M side of the MMA and up to 256 tokens the N side, and K is
 // shared by the CTAs of a cluster, whose partial tiles meet through distributed shared memory as in fp8_small_kernel
 // (added in CTA order: repeated calls are bitwise identical).
-constexpr int kMidThreads = 512, kMidTok = 256, kMidMaxStages = 8;
+constexpr int kMidThreads = 512, kMidMaxStages = 8;
 struct MidBars {
   uint64_t full[kMidMaxStages], empty[kMidMaxStages];
   uint64_t acc;
@@ -1507,9 +1508,8 @@ struct MidBars {
   int abort, failed;  // as in SmallBars
 };
 constexpr int kMidSmemMax = 232448;
-// Shared memory of a stage (16 KB of weights, `pieces` tiles of `tok` tokens) and of the whole block; the partial tile
-// reuses the stages.
-inline int mid_stage(int pieces, int tok) { return kDecStageA + pieces * tok * BK; }
+static_assert(kMidRowBytes == BK && kMidStageWeights == kDecStageA, "a K block");
+// Shared memory of the block; the partial tile reuses the stages.
 inline int mid_smem(int pieces, int tok, int stages) {
   const int ring = stages * mid_stage(pieces, tok), part = tok * 128 * 4;
   return 1024 + (ring > part ? ring : part) + int(sizeof(MidBars)) + 16;
@@ -1933,8 +1933,7 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
   // tokens: 1.3 - 2.2 times faster below that line, up to 2.4 times slower above it); below 256 tokens up to two waves of
   // 128-row tiles.
   const int m_tiles_mid = kind == FB_EPI_SWIGLU ? ((n >> 1) + 63) / 64 : (n + 127) / 128;
-  auto mid_units = [&](int tile) { return m_tiles_mid * ((tokens + tile - 1) / tile); };
-  const int units = mid_units(kMidTok);
+  const int units = m_tiles_mid * ((tokens + kMidTok - 1) / kMidTok);
   const int pair_work = ((tokens + BM2 - 1) / BM2) * (kind == FB_EPI_SWIGLU ? ((n >> 1) + 127) / 128 : (n + BN - 1) / BN);
   const bool mid = !force_single && (pair ? 2 * pair_work <= pair_count() : units <= 2 * sm_count());
   CUtensorMap map_a, map_b;
@@ -1965,36 +1964,15 @@ int32_t fb_linear_fp8(const void* x_bf16, int32_t tokens, const uint8_t* w_codes
     }
     const int kb = k / BK;
     MidArgs g;
-    auto cluster_of = [&](int tile) {
-      int c = kb < kSmallMaxCluster ? kb : kSmallMaxCluster;
-      while (c > 1 && resident[c] < mid_units(tile)) --c;
-      return c;
-    };
-    auto slots_of = [&](int tile) { return ((tokens < tile ? tokens : tile) + 31) & ~31; };
-    auto intake = [&](int tile) { return kb * mid_stage(pieces, slots_of(tile)) / cluster_of(tile); };
-    // Tokens of a unit: 256, but where few hundred tokens make one wave of smaller units, 128, or 64 where K is short, if a CTA
-    // takes in no more than 100 KB in addition for it and K is summed in no fewer chains (the error against fp64 grows with
-    // a chain's length: 2560 x 6144 at 300 tokens 1.10e-6 in three, 1.27e-6 in two). The partial tile and the outputs are then
-    // shared out more evenly. (us per call, 256 and smaller: 1280 x 2560 at 200 tokens 13.1 and 12.0, at 300 16.6 and 13.1;
-    // 2560 x 640 at 300 23.4 and 16.9, at 640 29.0 and 22.4; 2560 x 6144 at 300 36.9 and 33.3. Beyond the first line: 2560 x 6144
-    // at 400 39.0 and 52.9, 9216 x 2560 at 140 19.9 and 23.2, 2560 x 640 at 512 25.8 and 29.0; above 640 tokens level or
-    // slower.)
-    auto chains_of = [&](int tile) {
-      const int c = cluster_of(tile) * (kMidTok / tile);
-      return c < kb ? c : kb;
-    };
-    g.tile = kMidTok;
-    if (tokens > 160 && tokens <= 640)
-      for (int tile = k <= 1024 ? 64 : 128; tile < kMidTok && g.tile == kMidTok; tile *= 2)
-        if (mid_units(tile) <= sm_count() && intake(tile) <= intake(kMidTok) + 100 * 1024 && chains_of(tile) >= chains_of(kMidTok))
-          g.tile = tile;
-    g.cluster = cluster_of(g.tile);
-    g.tok = slots_of(g.tile);
+    const MidUnits u = mid_units(tokens, m_tiles_mid, kb, pieces, sm_count(), resident);
+    g.tile = u.tile;
+    g.cluster = u.cluster;
+    g.tok = u.slots;
     g.m_tiles = m_tiles_mid;
     g.stages = (kb + g.cluster - 1) / g.cluster;
     if (g.stages > kMidMaxStages) g.stages = kMidMaxStages;
     while (g.stages > 1 && mid_smem(pieces, g.tok, g.stages) > kMidSmemMax) --g.stages;
-    const dim3 grid(unsigned(mid_units(g.tile) * g.cluster)), block(kMidThreads);
+    const dim3 grid(unsigned(u.units * g.cluster)), block(kMidThreads);
     const size_t smem = size_t(mid_smem(pieces, g.tok, g.stages));
     auto* kernel = g.tile < kMidTok ? (pieces == 2 ? fp8_mid_kernel<2, true> : fp8_mid_kernel<1, true>)
                                     : (pieces == 2 ? fp8_mid_kernel<2, false> : fp8_mid_kernel<1, false>);

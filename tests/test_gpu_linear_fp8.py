@@ -381,10 +381,15 @@ def test_linear_fp8_wide_tiles(T, n, k, kind, path):
 
 @pytest.mark.parametrize("path", ["auto", "a8"])
 @pytest.mark.parametrize("T,n,k,kind", [
+    # (which units a count takes is asserted on the CPU, test_mid_units.py)
     (161, 1280, 2560, "swiglu"),        # units of 128 tokens: the first count that takes them, a ragged second unit
     (300, 2560, 6144, "gr_write"),      # three units, K over a cluster of two
-    (193, 2560, 640, "shared_scale"),   # units of 64 tokens, the last one of one token
+    (193, 2560, 640, "shared_scale"),   # units of 128 in clusters of three: 64 would sum K in fewer chains
+    (257, 2560, 640, "shared_scale"),   # units of 64 tokens, four chains for five K blocks, the last unit of one token
+    (257, 2560, 896, "gr_write"),       # four chains of one, two, two and two K blocks
+    (385, 1280, 896, "store_bf16"),     # units of 64 tokens in clusters of two, whose CTAs hold three and four chains
     (640, 2560, 640, "shared_scale"),   # the last count, too many units of 64 tokens for one wave: 128
+    (512, 1408, 1280, "store_f32"),     # units of 128 would not fit beside each other: 256
     (255, 192, 128, "store_f32"),       # one K block, no cluster, half a row tile
     (999, 256, 2560, "store_bf16"),     # the activation kernel's last count with a block per token
     (1001, 256, 2560, "store_f32"),     # and its first with a warp per token, a ragged last block
@@ -393,3 +398,46 @@ def test_linear_fp8_wide_tiles(T, n, k, kind, path):
 def test_units_and_splits_chosen_by_the_token_count(T, n, k, kind, path):
     """The smaller units of the middle widths and the two forms of the activation kernel, at the counts where they change."""
     test_linear_fp8_small_and_middle_widths(T, n, k, kind, path)
+
+
+@pytest.mark.parametrize("T,k", [(1001, 2560), (1004, 384), (1000, 2568)])
+def test_token_pieces_of_many_tokens_are_bit_exact(T, k):
+    """A warp per token (from 1000 tokens on, rows of at most 2560 values): codes, pieces and scales of whole and ragged blocks of
+    eight tokens against the host's, with rows of zeros and tiny values. Longer rows take a block per token."""
+    torch = _torch()
+    from fngine_b200 import linear
+    x = synth.activations(63, T, hidden=k) * np.logspace(-3, 3, T, dtype=np.float32)[:, None]
+    x[5] = x[T - 1] = 0.0
+    x[9, :100] *= 1e-4
+    xb = synth.to_bf16_bits(x)
+    xd = torch.from_numpy(xb.view(np.int16)).cuda().view(torch.bfloat16)
+    codes, scales = linear.fp8_quantize_tokens(xd)
+    want_c, want_s = O.quantize_tokens_e4m3(xb)
+    assert np.array_equal(codes.cpu().numpy(), want_c)
+    assert np.array_equal(scales.cpu().numpy().view(np.uint32), want_s.view(np.uint32))
+    hi, lo, sc = linear.fp8_split_tokens(xd)
+    w_hi, w_lo, w_sc = O.split_tokens_e4m3x2(xb)
+    assert np.array_equal(hi.cpu().numpy(), w_hi) and np.array_equal(lo.cpu().numpy(), w_lo)
+    assert np.array_equal(sc.cpu().numpy().view(np.uint32), w_sc.view(np.uint32))
+
+
+def test_smaller_units_sum_in_shorter_chains():
+    """300 tokens of 2560 x 6144 take units of 128 tokens in clusters of two, two chains of twelve K blocks in each CTA; the same
+    rows among 641 tokens take units of 256 in clusters of two, one chain of 24. An fp32 chain's error grows with its length
+    (0.82 of it measured here, 1 without the second chain), and it is the sums' only error: the inputs' products are exact."""
+    torch = _torch()
+    from fngine_b200 import linear
+    n, k = 2560, 6144
+    weight = make_weight(torch, 311, n, k, False)
+    x = bf16_tensor(torch, synth.activations(312, 641, hidden=k))
+    pieces = [p.cpu().numpy() for p in linear.fp8_split_tokens(x)]  # the values that the sums are of
+    tab = O.e4m3_table().astype(np.float64)
+    kept = torch.from_numpy((tab[pieces[0]] + tab[pieces[1]]) * pieces[2].astype(np.float64)[:, None]).cuda()
+    ref = exact_acc(torch, kept[:300], weight)
+    err = []
+    for T in (300, 641):
+        out = torch.full((T, n), float("nan"), dtype=torch.float32, device="cuda")
+        linear.linear_fp8(x[:T], weight, linear.store_f32(out), linear.linear_fp8_workspace(weight, T))
+        torch.cuda.synchronize()
+        err.append(float((out[:300].double() - ref).norm() / ref.norm()))
+    assert err[0] <= 0.9 * err[1] and err[1] <= 5e-6, err
