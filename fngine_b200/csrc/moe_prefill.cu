@@ -142,10 +142,15 @@ __device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) {
 // global memory (so all earlier ones are complete too), and data of a predecessor is never read through const __restrict__
 // pointers, which would allow the load ahead of the wait. Layers of 96 IQ4_NL
 // tokens 373 -> 355 us, of 50 tokens at 640 268 -> 248.
-// Pairs are counted and numbered in one pass: a block counts its pairs in shared memory (the count a pair finds is its number
-// within the block), adds the sums to the expert's count once, and the value it meets there plus the block's number is the
-// pair's number within its expert, left in token_pair for the scatter kernel. (One atomic per pair, in two kernels, met a
-// popular expert's counter 4000 times at 8192 tokens.)
+// From kBlockNumbers tokens on, pairs are counted and numbered in one pass by blocks: a block counts its pairs in shared memory
+// (the count a pair finds is its number within the block), adds the sums to the expert's count once, and the value it meets
+// there plus the block's number is the pair's number within its expert, left in token_pair for the scatter kernel. (One atomic
+// per pair, in two kernels, met a popular expert's counter 4000 times at 8192 tokens: the route call 41 us, 20.5 so.) With fewer
+// tokens the blocks' clearing and adding costs more than it saves: the route call takes every pair's number from the expert's
+// count itself (us, by blocks / so: 1 token 10.3 / 9.2, 64 11.3 / 10.4, 400 11.4 / 10.5, 1000 level, zipf-distributed experts at 1500 12.4 /
+// 13.2), the one for dispatched rows counts first and numbers in the scatter kernel (100 rows 10.3 / 8.3, 300 10.3 / 8.4,
+// 1000 level, 2048 10.4 / 12.4).
+constexpr int kBlockNumbers = 1000;
 struct PairNumbers {
   int count[kExperts];  // pairs of the block, then the pairs of blocks before it
   __device__ __forceinline__ void clear(int threads) {
@@ -160,19 +165,21 @@ struct PairNumbers {
   }
 };
 
-// Top-10 per token (one warp each, PER_WARP in turn), per-expert pair counts and the pairs' numbers (token_pair, may be absent).
+// Top-10 per token (one warp each, PER_WARP in turn), per-expert pair counts and the pairs' numbers (token_pair, may be absent;
+// BLOCKS: by blocks). Rows of equal logits take the general path behind the pruned one: 2.3 us with the general path alone, 3.9 for
+// 1 to 4 tokens, 9.4 and 12.7 where all rows of 4096 are so.
 // PER_WARP 4 from 4096 tokens on: fewer meetings on a popular expert's counter; below that single tokens fill the GPU.
 // The routing launches of 8192 tokens together: 45 us, 25 so (selection by the pruned search and numbering).
-template <int PER_WARP>
+template <int PER_WARP, bool BLOCKS>
 __global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int stride, int T, int32_t* topk_e, float* topk_w,
                                                       int32_t* count, int32_t* token_pair) {
-  __shared__ PairNumbers s_num;
+  __shared__ PairNumbers s_num;  // (BLOCKS only)
   __shared__ __align__(16) uint2 s_scratch[8][32];
   __shared__ int s_ids[8][kTopK];
   __shared__ float s_vals[8][kTopK];
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = (blockIdx.x * 8 + warp) * PER_WARP;
-  if (token_pair) {
+  if (BLOCKS) {
     s_num.clear(256);
     __syncthreads();
   }
@@ -196,11 +203,12 @@ __global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int s
         if (lane == k) wt = w[k];
       topk_e[t * kTopK + lane] = id[i];
       topk_w[t * kTopK + lane] = wt;
-      if (token_pair) number[i] = s_num.add(id[i]);
+      if constexpr (BLOCKS) number[i] = s_num.add(id[i]);
+      else if (token_pair) token_pair[t * kTopK + lane] = atomicAdd(&count[id[i]], 1);
     }
     __syncwarp();
   }
-  if (!token_pair) return;
+  if constexpr (!BLOCKS) return;
   __syncthreads();
   s_num.publish(count, 256);
   __syncthreads();
@@ -213,13 +221,16 @@ __global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int s
 // experts other ranks own ([lo, hi) is this rank's range) become -1 and take no part. With a share
 // table (placement with copies) the rule is per expert instead: share[e] < 0 = not held here, else
 // (n << 8) | i = this rank holds copy i of n and takes the rows r with r % n == i.
+template <bool BLOCKS>
 __global__ void __launch_bounds__(256) pf_import_kernel(const int32_t* in_e, const float* in_w, int lo, int hi,
                                                         const int32_t* share, int n, int32_t* topk_e, float* topk_w,
                                                         int32_t* count, int32_t* token_pair) {
-  __shared__ PairNumbers s_num;
+  __shared__ PairNumbers s_num;  // (BLOCKS only)
   pdl_launch_dependents();
-  s_num.clear(256);
-  __syncthreads();
+  if constexpr (BLOCKS) {
+    s_num.clear(256);
+    __syncthreads();
+  }
   pdl_wait_prior();
   const int i = blockIdx.x * 256 + threadIdx.x;
   int e = -1, number = 0;
@@ -233,8 +244,13 @@ __global__ void __launch_bounds__(256) pf_import_kernel(const int32_t* in_e, con
     if (!local) e = -1;
     topk_e[i] = e;
     topk_w[i] = in_w[i];
-    if (local) number = s_num.add(e);
+    if constexpr (BLOCKS) {
+      if (local) number = s_num.add(e);
+    } else {
+      if (local) atomicAdd(&count[e], 1);
+    }
   }
+  if constexpr (!BLOCKS) return;
   __syncthreads();
   s_num.publish(count, 256);
   __syncthreads();
@@ -262,7 +278,7 @@ __device__ __forceinline__ void list_tiles(int expert, int first_pair, int count
     if (at < max_tiles) tiles[at] = make_int4(expert, 0, first_pair + full * TILE, rest);
   }
 }
-__global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int32_t* offset, int4* tiles_gu,
+__global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int32_t* offset, int32_t* cursor, int4* tiles_gu,
                                                       int4* tiles_dn, int32_t* meta, int inter, int max_units_gu,
                                                       int max_units_dn) {
   pdl_launch_dependents();
@@ -294,6 +310,7 @@ __global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int3
     total += s_scan[i];
   }
   offset[tid] = first;
+  cursor[tid] = 0;
   __syncthreads();
   const int mg = inter / kTileM, md = H / kTileM;
   if (warp < 2) {  // warp k: list k
@@ -316,11 +333,12 @@ __global__ void __launch_bounds__(512) pf_scan_kernel(const int32_t* count, int3
   list_tiles<kTileNDown>(tid, first, c, s_cursor[1], tiles_dn, max_units_dn / md);
 }
 
-// Pairs grouped by expert, a pair's place being its number within the expert. The numbers depend on the atomics, the results do
+// Pairs grouped by expert, a pair's place being its number within the expert (from token_pair; CURSOR: taken here). The numbers depend on the atomics, the results do
 // not: every pair's h and y rows depend only on (token, expert) and the combine adds a token's ten rows in ascending-expert
 // order.
+template <bool CURSOR>
 __global__ void __launch_bounds__(256) pf_scatter_kernel(const int32_t* topk_e, const float* topk_w, const int32_t* offset,
-                                                         int32_t* pair_token, float* pair_weight, int32_t* token_pair, int T) {
+                                                         int32_t* cursor, int32_t* pair_token, float* pair_weight, int32_t* token_pair, int T) {
   pdl_launch_dependents();
   pdl_wait_prior();
   const int i = blockIdx.x * 256 + threadIdx.x;
@@ -330,7 +348,7 @@ __global__ void __launch_bounds__(256) pf_scatter_kernel(const int32_t* topk_e, 
     token_pair[i] = -1;
     return;
   }
-  const int pos = offset[e] + token_pair[i];
+  const int pos = offset[e] + (CURSOR ? atomicAdd(&cursor[e], 1) : token_pair[i]);
   pair_token[pos] = i / kTopK;
   pair_weight[pos] = topk_w[i];
   token_pair[i] = pos;
@@ -492,13 +510,13 @@ cudaError_t launch_grouped(const GgArgs& a, const GgMaps& maps, cudaStream_t str
 }
 
 // Offsets, token tiles and pair lists from the counts and the top-10 entries of `rows` tokens.
-cudaError_t launch_pair_lists(const fb_moe_prefill_workspace* ws, int rows, cudaStream_t s) {
-  const cudaError_t e = launch_pdl(pf_scan_kernel, dim3(1), dim3(512), 0, s, ws->expert_count, ws->expert_offset,
+cudaError_t launch_pair_lists(const fb_moe_prefill_workspace* ws, int rows, bool numbered, cudaStream_t s) {
+  const cudaError_t e = launch_pdl(pf_scan_kernel, dim3(1), dim3(512), 0, s, ws->expert_count, ws->expert_offset, ws->expert_cursor,
                                    static_cast<int4*>(ws->units_gate_up), static_cast<int4*>(ws->units_down),
                                    ws->meta, ws->inter, ws->max_units_gate_up, ws->max_units_down);
   if (e != cudaSuccess) return e;
-  return launch_pdl(pf_scatter_kernel, dim3((rows * kTopK + 255) / 256), dim3(256), 0, s, ws->topk_expert, ws->topk_weight,
-                    ws->expert_offset, ws->pair_token, ws->pair_weight, ws->token_pair, rows);
+  return launch_pdl(numbered ? pf_scatter_kernel<false> : pf_scatter_kernel<true>, dim3((rows * kTopK + 255) / 256), dim3(256), 0, s,
+                    ws->topk_expert, ws->topk_weight, ws->expert_offset, ws->expert_cursor, ws->pair_token, ws->pair_weight, ws->token_pair, rows);
 }
 
 size_t up256(size_t v) { return (v + 255) & ~size_t(255); }
@@ -617,9 +635,10 @@ int32_t fb_moe_route(const float* router_logits, int32_t logits_stride, const vo
   if (e == cudaSuccess) e = clear_fixed(ws, tokens, s);
   if (e != cudaSuccess) return check_launch("route: memset");
   const int per_warp = tokens >= 4096 ? 4 : 1;
-  e = launch_pdl(per_warp == 4 ? pf_topk_kernel<4> : pf_topk_kernel<1>, dim3((tokens + 8 * per_warp - 1) / (8 * per_warp)), dim3(256),
+  auto* kernel = per_warp == 4 ? pf_topk_kernel<4, true> : tokens >= kBlockNumbers ? pf_topk_kernel<1, true> : pf_topk_kernel<1, false>;
+  e = launch_pdl(kernel, dim3((tokens + 8 * per_warp - 1) / (8 * per_warp)), dim3(256),
                  0, s, router_logits, logits_stride, tokens, ws->topk_expert, ws->topk_weight, ws->expert_count, ws->token_pair);
-  if (e == cudaSuccess) e = launch_pair_lists(ws, tokens, s);
+  if (e == cudaSuccess) e = launch_pair_lists(ws, tokens, true, s);
   const int32_t st = check_launch("route");
   return st ? st : int32_t(e);
 }
@@ -628,7 +647,7 @@ int32_t fb_moe_topk(const float* router_logits, int32_t logits_stride, int32_t t
                     float* topk_weight, void* stream) {
   if (!router_logits || logits_stride < kExperts || tokens < 1 || !topk_expert || !topk_weight)
     return invalid("topk: bad arguments");
-  const cudaError_t e = launch_pdl(pf_topk_kernel<1>, dim3((tokens + 7) / 8), dim3(256), 0, as_stream(stream), router_logits,
+  const cudaError_t e = launch_pdl(pf_topk_kernel<1, false>, dim3((tokens + 7) / 8), dim3(256), 0, as_stream(stream), router_logits,
                                    logits_stride, tokens, topk_expert, topk_weight, static_cast<int32_t*>(nullptr),
                                    static_cast<int32_t*>(nullptr));
   const int32_t st = check_launch("topk");
@@ -659,9 +678,9 @@ static int32_t route_ep_impl(const int32_t* topk_expert, const float* topk_weigh
   if (e == cudaSuccess) e = clear_fixed(ws, rows, s);
   if (e != cudaSuccess) return check_launch("route_ep: memset");
   const int n = rows * kTopK;
-  e = launch_pdl(pf_import_kernel, dim3((n + 255) / 256), dim3(256), 0, s, topk_expert, topk_weight, expert_lo, expert_hi, share,
+  e = launch_pdl(rows >= kBlockNumbers ? pf_import_kernel<true> : pf_import_kernel<false>, dim3((n + 255) / 256), dim3(256), 0, s, topk_expert, topk_weight, expert_lo, expert_hi, share,
                  n, ws->topk_expert, ws->topk_weight, ws->expert_count, ws->token_pair);
-  if (e == cudaSuccess) e = launch_pair_lists(ws, rows, s);
+  if (e == cudaSuccess) e = launch_pair_lists(ws, rows, rows >= kBlockNumbers, s);
   const int32_t st = check_launch("route_ep");
   return st ? st : int32_t(e);
 }

@@ -233,7 +233,7 @@ typedef struct fb_moe_prefill_workspace {
   int32_t* meta;          /* [0] gate/up units [1] down units [2] pairs */
   int32_t* expert_count;  /* [512] */
   int32_t* expert_offset; /* [513] */
-  int32_t* expert_cursor; /* [512], not used */
+  int32_t* expert_cursor; /* [512] */
   int32_t* topk_expert;   /* [capacity][10] */
   float* topk_weight;     /* [capacity][10] */
   int32_t* pair_token;    /* [capacity*10] pairs grouped by expert */

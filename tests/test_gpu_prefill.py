@@ -506,9 +506,9 @@ def test_token_boxes_and_gate_up_matrices_at_any_even_address(fg, fd, inter):
         assert ws.status() == 0 and torch.equal(got, y), (g_at, u_at)
 
 
-@pytest.mark.parametrize("T", [1, 31, 4095, 4099])
+@pytest.mark.parametrize("T", [1, 31, 999, 1000, 4095, 4099])
 def test_route_numbers_every_pair_once(T):
-    """Selection and pair lists of one and of four tokens per warp, ragged: the ten largest logits (NaN never wins, equal
+    """Selection and pair lists of one and of four tokens per warp, ragged, pairs numbered one by one and by blocks: the ten largest logits (NaN never wins, equal
     logits go to the lower id), every pair in its expert's range exactly once; the same for the half of the experts that a
     shard holds."""
     torch = _torch()
