@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(128) router_kernel(const __nv_bfloat16* w, int
 
 // The same logits, bit for bit, at prefill width (tokens > kMaxTok). Bound: the fp32 pipe (tokens x rows x 2560
 // multiply-adds). router_kernel above re-reads x for every row and keeps four tokens in flight: 0.96 us per token,
-// 963 us at 1003 tokens; this kernel takes 90 us there (3.7 waves of blocks).
+// 963 us at 1003 tokens; this kernel takes 87 us there (3.7 waves of blocks).
 // A block owns 32 rows (ROWS) x 32 tokens; its sixteen warps split K the way router_kernel's lanes do: the partial sum of
 // lane l (elements 256 c + 8 l + i, added over c, then i) belongs to warp l mod 16, which adds those of lanes l and
 // l + 16; the sixteen results meet in shared memory in the butterfly's order. A thread accumulates 8 rows x 4 tokens. bf16
@@ -231,8 +231,9 @@ __device__ __forceinline__ uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
   return d;
 }
-__device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
+// 16 bytes, or 16 zeros (nothing is read then).
+__device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src, bool read) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src), "r"(read ? 16 : 0) : "memory");
 }
 
 template <bool XBF16, int ROWS>
@@ -244,21 +245,26 @@ __global__ void __launch_bounds__(512, 1) router_tile_kernel(const __nv_bfloat16
   pdl_wait_prior();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row_base = blockIdx.x * ROWS, tok_base = blockIdx.y * kRtTok;
-  // a warp copies two weight rows and two token rows of a chunk; rows and tokens beyond the end repeat the last one
-  // (they are computed and not stored)
+  // a warp copies two weight rows and two token rows of a chunk; rows and tokens beyond the end are zeros (they are computed
+  // and not stored). Repeats of the last one in their place were read by all warps at once, and the copies waited for that
+  // one line (513 rows, bf16, us: 17 tokens 13.2 -> 8.9, 33 21.5 -> 10.0, 100 17.3 -> 13.7, 1003 89.9 -> 87.2).
   auto fetch = [&](int c) {
     uint8_t* buf = smem + (c % kRtBufs) * kBuf;
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       const int r = warp + 16 * p;
-      if (r < ROWS) cp_async_16(buf + r * kRtWPitch + 16 * lane, w + size_t(min(row_base + r, rows - 1)) * H + kRtChunk * c + 8 * lane);
+      if (r < ROWS) {
+        const bool in = row_base + r < rows;
+        cp_async_16(buf + r * kRtWPitch + 16 * lane, w + size_t(in ? row_base + r : 0) * H + kRtChunk * c + 8 * lane, in);
+      }
       uint8_t* xd = buf + ROWS * kRtWPitch + r * kXPitch + 16 * lane;
-      const size_t at = size_t(min(tok_base + r, tokens - 1)) * H + kRtChunk * c;
+      const bool in = tok_base + r < tokens;
+      const size_t at = size_t(in ? tok_base + r : 0) * H + kRtChunk * c;
       if constexpr (XBF16) {
-        cp_async_16(xd, static_cast<const __nv_bfloat16*>(xv) + at + 8 * lane);
+        cp_async_16(xd, static_cast<const __nv_bfloat16*>(xv) + at + 8 * lane, in);
       } else {
-        cp_async_16(xd, static_cast<const float*>(xv) + at + 4 * lane);
-        cp_async_16(xd + 512, static_cast<const float*>(xv) + at + 128 + 4 * lane);
+        cp_async_16(xd, static_cast<const float*>(xv) + at + 4 * lane, in);
+        cp_async_16(xd + 512, static_cast<const float*>(xv) + at + 128 + 4 * lane, in);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -1600,8 +1606,8 @@ int32_t fb_router_logits(const void* w_bf16, int32_t rows, const void* x, int32_
   if (!w_bf16 || !x || !logits || rows <= 0 || tokens <= 0 || logits_stride < rows)
     return invalid("router_logits: bad arguments");
   if (tokens > kMaxTok) {
-    // Tiles of fewer rows while they run as one wave (513 rows, us: 17 tokens 26.7 -> 14.6, 40 27.1 -> 19.2, 100 28.0 ->
-    // 20.2); beyond that each wave of smaller blocks costs as much as it saves.
+    // Tiles of fewer rows while they run as one wave (513 rows, us, while rows beyond the end were still read: 17 tokens 26.7 ->
+    // 14.6, 40 27.1 -> 19.2, 100 28.0 -> 20.2); beyond that each wave of smaller blocks costs as much as it saves.
     const int tok_tiles = (tokens + kRtTok - 1) / kRtTok;
     auto tiles = [&](int r) { return ((rows + r - 1) / r) * tok_tiles; };
     auto launch = [&](auto kernel, PerDeviceOnce& once, int r, int smem) {
