@@ -34,6 +34,10 @@
 // kept exactly and the same epilogues, a stream over the weight codes that reaches 0.9 of the HBM copy
 // rate; see "decode-width projection" below, and "few row tiles" for the cluster kernel that takes all matrices of at most
 // one row tile per multiprocessor. fb_linear_fp8 routes T <= 16 there.
+//
+// Times of calls in this file ("us per call"), unless a comment says otherwise: device events around eight calls on eight
+// weights one after another (one weight from 513 tokens on), on two sets of weights and inputs in turn, the best of six runs.
+// With more sets in turn a call of many tokens takes longer (4096 x 9216 x 2560: 137 and 160 us).
 #include "common.cuh"
 #include "mid_units.h"
 
@@ -153,10 +157,11 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t pair) {
   return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
+constexpr int kSplitWarpTokens = 1000, kSplitWarpPer = 10;  // 16-byte pieces of a row that a lane holds
 template <int GROUP>
 __global__ void __launch_bounds__(256) fp8_quantize_tokens_kernel(const __nv_bfloat16* x, int tokens, int K, uint8_t* codes,
                                                                   uint8_t* codes_lo, float* scales, uint32_t* status) {
-  constexpr int kPer = GROUP == 256 ? 2 : 10;
+  constexpr int kPer = GROUP == 256 ? 2 : kSplitWarpPer;
   pdl_wait_prior();
   // (behind the wait: fp8_mid_kernel asks for its weights, which the kernel ahead of this one may have written, before it
   // waits for this one; nor do its early loads compete with the call before)
@@ -1826,14 +1831,14 @@ const int* small_clusters() {
   return e == cudaSuccess ? table : nullptr;
 }
 
-// The activation kernel of `tokens` rows; `chained`: it may start while the call before runs out. A warp per token where there
-// are enough of them for all warps and a row fits its registers (us per call: 9216 x 2560 at 4096 tokens 135.1 -> 133.5,
-// 1280 x 2560 at 4000 50.0 -> 48.5, at 1003 22.6 -> 22.2; level at 600 and 1200); a block per token elsewhere (with warps,
-// 2560 x 6144 at 300 36.9 -> 41.0, 16384 x 2560 at 30 16.0 -> 17.0).
-constexpr int kSplitWarpTokens = 1000;
+// The activation kernel of `tokens` rows; `chained`: it may start while the call before runs out. A warp per token from
+// kSplitWarpTokens tokens on, where a row fits a warp's registers; a block per token elsewhere. (Whole calls in captured graphs, us,
+// block / warp: 1280 x 2560 SwiGlu at 100 tokens 9.5 / 10.0, at 300 12.8 / 13.2, at 600 17.1 / 17.4, at 800 21.0 / 21.2, at 1000 23.7 / 21.6,
+// at 1184 27.5 / 26.9, at 4000 50.4 / 48.8; 2560 x 640 at 300 16.8 / 16.7, at 1000 17.3 / 16.5, at 4000 34.8 / 32.2; 9216 x 2560 at 300 24.9 / 25.7, at 800
+// 38.7 / 38.9, at 2000 75 / 71; with warps for rows longer than their registers, 2560 x 6144 at 300 36.9 -> 41.0.)
 cudaError_t launch_split(bool chained, const __nv_bfloat16* x, int tokens, int k, uint8_t* codes, uint8_t* codes_lo, float* scales,
                          uint32_t* status, cudaStream_t stream) {
-  const bool warps = tokens >= kSplitWarpTokens && k <= 2560;
+  const bool warps = tokens >= kSplitWarpTokens && k <= 32 * 8 * kSplitWarpPer;
   auto* kernel = warps ? fp8_quantize_tokens_kernel<32> : fp8_quantize_tokens_kernel<256>;
   const dim3 grid(unsigned(warps ? (tokens + 7) / 8 : tokens));
   if (chained) return launch_pdl(kernel, grid, dim3(256), 0, stream, x, tokens, k, codes, codes_lo, scales, status);

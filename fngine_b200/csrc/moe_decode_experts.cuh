@@ -78,9 +78,10 @@ __device__ __forceinline__ void iq3s_sub_dot(uint32_t qs_lo, uint32_t qs_hi, uin
   for (int l = 0; l < 8; ++l) {
     const uint32_t g = lds_word(__dp2a_lo(idx[l >> 1], (l & 1) ? 0x8000u : 0x0080u, grid_at));
     // byte0 = the pre-scaled nibble of look-up l, bytes 1-3 = the table's address bytes
-    // (computing the masks instead - isolate the nibble, one wide multiply that sends bit j to the top of
-    // byte j, one sign-replicating byte-permute - frees a third of the shared-memory wavefronts but the
-    // multiplies queue up in the dispatch stage: measured 96 us against 80 us per layer launch)
+    // (Computing the masks instead frees a third of the shared-memory wavefronts, and loses: isolating the nibble, one wide multiply
+    // that sends bit j to the top of byte j and one sign-replicating byte-permute took 96 us a layer launch of sixteen tokens where
+    // loads took 80, the multiplies queuing up in the dispatch stage; a later form without the isolation, see gate_up_sub, eight
+    // layers in 640 us where loads take 626.)
     const uint32_t maddr = prmt((l & 1) ? s_odd : s_even, sign_base, 0x7650u | uint32_t(l >> 1));
     x[l] = g ^ lds_word(maddr);
   }

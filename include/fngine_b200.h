@@ -256,7 +256,9 @@ int32_t fb_moe_route(const float* router_logits, int32_t logits_stride, const vo
                      int32_t layer, const uint32_t* seq, void* control, int32_t tokens,
                      const fb_moe_prefill_workspace* ws, void* stream);
 /* moe_grouped_gate_up, src/kernels/moe/moe.h:209-211: h[pair] = bf16(silu(gate . x) * (up . x)), x bf16
- * [tokens][2560]. `expert_blob` is the device table of blob addresses ([512]) or NULL to address
+ * [tokens][2560]. Matrices may lie at any even address; the aligned 16-byte words that hold the first and last bytes
+ * of a gate or up matrix are read whole.
+ * `expert_blob` is the device table of blob addresses ([512]) or NULL to address
  * expert e at layout->slots + e * blob_stride. */
 int32_t fb_moe_grouped_gate_up(const fb_moe_expert_layout* layout, const uint8_t* const* expert_blob, const void* x_bf16,
                                int32_t tokens, const fb_moe_prefill_workspace* ws, void* stream);

@@ -547,3 +547,40 @@ def test_route_numbers_every_pair_once(T):
     L.check(L.load().fb_moe_route_ep(ed.data_ptr(), wd.data_ptr(), 0, 256, T, C.byref(ws.ws), torch.cuda.current_stream().cuda_stream), "route_ep")
     torch.cuda.synchronize()
     check(np.arange(512) < 256)
+
+
+def test_h_of_large_gates():
+    """Gates from a hundredth to thousands, of both signs: h is one bf16 rounding of silu(g) * u in fp64, plus what fp32 sums of g
+    and u move it; far below zero it is zero and nothing is NaN. (silu is computed as g / (1 + 2^(-g log2 e)); its error, 2^-17
+    where it is largest, is far inside the rounding's 2^-8.)"""
+    torch = _torch()
+    from fngine_b200 import moe, prefill
+    T, inter = 96, 512
+    layer = moe.synth_layer(IQ3_S, IQ3_S, inter, 16, 909)
+    ws = prefill.PrefillWorkspace(T, inter)
+    x = synth.activations(45, T) * np.logspace(-2, 4, T, dtype=np.float32)[:, None]
+    xd = torch.from_numpy(synth.to_bf16_bits(x).view(np.int16)).cuda().view(torch.bfloat16)
+    lg = torch.full((T, 512), -30.0, device="cuda")
+    lg[:, :16] = torch.randn(T, 16, generator=torch.Generator(device="cuda").manual_seed(8), device="cuda")
+    run_prefill(torch, layer, ws, lg, xd, T)
+    assert ws.status() == 0
+    off = ws.ints(ws.ws.expert_offset, 513)
+    tok = torch.from_numpy(ws.ints(ws.ws.pair_token, T * 10)).cuda().long()
+    h = torch.from_numpy(synth.bf16_bits_to_f32(ws.h(T * 10))).cuda().double()
+    stride, gate = layer.layout.blob_stride, inter * O.row_bytes(IQ3_S, H)
+    lowest, highest = 0.0, 0.0
+    for e in range(16):
+        w = moe.dequant_rows(IQ3_S, layer.slots[e * stride:e * stride + 2 * gate], 2 * inter, H).to(torch.bfloat16).double()
+        p0, p1 = int(off[e]), int(off[e + 1])
+        xe = xd[tok[p0:p1]].double()
+        acc, mag = xe @ w.T, xe.abs() @ w.abs().T
+        g, u = acc[:, :inter], acc[:, inter:]
+        lowest, highest = min(lowest, float(g.min())), max(highest, float(g.max()))
+        silu = g * torch.sigmoid(g)
+        # fp32 sums: 2^-20 of the magnitudes' sum is four times what 2560 / 16 chained additions of random sign leave
+        room = 2.0 ** -20 * (1.1 * u.abs() * mag[:, :inter] + silu.abs() * mag[:, inter:])
+        got, want = h[p0:p1], silu * u
+        assert bool(torch.isfinite(got).all())
+        assert bool(((got - want).abs() <= 2.0 ** -8 * 1.01 * want.abs() + 1.01 * room + 1e-30).all()), e
+        assert float(got[g < -100.0].abs().max()) == 0.0
+    assert lowest < -500.0 and highest > 500.0
