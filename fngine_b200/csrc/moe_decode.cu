@@ -451,7 +451,7 @@ __device__ __forceinline__ void select_block(LoadF load, const int32_t* slot_of,
   }
   // (One warp per token. All sixteen warps on each token's slices - maxima, threshold, candidates and ranking behind a
   // barrier each - was slower at every batch: 3.3 against 2.5 us at one token, 6 against 3 at sixteen.)
-  if (warp < T) warp_top10_pruned([&](int e) { return load(warp, e); }, scratch.cand[warp], s_id[warp], s_val[warp]);
+  if (warp < T) warp_top10_pruned<false>([&](int e) { return load(warp, e); }, scratch.cand[warp], s_id[warp], s_val[warp]);
   __syncthreads();
   const int np = T * kTopK;
   const bool small = np <= 32;

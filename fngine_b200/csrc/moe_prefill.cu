@@ -166,8 +166,7 @@ struct PairNumbers {
 };
 
 // Top-10 per token (one warp each, PER_WARP in turn), per-expert pair counts and the pairs' numbers (token_pair, may be absent;
-// BLOCKS: by blocks). Rows of equal logits take the general path behind the pruned one: 2.3 us with the general path alone, 3.9 for
-// 1 to 4 tokens, 9.4 and 12.7 where all rows of 4096 are so.
+// BLOCKS: by blocks).
 // PER_WARP 4 from 4096 tokens on: fewer meetings on a popular expert's counter; below that single tokens fill the GPU.
 // The routing launches of 8192 tokens together: 45 us, 25 so (selection by the pruned search and numbering).
 template <int PER_WARP, bool BLOCKS>
@@ -189,7 +188,7 @@ __global__ void __launch_bounds__(256) pf_topk_kernel(const float* logits, int s
   for (int i = 0; i < PER_WARP; ++i) {
     const int t = t0 + i;
     if (t >= T) break;
-    warp_top10_pruned([&](int e) { return logits[size_t(t) * stride + e]; }, s_scratch[warp], s_ids[warp], s_vals[warp]);
+    warp_top10_pruned<true>([&](int e) { return logits[size_t(t) * stride + e]; }, s_scratch[warp], s_ids[warp], s_vals[warp]);
     __syncwarp();
     float vals[kTopK], w[kTopK];
 #pragma unroll

@@ -520,7 +520,17 @@ def test_route_numbers_every_pair_once(T):
     lg[0, :512] = 1.5  # all equal
     lg[T // 2, 40:300] = float("nan")
     lg[T - 1, 100:140] = 9.0
-    key = torch.where(torch.isnan(lg[:, :512]), torch.full_like(lg[:, :512], -float("inf")), lg[:, :512])
+    if T > 8:
+        lg[1, 60:500] = 8.0  # more equal ones than a warp's lanes behind one, eight and ten larger ones; zeros of both signs
+        lg[1, 501] = 9.0
+        lg[2, 60:500] = 8.0
+        lg[2, 200:360:20] = torch.arange(8, device="cuda") + 9.0
+        lg[3, 60:500] = 8.0
+        lg[3, 1:60:6] = 9.0
+        lg[4] = 0.0
+        lg[4, ::2] = -0.0
+        lg[5, :505] = -float("inf")
+    key = torch.where(torch.isnan(lg[:, :512]), torch.full_like(lg[:, :512], -float("inf")), lg[:, :512]) + 0.0  # -0 is 0
     want = torch.sort(key, dim=1, descending=True, stable=True).indices[:, :10]
     ws = prefill.PrefillWorkspace(T, 512)
     prefill.moe_route(lg, lg, None, 0, None, None, T, ws, logits_stride=513)
